@@ -111,6 +111,13 @@ SBVR_API int sbvr_linear_f16(const void* x, const uint32_t* bvr, const void* coe
                     int C, const void* bias, void* y, int M, int N, int K, int S, int G, int algo,
                     sbvr_workspace_t* ws, sbvr_stream_t stream);
 
+/* The same with unpadded activations: rows of K_in <= K elements (row pitch K_in), the product as if they were padded with
+ * zeros to K (what the reference's encoder does to the weight's inner dimension, sbvr/core.py:666-673).  K_in < K needs a
+ * workspace of sbvr_workspace_bytes(...): the padded rows are staged in it where the kernel picked reads whole rows. */
+SBVR_API int sbvr_linear_padded_f16(const void* x, int K_in, const uint32_t* bvr, const void* coeff_idx, int idx_bytes,
+                                    const void* coeff, int C, const void* bias, void* y, int M, int N, int K, int S, int G,
+                                    int algo, sbvr_workspace_t* ws, sbvr_stream_t stream);
+
 /* Same product with HOST x and y: copies x in, runs sbvr_linear_f16, copies y out, all on `stream`
  * (weights stay on the device).  The end-to-end form of the call the reference binding makes with a
  * CPU activation tensor.  x_host / y_host should be pinned for the copies to be asynchronous. */

@@ -3,7 +3,8 @@
     python sbvr-cpu-arm_b200/build.py [--force] [--verbose]
 
 Each csrc/*.cu is compiled to an object file (in parallel) and the objects are linked
-into sbvr-cpu-arm_b200/lib/libsbvr_b200.so.  nvcc cross-compiles, so no GPU is needed.
+into sbvr-cpu-arm_b200/lib/libsbvr_b200.so; csrc/pyext.cpp becomes the extension module
+lib/_sbvr_native.so beside it.  nvcc cross-compiles, so no GPU is needed.
 """
 from __future__ import annotations
 
@@ -18,6 +19,7 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "lib")
 OBJ_DIR = os.path.join(HERE, "build")
 LIB = os.path.join(OUT_DIR, "libsbvr_b200.so")
+NATIVE = os.path.join(OUT_DIR, "_sbvr_native.so")
 
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
@@ -63,7 +65,32 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    build_native(force, verbose)
     return LIB
+
+
+def build_native(force: bool = False, verbose: bool = False) -> str:
+    """lib/_sbvr_native.so: the Python extension module between the package and the library (csrc/pyext.cpp)."""
+    src = os.path.join(CSRC, "pyext.cpp")
+    if not (force or _stale(NATIVE, [src, LIB, os.path.join(HERE, "..", "include", "sbvr_b200.h")])):
+        return NATIVE
+    import sysconfig
+    import torch
+    from torch.utils import cpp_extension
+    troot = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.dirname(os.path.dirname(NVCC))
+    inc = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wno-deprecated-declarations",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += [a for d in inc for a in ("-isystem", d)] + [src, "-o", NATIVE]
+    cmd += ["-L" + OUT_DIR, "-lsbvr_b200", "-L" + troot, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
+            "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+    if r.returncode:
+        raise RuntimeError("g++ failed for pyext.cpp")
+    return NATIVE
 
 
 if __name__ == "__main__":

@@ -244,6 +244,25 @@ int sbvr_linear_f16(const void* x, const uint32_t* bvr, const void* coeff_idx, i
     return launch_linear_simt(xh, w, bh, yh, M, st);
 }
 
+int sbvr_linear_padded_f16(const void* x, int K_in, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff,
+                           int C, const void* bias, void* y, int M, int N, int K, int S, int G, int algo, sbvr_workspace_t* ws,
+                           sbvr_stream_t stream) {
+    if (K_in == K)
+        return sbvr_linear_f16(x, bvr, coeff_idx, idx_bytes, coeff, C, bias, y, M, N, K, S, G, algo, ws, stream);
+    if (!x || M < 1 || K_in < 1 || K_in > K) return SBVR_ERR_BAD_ARG;
+    if (reinterpret_cast<uintptr_t>(x) & 1) return SBVR_ERR_ALIGN;
+    if (!ws) return SBVR_ERR_WORKSPACE;
+    // the padded rows live at the end of the workspace, away from the kernels' scratch
+    const size_t xb = ((size_t)M * K * 2 + 255) / 256 * 256;
+    if (xb > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
+    sbvr_workspace shrunk = *ws;
+    shrunk.dyn_bytes = (ws->dyn_bytes - xb) / 256 * 256;
+    __half* xd = reinterpret_cast<__half*>(ws->dyn + shrunk.dyn_bytes);
+    const int rc = launch_pad_rows(reinterpret_cast<const __half*>(x), xd, M, K_in, K, reinterpret_cast<cudaStream_t>(stream));
+    if (rc) return rc;
+    return sbvr_linear_f16(xd, bvr, coeff_idx, idx_bytes, coeff, C, bias, y, M, N, K, S, G, algo, &shrunk, stream);
+}
+
 int sbvr_linear_fused_f16(int x_op, const void* x, const void* delta, const void* norm_weight, void* h_out, float eps,
                           const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff, int C,
                           const void* bias, void* y, int M, int N, int K, int S, int G, sbvr_workspace_t* ws,

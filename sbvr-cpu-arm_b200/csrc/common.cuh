@@ -120,6 +120,8 @@ inline int set_max_smem_once(SmemOnce& once, Kernel kernel, int bytes) {
 }
 
 int launch_decode(const PackedW& w, __half* W, int ldw, int Kout, cudaStream_t st);
+// out[m][0 .. K) = in[m][0 .. Kin) followed by zeros (glue.cu)
+int launch_pad_rows(const __half* in, __half* out, int M, int Kin, int K, cudaStream_t st);
 int launch_linear_simt(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, cudaStream_t st);
 // What the decode GEMV makes its activations of while it brings them in.
 struct XOp {

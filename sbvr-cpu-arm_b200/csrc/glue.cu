@@ -489,6 +489,30 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const __half* __re
         *reinterpret_cast<uint4*>(out + dst + (size_t)i * 8) = *reinterpret_cast<const uint4*>(table + src + (size_t)i * 8);
 }
 
+// rows of Kin halves -> rows of K (K % 8 == 0), zeros behind; one thread per 8 output elements, any Kin
+__global__ void __launch_bounds__(256) pad_rows_kernel(const __half* __restrict__ in, __half* __restrict__ out, int M, int Kin,
+                                                       int K) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int kv = K / 8;
+    const size_t nvec = (size_t)M * kv;
+    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += (size_t)gridDim.x * blockDim.x) {
+        const size_t m = v / kv;
+        const int k0 = (int)(v - m * kv) * 8;
+        __align__(16) __half o[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = (k0 + e < Kin) ? in[m * Kin + k0 + e] : __float2half(0.0f);
+        *reinterpret_cast<uint4*>(out + v * 8) = *reinterpret_cast<const uint4*>(o);
+    }
+}
+
+int launch_pad_rows(const __half* in, __half* out, int M, int Kin, int K, cudaStream_t st) {
+    if (K % 8) return SBVR_ERR_SHAPE;
+    const size_t blocks = ((size_t)M * (K / 8) + 255) / 256;
+    SBVR_CUDA_TRY(launch_pdl(pad_rows_kernel, dim3((unsigned)(blocks < 2368 ? blocks : 2368)), dim3(256), 0, st, in, out, M, Kin, K));
+    return SBVR_OK;
+}
+
 // index of the first maximum of each row (torch.argmax's tie rule); NaN wins like in torch.
 // grid (rows, parts): part `blockIdx.y` scans its slice of the row and leaves (value, index) in `partial`
 // (or, with one part, writes the result); argmax_final_kernel picks the winner of the parts.

@@ -7,7 +7,10 @@ binding raised RuntimeError from `std::runtime_error` (reference sbvr/kernels/sb
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
+
+import torch  # noqa: F401  (the extension module resolves its symbols in torch's libraries)
 
 _PKG_ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 LIB_PATH = os.path.join(_PKG_ROOT, "lib", "libsbvr_b200.so")
@@ -18,6 +21,14 @@ if not os.path.exists(LIB_PATH):
         "(there is no CPU or PyTorch fallback for the SBVR kernels)")
 
 lib = ctypes.CDLL(LIB_PATH)
+
+# The host path between the Python API and the library (csrc/pyext.cpp), an extension module beside it.
+NATIVE_PATH = os.path.join(_PKG_ROOT, "lib", "_sbvr_native.so")
+if not os.path.exists(NATIVE_PATH):
+    raise ImportError(f"{NATIVE_PATH} not found: build it with `python sbvr-cpu-arm_b200/build.py`")
+_spec = importlib.util.spec_from_file_location("_sbvr_native", NATIVE_PATH)
+native = importlib.util.module_from_spec(_spec)
+_spec.loader.exec_module(native)
 
 _vp, _i, _sz = ctypes.c_void_p, ctypes.c_int, ctypes.c_size_t
 _ip = ctypes.POINTER(ctypes.c_int)
@@ -44,6 +55,8 @@ lib.sbvr_decode_f16.argtypes = [_vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, 
 lib.sbvr_decode_f16.restype = _i
 lib.sbvr_linear_f16.argtypes = [_vp, _vp, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp]
 lib.sbvr_linear_f16.restype = _i
+lib.sbvr_linear_padded_f16.argtypes = [_vp, _i, _vp, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp]
+lib.sbvr_linear_padded_f16.restype = _i
 lib.sbvr_linear_fused_f16.argtypes = [_i, _vp, _vp, _vp, _vp, ctypes.c_float, _vp, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i,
                                       _i, _i, _vp, _vp]
 lib.sbvr_linear_fused_f16.restype = _i
@@ -89,7 +102,7 @@ lib.sbvr_ll_reduce_add_rmsnorm_digits_f16.restype = _i
 lib.sbvr_allreduce_add_rmsnorm_digits_f16.argtypes = [_vp, _vp, _vp, _i, _i, _i, _i, _sz, _vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp, _vp]
 lib.sbvr_allreduce_add_rmsnorm_digits_f16.restype = _i
 
-EXPORTS = ["sbvr_popc_mm_f16", "sbvr_linear_t_f16", "sbvr_encode_mse_f16", "sbvr_encode_select_f16", "sbvr_encode_pack", "sbvr_rope_attention_f16", "sbvr_linear_fused_f16", "sbvr_allreduce_add_rmsnorm_f16", "sbvr_linear_push_f16", "sbvr_ll_reduce_add_rmsnorm_f16", "sbvr_ll_reduce_add_rmsnorm_digits_f16", "sbvr_allreduce_add_rmsnorm_digits_f16", "sbvr_add_rmsnorm_f16", "sbvr_rope_append_f16", "sbvr_attention_f16", "sbvr_silu_mul_f16",
+EXPORTS = ["sbvr_linear_padded_f16", "sbvr_popc_mm_f16", "sbvr_linear_t_f16", "sbvr_encode_mse_f16", "sbvr_encode_select_f16", "sbvr_encode_pack", "sbvr_rope_attention_f16", "sbvr_linear_fused_f16", "sbvr_allreduce_add_rmsnorm_f16", "sbvr_linear_push_f16", "sbvr_ll_reduce_add_rmsnorm_f16", "sbvr_ll_reduce_add_rmsnorm_digits_f16", "sbvr_allreduce_add_rmsnorm_digits_f16", "sbvr_add_rmsnorm_f16", "sbvr_rope_append_f16", "sbvr_attention_f16", "sbvr_silu_mul_f16",
            "sbvr_embedding_f16", "sbvr_argmax_f16", "sbvr_linear_f16_noalloc", "sbvr_workspace_bytes", "sbvr_strerror", "sbvr_last_cuda_error", "sbvr_last_timeout_where", "sbvr_last_timeout_info", "sbvr_query", "sbvr_workspace_create",
            "sbvr_workspace_destroy", "sbvr_workspace_status", "sbvr_decode_f16", "sbvr_linear_f16",
            "sbvr_linear_f16_host"]
@@ -173,4 +186,8 @@ def workspace(device: int, stream: int, nbytes: int = 0) -> Workspace:
     if ws is None:
         ws = Workspace(device, max(nbytes, Workspace.DEFAULT_BYTES))
         _workspaces[key] = ws
+        native.set_workspace(device, stream, ws.handle.value, ws.nbytes)
     return ws
+
+
+native.set_workspace_callback(workspace)

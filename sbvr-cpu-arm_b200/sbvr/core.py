@@ -14,9 +14,9 @@ Packed tensors (GPU layout of the reference, sbvr/core.py:724-805):
 """
 from __future__ import annotations
 
+import math
 from typing import Optional
 
-import numpy as np
 import torch
 
 from . import _lib
@@ -249,21 +249,12 @@ class sbvr(torch.nn.Module):
             self.coeff_cache.shape[0])
 
     # -- operations ---------------------------------------------------------------------------
-    @torch.inference_mode()
     def decode(self) -> torch.Tensor:
         """Dense fp16 tensor of the original shape (reference `decode`, sbvr/core.py:926-949), computed by
         the CUDA decode kernel, bit-exact with the reference."""
-        dev = self.bvr.device
-        di = _cuda_index(dev)
-        N, Kp = self.out_features, self.in_features_padded
-        K = int(self.original_data_shape[-1])
-        out = torch.empty((N, K), dtype=torch.float16, device=dev)
-        b, ix, ib, c, C = self._abi_args()
-        with torch.cuda.device(di):
-            st = torch.cuda.current_stream().cuda_stream
-            _lib.check(_lib.lib.sbvr_decode_f16(b, ix, ib, c, C, out.data_ptr(), K, N, Kp, K, self.num_sums,
-                                                self.bvr_len, st), "sbvr_decode_f16")
-        return out.view(self.original_data_shape) if out.numel() == int(np.prod(self.original_data_shape)) else out
+        out = _lib.native.decode(self)
+        shape = self.original_data_shape
+        return out.view(shape) if len(shape) != 2 and out.numel() == math.prod(shape) else out
 
     def _serialize(self) -> _sbvr_serialized:
         if self.coeff_idx is None:
@@ -283,7 +274,6 @@ class sbvr(torch.nn.Module):
                 f"coeff_cache={tuple(self.coeff_cache.shape)}")
 
 
-@torch.inference_mode()
 def linear(x: torch.Tensor, w: sbvr, bias: Optional[torch.Tensor] = None, algo: int = 0,
            out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y = x @ W.T (+ bias) with fp16 `x` [..., K] and a packed weight `w`, fp32 accumulation, fp16 result.
@@ -291,45 +281,14 @@ def linear(x: torch.Tensor, w: sbvr, bias: Optional[torch.Tensor] = None, algo: 
     The product the reference's Llama flow computes with the decoded weight (sbvr_utils/utils_llama.py:147)
     and its `_sbvr_row_deq_mm_T` binding computes on a transposed encoding (sbvr/kernels/sbvr_ops.cpp:79-120).
     `bias` may be None or an empty tensor (the reference's "no bias" convention, sbvr/core.py:353-358).
+    Runs in inference mode, like every operation of the package (csrc/pyext.cpp).
     """
-    if x.dtype != torch.float16:
-        raise ValueError("activations must be float16")
-    dev = w.bvr.device
-    di = _cuda_index(dev)
-    if x.device != dev:
-        raise ValueError(f"activation on {x.device}, weight on {dev}")
-    K = int(w.original_data_shape[-1])
-    Kp, N = w.in_features_padded, w.out_features
-    if x.shape[-1] != K:
-        raise ValueError(_r_str(f"inner dimension mismatch: activation {x.shape[-1]}, weight {K}"))
-    lead = x.shape[:-1]
-    x2 = x.reshape(-1, K)
-    if Kp != K:
-        x2 = torch.nn.functional.pad(x2, (0, Kp - K))
-    x2 = x2.contiguous()
-    M = x2.shape[0]
-    if bias is not None and bias.numel() == 0:
-        bias = None
-    if bias is not None:
-        if bias.numel() != N or bias.dtype != torch.float16:
-            raise ValueError("bias must be float16 of length N")
-        bias = bias.contiguous()
-    y = out if out is not None else torch.empty((M, N), dtype=torch.float16, device=dev)
-    if M == 0:
-        return y.view(*lead, N)
-    b, ix, ib, c, C = w._abi_args()
-    with torch.cuda.device(di):
-        st = torch.cuda.current_stream().cuda_stream
-        ws = _lib.workspace(di, st, _lib.workspace_bytes(di, M, N, Kp) if M > 4 else 0)
-        _lib.check(_lib.lib.sbvr_linear_f16(x2.data_ptr(), b, ix, ib, c, C, _ptr(bias), y.data_ptr(), M, N, Kp,
-                                            w.num_sums, w.bvr_len, algo, ws.handle, st), "sbvr_linear_f16")
-    return y.view(*lead, N)
+    return _lib.native.linear(x, w, bias, algo, out)
 
 
 XOP_NONE, XOP_SILU_MUL, XOP_ADD_RMSNORM, XOP_DIGITS = 0, 1, 2, 3
 
 
-@torch.inference_mode()
 def linear_fused(op: int, x: torch.Tensor, w: sbvr, out: torch.Tensor, delta: Optional[torch.Tensor] = None,
                  norm_weight: Optional[torch.Tensor] = None, h_out: Optional[torch.Tensor] = None, eps: float = 0.0,
                  bias: Optional[torch.Tensor] = None) -> bool:
@@ -338,26 +297,9 @@ def linear_fused(op: int, x: torch.Tensor, w: sbvr, out: torch.Tensor, delta: Op
     with x + delta stored to h_out;  XOP_DIGITS: out = x @ W.T where the kernel launched directly before on this stream
     (an all-reduce + RMSNorm with emit_digits) has already left x quantised in the stream's workspace.
     Returns False (and computes nothing) where the decode kernel does not apply."""
-    dev = w.bvr.device
-    di = _cuda_index(dev)
-    Kp, N = w.in_features_padded, w.out_features
-    M = x.shape[0]
-    if M > 4 or int(w.original_data_shape[-1]) != Kp or not x.is_contiguous():
-        return False
-    b, ix, ib, c, C = w._abi_args()
-    with torch.cuda.device(di):
-        st = torch.cuda.current_stream().cuda_stream
-        ws = _lib.workspace(di, st)
-        rc = _lib.lib.sbvr_linear_fused_f16(op, x.data_ptr(), _ptr(delta), _ptr(norm_weight), _ptr(h_out), float(eps), b,
-                                            ix, ib, c, C, _ptr(bias), out.data_ptr(), M, N, Kp, w.num_sums, w.bvr_len,
-                                            ws.handle, st)
-    if rc == -7:
-        return False
-    _lib.check(rc, "sbvr_linear_fused_f16")
-    return True
+    return _lib.native.linear_fused(op, x, w, out, delta, norm_weight, h_out, eps, bias)
 
 
-@torch.inference_mode()
 def mm_T(lhs, rhs: sbvr, bias=None):
     """`lhs @ rhs.T + bias` (reference `mm_T`, sbvr/core.py:1029-1039).  `lhs` may be an fp16 tensor (-> `linear`) or, as
     in the reference, an `sbvr` object: then both operands stay encoded and the product runs on the popcount kernel
@@ -365,39 +307,19 @@ def mm_T(lhs, rhs: sbvr, bias=None):
     coefficients, group length other than 256) are decoded on the GPU and go through `linear`."""
     if not isinstance(lhs, sbvr):
         return linear(lhs, rhs, bias)
-    ok = (lhs.bvr_len == 256 and rhs.bvr_len == 256 and lhs.coeff_idx is not None and rhs.coeff_idx is not None and
-          2 <= lhs.num_sums <= 4 and 2 <= rhs.num_sums <= 4 and lhs.in_features_padded == rhs.in_features_padded and
-          lhs.bvr.device == rhs.bvr.device)
-    if not ok:
-        return linear(lhs.decode(), rhs, bias)
-    dev = rhs.bvr.device
-    di = _cuda_index(dev)
-    M, N, K = lhs.out_features, rhs.out_features, rhs.in_features_padded
-    if bias is not None and bias.numel() == 0:
-        bias = None
-    if bias is not None:
-        if bias.numel() != N or bias.dtype != torch.float16:
-            raise ValueError("bias must be float16 of length N")
-        bias = bias.contiguous()
-    y = torch.empty((M, N), dtype=torch.float16, device=dev)
-    lb, lix, lib_, lc, lC = lhs._abi_args()
-    rb, rix, rib, rc, rC = rhs._abi_args()
-    with torch.cuda.device(di):
-        st = torch.cuda.current_stream().cuda_stream
-        _lib.check(_lib.lib.sbvr_popc_mm_f16(lb, lix, lib_, lc, lC, lhs.num_sums, rb, rix, rib, rc, rC, rhs.num_sums,
-                                             _ptr(bias), y.data_ptr(), M, N, K, st), "sbvr_popc_mm_f16")
-    return y
+    y = _lib.native.mm_T(lhs, rhs, bias)
+    return linear(lhs.decode(), rhs, bias) if y is None else y
 
 
 def row_deq_mm_T(x: torch.Tensor, w_t: sbvr, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """`x @ W.T + bias` for a weight encoded transposed (`sbvr(W, trans=True)` in the reference, sbvr/core.py:244-245:
     `w_t` holds W^T, so `w_t.decode()` is [K, N]).  What the reference's `_sbvr_row_deq_mm_T` call sites compute
     (test_sbvr.py:588-592); the result has the padded width `w_t.in_features_padded`, as there."""
-    from . import sbvr_cuda
-    if w_t.coeff_idx is None:
+    p = w_t._parameters
+    idx = p.get("coeff_idx")
+    if idx is None:
         raise ValueError(_r_str("the transposed layout needs codebook indices (the reference has no direct form)"))
-    return sbvr_cuda._sbvr_row_deq_mm_T(x.reshape(-1, x.shape[-1]), w_t.bvr, w_t.coeff_idx, w_t.coeff_cache,
-                                        bias if bias is not None else w_t._get_dummy_bias(), 0)
+    return _lib.native.row_deq(x if x.dim() == 2 else x.reshape(-1, x.shape[-1]), p["bvr"], idx, p["coeff_cache"], bias)
 
 
 def load(filename, device=None, verbose_level=1, cpu_kernel=False, cpu_kernel_v2=False) -> sbvr:

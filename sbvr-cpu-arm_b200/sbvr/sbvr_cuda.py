@@ -29,37 +29,12 @@ def _sbvr_cuda_init() -> None:
     _lib.query(torch.cuda.current_device())
 
 
-@torch.inference_mode()
 def _sbvr_row_deq_mm_T(l_w: torch.Tensor, r_bvr: torch.Tensor, r_coeff_idx: torch.Tensor, r_coeff_cache: torch.Tensor,
                        bias: torch.Tensor, use_shfl: int = 0) -> torch.Tensor:
     """out[M, N] = l_w[M, K] @ W^T + bias with the weight in the transposed encoding: r_bvr uint32 [N/32, K, S],
     r_coeff_idx [N/256, K], r_coeff_cache fp16 [C, S] (reference sbvr_row_deq_mm_T, sbvr_ops.cpp:79-120).
     `use_shfl` selected between two reference kernels with the same result; it is accepted and ignored."""
-    if l_w.dtype != torch.float16 or r_coeff_cache.dtype != torch.float16:
-        raise ValueError("activations and coefficients must be float16")
-    if r_bvr.dtype == torch.int32:
-        r_bvr = r_bvr.view(torch.uint32)
-    if r_bvr.dtype != torch.uint32 or r_bvr.dim() != 3:
-        raise ValueError("r_bvr must be uint32 [N/32, K, S]")
-    di = _dev_index(l_w)
-    M, K = int(l_w.shape[0]), int(r_bvr.shape[1])
-    N, S, C = int(r_bvr.shape[0]) * 32, int(r_bvr.shape[2]), int(r_coeff_cache.shape[0])
-    if l_w.shape[1] != K:
-        raise ValueError(f"inner dimension mismatch: activation {l_w.shape[1]}, weight {K}")
-    G = N // int(r_coeff_idx.shape[0])
-    ib = _idx_bytes(r_coeff_idx, r_coeff_cache)
-    l_w, r_bvr, r_coeff_idx, r_coeff_cache = (t.contiguous() for t in (l_w, r_bvr, r_coeff_idx, r_coeff_cache))
-    b = bias.contiguous() if (bias is not None and bias.numel() == N) else None
-    out = torch.empty((M, N), dtype=torch.float16, device=l_w.device)
-    if M == 0:
-        return out
-    with torch.cuda.device(di):
-        st = torch.cuda.current_stream().cuda_stream
-        ws = _lib.workspace(di, st)
-        _lib.check(_lib.lib.sbvr_linear_t_f16(l_w.data_ptr(), r_bvr.data_ptr(), r_coeff_idx.data_ptr(), ib,
-                                              r_coeff_cache.data_ptr(), C, None if b is None else b.data_ptr(),
-                                              out.data_ptr(), M, N, K, S, G, ws.handle, st), "sbvr_linear_t_f16")
-    return out
+    return _lib.native.row_deq(l_w, r_bvr, r_coeff_idx, r_coeff_cache, bias)
 
 
 @torch.inference_mode()
