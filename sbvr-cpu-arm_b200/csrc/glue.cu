@@ -326,131 +326,223 @@ __global__ void __launch_bounds__(128) attention_combine_kernel(const float* __r
 }
 
 // ---------------------------------------------------------------------------------------------
-// Causal prefill: QB consecutive tokens of a sequence share a CTA, so that a K or V row is fetched once for
-// 16 = QB * R (query token, query head) pairs instead of once per token.  grid sequences * n_kv * ceil(tps / QB).
-// Same arithmetic as attention_kernel: scores and probabilities in fp32, running maximum per pair.
+// Causal prefill on the tensor cores: a CTA takes 64 (query token, query head) pairs that share one KV head (64 / R
+// consecutive tokens of a sequence x its R query heads), each of its four warps 16 of them, and walks the keys 64 at a time
+// with a running maximum and sum per pair.  grid sequences * n_kv * ceil(tokens / (64 / R)), longest contexts first.
+//
+//   scores   q . k: mma.sync m16n8k16 on the fp16 values themselves, fp32 accumulation, scaled in fp32
+//   weights  exp2 in fp32; for the product with V each is split into two fp16 parts (p = hi + lo to 2^-22), two MMAs per
+//            tile, so that the probabilities keep their fp32 precision
+//
+// K and V tiles come through cp.async, double buffered, rows of 256 bytes with their 16-byte chunks XOR-swizzled by the row
+// (ldmatrix without bank conflicts).  What bounds it is the tensor pipe's legacy path and the exponentials.  The CUDA-core
+// kernel this replaces read K and V once per 16 pairs and was bound by fp32 FMA issue: 1 790 us per layer at 2 x 1500
+// tokens, 32 query heads, 8 KV heads.
 // ---------------------------------------------------------------------------------------------
+constexpr int AP_ROWS = 64, AP_KEYS = 64, AP_THREADS = 128;
+constexpr int AP_TILE = AP_KEYS * AT_D * 2;                    // bytes of a K or V tile
+constexpr int AP_SMEM = 4 * AP_TILE;
+
+__device__ __forceinline__ void ap_cp16(uint32_t dst, const void* src, bool on) {
+    const uint32_t bytes = on ? 16u : 0u;                      // 0: sixteen zero bytes
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void ap_ldm4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ void ap_ldm4t(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr)
+                 : "memory");
+}
+__device__ __forceinline__ void ap_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float ap_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// fp16 pair of (lo, hi) and what the rounding left over, as a second pair
+__device__ __forceinline__ uint32_t ap_split(float lo, float hi, uint32_t& rest) {
+    const __half2 h = __floats2half2_rn(lo, hi);
+    const float2 f = __half22float2(h);
+    const __half2 r = __floats2half2_rn(lo - f.x, hi - f.y);
+    rest = *reinterpret_cast<const uint32_t*>(&r);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 template <int R>
-__global__ void __launch_bounds__(128) attention_block_kernel(const __half* __restrict__ qkv, const __half* __restrict__ kcache,
-                                                              const __half* __restrict__ vcache,
-                                                              const int* __restrict__ positions, __half* __restrict__ out,
-                                                              int tokens_per_seq, int n_heads, int n_kv, int max_ctx,
-                                                              float scale) {
-    constexpr int QB = 16 / R, NQ = 16;
-    __shared__ float qs[NQ][AT_D];
-    __shared__ float wm[4][NQ], wl[4][NQ];
-    __shared__ float wacc[4][NQ][AT_D];
-    __shared__ int ctx_s[QB];
+__global__ void __launch_bounds__(AP_THREADS, 2)
+    attention_prefill_kernel(const __half* __restrict__ qkv, const __half* __restrict__ kcache, const __half* __restrict__ vcache,
+                             const int* __restrict__ positions, __half* __restrict__ out, int tokens_per_seq, int n_heads, int n_kv,
+                             int max_ctx, float scale) {
+    constexpr int QT = AP_ROWS / R;                            // tokens of a CTA
+    extern __shared__ __align__(128) unsigned char ap_smem[];
+    __shared__ int ctx_s[QT];
     pdl_launch_dependents();
     pdl_wait();
-    const int nblk = (tokens_per_seq + QB - 1) / QB;
-    // the blocks with the longest context are scheduled first (they finish last otherwise)
-    const int rest = blockIdx.x % ((int)gridDim.x / nblk), qblk = nblk - 1 - (int)blockIdx.x / ((int)gridDim.x / nblk);
+    const int nblk = (tokens_per_seq + QT - 1) / QT;
+    const int per = (int)gridDim.x / nblk;                     // sequences * n_kv
+    const int rest = blockIdx.x % per, qblk = nblk - 1 - (int)blockIdx.x / per;
     const int kvh = rest % n_kv, seq = rest / n_kv;
-    const int t0 = seq * tokens_per_seq + qblk * QB;
-    const int nq = min(QB, tokens_per_seq - qblk * QB);
+    const int t0 = seq * tokens_per_seq + qblk * QT;
+    const int nq = min(QT, tokens_per_seq - qblk * QT);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x < QB) ctx_s[threadIdx.x] = (threadIdx.x < nq) ? min(positions[t0 + threadIdx.x] + 1, max_ctx) : 0;
-    for (int i = threadIdx.x; i < NQ * AT_D; i += 128) {
-        const int q = i / AT_D, dd = i % AT_D, j = q / R, r = q % R;
-        qs[q][dd] = (j < nq) ? __half2float(qkv[(size_t)(t0 + j) * (n_heads + 2 * n_kv) * AT_D +
-                                                 (size_t)(kvh * R + r) * AT_D + dd]) * scale
-                             : 0.0f;
-    }
+    const int gid = lane >> 2, tig = lane & 3;
+    for (int j = threadIdx.x; j < QT; j += AP_THREADS) ctx_s[j] = (j < nq) ? min(positions[t0 + j] + 1, max_ctx) : 0;
     __syncthreads();
-    int P = 0;
-#pragma unroll
-    for (int j = 0; j < QB; ++j) P = max(P, ctx_s[j]);
+    int P = 0, pmin = 0x7fffffff;                              // keys any / every live token of the CTA attends to
+    for (int j = 0; j < nq; ++j) P = max(P, ctx_s[j]), pmin = min(pmin, ctx_s[j]);
     const __half* kb = kcache + ((size_t)seq * n_kv + kvh) * max_ctx * AT_D;
     const __half* vb = vcache + ((size_t)seq * n_kv + kvh) * max_ctx * AT_D;
+    const uint32_t ks0 = smem_u32(ap_smem), vs0 = ks0 + 2 * AP_TILE;
 
-    float m[NQ], l[NQ], acc[NQ][4];
+    auto load_tile = [&](int tile, int buf) {
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        m[q] = -INFINITY, l[q] = 0.0f;
+        for (int i = 0; i < AP_KEYS * 16 / AP_THREADS; ++i) {
+            const int c = i * AP_THREADS + (int)threadIdx.x;
+            const int row = c >> 4, ch = c & 15;
+            const int key = tile * AP_KEYS + row;
+            const bool on = key < P;
+            const size_t src = (size_t)(on ? key : 0) * AT_D + ch * 8;
+            const uint32_t dst = (uint32_t)(buf * AP_TILE + row * 256 + ((ch ^ (row & 7)) << 4));
+            ap_cp16(ks0 + dst, kb + src, on);
+            ap_cp16(vs0 + dst, vb + src, on);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int ntile = (P + AP_KEYS - 1) / AP_KEYS;
+    if (ntile > 0) load_tile(0, 0);
+
+    // this thread's two rows of the warp's sixteen, and their queries as MMA fragments
+    int ctx[2];
+    uint32_t qf[8][4];
+    const size_t tok_pitch = (size_t)(n_heads + 2 * n_kv) * AT_D;
+    const bool even = (reinterpret_cast<uintptr_t>(qkv) & 3) == 0;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[q][e] = 0.0f;
+    for (int h = 0; h < 2; ++h) {
+        const int row = warp * 16 + gid + 8 * h, j = row / R, r = row % R;
+        ctx[h] = ctx_s[j];
+        const __half* q = qkv + (size_t)(t0 + min(j, nq - 1)) * tok_pitch + (size_t)(kvh * R + r) * AT_D + tig * 2;
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const __half* e = q + kk * 16 + c * 8;
+                uint32_t v;
+                if (even) v = *reinterpret_cast<const uint32_t*>(e);
+                else v = (uint32_t)__half_as_ushort(e[0]) | ((uint32_t)__half_as_ushort(e[1]) << 16);
+                qf[kk][h + 2 * c] = v;
+            }
     }
-    for (int base = warp * 32; base < P; base += 128) {
-        const int p = base + lane;
-        float sc[NQ];
+    float o[16][4], mx[2] = {-INFINITY, -INFINITY}, sum[2] = {0.0f, 0.0f};
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) sc[q] = 0.0f;
-        if (p < P) {
-            const uint4* kr = reinterpret_cast<const uint4*>(kb + (size_t)p * AT_D);
-#pragma unroll 4
-            for (int c = 0; c < AT_D / 8; ++c) {
-                const uint4 kv = __ldg(kr + c);
-                const __half2* kh = reinterpret_cast<const __half2*>(&kv);
-                float kf[8];
+    for (int i = 0; i < 16; ++i)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 f = __half22float2(kh[e]);
-                    kf[2 * e] = f.x, kf[2 * e + 1] = f.y;
-                }
+        for (int e = 0; e < 4; ++e) o[i][e] = 0.0f;
+    const float sl2 = scale * 1.4426950408889634f;             // exponentials to base 2
+    const int lrow = lane & 7;
+    const uint32_t k_row = (uint32_t)((lrow + ((lane >> 4) & 1) * 8) * 256);
+    const uint32_t v_row = (uint32_t)((lrow + ((lane >> 3) & 1) * 8) * 256);
+    const int k_ch = (lane >> 3) & 1, v_ch = lane >> 4;
+
+#pragma unroll 1
+    for (int t = 0; t < ntile; ++t) {
+        const int buf = t & 1;
+        if (t + 1 < ntile) {
+            load_tile(t + 1, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const uint32_t kt = ks0 + buf * AP_TILE, vt = vs0 + buf * AP_TILE;
+        float s[8][4];
 #pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    const float4 a = *reinterpret_cast<const float4*>(&qs[q][c * 8]);
-                    const float4 b = *reinterpret_cast<const float4*>(&qs[q][c * 8 + 4]);
-                    sc[q] += kf[0] * a.x + kf[1] * a.y + kf[2] * a.z + kf[3] * a.w + kf[4] * b.x + kf[5] * b.y +
-                             kf[6] * b.z + kf[7] * b.w;
-                }
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[i][e] = 0.0f;
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+#pragma unroll
+            for (int np = 0; np < 4; ++np) {
+                uint32_t b[4];
+                ap_ldm4(kt + np * 16 * 256 + k_row + (uint32_t)(((kk * 2 + k_ch) ^ lrow) << 4), b);
+                ap_mma(s[np * 2], qf[kk], b[0], b[1]);
+                ap_mma(s[np * 2 + 1], qf[kk], b[2], b[3]);
             }
         }
-        float w[NQ];
+        if ((t + 1) * AP_KEYS > pmin) {                        // some token's context ends inside or before this tile
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) {
-            const bool on = p < ctx_s[q / R];      // causal: token j sees positions up to its own
-            float cm = on ? sc[q] : -INFINITY;
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int o = 16; o; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
-            const float nm = fmaxf(m[q], cm);
-            const float corr = (m[q] == -INFINITY) ? 0.0f : __expf(m[q] - nm);
-            w[q] = on ? __expf(sc[q] - nm) : 0.0f;
-            l[q] = l[q] * corr + warp_sum(w[q]);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[q][e] *= corr;
-            m[q] = nm;
+                for (int e = 0; e < 4; ++e)
+                    if (t * AP_KEYS + i * 8 + tig * 2 + (e & 1) >= ctx[e >> 1]) s[i][e] = -INFINITY;
         }
-        const int np = min(32, P - base);
-        for (int j0 = 0; j0 < np; j0 += 4) {       // four V rows in flight; rows past the end carry weight 0
-            uint2 vv[4];
+        float base[2];
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                vv[u] = __ldg(reinterpret_cast<const uint2*>(vb + (size_t)min(base + j0 + u, max_ctx - 1) * AT_D) + lane);
+        for (int h = 0; h < 2; ++h) {
+            float m = mx[h];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const __half2* vh = reinterpret_cast<const __half2*>(&vv[u]);
-                const float2 f0 = __half22float2(vh[0]), f1 = __half22float2(vh[1]);
+            for (int i = 0; i < 8; ++i) m = fmaxf(m, fmaxf(s[i][2 * h], s[i][2 * h + 1]));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            base[h] = (m == -INFINITY) ? 0.0f : m * sl2;       // a row without any key so far
+            const float corr = (mx[h] == -INFINITY) ? 0.0f : ap_exp2(mx[h] * sl2 - base[h]);
+            mx[h] = m;
+            sum[h] *= corr;
 #pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    const float wj = __shfl_sync(0xffffffffu, w[q], j0 + u);
-                    acc[q][0] += wj * f0.x, acc[q][1] += wj * f0.y, acc[q][2] += wj * f1.x, acc[q][3] += wj * f1.y;
-                }
+            for (int i = 0; i < 16; ++i) o[i][2 * h] *= corr, o[i][2 * h + 1] *= corr;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                s[i][e] = ap_exp2(fmaf(s[i][e], sl2, -base[e >> 1]));
+                sum[e >> 1] += s[i][e];
+            }
+#pragma unroll
+        for (int kq = 0; kq < 4; ++kq) {                       // sixteen keys at a time
+            uint32_t ph[4], pl[4];
+            ph[0] = ap_split(s[2 * kq][0], s[2 * kq][1], pl[0]);
+            ph[1] = ap_split(s[2 * kq][2], s[2 * kq][3], pl[1]);
+            ph[2] = ap_split(s[2 * kq + 1][0], s[2 * kq + 1][1], pl[2]);
+            ph[3] = ap_split(s[2 * kq + 1][2], s[2 * kq + 1][3], pl[3]);
+#pragma unroll
+            for (int nd = 0; nd < 8; ++nd) {
+                uint32_t b[4];
+                ap_ldm4t(vt + kq * 16 * 256 + v_row + (uint32_t)(((nd * 2 + v_ch) ^ lrow) << 4), b);
+                ap_mma(o[nd * 2], ph, b[0], b[1]);
+                ap_mma(o[nd * 2 + 1], ph, b[2], b[3]);
+                ap_mma(o[nd * 2], pl, b[0], b[1]);
+                ap_mma(o[nd * 2 + 1], pl, b[2], b[3]);
             }
         }
+        __syncthreads();                                       // the buffer may be overwritten
     }
+    const bool even_o = (reinterpret_cast<uintptr_t>(out) & 3) == 0;
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-        if (lane == 0) wm[warp][q] = m[q], wl[warp][q] = l[q];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) wacc[warp][q][lane * 4 + e] = acc[q][e];
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < NQ * AT_D; i += 128) {
-        const int q = i / AT_D, dd = i % AT_D, j = q / R, r = q % R;
+    for (int h = 0; h < 2; ++h) {
+        float l = sum[h];
+        l += __shfl_xor_sync(0xffffffffu, l, 1);
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        const int row = warp * 16 + gid + 8 * h, j = row / R, r = row % R;
         if (j >= nq) continue;
-        float gm = -INFINITY;
+        __half* dst = out + ((size_t)(t0 + j) * n_heads + kvh * R + r) * AT_D + tig * 2;
 #pragma unroll
-        for (int w4 = 0; w4 < 4; ++w4) gm = fmaxf(gm, wm[w4][q]);
-        float gl = 0.0f, ga = 0.0f;
-#pragma unroll
-        for (int w4 = 0; w4 < 4; ++w4) {
-            const float c = (wm[w4][q] == -INFINITY) ? 0.0f : __expf(wm[w4][q] - gm);
-            gl += wl[w4][q] * c;
-            ga += wacc[w4][q][dd] * c;
+        for (int i = 0; i < 16; ++i) {
+            const __half2 v = __floats2half2_rn(o[i][2 * h] * inv, o[i][2 * h + 1] * inv);
+            if (even_o) *reinterpret_cast<__half2*>(dst + i * 8) = v;
+            else dst[i * 8] = __low2half(v), dst[i * 8 + 1] = __high2half(v);
         }
-        out[((size_t)(t0 + j) * n_heads + kvh * R + r) * AT_D + dd] = __float2half_rn(gl > 0.0f ? ga / gl : 0.0f);
     }
 }
 
@@ -633,19 +725,25 @@ static int attention_launch(const void* qkv, void* kcache, void* vcache, const i
     __half* vc = reinterpret_cast<__half*>(vcache);
     __half* o = reinterpret_cast<__half*>(out);
     if (!inv_freq && nsplit == 1 && tokens_per_seq >= 8) {      // prefill: tokens of a sequence share K / V fetches
-        const int QB = 16 / R, nblk = (tokens_per_seq + QB - 1) / QB;
+        if (R != 1 && R != 2 && R != 4 && R != 8) return SBVR_ERR_UNSUPPORTED;
+        const int QT = AP_ROWS / R, nblk = (tokens_per_seq + QT - 1) / QT;
         const dim3 bgrid((unsigned)((tokens / tokens_per_seq) * n_kv * nblk));
-#define SBVR_ATTB(RR)                                                                                               \
-    SBVR_CUDA_TRY(launch_pdl(attention_block_kernel<RR>, bgrid, dim3(128), 0, st, q, static_cast<const __half*>(kc), \
-                             static_cast<const __half*>(vc), positions, o, tokens_per_seq, n_heads, n_kv, max_ctx, scale))
+#define SBVR_ATTP(RR)                                                                                                       \
+    do {                                                                                                                    \
+        static SmemOnce once;                                                                                               \
+        const int rc = set_max_smem_once(once, attention_prefill_kernel<RR>, AP_SMEM);                                      \
+        if (rc) return rc;                                                                                                  \
+        SBVR_CUDA_TRY(launch_pdl(attention_prefill_kernel<RR>, bgrid, dim3(AP_THREADS), (size_t)AP_SMEM, st, q,             \
+                                 static_cast<const __half*>(kc), static_cast<const __half*>(vc), positions, o, tokens_per_seq, \
+                                 n_heads, n_kv, max_ctx, scale));                                                           \
+    } while (0)
         switch (R) {
-            case 1: SBVR_ATTB(1); break;
-            case 2: SBVR_ATTB(2); break;
-            case 4: SBVR_ATTB(4); break;
-            case 8: SBVR_ATTB(8); break;
-            default: return SBVR_ERR_UNSUPPORTED;
+            case 1: SBVR_ATTP(1); break;
+            case 2: SBVR_ATTP(2); break;
+            case 4: SBVR_ATTP(4); break;
+            default: SBVR_ATTP(8); break;
         }
-#undef SBVR_ATTB
+#undef SBVR_ATTP
         return SBVR_OK;
     }
 #define SBVR_ATT(RR)                                                                                              \
