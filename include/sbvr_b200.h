@@ -102,7 +102,7 @@ SBVR_API int sbvr_decode_f16(const uint32_t* bvr, const void* coeff_idx, int idx
  *       memory), bvr / coeff_idx / coeff / x 16-byte aligned; needs a workspace: status word, activation digits,
  *       partial sums);
  *   3 = tcgen05 fp16 GEMM with in-kernel dequantisation for batches and prefill (S in {2,3,4}, any M,
- *       N a multiple of 128; needs a workspace of sbvr_workspace_bytes(...));
+ *       any N; needs a workspace of sbvr_workspace_bytes(...));
  *   4 = tcgen05 FP4 tensor-core kernel for small batches (2 <= M <= 32, at most 16 for G = 128; S, G, N and alignment as
  *       for algo 2, K a multiple of 256 and at most 32768; the activations are quantised by a small kernel in front;
  *       needs a workspace of sbvr_workspace_bytes(...)).  Never picked by algo 0 (see the note at the dispatch in

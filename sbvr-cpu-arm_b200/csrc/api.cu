@@ -198,24 +198,36 @@ int sbvr_decode_f16(const uint32_t* bvr, const void* coeff_idx, int idx_bytes, c
     return launch_decode(w, reinterpret_cast<__half*>(W), ldw, K_out, reinterpret_cast<cudaStream_t>(stream));
 }
 
-int sbvr_linear_f16(const void* x, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff, int C,
-                    const void* bias, void* y, int M, int N, int K, int S, int G, int algo, sbvr_workspace_t* ws,
-                    sbvr_stream_t stream) {
+// Rows of Kin <= K elements; see sbvr_linear_padded_f16.
+static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff, int C,
+                      const void* bias, void* y, int M, int N, int K, int S, int G, int algo, const sbvr_workspace* ws,
+                      sbvr_stream_t stream) {
     PackedW w;
     int rc = make_packed(&w, bvr, coeff_idx, idx_bytes, coeff, C, N, K, S, G);
     if (rc) return rc;
-    if (!x || !y || M < 1) return SBVR_ERR_BAD_ARG;
-    if ((reinterpret_cast<uintptr_t>(x) & 3) || (reinterpret_cast<uintptr_t>(y) & 1)) return SBVR_ERR_ALIGN;
+    if (!x || !y || M < 1 || Kin < 1 || Kin > K) return SBVR_ERR_BAD_ARG;
+    if ((reinterpret_cast<uintptr_t>(x) & (Kin == K ? 3 : 1)) || (reinterpret_cast<uintptr_t>(y) & 1)) return SBVR_ERR_ALIGN;
     if (algo < 0 || algo > 4) return SBVR_ERR_BAD_ARG;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const __half* xh = reinterpret_cast<const __half*>(x);
     const __half* bh = reinterpret_cast<const __half*>(bias);
     __half* yh = reinterpret_cast<__half*>(y);
+    // padded rows, where a kernel needs them, live at the end of the workspace, away from the kernels' scratch
+    sbvr_workspace shrunk;
+    size_t padded = 0;
+    if (Kin != K) {
+        if (!ws) return SBVR_ERR_WORKSPACE;
+        padded = ((size_t)M * K * 2 + 255) / 256 * 256;
+        if (padded > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
+        shrunk = *ws;
+        shrunk.dyn_bytes = (ws->dyn_bytes - padded) / 256 * 256;
+        ws = &shrunk;
+    }
     if (algo == 0) {
         DeviceInfo di;
         algo = 1;
         if (ws && device_info(ws->device, &di) == SBVR_OK && di.cc_major == 10) {
-            if (linear_tcs_supported(w, M) && !(reinterpret_cast<uintptr_t>(x) & 15) &&
+            if (linear_tcs_supported(w, M) && (Kin != K || !(reinterpret_cast<uintptr_t>(x) & 15)) &&
                 linear_tcs_workspace_bytes(w, M, di.sm_count) <= ws->dyn_bytes) algo = 2;
             // The small-batch FP4 kernel (algo 4) is measured faster than the GEMM for up to 16 rows on large weights (26.3
             // against 34.3 us at 14336 x 4096, M = 16), but is not picked automatically: in the 70B batch-16 decode of the
@@ -228,15 +240,25 @@ int sbvr_linear_f16(const void* x, const uint32_t* bvr, const void* coeff_idx, i
             else if (auto_small_batch() && M <= 16 && linear_tcb_supported(w, M) &&
                      (size_t)(w.N / (w.S == 2 ? 64 : 32) / 3) * (size_t)(w.K / 256) >= (size_t)8 * di.sm_count &&
                      linear_tcb_workspace_bytes(w, M, di.sm_count) <= ws->dyn_bytes) algo = 4;
+            // A small problem is done by the SIMT kernel's one launch before the GEMM's second has started: measured 2.8 against
+            // 5.7 us at 64 x 128 (M = 1), 5.2 against 9.8 at 300 x 512 (M = 8), 7.0 against 8.2 at 3000 x 1024 (M = 4), but 22
+            // against 12 at 3000 x 3072.  Its time is that of K x (blocks of four rows) as long as all blocks run at once.
+            else if ((long long)K * ((M + 3) / 4) <= 1024 && (long long)((N + 31) / 32) * ((M + 3) / 4) <= 4LL * di.sm_count) algo = 1;
             else if (linear_gemm_supported(w, M) &&
                      linear_gemm_workspace_bytes(w, M, di.sm_count) <= ws->dyn_bytes) algo = 3;
         }
+    }
+    if (Kin != K && algo != 3) {                   // the GEMM pads while it re-tiles
+        __half* xd = reinterpret_cast<__half*>(ws->dyn + ws->dyn_bytes);
+        rc = launch_pad_rows(xh, xd, M, Kin, K, st);
+        if (rc) return rc;
+        xh = xd;
     }
     if (algo == 2) {
         if (!ws) return SBVR_ERR_WORKSPACE;
         return launch_linear_tcs(xh, w, bh, yh, M, ws->device, ws->status, ws->xchg, ws->dyn, ws->dyn_bytes, st);
     }
-    if (algo == 3) return launch_linear_gemm(xh, w, bh, yh, M, ws, st);
+    if (algo == 3) return launch_linear_gemm(xh, Kin, w, bh, yh, M, ws, st);
     if (algo == 4) {
         if (!ws) return SBVR_ERR_WORKSPACE;
         return launch_linear_tcb(xh, w, bh, yh, M, ws->device, ws->status, ws->xchg, ws->dyn, ws->dyn_bytes, st);
@@ -244,23 +266,16 @@ int sbvr_linear_f16(const void* x, const uint32_t* bvr, const void* coeff_idx, i
     return launch_linear_simt(xh, w, bh, yh, M, st);
 }
 
+int sbvr_linear_f16(const void* x, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff, int C,
+                    const void* bias, void* y, int M, int N, int K, int S, int G, int algo, sbvr_workspace_t* ws,
+                    sbvr_stream_t stream) {
+    return linear_any(x, K, bvr, coeff_idx, idx_bytes, coeff, C, bias, y, M, N, K, S, G, algo, ws, stream);
+}
+
 int sbvr_linear_padded_f16(const void* x, int K_in, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff,
                            int C, const void* bias, void* y, int M, int N, int K, int S, int G, int algo, sbvr_workspace_t* ws,
                            sbvr_stream_t stream) {
-    if (K_in == K)
-        return sbvr_linear_f16(x, bvr, coeff_idx, idx_bytes, coeff, C, bias, y, M, N, K, S, G, algo, ws, stream);
-    if (!x || M < 1 || K_in < 1 || K_in > K) return SBVR_ERR_BAD_ARG;
-    if (reinterpret_cast<uintptr_t>(x) & 1) return SBVR_ERR_ALIGN;
-    if (!ws) return SBVR_ERR_WORKSPACE;
-    // the padded rows live at the end of the workspace, away from the kernels' scratch
-    const size_t xb = ((size_t)M * K * 2 + 255) / 256 * 256;
-    if (xb > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
-    sbvr_workspace shrunk = *ws;
-    shrunk.dyn_bytes = (ws->dyn_bytes - xb) / 256 * 256;
-    __half* xd = reinterpret_cast<__half*>(ws->dyn + shrunk.dyn_bytes);
-    const int rc = launch_pad_rows(reinterpret_cast<const __half*>(x), xd, M, K_in, K, reinterpret_cast<cudaStream_t>(stream));
-    if (rc) return rc;
-    return sbvr_linear_f16(xd, bvr, coeff_idx, idx_bytes, coeff, C, bias, y, M, N, K, S, G, algo, &shrunk, stream);
+    return linear_any(x, K_in, bvr, coeff_idx, idx_bytes, coeff, C, bias, y, M, N, K, S, G, algo, ws, stream);
 }
 
 int sbvr_linear_fused_f16(int x_op, const void* x, const void* delta, const void* norm_weight, void* h_out, float eps,

@@ -149,8 +149,9 @@ int launch_linear_tcb(const __half* x, const PackedW& w, const __half* bias, __h
                       unsigned int* status, unsigned long long* xchg, char* scratch, size_t scratch_bytes, cudaStream_t st);
 bool linear_gemm_supported(const PackedW& w, int M);
 size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count);
-int launch_linear_gemm(const __half* x, const PackedW& w, const __half* bias, __half* y, int M,
-                       sbvr_workspace* ws, cudaStream_t st);
+// x rows of Kin <= K elements (row pitch Kin), as if padded with zeros to K
+int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half* bias, __half* y, int M,
+                       const sbvr_workspace* ws, cudaStream_t st);
 
 // ---------------------------------------------------------------------------------------------
 // device side

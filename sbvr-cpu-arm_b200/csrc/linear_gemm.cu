@@ -109,36 +109,106 @@ __device__ __forceinline__ void gm_ld32(uint32_t taddr, float (&d)[32]) {
 // ---------------------------------------------------------------------------------------------
 // activations -> blocked, K-permuted layout
 // ---------------------------------------------------------------------------------------------
-// One thread per 16-byte chunk: chunk (mt, kst, rg, kc, rr) holds row mt*NX + rg*8 + rr, positions kc*8 .. kc*8+7
-// of 64-k stage kst; position p of a stage is k = 64 kst + 32 (p / 32) + (p % 32) / 2 + 16 (p & 1).
-__global__ void gemm_retile_x_kernel(const __half* __restrict__ x, __half* __restrict__ xt, int M, int K, int NX,
-                                     int MT) {
+// Position p of a 64-k stage is k = 64 kst + 32 (p / 32) + (p % 32) / 2 + 16 (p & 1): eight elements and the eight sixteen
+// further on interleave into two 16-byte chunks.  One thread makes such a pair from two 16-byte loads; the 32 lanes of a
+// warp are 8 rows x the 4 pairs of a stage, so that a warp reads whole 128-byte row segments and writes one whole 1 KB
+// core-matrix block [kc (8)][row (8)][16 B].  (One chunk per thread, gathered with eight 2-byte loads, took 32 us at
+// 2048 x 4096.)  Rows of Kin <= K elements are padded with zeros; rows that cannot be read in 16-byte pieces element by element.
+__global__ void __launch_bounds__(256) gemm_retile_x_kernel(const __half* __restrict__ x, __half* __restrict__ xt, int M, int Kin,
+                                                            int K, int NX, int MT) {
     pdl_launch_dependents();
     pdl_wait();
-    const int KST = K / 64;
-    const size_t chunks = (size_t)MT * KST * NX * 8;
-    for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < chunks; c += (size_t)gridDim.x * blockDim.x) {
-        const int rr = (int)(c & 7), kc = (int)((c >> 3) & 7);
-        size_t rest = c >> 6;
-        const int rg = (int)(rest % (NX / 8));
-        rest /= (NX / 8);
+    const int KST = K / 64, RG = NX / 8;
+    const int lane = threadIdx.x & 31, rr = lane & 7, pr = lane >> 3;     // row of the group; pair: k offset 32 (pr / 2) + 8 (pr % 2)
+    const size_t blocks = (size_t)MT * KST * RG;                          // 1 KB blocks, in the order they lie in xt
+    const bool vec = (Kin % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
+    const int koff = 32 * (pr >> 1) + 8 * (pr & 1);
+    for (size_t b = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); b < blocks; b += (size_t)gridDim.x * 8) {
+        const int rg = (int)(b % RG);
+        const size_t rest = b / RG;
         const int kst = (int)(rest % KST), mt = (int)(rest / KST);
         const int m = mt * NX + rg * 8 + rr;
-        __align__(16) __half v[8];
+        const int k = kst * 64 + koff;
+        uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+        if (m < M) {
+            const __half* row = x + (size_t)m * Kin;
+            if (vec) {
+                if (k < Kin) lo = __ldg(reinterpret_cast<const uint4*>(row + k));
+                if (k + 16 < Kin) hi = __ldg(reinterpret_cast<const uint4*>(row + k + 16));
+            } else {
+                __align__(16) __half a[8], c[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int p = kc * 8 + e;
-            const int k = kst * 64 + (p & 32) + ((p & 31) >> 1) + 16 * (p & 1);
-            v[e] = (m < M) ? x[(size_t)m * K + k] : __float2half(0.0f);
+                for (int e = 0; e < 8; ++e) {
+                    a[e] = (k + e < Kin) ? row[k + e] : __float2half(0.0f);
+                    c[e] = (k + 16 + e < Kin) ? row[k + 16 + e] : __float2half(0.0f);
+                }
+                lo = *reinterpret_cast<const uint4*>(a), hi = *reinterpret_cast<const uint4*>(c);
+            }
         }
-        *reinterpret_cast<uint4*>(xt + c * 8) = *reinterpret_cast<const uint4*>(v);
+        uint4* dst = reinterpret_cast<uint4*>(xt) + b * 64 + (size_t)(2 * pr) * 8 + rr;
+        dst[0] = make_uint4(__byte_perm(lo.x, hi.x, 0x5410), __byte_perm(lo.x, hi.x, 0x7632), __byte_perm(lo.y, hi.y, 0x5410),
+                            __byte_perm(lo.y, hi.y, 0x7632));
+        dst[8] = make_uint4(__byte_perm(lo.z, hi.z, 0x5410), __byte_perm(lo.z, hi.z, 0x7632), __byte_perm(lo.w, hi.w, 0x5410),
+                            __byte_perm(lo.w, hi.w, 0x7632));
     }
 }
 
 // ---------------------------------------------------------------------------------------------
 // the GEMM
 // ---------------------------------------------------------------------------------------------
-template <int S, int NX>
+// Split K: the sum of the KS parts of one output tile (rows activation rows x cols weight rows, row pitch N), in part order.
+// A thread takes four neighbouring weight rows of four activation rows, all of a part's loads in flight together: one element
+// and one part at a time was a chain of 64 x KS L2 round trips (71 -> 38 us at 512 x 4096 x 4096).
+static __device__ __forceinline__ void gm_add_parts(const float* part, size_t plane, int KS, int rows, int cols, int N,
+                                                 const __half* bias, __half* y, int tid) {
+    constexpr int W = GM_DTHREADS / 32;
+    const int c = (tid & 31) * 4;
+    if (c >= cols) return;
+    const bool quad = (N % 4 == 0) && c + 4 <= cols;
+    float b[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = (bias && c + j < cols) ? __half2float(bias[c + j]) : 0.0f;
+    for (int m = tid >> 5; m < rows; m += 4 * W) {
+        float v[4][4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[u][j] = 0.0f;
+        for (int q = 0; q < KS; ++q) {
+            const float* src = part + (size_t)q * plane + c;
+            float t[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int mu = m + u * W;
+                const float* s = src + (size_t)mu * N;
+                if (mu < rows && quad) {
+                    const float4 f = __ldcg(reinterpret_cast<const float4*>(s));
+                    t[u][0] = f.x, t[u][1] = f.y, t[u][2] = f.z, t[u][3] = f.w;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) t[u][j] = (mu < rows && c + j < cols) ? __ldcg(s + j) : 0.0f;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[u][j] += t[u][j];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int mu = m + u * W;
+            if (mu >= rows) break;
+            __half* dst = y + (size_t)mu * N + c;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (c + j < cols) dst[j] = __float2half_rn(v[u][j] + b[j]);
+        }
+    }
+}
+
+// SPLIT: K is split over several CTAs (p.KS > 1).  A kernel of its own: its CTAs have one work item each (gm_plan), so that the
+// epilogue, which needs the registers of the decoding loop, comes behind that loop and not inside it.
+template <int S, int NX, bool SPLIT>
 __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NX >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -289,7 +359,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
         };
         auto set_item = [&](Pos& q) {              // the divisions happen once per work item, not per stage
             q.kst0 = (q.item % p.KS) * SPP;
-            q.n = (q.item / (p.KS * p.MT)) * 128 + r;
+            q.n = min((q.item / (p.KS * p.MT)) * 128 + r, p.N - 1);      // rows past the last one repeat it and are dropped
         };
         auto advance = [&](Pos& q, int by) {
             q.ks += by;
@@ -335,27 +405,29 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
             const int m0 = mt * NX;
             if (!dead) {
                 gm_fence_after();
-                const float bias = (p.bias && p.KS == 1) ? __half2float(p.bias[n]) : 0.0f;
+                const bool on = n < N;
+                const float bias = (p.bias && !SPLIT && on) ? __half2float(p.bias[n]) : 0.0f;
                 for (int c = wg; c < NX / 32; c += GM_DWGS) {
                     float d[32];
                     gm_ld32(tbase + lane_sel + c * 32, d);
-                    if (p.KS == 1) {
+                    if constexpr (!SPLIT) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
                             const int m = m0 + c * 32 + i;
-                            if (m < p.M) p.y[(size_t)m * N + n] = __float2half_rn(d[i] + bias);
+                            if (on && m < p.M) p.y[(size_t)m * N + n] = __float2half_rn(d[i] + bias);
                         }
                     } else {
                         float* dst = p.part + ((size_t)kp * p.MT * NX + m0 + c * 32) * N + n;
 #pragma unroll
-                        for (int i = 0; i < 32; ++i) dst[(size_t)i * N] = d[i];
+                        for (int i = 0; i < 32; ++i)
+                            if (on) dst[(size_t)i * N] = d[i];
                     }
                 }
                 gm_fence_before();
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(d_empty);
-            if (p.KS > 1) {
+            if constexpr (SPLIT) {
                 // split K: the CTA that delivers the last part adds all parts in part order
                 __threadfence();
                 named_bar_sync(1, GM_DTHREADS);
@@ -371,17 +443,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                 named_bar_sync(1, GM_DTHREADS);                // everyone has read the flag before it is rewritten
                 if (last) {
                     __threadfence();
-                    const size_t plane = (size_t)p.MT * NX * N;
-                    for (int e = dtid; e < NX * 128; e += GM_DTHREADS) {
-                        const int mm = e >> 7, nn = e & 127;
-                        const int m = m0 + mm;
-                        if (m >= p.M) continue;
-                        const size_t o = (size_t)m * N + nt * 128 + nn;
-                        float v = 0.0f;
-                        for (int q = 0; q < p.KS; ++q) v += __ldcg(p.part + (size_t)q * plane + o);
-                        if (p.bias) v += __half2float(p.bias[nt * 128 + nn]);
-                        p.y[o] = __float2half_rn(v);
-                    }
+                    gm_add_parts(p.part + (size_t)m0 * N + nt * 128, (size_t)p.MT * NX * N, p.KS, min(NX, p.M - m0), min(128, N - nt * 128),
+                                 N, p.bias ? p.bias + nt * 128 : nullptr, p.y + (size_t)m0 * N + nt * 128, dtid);
                 }
             }
             ep_item += grid;
@@ -424,7 +487,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
         uint32_t l_nn = line_of(nn);
 
         auto decode_stage = [&](const Pos& q, const uint32_t (&w)[2][S], const unsigned short (&c)[S]) {
-            while (ep_item < q.item) epilogue();   // items whose stages have all been handed to the issuer
+            if constexpr (!SPLIT)                  // (a CTA of a split problem has one item)
+                while (ep_item < q.item) epilogue();   // items whose stages have all been handed to the issuer
             // A lone bit at position 10 .. 14 of a half is the number 2^-14, 2^-13, 2^-11, 2^-7, 2^1: masking a packed
             // word with 0x04000400 << i leaves (bit, bit + 16) as such a half2, and one HFMA2 with c_s divided by that
             // number adds c_s where the bit is set.  Three shifted copies of the word bring all 16 bit pairs into the
@@ -562,7 +626,7 @@ bool linear_gemm_supported(const PackedW& w, int M) {
     if (w.S < 2 || w.S > 4) return false;
     if (w.G != 256 && w.G != 128) return false;
     if (M < 1) return false;
-    if (w.N % 128 || w.K % 64) return false;
+    if (w.K % 64) return false;
     if (w.idx_bytes < 0 || w.idx_bytes > 2) return false;
     if (w.S != 3 && (reinterpret_cast<uintptr_t>(w.bvr) & (w.S * 4 - 1))) return false;   // vector loads of a row's planes
     return true;
@@ -571,7 +635,7 @@ bool linear_gemm_supported(const PackedW& w, int M) {
 static void gm_plan(const PackedW& w, int M, int sm_count, GmPlan* pl) {
     pl->NX = gm_nx(M);
     pl->MT = (M + pl->NX - 1) / pl->NX;
-    pl->NT = w.N / 128;
+    pl->NT = (w.N + 127) / 128;
     const int KST = w.K / 64;
     int ks = 1;
     const int tiles = pl->NT * pl->MT;
@@ -598,13 +662,17 @@ size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count) {
     return pl.xt_bytes + pl.part_bytes;
 }
 
+template <int S, int NX, bool SPLIT>
+static int gm_launch_split(const GmParams& p, int grid, int smem, cudaStream_t st) {
+    static SmemOnce once;
+    const int rc = set_max_smem_once(once, linear_gemm_kernel<S, NX, SPLIT>, 227 * 1024);
+    if (rc) return rc;
+    SBVR_CUDA_TRY(launch_pdl(linear_gemm_kernel<S, NX, SPLIT>, dim3(grid), dim3(GM_THREADS), (size_t)smem, st, p));
+    return SBVR_OK;
+}
 template <int S, int NX>
 static int gm_launch_inst(const GmParams& p, int grid, int smem, cudaStream_t st) {
-    static SmemOnce once;
-    const int rc = set_max_smem_once(once, linear_gemm_kernel<S, NX>, 227 * 1024);
-    if (rc) return rc;
-    SBVR_CUDA_TRY(launch_pdl(linear_gemm_kernel<S, NX>, dim3(grid), dim3(GM_THREADS), (size_t)smem, st, p));
-    return SBVR_OK;
+    return p.KS > 1 ? gm_launch_split<S, NX, true>(p, grid, smem, st) : gm_launch_split<S, NX, false>(p, grid, smem, st);
 }
 template <int S>
 static int gm_launch_nx(const GmParams& p, int NX, int grid, int smem, cudaStream_t st) {
@@ -616,7 +684,7 @@ static int gm_launch_nx(const GmParams& p, int NX, int grid, int smem, cudaStrea
     }
 }
 
-int launch_linear_gemm(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, sbvr_workspace* ws,
+int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half* bias, __half* y, int M, const sbvr_workspace* ws,
                        cudaStream_t st) {
     if (!linear_gemm_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
     if (!ws) return SBVR_ERR_WORKSPACE;
@@ -629,10 +697,9 @@ int launch_linear_gemm(const __half* x, const PackedW& w, const __half* bias, __
     if (pl.xt_bytes + pl.part_bytes > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
     __half* xt = reinterpret_cast<__half*>(ws->dyn);
     {
-        const size_t chunks = (size_t)pl.MT * pl.NX * w.K / 8;
-        const int blocks = (int)((chunks + 255) / 256 < (size_t)di.sm_count * 8 ? (chunks + 255) / 256
-                                                                               : (size_t)di.sm_count * 8);
-        SBVR_CUDA_TRY(launch_pdl(gemm_retile_x_kernel, dim3(blocks), dim3(256), 0, st, x, xt, M, w.K, pl.NX, pl.MT));
+        const size_t nblk = ((size_t)pl.MT * pl.NX / 8 * (w.K / 64) + 7) / 8;
+        const int blocks = (int)(nblk < (size_t)di.sm_count * 16 ? nblk : (size_t)di.sm_count * 16);
+        SBVR_CUDA_TRY(launch_pdl(gemm_retile_x_kernel, dim3(blocks), dim3(256), 0, st, x, xt, M, Kin, w.K, pl.NX, pl.MT));
     }
     GmParams p;
     p.xt = xt, p.bvr = w.bvr, p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y;

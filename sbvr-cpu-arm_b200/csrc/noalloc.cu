@@ -116,8 +116,8 @@ extern "C" int sbvr_linear_f16_noalloc(const void* x, const uint32_t* bvr, const
         kind = 1;
         need = linear_tcs_workspace_bytes(w, M, di.sm_count);       // activation digits + partial sums of shared row tiles
     } else if (di.cc_major == 10 && linear_gemm_supported(w, M)) {
-        kind = 2;
         need = linear_gemm_workspace_bytes(w, M, di.sm_count);      // re-tiled activations + fp32 parts of a split K
+        if (need <= ws.dyn_bytes || N % 128 == 0) kind = 2;         // ragged rows that do not fit: the SIMT kernel
     }
     if (kind == 0) return launch_linear_simt(xh, w, bh, yh, M, st);
     if (need > ws.dyn_bytes) return SBVR_ERR_NOALLOC_LIMIT;         // nothing has been launched
@@ -126,7 +126,7 @@ extern "C" int sbvr_linear_f16_noalloc(const void* x, const uint32_t* bvr, const
     if (kind == 1)
         rc = launch_linear_tcs(xh, w, bh, yh, M, dev, ws.status, ws.xchg, ws.dyn, ws.dyn_bytes, st);
     else
-        rc = launch_linear_gemm(xh, w, bh, yh, M, &ws, st);
+        rc = launch_linear_gemm(xh, K, w, bh, yh, M, &ws, st);
     if (rc == SBVR_ERR_WORKSPACE) return SBVR_ERR_NOALLOC_LIMIT;
     return rc;
 }

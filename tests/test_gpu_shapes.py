@@ -1,0 +1,71 @@
+"""Sizes at the edges of the kernels' tiles, through the package API, against the oracle.
+
+Tolerance of the linears: max|y - ref| / max|ref| <= 2e-3 (one fp16 rounding of the result, 2^-11, and weights formed in
+fp16 with one rounding per plane, about 2^-11 each: measured near 6e-4)."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import sbvr_oracle as O
+from test_gpu_parity import check_status, h2n, to_sbvr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M", [1, 3, 5, 37, 130])
+@pytest.mark.parametrize("N", [40, 128, 129, 1000])
+@pytest.mark.parametrize("K", [120, 256, 1000])
+@pytest.mark.parametrize("S,mode", [(2, "u8"), (3, "u8"), (4, "u16"), (4, "direct")])
+def test_linear_any_rows_any_inner_length(M, N, K, S, mode):
+    import sbvr
+    Kp = -(-K // 256) * 256
+    p = O.make_packed(N, Kp, S, G=256, mode=mode, C=256 if mode == "u8" else 1000, seed=N + K + S)
+    w = to_sbvr(p)
+    w.original_data_shape = torch.Size((N, K))
+    rng = np.random.default_rng(M)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    bias = rng.standard_normal(N).astype(np.float16)
+    y = h2n(sbvr.linear(torch.from_numpy(x).cuda(), w, torch.from_numpy(bias).cuda()))
+    xp = np.zeros((M, Kp), np.float16)
+    xp[:, :K] = x
+    ref = O.linear_c(xp, p["bvr"], p.get("coeff_idx"), p["coeff"], G=256).astype(np.float64) + bias
+    assert y.shape == (M, N)
+    assert np.abs(y - ref).max() / np.abs(ref).max() <= 2e-3
+    check_status()
+
+
+@pytest.mark.parametrize("N,K", [(1, 256), (31, 250), (33, 8), (64, 1000), (40, 777)])
+@pytest.mark.parametrize("S", [1, 3, 4, 6])
+def test_decode_ragged_bit_exact(N, K, S):
+    Kp = -(-K // 256) * 256
+    p = O.make_packed(N, Kp, S, G=256, mode="u8", C=200, seed=N + K)
+    w = to_sbvr(p)
+    w.original_data_shape = torch.Size((N, K))
+    ref = O.decode_c(p["bvr"], p["coeff_idx"], p["coeff"], G=256)[:, :K]
+    assert np.array_equal(h2n(w.decode()).view(np.uint16), np.ascontiguousarray(ref).view(np.uint16))
+
+
+@pytest.mark.parametrize("tps", [8, 31, 64, 65, 200])
+@pytest.mark.parametrize("nh,nkv", [(2, 2), (4, 2), (8, 2), (16, 2)])
+def test_prefill_attention_against_softmax(tps, nh, nkv):
+    """Query heads per KV head 1, 2, 4, 8; the tokens continue a context that is already in the cache; the last positions fall
+    beyond the cache (they attend to all of it).  fp32 scores and weights, one fp16 rounding (2^-11) of the result."""
+    from sbvr import _lib
+    d, B, mc, start = 128, 2, 150, 7
+    g = torch.Generator(device="cuda").manual_seed(tps + nh)
+    T = B * tps
+    qkv = torch.randn((T, (nh + 2 * nkv) * d), device="cuda", generator=g).half()
+    K = torch.randn((B, nkv, mc, d), device="cuda", generator=g).half()
+    V = torch.randn((B, nkv, mc, d), device="cuda", generator=g).half()
+    pos = (torch.arange(tps, device="cuda", dtype=torch.int32) + start).repeat(B)
+    out = torch.full((T, nh * d), float("nan"), dtype=torch.float16, device="cuda")
+    _lib.check(_lib.lib.sbvr_attention_f16(qkv.data_ptr(), K.data_ptr(), V.data_ptr(), pos.data_ptr(), out.data_ptr(), None, T, tps,
+                                           nh, nkv, d, mc, d ** -0.5, 1, torch.cuda.current_stream().cuda_stream))
+    q = qkv[:, :nh * d].view(B, tps, nh, d).permute(0, 2, 1, 3).double()
+    kk = K.double().repeat_interleave(nh // nkv, 1)
+    vv = V.double().repeat_interleave(nh // nkv, 1)
+    s = q @ kk.transpose(2, 3) * d ** -0.5
+    lim = torch.clamp(pos[:tps].long() + 1, max=mc)
+    s = s.masked_fill(torch.arange(mc, device="cuda")[None, None, None, :] >= lim[None, None, :, None], float("-inf"))
+    ref = (torch.softmax(s, -1) @ vv).permute(0, 2, 1, 3).reshape(T, nh * d)
+    assert ((out.double() - ref).abs().max() / ref.abs().max()).item() < 1e-3
