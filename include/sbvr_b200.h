@@ -181,6 +181,46 @@ SBVR_API int sbvr_encode_select_f16(const void* data, int groups, const void* li
  * bit i (`_change_coeff_sel_to_bvr` and the layout change of `_encode_to_sbvr`, sbvr/core.py:842-876, :783). */
 SBVR_API int sbvr_encode_pack(const uint8_t* sel, int N, int Kp, int S, uint32_t* bvr, sbvr_stream_t stream);
 
+/* ---- the encoder's walk over the groups (reference sbvr/core.py:555-653) --------------------------------------------
+ * stats[b] = maximum, minimum, 95 % quantile and mean of group b (fp32 [groups, 4]). */
+SBVR_API int sbvr_encode_stats_f16(const void* data, int groups, float* stats, sbvr_stream_t stream);
+
+typedef struct sbvr_encode_result {     /* in host memory the device can write (pinned) */
+    int group;                          /* the next group that misses the codebook; `groups` when every group is decided */
+    int status;                         /* 0: no candidate is better than the best stored line; 1: one is, see mse and line;
+                                           2: the caller has to search this group's space himself */
+    float mse;
+    float cached_mse;                   /* the best stored line of that group (infinity and -1 in a warm-up step) */
+    int cached_at;
+    unsigned short line[4];             /* the winner, fp16 bits, in the order it was generated (not sorted) */
+    int reserved;
+} sbvr_encode_result_t;
+typedef struct sbvr_encode_walk {
+    const void* data;                   /* fp16 [groups, 256] */
+    const float* stats;                 /* of sbvr_encode_stats_f16 */
+    const void* lines;                  /* the codebook, fp16 [.., S] */
+    float* best_mse;                    /* [groups], infinity at first: best stored line of every undecided group */
+    int* best_at;                       /* [groups] */
+    void* scratch;                      /* 16 bytes of device memory */
+    sbvr_encode_result_t* result;
+    const void* unit[2];                /* plain and extended search space: fp16 [R, S] and [B] */
+    const void* bias[2];
+    int R[2], B[2], per_dim[2];
+    int S, groups, s_search_num;
+    int from;                           /* first undecided group */
+    int line0, line1;                   /* stored lines that the undecided groups have not been compared with */
+    int warm;                           /* 1: search group `from` whatever the codebook holds */
+    int search;                         /* 0: only find the next miss */
+    int misses;                         /* groups before `from` that were searched */
+    int append_at;                      /* >= 0: `append` is stored as that line of the codebook first */
+    unsigned short append[4];
+    double extend_ratio;
+    double cutoff;                      /* a group whose best mse is below it takes its best stored line */
+} sbvr_encode_walk_t;
+/* One step of the walk: compares lines [line0, line1) with the undecided groups, finds the first of them that misses and
+ * searches its own candidates.  Synchronises `stream`; the answer is in *result. */
+SBVR_API int sbvr_encode_advance(const sbvr_encode_walk_t* walk, sbvr_stream_t stream);
+
 /* ---- the kernels between the linears of a Llama decoder layer ----------------------------------------------
  * Each replaces a chain of eager PyTorch ops of the reference model (models/sbvr_llama.py) by one launch.
  * All tensors fp16, contiguous, 16-byte aligned unless noted. */

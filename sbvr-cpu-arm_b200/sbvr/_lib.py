@@ -102,10 +102,30 @@ lib.sbvr_ll_reduce_add_rmsnorm_digits_f16.restype = _i
 lib.sbvr_allreduce_add_rmsnorm_digits_f16.argtypes = [_vp, _vp, _vp, _i, _i, _i, _i, _sz, _vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp, _vp]
 lib.sbvr_allreduce_add_rmsnorm_digits_f16.restype = _i
 
-EXPORTS = ["sbvr_linear_padded_f16", "sbvr_popc_mm_f16", "sbvr_linear_t_f16", "sbvr_encode_mse_f16", "sbvr_encode_select_f16", "sbvr_encode_pack", "sbvr_rope_attention_f16", "sbvr_linear_fused_f16", "sbvr_allreduce_add_rmsnorm_f16", "sbvr_linear_push_f16", "sbvr_ll_reduce_add_rmsnorm_f16", "sbvr_ll_reduce_add_rmsnorm_digits_f16", "sbvr_allreduce_add_rmsnorm_digits_f16", "sbvr_add_rmsnorm_f16", "sbvr_rope_append_f16", "sbvr_attention_f16", "sbvr_silu_mul_f16",
+EXPORTS = ["sbvr_linear_padded_f16", "sbvr_encode_stats_f16", "sbvr_encode_advance", "sbvr_popc_mm_f16", "sbvr_linear_t_f16", "sbvr_encode_mse_f16", "sbvr_encode_select_f16", "sbvr_encode_pack", "sbvr_rope_attention_f16", "sbvr_linear_fused_f16", "sbvr_allreduce_add_rmsnorm_f16", "sbvr_linear_push_f16", "sbvr_ll_reduce_add_rmsnorm_f16", "sbvr_ll_reduce_add_rmsnorm_digits_f16", "sbvr_allreduce_add_rmsnorm_digits_f16", "sbvr_add_rmsnorm_f16", "sbvr_rope_append_f16", "sbvr_attention_f16", "sbvr_silu_mul_f16",
            "sbvr_embedding_f16", "sbvr_argmax_f16", "sbvr_linear_f16_noalloc", "sbvr_workspace_bytes", "sbvr_strerror", "sbvr_last_cuda_error", "sbvr_last_timeout_where", "sbvr_last_timeout_info", "sbvr_query", "sbvr_workspace_create",
            "sbvr_workspace_destroy", "sbvr_workspace_status", "sbvr_decode_f16", "sbvr_linear_f16",
            "sbvr_linear_f16_host"]
+
+
+class EncodeResult(ctypes.Structure):
+    """sbvr_encode_result_t of include/sbvr_b200.h."""
+    _fields_ = [("group", _i), ("status", _i), ("mse", _f), ("cached_mse", _f), ("cached_at", _i),
+                ("line", ctypes.c_ushort * 4), ("reserved", _i)]
+
+
+class EncodeWalk(ctypes.Structure):
+    """sbvr_encode_walk_t of include/sbvr_b200.h."""
+    _fields_ = [("data", _vp), ("stats", _vp), ("lines", _vp), ("best_mse", _vp), ("best_at", _vp), ("scratch", _vp),
+                ("result", _vp), ("unit", _vp * 2), ("bias", _vp * 2), ("R", _i * 2), ("B", _i * 2), ("per_dim", _i * 2),
+                ("S", _i), ("groups", _i), ("s_search_num", _i), ("from_", _i), ("line0", _i), ("line1", _i), ("warm", _i),
+                ("search", _i), ("misses", _i), ("append_at", _i), ("append", ctypes.c_ushort * 4), ("extend_ratio", ctypes.c_double), ("cutoff", ctypes.c_double)]
+
+
+lib.sbvr_encode_stats_f16.argtypes = [_vp, _i, _vp, _vp]
+lib.sbvr_encode_stats_f16.restype = _i
+lib.sbvr_encode_advance.argtypes = [ctypes.POINTER(EncodeWalk), _vp]
+lib.sbvr_encode_advance.restype = _i
 
 
 class PushDesc(ctypes.Structure):

@@ -10,23 +10,25 @@ to every candidate coefficient line as tensors.  What it decides per group is ke
     (:400-483, :368-386), takes the best candidate, and if that beats the codebook's best, stores it as a new line
     (or reuses a line within 0.01 % of it) (:605-653).
 
-How it is computed is different: the MSEs come from `sbvr_encode_mse_f16` (one thread per (group, candidate), nothing
-of size candidates x 256 x 2^S is ever stored), and the codebook look-up runs for a whole batch of groups in one launch.
-Because a group's decision depends on the codebook as its predecessors left it, the batch is speculative: the host
-replays the decisions in order, and when a group adds a line, only that one line is evaluated against the rest of the
-batch.  The result is the same as the sequential walk.
+How it is computed is different.  A step of the walk (`sbvr_encode_advance`) compares the line the last step added with
+every undecided group, finds the first group whose best stored line is not good enough, and generates and evaluates that
+group's own candidates in one kernel; the host decides from the winner alone.  Nothing of size candidates x 256 x 2^S is
+ever stored, and every group meets every line exactly once, so the result is that of the sequential walk.
 
 The search space of a group is generated with the same tensor operations and the same fp16 roundings as the
-reference's; `space_device` says where ("cpu" reproduces a reference run on CPU bit for bit, "cuda" is what the
-reference does when a GPU is present and is much faster).
+reference's; `space_device` says where: "cpu" runs the tensor operations on the CPU and reproduces a reference run there
+bit for bit; "cuda" is what the reference does when a GPU is present, with the roundings of the CUDA tensor operations
+restated in the search kernel (groups it does not cover take the operations themselves).
 """
 from __future__ import annotations
 
+import ctypes
 import itertools
 import math
 from dataclasses import dataclass, field
 from typing import List, Optional, Tuple
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -48,7 +50,7 @@ class EncoderConfig:
     acceptable_mse: float = 10 ** -12
     extend_ratio: float = 1.2
     max_cache_lines: int = 2 ** 16
-    batch_groups: int = 256            # groups looked up in the codebook per launch
+    batch_groups: int = 256            # accepted; the look-up covers all undecided groups at once
     space_device: str = "cuda"
     mse_history: List[float] = field(default_factory=list)
 
@@ -82,12 +84,16 @@ def _ratio_bias_scale_lines(r_list, b_list, s_list, S: int) -> torch.Tensor:
     return (b_list.view(-1, 1, 1, 1) + scaled.unsqueeze(0)).view(-1, S)
 
 
-def _grid_lines(data: torch.Tensor, conf: EncoderConfig, S: int, extended: bool) -> torch.Tensor:
-    """A plain grid over the data range, one axis per coefficient (`_get_additional_search_space`, sbvr/core.py:368-386)."""
+def _grid_intervals(conf: EncoderConfig, S: int, extended: bool) -> int:
     budget = conf.r_search_num * conf.b_search_num * conf.s_search_num * 1.4
     if extended:
         budget *= conf.search_extend_ratio ** 3
-    per_dim = int(budget ** (1 / S))
+    return int(budget ** (1 / S))
+
+
+def _grid_lines(data: torch.Tensor, conf: EncoderConfig, S: int, extended: bool) -> torch.Tensor:
+    """A plain grid over the data range, one axis per coefficient (`_get_additional_search_space`, sbvr/core.py:368-386)."""
+    per_dim = _grid_intervals(conf, S, extended)
     lo, hi = torch.min(data), torch.max(data)
     edges = torch.linspace(lo, hi, S + 1, device=data.device, dtype=data.dtype)
     axes = []
@@ -96,6 +102,29 @@ def _grid_lines(data: torch.Tensor, conf: EncoderConfig, S: int, extended: bool)
         axes.append(torch.linspace(edges[i] - slack, edges[i + 1] + slack, per_dim + 1, device=data.device,
                                    dtype=data.dtype))
     return torch.cartesian_prod(*axes).view(-1, S)
+
+
+def _ratio_list(conf: EncoderConfig, extended: bool, device, dtype=torch.float16) -> torch.Tensor:
+    """The ratios of neighbouring coefficients: below one, then above (sbvr/core.py:404-430)."""
+    r_lo = (math.pi / 6, 0.94)
+    r_hi = (1.06, math.pi * 2 / 3)
+    r_lo_step = (r_lo[1] - r_lo[0]) / (conf.r_search_num / 2)
+    r_hi_step = (r_hi[1] - r_hi[0]) / (conf.r_search_num / 2)
+    if extended:
+        r_lo_step /= conf.extend_ratio
+        r_hi_step /= conf.extend_ratio
+    kw = dict(device=device, dtype=dtype)
+    return torch.cat((-torch.arange(r_lo[0] + r_lo_step, r_lo[1] + r_lo_step, r_lo_step, **kw),
+                      -torch.arange(r_hi[0] + r_hi_step, r_hi[1] + r_hi_step, r_hi_step, **kw)))
+
+
+def _bias_list(conf: EncoderConfig, b_hi, extended: bool, device, dtype=torch.float16) -> torch.Tensor:
+    b_lo = -b_hi
+    b_step = (b_hi - b_lo) / conf.b_search_num
+    if extended:
+        b_step /= conf.extend_ratio
+    kw = dict(device=device, dtype=dtype)
+    return torch.arange(b_lo, b_hi, b_step, **kw) if b_step != 0 else torch.tensor([b_lo], **kw)
 
 
 def group_search_space(data: torch.Tensor, conf: EncoderConfig, extended: bool) -> torch.Tensor:
@@ -107,29 +136,19 @@ def group_search_space(data: torch.Tensor, conf: EncoderConfig, extended: bool) 
     d_max, d_avg, d_min = torch.max(data), torch.mean(data), torch.min(data)
     d_95 = torch.quantile(data.to(torch.float), 0.95)
 
-    r_lo = (math.pi / 6, 0.94)                    # ratios below one ...
-    r_hi = (1.06, math.pi * 2 / 3)                # ... and above
-    r_lo_step = (r_lo[1] - r_lo[0]) / (conf.r_search_num / 2)
-    r_hi_step = (r_hi[1] - r_hi[0]) / (conf.r_search_num / 2)
     b_hi = abs(d_avg) * 2.0 / S
     if b_hi < 0.3:
         b_hi = 0.3
-    b_lo = -b_hi
-    b_step = (b_hi - b_lo) / conf.b_search_num
     s_hi = (d_max - d_min) * 1.1
     s_lo = 2 * d_95
     s_step = (s_hi - s_lo) / conf.s_search_num
     if extended:
-        r_lo_step /= conf.extend_ratio
-        r_hi_step /= conf.extend_ratio
-        b_step /= conf.extend_ratio
         s_step /= conf.extend_ratio
 
     kw = dict(device=data.device, dtype=data.dtype)
-    r_list = torch.cat((-torch.arange(r_lo[0] + r_lo_step, r_lo[1] + r_lo_step, r_lo_step, **kw),
-                        -torch.arange(r_hi[0] + r_hi_step, r_hi[1] + r_hi_step, r_hi_step, **kw)))
+    r_list = _ratio_list(conf, extended, data.device, data.dtype)
     s_list = torch.arange(s_lo + s_step, s_hi + s_step, s_step, **kw) if s_step != 0 else torch.tensor([s_lo], **kw)
-    b_list = torch.arange(b_lo, b_hi, b_step, **kw) if b_step != 0 else torch.tensor([b_lo], **kw)
+    b_list = _bias_list(conf, b_hi, extended, data.device, data.dtype)
 
     space = _ratio_bias_scale_lines(r_list, b_list, s_list, S)
     if S <= 6:
@@ -174,42 +193,81 @@ def pack_selectors(sel: torch.Tensor, S: int) -> torch.Tensor:
 # ---------------------------------------------------------------------------------------------------------------
 class _Codebook:
     """The growing coefficient cache and the running statistics that steer the search (the mutable part of the
-    reference's `_sbvr_enc_conf`: coeff_cache, num_coeff_cache_lines, mse_history, cache_hits, group_idx)."""
+    reference's `_sbvr_enc_conf`: coeff_cache, num_coeff_cache_lines, mse_history, cache_hits, group_idx).  The lines are
+    kept on the device and mirrored here, so that a step needs no copy back."""
 
     def __init__(self, conf: EncoderConfig, device):
         self.conf = conf
         self.lines = torch.zeros((conf.max_cache_lines, conf.num_sums), dtype=torch.float16, device=device)
+        self.host = np.zeros((256, conf.num_sums), dtype=np.float16)
         self.n = 0
-        self.hits = 0
-        self.seen = 0
         self.history: List[float] = list(conf.mse_history)
+        self._cutoff: Optional[float] = None
+
+    def accept(self, mse: float) -> None:
+        self.history.append(mse)
+        self._cutoff = None
 
     def cutoff(self) -> float:
         """0.99 x the mean MSE of the most recent accepted searches, not below `acceptable_mse` (sbvr/core.py:563-568)."""
-        window = self.history[-min(len(self.history), self.conf.mse_window_size):]
-        return max((sum(window) / len(window)) * 0.99, self.conf.acceptable_mse)
+        if self._cutoff is None:
+            window = self.history[-min(len(self.history), self.conf.mse_window_size):]
+            self._cutoff = max((sum(window) / len(window)) * 0.99, self.conf.acceptable_mse)
+        return self._cutoff
 
-    def find_or_add(self, line: torch.Tensor) -> Tuple[int, bool]:
+    def find_or_add(self, line: np.ndarray) -> Tuple[int, bool]:
         """Index of a stored line within 0.01 % (summed magnitude, fp16 arithmetic) of `line`, else the index it is
-        appended at (sbvr/core.py:634-646).  Returns (index, appended)."""
+        appended at (sbvr/core.py:634-646).  Returns (index, appended); the caller stores an appended line on the device."""
         if self.n:
-            diff = self.lines[:self.n] - line.unsqueeze(0)
-            close = diff.abs().sum(-1) < line.abs().sum(-1) * 0.0001
-            if bool(close.any()):
-                return int(close.nonzero(as_tuple=True)[0][0]), False
-        self.lines[self.n] = line
+            def mag(v):                            # |v| summed over the last dimension, fp32 sum rounded to fp16
+                return np.abs(v).astype(np.float32).sum(-1).astype(np.float16)
+            near = (mag(line).astype(np.float32) * np.float32(0.0001)).astype(np.float16)
+            stored = self.host[:self.n]
+            # fp32 first: the fp16 arithmetic of numpy is slow, and almost no line is anywhere near
+            rough = np.abs(stored.astype(np.float32) - line.astype(np.float32)).sum(-1) <= 2 * float(near) + 1e-4
+            for i in np.nonzero(rough)[0]:
+                if mag(stored[i] - line) < near:
+                    return int(i), False
+        if self.n == len(self.host):
+            self.host = np.concatenate((self.host, np.zeros_like(self.host)))
+        self.host[self.n] = line
         self.n += 1
         return self.n - 1, True
 
 
-def _full_search(group: torch.Tensor, book: _Codebook, extended: bool) -> Tuple[float, int, torch.Tensor]:
-    """Best candidate of the group's own search space: (mse, index, the space [n, S] on the GPU)."""
-    conf = book.conf
+def _full_search(group: torch.Tensor, conf: EncoderConfig, extended: bool) -> Tuple[float, np.ndarray]:
+    """Best candidate of the group's own search space by tensor operations: (mse, line)."""
     src = group if conf.space_device == "cuda" else group.to(conf.space_device)
     space = group_search_space(src, conf, extended).to(group.device)
     mse = _mse(group.view(1, GROUP), space, conf.num_sums)[0]
     at = torch.argmin(mse)                                   # the first of equal minima, like the reference's argmin
-    return float(mse[at]), int(at), space
+    return float(mse[at]), space[at].cpu().numpy()
+
+
+class _SearchTables:
+    """What the candidates of all groups have in common, plain and extended: the power lines over the span of their sums and
+    the biases, made by the tensor operations of `group_search_space` (fp16 on the device), and the grid's intervals."""
+
+    def __init__(self, conf: EncoderConfig, device):
+        S = conf.num_sums
+        self.unit, self.bias, self.per_dim = [], [], []
+        for extended in (False, True):
+            r_list, b_list = _ratio_list(conf, extended, device), _bias_list(conf, 0.3, extended, device)
+            powers = r_list.unsqueeze(1) ** torch.arange(S, device=device).unsqueeze(0)
+            sums = powers @ _bin_combs(S, device, torch.float16).T
+            self.unit.append((powers / (sums.max(dim=1)[0] - sums.min(dim=1)[0]).unsqueeze(1)).contiguous())
+            self.bias.append(b_list)
+            self.per_dim.append(_grid_intervals(conf, S, extended))
+
+
+def _sorted_line(bits, S: int, device) -> np.ndarray:
+    """A candidate's coefficients in ascending magnitude; equal magnitudes in the order the device's sort leaves them in."""
+    line = np.array(bits[:S], dtype=np.uint16).view(np.float16)
+    mag = np.abs(line)
+    if len(set(mag.tolist())) == S:
+        return line[np.argsort(mag)]
+    t = torch.from_numpy(line).to(device).view(1, S)
+    return torch.gather(t, 1, torch.sort(t.abs(), dim=1)[1])[0].cpu().numpy()
 
 
 @torch.inference_mode()
@@ -227,81 +285,93 @@ def encode(data: torch.Tensor, conf: EncoderConfig, device: Optional[torch.devic
     N = flat.shape[0]
     if Kp != K:
         flat = torch.nn.functional.pad(flat, (0, Kp - K))
-    groups = flat.contiguous().view(-1, GROUP)               # group i = (row i // (Kp/256), block i % (Kp/256))
+    flat = flat.contiguous()
+    if flat.data_ptr() % 16:
+        flat = flat.clone()
+    groups = flat.view(-1, GROUP)                            # group i = (row i // (Kp/256), block i % (Kp/256))
     NG = groups.shape[0]
     with torch.cuda.device(dev):
+        st = torch.cuda.current_stream().cuda_stream
         book = _Codebook(conf, dev)
-        sel = torch.empty((NG, GROUP), dtype=torch.uint8, device=dev)
-        line_of = [0] * NG
-        one = torch.zeros(1, dtype=torch.int32, device=dev)
-
-        def select_from(space: torch.Tensor, at: int, gi: int):
-            one.fill_(at)
-            _select(groups[gi:gi + 1], space, one, S, sel[gi:gi + 1])
-
-        def search_and_store(gi: int, cached_mse: float, cached_at: int, warm: bool) -> Tuple[bool, Optional[int]]:
-            """The miss path of one group.  Returns (the stored line `cached_at` was kept, index of an appended line)."""
-            hitrate = book.hits / book.seen
-            new_mse, at, space = _full_search(groups[gi], book, hitrate > 0.6 or warm)
-            if new_mse >= cached_mse:                        # the codebook already has something at least as good
-                line_of[gi] = cached_at
-                return True, None
-            idx, appended = book.find_or_add(space[at])
-            line_of[gi] = idx
-            select_from(space, at, gi)                       # selectors of the candidate itself, also when an old line is reused
-            book.history.append(new_mse)
-            return False, (idx if appended else None)
-
+        best_mse = torch.full((NG,), float("inf"), dtype=torch.float32, device=dev)
+        line_of = torch.zeros(NG, dtype=torch.int32, device=dev)            # of undecided groups: the best stored line so far
+        scratch = torch.empty(2, dtype=torch.int64, device=dev)
+        pinned = torch.empty(ctypes.sizeof(_lib.EncodeResult), dtype=torch.uint8, pin_memory=True)
+        res = _lib.EncodeResult.from_address(pinned.data_ptr())
+        walk = _lib.EncodeWalk(data=groups.data_ptr(), lines=book.lines.data_ptr(), best_mse=best_mse.data_ptr(),
+                               best_at=line_of.data_ptr(), scratch=scratch.data_ptr(), result=pinned.data_ptr(), S=S, groups=NG,
+                               s_search_num=conf.s_search_num, extend_ratio=conf.extend_ratio, append_at=-1)
+        # one coefficient has a grid axis of 10^5 points, beyond what fp16 steps can count: tensor operations
+        kernel_search = conf.space_device == "cuda" and S > 1
+        if kernel_search:
+            tables = _SearchTables(conf, dev)
+            group_stats = torch.empty((NG, 4), dtype=torch.float32, device=dev)
+            _lib.check(_lib.lib.sbvr_encode_stats_f16(groups.data_ptr(), NG, group_stats.data_ptr(), st), "sbvr_encode_stats_f16")
+            walk.stats = group_stats.data_ptr()
+            for e in (0, 1):
+                walk.unit[e], walk.bias[e] = tables.unit[e].data_ptr(), tables.bias[e].data_ptr()
+                walk.R[e], walk.B[e] = tables.unit[e].shape[0], tables.bias[e].shape[0]
+                walk.per_dim[e] = tables.per_dim[e]
+        advance, walk_ref = _lib.lib.sbvr_encode_advance, ctypes.byref(walk)
+        own_groups, own_lines, own_index = [], [], []      # groups that keep their own candidate, it, the line it is filed under
         gi = 0
+        hits = None
         while gi < NG:
-            if book.n < conf.cache_warmup_num:               # warm-up: every group searches its own space
-                book.seen += 1
-                search_and_store(gi, float("inf"), -1, True)
-                gi += 1
-                if progress:
-                    progress(gi, NG)
-                continue
-            g1 = min(NG, gi + conf.batch_groups)
-            mse = _mse(groups[gi:g1], book.lines[:book.n], S)
-            at = torch.argmin(mse, dim=1)
-            best_mse = mse.gather(1, at.unsqueeze(1)).squeeze(1).tolist()
-            best_at = at.tolist()
-            from_book = []                                   # groups of this batch whose selectors come from a stored line
-            for b in range(g1 - gi):
-                g = gi + b
-                book.seen += 1
-                if best_mse[b] < book.cutoff():
-                    book.hits += 1
-                    line_of[g] = best_at[b]
-                    from_book.append(g)
-                    continue
-                if book.n >= conf.max_cache_lines:           # full codebook: the best stored line has to do
-                    line_of[g] = best_at[b]
-                    from_book.append(g)
-                    continue
-                kept, added = search_and_store(g, best_mse[b], best_at[b], False)
-                if kept:
-                    from_book.append(g)
-                if added is not None and g + 1 < g1:         # the rest of the batch has not seen the new line yet
-                    extra = _mse(groups[g + 1:g1], book.lines[added:added + 1], S)[:, 0].tolist()
-                    for r, m in enumerate(extra):
-                        if m < best_mse[b + 1 + r]:
-                            best_mse[b + 1 + r], best_at[b + 1 + r] = m, added
-            if from_book:
-                rows = torch.tensor(from_book, dtype=torch.long, device=dev)
-                which = torch.tensor([line_of[g] for g in from_book], dtype=torch.int32, device=dev)
-                tmp = torch.empty((len(from_book), GROUP), dtype=torch.uint8, device=dev)
-                _select(groups[rows].contiguous(), book.lines, which, S, tmp)
-                sel[rows] = tmp
-            gi = g1
+            warm = book.n < conf.cache_warmup_num          # every group searches its own space
+            full = book.n >= conf.max_cache_lines          # the best stored line has to do
+            walk.from_, walk.line1, walk.warm = gi, book.n, int(warm)
+            full = full and not warm
+            walk.search = int(kernel_search and not full)
+            walk.cutoff = 0.0 if warm else float("inf") if full else book.cutoff()
+            _lib.check(advance(walk_ref, st), "sbvr_encode_advance")
+            walk.append_at = -1
+            if not warm:
+                walk.line0 = walk.line1
+            g = res.group
+            if full:
+                hits = gi - walk.misses + int((best_mse[gi:].double() < book.cutoff()).sum())
+                break
+            if g >= NG:
+                hits = NG - walk.misses
+                break
+            if res.status == 2:
+                new_mse, line = _full_search(groups[g], conf, warm or (g - walk.misses) / (g + 1) > 0.6)
+                better = new_mse < res.cached_mse
+            elif res.status == 1:
+                new_mse, line, better = res.mse, _sorted_line(res.line, S, dev), True
+            else:
+                better = False                             # the codebook already has something at least as good
+            walk.misses += 1
+            if better:
+                at, appended = book.find_or_add(line)
+                if appended:
+                    walk.append_at = at
+                    walk.append[:S] = line.view(np.uint16).tolist()
+                own_groups.append(g)                       # selectors of the candidate itself, also when an old line is reused
+                own_lines.append(line)
+                own_index.append(at)
+                book.accept(new_mse)
+            gi = g + 1
             if progress:
                 progress(gi, NG)
+        if walk.append_at >= 0:
+            book.lines[walk.append_at] = torch.from_numpy(book.host[walk.append_at]).to(dev)
 
         C = book.n
         cache = book.lines[:C].contiguous()
-        idx = torch.tensor(line_of, dtype=torch.int32, device=dev).view(N, Kp // GROUP).T.contiguous()
+        sel = torch.empty((NG, GROUP), dtype=torch.uint8, device=dev)
+        if own_groups:
+            rows = torch.tensor(own_groups, dtype=torch.long, device=dev)
+            line_of[rows] = torch.tensor(own_index, dtype=torch.int32, device=dev)
+        _select(groups, book.lines, line_of, S, sel)
+        if own_groups:
+            tmp = torch.empty((len(own_groups), GROUP), dtype=torch.uint8, device=dev)
+            _select(groups[rows], torch.from_numpy(np.stack(own_lines)).to(dev), torch.arange(len(own_groups), dtype=torch.int32, device=dev),
+                    S, tmp)
+            sel[rows] = tmp
+        idx = line_of.view(N, Kp // GROUP).T.contiguous()
         idx = idx.to(torch.uint8) if C <= 256 else idx.to(torch.int16).view(torch.uint16)   # C <= 65536: the bits fit
         bvr = pack_selectors(sel.view(N, Kp), S)
         torch.cuda.synchronize(dev)
-    stats = {"groups": NG, "cache_lines": C, "cache_hits": book.hits, "searches": len(book.history) - len(conf.mse_history)}
+    stats = {"groups": NG, "cache_lines": C, "cache_hits": NG - walk.misses if hits is None else hits, "searches": len(book.history) - len(conf.mse_history)}
     return bvr, idx, cache, stats

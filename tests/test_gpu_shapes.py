@@ -69,3 +69,54 @@ def test_prefill_attention_against_softmax(tps, nh, nkv):
     s = s.masked_fill(torch.arange(mc, device="cuda")[None, None, None, :] >= lim[None, None, :, None], float("-inf"))
     ref = (torch.softmax(s, -1) @ vv).permute(0, 2, 1, 3).reshape(T, nh * d)
     assert ((out.double() - ref).abs().max() / ref.abs().max()).item() < 1e-3
+
+
+@pytest.mark.parametrize("S", [2, 3, 4])
+@pytest.mark.parametrize("extended", [False, True])
+def test_search_kernel_equals_the_tensor_operations(S, extended):
+    """The winner of the search kernel, which generates the candidates itself, is bit for bit that of the search space made by
+    the tensor operations: data scales over three decades, a stored line good enough to win, groups the kernel leaves to
+    its caller."""
+    from sbvr import _lib, encoder
+    import ctypes
+    conf = encoder.EncoderConfig(num_sums=S)
+    dev = torch.device("cuda")
+    g = torch.Generator(device="cuda").manual_seed(S)
+    scale = 10 ** torch.linspace(-3, -0.3, 24, device="cuda")
+    data = (torch.randn((24, 256), device="cuda", generator=g) * scale[:, None]).half()
+    data[5] = data[5].abs()
+    data[7] += 2.0
+    tables = encoder._SearchTables(conf, dev)
+    stats = torch.empty((24, 4), device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    _lib.check(_lib.lib.sbvr_encode_stats_f16(data.data_ptr(), 24, stats.data_ptr(), st))
+    assert torch.equal(stats[:, 0], data.float().amax(1)) and torch.equal(stats[:, 1], data.float().amin(1))
+    assert torch.equal(stats[:, 2], torch.quantile(data.float(), 0.95, dim=1))
+    pinned = torch.empty(ctypes.sizeof(_lib.EncodeResult), dtype=torch.uint8, pin_memory=True)
+    res = _lib.EncodeResult.from_address(pinned.data_ptr())
+    lines = torch.zeros((4, S), dtype=torch.float16, device="cuda")
+    scratch = torch.empty(2, dtype=torch.int64, device="cuda")
+    at = torch.zeros(24, dtype=torch.int32, device="cuda")
+    for i in range(24):
+        # hits / seen of the groups before decides whether the search is extended
+        mse = torch.full((24,), float("inf"), device="cuda")
+        w = _lib.EncodeWalk(data=data.data_ptr(), stats=stats.data_ptr(), lines=lines.data_ptr(), best_mse=mse.data_ptr(),
+                            best_at=at.data_ptr(), scratch=scratch.data_ptr(), result=pinned.data_ptr(), S=S, groups=24,
+                            s_search_num=conf.s_search_num, extend_ratio=conf.extend_ratio, append_at=-1, from_=i, search=1,
+                            warm=int(extended), misses=i, cutoff=0.0)
+        for e in (0, 1):
+            w.unit[e], w.bias[e] = tables.unit[e].data_ptr(), tables.bias[e].data_ptr()
+            w.R[e], w.B[e], w.per_dim[e] = tables.unit[e].shape[0], tables.bias[e].shape[0], tables.per_dim[e]
+        _lib.check(_lib.lib.sbvr_encode_advance(ctypes.byref(w), st))
+        assert res.group == i
+        if res.status == 2:                        # 7: a large mean; 5: perhaps an empty scale range (max - min below twice the quantile)
+            assert i in (5, 7)
+            continue
+        assert i != 7
+        best, line = encoder._full_search(data[i], conf, extended)
+        assert res.status == 1 and res.mse == best, (i, res.status, res.mse, best)
+        assert np.array_equal(encoder._sorted_line(res.line, S, dev).view(np.uint16), line.view(np.uint16)), i
+        # a stored line that is exactly as good keeps its place
+        mse[i] = best
+        _lib.check(_lib.lib.sbvr_encode_advance(ctypes.byref(w), st))
+        assert res.status == (1 if extended else 0)            # (a warm-up step looks at no stored line)
