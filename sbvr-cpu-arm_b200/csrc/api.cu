@@ -9,12 +9,24 @@ namespace sbvr {
 
 thread_local int g_last_cuda_error = 0;
 
-static bool auto_small_batch() {
-    static const bool on = [] {
-        const char* e = getenv("SBVR_AUTO_SMALL_BATCH");
-        return e && e[0] == '1';
-    }();
-    return on;
+int xop_check(const XOp* xop, const __half* x, int M, int K, int* op, const __half** delta, const __half** norm_w, __half** h_out,
+              float* eps) {
+    *op = xop ? xop->op : SBVR_XOP_NONE;
+    *delta = xop ? xop->delta : nullptr, *norm_w = xop ? xop->norm_w : nullptr, *h_out = xop ? xop->h_out : nullptr;
+    *eps = xop ? xop->eps : 0.0f;
+    if (*op != SBVR_XOP_ADD_RMSNORM) return SBVR_OK;
+    if (!*norm_w) return SBVR_ERR_BAD_ARG;
+    if (*h_out) {                                  // h_out is written while other blocks still read x and delta for the row's mean square
+        const uintptr_t n = (uintptr_t)M * K * 2, ho = reinterpret_cast<uintptr_t>(*h_out);
+        auto overlaps = [&](const void* q) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(q);
+            return q && ho < a + n && a < ho + n;
+        };
+        if (overlaps(x) || overlaps(*delta)) return SBVR_ERR_BAD_ARG;
+    }
+    if ((reinterpret_cast<uintptr_t>(*delta) | reinterpret_cast<uintptr_t>(*norm_w) | reinterpret_cast<uintptr_t>(*h_out)) & 15)
+        return SBVR_ERR_ALIGN;
+    return SBVR_OK;
 }
 
 bool pdl_enabled() {
@@ -148,11 +160,13 @@ int sbvr_workspace_bytes(int device, int M, int N, int K, size_t* bytes) {
     const size_t fixed = SBVR_WS_FIXED_BYTES;
     const size_t stage = (((size_t)M * K * 2 + 255) / 256 + ((size_t)M * N * 2 + 255) / 256) * 256;   // host-pointer staging
     size_t kern = linear_gemm_workspace_bytes(w, M, di.sm_count);
-    if (M >= 2 && M <= 32) {                       // the small-batch kernel's digits and partial sums (two planes: widest tiles)
-        w.S = 2;
-        const size_t tcb = linear_tcb_workspace_bytes(w, M, di.sm_count);
-        w.S = 4;
-        if (tcb > kern) kern = tcb;
+    if (M >= 2 && M <= 32 && K % 256 == 0) {       // the small-batch kernel's digits and partial sums, whatever the encoding
+        for (int s = 2; s <= 4; ++s)
+            for (int g = 128; g <= 256; g += 128) {
+                w.S = s, w.G = g;
+                const size_t sb = linear_sb_workspace_bytes(w, M, di);
+                if (sb > kern) kern = sb;
+            }
     }
     *bytes = fixed + kern + stage + ((size_t)8 << 20);
     if (*bytes < ((size_t)32 << 20)) *bytes = (size_t)32 << 20;
@@ -229,17 +243,7 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
         if (ws && device_info(ws->device, &di) == SBVR_OK && di.cc_major == 10) {
             if (linear_tcs_supported(w, M) && (Kin != K || !(reinterpret_cast<uintptr_t>(x) & 15)) &&
                 linear_tcs_workspace_bytes(w, M, di.sm_count) <= ws->dyn_bytes) algo = 2;
-            // The small-batch FP4 kernel (algo 4) is measured faster than the GEMM for up to 16 rows on large weights (26.3
-            // against 34.3 us at 14336 x 4096, M = 16), but is not picked automatically: in the 70B batch-16 decode of the
-            // benchmark one of its bounded waits ran out in three of eleven runs (compute warps waiting for a digit stage), and the
-            // cause has not been found.  (The kernel has since been given one release barrier per warpgroup and stage instead of
-            // one barrier with three arriving commits; two runs of the benchmark with the automatic choice on then passed,
-            // which against a failure rate of about one in four proves little.)  It stays available on request, and
-            // SBVR_AUTO_SMALL_BATCH=1 in the environment puts it back into this choice (for weights that give every SM at
-            // least eight steps).
-            else if (auto_small_batch() && M <= 16 && linear_tcb_supported(w, M) &&
-                     (size_t)(w.N / (w.S == 2 ? 64 : 32) / 3) * (size_t)(w.K / 256) >= (size_t)8 * di.sm_count &&
-                     linear_tcb_workspace_bytes(w, M, di.sm_count) <= ws->dyn_bytes) algo = 4;
+            else if (M <= 16 && linear_sb_supported(w, M) && linear_sb_workspace_bytes(w, M, di) <= ws->dyn_bytes) algo = 4;
             // A small problem is done by the SIMT kernel's one launch before the GEMM's second has started: measured 2.8 against
             // 5.7 us at 64 x 128 (M = 1), 5.2 against 9.8 at 300 x 512 (M = 8), 7.0 against 8.2 at 3000 x 1024 (M = 4), but 22
             // against 12 at 3000 x 3072.  Its time is that of K x (blocks of four rows) as long as all blocks run at once.
@@ -261,7 +265,7 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
     if (algo == 3) return launch_linear_gemm(xh, Kin, w, bh, yh, M, ws, st);
     if (algo == 4) {
         if (!ws) return SBVR_ERR_WORKSPACE;
-        return launch_linear_tcb(xh, w, bh, yh, M, ws->device, ws->status, ws->xchg, ws->dyn, ws->dyn_bytes, st);
+        return launch_linear_sb(xh, w, bh, yh, M, ws->device, ws->status, ws->counters, ws->dyn, ws->dyn_bytes, st);
     }
     return launch_linear_simt(xh, w, bh, yh, M, st);
 }

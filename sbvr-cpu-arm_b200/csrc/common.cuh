@@ -141,12 +141,15 @@ size_t linear_tcs_workspace_bytes(const PackedW& w, int M, int sm_count);
 int launch_linear_tcs(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, int device,
                       unsigned int* status, unsigned long long* xchg, char* scratch, size_t scratch_bytes, cudaStream_t st,
                       const XOp* xop = nullptr, const sbvr_push_desc_t* push = nullptr);
-// The small-batch kernel (linear_tcb.cu), 2 .. 32 activation rows: same scratch rules; it uses the first words of the
-// exchange region as arrival counters and leaves them zero.
-bool linear_tcb_supported(const PackedW& w, int M);
-size_t linear_tcb_workspace_bytes(const PackedW& w, int M, int sm_count);
-int launch_linear_tcb(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, int device,
-                      unsigned int* status, unsigned long long* xchg, char* scratch, size_t scratch_bytes, cudaStream_t st);
+// Validates an op in front of a linear and spreads it over the quantiser's parameters (api.cu).
+int xop_check(const XOp* xop, const __half* x, int M, int K, int* op, const __half** delta, const __half** norm_w, __half** h_out,
+              float* eps);
+// The small-batch kernel (linear_sb.cu), 2 .. 32 activation rows: status words, the workspace's arrival counters (left zero)
+// and 256-byte aligned scratch are the caller's.
+bool linear_sb_supported(const PackedW& w, int M);
+size_t linear_sb_workspace_bytes(const PackedW& w, int M, const DeviceInfo& di);
+int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, int device, unsigned int* status,
+                     unsigned int* counters, char* scratch, size_t scratch_bytes, cudaStream_t st, const XOp* xop = nullptr);
 bool linear_gemm_supported(const PackedW& w, int M);
 size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count);
 // x rows of Kin <= K elements (row pitch Kin), as if padded with zeros to K

@@ -1,0 +1,754 @@
+// SBVR linear for small activation batches (2 .. 32 rows): FP4 tensor-core dot products of plane bits with activation digits,
+// like the decode GEMV, but with the digits' weights and the activations' block step carried by the MMA's own block scale
+// factors, so that the tensor pipe sums over digits and nothing but one multiply-add per (row, plane, digit half, activation
+// row, 256-k block) is left for the CUDA cores.
+//
+//   y[m, n] = sum_g sum_s c[g, n, s] * sum_{k in g} x[m, k] * bit_s[n, k]
+//
+// Operands of tcgen05.mma kind::mxf4.block_scale.scale_vec::2X (K = 64 per instruction, fp32 accumulation in tensor memory):
+//
+//  A (tensor memory)  128 lanes = TN output rows x their planes; a lane's 256 plane bits of a k block are expanded to 4-bit
+//      E2M1 codes by six integer instructions per packed word (`(w << 1) & 0x2222.., w & 0x2222.., w & 0x4444..,
+//      (w >> 1) & 0x4444..`): a set bit becomes 1, 1, 2, 2 for k % 4 = 0 .. 3.
+//  B (shared memory)  x is quantised per (activation row, 256-k block) to 16-bit block fixed point q = round(x / step),
+//      step a power of two, and q + 0x24924 is cut into six 3-bit fields t, digit = t - 4 in {-4 .. 3}, so that
+//      q = sum_d 8^d digit_d.  Every digit is an exact E2M1 value (halved where the plane bit counts 2).  One MMA
+//      multiplies the plane bits by ONE digit of all activation rows (M > 16: N = 32 rows) or by two digits of up to
+//      16 rows (N = 2 x 16), with the scale factor 8^d * step of that digit and row as the B block scale (UE8M0, a power
+//      of two): the accumulator column of an activation row then holds sum_k bit * x^ directly, whatever the digit.
+//      M <= 16 leaves two columns per activation row (even and odd digits), added on the way out.
+//
+// Structure.  K is cut into chunks of at most eight (M > 16: four) 256-k blocks, and a CTA works on one chunk: its digits
+// (12 or 24 KB per block, written by the quantiser kernel) stay in shared memory and their scale factors in tensor memory for
+// the whole launch, so the only things that move are packed words.  Four warpgroups take (row tile, k block) units in order,
+// each on its own, with one A and one D buffer: as soon as the MMAs of unit i are done, the sums are requested, the next
+// unit's words are expanded into A while they arrive, and the MMAs of unit i + 1 are released; the multiply-adds and the
+// shared-memory loads of unit i + 2 run beside them.  A tile that several warpgroups share meets in shared memory; the chunks'
+// sums meet in scratch, where the warp that arrives last at a quarter tile's counter adds them in chunk order (the same bits
+// on every run; nobody waits for another CTA).  Every wait is bounded.
+//
+// What bounds it: a unit (4.6 KB of weight) is 12 MMAs of 17 cycles and about 220 issue slots per scheduler, against 200 cycles
+// of its SM's share of HBM; measured about 290 cycles.  The form before this one (three warpgroups in lockstep over shared
+// digit stages) spent 1 500 cycles per three units on the latency chain of a compute warp.
+//
+// Replaces the M > 1 use of `_sbvr_row_deq_mm_T` (reference sbvr/kernels/sbvr_kernel.cu:121-191) for 2 .. 32 rows.
+#include <cuda.h>
+
+#include "common.cuh"
+#include "tc_stream.cuh"
+
+namespace sbvr {
+
+constexpr int SB_NWG = 4;
+constexpr int SB_CW0 = 4;                       // warps 0 .. 3: issuers (warp 0 also sets up); compute warps behind
+constexpr int SB_THREADS = (SB_CW0 + 4 * SB_NWG) * 32;
+constexpr int SB_SF_BYTES = 512;                // 32 rows x 16 B of B scale factors (and poison marks) per k block
+constexpr int SB_ASTAGE = TS_STAGE_WORDS + 512; // packed words of a unit + its coefficient data
+constexpr int SB_MAX_STAGES = 4;
+constexpr int SB_HDR = 1024;
+__host__ __device__ constexpr int sb_blob(int NJ) { return NJ * 4096 + SB_SF_BYTES; }
+// k blocks of a CTA at most: what shared memory (digits) and, for two groups per block, tensor memory hold
+__host__ __device__ constexpr int sb_chunk(int NSUB, int NJ) { return NJ == 6 ? 4 : NSUB == 2 ? 6 : 8; }
+// Tensor memory: per warpgroup A (32 columns) and D (32 per group of a block), then the B scale factors of every k block (16
+// columns each: three 4-column blocks; an MMA's scale-factor address designates one), then unit scale factors for A
+__host__ __device__ constexpr int sb_wgcols(int NSUB) { return 32 + NSUB * 32; }
+__host__ __device__ constexpr int sb_sf_col(int NSUB) { return SB_NWG * sb_wgcols(NSUB); }
+
+struct SbParams {
+    const unsigned char* xb;      // [KB][sb_blob] written by sb_quant_kernel
+    const void* idx;
+    const __half* coeff;
+    const __half* bias;
+    __half* y;
+    unsigned int* status;
+    unsigned int* counters;       // one per (tile, part of its rows), zero between launches
+    float* part;                  // [KC][NT][MP][TN] sums of the chunks (KC > 1)
+    int M, N, K, KB, NT, C, KC, GN, cache_in_smem, stages;
+    int psh;                      // log2 of the parts of a tile that are counted separately
+    int off_cache, off_ring, off_res;
+};
+
+struct SbQuant {
+    const __half* x;
+    unsigned char* xb;
+    int M, K;
+    int x_op;
+    const __half* delta;
+    const __half* norm_w;
+    __half* h_out;
+    float eps;
+};
+
+// ---------------------------------------------------------------------------------------------
+// activations (with the op in front of the linear) -> digit blob, once per call
+// ---------------------------------------------------------------------------------------------
+// One block per 256-k block and four (padded) activation rows, one warp per row.  Lane (kw, j) owns the eight elements
+// k = 32 kw + j + 4 e, which are one 32-bit word (nibble e) of every digit: the K order in which the weight expansion
+// leaves the plane bits.  Blob of a k block: [MMA j (NJ)][row group (4)][kw (8)][row (8)][16 B], then 32 rows x 16 B:
+// words 0 .. 2 hold the scale bytes of MMA 2 i (bytes 0, 1) and 2 i + 1 (bytes 2, 3) for that B row, word 3 of row m whether
+// activation row m of this block holds a non-finite value.
+template <int NJ>
+__global__ void __launch_bounds__(128) sb_quant_kernel(const SbQuant p) {
+    __shared__ __align__(16) __half row[4][256];
+    pdl_launch_dependents();
+    pdl_wait();                                    // the activations come from the previous kernel of the stream
+    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int kb = blockIdx.x, K = p.K, M = p.M, m = blockIdx.y * 4 + wl;
+    const int kw = lane >> 2, j = lane & 3;
+    uint32_t words[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+    int ex = 14;
+    bool poison = false;
+    if (m < M) {
+        // this warp's 256 activations: lane l brings elements 8 l .. 8 l + 7
+        const size_t off = (size_t)m * K + (size_t)kb * 256 + lane * 8;
+        uint4 o;
+        __half2* oh = reinterpret_cast<__half2*>(&o);
+        if (p.x_op == SBVR_XOP_SILU_MUL) {
+            const __half* gp = p.x + (size_t)m * 2 * K + (size_t)kb * 256 + lane * 8;
+            const uint4 g = __ldg(reinterpret_cast<const uint4*>(gp));
+            const uint4 u = __ldg(reinterpret_cast<const uint4*>(gp + K));
+            const __half2* gh = reinterpret_cast<const __half2*>(&g);
+            const __half2* uh = reinterpret_cast<const __half2*>(&u);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __half22float2(gh[e]);
+                oh[e] = __hmul2(__floats2half2_rn(f.x / (1.0f + expf(-f.x)), f.y / (1.0f + expf(-f.y))), uh[e]);
+            }
+        } else if (p.x_op == SBVR_XOP_ADD_RMSNORM) {
+            // mean of (h + delta)^2 over the whole row, the sum formed in fp16 like the separate kernel does
+            float sq = 0.0f;
+#pragma unroll 4
+            for (int c = lane; c < K / 8; c += 32) {
+                uint4 a = __ldg(reinterpret_cast<const uint4*>(p.x + (size_t)m * K) + c);
+                __half2* ah = reinterpret_cast<__half2*>(&a);
+                if (p.delta) {
+                    const uint4 b = __ldg(reinterpret_cast<const uint4*>(p.delta + (size_t)m * K) + c);
+                    const __half2* bh = reinterpret_cast<const __half2*>(&b);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) ah[e] = __hadd2(ah[e], bh[e]);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 f = __half22float2(ah[e]);
+                    sq += f.x * f.x + f.y * f.y;
+                }
+            }
+#pragma unroll
+            for (int s = 16; s; s >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, s);
+            const float rs = rsqrtf(sq / (float)K + p.eps);
+            uint4 a = __ldg(reinterpret_cast<const uint4*>(p.x + off));
+            __half2* ah = reinterpret_cast<__half2*>(&a);
+            if (p.delta) {
+                const uint4 b = __ldg(reinterpret_cast<const uint4*>(p.delta + off));
+                const __half2* bh = reinterpret_cast<const __half2*>(&b);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) ah[e] = __hadd2(ah[e], bh[e]);
+            }
+            if (p.h_out) *reinterpret_cast<uint4*>(p.h_out + off) = a;
+            const uint4 wv = __ldg(reinterpret_cast<const uint4*>(p.norm_w + (size_t)kb * 256 + lane * 8));
+            const __half2* wh = reinterpret_cast<const __half2*>(&wv);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float2 f = __half22float2(ah[e]);
+                oh[e] = __hmul2(wh[e], __floats2half2_rn(f.x * rs, f.y * rs));
+            }
+        } else if ((reinterpret_cast<uintptr_t>(p.x) & 15) == 0) {
+            o = __ldg(reinterpret_cast<const uint4*>(p.x + off));
+        } else {
+            __half* e = reinterpret_cast<__half*>(&o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) e[i] = p.x[off + i];
+        }
+        reinterpret_cast<uint4*>(row[wl])[lane] = o;
+        __syncwarp();
+        const __half* xp = row[wl] + 32 * kw + j;
+        float v[8];
+        float a = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            v[e] = __half2float(xp[4 * e]);
+            float av = fabsf(v[e]);
+            if (!(av == av)) av = __int_as_float(0x7f800000);     // NaN counts as infinity
+            a = fmaxf(a, av);
+        }
+#pragma unroll
+        for (int s = 16; s; s >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, s));
+        float inv = 0.0f;
+        if (a >= __int_as_float(0x7f800000)) {
+            poison = true;
+        } else if (a > 0.0f) {
+            ex = (int)((__float_as_uint(a) >> 23) & 0xFF) - 127;              // a = 1.f * 2^ex, ex in [-24, 15]
+            inv = __uint_as_float((uint32_t)(14 - ex + 127) << 23);
+        }
+        // E2M1 codes of digit t - 4 (t = 0 .. 7), one nibble each: the value itself for j = 0, 1, half of it for j = 2, 3
+        const uint32_t lut = (j < 2) ? 0x5420ACDEu : 0x32109ABCu;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const int q = poison ? 0 : __float2int_rn(v[e] * inv);            // |q| <= 2^15
+            const uint32_t u = (uint32_t)(q + 0x24924);
+#pragma unroll
+            for (int d = 0; d < 6; ++d) {
+                const uint32_t t = (u >> (3 * d)) & 7u;
+                words[d] |= ((lut >> (4u * t)) & 0xFu) << (4 * e);
+            }
+        }
+    }
+    unsigned char* blob = p.xb + (size_t)kb * sb_blob(NJ);
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+        const int jm = (NJ == 6) ? d : (d >> 1);
+        const int r = (NJ == 6) ? m : ((d & 1) * 16 + m);
+        *reinterpret_cast<uint32_t*>(blob + jm * 4096 + (r >> 3) * 1024 + kw * 128 + (r & 7) * 16 + j * 4) = words[d];
+    }
+    // scale bytes 127 + exponent, each twice (two 32-element blocks per MMA); rows beyond M: 2^0 on zero digits
+    auto two = [&](int d) -> uint32_t { return (m < M ? (uint32_t)(127 + 3 * d + ex - 14) : 127u) * 0x0101u; };
+    uint4* sf = reinterpret_cast<uint4*>(blob + NJ * 4096);
+    const uint32_t pw = poison ? 1u : 0u;
+    if (NJ == 6) {
+        if (lane == 0) sf[m] = make_uint4(two(0) | (two(1) << 16), two(2) | (two(3) << 16), two(4) | (two(5) << 16), pw);
+    } else if (lane < 2) {                         // even digits in row m, odd ones in row 16 + m; MMA j has digits 2 j, 2 j + 1
+        sf[lane * 16 + m] = make_uint4(two(lane) | (two(2 + lane) << 16), two(4 + lane) | 0x7F7F0000u, 0x7F7F7F7Fu, pw);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// the product
+// ---------------------------------------------------------------------------------------------
+template <int S, int NSUB, int NJ, int IDXB>
+__global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_constant__ CUtensorMap tmap, const SbParams p) {
+    pdl_launch_dependents();
+    extern __shared__ __align__(1024) unsigned char smem[];
+    constexpr int SP = ts_sp(S);
+    constexpr int TN = ts_tn(S);
+    constexpr int MP = (NJ == 3) ? 16 : 32;        // activation rows the accumulators cover
+    constexpr int WGCOLS = sb_wgcols(NSUB);
+    constexpr int BLOB = sb_blob(NJ);
+    constexpr int WROW = TN * S * 4;               // bytes of one 32-k row of a stage
+    constexpr int CI_BYTES = (IDXB == 0) ? TN * S * 2 : TN * IDXB;
+    constexpr uint32_t A_TX = 8 * WROW + NSUB * CI_BYTES;
+    constexpr int SFB_COL = sb_sf_col(NSUB);
+    constexpr int SFA_COL = SFB_COL + 16 * sb_chunk(NSUB, NJ);
+    static_assert(SFA_COL + 32 <= TS_TMEM_COLS, "tensor memory");
+    // instruction descriptor: A, B = E2M1, scales UE8M0, M = 128, N = 32, K-major both; the scale-factor byte pair is added per MMA
+    constexpr uint32_t IDESC = (1u << 7) | (1u << 10) | ((uint32_t)(32 >> 3) << 17) | (1u << 23) | (8u << 24);
+
+    uint64_t* a_full = reinterpret_cast<uint64_t*>(smem);                            // [SB_NWG][SB_MAX_STAGES] unit landed
+    uint64_t* mma_bar = a_full + SB_NWG * SB_MAX_STAGES;                             // [SB_NWG] MMAs of a unit done
+    uint64_t* b_full = mma_bar + SB_NWG;                                             // [8] digits of a k block landed
+    uint64_t* sf_ready = b_full + 8;                                                 // [8] its scale factors in tensor memory
+    uint64_t* cache_bar = sf_ready + 8;                                              // [1] codebook landed
+    uint64_t* tmem_ready = cache_bar + 1;                                            // [1] tensor memory allocated
+    constexpr int SF0 = SB_NWG * (SB_MAX_STAGES + 1) + 8, NBAR = SF0 + 8 + 2;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SB_HDR - 64);
+    uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(smem + SB_HDR - 16);
+
+    const int N = p.N, M = p.M, KC = p.KC;
+    const int grp = (int)blockIdx.x / KC, chunk = (int)blockIdx.x - grp * KC;
+    const int kb0 = chunk * p.KB / KC, nkb = (chunk + 1) * p.KB / KC - kb0;
+    const int t0 = (int)((long long)grp * p.NT / p.GN), ntc = (int)((long long)(grp + 1) * p.NT / p.GN) - t0;
+    const int units = ntc * nkb;
+    unsigned char* Bs = smem + SB_HDR;                                               // [nkb][BLOB]
+    __half* cache_s = reinterpret_cast<__half*>(smem + p.off_cache);
+    unsigned char* ring = smem + p.off_ring;                                         // [SB_NWG][stages][SB_ASTAGE]
+    float* res = reinterpret_cast<float*>(smem + p.off_res);                         // [SB_NWG][2][MP][TN]: first, last shared tile
+    const int ST = p.stages;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+
+    if (threadIdx.x < NBAR) {
+        mbar_init(&a_full[threadIdx.x], ((int)threadIdx.x >= SF0 && (int)threadIdx.x < SF0 + 8) ? 4u : 1u);      // (sf_ready: four warps)
+        if (threadIdx.x == 0) *abort_flag = 0;
+        fence_mbar_init();
+    }
+    __syncthreads();
+    const bool bulk_cache = p.cache_in_smem && ((p.C * S * 2) % 16 == 0);
+
+    if (warp < SB_NWG) {
+        // ------------------------------ issuer warps, one per warpgroup ------------------------------
+        const int w = warp;
+        const int u0 = w * units / SB_NWG, n_w = (w + 1) * units / SB_NWG - u0;
+        const uint32_t ring_ws = smem_u32(ring + (size_t)w * ST * SB_ASTAGE);
+        const uint32_t full_ws = smem_u32(a_full + w * SB_MAX_STAGES);
+        const unsigned char* cbytes_g = (IDXB == 0) ? reinterpret_cast<const unsigned char*>(p.coeff)
+                                                    : reinterpret_cast<const unsigned char*>(p.idx);
+        constexpr int CIROW_PER_N = (IDXB == 0) ? S * 2 : IDXB;
+        int ltile = t0 + u0 / nkb, lkl = u0 % nkb, issued = 0, lslot = 0;
+        auto load_unit = [&]() {
+            const int kb = kb0 + lkl, tile = ltile;
+            if (++lkl == nkb) lkl = 0, ++ltile;
+            const uint32_t stg = ring_ws + (uint32_t)lslot * SB_ASTAGE;
+            const uint32_t bar = full_ws + (uint32_t)lslot * 8u;
+            const int c0 = tile * TN * S, c1 = kb * 8;
+            const unsigned char* csrc = cbytes_g + ((size_t)(kb * NSUB) * N + (size_t)tile * TN) * CIROW_PER_N;
+            if (elect_one()) {
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(A_TX) : "memory");
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                    ::"r"(stg), "l"(reinterpret_cast<uint64_t>(&tmap)), "r"(c0), "r"(c1), "r"(bar)
+                    : "memory");
+#pragma unroll
+                for (int sub = 0; sub < NSUB; ++sub)
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     stg + TS_STAGE_WORDS + sub * CI_BYTES),
+                                 "l"(csrc + (size_t)sub * N * CIROW_PER_N), "r"((uint32_t)CI_BYTES), "r"(bar)
+                                 : "memory");
+            }
+            __syncwarp();
+            ++issued;
+            lslot = (lslot + 1 == ST) ? 0 : lslot + 1;
+        };
+        {
+            const int first = n_w < ST ? n_w : ST;                 // the weights do not depend on the kernel in front
+#pragma unroll 1
+            for (int i = 0; i < first; ++i) load_unit();
+        }
+        if (w == 0) {
+            if (bulk_cache && lane == 0) {
+                mbar_arrive_expect_tx(cache_bar, (uint32_t)(p.C * S * 2));
+                bulk_g2s(cache_s, p.coeff, (uint32_t)(p.C * S * 2), cache_bar);
+            }
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_s)),
+                         "r"((uint32_t)TS_TMEM_COLS)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+            ts_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tmem_ready);
+            pdl_wait();                            // the blob is written by the kernel in front of this one
+            if (lane == 0) {
+#pragma unroll 1
+                for (int b = 0; b < nkb; ++b) {
+                    mbar_arrive_expect_tx(&b_full[b], (uint32_t)BLOB);
+                    bulk_g2s(Bs + (size_t)b * BLOB, p.xb + (size_t)(kb0 + b) * BLOB, (uint32_t)BLOB, &b_full[b]);
+                }
+            }
+            __syncwarp();
+        }
+        ts_wait(smem_u32(tmem_ready), 0u, abort_flag, p.status, 0x420u);
+        ts_fence_after();
+        const uint32_t tbase = __shfl_sync(0xffffffffu, *tmem_base_s, 0);
+        const uint32_t ac = tbase + w * WGCOLS, dc = ac + 32, sfa = tbase + SFA_COL;
+        const uint32_t bs0 = smem_u32(Bs), mbar = smem_u32(&mma_bar[w]);
+        int kl = u0 % nkb;
+#pragma unroll 1
+        for (int i = 0; i < n_w; ++i) {
+            const uint64_t bd = ts_bdesc(bs0 + (uint32_t)kl * BLOB);
+            const uint32_t sc = tbase + SFB_COL + kl * 16;
+            if (i < nkb) {                         // this block's digits and scale factors are in place (first time round)
+                ts_wait(smem_u32(&b_full[kl]), 0u, abort_flag, p.status, 0x422u);
+                ts_wait(smem_u32(&sf_ready[kl]), 0u, abort_flag, p.status, 0x421u);
+            }
+            if (++kl == nkb) kl = 0;
+            named_bar_sync(1 + w, 160);            // A of unit i is in tensor memory, D has been read
+            ts_fence_after();
+            if (elect_one()) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int jm = 0; jm < NJ; ++jm) {
+                        const int sub = (NSUB == 2) ? (c >> 1) : 0;
+                        const bool first = (jm == 0) && ((NSUB == 2) ? ((c & 1) == 0) : (c == 0));
+                        const uint32_t sfid = (uint32_t)((jm & 1) * 2);
+                        ts_mma(dc + sub * 32, ac + c * 8, bd + (uint64_t)((jm * 4096 + c * 256) >> 4),
+                               IDESC | (sfid << 4) | (sfid << 29), sfa, sc + 4 * (jm >> 1), (uint32_t)!first);
+                    }
+                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
+            }
+            __syncwarp();
+            if (issued < n_w) {                    // every compute warp has read the stage of unit i: refill it
+                fence_proxy_async();
+                load_unit();
+            }
+        }
+        if (lane == 0) {                           // no copy of this warp is in flight when the CTA leaves
+            const int firstj = issued > ST ? issued - ST : 0;
+#pragma unroll 1
+            for (int jx = firstj; jx < issued; ++jx)
+                ts_wait(full_ws + (uint32_t)(jx % ST) * 8u, (uint32_t)((jx / ST) & 1), abort_flag, p.status, 0x423u, false);
+            if (w == 0 && bulk_cache) ts_wait(smem_u32(cache_bar), 0u, abort_flag, p.status, 0x411u, false);
+            for (int b = 0; w == 0 && b < nkb; ++b) ts_wait(smem_u32(&b_full[b]), 0u, abort_flag, p.status, 0x412u, false);
+        }
+    } else {
+        // ------------------------------ compute warpgroups ------------------------------
+        const int w = (warp - SB_CW0) >> 2, wl = warp & 3;
+        const int u0 = w * units / SB_NWG, n_w = (w + 1) * units / SB_NWG - u0;
+        const int r = wl * 32 + lane;              // MMA row = tensor-memory lane
+        const int nl = r / SP, s = r % SP;
+        const bool live_row = (S != 3) || (s < S);
+        const uint32_t lane_sel = (uint32_t)(wl * 32) << 16;
+        const unsigned char* ring_w = ring + (size_t)w * ST * SB_ASTAGE;
+        const uint32_t full_ws = smem_u32(a_full + w * SB_MAX_STAGES);
+        const uint32_t mbar = smem_u32(&mma_bar[w]);
+
+        if (p.cache_in_smem && !bulk_cache) {
+            const int tid = threadIdx.x - SB_CW0 * 32;
+            for (int i = tid; i < p.C * S; i += SB_NWG * 128) cache_s[i] = p.coeff[i];
+            named_bar_sync(15, SB_NWG * 128);
+        }
+        ts_wait(smem_u32(tmem_ready), 0u, abort_flag, p.status, 0x430u);
+        ts_fence_after();
+        const uint32_t tbase = __shfl_sync(0xffffffffu, *tmem_base_s, 0);
+        if (w == 0) {
+            // scale factors, for the whole launch: every byte 2^0 for A; for B word i (MMAs 2 i, 2 i + 1) of a row in column 0 of
+            // the block's i-th 4-column block, the same in all four lane quadrants
+            uint32_t f[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) f[i] = 0x7F7F7F7Fu;
+            ts_st32(tbase + lane_sel + SFA_COL, f);
+#pragma unroll 1
+            for (int b = 0; b < nkb; ++b) {
+                ts_wait(smem_u32(&b_full[b]), 0u, abort_flag, p.status, 0x433u);
+                const uint4 sf = reinterpret_cast<const uint4*>(Bs + (size_t)b * BLOB + NJ * 4096)[lane];
+                asm volatile(
+                    "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%4,%4,%4,%2,%4,%4,%4,%3,%4,%4,%4,%4,%4,%4,%4};" ::"r"(
+                        tbase + lane_sel + SFB_COL + b * 16),
+                    "r"(sf.x), "r"(sf.y), "r"(sf.z), "r"(0x7F7F7F7Fu)
+                    : "memory");
+                ts_wait_st();
+                ts_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sf_ready[b]);
+            }
+        }
+        if (bulk_cache) ts_wait(smem_u32(cache_bar), 0u, abort_flag, p.status, 0x431u);
+
+        const uint32_t a_addr = tbase + w * WGCOLS + lane_sel, d_addr = a_addr + 32;
+        float acc[MP];
+#pragma unroll
+        for (int m = 0; m < MP; ++m) acc[m] = 0.0f;
+        const int wpos = nl * S + s;
+        // Sums of one tile's units: planes added by shuffles, every thread of a row's planes keeps the activation rows
+        // m = s (mod SP).  A tile that is all this warpgroup's goes out at once, one that it shares with a neighbour (its first
+        // or its last) to shared memory.
+        int tile = t0 + u0 / nkb, have = 0;        // tile of the sums, units of it in them
+        auto deposit = [&](bool last) {
+            const bool whole = have == nkb;
+            float* dst = whole ? p.part + ((size_t)chunk * p.NT + tile) * (MP * TN) + nl : res + (size_t)(w * 2 + (last ? 1 : 0)) * (MP * TN) + nl;
+            const int n = tile * TN + nl;
+            unsigned int pm = 0u;                  // activation rows of this chunk with a non-finite value
+            for (int b = 0; whole && b < nkb; ++b)
+                pm |= __ballot_sync(0xffffffffu, lane < MP && reinterpret_cast<const uint4*>(Bs + (size_t)b * BLOB + NJ * 4096)[lane].w != 0u);
+            const float bias = (whole && KC == 1 && p.bias) ? __half2float(p.bias[n]) : 0.0f;
+#pragma unroll
+            for (int m = 0; m < MP; ++m) {
+                float v = acc[m];
+                acc[m] = 0.0f;
+                v += __shfl_xor_sync(0xffffffffu, v, 1);
+                if (SP == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
+                if ((m % SP) == s) {
+                    if (!whole) {
+                        dst[m * TN] = v;
+                    } else {
+                        if ((pm >> m) & 1u) v = __int_as_float(0x7fc00000);
+                        if (KC > 1) __stcg(dst + m * TN, v);
+                        else if (m < M) p.y[(size_t)m * N + n] = __float2half_rn(v + bias);
+                    }
+                }
+            }
+            have = 0;
+            ++tile;
+        };
+        uint32_t wv[8];
+        float cf[NSUB], cp[NSUB];                  // coefficients of the unit in A, of the unit in D
+        int aslot = 0;
+        uint32_t apar = 0u;
+        auto fetch = [&]() {                       // the next unit's packed words and coefficients
+            ts_wait(full_ws + (uint32_t)aslot * 8u, apar, abort_flag, p.status, 0x432u);
+            const unsigned char* stg = ring_w + (size_t)aslot * SB_ASTAGE;
+            const uint32_t* wsrc = reinterpret_cast<const uint32_t*>(stg) + wpos;
+#pragma unroll
+            for (int kw = 0; kw < 8; ++kw) wv[kw] = live_row ? wsrc[kw * (WROW / 4)] : 0u;
+#pragma unroll
+            for (int sub = 0; sub < NSUB; ++sub) {
+                const unsigned char* cs = stg + TS_STAGE_WORDS + sub * CI_BYTES;
+                float c = 0.0f;
+                if constexpr (IDXB == 0) {
+                    if (live_row) c = __half2float(reinterpret_cast<const __half*>(cs)[nl * S + s]);
+                } else {
+                    const uint32_t ci = (IDXB == 1) ? (uint32_t)cs[nl] : (uint32_t)reinterpret_cast<const unsigned short*>(cs)[nl];
+                    if (live_row) c = __half2float((p.cache_in_smem ? cache_s : p.coeff)[(size_t)ci * S + s]);
+                }
+                cf[sub] = c;
+            }
+            if (++aslot == ST) {
+                aslot = 0;
+                apar ^= 1u;
+            }
+        };
+        if (n_w > 0) fetch();
+        int kl = u0 % nkb;                         // k block of unit i - 1
+#pragma unroll 1
+        for (int i = 0; i <= n_w; ++i) {
+            uint32_t d[NSUB][4][8];
+            if (i > 0) {
+                ts_wait(mbar, (uint32_t)((i - 1) & 1), abort_flag, p.status, 0x434u);
+                ts_fence_after();
+#pragma unroll
+                for (int sub = 0; sub < NSUB; ++sub) {
+                    ts_ld16_issue(d_addr + sub * 32, d[sub][0], d[sub][1]);
+                    ts_ld16_issue(d_addr + sub * 32 + 16, d[sub][2], d[sub][3]);
+                }
+            }
+            if (i < n_w) {
+                // packed words of this thread's row -> 32 words of 4-bit elements {0, 1 | 1 | 2 | 2}
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const uint32_t w0 = wv[2 * h], w1 = wv[2 * h + 1];
+                    ts_st8(a_addr + h * 8, (w0 << 1) & 0x22222222u, w0 & 0x22222222u, w0 & 0x44444444u, (w0 >> 1) & 0x44444444u,
+                           (w1 << 1) & 0x22222222u, w1 & 0x22222222u, w1 & 0x44444444u, (w1 >> 1) & 0x44444444u);
+                }
+            }
+            if (i > 0) {
+#pragma unroll
+                for (int sub = 0; sub < NSUB; ++sub)
+#pragma unroll
+                    for (int g4 = 0; g4 < 4; ++g4) ts_wait_ld(d[sub][g4]);
+            }
+            if (i < n_w) {
+                ts_wait_st();
+                ts_fence_before();
+                ts_bar_arrive(1 + w, 160);         // releases the MMAs of unit i; also: its stage has been read
+            }
+            if (i > 0) {
+#pragma unroll
+                for (int sub = 0; sub < NSUB; ++sub)
+#pragma unroll
+                    for (int m = 0; m < MP; ++m) {
+                        float v = __uint_as_float(d[sub][m >> 3][m & 7]);
+                        if (NJ == 3) v += __uint_as_float(d[sub][2 + (m >> 3)][m & 7]);
+                        acc[m] = fmaf(v, cp[sub], acc[m]);
+                    }
+                ++have;
+                if (++kl == nkb || i == n_w) {
+                    kl = 0;
+                    // (a shared tile's sums: the last tile of the warpgroup's range unless the range lies inside one tile)
+                    deposit(i == n_w && tile > t0 + u0 / nkb);
+                }
+            }
+#pragma unroll
+            for (int sub = 0; sub < NSUB; ++sub) cp[sub] = cf[sub];
+            if (i + 1 < n_w) fetch();
+        }
+    }
+    ts_fence_before();
+    __syncthreads();
+    ts_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*tmem_base_s), "r"((uint32_t)TS_TMEM_COLS)
+                     : "memory");
+
+    // ------------------------------ tiles shared by warpgroups ------------------------------
+    // Tile `tl` of the range has units [tl nkb, (tl + 1) nkb), warpgroup w the units [w U / 4, (w + 1) U / 4); where a boundary
+    // lies inside a tile its warpgroups' sums are added here, in warpgroup order.
+    {
+        int done = -1;
+#pragma unroll 1
+        for (int wb = 1; wb < SB_NWG; ++wb) {
+            const int bd = wb * units / SB_NWG, tl = bd / nkb;
+            if (bd == tl * nkb || tl == done) continue;       // a tile boundary, or the tile has been dealt with
+            done = tl;
+            for (int q = threadIdx.x; q < MP * TN; q += SB_THREADS) {
+                const int m = q / TN, n = (t0 + tl) * TN + q % TN;
+                float v = 0.0f;
+#pragma unroll
+                for (int w = 0; w < SB_NWG; ++w) {
+                    const int a = w * units / SB_NWG, b = (w + 1) * units / SB_NWG;
+                    if (a < (tl + 1) * nkb && b > tl * nkb && a < b) v += res[(size_t)(w * 2 + (tl > a / nkb ? 1 : 0)) * (MP * TN) + q];
+                }
+                bool poison = false;
+                for (int b = 0; b < nkb; ++b) poison |= reinterpret_cast<const uint4*>(Bs + (size_t)b * BLOB + NJ * 4096)[m].w != 0u;
+                if (poison) v = __int_as_float(0x7fc00000);
+                if (KC > 1) __stcg(p.part + ((size_t)chunk * p.NT + t0 + tl) * (MP * TN) + q, v);
+                else if (m < M) p.y[(size_t)m * N + n] = __float2half_rn(v + (p.bias ? __half2float(p.bias[n]) : 0.0f));
+            }
+        }
+    }
+    // ------------------------------ the chunks' sums ------------------------------
+    if (KC > 1) {
+        __threadfence();                           // this thread's sums, before its CTA's arrival below
+        __syncthreads();
+        // A tile's rows are counted in 2^psh parts; the arrivals of 32 parts are in flight together, then the warp adds the
+        // chunks of those at which it arrived last.
+        const int np = ntc << p.psh, per = (MP * TN) >> p.psh;
+        unsigned int* cnt = p.counters + ((size_t)t0 << p.psh);
+        const size_t plane = (size_t)p.NT * (MP * TN);
+        for (int p0 = warp; p0 < np; p0 += 32 * (SB_THREADS / 32)) {
+            const int mypart = p0 + lane * (SB_THREADS / 32);
+            unsigned int last = 0u;
+            if (mypart < np) {
+                last = atomicAdd(cnt + mypart, 1u) == (unsigned int)(KC - 1) ? 1u : 0u;
+                if (last) cnt[mypart] = 0u;
+            }
+            __syncwarp();
+            unsigned int todo = __ballot_sync(0xffffffffu, last != 0u);
+            if (todo) __threadfence();
+            while (todo) {
+                const int part = p0 + (__ffs((int)todo) - 1) * (SB_THREADS / 32);
+                todo &= todo - 1u;
+                const int tl = part >> p.psh;
+                const float* src = p.part + (size_t)(t0 + tl) * (MP * TN);
+                for (int q = (part & ((1 << p.psh) - 1)) * per + lane, e = q + per - lane; q < e; q += 128) {
+                    float v[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) v[u] = 0.0f;
+                    for (int c = 0; c < KC; c += 2) {          // eight loads in flight
+                        float t[2][4];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int u = 0; u < 4; ++u)
+                                t[h][u] = (c + h < KC && q + 32 * u < e && (q + 32 * u) / TN < M) ? __ldcg(src + (size_t)(c + h) * plane + q + 32 * u) : 0.0f;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h)
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) v[u] += t[h][u];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int qq = q + 32 * u, m = qq / TN, n = (t0 + tl) * TN + qq % TN;
+                        if (qq < e && m < M) p.y[(size_t)m * N + n] = __float2half_rn(v[u] + (p.bias ? __half2float(p.bias[n]) : 0.0f));
+                    }
+                }
+            }
+        }
+    }
+    if (threadIdx.x == 0 && *abort_flag) {         // which problem gave up: N, and K / 256 | M | CTA (for the host's message)
+        atomicExch(p.status + 2, (unsigned int)p.N);
+        atomicExch(p.status + 3, ((unsigned int)p.KB << 16) | ((unsigned int)M << 8) | (blockIdx.x & 0xFFu));
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// host
+// ---------------------------------------------------------------------------------------------
+struct SbPlan {
+    int KB, NT, NJ, KC, GN, cache_in_smem, stages, psh, smem;
+    int off_cache, off_ring, off_res;
+    size_t blob_bytes, part_bytes;
+};
+
+static int sb_plan(const PackedW& w, int M, const DeviceInfo& di, SbPlan* pl) {
+    const int TN = ts_tn(w.S), NSUB = 256 / w.G;
+    pl->NJ = M <= 16 ? 3 : 6;
+    const int MP = pl->NJ == 3 ? 16 : 32;
+    pl->KB = w.K / 256;
+    pl->NT = w.N / TN;
+    if (pl->KB < 1 || pl->NT < 1) return SBVR_ERR_UNSUPPORTED;
+    // Chunks as large as shared memory holds; smaller ones while less than two thirds of the SMs would have work and a
+    // warpgroup more than one unit.
+    pl->KC = (pl->KB + sb_chunk(NSUB, pl->NJ) - 1) / sb_chunk(NSUB, pl->NJ);
+    auto groups = [&](int kc) { const int g = di.sm_count / kc; return g < 1 ? 1 : (g < pl->NT ? g : pl->NT); };
+    while (groups(pl->KC) * pl->KC * 3 <= di.sm_count * 2 && pl->KC * 2 <= pl->KB && pl->KC * 2 <= 16 &&
+           (pl->NT + groups(pl->KC) - 1) / groups(pl->KC) * (pl->KB / pl->KC) > SB_NWG)
+        pl->KC *= 2;
+    pl->GN = groups(pl->KC);
+    const int nkb = (pl->KB + pl->KC - 1) / pl->KC;
+    // quarter tiles where the workspace has that many counters, else (very wide layers) whole tiles
+    pl->psh = pl->NT * 4 <= SBVR_WS_COUNTERS ? 2 : 0;
+    if (pl->KC > 1 && pl->NT > SBVR_WS_COUNTERS) return SBVR_ERR_UNSUPPORTED;
+    pl->blob_bytes = ((size_t)pl->KB * sb_blob(pl->NJ) + 255) / 256 * 256;
+    pl->part_bytes = pl->KC > 1 ? (size_t)pl->KC * pl->NT * MP * TN * 4 : 0;
+    const int cache_bytes = w.idx_bytes ? ts_round_up(w.C * w.S * 2, 16) : 0;
+    auto layout = [&](int cb, int stages) {
+        pl->off_cache = SB_HDR + nkb * sb_blob(pl->NJ);
+        pl->off_ring = ts_round_up(pl->off_cache + cb, 128);
+        pl->off_res = pl->off_ring + SB_NWG * stages * SB_ASTAGE;
+        return pl->off_res + SB_NWG * 2 * MP * TN * 4;
+    };
+    pl->cache_in_smem = (w.idx_bytes && cache_bytes <= 65536 && layout(cache_bytes, 2) <= di.smem_optin) ? 1 : 0;
+    const int cb = pl->cache_in_smem ? cache_bytes : 0;
+    int st = SB_MAX_STAGES;
+    while (st > 2 && layout(cb, st) > di.smem_optin) --st;
+    pl->stages = st;
+    pl->smem = layout(cb, st);
+    if (pl->smem > di.smem_optin) return SBVR_ERR_UNSUPPORTED;
+    return SBVR_OK;
+}
+
+bool linear_sb_supported(const PackedW& w, int M) {
+    if (w.S < 2 || w.S > 4) return false;
+    if (w.G != 256 && w.G != 128) return false;
+    if (M < 2 || M > 32) return false;
+    if (w.G == 128 && M > 16) return false;
+    if (w.N % ts_tn(w.S) || w.K % 256 || w.K > 32768) return false;
+    if (w.idx_bytes < 0 || w.idx_bytes > 2) return false;
+    if (reinterpret_cast<uintptr_t>(w.coeff) & 15) return false;                 // bulk copies
+    if (reinterpret_cast<uintptr_t>(w.bvr) & 15) return false;                   // tensor map base
+    if (w.idx_bytes && (reinterpret_cast<uintptr_t>(w.idx) & 15)) return false;
+    if ((size_t)(w.N / ts_tn(w.S)) * (size_t)(w.K / 256) >= ((size_t)1 << 24)) return false;   // 32-bit unit arithmetic
+    if ((size_t)w.N * w.S >= ((size_t)1 << 31)) return false;                    // 32-bit tensor coordinates
+    DeviceInfo di;
+    int dev = 0;
+    SbPlan pl;
+    if (cudaGetDevice(&dev) != cudaSuccess || device_info(dev, &di) != SBVR_OK) return false;
+    return sb_plan(w, M, di, &pl) == SBVR_OK;
+}
+
+size_t linear_sb_workspace_bytes(const PackedW& w, int M, const DeviceInfo& di) {
+    SbPlan pl;
+    if (sb_plan(w, M, di, &pl) != SBVR_OK) return 0;
+    return pl.blob_bytes + pl.part_bytes;
+}
+
+template <int S, int NSUB, int NJ, int IDXB>
+static int sb_launch_inst(const CUtensorMap& tm, const SbParams& p, int grid, int smem, cudaStream_t st) {
+    static SmemOnce once;
+    const int rc = set_max_smem_once(once, linear_sb_kernel<S, NSUB, NJ, IDXB>, 227 * 1024);
+    if (rc) return rc;
+    SBVR_CUDA_TRY(launch_pdl(linear_sb_kernel<S, NSUB, NJ, IDXB>, dim3(grid), dim3(SB_THREADS), (size_t)smem, st, tm, p));
+    return SBVR_OK;
+}
+template <int S, int NSUB, int NJ>
+static int sb_launch_idx(const CUtensorMap& tm, const SbParams& p, int idxb, int grid, int smem, cudaStream_t st) {
+    switch (idxb) {
+        case 0: return sb_launch_inst<S, NSUB, NJ, 0>(tm, p, grid, smem, st);
+        case 1: return sb_launch_inst<S, NSUB, NJ, 1>(tm, p, grid, smem, st);
+        default: return sb_launch_inst<S, NSUB, NJ, 2>(tm, p, grid, smem, st);
+    }
+}
+template <int S>
+static int sb_launch_g(const CUtensorMap& tm, const SbParams& p, int G, int NJ, int idxb, int grid, int smem, cudaStream_t st) {
+    if (G == 128) return sb_launch_idx<S, 2, 3>(tm, p, idxb, grid, smem, st);
+    return NJ == 3 ? sb_launch_idx<S, 1, 3>(tm, p, idxb, grid, smem, st) : sb_launch_idx<S, 1, 6>(tm, p, idxb, grid, smem, st);
+}
+
+// `counters` (zero between calls: the kernel leaves them zero) and `scratch` (256-byte aligned,
+// linear_sb_workspace_bytes long: digit blob and the chunks' sums) are the caller's.
+int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, int device, unsigned int* status,
+                     unsigned int* counters, char* scratch, size_t scratch_bytes, cudaStream_t st, const XOp* xop) {
+    if (!linear_sb_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
+    if (!status || !counters || !scratch) return SBVR_ERR_WORKSPACE;
+    if (reinterpret_cast<uintptr_t>(x) & 1) return SBVR_ERR_ALIGN;
+    if (reinterpret_cast<uintptr_t>(scratch) & 255) return SBVR_ERR_ALIGN;
+    DeviceInfo di;
+    int rc = device_info(device, &di);
+    if (rc) return rc;
+    if (di.cc_major != 10) return SBVR_ERR_UNSUPPORTED;
+    SbPlan pl;
+    rc = sb_plan(w, M, di, &pl);
+    if (rc) return rc;
+    if (pl.blob_bytes + pl.part_bytes > scratch_bytes) return SBVR_ERR_WORKSPACE;
+    CUtensorMap tm;
+    rc = ts_tensor_map(w, 1, &tm);
+    if (rc) return rc;
+    SbQuant q;
+    q.x = x, q.xb = reinterpret_cast<unsigned char*>(scratch), q.M = M, q.K = w.K;
+    rc = xop_check(xop, x, M, w.K, &q.x_op, &q.delta, &q.norm_w, &q.h_out, &q.eps);
+    if (rc) return rc;
+    if (pl.NJ == 3) SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel<3>, dim3(pl.KB, 4), dim3(128), 0, st, q));
+    else SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel<6>, dim3(pl.KB, 8), dim3(128), 0, st, q));
+    SbParams p;
+    p.xb = q.xb;
+    p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status, p.counters = counters;
+    p.part = reinterpret_cast<float*>(scratch + pl.blob_bytes);
+    p.M = M, p.N = w.N, p.K = w.K, p.KB = pl.KB, p.NT = pl.NT, p.C = w.C, p.KC = pl.KC, p.GN = pl.GN;
+    p.cache_in_smem = pl.cache_in_smem, p.stages = pl.stages, p.psh = pl.psh;
+    p.off_cache = pl.off_cache, p.off_ring = pl.off_ring, p.off_res = pl.off_res;
+    const int grid = pl.GN * pl.KC;
+    switch (w.S) {
+        case 2: return sb_launch_g<2>(tm, p, w.G, pl.NJ, w.idx_bytes, grid, pl.smem, st);
+        case 3: return sb_launch_g<3>(tm, p, w.G, pl.NJ, w.idx_bytes, grid, pl.smem, st);
+        default: return sb_launch_g<4>(tm, p, w.G, pl.NJ, w.idx_bytes, grid, pl.smem, st);
+    }
+}
+
+}  // namespace sbvr

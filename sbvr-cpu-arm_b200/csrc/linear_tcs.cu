@@ -984,24 +984,8 @@ int launch_linear_tcs(const __half* x, const PackedW& w, const __half* bias, __h
     if ((size_t)pl.grid * 2 * M * ts_tn(w.S) * 8 > SBVR_WS_XCHG_BYTES) return SBVR_ERR_UNSUPPORTED;
     XqParams xp;
     xp.x = x, xp.xq = reinterpret_cast<unsigned char*>(scratch), xp.K = w.K, xp.KB = pl.KB, xp.M = M;
-    xp.x_op = xop ? xop->op : SBVR_XOP_NONE;
-    xp.delta = xop ? xop->delta : nullptr, xp.norm_w = xop ? xop->norm_w : nullptr, xp.h_out = xop ? xop->h_out : nullptr;
-    xp.eps = xop ? xop->eps : 0.0f;
-    if (xp.x_op == SBVR_XOP_ADD_RMSNORM) {
-        // h_out is written while other blocks still read x and delta for the row's mean square
-        if (!xp.norm_w) return SBVR_ERR_BAD_ARG;
-        if (xp.h_out) {
-            const uintptr_t n = (uintptr_t)M * w.K * 2, ho = reinterpret_cast<uintptr_t>(xp.h_out);
-            auto overlaps = [&](const void* q) {
-                const uintptr_t a = reinterpret_cast<uintptr_t>(q);
-                return q && ho < a + n && a < ho + n;
-            };
-            if (overlaps(x) || overlaps(xp.delta)) return SBVR_ERR_BAD_ARG;
-        }
-        if ((reinterpret_cast<uintptr_t>(xp.delta) | reinterpret_cast<uintptr_t>(xp.norm_w) |
-             reinterpret_cast<uintptr_t>(xp.h_out)) & 15)
-            return SBVR_ERR_ALIGN;
-    }
+    rc = xop_check(xop, x, M, w.K, &xp.x_op, &xp.delta, &xp.norm_w, &xp.h_out, &xp.eps);
+    if (rc) return rc;
     CUtensorMap tm;
     rc = ts_tensor_map(w, pl.KS, &tm);
     if (rc) return rc;
