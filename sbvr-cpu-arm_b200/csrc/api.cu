@@ -265,7 +265,8 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
     if (algo == 3) return launch_linear_gemm(xh, Kin, w, bh, yh, M, ws, st);
     if (algo == 4) {
         if (!ws) return SBVR_ERR_WORKSPACE;
-        return launch_linear_sb(xh, w, bh, yh, M, ws->device, ws->status, ws->counters, ws->dyn, ws->dyn_bytes, st);
+        return launch_linear_sb(xh, w, bh, yh, M, ws->device, ws->status, reinterpret_cast<unsigned int*>(ws->xchg), ws->dyn,
+                                ws->dyn_bytes, st);
     }
     return launch_linear_simt(xh, w, bh, yh, M, st);
 }

@@ -21,11 +21,14 @@
 // Structure.  K is cut into chunks of at most eight (M > 16: four) 256-k blocks, and a CTA works on one chunk: its digits
 // (12 or 24 KB per block, written by the quantiser kernel) stay in shared memory and their scale factors in tensor memory for
 // the whole launch, so the only things that move are packed words.  Four warpgroups take (row tile, k block) units in order,
-// each on its own, with one A and one D buffer: as soon as the MMAs of unit i are done, the sums are requested, the next
-// unit's words are expanded into A while they arrive, and the MMAs of unit i + 1 are released; the multiply-adds and the
-// shared-memory loads of unit i + 2 run beside them.  A tile that several warpgroups share meets in shared memory; the chunks'
-// sums meet in scratch, where the warp that arrives last at a quarter tile's counter adds them in chunk order (the same bits
-// on every run; nobody waits for another CTA).  Every wait is bounded.
+// each on its own, with two A buffers and one D buffer: while the MMAs of unit i run, unit i + 1 is expanded into the other
+// A buffer and unit i + 2 read from shared memory; as soon as they are done the sums are read and the MMAs of unit i + 1
+// released, and the multiply-adds run beside those.  (Two groups per k block take two D buffers and leave room for one A.)  A
+// warp holds all sums of a quarter of a tile's rows.  The chunks' sums of a
+// quarter meet in scratch: every warp stores its own, counts its arrival a unit later (the stores have landed by then), looks
+// at the answer another unit later, and adds them in chunk order if it was the last (the same bits on every run; nobody waits
+// for another CTA, and all of it but the last tile's runs beside the other warpgroups' units).  A tile that several warpgroups
+// share is put together in shared memory at the end.  Every wait is bounded.
 //
 // What bounds it: a unit (4.6 KB of weight) is 12 MMAs of 17 cycles and about 220 issue slots per scheduler, against 200 cycles
 // of its SM's share of HBM; measured about 290 cycles.  The form before this one (three warpgroups in lockstep over shared
@@ -47,12 +50,13 @@ constexpr int SB_ASTAGE = TS_STAGE_WORDS + 512; // packed words of a unit + its 
 constexpr int SB_MAX_STAGES = 4;
 constexpr int SB_HDR = 1024;
 __host__ __device__ constexpr int sb_blob(int NJ) { return NJ * 4096 + SB_SF_BYTES; }
-// k blocks of a CTA at most: what shared memory (digits) and, for two groups per block, tensor memory hold
-__host__ __device__ constexpr int sb_chunk(int NSUB, int NJ) { return NJ == 6 ? 4 : NSUB == 2 ? 6 : 8; }
-// Tensor memory: per warpgroup A (32 columns) and D (32 per group of a block), then the B scale factors of every k block (16
-// columns each: three 4-column blocks; an MMA's scale-factor address designates one), then unit scale factors for A
-__host__ __device__ constexpr int sb_wgcols(int NSUB) { return 32 + NSUB * 32; }
-__host__ __device__ constexpr int sb_sf_col(int NSUB) { return SB_NWG * sb_wgcols(NSUB); }
+__host__ __device__ constexpr int sb_chunk(int NJ) { return NJ == 6 ? 4 : 8; }       // k blocks of a CTA at most (shared memory)
+__host__ __device__ constexpr int sb_sfcols(int NJ) { return NJ == 6 ? 16 : 8; }
+// Tensor memory: per warpgroup A (32 columns each) and D (32 per group of a block), then the B scale factors of every k block (16
+// or 8 columns each, one 4-column block per two MMAs; an MMA's scale-factor address designates a block), then unit factors for A
+constexpr int SB_WGCOLS = 96;                   // A x 2 and D, or A and D x 2
+constexpr int SB_SFB_COL = SB_NWG * SB_WGCOLS, SB_SFA_COL = SB_SFB_COL + 64;
+static_assert(SB_SFA_COL + 32 <= TS_TMEM_COLS, "tensor memory");
 
 struct SbParams {
     const unsigned char* xb;      // [KB][sb_blob] written by sb_quant_kernel
@@ -61,10 +65,9 @@ struct SbParams {
     const __half* bias;
     __half* y;
     unsigned int* status;
-    unsigned int* counters;       // one per (tile, part of its rows), zero between launches
+    unsigned int* counters;       // one per quarter of a tile's rows, zero between launches
     float* part;                  // [KC][NT][MP][TN] sums of the chunks (KC > 1)
     int M, N, K, KB, NT, C, KC, GN, cache_in_smem, stages;
-    int psh;                      // log2 of the parts of a tile that are counted separately
     int off_cache, off_ring, off_res;
 };
 
@@ -82,18 +85,19 @@ struct SbQuant {
 // ---------------------------------------------------------------------------------------------
 // activations (with the op in front of the linear) -> digit blob, once per call
 // ---------------------------------------------------------------------------------------------
-// One block per 256-k block and four (padded) activation rows, one warp per row.  Lane (kw, j) owns the eight elements
+// One block per 256-k block and two (padded) activation rows, one warp per row: with 64 threads a block fits beside a resident
+// CTA of the product (61 440 of the SM's registers), and both wait for their predecessors there.  Lane (kw, j) owns the eight elements
 // k = 32 kw + j + 4 e, which are one 32-bit word (nibble e) of every digit: the K order in which the weight expansion
 // leaves the plane bits.  Blob of a k block: [MMA j (NJ)][row group (4)][kw (8)][row (8)][16 B], then 32 rows x 16 B:
 // words 0 .. 2 hold the scale bytes of MMA 2 i (bytes 0, 1) and 2 i + 1 (bytes 2, 3) for that B row, word 3 of row m whether
 // activation row m of this block holds a non-finite value.
 template <int NJ>
-__global__ void __launch_bounds__(128) sb_quant_kernel(const SbQuant p) {
-    __shared__ __align__(16) __half row[4][256];
+__global__ void __launch_bounds__(64) sb_quant_kernel(const SbQuant p) {
+    __shared__ __align__(16) __half row[2][256];
     pdl_launch_dependents();
     pdl_wait();                                    // the activations come from the previous kernel of the stream
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kb = blockIdx.x, K = p.K, M = p.M, m = blockIdx.y * 4 + wl;
+    const int kb = blockIdx.x, K = p.K, M = p.M, m = blockIdx.y * 2 + wl;
     const int kw = lane >> 2, j = lane & 3;
     uint32_t words[6] = {0u, 0u, 0u, 0u, 0u, 0u};
     int ex = 14;
@@ -214,6 +218,67 @@ __global__ void __launch_bounds__(128) sb_quant_kernel(const SbQuant p) {
 // ---------------------------------------------------------------------------------------------
 // the product
 // ---------------------------------------------------------------------------------------------
+// Two fp32 values in one 64-bit register: the packed add and multiply-add issue once for both.
+struct SbPair {
+    unsigned long long b;
+    __device__ SbPair() {}
+    __device__ SbPair(uint32_t lo, uint32_t hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "r"(lo), "r"(hi)); }
+    __device__ SbPair(float lo, float hi) { asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(lo), "f"(hi)); }
+    __device__ void get(float& lo, float& hi) const { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(b)); }
+    __device__ SbPair operator+(const SbPair& o) const {
+        SbPair r;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.b) : "l"(b), "l"(o.b));
+        return r;
+    }
+    __device__ SbPair mul_add(const SbPair& f, const SbPair& o) const {      // this * f + o
+        SbPair r;
+        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.b) : "l"(b), "l"(f.b), "l"(o.b));
+        return r;
+    }
+};
+
+// A warp's stores so far become visible, then its arrival is counted; lane 0 gets the arrivals before it.
+__device__ __forceinline__ unsigned int sb_arrive(unsigned int* counter, int lane) {
+    unsigned int old = 0u;
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) old = atomicAdd(counter, 1u);
+    return old;
+}
+
+// The chunks' sums of a quarter of a tile's rows -> y, in chunk order; the counter goes back to zero.
+template <int MP, int TN>
+__device__ __forceinline__ void sb_add_chunks(const SbParams& p, int tile, int quarter, int lane) {
+    constexpr int QR = TN / 4, PER = MP * QR / 32;
+    if (lane == 0) p.counters[tile * 4 + quarter] = 0u;
+    __threadfence();
+    const size_t plane = (size_t)p.NT * (MP * TN);
+    const float* src = p.part + (size_t)tile * (MP * TN) + quarter * QR;
+    float v[PER];
+#pragma unroll
+    for (int u = 0; u < PER; ++u) v[u] = 0.0f;
+#pragma unroll 1
+    for (int c = 0; c < p.KC; c += 2) {            // two chunks' loads in flight
+        float t[2][PER];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const int q = lane + 32 * u, m = q / QR;
+                t[h][u] = (c + h < p.KC && m < p.M) ? __ldcg(src + (size_t)(c + h) * plane + m * TN + q % QR) : 0.0f;
+            }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int u = 0; u < PER; ++u) v[u] += t[h][u];
+    }
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+        const int q = lane + 32 * u, m = q / QR, n = tile * TN + quarter * QR + q % QR;
+        if (m < p.M) p.y[(size_t)m * p.N + n] = __float2half_rn(v[u] + (p.bias ? __half2float(p.bias[n]) : 0.0f));
+    }
+}
+
 template <int S, int NSUB, int NJ, int IDXB>
 __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_constant__ CUtensorMap tmap, const SbParams p) {
     pdl_launch_dependents();
@@ -221,14 +286,13 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
     constexpr int SP = ts_sp(S);
     constexpr int TN = ts_tn(S);
     constexpr int MP = (NJ == 3) ? 16 : 32;        // activation rows the accumulators cover
-    constexpr int WGCOLS = sb_wgcols(NSUB);
+    constexpr int NV = MP / SP;                    // ... and how many of them one thread finishes
+    constexpr int ABUF = NSUB == 2 ? 1 : 2;        // A buffers
+    constexpr int SFC = sb_sfcols(NJ);
     constexpr int BLOB = sb_blob(NJ);
     constexpr int WROW = TN * S * 4;               // bytes of one 32-k row of a stage
     constexpr int CI_BYTES = (IDXB == 0) ? TN * S * 2 : TN * IDXB;
     constexpr uint32_t A_TX = 8 * WROW + NSUB * CI_BYTES;
-    constexpr int SFB_COL = sb_sf_col(NSUB);
-    constexpr int SFA_COL = SFB_COL + 16 * sb_chunk(NSUB, NJ);
-    static_assert(SFA_COL + 32 <= TS_TMEM_COLS, "tensor memory");
     // instruction descriptor: A, B = E2M1, scales UE8M0, M = 128, N = 32, K-major both; the scale-factor byte pair is added per MMA
     constexpr uint32_t IDESC = (1u << 7) | (1u << 10) | ((uint32_t)(32 >> 3) << 17) | (1u << 23) | (8u << 24);
 
@@ -240,6 +304,7 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
     uint64_t* tmem_ready = cache_bar + 1;                                            // [1] tensor memory allocated
     constexpr int SF0 = SB_NWG * (SB_MAX_STAGES + 1) + 8, NBAR = SF0 + 8 + 2;
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + SB_HDR - 64);
+    volatile unsigned int* poison_s = reinterpret_cast<volatile unsigned int*>(smem + SB_HDR - 48);      // activation rows with a non-finite value
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(smem + SB_HDR - 16);
 
     const int N = p.N, M = p.M, KC = p.KC;
@@ -262,6 +327,8 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
     __syncthreads();
     const bool bulk_cache = p.cache_in_smem && ((p.C * S * 2) % 16 == 0);
 
+    int pend = 0, ptile = 0;                       // a tile of which the chunks' sums are being counted: 1 stored, 2 counted
+    unsigned int old = 0u;
     if (warp < SB_NWG) {
         // ------------------------------ issuer warps, one per warpgroup ------------------------------
         const int w = warp;
@@ -326,13 +393,13 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
         ts_wait(smem_u32(tmem_ready), 0u, abort_flag, p.status, 0x420u);
         ts_fence_after();
         const uint32_t tbase = __shfl_sync(0xffffffffu, *tmem_base_s, 0);
-        const uint32_t ac = tbase + w * WGCOLS, dc = ac + 32, sfa = tbase + SFA_COL;
+        const uint32_t ac0 = tbase + w * SB_WGCOLS, dc = ac0 + ABUF * 32, sfa = tbase + SB_SFA_COL;
         const uint32_t bs0 = smem_u32(Bs), mbar = smem_u32(&mma_bar[w]);
         int kl = u0 % nkb;
 #pragma unroll 1
         for (int i = 0; i < n_w; ++i) {
             const uint64_t bd = ts_bdesc(bs0 + (uint32_t)kl * BLOB);
-            const uint32_t sc = tbase + SFB_COL + kl * 16;
+            const uint32_t sc = tbase + SB_SFB_COL + kl * SFC, ac = ac0 + (ABUF == 2 ? (i & 1) * 32 : 0);
             if (i < nkb) {                         // this block's digits and scale factors are in place (first time round)
                 ts_wait(smem_u32(&b_full[kl]), 0u, abort_flag, p.status, 0x422u);
                 ts_wait(smem_u32(&sf_ready[kl]), 0u, abort_flag, p.status, 0x421u);
@@ -393,16 +460,17 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
             uint32_t f[32];
 #pragma unroll
             for (int i = 0; i < 32; ++i) f[i] = 0x7F7F7F7Fu;
-            ts_st32(tbase + lane_sel + SFA_COL, f);
+            ts_st32(tbase + lane_sel + SB_SFA_COL, f);
+            unsigned int pm = 0u;
 #pragma unroll 1
             for (int b = 0; b < nkb; ++b) {
                 ts_wait(smem_u32(&b_full[b]), 0u, abort_flag, p.status, 0x433u);
                 const uint4 sf = reinterpret_cast<const uint4*>(Bs + (size_t)b * BLOB + NJ * 4096)[lane];
-                asm volatile(
-                    "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%4,%4,%4,%2,%4,%4,%4,%3,%4,%4,%4,%4,%4,%4,%4};" ::"r"(
-                        tbase + lane_sel + SFB_COL + b * 16),
-                    "r"(sf.x), "r"(sf.y), "r"(sf.z), "r"(0x7F7F7F7Fu)
-                    : "memory");
+                const uint32_t at = tbase + lane_sel + SB_SFB_COL + b * SFC;
+                ts_st8(at, sf.x, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, sf.y, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
+                if (NJ == 6) ts_st8(at + 8, sf.z, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
+                pm |= __ballot_sync(0xffffffffu, lane < MP && sf.w != 0u);
+                if (wl == 0 && b == nkb - 1) *poison_s = pm;
                 ts_wait_st();
                 ts_fence_before();
                 __syncwarp();
@@ -411,47 +479,69 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
         }
         if (bulk_cache) ts_wait(smem_u32(cache_bar), 0u, abort_flag, p.status, 0x431u);
 
-        const uint32_t a_addr = tbase + w * WGCOLS + lane_sel, d_addr = a_addr + 32;
-        float acc[MP];
+        const uint32_t a_addr = tbase + w * SB_WGCOLS + lane_sel, d_addr = a_addr + ABUF * 32;
+        SbPair acc[MP / 2];                        // sums of this lane's (row, plane), two activation rows each
 #pragma unroll
-        for (int m = 0; m < MP; ++m) acc[m] = 0.0f;
+        for (int m = 0; m < MP / 2; ++m) acc[m] = SbPair(0.0f, 0.0f);
         const int wpos = nl * S + s;
-        // Sums of one tile's units: planes added by shuffles, every thread of a row's planes keeps the activation rows
-        // m = s (mod SP).  A tile that is all this warpgroup's goes out at once, one that it shares with a neighbour (its first
-        // or its last) to shared memory.
         int tile = t0 + u0 / nkb, have = 0;        // tile of the sums, units of it in them
+        auto settle = [&]() {                      // the next step of counting the pending tile
+            if (pend == 1) {
+                old = sb_arrive(p.counters + ptile * 4 + wl, lane);
+                pend = 2;
+            } else if (pend == 2) {
+                pend = 0;
+                if (__shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<MP, TN>(p, ptile, wl, lane);
+            }
+        };
+        // Sums of one tile's units: planes added across their lanes, after which a lane has the activation rows
+        // m = s NV .. s NV + NV - 1 of its output row.  A tile that is all this warpgroup's goes out at once, one that it
+        // shares with a neighbour (its first or its last) to shared memory.
         auto deposit = [&](bool last) {
-            const bool whole = have == nkb;
-            float* dst = whole ? p.part + ((size_t)chunk * p.NT + tile) * (MP * TN) + nl : res + (size_t)(w * 2 + (last ? 1 : 0)) * (MP * TN) + nl;
-            const int n = tile * TN + nl;
-            unsigned int pm = 0u;                  // activation rows of this chunk with a non-finite value
-            for (int b = 0; whole && b < nkb; ++b)
-                pm |= __ballot_sync(0xffffffffu, lane < MP && reinterpret_cast<const uint4*>(Bs + (size_t)b * BLOB + NJ * 4096)[lane].w != 0u);
-            const float bias = (whole && KC == 1 && p.bias) ? __half2float(p.bias[n]) : 0.0f;
+            float v[MP];
 #pragma unroll
-            for (int m = 0; m < MP; ++m) {
-                float v = acc[m];
-                acc[m] = 0.0f;
-                v += __shfl_xor_sync(0xffffffffu, v, 1);
-                if (SP == 4) v += __shfl_xor_sync(0xffffffffu, v, 2);
-                if ((m % SP) == s) {
-                    if (!whole) {
-                        dst[m * TN] = v;
-                    } else {
-                        if ((pm >> m) & 1u) v = __int_as_float(0x7fc00000);
-                        if (KC > 1) __stcg(dst + m * TN, v);
-                        else if (m < M) p.y[(size_t)m * N + n] = __float2half_rn(v + bias);
-                    }
+            for (int m = 0; m < MP / 2; ++m) acc[m].get(v[2 * m], v[2 * m + 1]), acc[m] = SbPair(0.0f, 0.0f);
+#pragma unroll
+            for (int o = SP / 2, n2 = MP / 2; o; o >>= 1, n2 >>= 1) {
+                const bool up = (s & o) != 0;
+#pragma unroll
+                for (int i = 0; i < n2; ++i) {
+                    const float keep = up ? v[i + n2] : v[i], send = up ? v[i] : v[i + n2];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            if (have != nkb) {
+                float* dst = res + (size_t)(w * 2 + (last ? 1 : 0)) * (MP * TN) + nl;
+#pragma unroll
+                for (int e = 0; e < NV; ++e) dst[(s * NV + e) * TN] = v[e];
+            } else {
+                const unsigned int pm = *poison_s;
+#pragma unroll
+                for (int e = 0; e < NV; ++e)
+                    if ((pm >> (s * NV + e)) & 1u) v[e] = __int_as_float(0x7fc00000);
+                if (KC > 1) {
+                    while (pend) settle();         // (one k block per chunk: a tile every unit)
+                    float* dst = p.part + ((size_t)chunk * p.NT + tile) * (MP * TN) + nl;
+#pragma unroll
+                    for (int e = 0; e < NV; ++e)
+                        if (s * NV + e < M) __stcg(dst + (s * NV + e) * TN, v[e]);
+                    pend = 1, ptile = tile;
+                } else {
+                    const int n = tile * TN + nl;
+                    const float bias = p.bias ? __half2float(p.bias[n]) : 0.0f;
+#pragma unroll
+                    for (int e = 0; e < NV; ++e)
+                        if (s * NV + e < M) p.y[(size_t)(s * NV + e) * N + n] = __float2half_rn(v[e] + bias);
                 }
             }
             have = 0;
             ++tile;
         };
-        uint32_t wv[8];
-        float cf[NSUB], cp[NSUB];                  // coefficients of the unit in A, of the unit in D
+        uint32_t wv[8];                            // packed words and coefficients of the unit to be expanded next
+        float cf[NSUB], c1[NSUB], c0[NSUB];        // ... of the expanded one, and of the one whose sums are read
         int aslot = 0;
         uint32_t apar = 0u;
-        auto fetch = [&]() {                       // the next unit's packed words and coefficients
+        auto fetch = [&]() {
             ts_wait(full_ws + (uint32_t)aslot * 8u, apar, abort_flag, p.status, 0x432u);
             const unsigned char* stg = ring_w + (size_t)aslot * SB_ASTAGE;
             const uint32_t* wsrc = reinterpret_cast<const uint32_t*>(stg) + wpos;
@@ -474,60 +564,77 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                 apar ^= 1u;
             }
         };
-        if (n_w > 0) fetch();
-        int kl = u0 % nkb;                         // k block of unit i - 1
+        // packed words of this thread's row -> 32 words of 4-bit elements {0, 1 | 1 | 2 | 2}
+        auto expand = [&](int buf) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const uint32_t w0 = wv[2 * h], w1 = wv[2 * h + 1];
+                ts_st8(a_addr + buf * 32 + h * 8, (w0 << 1) & 0x22222222u, w0 & 0x22222222u, w0 & 0x44444444u, (w0 >> 1) & 0x44444444u,
+                       (w1 << 1) & 0x22222222u, w1 & 0x22222222u, w1 & 0x44444444u, (w1 >> 1) & 0x44444444u);
+            }
+        };
+        if (n_w > 0) {
+            fetch();
+            expand(0);
+#pragma unroll
+            for (int sub = 0; sub < NSUB; ++sub) c1[sub] = cf[sub];
+            if (n_w > 1) fetch();
+            ts_wait_st();
+            ts_fence_before();
+            ts_bar_arrive(1 + w, 160);             // releases the MMAs of unit 0
+        }
+        int kl = u0 % nkb;                         // k block of unit i
 #pragma unroll 1
-        for (int i = 0; i <= n_w; ++i) {
+        for (int i = 0; i < n_w; ++i) {
+            const bool more = i + 1 < n_w;
+            auto next = [&]() {                    // unit i + 1 into A, unit i + 2 out of shared memory
+                if (more) {
+                    expand(ABUF == 2 ? (i + 1) & 1 : 0);
+#pragma unroll
+                    for (int sub = 0; sub < NSUB; ++sub) c1[sub] = cf[sub];
+                    if (i + 2 < n_w) fetch();
+                }
+            };
+#pragma unroll
+            for (int sub = 0; sub < NSUB; ++sub) c0[sub] = c1[sub];
+            if (ABUF == 2) next();
+            ts_wait(mbar, (uint32_t)(i & 1), abort_flag, p.status, 0x434u);
+            ts_fence_after();
             uint32_t d[NSUB][4][8];
-            if (i > 0) {
-                ts_wait(mbar, (uint32_t)((i - 1) & 1), abort_flag, p.status, 0x434u);
-                ts_fence_after();
 #pragma unroll
-                for (int sub = 0; sub < NSUB; ++sub) {
-                    ts_ld16_issue(d_addr + sub * 32, d[sub][0], d[sub][1]);
-                    ts_ld16_issue(d_addr + sub * 32 + 16, d[sub][2], d[sub][3]);
-                }
+            for (int sub = 0; sub < NSUB; ++sub) {
+                ts_ld16_issue(d_addr + sub * 32, d[sub][0], d[sub][1]);
+                ts_ld16_issue(d_addr + sub * 32 + 16, d[sub][2], d[sub][3]);
             }
-            if (i < n_w) {
-                // packed words of this thread's row -> 32 words of 4-bit elements {0, 1 | 1 | 2 | 2}
+            if (ABUF == 1) next();
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const uint32_t w0 = wv[2 * h], w1 = wv[2 * h + 1];
-                    ts_st8(a_addr + h * 8, (w0 << 1) & 0x22222222u, w0 & 0x22222222u, w0 & 0x44444444u, (w0 >> 1) & 0x44444444u,
-                           (w1 << 1) & 0x22222222u, w1 & 0x22222222u, w1 & 0x44444444u, (w1 >> 1) & 0x44444444u);
-                }
-            }
-            if (i > 0) {
+            for (int sub = 0; sub < NSUB; ++sub)
 #pragma unroll
-                for (int sub = 0; sub < NSUB; ++sub)
-#pragma unroll
-                    for (int g4 = 0; g4 < 4; ++g4) ts_wait_ld(d[sub][g4]);
-            }
-            if (i < n_w) {
+                for (int g4 = 0; g4 < 4; ++g4) ts_wait_ld(d[sub][g4]);
+            if (more) {
                 ts_wait_st();
                 ts_fence_before();
-                ts_bar_arrive(1 + w, 160);         // releases the MMAs of unit i; also: its stage has been read
+                ts_bar_arrive(1 + w, 160);         // releases the MMAs of unit i + 1; also: its stage has been read
             }
-            if (i > 0) {
 #pragma unroll
-                for (int sub = 0; sub < NSUB; ++sub)
+            for (int sub = 0; sub < NSUB; ++sub) {
+                const SbPair cc(c0[sub], c0[sub]);
 #pragma unroll
-                    for (int m = 0; m < MP; ++m) {
-                        float v = __uint_as_float(d[sub][m >> 3][m & 7]);
-                        if (NJ == 3) v += __uint_as_float(d[sub][2 + (m >> 3)][m & 7]);
-                        acc[m] = fmaf(v, cp[sub], acc[m]);
-                    }
-                ++have;
-                if (++kl == nkb || i == n_w) {
-                    kl = 0;
-                    // (a shared tile's sums: the last tile of the warpgroup's range unless the range lies inside one tile)
-                    deposit(i == n_w && tile > t0 + u0 / nkb);
+                for (int m = 0; m < MP; m += 2) {
+                    SbPair v(d[sub][m >> 3][m & 7], d[sub][m >> 3][(m & 7) + 1]);
+                    if (NJ == 3) v = v + SbPair(d[sub][2 + (m >> 3)][m & 7], d[sub][2 + (m >> 3)][(m & 7) + 1]);
+                    acc[m / 2] = v.mul_add(cc, acc[m / 2]);
                 }
             }
-#pragma unroll
-            for (int sub = 0; sub < NSUB; ++sub) cp[sub] = cf[sub];
-            if (i + 1 < n_w) fetch();
+            ++have;
+            if (KC > 1 && pend) settle();
+            if (++kl == nkb || !more) {
+                kl = 0;
+                // (a shared tile's sums: the last tile of the warpgroup's range unless the range lies inside one tile)
+                deposit(!more && tile > t0 + u0 / nkb);
+            }
         }
+        if (KC > 1 && pend == 1) settle();         // counted; the answer is looked at below
     }
     ts_fence_before();
     __syncthreads();
@@ -538,79 +645,38 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
 
     // ------------------------------ tiles shared by warpgroups ------------------------------
     // Tile `tl` of the range has units [tl nkb, (tl + 1) nkb), warpgroup w the units [w U / 4, (w + 1) U / 4); where a boundary
-    // lies inside a tile its warpgroups' sums are added here, in warpgroup order.
-    {
-        int done = -1;
-#pragma unroll 1
-        for (int wb = 1; wb < SB_NWG; ++wb) {
-            const int bd = wb * units / SB_NWG, tl = bd / nkb;
-            if (bd == tl * nkb || tl == done) continue;       // a tile boundary, or the tile has been dealt with
-            done = tl;
-            for (int q = threadIdx.x; q < MP * TN; q += SB_THREADS) {
-                const int m = q / TN, n = (t0 + tl) * TN + q % TN;
+    // lies inside a tile its warpgroups' sums are added here, in warpgroup order, by a warp per quarter of the tile.
+    unsigned int shared_old = 0u;
+    int shared_tile = -1;
+    if (warp < 4 * (SB_NWG - 1)) {
+        constexpr int QR = TN / 4;                 // rows of a quarter
+        const int wb = (warp >> 2) + 1, qt = warp & 3;
+        const int bd = wb * units / SB_NWG, tl = bd / nkb;
+        // (a tile with several boundaries belongs to the first of them)
+        if (bd != tl * nkb && (wb == 1 || (wb - 1) * units / SB_NWG <= tl * nkb)) {
+            const unsigned int pm = *poison_s;
+            for (int q = lane; q < MP * QR; q += 32) {
+                const int m = q / QR, nl = qt * QR + q % QR, n = (t0 + tl) * TN + nl;
+                if (m >= M) break;
                 float v = 0.0f;
 #pragma unroll
                 for (int w = 0; w < SB_NWG; ++w) {
                     const int a = w * units / SB_NWG, b = (w + 1) * units / SB_NWG;
-                    if (a < (tl + 1) * nkb && b > tl * nkb && a < b) v += res[(size_t)(w * 2 + (tl > a / nkb ? 1 : 0)) * (MP * TN) + q];
+                    if (a < (tl + 1) * nkb && b > tl * nkb && a < b) v += res[(size_t)(w * 2 + (tl > a / nkb ? 1 : 0)) * (MP * TN) + m * TN + nl];
                 }
-                bool poison = false;
-                for (int b = 0; b < nkb; ++b) poison |= reinterpret_cast<const uint4*>(Bs + (size_t)b * BLOB + NJ * 4096)[m].w != 0u;
-                if (poison) v = __int_as_float(0x7fc00000);
-                if (KC > 1) __stcg(p.part + ((size_t)chunk * p.NT + t0 + tl) * (MP * TN) + q, v);
-                else if (m < M) p.y[(size_t)m * N + n] = __float2half_rn(v + (p.bias ? __half2float(p.bias[n]) : 0.0f));
+                if ((pm >> m) & 1u) v = __int_as_float(0x7fc00000);
+                if (KC > 1) __stcg(p.part + ((size_t)chunk * p.NT + t0 + tl) * (MP * TN) + m * TN + nl, v);
+                else p.y[(size_t)m * N + n] = __float2half_rn(v + (p.bias ? __half2float(p.bias[n]) : 0.0f));
+            }
+            if (KC > 1) {
+                shared_tile = t0 + tl;
+                shared_old = sb_arrive(p.counters + shared_tile * 4 + qt, lane);
             }
         }
     }
-    // ------------------------------ the chunks' sums ------------------------------
-    if (KC > 1) {
-        __threadfence();                           // this thread's sums, before its CTA's arrival below
-        __syncthreads();
-        // A tile's rows are counted in 2^psh parts; the arrivals of 32 parts are in flight together, then the warp adds the
-        // chunks of those at which it arrived last.
-        const int np = ntc << p.psh, per = (MP * TN) >> p.psh;
-        unsigned int* cnt = p.counters + ((size_t)t0 << p.psh);
-        const size_t plane = (size_t)p.NT * (MP * TN);
-        for (int p0 = warp; p0 < np; p0 += 32 * (SB_THREADS / 32)) {
-            const int mypart = p0 + lane * (SB_THREADS / 32);
-            unsigned int last = 0u;
-            if (mypart < np) {
-                last = atomicAdd(cnt + mypart, 1u) == (unsigned int)(KC - 1) ? 1u : 0u;
-                if (last) cnt[mypart] = 0u;
-            }
-            __syncwarp();
-            unsigned int todo = __ballot_sync(0xffffffffu, last != 0u);
-            if (todo) __threadfence();
-            while (todo) {
-                const int part = p0 + (__ffs((int)todo) - 1) * (SB_THREADS / 32);
-                todo &= todo - 1u;
-                const int tl = part >> p.psh;
-                const float* src = p.part + (size_t)(t0 + tl) * (MP * TN);
-                for (int q = (part & ((1 << p.psh) - 1)) * per + lane, e = q + per - lane; q < e; q += 128) {
-                    float v[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) v[u] = 0.0f;
-                    for (int c = 0; c < KC; c += 2) {          // eight loads in flight
-                        float t[2][4];
-#pragma unroll
-                        for (int h = 0; h < 2; ++h)
-#pragma unroll
-                            for (int u = 0; u < 4; ++u)
-                                t[h][u] = (c + h < KC && q + 32 * u < e && (q + 32 * u) / TN < M) ? __ldcg(src + (size_t)(c + h) * plane + q + 32 * u) : 0.0f;
-#pragma unroll
-                        for (int h = 0; h < 2; ++h)
-#pragma unroll
-                            for (int u = 0; u < 4; ++u) v[u] += t[h][u];
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int qq = q + 32 * u, m = qq / TN, n = (t0 + tl) * TN + qq % TN;
-                        if (qq < e && m < M) p.y[(size_t)m * N + n] = __float2half_rn(v[u] + (p.bias ? __half2float(p.bias[n]) : 0.0f));
-                    }
-                }
-            }
-        }
-    }
+    if (pend == 2 && __shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<MP, TN>(p, ptile, warp & 3, lane);
+    if (shared_tile >= 0 && __shfl_sync(0xffffffffu, shared_old, 0) == (unsigned int)(KC - 1))
+        sb_add_chunks<MP, TN>(p, shared_tile, warp & 3, lane);
     if (threadIdx.x == 0 && *abort_flag) {         // which problem gave up: N, and K / 256 | M | CTA (for the host's message)
         atomicExch(p.status + 2, (unsigned int)p.N);
         atomicExch(p.status + 3, ((unsigned int)p.KB << 16) | ((unsigned int)M << 8) | (blockIdx.x & 0xFFu));
@@ -621,13 +687,13 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
 // host
 // ---------------------------------------------------------------------------------------------
 struct SbPlan {
-    int KB, NT, NJ, KC, GN, cache_in_smem, stages, psh, smem;
+    int KB, NT, NJ, KC, GN, cache_in_smem, stages, smem;
     int off_cache, off_ring, off_res;
     size_t blob_bytes, part_bytes;
 };
 
 static int sb_plan(const PackedW& w, int M, const DeviceInfo& di, SbPlan* pl) {
-    const int TN = ts_tn(w.S), NSUB = 256 / w.G;
+    const int TN = ts_tn(w.S);
     pl->NJ = M <= 16 ? 3 : 6;
     const int MP = pl->NJ == 3 ? 16 : 32;
     pl->KB = w.K / 256;
@@ -635,16 +701,14 @@ static int sb_plan(const PackedW& w, int M, const DeviceInfo& di, SbPlan* pl) {
     if (pl->KB < 1 || pl->NT < 1) return SBVR_ERR_UNSUPPORTED;
     // Chunks as large as shared memory holds; smaller ones while less than two thirds of the SMs would have work and a
     // warpgroup more than one unit.
-    pl->KC = (pl->KB + sb_chunk(NSUB, pl->NJ) - 1) / sb_chunk(NSUB, pl->NJ);
+    pl->KC = (pl->KB + sb_chunk(pl->NJ) - 1) / sb_chunk(pl->NJ);
     auto groups = [&](int kc) { const int g = di.sm_count / kc; return g < 1 ? 1 : (g < pl->NT ? g : pl->NT); };
     while (groups(pl->KC) * pl->KC * 3 <= di.sm_count * 2 && pl->KC * 2 <= pl->KB && pl->KC * 2 <= 16 &&
            (pl->NT + groups(pl->KC) - 1) / groups(pl->KC) * (pl->KB / pl->KC) > SB_NWG)
         pl->KC *= 2;
     pl->GN = groups(pl->KC);
     const int nkb = (pl->KB + pl->KC - 1) / pl->KC;
-    // quarter tiles where the workspace has that many counters, else (very wide layers) whole tiles
-    pl->psh = pl->NT * 4 <= SBVR_WS_COUNTERS ? 2 : 0;
-    if (pl->KC > 1 && pl->NT > SBVR_WS_COUNTERS) return SBVR_ERR_UNSUPPORTED;
+    if (pl->KC > 1 && (size_t)pl->NT * 16 > SBVR_WS_XCHG_BYTES) return SBVR_ERR_UNSUPPORTED;     // arrival counters
     pl->blob_bytes = ((size_t)pl->KB * sb_blob(pl->NJ) + 255) / 256 * 256;
     pl->part_bytes = pl->KC > 1 ? (size_t)pl->KC * pl->NT * MP * TN * 4 : 0;
     const int cache_bytes = w.idx_bytes ? ts_round_up(w.C * w.S * 2, 16) : 0;
@@ -711,7 +775,7 @@ static int sb_launch_g(const CUtensorMap& tm, const SbParams& p, int G, int NJ, 
     return NJ == 3 ? sb_launch_idx<S, 1, 3>(tm, p, idxb, grid, smem, st) : sb_launch_idx<S, 1, 6>(tm, p, idxb, grid, smem, st);
 }
 
-// `counters` (zero between calls: the kernel leaves them zero) and `scratch` (256-byte aligned,
+// `counters` (SBVR_WS_XCHG_BYTES, zero between calls: the kernel leaves them zero) and `scratch` (256-byte aligned,
 // linear_sb_workspace_bytes long: digit blob and the chunks' sums) are the caller's.
 int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, int device, unsigned int* status,
                      unsigned int* counters, char* scratch, size_t scratch_bytes, cudaStream_t st, const XOp* xop) {
@@ -734,14 +798,14 @@ int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __ha
     q.x = x, q.xb = reinterpret_cast<unsigned char*>(scratch), q.M = M, q.K = w.K;
     rc = xop_check(xop, x, M, w.K, &q.x_op, &q.delta, &q.norm_w, &q.h_out, &q.eps);
     if (rc) return rc;
-    if (pl.NJ == 3) SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel<3>, dim3(pl.KB, 4), dim3(128), 0, st, q));
-    else SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel<6>, dim3(pl.KB, 8), dim3(128), 0, st, q));
+    if (pl.NJ == 3) SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel<3>, dim3(pl.KB, 8), dim3(64), 0, st, q));
+    else SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel<6>, dim3(pl.KB, 16), dim3(64), 0, st, q));
     SbParams p;
     p.xb = q.xb;
     p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status, p.counters = counters;
     p.part = reinterpret_cast<float*>(scratch + pl.blob_bytes);
     p.M = M, p.N = w.N, p.K = w.K, p.KB = pl.KB, p.NT = pl.NT, p.C = w.C, p.KC = pl.KC, p.GN = pl.GN;
-    p.cache_in_smem = pl.cache_in_smem, p.stages = pl.stages, p.psh = pl.psh;
+    p.cache_in_smem = pl.cache_in_smem, p.stages = pl.stages;
     p.off_cache = pl.off_cache, p.off_ring = pl.off_ring, p.off_res = pl.off_res;
     const int grid = pl.GN * pl.KC;
     switch (w.S) {
