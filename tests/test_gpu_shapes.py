@@ -120,3 +120,41 @@ def test_search_kernel_equals_the_tensor_operations(S, extended):
         mse[i] = best
         _lib.check(_lib.lib.sbvr_encode_advance(ctypes.byref(w), st))
         assert res.status == (1 if extended else 0)            # (a warm-up step looks at no stored line)
+
+
+@pytest.mark.parametrize("N,K,G", [(32, 1, 32), (96, 77, 32), (256, 255, 256), (512, 3001, 128), (1024, 5000, 256)])
+@pytest.mark.parametrize("S", [2, 3, 4])
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9])
+def test_transposed_layout_ragged(N, K, G, S, M):
+    """Group lengths down to one word row, odd input counts, every number of column tiles; activations over six decades.  One
+    fp16 rounding of the result (2^-11) and 2^-23 of the largest product."""
+    from sbvr import sbvr_cuda
+    p = O.make_packed(K, N, S, G=G, mode="u8", C=200, seed=N + K + S)
+    rng = np.random.default_rng(M)
+    x = (rng.standard_normal((M, K)) * 10.0 ** rng.uniform(-4, 2, (M, 1))).astype(np.float16)
+    bias = rng.standard_normal(N).astype(np.float16)
+    f = lambda a: torch.from_numpy(a).cuda()
+    y = sbvr_cuda._sbvr_row_deq_mm_T(f(x), f(p["bvr"].view(np.int32)), f(p["coeff_idx"]), f(p["coeff"]), f(bias))
+    ref = O.linear_t_f64(x, p["bvr"], p["coeff_idx"], p["coeff"], bias, G=G)
+    err = np.abs(h2n(y).astype(np.float64) - ref).max(1) / np.abs(ref).max(1)
+    assert err.max() <= 1e-3, err
+    if M > 1:                                      # a non-finite activation stays in its row
+        x[1, K // 2] = np.inf
+        z = h2n(sbvr_cuda._sbvr_row_deq_mm_T(f(x), f(p["bvr"].view(np.int32)), f(p["coeff_idx"]), f(p["coeff"]), f(bias)))
+        assert np.array_equal(z[0], h2n(y)[0]) and not np.isfinite(z[1]).any()
+    check_status()
+
+
+@pytest.mark.parametrize("N", [3, 64, 333])
+@pytest.mark.parametrize("K", [256, 768, 4352])
+@pytest.mark.parametrize("LS,RS", [(2, 3), (3, 2), (4, 4), (2, 4)])
+@pytest.mark.parametrize("M", [1, 2, 5, 17])
+def test_product_of_two_encodings_edges(N, K, LS, RS, M):
+    """Fewer groups than warps, rows that do not fill a tile, several passes over the activation rows; exact counts and fp32
+    sums, one fp16 rounding (2^-11)."""
+    import sbvr
+    pl = O.make_packed(M, K, LS, G=256, mode="u8", seed=M + LS)
+    pr = O.make_packed(N, K, RS, G=256, mode="u16", C=300, seed=N + RS)
+    y = h2n(sbvr.mm_T(to_sbvr(pl), to_sbvr(pr))).astype(np.float64)
+    ref = O.popc_mm_f64(pl["bvr"], pl["coeff_idx"], pl["coeff"], pr["bvr"], pr["coeff_idx"], pr["coeff"], None)
+    assert np.abs(y - ref).max() / np.abs(ref).max() <= 1e-3
