@@ -243,8 +243,9 @@ SBVR_API int sbvr_rope_append_f16(void* qkv, const int* positions, const float* 
 /* out[token][head][:] = softmax(q . K^T * scale) . V over cache positions 0 .. positions[token] of the token's
  * sequence, grouped-query (n_heads % n_kv == 0, ratio 1, 2, 4 or 8), head_dim 128.  Serves decode (one token per
  * sequence) and causal prefill (every token attends up to itself; its k, v must be in the cache already).
- * nsplit > 1 splits the positions over CTAs (decode at long context), a second small launch merges the splits; it
- * needs `scratch` of tokens * n_heads * nsplit * 130 floats.  repeat_kv + eager_attention_forward (models/sbvr_llama.py:243-278). */
+ * nsplit > 1 splits the positions over a cluster of up to 16 CTAs (decode at long context); `scratch` of
+ * tokens * n_heads * nsplit * 130 floats is asked for then, as before, but no longer used.
+ * repeat_kv + eager_attention_forward (models/sbvr_llama.py:243-278). */
 SBVR_API int sbvr_attention_f16(const void* qkv, const void* kcache, const void* vcache, const int* positions,
                                 void* out, float* scratch, int tokens, int tokens_per_seq, int n_heads, int n_kv,
                                 int head_dim, int max_ctx, float scale, int nsplit, sbvr_stream_t stream);
@@ -271,7 +272,8 @@ SBVR_API int sbvr_argmax_f16(const void* logits, int* out, float* scratch, int r
 /* ---- decode linears with the preceding element-wise op folded in ---------------------------------------------
  * The decode GEMV (algo 2 of sbvr_linear_f16: M <= 4, N % 32 == 0, K % 256 == 0) turns the activation row into
  * block-fixed-point digits in a small kernel of its own before the product; the op in front of the linear is applied
- * there instead of in a launch of its own:
+ * there instead of in a launch of its own.  So does the small-batch kernel (algo 4) for 5 .. 16 rows, and for fewer where the
+ * GEMV does not apply (needs a workspace of sbvr_workspace_bytes(...); not with SBVR_XOP_DIGITS):
  *   SBVR_XOP_SILU_MUL     x = fp16(silu(g)) * u, `x` pointing at rows [g (K) | u (K)] of pitch 2K
  *                         (LlamaMLP.forward, models/sbvr_llama.py:238-240, in front of down_proj)
  *   SBVR_XOP_ADD_RMSNORM  x = norm_weight * fp16((h + delta) * rsqrt(mean((h + delta)^2) + eps)) with h = `x`
@@ -283,7 +285,7 @@ SBVR_API int sbvr_argmax_f16(const void* logits, int* out, float* scratch, int r
  *                         RMSNorm calls below with emit_digits = 1 for the same M and K.  Saves the quantiser launch of
  *                         rows longer than 4096.  Group length 256 only.
  * Same rounding as sbvr_silu_mul_f16 / sbvr_add_rmsnorm_f16 followed by sbvr_linear_f16.  Returns
- * SBVR_ERR_UNSUPPORTED where the decode GEMV does not apply (the caller then runs the separate kernels). */
+ * SBVR_ERR_UNSUPPORTED where neither applies (the caller then runs the separate kernels). */
 enum { SBVR_XOP_NONE = 0, SBVR_XOP_SILU_MUL = 1, SBVR_XOP_ADD_RMSNORM = 2, SBVR_XOP_DIGITS = 3 };
 SBVR_API int sbvr_linear_fused_f16(int x_op, const void* x, const void* delta, const void* norm_weight, void* h_out,
                                    float eps, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff,

@@ -129,7 +129,11 @@ int sbvr_workspace_create(sbvr_workspace_t** out, int device, size_t bytes) {
     ws->base = nullptr;
     ws->pinned_status = nullptr;
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&ws->base), bytes);
+    // The clearing runs on the legacy default stream, which streams created as non-blocking do not wait for: without the
+    // synchronisation a first kernel on such a stream could leave tags and counts that the clearing then erased, and its
+    // waits ran out.
     if (e == cudaSuccess) e = cudaMemset(ws->base, 0, fixed);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);
     if (e == cudaSuccess) e = cudaMallocHost(&ws->pinned_status, 16);
     if (e != cudaSuccess) {
         g_last_cuda_error = (int)e;
@@ -302,7 +306,13 @@ int sbvr_linear_fused_f16(int x_op, const void* x, const void* delta, const void
     xop.op = x_op;
     xop.delta = reinterpret_cast<const __half*>(delta), xop.norm_w = reinterpret_cast<const __half*>(norm_weight);
     xop.h_out = reinterpret_cast<__half*>(h_out), xop.eps = eps;
-    if (!linear_tcs_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
+    if (!linear_tcs_supported(w, M)) {             // more rows (or digits that do not fit the GEMV): the small-batch kernel
+        if (x_op == SBVR_XOP_DIGITS || M > 16 || !linear_sb_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
+        if (linear_sb_workspace_bytes(w, M, di) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
+        return launch_linear_sb(reinterpret_cast<const __half*>(x), w, reinterpret_cast<const __half*>(bias),
+                                reinterpret_cast<__half*>(y), M, ws->device, ws->status, reinterpret_cast<unsigned int*>(ws->xchg),
+                                ws->dyn, ws->dyn_bytes, reinterpret_cast<cudaStream_t>(stream), &xop);
+    }
     if (linear_tcs_workspace_bytes(w, M, di.sm_count) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
     return launch_linear_tcs(reinterpret_cast<const __half*>(x), w, reinterpret_cast<const __half*>(bias),
                              reinterpret_cast<__half*>(y), M, ws->device, ws->status, ws->xchg, ws->dyn,

@@ -6,9 +6,13 @@
 // to fp16; the rotary products and their sum are separate fp16 operations; SiLU is rounded to fp16 before the
 // multiplication.  Attention keeps scores and probabilities in fp32 (the reference rounds the scores and the
 // probabilities to fp16), which is inside the 1e-2 tolerance of the layer outputs.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace sbvr {
+
+namespace cg = cooperative_groups;
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -122,207 +126,220 @@ __global__ void __launch_bounds__(256) rope_append_kernel(__half* __restrict__ q
 
 // ---------------------------------------------------------------------------------------------
 // attention of one query token over cache positions [0, pos]; head_dim 128; grouped-query: the R = n_heads / n_kv
-// query heads of a KV head are served together.   grid (tokens * n_kv, nsplit), 128 threads
-//   nsplit == 1: writes out[t, head, :] fp16.   nsplit > 1: writes (max, sum, unnormalised acc) per split.
+// query heads of a KV head are served together.  grid tokens * n_kv * nsplit, 128 threads; the nsplit CTAs of a (token, KV
+// head) are a cluster that splits the positions and merges (max, sum, unnormalised sums) through distributed shared memory.
+//
+// Positions are taken AT_TILE at a time, K and V rows through cp.async, double buffered.  Scores: eight lanes per position,
+// sixteen dims each (two 16-byte chunks 128 bytes apart: no bank conflicts).  Weights: a warp per head, running maximum.
+// P.V: a thread owns two dims and half of a tile's positions.  It is a chain of latencies (position, rows, three barriers
+// per tile, the merge); with a lane per position, a quarter of the positions per warp and a second kernel for the merge it took
+// 10.8 + 3.2 us at 576 positions, 32 query heads, 8 KV heads, one token.
 // ---------------------------------------------------------------------------------------------
 constexpr int AT_D = 128;
-constexpr int AT_RMAX = 8;
+constexpr int AT_TILE = 64;
+constexpr int AT_MAX_CLUSTER = 16;
+constexpr int AT_SMEM = 4 * AT_TILE * AT_D * 2;                // K and V tiles x 2
 
-// `inv_freq` != NULL (decode, one token per sequence): the rotary embedding is applied here -- q on its way into shared
-// memory; the token's own k by the CTA whose positions include it, which also appends k and v to the cache and
-// takes them from shared memory (the cache rows are read through the read-only path).
+__device__ __forceinline__ void at_cp16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// `inv_freq` != NULL (decode, one token per sequence): the rotary embedding is applied here -- q on its way into registers;
+// the token's own k by the CTA whose positions include it, which also appends k and v to the cache and puts them into its tile
+// itself.
 template <int R>
 __global__ void __launch_bounds__(128) attention_kernel(const __half* __restrict__ qkv, __half* kcache, __half* vcache,
                                                         const int* __restrict__ positions, __half* __restrict__ out,
-                                                        float* __restrict__ part, int tokens_per_seq, int n_heads, int n_kv, int max_ctx, float scale,
+                                                        int tokens_per_seq, int n_heads, int n_kv, int max_ctx, float scale,
                                                         int nsplit, const float* __restrict__ inv_freq, float attn_scaling) {
-    __shared__ float qs[R][AT_D];
-    __shared__ float wm[4][R], wl[4][R];
-    __shared__ float wacc[4][R][AT_D];
-    __shared__ __half cs_s[2][AT_D / 2];
+    constexpr int RH = R < 4 ? R : 4;              // heads whose queries a thread holds at a time
+    extern __shared__ __align__(128) unsigned char at_smem[];
+    __shared__ __align__(16) __half qs[R][AT_D];
     __shared__ __align__(16) __half knew[AT_D], vnew[AT_D];
+    __shared__ __half cs_s[2][AT_D / 2];
+    __shared__ __align__(16) float sc[AT_TILE][R];              // scores, then weights
+    __shared__ float corr_s[R];
+    __shared__ float wm[R], wl[R];                              // the CTA's maximum and sum
+    __shared__ __align__(16) float wacc[2][R][AT_D];            // per half of the threads; [0]: their sum, read by the cluster
     pdl_launch_dependents();
     pdl_wait();
-    const int t = blockIdx.x / n_kv, kvh = blockIdx.x - t * n_kv;
-    const int split = blockIdx.y;
+    const int unit = (int)blockIdx.x / nsplit, split = (int)blockIdx.x - unit * nsplit;
+    const int t = unit / n_kv, kvh = unit - t * n_kv;
     const int seq = t / tokens_per_seq;
     const int pos = positions[t];
     const int ctx = min(pos + 1, max_ctx);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const __half* tok = qkv + (size_t)t * (n_heads + 2 * n_kv) * AT_D;
     const __half* qrow = tok + (size_t)kvh * R * AT_D;
     const int per = (ctx + nsplit - 1) / nsplit;
-    const int p0 = split * per, p1 = min(ctx, p0 + per);
+    const int p0 = min(ctx, split * per), p1 = min(ctx, p0 + per);
     __half* kb = kcache + ((size_t)seq * n_kv + kvh) * max_ctx * AT_D;
     __half* vb = vcache + ((size_t)seq * n_kv + kvh) * max_ctx * AT_D;
     const bool rope = inv_freq != nullptr;
-    // position of the row that comes from shared memory instead of the cache (-1: none)
+    // position whose rows do not come from the cache (-1: none)
     const int own = (rope && pos < max_ctx && pos >= p0 && pos < p1) ? pos : -1;
+    const uint32_t ks0 = smem_u32(at_smem), vs0 = ks0 + 2 * AT_TILE * AT_D * 2;
+    auto load_tile = [&](int base, int buf) {
+        const int n = min(AT_TILE, p1 - base);
+        for (int c = tid; c < n * 16; c += 128) {
+            const int row = c >> 4, ch = c & 15;
+            if (base + row == own) continue;
+            const size_t src = (size_t)(base + row) * AT_D + ch * 8;
+            const uint32_t dst = (uint32_t)(buf * AT_TILE * AT_D * 2 + row * 256 + ch * 16);
+            at_cp16(ks0 + dst, kb + src);
+            at_cp16(vs0 + dst, vb + src);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (p0 < p1) load_tile(p0, 0);
     if (rope) {
-        if (threadIdx.x < AT_D / 2) {
-            const float ang = (float)pos * inv_freq[threadIdx.x];
-            cs_s[0][threadIdx.x] = __float2half_rn(cosf(ang) * attn_scaling);
-            cs_s[1][threadIdx.x] = __float2half_rn(sinf(ang) * attn_scaling);
+        if (tid < AT_D / 2) {
+            const float ang = (float)pos * inv_freq[tid];
+            cs_s[0][tid] = __float2half_rn(cosf(ang) * attn_scaling);
+            cs_s[1][tid] = __float2half_rn(sinf(ang) * attn_scaling);
         }
         __syncthreads();
-        for (int i = threadIdx.x; i < R * AT_D; i += 128) {
-            const int r = i / AT_D, dd = i % AT_D, i2 = dd % (AT_D / 2);
+        auto rot = [&](const __half* row, int dd) {            // products and sum are separate fp16 operations
+            const int i2 = dd % (AT_D / 2);
             const __half c = cs_s[0][i2], sn = cs_s[1][i2];
-            const __half x = qrow[i];
-            const __half y = (dd < AT_D / 2) ? __hneg(qrow[r * AT_D + dd + AT_D / 2]) : qrow[r * AT_D + dd - AT_D / 2];
-            qs[r][dd] = __half2float(__hadd(__hmul(x, c), __hmul(y, sn))) * scale;
-        }
+            const __half y = (dd < AT_D / 2) ? __hneg(row[dd + AT_D / 2]) : row[dd - AT_D / 2];
+            return __hadd(__hmul(row[dd], c), __hmul(y, sn));
+        };
+#pragma unroll
+        for (int r = 0; r < R; ++r) qs[r][tid] = rot(qrow + r * AT_D, tid);
         if (own >= 0) {                            // this CTA holds the new token's position
-            const __half* krow = tok + (size_t)(n_heads + kvh) * AT_D;
-            const __half* vrow = tok + (size_t)(n_heads + n_kv + kvh) * AT_D;
-            const int dd = threadIdx.x, i2 = dd % (AT_D / 2);
-            const __half c = cs_s[0][i2], sn = cs_s[1][i2];
-            const __half y = (dd < AT_D / 2) ? __hneg(krow[dd + AT_D / 2]) : krow[dd - AT_D / 2];
-            const __half kr1 = __hadd(__hmul(krow[dd], c), __hmul(y, sn));
-            knew[dd] = kr1, vnew[dd] = vrow[dd];
-            kb[(size_t)pos * AT_D + dd] = kr1;
-            vb[(size_t)pos * AT_D + dd] = vrow[dd];
+            const __half kr = rot(tok + (size_t)(n_heads + kvh) * AT_D, tid);
+            const __half vr = tok[(size_t)(n_heads + n_kv + kvh) * AT_D + tid];
+            knew[tid] = kr, vnew[tid] = vr;
+            kb[(size_t)pos * AT_D + tid] = kr;
+            vb[(size_t)pos * AT_D + tid] = vr;
         }
     } else {
-        for (int i = threadIdx.x; i < R * AT_D; i += 128) qs[i / AT_D][i % AT_D] = __half2float(qrow[i]) * scale;
+#pragma unroll
+        for (int r = 0; r < R; ++r) qs[r][tid] = qrow[r * AT_D + tid];
     }
-    __syncthreads();
+    if (tid < R) wm[tid] = -INFINITY, wl[tid] = 0.0f;
 
-    float m[R], l[R], acc[R][4];
+    const int sub = lane & 7;
+    const int d2 = tid & 63, hf = tid >> 6;
+    float acc[R][2];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        m[r] = -INFINITY, l[r] = 0.0f;
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[r][e] = 0.0f;
-    }
-    // The CTA's positions are cut into four contiguous quarters, one per warp; a warp takes up to 32 consecutive
-    // positions at a time: lane <-> position for the scores, lane <-> 4 dims for P.V.
-    const int quarter = (p1 - p0 + 3) / 4;
-    const int w0 = min(p1, p0 + warp * quarter), w1 = min(p1, w0 + quarter);
-    for (int base = w0; base < w1; base += 32) {
-        const int p = base + lane;
-        const int p1 = w1;                         // this warp's end (shadows the CTA's)
-        float sc[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) sc[r] = 0.0f;
-        if (p < p1) {
-            const uint4* kr = reinterpret_cast<const uint4*>(kb + (size_t)p * AT_D);
-            const uint4* ks = reinterpret_cast<const uint4*>(knew);
-#pragma unroll
-            for (int c = 0; c < AT_D / 8; ++c) {
-                const uint4 kv = (p == own) ? ks[c] : __ldg(kr + c);
-                const __half2* kh = reinterpret_cast<const __half2*>(&kv);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float2 f = __half22float2(kh[e]);
-#pragma unroll
-                    for (int r = 0; r < R; ++r) sc[r] += f.x * qs[r][c * 8 + 2 * e] + f.y * qs[r][c * 8 + 2 * e + 1];
-                }
-            }
+    for (int r = 0; r < R; ++r) acc[r][0] = acc[r][1] = 0.0f;
+    int buf = 0;
+#pragma unroll 1
+    for (int base = p0; base < p1; base += AT_TILE, buf ^= 1) {
+        const int n = min(AT_TILE, p1 - base);
+        if (base + AT_TILE < p1) {
+            load_tile(base + AT_TILE, buf ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
         } else {
-#pragma unroll
-            for (int r = 0; r < R; ++r) sc[r] = -INFINITY;
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
-        // online softmax: new running maximum per head, rescale, then this chunk's weights
-        float w[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            float cm = sc[r];
-#pragma unroll
-            for (int o = 16; o; o >>= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, o));
-            const float nm = fmaxf(m[r], cm);
-            const float corr = (m[r] == -INFINITY) ? 0.0f : __expf(m[r] - nm);
-            w[r] = (p < p1) ? __expf(sc[r] - nm) : 0.0f;
-            l[r] = l[r] * corr + warp_sum(w[r]);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[r][e] *= corr;
-            m[r] = nm;
+        unsigned char* kt = at_smem + buf * AT_TILE * AT_D * 2;
+        unsigned char* vt = kt + 2 * AT_TILE * AT_D * 2;
+        if (own >= base && own < base + n) {
+            reinterpret_cast<__half*>(kt + (own - base) * 256)[tid] = knew[tid];       // (written by this thread)
+            reinterpret_cast<__half*>(vt + (own - base) * 256)[tid] = vnew[tid];
         }
-        const int np = min(32, p1 - base);
-        for (int j0 = 0; j0 < np; j0 += 8) {       // eight V rows in flight; rows past the end carry weight 0
-            uint2 vv[8];
+        __syncthreads();                           // tile and queries are in place
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                vv[u] = (base + j0 + u == own)
-                            ? reinterpret_cast<const uint2*>(vnew)[lane]
-                            : __ldg(reinterpret_cast<const uint2*>(vb + (size_t)min(base + j0 + u, max_ctx - 1) * AT_D) + lane);
+        for (int r0 = 0; r0 < R; r0 += RH) {
+            float q[RH][16];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const __half2* vh = reinterpret_cast<const __half2*>(&vv[u]);
-                const float2 f0 = __half22float2(vh[0]), f1 = __half22float2(vh[1]);
+            for (int r = 0; r < RH; ++r)
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const float wj = __shfl_sync(0xffffffffu, w[r], j0 + u);
-                    acc[r][0] += wj * f0.x, acc[r][1] += wj * f0.y, acc[r][2] += wj * f1.x, acc[r][3] += wj * f1.y;
+                for (int c = 0; c < 2; ++c) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(&qs[r0 + r][(sub + 8 * c) * 8]);
+                    const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 f = __half22float2(h[e]);
+                        q[r][c * 8 + 2 * e] = f.x, q[r][c * 8 + 2 * e + 1] = f.y;
+                    }
+                }
+            for (int pb = warp * 4; pb < n; pb += 16) {
+                const int p = pb + (lane >> 3), pr = min(p, n - 1);           // (positions past the end are dropped)
+                float s[RH];
+#pragma unroll
+                for (int r = 0; r < RH; ++r) s[r] = 0.0f;
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const uint4 v = *reinterpret_cast<const uint4*>(kt + pr * 256 + (sub + 8 * c) * 16);
+                    const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float2 f = __half22float2(h[e]);
+#pragma unroll
+                        for (int r = 0; r < RH; ++r) s[r] += f.x * q[r][c * 8 + 2 * e] + f.y * q[r][c * 8 + 2 * e + 1];
+                    }
+                }
+#pragma unroll
+                for (int r = 0; r < RH; ++r) {
+#pragma unroll
+                    for (int o = 4; o; o >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+                    if (sub == r && p < n) sc[p][r0 + r] = s[r] * scale;
                 }
             }
         }
+        __syncthreads();                           // scores
+        for (int r = warp; r < R; r += 4) {
+            const float m0 = wm[r];
+            float a = (lane < n) ? sc[lane][r] : -INFINITY, c = (lane + 32 < n) ? sc[lane + 32][r] : -INFINITY;
+            float m = fmaxf(a, c);
+#pragma unroll
+            for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            m = fmaxf(m, m0);
+            const float corr = (m0 == -INFINITY) ? 0.0f : __expf(m0 - m);
+            a = (lane < n) ? __expf(a - m) : 0.0f, c = (lane + 32 < n) ? __expf(c - m) : 0.0f;
+            sc[lane][r] = a, sc[lane + 32][r] = c;
+            const float l = warp_sum(a + c);
+            __syncwarp();
+            if (lane == 0) wm[r] = m, wl[r] = wl[r] * corr + l, corr_s[r] = corr;
+        }
+        __syncthreads();                           // weights
+#pragma unroll
+        for (int r = 0; r < R; ++r) acc[r][0] *= corr_s[r], acc[r][1] *= corr_s[r];
+        const int a1 = min(n, (hf + 1) * (AT_TILE / 2));
+#pragma unroll 8
+        for (int p = hf * (AT_TILE / 2); p < a1; ++p) {
+            const float2 v = __half22float2(*reinterpret_cast<const __half2*>(vt + p * 256 + d2 * 4));
+#pragma unroll
+            for (int r = 0; r < R; ++r) acc[r][0] += sc[p][r] * v.x, acc[r][1] += sc[p][r] * v.y;
+        }
+        __syncthreads();                           // tile and weights may be overwritten
     }
-    // merge the four warps
+#pragma unroll
+    for (int r = 0; r < R; ++r) *reinterpret_cast<float2*>(&wacc[hf][r][d2 * 2]) = make_float2(acc[r][0], acc[r][1]);
+    __syncthreads();
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        if (lane == 0) wm[warp][r] = m[r], wl[warp][r] = l[r];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) wacc[warp][r][lane * 4 + e] = acc[r][e];
+        const float v = wacc[0][r][tid] + wacc[1][r][tid];
+        if (nsplit == 1) out[((size_t)t * n_heads + kvh * R + r) * AT_D + tid] = __float2half_rn(wl[r] > 0.0f ? v / wl[r] : 0.0f);
+        else wacc[0][r][tid] = v;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < R * AT_D; i += 128) {
+    if (nsplit == 1) return;
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    // every CTA of the cluster finishes its share of the (head, dim) pairs, the splits in order
+    for (int i = split * 128 + tid; i < R * AT_D; i += nsplit * 128) {
         const int r = i / AT_D, dd = i % AT_D;
-        float gm = -INFINITY;
+        float mv[AT_MAX_CLUSTER], gm = -INFINITY;
 #pragma unroll
-        for (int w4 = 0; w4 < 4; ++w4) gm = fmaxf(gm, wm[w4][r]);
+        for (int k = 0; k < AT_MAX_CLUSTER; ++k) {
+            mv[k] = (k < nsplit) ? *cluster.map_shared_rank(&wm[r], k) : -INFINITY;
+            gm = fmaxf(gm, mv[k]);
+        }
         float gl = 0.0f, ga = 0.0f;
 #pragma unroll
-        for (int w4 = 0; w4 < 4; ++w4) {
-            const float c = (wm[w4][r] == -INFINITY) ? 0.0f : __expf(wm[w4][r] - gm);
-            gl += wl[w4][r] * c;
-            ga += wacc[w4][r][dd] * c;
+        for (int k = 0; k < AT_MAX_CLUSTER; ++k) {
+            if (k >= nsplit) break;
+            const float c = (mv[k] == -INFINITY) ? 0.0f : __expf(mv[k] - gm);
+            gl += *cluster.map_shared_rank(&wl[r], k) * c;
+            ga += *cluster.map_shared_rank(&wacc[0][r][dd], k) * c;
         }
-        const int head = kvh * R + r;
-        if (nsplit == 1) {
-            out[((size_t)t * n_heads + head) * AT_D + dd] = __float2half_rn(gl > 0.0f ? ga / gl : 0.0f);
-        } else {
-            float* pp = part + (((size_t)t * n_heads + head) * nsplit + split) * (AT_D + 2);
-            pp[2 + dd] = ga;
-            if (dd == 0) pp[0] = gm, pp[1] = gl;
-        }
+        out[((size_t)t * n_heads + kvh * R + r) * AT_D + dd] = __float2half_rn(gl > 0.0f ? ga / gl : 0.0f);
     }
-}
-
-// merges the splits of one (token, head)                                   grid tokens * n_heads, 128 threads
-__global__ void __launch_bounds__(128) attention_combine_kernel(const float* __restrict__ part, __half* __restrict__ out,
-                                                                int nsplit) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const float* pp = part + (size_t)blockIdx.x * nsplit * (AT_D + 2);
-    // all loads of a batch of eight splits are issued before any is used (one L2 latency per batch, not per split)
-    float gm = -INFINITY;
-    for (int s0 = 0; s0 < nsplit; s0 += 8) {
-        float mv[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) mv[u] = (s0 + u < nsplit) ? pp[(size_t)(s0 + u) * (AT_D + 2)] : -INFINITY;
-#pragma unroll
-        for (int u = 0; u < 8; ++u) gm = fmaxf(gm, mv[u]);
-    }
-    float gl = 0.0f, ga = 0.0f;
-    for (int s0 = 0; s0 < nsplit; s0 += 8) {
-        float mv[8], lv[8], av[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const bool on = s0 + u < nsplit;
-            const float* q = pp + (size_t)(on ? s0 + u : 0) * (AT_D + 2);
-            mv[u] = on ? q[0] : -INFINITY;
-            lv[u] = on ? q[1] : 0.0f;
-            av[u] = on ? q[2 + threadIdx.x] : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const float c = (mv[u] == -INFINITY) ? 0.0f : __expf(mv[u] - gm);
-            gl += lv[u] * c;
-            ga += av[u] * c;
-        }
-    }
-    out[(size_t)blockIdx.x * AT_D + threadIdx.x] = __float2half_rn(gl > 0.0f ? ga / gl : 0.0f);
+    cluster.sync();                                // nobody leaves while its shared memory is being read
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -673,6 +690,21 @@ __global__ void __launch_bounds__(32) argmax_final_kernel(const float* __restric
     if (threadIdx.x == 0) out[blockIdx.x] = idx;
 }
 
+// Tiles beyond the default shared memory, clusters beyond the portable eight CTAs; once per device.
+template <typename Kernel>
+static int at_setup(SmemOnce& once, Kernel kernel) {
+    int dev = 0;
+    SBVR_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return SBVR_ERR_BAD_ARG;
+    std::lock_guard<std::mutex> lock(once.mu);
+    if (!once.done[dev]) {
+        SBVR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM));
+        SBVR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        once.done[dev] = true;
+    }
+    return SBVR_OK;
+}
+
 }  // namespace sbvr
 
 using namespace sbvr;
@@ -719,7 +751,6 @@ static int attention_launch(const void* qkv, void* kcache, void* vcache, const i
     if ((reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15) return SBVR_ERR_ALIGN;
     const int R = n_heads / n_kv;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    const dim3 grid((unsigned)(tokens * n_kv), (unsigned)nsplit);
     const __half* q = reinterpret_cast<const __half*>(qkv);
     __half* kc = reinterpret_cast<__half*>(kcache);
     __half* vc = reinterpret_cast<__half*>(vcache);
@@ -746,9 +777,18 @@ static int attention_launch(const void* qkv, void* kcache, void* vcache, const i
 #undef SBVR_ATTP
         return SBVR_OK;
     }
-#define SBVR_ATT(RR)                                                                                              \
-    SBVR_CUDA_TRY(launch_pdl(attention_kernel<RR>, grid, dim3(128), 0, st, q, kc, vc, positions, o, scratch,     \
-                             tokens_per_seq, n_heads, n_kv, max_ctx, scale, nsplit, inv_freq, attn_scaling))
+    int cs = 1;                                    // splits: a power of two of at most 16
+    while (cs * 2 <= nsplit && cs * 2 <= AT_MAX_CLUSTER) cs *= 2;
+    nsplit = cs;
+#define SBVR_ATT(RR)                                                                                                        \
+    do {                                                                                                                    \
+        static SmemOnce once;                                                                                               \
+        const int rc = at_setup(once, attention_kernel<RR>);                                                                \
+        if (rc) return rc;                                                                                                  \
+        SBVR_CUDA_TRY(launch_pdl_cluster(attention_kernel<RR>, dim3((unsigned)(tokens * n_kv * nsplit)), dim3(128), nsplit, \
+                                         (size_t)AT_SMEM, st, q, kc, vc, positions, o, tokens_per_seq, n_heads, n_kv, max_ctx, \
+                                         scale, nsplit, inv_freq, attn_scaling));                                           \
+    } while (0)
     switch (R) {
         case 1: SBVR_ATT(1); break;
         case 2: SBVR_ATT(2); break;
@@ -757,9 +797,6 @@ static int attention_launch(const void* qkv, void* kcache, void* vcache, const i
         default: return SBVR_ERR_UNSUPPORTED;
     }
 #undef SBVR_ATT
-    if (nsplit > 1)
-        SBVR_CUDA_TRY(launch_pdl(attention_combine_kernel, dim3(tokens * n_heads), dim3(128), 0, st,
-                                 static_cast<const float*>(scratch), o, nsplit));
     return SBVR_OK;
 }
 

@@ -408,6 +408,8 @@ __global__ void __launch_bounds__(ts_threads(NSUB, M, KS), 1)
                                 *abort_flag = 1;
                                 atomicExch(p.status, 1u);
                                 atomicExch(p.status + 1, 0x340u);
+                                atomicExch(p.status + 2, (unsigned int)N);
+                                atomicExch(p.status + 3, ((unsigned int)KB << 16) | (blockIdx.x & 0xFFFFu));
                                 break;
                             }
                         }

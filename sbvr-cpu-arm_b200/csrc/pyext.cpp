@@ -219,11 +219,13 @@ PyObject* py_linear_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
         Weight w;
         read_weight(a[2], &w);
         const int64_t Kp = (int64_t)w.KW * 32, M = x.size(0);
-        if (M > 4 || w.K != Kp || !x.is_contiguous()) Py_RETURN_FALSE;
+        if (M > 16 || w.K != Kp || !x.is_contiguous()) Py_RETURN_FALSE;
         c10::cuda::OptionalCUDAGuard guard;
         if (c10::cuda::current_device() != w.dev) guard.set_index(w.dev);
         const uintptr_t st = (uintptr_t)c10::cuda::getCurrentCUDAStream(w.dev).stream();
-        sbvr_workspace_t* ws = workspace(w.dev, st, 0);
+        size_t need = 0;
+        if (M > 1) check(sbvr_workspace_bytes(w.dev, (int)M, w.N, (int)Kp, &need), "sbvr_workspace_bytes");
+        sbvr_workspace_t* ws = workspace(w.dev, st, need);
         int rc;
         {
             ReleaseGil nogil;

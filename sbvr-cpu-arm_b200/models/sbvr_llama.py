@@ -310,9 +310,9 @@ class SBVRLlamaForCausalLM(torch.nn.Module):
         return b
 
     def _nsplit(self, tokens: int) -> int:
-        # decode with few tokens: split the context so that about one CTA per SM works
+        # decode with few tokens: split the context so that about two CTAs per SM work
         ctas = tokens * self.n_kv
-        return 1 if ctas >= 96 else max(1, min(16, 192 // ctas))
+        return 1 if ctas >= 192 else max(1, min(16, 296 // ctas))
 
     # ------------------------------------------------------------------ one forward over `tokens` rows
     def _all_reduce(self, t: torch.Tensor):
@@ -327,17 +327,17 @@ class SBVRLlamaForCausalLM(torch.nn.Module):
         T, H = b.tokens, c.hidden_size
         eps = float(c.rms_norm_eps)
         scale = 1.0 / math.sqrt(c.head_dim)
-        nsplit = self._nsplit(T)
+        nsplit = self._nsplit(T) if tokens_per_seq < 8 else 1      # (a prompt's tokens share their K and V tiles instead)
         ck = _lib.check
         # Tensor parallel with few rows: the partial outputs of o and down go to symmetric memory and one fused
         # kernel all-reduces them, adds the residual and applies the next RMSNorm.  Otherwise NCCL + add_rmsnorm.
         comm = self._comm if (self._comm is not None and T <= self._comm.max_rows) else None
         ws = _lib.workspace(self.device.index or 0, st) if comm is not None else None
         n_layers = len(self.layers)
-        # Up to four rows (decode): the residual add + RMSNorm in front of q|k|v, gate|up and lm_head and the
+        # Up to sixteen rows (decode): the residual add + RMSNorm in front of q|k|v, gate|up and lm_head and the
         # SiLU * up in front of down are folded into those linears' kernels.  The folded norm cannot update the
         # residual in place (other CTAs still read it), so the residual alternates between two buffers.
-        fuse = self.fuse_glue and T <= 4
+        fuse = self.fuse_glue and T <= 16
         hc, ho = b.h, b.h2                         # current residual, spare buffer
 
         def norm_linear(lin, delta, weight, out, keep_residual=True):

@@ -158,3 +158,35 @@ def test_product_of_two_encodings_edges(N, K, LS, RS, M):
     y = h2n(sbvr.mm_T(to_sbvr(pl), to_sbvr(pr))).astype(np.float64)
     ref = O.popc_mm_f64(pl["bvr"], pl["coeff_idx"], pl["coeff"], pr["bvr"], pr["coeff_idx"], pr["coeff"], None)
     assert np.abs(y - ref).max() / np.abs(ref).max() <= 1e-3
+
+
+@pytest.mark.parametrize("M", [1, 2, 4, 5, 16])
+@pytest.mark.parametrize("N,K", [(96, 512), (64, 4096), (160, 8192), (128, 14336)])
+@pytest.mark.parametrize("op", ["norm", "norm_nodelta", "silu"])
+def test_ops_folded_into_decode_linears(M, N, K, op):
+    """The op in front of the linear, applied in its kernels, against the separate kernels followed by the linear: the new
+    residual is exact; the product differs where a normalised value lands on the other side of an fp16 rounding (the sum of
+    squares is formed in another order), 2^-11 of single elements."""
+    import sbvr
+    from sbvr import _lib
+    from sbvr.core import XOP_ADD_RMSNORM, XOP_SILU_MUL, linear_fused
+    p = O.make_packed(N, K, 4, G=256, mode="u8", seed=N + K)
+    w = to_sbvr(p)
+    g = torch.Generator(device="cuda").manual_seed(M + K)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=g).half()
+    st = torch.cuda.current_stream().cuda_stream
+    y = torch.empty((M, N), dtype=torch.float16, device="cuda")
+    if op == "silu":
+        gu, act = rnd(M, 2 * K), torch.empty((M, K), dtype=torch.float16, device="cuda")
+        _lib.check(_lib.lib.sbvr_silu_mul_f16(gu.data_ptr(), act.data_ptr(), M, K, st))
+        assert linear_fused(XOP_SILU_MUL, gu, w, y)
+    else:
+        h, d, nw = rnd(M, K), rnd(M, K) if op == "norm" else None, 1 + 0.1 * rnd(K)
+        act, ho, ho2 = torch.empty_like(h), torch.empty_like(h), torch.empty_like(h)
+        _lib.check(_lib.lib.sbvr_add_rmsnorm_f16(h.data_ptr(), None if d is None else d.data_ptr(), nw.data_ptr(), ho.data_ptr(),
+                                                 act.data_ptr(), M, K, 1e-5, st))
+        assert linear_fused(XOP_ADD_RMSNORM, h, w, y, delta=d, norm_weight=nw, h_out=ho2, eps=1e-5)
+        assert torch.equal(ho, ho2)
+    ref = sbvr.linear(act, w).float()
+    assert ((y.float() - ref).abs().max() / ref.abs().max()).item() < (1e-6 if op == "silu" and M <= 4 else 2e-3)
+    check_status()
