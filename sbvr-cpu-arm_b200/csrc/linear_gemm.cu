@@ -27,9 +27,13 @@
 // round-robin and, once the MMAs of a work item have finished, read D from tensor memory, add the bias and
 // write fp16 (or fp32 partial sums when K is split over several CTAs: small activation batches on wide GPUs;
 // the last CTA to arrive adds the parts in a fixed order, so results do not depend on timing).  Warp 16 issues
-// the MMAs from one elected lane; warp 17 streams the activation blocks.  At M = 2048 the tensor pipe is busy about
-// half of the time: a stage costs the decoders about 630 issue slots per scheduler against 512 tensor cycles, and
-// the serial work of the issuer warp (barrier polls, four MMAs, three commits per stage) sits on the same path.  Every wait is bounded; on a time-out
+// the MMAs from one elected lane; warp 17 streams the activation blocks.
+//
+// What bounds it (2048 x 14336 x 4096, S = 4, 256-row tiles, about 850 cycles per 64-k stage): the decoders, about 540 instructions
+// per scheduler and stage with half of the integer pipe busy; without their arithmetic a stage takes 640, with 512 of tensor time.
+// The issuing lane was as long before (a probe of two barriers for the next stages, elections and descriptor arithmetic on the path
+// between two stages: 740 cycles with everything in place); now one barrier stands for both operands, the next stage's is read
+// ahead, descriptors move by constants and the tensor-memory addresses are immediates.  Every wait is bounded; on a time-out
 // the kernel records it in the status word, skips the remaining work without skipping a barrier, frees its
 // tensor memory and returns.
 #include "common.cuh"
@@ -41,10 +45,13 @@ constexpr int GM_DTHREADS = GM_DWGS * 128;
 constexpr int GM_IWARP = GM_DWGS * 4;
 constexpr int GM_PWARP = GM_IWARP + 1;
 constexpr int GM_THREADS = (GM_PWARP + 1) * 32;
-constexpr int GM_ASLOTS = 6;                    // decoded 128 x 64 weight tiles resident in tensor memory
-constexpr int GM_A_COL = 256;                   // D occupies columns [0, NX), the A ring [256, 256 + 32 slots)
 constexpr int GM_TMEM_COLS = 512;
-constexpr int GM_XSTAGES = 6;
+// NX activation rows per tile.  NX = GM_WIDE stands for any multiple of 32 in (256, 384] (GmParams::nx): every stage is then two
+// MMAs per 16 k, 256 columns and the rest, and a decoded weight tile serves up to 1.5 times as many activations.
+constexpr int GM_WIDE = 384;
+// Ring of 64-k stages: a decoded 128 x 64 weight tile in tensor memory and the activation block in shared memory.
+__host__ __device__ constexpr int gm_slots(int NX) { return NX == GM_WIDE ? 4 : 6; }
+__host__ __device__ constexpr int gm_a_col(int NX) { return NX == GM_WIDE ? 384 : 256; }   // D occupies columns [0, NX), the A ring is behind
 constexpr int GM_HDR = 1024;
 
 struct GmParams {
@@ -58,22 +65,21 @@ struct GmParams {
     unsigned int* counters;      // one per output tile, zero between launches
     unsigned int* status;
     int M, N, K, C, G, idx_bytes;
+    int nx;                      // activation rows of a tile
     int NT, MT, KS, SPP, items;  // weight-row tiles, activation-row tiles, k parts, 64-k stages per part
 };
 
 __device__ __forceinline__ void gm_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void gm_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ uint64_t gm_bdesc(uint32_t saddr) {
-    // K-major, no swizzle: 128 B between core matrices along K, 1024 B between 8-row groups; version 1
-    return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)(128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
-           ((uint64_t)1 << 46);
-}
-__device__ __forceinline__ void gm_mma(uint32_t d_t, uint32_t a_t, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// B descriptor: K-major, no swizzle, 128 B between core matrices along K, 1024 B between 8-row groups; version 1.  Its upper word is
+// a constant; the lower one moves by (bytes >> 4).
+__device__ __forceinline__ uint32_t gm_bdesc_lo(uint32_t saddr) { return (saddr >> 4) | ((128u >> 4) << 16); }
+__device__ __forceinline__ void gm_mma(uint32_t d_t, uint32_t a_t, uint32_t bdesc_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_t),
-        "r"(a_t), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "{\n\t.reg .pred p;\n\t.reg .b64 d;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 d, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %3, p;\n\t}" ::"r"(d_t),
+        "r"(a_t), "r"(bdesc_lo), "r"(idesc), "r"(accumulate), "r"((1024u >> 4) | (1u << 14))
         : "memory");
 }
 __device__ __forceinline__ void gm_commit(uint64_t* bar) {
@@ -211,30 +217,28 @@ static __device__ __forceinline__ void gm_add_parts(const float* part, size_t pl
 template <int S, int NX, bool SPLIT>
 __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NX >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-    constexpr int STAGE_BYTES = NX * 128;
+    constexpr int NX1 = NX == GM_WIDE ? 256 : NX;  // columns of the first MMA
+    constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NX1 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    constexpr int GM_SLOTS = gm_slots(NX), GM_A_COL = gm_a_col(NX);
+    const int nx = NX == GM_WIDE ? p.nx : NX;
+    const uint32_t STAGE_BYTES = (uint32_t)nx * 128u;
+    const uint32_t idesc2 = (1u << 4) | ((uint32_t)((nx - NX1) >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 
-    uint64_t* x_full = reinterpret_cast<uint64_t*>(smem);        // [GM_XSTAGES] activation block landed
-    uint64_t* x_empty = x_full + GM_XSTAGES;                     // [GM_XSTAGES] ... and read by its MMAs
-    uint64_t* a_full = x_empty + GM_XSTAGES;                     // [GM_ASLOTS]  weight tile stored
-    uint64_t* a_empty = a_full + GM_ASLOTS;                      // [GM_ASLOTS]  ... and read by its MMAs
-    uint64_t* d_full = a_empty + GM_ASLOTS;                      // [1] all MMAs of a work item done
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem);          // [GM_SLOTS] activation block landed and weight tile stored
+    uint64_t* empty = full + GM_SLOTS;                           // [GM_SLOTS] both read by the stage's MMAs
+    uint64_t* d_full = empty + GM_SLOTS;                         // [1] all MMAs of a work item done
     uint64_t* d_empty = d_full + 1;                              // [1] D read out
     volatile int* flags = reinterpret_cast<volatile int*>(d_empty + 1);     // [0] abort, [1] "last part" flag
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(smem + GM_HDR - 16);
-    unsigned char* xs = smem + GM_HDR;                           // [GM_XSTAGES][STAGE_BYTES]
+    unsigned char* xs = smem + GM_HDR;                           // [GM_SLOTS][STAGE_BYTES]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     pdl_launch_dependents();
     pdl_wait();                                    // the re-tiled activations come from the previous kernel
     if (threadIdx.x == 0) {
-        for (int i = 0; i < GM_XSTAGES; ++i) {
-            mbar_init(&x_full[i], 1);
-            mbar_init(&x_empty[i], 1);
-        }
-        for (int i = 0; i < GM_ASLOTS; ++i) {
-            mbar_init(&a_full[i], 4);
-            mbar_init(&a_empty[i], 1);
+        for (int i = 0; i < GM_SLOTS; ++i) {
+            mbar_init(&full[i], 5);                // the activation producer and four decoder warps
+            mbar_init(&empty[i], 1);
         }
         mbar_init(d_full, 1);
         mbar_init(d_empty, GM_DWGS * 4);
@@ -265,15 +269,14 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                 const unsigned char* src = reinterpret_cast<const unsigned char*>(p.xt) +
                                            ((size_t)mt * (p.K / 64) + (size_t)kp * SPP) * STAGE_BYTES;
                 for (int ks = 0; ks < SPP; ++ks, ++it) {
-                    const int st = it % GM_XSTAGES;
-                    const uint32_t ph = (uint32_t)(it / GM_XSTAGES) & 1u;
-                    if (flags[0] || !mbar_wait_async(&x_empty[st], ph ^ 1u)) {
+                    const int st = it % GM_SLOTS;
+                    const uint32_t ph = (uint32_t)(it / GM_SLOTS) & 1u;
+                    if (flags[0] || !mbar_wait_async(&empty[st], ph ^ 1u)) {
                         ok = false;
                         break;
                     }
-                    mbar_arrive_expect_tx(&x_full[st], (uint32_t)STAGE_BYTES);
-                    bulk_g2s(xs + (size_t)st * STAGE_BYTES, src + (size_t)ks * STAGE_BYTES, (uint32_t)STAGE_BYTES,
-                             &x_full[st]);
+                    mbar_arrive_expect_tx(&full[st], STAGE_BYTES);
+                    bulk_g2s(xs + (size_t)st * STAGE_BYTES, src + (size_t)ks * STAGE_BYTES, STAGE_BYTES, &full[st]);
                 }
             }
             if (!ok) {
@@ -284,58 +287,50 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
         }
     } else if (warp == GM_IWARP) {
         // ------------------------------ MMA issuer ------------------------------
-        // A barrier poll costs a couple of hundred cycles on a busy SM even when the phase is complete, and two polls
-        // per stage in front of four MMAs made this warp the kernel's serial bottleneck.  So the lanes poll the
-        // barriers of the next LOOK stages in one go and the warp issues every stage found complete.
-        constexpr int LOOK = GM_XSTAGES < GM_ASLOTS ? GM_XSTAGES : GM_ASLOTS;
-        int it = 0, seq = 0, ready = 0;            // stages [it, ready) are known to have both operands in place
-        bool ok = true;
-        for (int item = blockIdx.x; item < p.items && ok; item += grid, ++seq) {
-            if (seq > 0) {                          // D of the previous item must have been read out
-                if (flags[0] || !mbar_wait_timed(d_empty, (uint32_t)(seq - 1) & 1u)) {
-                    ok = false;
-                    break;
-                }
-                gm_fence_after();
-            }
-            for (int ks = 0; ks < SPP; ++ks, ++it) {
-                const int st = it % GM_XSTAGES, slot = it % GM_ASLOTS;
-                if (it >= ready) {
-                    long long t0 = 0;
-                    for (;;) {
-                        const int s = it + lane;   // lane l looks at stage it + l
-                        bool okl = false;
-                        if (lane < LOOK)
-                            okl = mbar_test(&x_full[s % GM_XSTAGES], (uint32_t)(s / GM_XSTAGES) & 1u) &&
-                                  mbar_test(&a_full[s % GM_ASLOTS], (uint32_t)(s / GM_ASLOTS) & 1u);
-                        const uint32_t mask = __ballot_sync(0xffffffffu, okl);
-                        const int n = __ffs((int)~mask) - 1;       // stages complete in a row, starting at `it`
-                        if (n > 0) {
-                            ready = it + n;
-                            break;
-                        }
-                        if (t0 == 0) t0 = clock64();
-                        else if (flags[0] || clock64() - t0 > 2000000000LL) {
-                            ok = false;
-                            break;
-                        }
+        // One barrier per stage says that both operands are in place, and the barrier of the next stage is read before
+        // the MMAs of this one are issued, so that its latency runs beside them.
+        const int total = (int)blockIdx.x < p.items ? ((p.items - 1 - (int)blockIdx.x) / grid + 1) * SPP : 0;
+        bool ok = tbase == 0;                      // (an allocation of all columns can only start at column 0)
+        if (elect_one()) {
+            const uint32_t d0 = gm_bdesc_lo(smem_u32(xs)), dstep = STAGE_BYTES >> 4;
+            int ks = 0;
+            uint32_t ph = 0, dph = 1;              // dph: parity of the read-out of the item before
+            bool rdy = mbar_test(&full[0], 0u);
+            for (int it = 0; it < total && ok; it += GM_SLOTS, ph ^= 1u) {
+#pragma unroll
+                for (int slot = 0; slot < GM_SLOTS; ++slot) {
+                    if (it + slot >= total) break;
+                    if (ks == 0) {
+                        if (it + slot > 0 && !mbar_wait_timed(d_empty, dph)) ok = false;       // D of the previous item must have been read out
+                        dph ^= 1u;
+                    }
+                    if (!rdy) {                    // (spins: a warp parked by try_wait comes back later than the phase)
+                        const long long t0 = clock64();
+                        while (!mbar_test(&full[slot], ph))
+                            if (clock64() - t0 > 2000000000LL) {
+                                ok = false;
+                                break;
+                            }
                     }
                     if (!ok) break;
                     gm_fence_after();
-                }
-                const uint32_t bs = smem_u32(xs + (size_t)st * STAGE_BYTES);
-                if (elect_one()) {
+                    rdy = mbar_test(&full[(slot + 1) % GM_SLOTS], slot + 1 == GM_SLOTS ? ph ^ 1u : ph);
+                    const uint32_t d = d0 + (uint32_t)slot * dstep;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        gm_mma(tbase, tbase + GM_A_COL + slot * 32 + q * 8, gm_bdesc(bs + q * 256), IDESC,
-                               (uint32_t)((ks | q) != 0));
-                    gm_commit(&a_empty[slot]);
-                    gm_commit(&x_empty[st]);
-                    if (ks == SPP - 1) gm_commit(d_full);
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t acc = q ? 1u : (uint32_t)(ks != 0);
+                        gm_mma(0, GM_A_COL + slot * 32 + q * 8, d + q * 16, IDESC, acc);
+                        if (NX == GM_WIDE) gm_mma(NX1, GM_A_COL + slot * 32 + q * 8, d + NX1 * 8 + q * 16, idesc2, acc);
+                    }
+                    gm_commit(&empty[slot]);
+                    if (++ks == SPP) {
+                        gm_commit(d_full);
+                        ks = 0;
+                    }
                 }
-                __syncwarp();
             }
         }
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) {
             flags[0] = 1;
             if (lane == 0) {
@@ -347,12 +342,12 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
         // ------------------------------ decoder warpgroups ------------------------------
         const int wg = warp >> 2, wl = warp & 3;
         const int r = wl * 32 + lane;
-        const int dtid = threadIdx.x;              // 0 .. 383
+        const int dtid = threadIdx.x;              // 0 .. 511
         const uint32_t lane_sel = (uint32_t)(wl * 32) << 16;
         const int N = p.N;
         bool dead = false;
 
-        // The stages of all work items of this CTA form one sequence; this warpgroup takes every third one.
+        // The stages of all work items of this CTA form one sequence; this warpgroup takes every fourth one.
         struct Pos {
             int item, ks, it;
             int kst0, n;                           // first 64-k stage of the item's k part; this thread's weight row
@@ -402,12 +397,12 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                 flags[0] = 1;
             }
             dead = __any_sync(0xffffffffu, dead);
-            const int m0 = mt * NX;
+            const int m0 = mt * nx;
             if (!dead) {
                 gm_fence_after();
                 const bool on = n < N;
                 const float bias = (p.bias && !SPLIT && on) ? __half2float(p.bias[n]) : 0.0f;
-                for (int c = wg; c < NX / 32; c += GM_DWGS) {
+                for (int c = wg; c < nx / 32; c += GM_DWGS) {
                     float d[32];
                     gm_ld32(tbase + lane_sel + c * 32, d);
                     if constexpr (!SPLIT) {
@@ -508,14 +503,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                 mul[s][3] = __hmul2(c2, __float2half2_rn(128.0f));
                 mul[s][4] = __hmul2(c2, __float2half2_rn(0.5f));
             }
-            const int slot = q.it % GM_ASLOTS;
-            if (!dead && !mbar_wait_async(&a_empty[slot], ((uint32_t)(q.it / GM_ASLOTS) & 1u) ^ 1u)) {
-                dead = true;
-                flags[0] = 1;
-            }
-            dead = __any_sync(0xffffffffu, dead);
-            if (dead) return;
-            gm_fence_after();
+            const int slot = q.it % GM_SLOTS;
             uint32_t a[32];
             if (!__any_sync(0xffffffffu, big)) {
 #pragma unroll
@@ -565,11 +553,19 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                     }
                 }
             }
+            // the slot is waited for with the values in registers: the decode runs beside the MMAs that still read the slot
+            if (!dead && !mbar_wait_async(&empty[slot], ((uint32_t)(q.it / GM_SLOTS) & 1u) ^ 1u)) {
+                dead = true;
+                flags[0] = 1;
+            }
+            dead = __any_sync(0xffffffffu, dead);
+            if (dead) return;
+            gm_fence_after();
             gm_st32(tbase + lane_sel + GM_A_COL + slot * 32, a);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             gm_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&a_full[slot]);
+            if (lane == 0) mbar_arrive(&full[slot]);
         };
 
         while (cur.item < p.items) {
@@ -620,7 +616,25 @@ struct GmPlan {
     size_t xt_bytes, part_bytes;
 };
 
-static int gm_nx(int M) { return M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256; }
+// Activation rows of a tile.  More than 256 rows: the width with the least work on the busiest SM, whole rounds of tiles times the
+// time of a 64-k stage.  A stage of a 256-row tile waits for the decoders (the more planes the longer), one of a wider tile for
+// its MMAs; measured per stage at 2048 x 14336 x 4096, in cycles: 850 (S = 4), about 730 (S = 2) at 256 rows, 3 per row for wider
+// tiles (a second, small MMA costs more than its share of the columns).  Wide tiles win where they save rounds: 232 -> 210 us at
+// 2048 x 14336 x 4096 (7 rounds -> 5 of 352 rows), 350 -> 302 us at 3000 x 4096 x 14336 (3 -> 2), 78 -> 59 us at 1500 x 4096 x
+// 4096 (2 -> 1 of 384 rows); 2048 x 4096 stays at 256 rows (2 rounds either way).  Problems that do not fill the GPU at 256 rows
+// split K instead.
+static int gm_nx(int M, int NT, int S, int sm_count) {
+    if (M <= 256) return M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+    int best = 256;
+    long long cost = 0;
+    for (int nx = 256; nx <= GM_WIDE; nx += 32) {
+        const long long items = (long long)NT * ((M + nx - 1) / nx);
+        if (nx == 256 && items < sm_count) break;
+        const long long c = (items + sm_count - 1) / sm_count * (nx == 256 ? 610 + 60 * S : 3 * nx);
+        if (nx == 256 || c < cost) best = nx, cost = c;
+    }
+    return best;
+}
 
 bool linear_gemm_supported(const PackedW& w, int M) {
     if (w.S < 2 || w.S > 4) return false;
@@ -633,13 +647,13 @@ bool linear_gemm_supported(const PackedW& w, int M) {
 }
 
 static void gm_plan(const PackedW& w, int M, int sm_count, GmPlan* pl) {
-    pl->NX = gm_nx(M);
-    pl->MT = (M + pl->NX - 1) / pl->NX;
     pl->NT = (w.N + 127) / 128;
+    pl->NX = gm_nx(M, pl->NT, w.S, sm_count);
+    pl->MT = (M + pl->NX - 1) / pl->NX;
     const int KST = w.K / 64;
     int ks = 1;
     const int tiles = pl->NT * pl->MT;
-    if (tiles < sm_count && tiles <= SBVR_WS_COUNTERS) {
+    if (pl->NX <= 256 && tiles < sm_count && tiles <= SBVR_WS_COUNTERS) {
         // split K so that more SMs work, keeping at least 4 stages per part
         for (int cand = 2; cand <= KST / 4; ++cand) {
             if (KST % cand) continue;
@@ -651,7 +665,7 @@ static void gm_plan(const PackedW& w, int M, int sm_count, GmPlan* pl) {
     pl->SPP = KST / ks;
     pl->items = tiles * ks;
     pl->grid = pl->items < sm_count ? pl->items : sm_count;
-    pl->smem = GM_HDR + GM_XSTAGES * pl->NX * 128;
+    pl->smem = GM_HDR + gm_slots(pl->NX > 256 ? GM_WIDE : pl->NX) * pl->NX * 128;
     pl->xt_bytes = ((size_t)pl->MT * pl->NX * w.K * 2 + 255) / 256 * 256;
     pl->part_bytes = ks > 1 ? (size_t)ks * pl->MT * pl->NX * w.N * 4 : 0;
 }
@@ -680,7 +694,8 @@ static int gm_launch_nx(const GmParams& p, int NX, int grid, int smem, cudaStrea
         case 32: return gm_launch_inst<S, 32>(p, grid, smem, st);
         case 64: return gm_launch_inst<S, 64>(p, grid, smem, st);
         case 128: return gm_launch_inst<S, 128>(p, grid, smem, st);
-        default: return gm_launch_inst<S, 256>(p, grid, smem, st);
+        case 256: return gm_launch_inst<S, 256>(p, grid, smem, st);
+        default: return gm_launch_split<S, GM_WIDE, false>(p, grid, smem, st);
     }
 }
 
@@ -705,7 +720,7 @@ int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half*
     p.xt = xt, p.bvr = w.bvr, p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y;
     p.part = reinterpret_cast<float*>(ws->dyn + pl.xt_bytes);
     p.counters = ws->counters, p.status = ws->status;
-    p.M = M, p.N = w.N, p.K = w.K, p.C = w.C, p.G = w.G, p.idx_bytes = w.idx_bytes;
+    p.M = M, p.N = w.N, p.K = w.K, p.C = w.C, p.G = w.G, p.idx_bytes = w.idx_bytes, p.nx = pl.NX;
     p.NT = pl.NT, p.MT = pl.MT, p.KS = pl.KS, p.SPP = pl.SPP, p.items = pl.items;
     switch (w.S) {
         case 2: return gm_launch_nx<2>(p, pl.NX, pl.grid, pl.smem, st);

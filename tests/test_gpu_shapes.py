@@ -34,6 +34,12 @@ def test_linear_any_rows_any_inner_length(M, N, K, S, mode):
     check_status()
 
 
+@pytest.mark.parametrize("M,N,K,S", [(257, 19072, 256, 4), (257, 19072, 512, 2), (700, 14300, 512, 3), (700, 14336, 1000, 4), (1500, 4000, 256, 2)])
+def test_linear_wide_tiles(M, N, K, S):
+    """Sizes that take tiles of more than 256 activation rows (288, 352, 384) on a GPU of 148 SMs, with ragged last tiles."""
+    test_linear_any_rows_any_inner_length(M, N, K, S, "u16")
+
+
 @pytest.mark.parametrize("N,K", [(1, 256), (31, 250), (33, 8), (64, 1000), (40, 777)])
 @pytest.mark.parametrize("S", [1, 3, 4, 6])
 def test_decode_ragged_bit_exact(N, K, S):
