@@ -502,7 +502,7 @@ def small_m_and_prefill(torch, dev, stream):
                     x = torch.randn((M, K), device=dev, generator=gen).half()
                     outs = [torch.empty((M, N), dtype=torch.float16, device=dev) for _ in range(ncopy)]
                     for algo, name in ((3, "fp16 GEMM with in-kernel dequantisation (linear_gemm_kernel)"),
-                                       (4, "FP4 digits with block scale factors (xq8_kernel + linear_tcb_kernel)")):
+                                       (4, "FP4 digits with block scale factors (sb_quant_kernel + linear_sb_kernel)")):
                         us = median_graph_time_us(torch, stream, [(lambda w=w, o=o: sbvr.linear(x, w, None, algo=algo, out=o))
                                                                   for w, o in zip(ws_, outs)], repeats=3)
                         batch.append(dict(row(N, K, M, 4, G, us, IDXB, algo=algo), kernel=name))
@@ -779,7 +779,7 @@ def kernel_case(which):
         print(json.dumps({"kernel_case": which, **w.encoder_stats}))
         return
     M = {"gemv": 1, "gemm16": 16, "batch16": 16, "gemm2048": 2048}[which]
-    algo = {"gemm16": 3, "batch16": 4}.get(which, 0)      # M = 16: the fp16 GEMM or the small-batch FP4 kernel on request
+    algo = {"gemm16": 3, "batch16": 4}.get(which, 0)      # M = 16: the fp16 GEMM on request or the small-batch FP4 kernel
     ws_ = []
     for _ in range(6):
         bvr = torch.randint(-2**31, 2**31 - 1, (K // 32, N, S), dtype=torch.int32, device=dev, generator=gen)

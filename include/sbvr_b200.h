@@ -59,7 +59,7 @@ SBVR_API int sbvr_last_cuda_error(void);
 /* Which wait ran out, as recorded by the kernel, for the last SBVR_ERR_TIMEOUT that sbvr_workspace_status returned in this
  * process (0 if none): 0x3xx decode GEMV, 0x4xx small-batch kernel, 0x7xx all-reduce kernels, others the GEMM. */
 SBVR_API unsigned int sbvr_last_timeout_where(void);
-/* Two more words of that record where the kernel leaves them (small-batch kernel: N, and K / 256 << 16 | M << 8 | CTA). */
+/* Two more words of that record where the kernel leaves them (decode GEMV: N, and K / 256 << 16 | CTA). */
 SBVR_API unsigned int sbvr_last_timeout_info(int i);
 
 /* Device facts the launch heuristics use.  Replaces `_sbvr_cuda_init` (sbvr/kernels/sbvr_ops.cpp:122-150,
@@ -105,8 +105,9 @@ SBVR_API int sbvr_decode_f16(const uint32_t* bvr, const void* coeff_idx, int idx
  *       any N; needs a workspace of sbvr_workspace_bytes(...));
  *   4 = tcgen05 FP4 tensor-core kernel for small batches (2 <= M <= 32, at most 16 for G = 128; S, G, N and alignment as
  *       for algo 2, K a multiple of 256 and at most 32768; the activations are quantised by a small kernel in front;
- *       needs a workspace of sbvr_workspace_bytes(...)).  Never picked by algo 0 (see the note at the dispatch in
- *       csrc/api.cu): on request only. */
+ *       needs a workspace of sbvr_workspace_bytes(...)).
+ * algo 0 takes 2 for M <= 4, 4 for M <= 16 (and for fewer rows where 2 does not apply), 3 for more rows, and 1 for what none of
+ * them covers and for very small problems. */
 SBVR_API int sbvr_linear_f16(const void* x, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff,
                     int C, const void* bias, void* y, int M, int N, int K, int S, int G, int algo,
                     sbvr_workspace_t* ws, sbvr_stream_t stream);
