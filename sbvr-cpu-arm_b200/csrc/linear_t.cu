@@ -22,8 +22,8 @@
 // buffer of its own in shared memory (every load instruction is 512 contiguous bytes; lanes of a quad column read the same
 // entry back).  K is split over CTAs while less than two per SM exist; the parts are added in part order by the CTA that
 // arrives last at the word rows' counter, so results do not depend on timing.
-// Measured (S = 4, us; one predicated fp32 add per plane bit in brackets): 14336 x 4096: M = 1 17.9 (21.3), M = 4 27 (71), M = 8
-// 37 (128); 4096 x 4096, M = 1: 9.2 (9.2).  Bound by instruction issue (35 per warp for 32 outputs x 8 units) and, on small
+// Measured (S = 4, us; one predicated fp32 add per plane bit in brackets): 14336 x 4096: M = 1 17.8 (21.3), M = 4 26 (71), M = 8
+// 35 (128); 4096 x 4096, M = 1: 9.2 (9.2).  Bound by instruction issue (35 per warp for 32 outputs x 8 units) and, on small
 // weights, by the chain of line number, line, digits in front of the loop.
 #include "common.cuh"
 
@@ -280,18 +280,35 @@ __global__ void __launch_bounds__(LT_THREADS, 2) linear_t_kernel(const LtParams 
     __syncthreads();
     if (!last_s) return;
     __threadfence();
-    for (int e = threadIdx.x; e < outs; e += LT_THREADS) {
-        const int nl = e % (nw * 32), m = e / (nw * 32);
-        const float* src = p.part + m * pn + (int)blockIdx.x * nw * 32 + nl;
-        float v = 0.0f;
-        for (int q = 0; q < p.KS; q += 8) {        // eight parts' loads in flight
-            float tq[8];
+    // Eight parts in flight per thread and, for three rows and more, of four results: one result at a time was a chain of
+    // rows * KS / 8 round trips to L2 (8 rows of 1024 x 14336: 41.7 -> 28.3 us; one row is faster without).
+    constexpr int U = NT == 1 ? 1 : 4;
+    for (int e0 = threadIdx.x; e0 < outs; e0 += U * LT_THREADS) {
+        const float* src[U];
+        float v[U];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) tq[i] = (q + i < p.KS) ? __ldcg(src + (size_t)(q + i) * rows * pn) : 0.0f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) v += tq[i];
+        for (int u = 0; u < U; ++u) {
+            const int e = min(e0 + u * LT_THREADS, outs - 1);
+            src[u] = p.part + (e / (nw * 32)) * pn + (int)blockIdx.x * nw * 32 + e % (nw * 32);
+            v[u] = 0.0f;
         }
-        store(m, n0 + nl, v);
+        for (int q = 0; q < p.KS; q += 8) {
+            float tq[U][8];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    tq[u][i] = (q + i < p.KS && e0 + u * LT_THREADS < outs) ? __ldcg(src[u] + (size_t)(q + i) * rows * pn) : 0.0f;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[u] += tq[u][i];
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int e = e0 + u * LT_THREADS;
+            if (e < outs) store(e / (nw * 32), n0 + e % (nw * 32), v[u]);
+        }
     }
     if (threadIdx.x == 0) p.counters[blockIdx.x] = 0u;      // ready for the next launch
 }
@@ -352,7 +369,8 @@ extern "C" int sbvr_linear_t_f16(const void* x, const uint32_t* bvr_t, const voi
         if (KS > 64) KS = 64;
         if (KS < 1) KS = 1;
         int kchunk = ((K + KS - 1) / KS + quantum - 1) / quantum * quantum;
-        if (kchunk < 128) kchunk = (128 + quantum - 1) / quantum * quantum;
+        const int least = p.rows == 2 ? 256 : 128;      // two rows: fewer parts to add (10.2 -> 9.4 us at 1024 x 4096)
+        if (kchunk < least) kchunk = (least + quantum - 1) / quantum * quantum;
         const int cap = LT_MAX_KC / quantum * quantum;
         if (kchunk > cap) kchunk = cap;
         KS = (K + kchunk - 1) / kchunk;
