@@ -164,11 +164,11 @@ int sbvr_workspace_bytes(int device, int M, int N, int K, size_t* bytes) {
     const size_t fixed = SBVR_WS_FIXED_BYTES;
     const size_t stage = (((size_t)M * K * 2 + 255) / 256 + ((size_t)M * N * 2 + 255) / 256) * 256;   // host-pointer staging
     size_t kern = linear_gemm_workspace_bytes(w, M, di.sm_count);
-    if (M >= 2 && M <= 32 && K % 256 == 0) {       // the small-batch kernel's digits and partial sums, whatever the encoding
+    if (M >= 2 && M <= 16 && K % 256 == 0) {       // the small-batch kernel's digits and partial sums, whatever the encoding
         for (int s = 2; s <= 4; ++s)
             for (int g = 128; g <= 256; g += 128) {
                 w.S = s, w.G = g;
-                const size_t sb = linear_sb_workspace_bytes(w, M, di);
+                const size_t sb = linear_sb_workspace_bytes(w, di);
                 if (sb > kern) kern = sb;
             }
     }
@@ -247,7 +247,8 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
         if (ws && device_info(ws->device, &di) == SBVR_OK && di.cc_major == 10) {
             if (linear_tcs_supported(w, M) && (Kin != K || !(reinterpret_cast<uintptr_t>(x) & 15)) &&
                 linear_tcs_workspace_bytes(w, M, di.sm_count) <= ws->dyn_bytes) algo = 2;
-            else if (M <= 16 && linear_sb_supported(w, M) && linear_sb_workspace_bytes(w, M, di) <= ws->dyn_bytes) algo = 4;
+            else if (M <= 16 && linear_sb_supported(w, M) && linear_sb_preferred(w) && linear_sb_workspace_bytes(w, di) <= ws->dyn_bytes)
+                algo = 4;
             // A small problem is done by the SIMT kernel's one launch before the GEMM's second has started: measured 2.8 against
             // 5.7 us at 64 x 128 (M = 1), 5.2 against 9.8 at 300 x 512 (M = 8), 7.0 against 8.2 at 3000 x 1024 (M = 4), but 22
             // against 12 at 3000 x 3072.  Its time is that of K x (blocks of four rows) as long as all blocks run at once.
@@ -255,6 +256,13 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
             else if (linear_gemm_supported(w, M) &&
                      linear_gemm_workspace_bytes(w, M, di.sm_count) <= ws->dyn_bytes) algo = 3;
         }
+    }
+    // Algo 4 takes up to 32 rows (16 with groups of 128); beyond sixteen the GEMM does the work, on the weights the kernel takes.  The
+    // kernel's form for them (six digits) took 37 us at 14336 x 4096, M = 32, S = 4, 51 at 4096 x 14336 and 17.4 at 4096 x 4096,
+    // against the GEMM's 33, 34 and 16.
+    if (algo == 4 && M > 16) {
+        if (M > 32 || w.G != 256 || !linear_sb_supported(w, 16)) return SBVR_ERR_UNSUPPORTED;
+        algo = 3;
     }
     if (Kin != K && algo != 3) {                   // the GEMM pads while it re-tiles
         __half* xd = reinterpret_cast<__half*>(ws->dyn + ws->dyn_bytes);
@@ -308,7 +316,7 @@ int sbvr_linear_fused_f16(int x_op, const void* x, const void* delta, const void
     xop.h_out = reinterpret_cast<__half*>(h_out), xop.eps = eps;
     if (!linear_tcs_supported(w, M)) {             // more rows (or digits that do not fit the GEMV): the small-batch kernel
         if (x_op == SBVR_XOP_DIGITS || M > 16 || !linear_sb_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
-        if (linear_sb_workspace_bytes(w, M, di) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
+        if (linear_sb_workspace_bytes(w, di) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
         return launch_linear_sb(reinterpret_cast<const __half*>(x), w, reinterpret_cast<const __half*>(bias),
                                 reinterpret_cast<__half*>(y), M, ws->device, ws->status, reinterpret_cast<unsigned int*>(ws->xchg),
                                 ws->dyn, ws->dyn_bytes, reinterpret_cast<cudaStream_t>(stream), &xop);

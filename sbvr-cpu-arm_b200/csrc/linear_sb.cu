@@ -1,4 +1,4 @@
-// SBVR linear for small activation batches (2 .. 32 rows): FP4 tensor-core dot products of plane bits with activation digits,
+// SBVR linear for small activation batches (2 .. 16 rows): FP4 tensor-core dot products of plane bits with activation digits,
 // like the decode GEMV, but with the digits' weights and the activations' block step carried by the MMA's own block scale
 // factors, so that the tensor pipe sums over digits and nothing but one multiply-add per (row, plane, digit half, activation
 // row, 256-k block) is left for the CUDA cores.
@@ -10,16 +10,21 @@
 //  A (tensor memory)  128 lanes = TN output rows x their planes; a lane's 256 plane bits of a k block are expanded to 4-bit
 //      E2M1 codes by six integer instructions per packed word (`(w << 1) & 0x2222.., w & 0x2222.., w & 0x4444..,
 //      (w >> 1) & 0x4444..`): a set bit becomes 1, 1, 2, 2 for k % 4 = 0 .. 3.
-//  B (shared memory)  x is quantised per (activation row, 256-k block) to 16-bit block fixed point q = round(x / step),
-//      step a power of two, and q + 0x24924 is cut into six 3-bit fields t, digit = t - 4 in {-4 .. 3}, so that
-//      q = sum_d 8^d digit_d.  Every digit is an exact E2M1 value (halved where the plane bit counts 2).  One MMA
-//      multiplies the plane bits by ONE digit of all activation rows (M > 16: N = 32 rows) or by two digits of up to
-//      16 rows (N = 2 x 16), with the scale factor 8^d * step of that digit and row as the B block scale (UE8M0, a power
-//      of two): the accumulator column of an activation row then holds sum_k bit * x^ directly, whatever the digit.
-//      M <= 16 leaves two columns per activation row (even and odd digits), added on the way out.
+//  B (shared memory)  x is quantised per (activation row, 256-k block) to block fixed point in two levels: q = round(x / step)
+//      with the power of two step = 2^(e - 15) for a largest value of 1.f * 2^e, and what that rounding left over with step 2^-17.
+//      q + 0x24924 is cut into six 3-bit fields t, digit = t - 4 in {-4 .. 3}, so that q = sum_d 8^d digit_d.  Every digit
+//      is an exact E2M1 value (halved where the plane bit counts 2).  One MMA multiplies the plane bits by two digits of 16
+//      activation rows (N = 2 x 16), with the scale factor 8^d * step of that digit and row as the B block scale (UE8M0, a power
+//      of two): the two accumulator columns of an activation row (even and odd digits, added on the way out) then hold
+//      sum_k bit * x^ directly, whatever the digit and its level.
 //
-// Structure.  K is cut into chunks of at most eight (M > 16: four) 256-k blocks, and a CTA works on one chunk: its digits
-// (12 or 24 KB per block, written by the quantiser kernel) stay in shared memory and their scale factors in tensor memory for
+// Precision.  |x - x^| <= 2^(e - 33): fp16 activations keep all of their bits down to 2^-22 of their block's largest, and what is
+// lost below is far less than fp32's rounding of that largest value.  The first level alone, an error of 2^(e - 15), made zeros of
+// everything below 2^-15 of the largest: with one activation of 2^13 in every block, outputs whose weight there is zero were off by
+// 15 % (now 2.1e-4, the rounding of the result; 3.4e-4 for the fp16 GEMM, which sees the activations as they are and rounds weights).
+//
+// Structure.  K is cut into chunks of at most SB_CHUNK 256-k blocks, and a CTA works on one chunk: its digits (24 KB per block,
+// written by the quantiser kernel) stay in shared memory and their scale factors in tensor memory for
 // the whole launch, so the only things that move are packed words.  Four warpgroups take (row tile, k block) units in order,
 // each on its own, with two A buffers and one D buffer: while the MMAs of unit i run, unit i + 1 is expanded into the other
 // A buffer and unit i + 2 read from shared memory; as soon as they are done the sums are read and the MMAs of unit i + 1
@@ -30,13 +35,12 @@
 // for another CTA, and all of it but the last tile's runs beside the other warpgroups' units).  A tile that several warpgroups
 // share is put together in shared memory at the end.  Every wait is bounded.
 //
-// What bounds it: a unit (4.6 KB of weight) is 12 MMAs of 17 cycles and about 220 issue slots per scheduler, against 200 cycles
-// of its SM's share of HBM; measured about 290 cycles.  The form before this one (three warpgroups in lockstep over shared
-// digit stages) spent 1 500 cycles per three units on the latency chain of a compute warp.  Per call with the quantiser, M = 16,
-// S = 4 (that form, the fp16 GEMM in brackets): 14336 x 4096 21.9 us (26.3, 32.6), 4096 x 14336 26.2 (27.3, 35.4), 4096 x 4096 11.8
-// (17.0, 17.9), 1024 x 4096 9.2 (16.5, 12.8).
+// What bounds it: the tensor pipe on large weights (a unit is 24 MMAs of about 33 cycles, 790 of the 1 030 cycles that a unit takes at
+// 28672 x 8192), on small ones the two launches and the merge of the chunks.  Per call with the quantiser, M = 16, S = 4, us (the
+// fp16 GEMM in brackets): 4096 x 4096 12.5 (15.4), 1024 x 4096 10.8 (13.2), 14336 x 4096 27.9 (32.5), 10240 x 8192 46 (58),
+// 28672 x 8192 107 (112); with six digits, whose error the GEMM does not have, they took 11.8, 9.0, 21.9 and 67.
 //
-// Replaces the M > 1 use of `_sbvr_row_deq_mm_T` (reference sbvr/kernels/sbvr_kernel.cu:121-191) for 2 .. 32 rows.
+// Replaces the M > 1 use of `_sbvr_row_deq_mm_T` (reference sbvr/kernels/sbvr_kernel.cu:121-191) for 2 .. 16 rows.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -47,28 +51,30 @@ namespace sbvr {
 constexpr int SB_NWG = 4;
 constexpr int SB_CW0 = 4;                       // warps 0 .. 3: issuers (warp 0 also sets up); compute warps behind
 constexpr int SB_THREADS = (SB_CW0 + 4 * SB_NWG) * 32;
-constexpr int SB_SF_BYTES = 512;                // 32 rows x 16 B of B scale factors (and poison marks) per k block
+constexpr int SB_MP = 16;                       // activation rows the accumulators cover
+constexpr int SB_ND = 12;                       // digits of an activation
+constexpr int SB_NJ = SB_ND / 2;                // MMAs per 64 k: two digits each
+constexpr int SB_BLOB = SB_NJ * 4096 + 512;     // digits of a k block, then 32 rows x 16 B of scale factors (and poison marks)
 constexpr int SB_ASTAGE = TS_STAGE_WORDS + 512; // packed words of a unit + its coefficient data
 constexpr int SB_MAX_STAGES = 4;
 constexpr int SB_HDR = 1024;
-__host__ __device__ constexpr int sb_blob(int NJ) { return NJ * 4096 + SB_SF_BYTES; }
-__host__ __device__ constexpr int sb_chunk(int NJ) { return NJ == 6 ? 4 : 8; }       // k blocks of a CTA at most (shared memory)
-__host__ __device__ constexpr int sb_sfcols(int NJ) { return NJ == 6 ? 16 : 8; }
-// Tensor memory: per warpgroup A (32 columns each) and D (32 per group of a block), then the B scale factors of every k block (16
-// or 8 columns each, one 4-column block per two MMAs; an MMA's scale-factor address designates a block), then unit factors for A
+constexpr int SB_CHUNK = 4;                     // k blocks of a CTA at most (shared memory)
+constexpr int SB_SFCOLS = 12;
+// Tensor memory: per warpgroup A (32 columns each) and D (32 per group of a block), then the B scale factors of every k block (12
+// columns each, one 4-column block per two MMAs; an MMA's scale-factor address designates a block), then unit factors for A
 constexpr int SB_WGCOLS = 96;                   // A x 2 and D, or A and D x 2
 constexpr int SB_SFB_COL = SB_NWG * SB_WGCOLS, SB_SFA_COL = SB_SFB_COL + 64;
-static_assert(SB_SFA_COL + 32 <= TS_TMEM_COLS, "tensor memory");
+static_assert(SB_CHUNK * SB_SFCOLS <= 64 && SB_SFA_COL + 32 <= TS_TMEM_COLS, "tensor memory");
 
 struct SbParams {
-    const unsigned char* xb;      // [KB][sb_blob] written by sb_quant_kernel
+    const unsigned char* xb;      // [KB][SB_BLOB] written by sb_quant_kernel
     const void* idx;
     const __half* coeff;
     const __half* bias;
     __half* y;
     unsigned int* status;
     unsigned int* counters;       // one per quarter of a tile's rows, zero between launches
-    float* part;                  // [KC][NT][MP][TN] sums of the chunks (KC > 1)
+    float* part;                  // [KC][NT][SB_MP][TN] sums of the chunks (KC > 1)
     int M, N, K, KB, NT, C, KC, GN, cache_in_smem, stages;
     int off_cache, off_ring, off_res;
 };
@@ -87,23 +93,23 @@ struct SbQuant {
 // ---------------------------------------------------------------------------------------------
 // activations (with the op in front of the linear) -> digit blob, once per call
 // ---------------------------------------------------------------------------------------------
-// One block per 256-k block and two (padded) activation rows, one warp per row: with 64 threads a block fits beside a resident
-// CTA of the product (61 440 of the SM's registers), and both wait for their predecessors there.  Lane (kw, j) owns the eight elements
+// One block per 256-k block and two (padded) activation rows, one warp per row: with 64 threads of at most 32
+// registers a block fits beside a resident CTA of the product, which leaves 1 024 registers in each quarter of the SM, and both wait
+// for their predecessors there (with 40 registers a call took 6 us more: the quantiser started when the product had ended).  Lane (kw, j) owns the eight elements
 // k = 32 kw + j + 4 e, which are one 32-bit word (nibble e) of every digit: the K order in which the weight expansion
-// leaves the plane bits.  Blob of a k block: [MMA j (NJ)][row group (4)][kw (8)][row (8)][16 B], then 32 rows x 16 B:
+// leaves the plane bits.  Blob of a k block: [MMA j (SB_NJ)][row group (4)][kw (8)][row (8)][16 B], then 32 rows x 16 B:
 // words 0 .. 2 hold the scale bytes of MMA 2 i (bytes 0, 1) and 2 i + 1 (bytes 2, 3) for that B row, word 3 of row m whether
 // activation row m of this block holds a non-finite value.
-template <int NJ>
-__global__ void __launch_bounds__(64) sb_quant_kernel(const SbQuant p) {
+__global__ void __launch_bounds__(64, 32) sb_quant_kernel(const SbQuant p) {
     __shared__ __align__(16) __half row[2][256];
     pdl_launch_dependents();
     pdl_wait();                                    // the activations come from the previous kernel of the stream
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int kb = blockIdx.x, K = p.K, M = p.M, m = blockIdx.y * 2 + wl;
     const int kw = lane >> 2, j = lane & 3;
-    uint32_t words[6] = {0u, 0u, 0u, 0u, 0u, 0u};
-    int ex = 14;
+    int ex = 15;
     bool poison = false;
+    float inv = 0.0f;
     if (m < M) {
         // this warp's 256 activations: lane l brings elements 8 l .. 8 l + 7
         const size_t off = (size_t)m * K + (size_t)kb * 256 + lane * 8;
@@ -168,53 +174,53 @@ __global__ void __launch_bounds__(64) sb_quant_kernel(const SbQuant p) {
         reinterpret_cast<uint4*>(row[wl])[lane] = o;
         __syncwarp();
         const __half* xp = row[wl] + 32 * kw + j;
-        float v[8];
         float a = 0.0f;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-            v[e] = __half2float(xp[4 * e]);
-            float av = fabsf(v[e]);
+            float av = fabsf(__half2float(xp[4 * e]));
             if (!(av == av)) av = __int_as_float(0x7f800000);     // NaN counts as infinity
             a = fmaxf(a, av);
         }
 #pragma unroll
         for (int s = 16; s; s >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, s));
-        float inv = 0.0f;
         if (a >= __int_as_float(0x7f800000)) {
             poison = true;
         } else if (a > 0.0f) {
             ex = (int)((__float_as_uint(a) >> 23) & 0xFF) - 127;              // a = 1.f * 2^ex, ex in [-24, 15]
-            inv = __uint_as_float((uint32_t)(14 - ex + 127) << 23);
+            inv = __uint_as_float((uint32_t)(15 - ex + 127) << 23);
         }
-        // E2M1 codes of digit t - 4 (t = 0 .. 7), one nibble each: the value itself for j = 0, 1, half of it for j = 2, 3
-        const uint32_t lut = (j < 2) ? 0x5420ACDEu : 0x32109ABCu;
+    }
+    unsigned char* blob = p.xb + (size_t)kb * SB_BLOB;
+    // E2M1 codes of digit t - 4 (t = 0 .. 7), one nibble each: the value itself for j = 0, 1, half of it for j = 2, 3
+    const uint32_t lut = (j < 2) ? 0x5420ACDEu : 0x32109ABCu;
+    // one level after the other: a thread must not need more than 32 registers (see above)
+#pragma unroll 1
+    for (int level = 0; level < 2; ++level) {
+        uint32_t words[6] = {0u, 0u, 0u, 0u, 0u, 0u};
+        if (m < M && !poison) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int q = poison ? 0 : __float2int_rn(v[e] * inv);            // |q| <= 2^15
-            const uint32_t u = (uint32_t)(q + 0x24924);
+            for (int e = 0; e < 8; ++e) {
+                const float f = __half2float(row[wl][32 * kw + j + 4 * e]) * inv;              // exact
+                int q = __float2int_rn(f);                                                     // |q| <= 2^16
+                if (level) q = __float2int_rn((f - (float)q) * 131072.0f);                     // the difference is exact; |q| <= 2^16
+                const uint32_t u = (uint32_t)(q + 0x24924);
 #pragma unroll
-            for (int d = 0; d < 6; ++d) {
-                const uint32_t t = (u >> (3 * d)) & 7u;
-                words[d] |= ((lut >> (4u * t)) & 0xFu) << (4 * e);
+                for (int d = 0; d < 6; ++d) words[d] |= ((lut >> (4u * ((u >> (3 * d)) & 7u))) & 0xFu) << (4 * e);
             }
         }
-    }
-    unsigned char* blob = p.xb + (size_t)kb * sb_blob(NJ);
 #pragma unroll
-    for (int d = 0; d < 6; ++d) {
-        const int jm = (NJ == 6) ? d : (d >> 1);
-        const int r = (NJ == 6) ? m : ((d & 1) * 16 + m);
-        *reinterpret_cast<uint32_t*>(blob + jm * 4096 + (r >> 3) * 1024 + kw * 128 + (r & 7) * 16 + j * 4) = words[d];
+        for (int d = 0; d < 6; ++d) {
+            const int dd = level * 6 + d;
+            const int r = (dd & 1) * 16 + m;
+            *reinterpret_cast<uint32_t*>(blob + (dd >> 1) * 4096 + (r >> 3) * 1024 + kw * 128 + (r & 7) * 16 + j * 4) = words[d];
+        }
     }
     // scale bytes 127 + exponent, each twice (two 32-element blocks per MMA); rows beyond M: 2^0 on zero digits
-    auto two = [&](int d) -> uint32_t { return (m < M ? (uint32_t)(127 + 3 * d + ex - 14) : 127u) * 0x0101u; };
-    uint4* sf = reinterpret_cast<uint4*>(blob + NJ * 4096);
-    const uint32_t pw = poison ? 1u : 0u;
-    if (NJ == 6) {
-        if (lane == 0) sf[m] = make_uint4(two(0) | (two(1) << 16), two(2) | (two(3) << 16), two(4) | (two(5) << 16), pw);
-    } else if (lane < 2) {                         // even digits in row m, odd ones in row 16 + m; MMA j has digits 2 j, 2 j + 1
-        sf[lane * 16 + m] = make_uint4(two(lane) | (two(2 + lane) << 16), two(4 + lane) | 0x7F7F0000u, 0x7F7F7F7Fu, pw);
-    }
+    auto two = [&](int d) -> uint32_t { return (m < M ? (uint32_t)(127 + 3 * (d % 6) + ex - (d < 6 ? 15 : 32)) : 127u) * 0x0101u; };
+    uint4* sf = reinterpret_cast<uint4*>(blob + SB_NJ * 4096);
+    if (lane < 2)                                  // even digits in row m, odd ones in row 16 + m; MMA j has digits 2 j, 2 j + 1
+        sf[lane * 16 + m] = make_uint4(two(lane) | (two(2 + lane) << 16), two(4 + lane) | (two(6 + lane) << 16),
+                                       two(8 + lane) | (two(10 + lane) << 16), poison ? 1u : 0u);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -249,9 +255,9 @@ __device__ __forceinline__ unsigned int sb_arrive(unsigned int* counter, int lan
 }
 
 // The chunks' sums of a quarter of a tile's rows -> y, in chunk order; the counter goes back to zero.
-template <int MP, int TN>
+template <int TN>
 __device__ __forceinline__ void sb_add_chunks(const SbParams& p, int tile, int quarter, int lane) {
-    constexpr int QR = TN / 4, PER = MP * QR / 32;
+    constexpr int MP = SB_MP, QR = TN / 4, PER = MP * QR / 32, H = 16 / PER;
     if (lane == 0) p.counters[tile * 4 + quarter] = 0u;
     __threadfence();
     const size_t plane = (size_t)p.NT * (MP * TN);
@@ -260,17 +266,17 @@ __device__ __forceinline__ void sb_add_chunks(const SbParams& p, int tile, int q
 #pragma unroll
     for (int u = 0; u < PER; ++u) v[u] = 0.0f;
 #pragma unroll 1
-    for (int c = 0; c < p.KC; c += 2) {            // two chunks' loads in flight
-        float t[2][PER];
+    for (int c = 0; c < p.KC; c += H) {            // H chunks' loads in flight
+        float t[H][PER];
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < H; ++h)
 #pragma unroll
             for (int u = 0; u < PER; ++u) {
                 const int q = lane + 32 * u, m = q / QR;
                 t[h][u] = (c + h < p.KC && m < p.M) ? __ldcg(src + (size_t)(c + h) * plane + m * TN + q % QR) : 0.0f;
             }
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < H; ++h)
 #pragma unroll
             for (int u = 0; u < PER; ++u) v[u] += t[h][u];
     }
@@ -281,17 +287,16 @@ __device__ __forceinline__ void sb_add_chunks(const SbParams& p, int tile, int q
     }
 }
 
-template <int S, int NSUB, int NJ, int IDXB>
+template <int S, int NSUB, int IDXB>
 __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_constant__ CUtensorMap tmap, const SbParams p) {
     pdl_launch_dependents();
     extern __shared__ __align__(1024) unsigned char smem[];
     constexpr int SP = ts_sp(S);
     constexpr int TN = ts_tn(S);
-    constexpr int MP = (NJ == 3) ? 16 : 32;        // activation rows the accumulators cover
+    constexpr int MP = SB_MP, NJ = SB_NJ;
     constexpr int NV = MP / SP;                    // ... and how many of them one thread finishes
     constexpr int ABUF = NSUB == 2 ? 1 : 2;        // A buffers
-    constexpr int SFC = sb_sfcols(NJ);
-    constexpr int BLOB = sb_blob(NJ);
+    constexpr int SFC = SB_SFCOLS, BLOB = SB_BLOB;
     constexpr int WROW = TN * S * 4;               // bytes of one 32-k row of a stage
     constexpr int CI_BYTES = (IDXB == 0) ? TN * S * 2 : TN * IDXB;
     constexpr uint32_t A_TX = 8 * WROW + NSUB * CI_BYTES;
@@ -470,7 +475,7 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                 const uint4 sf = reinterpret_cast<const uint4*>(Bs + (size_t)b * BLOB + NJ * 4096)[lane];
                 const uint32_t at = tbase + lane_sel + SB_SFB_COL + b * SFC;
                 ts_st8(at, sf.x, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, sf.y, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
-                if (NJ == 6) ts_st8(at + 8, sf.z, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
+                ts_st8(at + 8, sf.z, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu, 0x7F7F7F7Fu);
                 pm |= __ballot_sync(0xffffffffu, lane < MP && sf.w != 0u);
                 if (wl == 0 && b == nkb - 1) *poison_s = pm;
                 ts_wait_st();
@@ -493,7 +498,7 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                 pend = 2;
             } else if (pend == 2) {
                 pend = 0;
-                if (__shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<MP, TN>(p, ptile, wl, lane);
+                if (__shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<TN>(p, ptile, wl, lane);
             }
         };
         // Sums of one tile's units: planes added across their lanes, after which a lane has the activation rows
@@ -602,32 +607,30 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
             if (ABUF == 2) next();
             ts_wait(mbar, (uint32_t)(i & 1), abort_flag, p.status, 0x434u);
             ts_fence_after();
-            uint32_t d[NSUB][4][8];
+            // the sums of one group: even and odd digits of every activation row
+            SbPair v[NSUB][MP / 2];
+            auto read = [&](int sub) {
+                uint32_t d[4][8];
+                ts_ld16_issue(d_addr + sub * 32, d[0], d[1]);
+                ts_ld16_issue(d_addr + sub * 32 + 16, d[2], d[3]);
+                if (ABUF == 1 && sub == 0) next();
 #pragma unroll
-            for (int sub = 0; sub < NSUB; ++sub) {
-                ts_ld16_issue(d_addr + sub * 32, d[sub][0], d[sub][1]);
-                ts_ld16_issue(d_addr + sub * 32 + 16, d[sub][2], d[sub][3]);
-            }
-            if (ABUF == 1) next();
+                for (int g4 = 0; g4 < 4; ++g4) ts_wait_ld(d[g4]);
 #pragma unroll
-            for (int sub = 0; sub < NSUB; ++sub)
+                for (int m = 0; m < MP; m += 2)
+                    v[sub][m / 2] = SbPair(d[m >> 3][m & 7], d[m >> 3][(m & 7) + 1]) + SbPair(d[2 + (m >> 3)][m & 7], d[2 + (m >> 3)][(m & 7) + 1]);
+            };
 #pragma unroll
-                for (int g4 = 0; g4 < 4; ++g4) ts_wait_ld(d[sub][g4]);
+            for (int sub = 0; sub < NSUB; ++sub) read(sub);      // (one after the other: both groups' columns at once spill)
             if (more) {
                 ts_wait_st();
                 ts_fence_before();
                 ts_bar_arrive(1 + w, 160);         // releases the MMAs of unit i + 1; also: its stage has been read
             }
 #pragma unroll
-            for (int sub = 0; sub < NSUB; ++sub) {
-                const SbPair cc(c0[sub], c0[sub]);
+            for (int sub = 0; sub < NSUB; ++sub)
 #pragma unroll
-                for (int m = 0; m < MP; m += 2) {
-                    SbPair v(d[sub][m >> 3][m & 7], d[sub][m >> 3][(m & 7) + 1]);
-                    if (NJ == 3) v = v + SbPair(d[sub][2 + (m >> 3)][m & 7], d[sub][2 + (m >> 3)][(m & 7) + 1]);
-                    acc[m / 2] = v.mul_add(cc, acc[m / 2]);
-                }
-            }
+                for (int m = 0; m < MP / 2; ++m) acc[m] = v[sub][m].mul_add(SbPair(c0[sub], c0[sub]), acc[m]);
             ++have;
             if (KC > 1 && pend) settle();
             if (++kl == nkb || !more) {
@@ -676,9 +679,9 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
             }
         }
     }
-    if (pend == 2 && __shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<MP, TN>(p, ptile, warp & 3, lane);
+    if (pend == 2 && __shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<TN>(p, ptile, warp & 3, lane);
     if (shared_tile >= 0 && __shfl_sync(0xffffffffu, shared_old, 0) == (unsigned int)(KC - 1))
-        sb_add_chunks<MP, TN>(p, shared_tile, warp & 3, lane);
+        sb_add_chunks<TN>(p, shared_tile, warp & 3, lane);
     if (threadIdx.x == 0 && *abort_flag) {         // which problem gave up: N, and K / 256 | M | CTA (for the host's message)
         atomicExch(p.status + 2, (unsigned int)p.N);
         atomicExch(p.status + 3, ((unsigned int)p.KB << 16) | ((unsigned int)M << 8) | (blockIdx.x & 0xFFu));
@@ -689,21 +692,19 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
 // host
 // ---------------------------------------------------------------------------------------------
 struct SbPlan {
-    int KB, NT, NJ, KC, GN, cache_in_smem, stages, smem;
+    int KB, NT, KC, GN, cache_in_smem, stages, smem;
     int off_cache, off_ring, off_res;
     size_t blob_bytes, part_bytes;
 };
 
-static int sb_plan(const PackedW& w, int M, const DeviceInfo& di, SbPlan* pl) {
-    const int TN = ts_tn(w.S);
-    pl->NJ = M <= 16 ? 3 : 6;
-    const int MP = pl->NJ == 3 ? 16 : 32;
+static int sb_plan(const PackedW& w, const DeviceInfo& di, SbPlan* pl) {
+    const int TN = ts_tn(w.S), MP = SB_MP;
     pl->KB = w.K / 256;
     pl->NT = w.N / TN;
     if (pl->KB < 1 || pl->NT < 1) return SBVR_ERR_UNSUPPORTED;
     // Chunks as large as shared memory holds; smaller ones while less than two thirds of the SMs would have work and a
     // warpgroup more than one unit.
-    pl->KC = (pl->KB + sb_chunk(pl->NJ) - 1) / sb_chunk(pl->NJ);
+    pl->KC = (pl->KB + SB_CHUNK - 1) / SB_CHUNK;
     auto groups = [&](int kc) { const int g = di.sm_count / kc; return g < 1 ? 1 : (g < pl->NT ? g : pl->NT); };
     while (groups(pl->KC) * pl->KC * 3 <= di.sm_count * 2 && pl->KC * 2 <= pl->KB && pl->KC * 2 <= 16 &&
            (pl->NT + groups(pl->KC) - 1) / groups(pl->KC) * (pl->KB / pl->KC) > SB_NWG)
@@ -711,11 +712,11 @@ static int sb_plan(const PackedW& w, int M, const DeviceInfo& di, SbPlan* pl) {
     pl->GN = groups(pl->KC);
     const int nkb = (pl->KB + pl->KC - 1) / pl->KC;
     if (pl->KC > 1 && (size_t)pl->NT * 16 > SBVR_WS_XCHG_BYTES) return SBVR_ERR_UNSUPPORTED;     // arrival counters
-    pl->blob_bytes = ((size_t)pl->KB * sb_blob(pl->NJ) + 255) / 256 * 256;
+    pl->blob_bytes = ((size_t)pl->KB * SB_BLOB + 255) / 256 * 256;
     pl->part_bytes = pl->KC > 1 ? (size_t)pl->KC * pl->NT * MP * TN * 4 : 0;
     const int cache_bytes = w.idx_bytes ? ts_round_up(w.C * w.S * 2, 16) : 0;
     auto layout = [&](int cb, int stages) {
-        pl->off_cache = SB_HDR + nkb * sb_blob(pl->NJ);
+        pl->off_cache = SB_HDR + nkb * SB_BLOB;
         pl->off_ring = ts_round_up(pl->off_cache + cb, 128);
         pl->off_res = pl->off_ring + SB_NWG * stages * SB_ASTAGE;
         return pl->off_res + SB_NWG * 2 * MP * TN * 4;
@@ -733,8 +734,7 @@ static int sb_plan(const PackedW& w, int M, const DeviceInfo& di, SbPlan* pl) {
 bool linear_sb_supported(const PackedW& w, int M) {
     if (w.S < 2 || w.S > 4) return false;
     if (w.G != 256 && w.G != 128) return false;
-    if (M < 2 || M > 32) return false;
-    if (w.G == 128 && M > 16) return false;
+    if (M < 2 || M > SB_MP) return false;
     if (w.N % ts_tn(w.S) || w.K % 256 || w.K > 32768) return false;
     if (w.idx_bytes < 0 || w.idx_bytes > 2) return false;
     if (reinterpret_cast<uintptr_t>(w.coeff) & 15) return false;                 // bulk copies
@@ -746,35 +746,57 @@ bool linear_sb_supported(const PackedW& w, int M) {
     int dev = 0;
     SbPlan pl;
     if (cudaGetDevice(&dev) != cudaSuccess || device_info(dev, &di) != SBVR_OK) return false;
-    return sb_plan(w, M, di, &pl) == SBVR_OK;
+    return sb_plan(w, di, &pl) == SBVR_OK;
 }
 
-size_t linear_sb_workspace_bytes(const PackedW& w, int M, const DeviceInfo& di) {
+// Where it is faster than the GEMM.  Up to four chunks of K always (M = 16, us, the GEMM in brackets: 2048 x 2048 9.4 (10.8),
+// 4096 x 4096 12.5 (15.4), with three planes 12.4 (14.4), two 12.4 (13.1), groups of 128 13.7 (15.1)), and on weights of few rows, which
+// leave the GEMM few tiles (128 x 14336 11.2 (23.6), 512 x 14336 17.0 (19.7), 1024 x 11008 17.8 (25.7), 1024 x 14336 19.4 (18.3)); with
+// up to eight chunks on weights of many rows (10240 x 8192 46 (58), 28672 x 8192 107 (112), but 8192 x 8192 38 (36) and, with groups of
+// 128, 28672 x 8192 116 (110)); beyond, the chunks' merge costs more than is gained: 4096 x 11008 33 (27), 4096 x 14336 40 (32).
+bool linear_sb_preferred(const PackedW& w) { return w.K <= 4096 || w.N <= 1024 || (w.K <= 8192 && w.N > 8192 && w.G == 256); }
+
+size_t linear_sb_workspace_bytes(const PackedW& w, const DeviceInfo& di) {
     SbPlan pl;
-    if (sb_plan(w, M, di, &pl) != SBVR_OK) return 0;
+    if (sb_plan(w, di, &pl) != SBVR_OK) return 0;
     return pl.blob_bytes + pl.part_bytes;
 }
 
-template <int S, int NSUB, int NJ, int IDXB>
-static int sb_launch_inst(const CUtensorMap& tm, const SbParams& p, int grid, int smem, cudaStream_t st) {
-    static SmemOnce once;
-    const int rc = set_max_smem_once(once, linear_sb_kernel<S, NSUB, NJ, IDXB>, 227 * 1024);
-    if (rc) return rc;
-    SBVR_CUDA_TRY(launch_pdl(linear_sb_kernel<S, NSUB, NJ, IDXB>, dim3(grid), dim3(SB_THREADS), (size_t)smem, st, tm, p));
+// The kernel asks for all of the SM's shared memory, once per device: a CTA whose size just filled a smaller carve-out (196 KB
+// with three planes and 4 096 lines) left no room for the next call's quantiser beside it, and a call took 8 us more.
+template <typename Kernel>
+static int sb_setup(SmemOnce& once, Kernel kernel, int bytes) {
+    int dev = 0;
+    SBVR_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return SBVR_ERR_BAD_ARG;
+    std::lock_guard<std::mutex> lock(once.mu);
+    if (!once.done[dev]) {
+        SBVR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        SBVR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        once.done[dev] = true;
+    }
     return SBVR_OK;
 }
-template <int S, int NSUB, int NJ>
+
+template <int S, int NSUB, int IDXB>
+static int sb_launch_inst(const CUtensorMap& tm, const SbParams& p, int grid, int smem, cudaStream_t st) {
+    static SmemOnce once;
+    const int rc = sb_setup(once, linear_sb_kernel<S, NSUB, IDXB>, 227 * 1024);
+    if (rc) return rc;
+    SBVR_CUDA_TRY(launch_pdl(linear_sb_kernel<S, NSUB, IDXB>, dim3(grid), dim3(SB_THREADS), (size_t)smem, st, tm, p));
+    return SBVR_OK;
+}
+template <int S, int NSUB>
 static int sb_launch_idx(const CUtensorMap& tm, const SbParams& p, int idxb, int grid, int smem, cudaStream_t st) {
     switch (idxb) {
-        case 0: return sb_launch_inst<S, NSUB, NJ, 0>(tm, p, grid, smem, st);
-        case 1: return sb_launch_inst<S, NSUB, NJ, 1>(tm, p, grid, smem, st);
-        default: return sb_launch_inst<S, NSUB, NJ, 2>(tm, p, grid, smem, st);
+        case 0: return sb_launch_inst<S, NSUB, 0>(tm, p, grid, smem, st);
+        case 1: return sb_launch_inst<S, NSUB, 1>(tm, p, grid, smem, st);
+        default: return sb_launch_inst<S, NSUB, 2>(tm, p, grid, smem, st);
     }
 }
 template <int S>
-static int sb_launch_g(const CUtensorMap& tm, const SbParams& p, int G, int NJ, int idxb, int grid, int smem, cudaStream_t st) {
-    if (G == 128) return sb_launch_idx<S, 2, 3>(tm, p, idxb, grid, smem, st);
-    return NJ == 3 ? sb_launch_idx<S, 1, 3>(tm, p, idxb, grid, smem, st) : sb_launch_idx<S, 1, 6>(tm, p, idxb, grid, smem, st);
+static int sb_launch_g(const CUtensorMap& tm, const SbParams& p, int G, int idxb, int grid, int smem, cudaStream_t st) {
+    return G == 128 ? sb_launch_idx<S, 2>(tm, p, idxb, grid, smem, st) : sb_launch_idx<S, 1>(tm, p, idxb, grid, smem, st);
 }
 
 // `counters` (SBVR_WS_XCHG_BYTES, zero between calls: the kernel leaves them zero) and `scratch` (256-byte aligned,
@@ -790,7 +812,7 @@ int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __ha
     if (rc) return rc;
     if (di.cc_major != 10) return SBVR_ERR_UNSUPPORTED;
     SbPlan pl;
-    rc = sb_plan(w, M, di, &pl);
+    rc = sb_plan(w, di, &pl);
     if (rc) return rc;
     if (pl.blob_bytes + pl.part_bytes > scratch_bytes) return SBVR_ERR_WORKSPACE;
     CUtensorMap tm;
@@ -800,8 +822,7 @@ int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __ha
     q.x = x, q.xb = reinterpret_cast<unsigned char*>(scratch), q.M = M, q.K = w.K;
     rc = xop_check(xop, x, M, w.K, &q.x_op, &q.delta, &q.norm_w, &q.h_out, &q.eps);
     if (rc) return rc;
-    if (pl.NJ == 3) SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel<3>, dim3(pl.KB, 8), dim3(64), 0, st, q));
-    else SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel<6>, dim3(pl.KB, 16), dim3(64), 0, st, q));
+    SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel, dim3(pl.KB, SB_MP / 2), dim3(64), 0, st, q));
     SbParams p;
     p.xb = q.xb;
     p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status, p.counters = counters;
@@ -811,9 +832,9 @@ int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __ha
     p.off_cache = pl.off_cache, p.off_ring = pl.off_ring, p.off_res = pl.off_res;
     const int grid = pl.GN * pl.KC;
     switch (w.S) {
-        case 2: return sb_launch_g<2>(tm, p, w.G, pl.NJ, w.idx_bytes, grid, pl.smem, st);
-        case 3: return sb_launch_g<3>(tm, p, w.G, pl.NJ, w.idx_bytes, grid, pl.smem, st);
-        default: return sb_launch_g<4>(tm, p, w.G, pl.NJ, w.idx_bytes, grid, pl.smem, st);
+        case 2: return sb_launch_g<2>(tm, p, w.G, w.idx_bytes, grid, pl.smem, st);
+        case 3: return sb_launch_g<3>(tm, p, w.G, w.idx_bytes, grid, pl.smem, st);
+        default: return sb_launch_g<4>(tm, p, w.G, w.idx_bytes, grid, pl.smem, st);
     }
 }
 

@@ -338,12 +338,22 @@ class SBVRLlamaForCausalLM(torch.nn.Module):
         # SiLU * up in front of down are folded into those linears' kernels.  The folded norm cannot update the
         # residual in place (other CTAs still read it), so the residual alternates between two buffers.
         fuse = self.fuse_glue and T <= 16
+
+        def folds(lin) -> bool:
+            """More than four rows: the small-batch kernel takes the op, so fold where `linear` would take that kernel too (the rule of
+            algo 0: linear_sb_preferred in csrc/linear_sb.cu); elsewhere the op's own launch and the GEMM are faster."""
+            if not (fuse and isinstance(lin, SBVRLinear)):
+                return False
+            w = lin.weight
+            K = w.in_features_padded
+            N = w.out_features
+            return T <= 4 or K <= 4096 or N <= 1024 or (K <= 8192 and N > 8192 and w.bvr_len == 256)
         hc, ho = b.h, b.h2                         # current residual, spare buffer
 
         def norm_linear(lin, delta, weight, out, keep_residual=True):
             """out = lin(rmsnorm(hc + delta) * weight); the residual becomes hc + delta."""
             nonlocal hc, ho
-            if fuse and isinstance(lin, SBVRLinear) and linear_fused(
+            if folds(lin) and linear_fused(
                     XOP_ADD_RMSNORM, hc, lin.weight, out, delta=delta, norm_weight=weight,
                     h_out=ho if keep_residual else None, eps=eps, bias=lin.bias):
                 if keep_residual:
@@ -398,7 +408,7 @@ class SBVRLlamaForCausalLM(torch.nn.Module):
             down_out = comm.partial_out(2 * li + 1, T) if comm is not None else b.down
             pushed = (comm is not None and fuse and self.pushed_allreduce and isinstance(layer.down_proj, SBVRLinear) and
                       comm.push_linear(2 * li + 1, XOP_SILU_MUL, b.gu, layer.down_proj.weight, T, bias=layer.down_proj.bias))
-            if not pushed and not (fuse and isinstance(layer.down_proj, SBVRLinear) and
+            if not pushed and not (folds(layer.down_proj) and
                                    linear_fused(XOP_SILU_MUL, b.gu, layer.down_proj.weight, down_out, bias=layer.down_proj.bias)):
                 ck(L.sbvr_silu_mul_f16(b.gu.data_ptr(), b.act.data_ptr(), T, self.inter, st), "silu_mul")
                 layer.down_proj(b.act, out=down_out)

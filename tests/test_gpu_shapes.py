@@ -196,3 +196,38 @@ def test_ops_folded_into_decode_linears(M, N, K, op):
     ref = sbvr.linear(act, w).float()
     assert ((y.float() - ref).abs().max() / ref.abs().max()).item() < (1e-6 if op == "silu" and M <= 4 else 2e-3)
     check_status()
+
+
+def _planes(p, G):
+    """Plane bits [S, N, K] and the coefficients of every element [S, N, K], in fp64."""
+    KW, N, S = p["bvr"].shape
+    bits = ((p["bvr"].transpose(2, 1, 0)[..., None] >> np.arange(32, dtype=np.uint32)) & 1).reshape(S, N, KW * 32)
+    c = p["coeff"].astype(np.float64)
+    c = c[p["coeff_idx"].astype(np.int64)] if p.get("coeff_idx") is not None else c
+    return bits.astype(np.float64), np.repeat(c.transpose(2, 1, 0), G, axis=2)
+
+
+@pytest.mark.parametrize("M", [5, 16])
+@pytest.mark.parametrize("N,K,G,S,mode", [(256, 2048, 256, 4, "u16"), (96, 4096, 128, 3, "u8"), (128, 768, 256, 2, "direct")])
+@pytest.mark.parametrize("power", [8, 11, 13, 15])
+@pytest.mark.parametrize("algo", [0, 4])
+def test_one_large_activation_among_small_ones(M, N, K, G, S, mode, power, algo):
+    """One activation of 2^power in every block of 256 values near one; half of the outputs have no plane bit there and must
+    come out as if it were not.  Error per output: one fp16 rounding (2^-11 of the value), and fp32 sums of up to K products per
+    plane, 2^-18 of the sum of their magnitudes (the activations themselves are held to 2^-33 of their block's largest)."""
+    import sbvr
+    p = O.make_packed(N, K, S, G=G, mode=mode, C=256 if mode == "u8" else 1000, seed=N + power)
+    rng = np.random.default_rng(M + power)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    at = np.arange(0, K, 256) + rng.integers(0, 256, K // 256)
+    x[:, at] = (np.exp2(power) * rng.uniform(1.0, 1.9, (M, K // 256))).astype(np.float16)
+    for k in at:
+        p["bvr"][k // 32, :N // 2, :] &= np.uint32(~(1 << (k % 32)) & 0xFFFFFFFF)
+    bits, c = _planes(p, G)
+    ref = x.astype(np.float64) @ (bits * c).sum(0).T
+    mass = np.abs(x.astype(np.float64)) @ (bits * np.abs(c)).sum(0).T
+    y = h2n(sbvr.linear(torch.from_numpy(x).cuda(), to_sbvr(p), None, algo=algo)).astype(np.float64)
+    ok = np.abs(ref) < 65000
+    assert ok[:, :N // 2].all()
+    assert (np.abs(y - ref) <= 2.0 ** -11 * np.abs(ref) + 2.0 ** -18 * mass + 2.0 ** -25)[ok].all()
+    check_status()
