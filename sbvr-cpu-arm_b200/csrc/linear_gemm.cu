@@ -50,7 +50,7 @@ constexpr int GM_TMEM_COLS = 512;
 // MMAs per 16 k, 256 columns and the rest, and a decoded weight tile serves up to 1.5 times as many activations.
 constexpr int GM_WIDE = 384;
 // Ring of 64-k stages: a decoded 128 x 64 weight tile in tensor memory and the activation block in shared memory.
-__host__ __device__ constexpr int gm_slots(int NX) { return NX == GM_WIDE ? 4 : 6; }
+__host__ __device__ constexpr int gm_slots(int NX, bool EXACT) { return (NX == GM_WIDE || EXACT) ? 4 : 6; }
 __host__ __device__ constexpr int gm_a_col(int NX) { return NX == GM_WIDE ? 384 : 256; }   // D occupies columns [0, NX), the A ring is behind
 constexpr int GM_HDR = 1024;
 
@@ -95,6 +95,28 @@ __device__ __forceinline__ void gm_st32(uint32_t taddr, const uint32_t (&a)[32])
         "r"(a[19]), "r"(a[20]), "r"(a[21]), "r"(a[22]), "r"(a[23]), "r"(a[24]), "r"(a[25]), "r"(a[26]), "r"(a[27]),
         "r"(a[28]), "r"(a[29]), "r"(a[30]), "r"(a[31])
         : "memory");
+}
+__device__ __forceinline__ void gm_st16(uint32_t taddr, const uint32_t (&a)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(a[4]), "r"(a[5]), "r"(a[6]), "r"(a[7]), "r"(a[8]), "r"(a[9]),
+        "r"(a[10]), "r"(a[11]), "r"(a[12]), "r"(a[13]), "r"(a[14]), "r"(a[15])
+        : "memory");
+}
+// A pair of weights as two fp16 parts each, of the same sign and never zero unless the weight is at most 2^-24: part one is cut
+// towards zero a little below the weight, part two is the rest (weights are multiples of 2^-24, so below 2^-3 it is exact; above,
+// the two parts hold 21 bits).  Same signs and no zeros, so that an infinite activation gives what one product would.
+__device__ __forceinline__ void gm_two_parts(float v0, float v1, bool odd, uint32_t& hi, uint32_t& lo) {
+    constexpr float BELOW = 1.0f - 1.0f / 4096;
+    asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(v1 * BELOW), "f"(v0 * BELOW));
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+    float r0 = v0 - f.x, r1 = v1 - f.y;
+    if (odd) {                                     // a coefficient that is not finite: part one says it all
+        if (!(fabsf(v0) < INFINITY)) r0 = 0.0f;
+        if (!(fabsf(v1) < INFINITY)) r1 = 0.0f;
+    }
+    const __half2 r = __floats2half2_rn(r0, r1);
+    lo = *reinterpret_cast<const uint32_t*>(&r);
 }
 __device__ __forceinline__ void gm_ld32(uint32_t taddr, float (&d)[32]) {
     uint32_t r[32];
@@ -214,12 +236,19 @@ static __device__ __forceinline__ void gm_add_parts(const float* part, size_t pl
 
 // SPLIT: K is split over several CTAs (p.KS > 1).  A kernel of its own: its CTAs have one work item each (gm_plan), so that the
 // epilogue, which needs the registers of the decoding loop, comes behind that loop and not inside it.
-template <int S, int NX, bool SPLIT>
+// EXACT: weights are formed in fp32 and multiplied in two fp16 parts (gm_two_parts), two MMAs per 16 k on the same activations, for
+// the row counts that are no multiple of 128, which the CUDA-core kernel with its fp32 weights served before.  Formed in fp16 with
+// one rounding per plane the weights gave errors of 3.1e-4 of the result (2-norm) where that kernel has 2.1e-4, the rounding of
+// the result; so have two parts.  37 x 3000 x 3000, S = 3: 17 us (14 with fp16 weights, 70 on CUDA cores); 1000 x 3000 x 4096,
+// S = 4: 62 us (37, 2 190).
+template <int S, int NX, bool SPLIT, bool EXACT>
 __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     constexpr int NX1 = NX == GM_WIDE ? 256 : NX;  // columns of the first MMA
     constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NX1 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-    constexpr int GM_SLOTS = gm_slots(NX), GM_A_COL = gm_a_col(NX);
+    constexpr int GM_SLOTS = gm_slots(NX, EXACT), GM_A_COL = gm_a_col(NX);
+    constexpr int ACOLS = EXACT ? 64 : 32;         // tensor-memory columns of a decoded tile
+    static_assert(GM_A_COL + GM_SLOTS * ACOLS <= GM_TMEM_COLS && NX <= GM_A_COL, "tensor memory");
     const int nx = NX == GM_WIDE ? p.nx : NX;
     const uint32_t STAGE_BYTES = (uint32_t)nx * 128u;
     const uint32_t idesc2 = (1u << 4) | ((uint32_t)((nx - NX1) >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -319,8 +348,9 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const uint32_t acc = q ? 1u : (uint32_t)(ks != 0);
-                        gm_mma(0, GM_A_COL + slot * 32 + q * 8, d + q * 16, IDESC, acc);
-                        if (NX == GM_WIDE) gm_mma(NX1, GM_A_COL + slot * 32 + q * 8, d + NX1 * 8 + q * 16, idesc2, acc);
+                        gm_mma(0, GM_A_COL + slot * ACOLS + q * 8, d + q * 16, IDESC, acc);
+                        if (EXACT) gm_mma(0, GM_A_COL + slot * ACOLS + 32 + q * 8, d + q * 16, IDESC, 1u);
+                        if (NX == GM_WIDE) gm_mma(NX1, GM_A_COL + slot * ACOLS + q * 8, d + NX1 * 8 + q * 16, idesc2, acc);
                     }
                     gm_commit(&empty[slot]);
                     if (++ks == SPP) {
@@ -484,6 +514,52 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
         auto decode_stage = [&](const Pos& q, const uint32_t (&w)[2][S], const unsigned short (&c)[S]) {
             if constexpr (!SPLIT)                  // (a CTA of a split problem has one item)
                 while (ep_item < q.item) epilogue();   // items whose stages have all been handed to the issuer
+            const int slot = q.it % GM_SLOTS;
+            // false: a wait ran out here or elsewhere
+            auto slot_free = [&]() -> bool {
+                if (!dead && !mbar_wait_async(&empty[slot], ((uint32_t)(q.it / GM_SLOTS) & 1u) ^ 1u)) {
+                    dead = true;
+                    flags[0] = 1;
+                }
+                dead = __any_sync(0xffffffffu, dead);
+                if (!dead) gm_fence_after();
+                return !dead;
+            };
+            auto hand_over = [&]() {
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                gm_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[slot]);
+            };
+            if constexpr (EXACT) {
+                float cf[S];
+                bool odd = false;
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                    cf[s] = __half2float(__ushort_as_half(c[s]));
+                    odd |= !(fabsf(cf[s]) < INFINITY);
+                }
+                odd = __any_sync(0xffffffffu, odd);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    uint32_t hi[16], lo[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        float v0 = 0.0f, v1 = 0.0f;
+#pragma unroll
+                        for (int s = 0; s < S; ++s) {
+                            if (w[h][s] & (1u << j)) v0 += cf[s];
+                            if (w[h][s] & (0x10000u << j)) v1 += cf[s];
+                        }
+                        gm_two_parts(v0, v1, odd, hi[j], lo[j]);
+                    }
+                    if (h == 0 && !slot_free()) return;
+                    gm_st16(tbase + lane_sel + GM_A_COL + slot * ACOLS + h * 16, hi);
+                    gm_st16(tbase + lane_sel + GM_A_COL + slot * ACOLS + 32 + h * 16, lo);
+                }
+                hand_over();
+                return;
+            }
             // A lone bit at position 10 .. 14 of a half is the number 2^-14, 2^-13, 2^-11, 2^-7, 2^1: masking a packed
             // word with 0x04000400 << i leaves (bit, bit + 16) as such a half2, and one HFMA2 with c_s divided by that
             // number adds c_s where the bit is set.  Three shifted copies of the word bring all 16 bit pairs into the
@@ -503,7 +579,6 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                 mul[s][3] = __hmul2(c2, __float2half2_rn(128.0f));
                 mul[s][4] = __hmul2(c2, __float2half2_rn(0.5f));
             }
-            const int slot = q.it % GM_SLOTS;
             uint32_t a[32];
             if (!__any_sync(0xffffffffu, big)) {
 #pragma unroll
@@ -554,18 +629,9 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                 }
             }
             // the slot is waited for with the values in registers: the decode runs beside the MMAs that still read the slot
-            if (!dead && !mbar_wait_async(&empty[slot], ((uint32_t)(q.it / GM_SLOTS) & 1u) ^ 1u)) {
-                dead = true;
-                flags[0] = 1;
-            }
-            dead = __any_sync(0xffffffffu, dead);
-            if (dead) return;
-            gm_fence_after();
-            gm_st32(tbase + lane_sel + GM_A_COL + slot * 32, a);
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            gm_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full[slot]);
+            if (!slot_free()) return;
+            gm_st32(tbase + lane_sel + GM_A_COL + slot * ACOLS, a);
+            hand_over();
         };
 
         while (cur.item < p.items) {
@@ -613,6 +679,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
 // ---------------------------------------------------------------------------------------------
 struct GmPlan {
     int NX, MT, NT, KS, SPP, items, grid, smem;
+    bool exact;
     size_t xt_bytes, part_bytes;
 };
 
@@ -623,8 +690,9 @@ struct GmPlan {
 // 2048 x 14336 x 4096 (7 rounds -> 5 of 352 rows), 350 -> 302 us at 3000 x 4096 x 14336 (3 -> 2), 78 -> 59 us at 1500 x 4096 x
 // 4096 (2 -> 1 of 384 rows); 2048 x 4096 stays at 256 rows (2 rounds either way).  Problems that do not fill the GPU at 256 rows
 // split K instead.
-static int gm_nx(int M, int NT, int S, int sm_count) {
-    if (M <= 256) return M <= 32 ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
+// Two-part weights fill the tensor memory of wide tiles: 256 rows at most, 64 at least (one instantiation less).
+static int gm_nx(int M, int NT, int S, int sm_count, bool exact) {
+    if (M <= 256 || exact) return (M <= 32 && !exact) ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
     int best = 256;
     long long cost = 0;
     for (int nx = 256; nx <= GM_WIDE; nx += 32) {
@@ -648,7 +716,8 @@ bool linear_gemm_supported(const PackedW& w, int M) {
 
 static void gm_plan(const PackedW& w, int M, int sm_count, GmPlan* pl) {
     pl->NT = (w.N + 127) / 128;
-    pl->NX = gm_nx(M, pl->NT, w.S, sm_count);
+    pl->exact = w.N % 128 != 0;
+    pl->NX = gm_nx(M, pl->NT, w.S, sm_count, pl->exact);
     pl->MT = (M + pl->NX - 1) / pl->NX;
     const int KST = w.K / 64;
     int ks = 1;
@@ -665,7 +734,7 @@ static void gm_plan(const PackedW& w, int M, int sm_count, GmPlan* pl) {
     pl->SPP = KST / ks;
     pl->items = tiles * ks;
     pl->grid = pl->items < sm_count ? pl->items : sm_count;
-    pl->smem = GM_HDR + gm_slots(pl->NX > 256 ? GM_WIDE : pl->NX) * pl->NX * 128;
+    pl->smem = GM_HDR + gm_slots(pl->NX > 256 ? GM_WIDE : pl->NX, pl->exact) * pl->NX * 128;
     pl->xt_bytes = ((size_t)pl->MT * pl->NX * w.K * 2 + 255) / 256 * 256;
     pl->part_bytes = ks > 1 ? (size_t)ks * pl->MT * pl->NX * w.N * 4 : 0;
 }
@@ -676,26 +745,31 @@ size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count) {
     return pl.xt_bytes + pl.part_bytes;
 }
 
-template <int S, int NX, bool SPLIT>
+template <int S, int NX, bool SPLIT, bool EXACT>
 static int gm_launch_split(const GmParams& p, int grid, int smem, cudaStream_t st) {
     static SmemOnce once;
-    const int rc = set_max_smem_once(once, linear_gemm_kernel<S, NX, SPLIT>, 227 * 1024);
+    const int rc = set_max_smem_once(once, linear_gemm_kernel<S, NX, SPLIT, EXACT>, 227 * 1024);
     if (rc) return rc;
-    SBVR_CUDA_TRY(launch_pdl(linear_gemm_kernel<S, NX, SPLIT>, dim3(grid), dim3(GM_THREADS), (size_t)smem, st, p));
+    SBVR_CUDA_TRY(launch_pdl(linear_gemm_kernel<S, NX, SPLIT, EXACT>, dim3(grid), dim3(GM_THREADS), (size_t)smem, st, p));
     return SBVR_OK;
 }
-template <int S, int NX>
+template <int S, int NX, bool EXACT = false>
 static int gm_launch_inst(const GmParams& p, int grid, int smem, cudaStream_t st) {
-    return p.KS > 1 ? gm_launch_split<S, NX, true>(p, grid, smem, st) : gm_launch_split<S, NX, false>(p, grid, smem, st);
+    return p.KS > 1 ? gm_launch_split<S, NX, true, EXACT>(p, grid, smem, st) : gm_launch_split<S, NX, false, EXACT>(p, grid, smem, st);
 }
 template <int S>
-static int gm_launch_nx(const GmParams& p, int NX, int grid, int smem, cudaStream_t st) {
-    switch (NX) {
-        case 32: return gm_launch_inst<S, 32>(p, grid, smem, st);
-        case 64: return gm_launch_inst<S, 64>(p, grid, smem, st);
-        case 128: return gm_launch_inst<S, 128>(p, grid, smem, st);
-        case 256: return gm_launch_inst<S, 256>(p, grid, smem, st);
-        default: return gm_launch_split<S, GM_WIDE, false>(p, grid, smem, st);
+static int gm_launch_nx(const GmParams& p, const GmPlan& pl, cudaStream_t st) {
+    if (pl.exact) switch (pl.NX) {
+        case 64: return gm_launch_inst<S, 64, true>(p, pl.grid, pl.smem, st);
+        case 128: return gm_launch_inst<S, 128, true>(p, pl.grid, pl.smem, st);
+        default: return gm_launch_inst<S, 256, true>(p, pl.grid, pl.smem, st);
+    }
+    switch (pl.NX) {
+        case 32: return gm_launch_inst<S, 32>(p, pl.grid, pl.smem, st);
+        case 64: return gm_launch_inst<S, 64>(p, pl.grid, pl.smem, st);
+        case 128: return gm_launch_inst<S, 128>(p, pl.grid, pl.smem, st);
+        case 256: return gm_launch_inst<S, 256>(p, pl.grid, pl.smem, st);
+        default: return gm_launch_split<S, GM_WIDE, false, false>(p, pl.grid, pl.smem, st);
     }
 }
 
@@ -723,9 +797,9 @@ int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half*
     p.M = M, p.N = w.N, p.K = w.K, p.C = w.C, p.G = w.G, p.idx_bytes = w.idx_bytes, p.nx = pl.NX;
     p.NT = pl.NT, p.MT = pl.MT, p.KS = pl.KS, p.SPP = pl.SPP, p.items = pl.items;
     switch (w.S) {
-        case 2: return gm_launch_nx<2>(p, pl.NX, pl.grid, pl.smem, st);
-        case 3: return gm_launch_nx<3>(p, pl.NX, pl.grid, pl.smem, st);
-        default: return gm_launch_nx<4>(p, pl.NX, pl.grid, pl.smem, st);
+        case 2: return gm_launch_nx<2>(p, pl, st);
+        case 3: return gm_launch_nx<3>(p, pl, st);
+        default: return gm_launch_nx<4>(p, pl, st);
     }
 }
 

@@ -231,3 +231,31 @@ def test_one_large_activation_among_small_ones(M, N, K, G, S, mode, power, algo)
     assert ok[:, :N // 2].all()
     assert (np.abs(y - ref) <= 2.0 ** -11 * np.abs(ref) + 2.0 ** -18 * mass + 2.0 ** -25)[ok].all()
     check_status()
+
+
+@pytest.mark.parametrize("M", [3, 17, 64, 65, 130, 300])
+@pytest.mark.parametrize("N,K,S,mode", [(40, 1024, 3, "u8"), (1000, 2048, 4, "u16"), (129, 512, 2, "direct"), (3000, 768, 4, "u8")])
+def test_odd_row_counts_keep_fp32_weights(M, N, K, S, mode):
+    """Rows that are no multiple of 128: weights are not rounded to fp16.  Error per output: one fp16 rounding of the result (2^-11 of
+    the value) and fp32 sums, 2^-18 of the sum of their products' magnitudes (fp16 weights would add 2^-11 of every product).  An
+    infinite activation gives what the CUDA-core kernel gives."""
+    import sbvr
+    p = O.make_packed(N, K, S, G=256, mode=mode, C=256 if mode == "u8" else 1000, seed=N + K)
+    p["coeff"][0] = np.float16(1.5) * np.arange(1, S + 1) / S          # some weights far above the others
+    rng = np.random.default_rng(M)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    x[0] = 0                                       # an output of almost nothing: a cancelling pair
+    x[0, :2] = 1, -1
+    bits, c = _planes(p, 256)
+    ref = x.astype(np.float64) @ (bits * c).sum(0).T
+    mass = np.abs(x.astype(np.float64)) @ (bits * np.abs(c)).sum(0).T
+    w = to_sbvr(p)
+    y = h2n(sbvr.linear(torch.from_numpy(x).cuda(), w, None)).astype(np.float64)
+    assert (np.abs(y - ref) <= 2.0 ** -11 * np.abs(ref) + 2.0 ** -18 * mass + 2.0 ** -25).all()
+    x[1, K // 3] = np.inf
+    x[2, 5] = -np.inf
+    xt = torch.from_numpy(x).cuda()
+    y, z = h2n(sbvr.linear(xt, w, None)), h2n(sbvr.linear(xt, w, None, algo=1))
+    assert np.array_equal(np.isnan(y), np.isnan(z)) and np.array_equal(np.isinf(y), np.isinf(z))
+    assert np.array_equal(np.sign(y[np.isinf(z)]), np.sign(z[np.isinf(z)])) and np.isinf(z).any()
+    check_status()
