@@ -124,6 +124,11 @@ int sbvr_workspace_create(sbvr_workspace_t** out, int device, size_t bytes) {
     SBVR_CUDA_TRY(cudaSetDevice(device));
     sbvr_workspace* ws = new (std::nothrow) sbvr_workspace();
     if (!ws) return SBVR_ERR_BAD_ARG;
+    ws->mu = new (std::nothrow) std::recursive_mutex();
+    if (!ws->mu) {
+        delete ws;
+        return SBVR_ERR_BAD_ARG;
+    }
     ws->device = device;
     ws->bytes = bytes;
     ws->base = nullptr;
@@ -139,6 +144,7 @@ int sbvr_workspace_create(sbvr_workspace_t** out, int device, size_t bytes) {
         g_last_cuda_error = (int)e;
         (void)cudaGetLastError();
         if (ws->base) cudaFree(ws->base);
+        delete ws->mu;
         delete ws;
         cudaSetDevice(prev);
         return SBVR_ERR_CUDA;
@@ -185,6 +191,7 @@ int sbvr_workspace_destroy(sbvr_workspace_t* ws) {
     if (ws->base) cudaFree(ws->base);
     if (ws->pinned_status) cudaFreeHost(ws->pinned_status);
     cudaSetDevice(prev);
+    delete ws->mu;
     delete ws;
     return SBVR_OK;
 }
@@ -230,6 +237,7 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
     const __half* xh = reinterpret_cast<const __half*>(x);
     const __half* bh = reinterpret_cast<const __half*>(bias);
     __half* yh = reinterpret_cast<__half*>(y);
+    WsLock lock(ws);
     // padded rows, where a kernel needs them, live at the end of the workspace, away from the kernels' scratch
     sbvr_workspace shrunk;
     size_t padded = 0;
@@ -314,6 +322,7 @@ int sbvr_linear_fused_f16(int x_op, const void* x, const void* delta, const void
     xop.op = x_op;
     xop.delta = reinterpret_cast<const __half*>(delta), xop.norm_w = reinterpret_cast<const __half*>(norm_weight);
     xop.h_out = reinterpret_cast<__half*>(h_out), xop.eps = eps;
+    WsLock lock(ws);
     if (!linear_tcs_supported(w, M)) {             // more rows (or digits that do not fit the GEMV): the small-batch kernel
         if (x_op == SBVR_XOP_DIGITS || M > 16 || !linear_sb_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
         if (linear_sb_workspace_bytes(w, di) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
@@ -343,6 +352,7 @@ int sbvr_linear_push_f16(int x_op, const void* x, const void* delta, const void*
     if (rc) return rc;
     if (di.cc_major != 10) return SBVR_ERR_UNSUPPORTED;
     if (G != 256 || !linear_tcs_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
+    WsLock lock(ws);
     if (linear_tcs_workspace_bytes(w, M, di.sm_count) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
     XOp xop;
     xop.op = x_op;
@@ -362,6 +372,7 @@ int sbvr_linear_f16_host(const void* x_host, const uint32_t* bvr, const void* co
     if (xb + yb + ((size_t)8 << 20) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
     char* xd = ws->dyn + ws->dyn_bytes - xb - yb;
     char* yd = xd + xb;
+    WsLock lock(ws);
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     SBVR_CUDA_TRY(cudaMemcpyAsync(xd, x_host, (size_t)M * K * 2, cudaMemcpyHostToDevice, st));
     sbvr_workspace shrunk = *ws;                 // keep the kernels' scratch away from the staging buffers

@@ -60,6 +60,9 @@ struct sbvr_workspace {
     char* dyn;                // rest: staging buffers of the host-pointer entry point, future scratch
     size_t dyn_bytes;
     void* pinned_status;      // host, 16 bytes
+    // Held by a call while it launches kernels that hand data to one another through the workspace: another thread's launches on
+    // the same stream must not come between them.  NULL where the caller serialises (sbvr_linear_f16_noalloc).
+    std::recursive_mutex* mu;
 };
 #define SBVR_WS_COUNTERS 8192
 #define SBVR_WS_XCHG_BYTES (1u << 20)
@@ -67,6 +70,13 @@ struct sbvr_workspace {
 #define SBVR_WS_FIXED_BYTES (256u + SBVR_WS_COUNTERS * 4u + SBVR_WS_XCHG_BYTES)
 
 namespace sbvr {
+
+struct WsLock {
+    std::recursive_mutex* mu;
+    explicit WsLock(const sbvr_workspace* ws) : mu(ws ? ws->mu : nullptr) { if (mu) mu->lock(); }
+    ~WsLock() { if (mu) mu->unlock(); }
+    WsLock(const WsLock&) = delete;
+};
 
 // Launch with programmatic stream serialization: the grid may be scheduled while its predecessor on the stream is
 // still running; every such kernel executes griddepcontrol.wait before it touches what the predecessor produced.

@@ -353,6 +353,7 @@ extern "C" int sbvr_linear_t_f16(const void* x, const uint32_t* bvr_t, const voi
     const int rc = device_info(ws->device, &di);
     if (rc) return rc;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    WsLock lock(ws);
     LtParams p;
     p.bvr = bvr_t, p.idx = coeff_idx, p.coeff = reinterpret_cast<const __half*>(coeff), p.idx_bytes = idx_bytes;
     p.bias = reinterpret_cast<const __half*>(bias);

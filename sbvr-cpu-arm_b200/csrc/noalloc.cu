@@ -108,6 +108,7 @@ extern "C" int sbvr_linear_f16_noalloc(const void* x, const uint32_t* bvr, const
     ws.dyn = ws.base + fixed;
     ws.dyn_bytes = SBVR_NOALLOC_BYTES - fixed;
     ws.pinned_status = nullptr;
+    ws.mu = nullptr;
     const bool aligned_x = !(reinterpret_cast<uintptr_t>(x) & 15);
     // which kernel serves the call, and how much of the array it needs
     int kind = 0;                                  // 0: SIMT kernel (no scratch), 1: decode GEMV, 2: batched GEMM

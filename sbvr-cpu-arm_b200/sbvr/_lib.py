@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import os
+import threading
 
 import torch  # noqa: F401  (the extension module resolves its symbols in torch's libraries)
 
@@ -186,6 +187,8 @@ _workspaces: dict = {}
 # workspace its kernels were recorded with (status word, counters, scratch), and would write into freed memory
 # on replay if the replaced allocation went back to the driver.
 _retired: list = []
+# Torch's threads share the default stream, and creating a workspace lets other threads run.
+_ws_lock = threading.Lock()
 
 
 def workspace_bytes(device: int, M: int, N: int, K: int) -> int:
@@ -197,16 +200,19 @@ def workspace_bytes(device: int, M: int, N: int, K: int) -> int:
 def workspace(device: int, stream: int, nbytes: int = 0) -> Workspace:
     """One workspace per (device, stream): calls on one stream are ordered, so they may share scratch.
     A workspace smaller than `nbytes` is replaced by a larger one; the old one stays allocated for the life of the
-    process (graphs captured earlier on this stream still point into it)."""
+    process (graphs captured earlier on this stream, and calls of other threads, still point into it)."""
     key = (device, stream)
     ws = _workspaces.get(key)
-    if ws is not None and ws.nbytes < nbytes:
-        _retired.append(ws)
-        ws = None
-    if ws is None:
-        ws = Workspace(device, max(nbytes, Workspace.DEFAULT_BYTES))
-        _workspaces[key] = ws
-        native.set_workspace(device, stream, ws.handle.value, ws.nbytes)
+    if ws is not None and ws.nbytes >= nbytes:
+        return ws
+    with _ws_lock:                                 # one thread creates, the others find what it made
+        ws = _workspaces.get(key)
+        if ws is None or ws.nbytes < nbytes:
+            new = Workspace(device, max(nbytes, Workspace.DEFAULT_BYTES))
+            if ws is not None:
+                _retired.append(ws)
+            native.set_workspace(device, stream, new.handle.value, new.nbytes)
+            _workspaces[key] = ws = new
     return ws
 
 

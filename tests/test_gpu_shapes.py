@@ -259,3 +259,29 @@ def test_odd_row_counts_keep_fp32_weights(M, N, K, S, mode):
     assert np.array_equal(np.isnan(y), np.isnan(z)) and np.array_equal(np.isinf(y), np.isinf(z))
     assert np.array_equal(np.sign(y[np.isinf(z)]), np.sign(z[np.isinf(z)])) and np.isinf(z).any()
     check_status()
+
+
+def test_threads_on_one_stream():
+    """Calls of several threads on the stream they share: a quantiser and the product that reads its digits, a re-tiling and its
+    GEMM, stay together."""
+    import threading
+    import sbvr
+    N, K = 512, 2048
+    w = to_sbvr(O.make_packed(N, K, 4, G=256, mode="u16", C=1000, seed=5))
+    g = torch.Generator(device="cuda").manual_seed(3)
+    xs = [torch.randn((m, K), device="cuda", generator=g).half() for m in (16, 5, 40, 12, 3, 64)]
+    want = [sbvr.linear(x, w) for x in xs]
+    bad = []
+
+    def work(i):
+        for _ in range(200):
+            if not torch.equal(sbvr.linear(xs[i], w), want[i]):
+                bad.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(xs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+    check_status()

@@ -94,6 +94,57 @@ def test_no_cpu_fallback():
         w.decode()
 
 
+def test_first_calls_of_several_threads_share_one_workspace(monkeypatch):
+    """Threads of a process share a stream, and creating a workspace lets the others run: all of them get the one that was
+    made, none that was handed out is destroyed, and the extension module never holds a dead one."""
+    import threading
+    import time
+    from sbvr import _lib
+    made, closed, published = [], [], []
+
+    class Handle:
+        value = 0
+
+    class Fake:
+        DEFAULT_BYTES = 1 << 10
+
+        def __init__(self, device, nbytes):
+            time.sleep(0.02)                       # what the allocation does: other threads run
+            self.nbytes, self.handle = nbytes, Handle()
+            self.handle.value = 0x1000 * (len(made) + 1)
+            made.append(self.handle.value)
+
+        def __del__(self):
+            closed.append(self.handle.value)
+
+    class Native:
+        @staticmethod
+        def set_workspace(device, stream, handle, nbytes):
+            published.append((handle, nbytes))
+
+    monkeypatch.setattr(_lib, "Workspace", Fake)
+    monkeypatch.setattr(_lib, "native", Native)
+    monkeypatch.setattr(_lib, "_workspaces", {})
+    monkeypatch.setattr(_lib, "_retired", [])
+    for need in (0, 1 << 20):                      # first use, then all of them need a larger one
+        got, start = [], threading.Barrier(6)
+
+        def first_call():
+            start.wait()
+            ws = _lib.workspace(0, 77, need)
+            got.append((ws.handle.value, ws.nbytes))
+
+        threads = [threading.Thread(target=first_call) for _ in range(6)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert len(set(got)) == 1 and got[0][1] >= need
+        assert published[-1] == got[0]
+        assert not closed, "a workspace that was handed out has been destroyed"
+    assert len(made) == 2
+
+
 def test_glue_and_fused_entry_points_validate_before_any_cuda_call():
     from sbvr import _lib
     L = _lib.lib
