@@ -132,8 +132,8 @@ def test_search_kernel_equals_the_tensor_operations(S, extended):
 @pytest.mark.parametrize("S", [2, 3, 4])
 @pytest.mark.parametrize("M", [1, 2, 3, 5, 8, 9])
 def test_transposed_layout_ragged(N, K, G, S, M):
-    """Group lengths down to one word row, odd input counts, every number of column tiles; activations over six decades.  One
-    fp16 rounding of the result (2^-11) and 2^-23 of the largest product."""
+    """Group lengths down to one word row, odd input counts, both kernels; activations over six decades.  One
+    fp16 rounding of the result (2^-11) and 2^-30 of the largest product for every plane bit."""
     from sbvr import sbvr_cuda
     p = O.make_packed(K, N, S, G=G, mode="u8", C=200, seed=N + K + S)
     rng = np.random.default_rng(M)
@@ -284,4 +284,42 @@ def test_threads_on_one_stream():
     for t in threads:
         t.join()
     assert not bad
+    check_status()
+
+
+@pytest.mark.parametrize("N,K,G,S,M", [(1056, 2401, 32, 3, 8), (1024, 4999, 64, 2, 5), (2048, 2816, 128, 4, 3), (1024, 2304, 256, 4, 8),
+                                       (4096, 4352, 256, 3, 1), (8192, 2304, 256, 2, 1), (1024, 3000, 256, 4, 17), (512, 700, 256, 4, 6)])
+def test_transposed_layout_one_large_product_among_small_ones(N, K, G, S, M):
+    """Every digit width and split of the integer form (the last size: the CUDA-core form), one activation in 200 far above the
+    others; outputs n % 32 == 0 have no plane bit there.  Error per output: one fp16 rounding (2^-11), fp32 sums of the parts
+    (2^-18 of the sum of the products' magnitudes) and half a step, 2^-30 of the largest product, for every plane bit.  A row
+    with an infinite activation comes out as products do."""
+    from sbvr import sbvr_cuda
+    p = O.make_packed(K, N, S, G=G, mode="u16", C=1000, seed=N + K + S)
+    rng = np.random.default_rng(M + K)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    at = np.arange(7, K, 200)
+    x[:, at] = (2.0 ** 13 * rng.uniform(1.0, 1.9, (M, len(at)))).astype(np.float16)
+    p["bvr"][:, at, :] &= np.uint32(0xFFFFFFFE)
+    f = lambda a: torch.from_numpy(a).cuda()
+    bits = ((f(p["bvr"].view(np.int32)).long()[..., None, :] >> torch.arange(32, device="cuda").view(1, 1, 32, 1)) & 1).double()
+    c = f(p["coeff"]).double()[f(p["coeff_idx"].astype(np.int64))].repeat_interleave(G // 32, 0)          # [N/32, K, S]
+    xd = f(x).double()
+    dense = lambda v: torch.einsum("wkns,wks->wnk", bits, v).reshape(N, K)
+    W = dense(c)
+    ref, mass = xd @ W.T, xd.abs() @ dense(c.abs()).T
+    largest = (xd.abs()[:, None, :] * c.abs().amax((0, 2))).amax(2)
+    half_steps = dense(torch.ones_like(c)).sum(1) * largest * 2.0 ** -30
+    args = [f(p["bvr"].view(np.int32)), f(p["coeff_idx"].view(np.int16)).view(torch.uint16), f(p["coeff"]), torch.zeros(0).half().cuda()]
+    y = sbvr_cuda._sbvr_row_deq_mm_T(f(x), *args).double()
+    ok = ref.abs() < 65000
+    assert ok[:, ::32].all()
+    assert ((y - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -18 * mass + half_steps + 2.0 ** -25)[ok].all()
+    if M > 1:
+        xi = x.copy()
+        xi[1, K // 2] = -np.inf
+        z, want = sbvr_cuda._sbvr_row_deq_mm_T(f(xi), *args).double(), f(xi).double() @ W.T
+        assert torch.equal(torch.isnan(z[1]), torch.isnan(want[1]))
+        inf = torch.isinf(want[1])
+        assert inf.any() and torch.equal(z[1][inf], want[1][inf]) and torch.equal(z[0], y[0])
     check_status()
