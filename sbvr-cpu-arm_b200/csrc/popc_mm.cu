@@ -19,8 +19,9 @@
 // one subtraction) are multiplied by the two coefficients and added in fp32.
 //
 // Measured (four planes on both sides, us; popcount instructions on CUDA cores, a sixteenth of the lanes each, in brackets):
-// 4096 x 4096: M = 1 6.4 (8.3), M = 4 8.4 (15.6), M = 16 24.8 (50); 14336 x 4096: M = 1 21.9 (17.9: half of the columns are
-// empty), M = 2 22 (25), M = 4 31 (42).  Bound by instruction issue at 335 per warp and group of 32 weight-plane rows.
+// 4096 x 4096: M = 1 7.1 (8.3), M = 4 9.4 (15.6), M = 16 24.4 (50); 14336 x 4096: M = 2 22 (25), M = 4 32 (41).  Bound by instruction
+// issue at 335 per warp and group of 32 weight-plane rows; 0.8 us of a call is the wait for the kernel in front, which may
+// be writing either operand.  With one activation row half of the columns are empty: on large weights popcounts win (popc_few_rows).
 #include "common.cuh"
 
 namespace sbvr {
@@ -204,13 +205,13 @@ __global__ void __launch_bounds__(PM_THREADS, NT <= 2 ? 4 : 2) popc_mm_kernel(co
     // words cost two round trips to memory, several times what its MMAs take.
     Group q[3];
     Lines ln, ln1;
-    lines_r(g0, ln);                                // the weight does not depend on the kernel in front
+    pdl_wait();                                     // either operand may be an encoding that the kernel in front is writing
+    lines_r(g0, ln);
     lines_r(g0 + 1, ln1);
-    load_r(g0, ln, q[0]);
-    load_r(g0 + 1, ln1, q[1]);
-    pdl_wait();
     lines_l(g0, ln);
     lines_l(g0 + 1, ln1);
+    load_r(g0, ln, q[0]);
+    load_r(g0 + 1, ln1, q[1]);
     load_l(g0, ln, q[0]);
     load_l(g0 + 1, ln1, q[1]);
     lines_r(g0 + 2, ln);
@@ -254,28 +255,157 @@ __global__ void __launch_bounds__(PM_THREADS, NT <= 2 ? 4 : 2) popc_mm_kernel(co
 }
 
 template <int LS, int RS, int NT>
-static int popc_launch_nt(PmParams p, cudaStream_t st) {
+static int popc_launch_nt(PmParams p, int sm_count, cudaStream_t st) {
     constexpr int MT = NT * (8 / (LS == 3 ? 4 : LS)), WR = PM_TW * 16 / (RS == 3 ? 4 : RS);
     // The groups are split over the warps of a CTA as long as all CTAs fit at once (four per SM by their registers, two with four tiles).
+    const long long gy = (p.M + MT - 1) / MT, whole = (p.N + PM_WARPS * WR - 1) / (PM_WARPS * WR);
+    p.ks = 1;
+    while (p.ks * 2 <= PM_WARPS && p.ks * 2 <= p.K / 256 && whole * gy * p.ks * 2 <= (NT <= 2 ? 4 : 2) * sm_count) p.ks *= 2;
+    const int rows = (PM_WARPS / p.ks) * WR;
+    const dim3 grid((p.N + rows - 1) / rows, (p.M + MT - 1) / MT);
+    SBVR_CUDA_TRY(launch_pdl(popc_mm_kernel<LS, RS, NT>, grid, dim3(PM_THREADS), 0, st, p));
+    return SBVR_OK;
+}
+// ---------------------------------------------------------------------------------------------
+// One or two activation rows on large weights: popcount instructions.  A warp owns 32 / RP weight rows (RP = planes per row, 4 for
+// RS = 3) and a quarter of K; lane = (row, plane) reads one packed word per 32 k, 128 contiguous bytes per warp.  The left operand
+// (at most 8 rows per pass) sits in shared memory with its coefficients.
+// ---------------------------------------------------------------------------------------------
+constexpr int PF_MT = 8;               // left rows per pass
+constexpr int PF_KQ = 4;               // K quarters per row block (one warp each)
+constexpr int PF_RB = 2;               // row blocks per CTA
+constexpr int PF_THREADS = 32 * PF_KQ * PF_RB;
+
+template <int LS, int RS>
+__global__ void __launch_bounds__(PF_THREADS) popc_few_kernel(const uint32_t* __restrict__ l_bvr, const void* __restrict__ l_idx,
+                                                             int l_idx_bytes, const __half* __restrict__ l_cache,
+                                                             const uint32_t* __restrict__ r_bvr, const void* __restrict__ r_idx,
+                                                             int r_idx_bytes, const __half* __restrict__ r_cache,
+                                                             const __half* __restrict__ bias, __half* __restrict__ y, int M,
+                                                             int m0, int N, int K) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int RP = (RS == 3) ? 4 : RS;
+    constexpr int ROWS = 32 / RP;                       // weight rows per warp
+    const int KW = K / 32, KB = K / 256;
+    const int mt = min(PF_MT, M - m0);
+    uint32_t* lw = reinterpret_cast<uint32_t*>(smem);                       // [KW][mt][LS]
+    float* lc = reinterpret_cast<float*>(smem + (size_t)KW * PF_MT * LS * 4);   // [KB][mt][LS]
+    float* red = lc + (size_t)KB * PF_MT * LS;                               // [PF_RB][PF_KQ][PF_MT][ROWS]
+    pdl_launch_dependents();
+    pdl_wait();
+    for (int i = threadIdx.x; i < KW * mt * LS; i += PF_THREADS) {
+        const int a = i % LS, m = (i / LS) % mt, kw = i / (LS * mt);
+        lw[(kw * PF_MT + m) * LS + a] = l_bvr[((size_t)kw * M + m0 + m) * LS + a];
+    }
+    for (int i = threadIdx.x; i < KB * mt * LS; i += PF_THREADS) {
+        const int a = i % LS, m = (i / LS) % mt, g = i / (LS * mt);
+        const size_t e = (size_t)g * M + m0 + m;
+        const size_t line = (l_idx_bytes == 1) ? reinterpret_cast<const uint8_t*>(l_idx)[e]
+                                               : reinterpret_cast<const uint16_t*>(l_idx)[e];
+        lc[(g * PF_MT + m) * LS + a] = __half2float(l_cache[line * LS + a]);
+    }
+    __syncthreads();
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rb = warp / PF_KQ, kq = warp % PF_KQ;
+    const int n = ((int)blockIdx.x * PF_RB + rb) * ROWS + lane / RP, b = lane % RP;
+    const bool live = (n < N) && (b < RS);
+    const int g0 = (KB * kq) / PF_KQ, g1 = (KB * (kq + 1)) / PF_KQ;
+    float acc[PF_MT];
+#pragma unroll
+    for (int m = 0; m < PF_MT; ++m) acc[m] = 0.0f;
+    for (int g = g0; g < g1; ++g) {                     // (two groups in flight cost occupancy here: 17.7 -> 26 us at 14336 x 4096)
+        uint32_t rw[8];
+        float cr = 0.0f;
+#pragma unroll
+        for (int kw = 0; kw < 8; ++kw) rw[kw] = live ? __ldcs(r_bvr + ((size_t)(g * 8 + kw) * N + n) * RS + b) : 0u;
+        if (live) {
+            const size_t e = (size_t)g * N + n;
+            const size_t line = (r_idx_bytes == 1) ? reinterpret_cast<const uint8_t*>(r_idx)[e]
+                                                   : reinterpret_cast<const uint16_t*>(r_idx)[e];
+            cr = __half2float(r_cache[line * RS + b]);
+        }
+#pragma unroll
+        for (int m = 0; m < PF_MT; ++m) {
+            if (m < mt) {
+                float s = 0.0f;
+#pragma unroll
+                for (int a = 0; a < LS; ++a) {
+                    int cnt = 0;
+#pragma unroll
+                    for (int kw = 0; kw < 8; ++kw) cnt += __popc(lw[((g * 8 + kw) * PF_MT + m) * LS + a] & rw[kw]);
+                    s += lc[(g * PF_MT + m) * LS + a] * (float)cnt;
+                }
+                acc[m] += cr * s;
+            }
+        }
+    }
+    // planes of a row sit in neighbouring lanes; then the K quarters meet in shared memory, in a fixed order
+#pragma unroll
+    for (int m = 0; m < PF_MT; ++m) {
+#pragma unroll
+        for (int o = RP / 2; o; o >>= 1) acc[m] += __shfl_xor_sync(0xffffffffu, acc[m], o);
+        if (b == 0) red[((rb * PF_KQ + kq) * PF_MT + m) * ROWS + lane / RP] = acc[m];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < PF_RB * mt * ROWS; i += PF_THREADS) {
+        const int r = i % ROWS, m = (i / ROWS) % mt, rbb = i / (ROWS * mt);
+        const int nn = ((int)blockIdx.x * PF_RB + rbb) * ROWS + r;
+        if (nn >= N) continue;
+        float v = 0.0f;
+#pragma unroll
+        for (int q = 0; q < PF_KQ; ++q) v += red[((rbb * PF_KQ + q) * PF_MT + m) * ROWS + r];
+        if (bias) v += __half2float(bias[nn]);
+        y[(size_t)(m0 + m) * N + nn] = __float2half_rn(v);
+    }
+}
+
+template <int LS, int RS>
+static size_t popc_few_smem(int K) {
+    constexpr int ROWS = 32 / ((RS == 3) ? 4 : RS);
+    return (size_t)(K / 32) * PF_MT * LS * 4 + (size_t)(K / 256) * PF_MT * LS * 4 + (size_t)PF_RB * PF_KQ * PF_MT * ROWS * 4;
+}
+template <int LS, int RS>
+static int popc_launch_few(const PmParams& p, cudaStream_t st) {
+    constexpr int ROWS = 32 / ((RS == 3) ? 4 : RS);
+    const size_t smem = popc_few_smem<LS, RS>(p.K);
+    if (smem > 200 * 1024) return SBVR_ERR_UNSUPPORTED;
+    static SmemOnce once;
+    const int rc = set_max_smem_once(once, popc_few_kernel<LS, RS>, 200 * 1024);
+    if (rc) return rc;
+    const int blocks = (p.N + PF_RB * ROWS - 1) / (PF_RB * ROWS);
+    for (int m0 = 0; m0 < p.M; m0 += PF_MT)
+        SBVR_CUDA_TRY(launch_pdl(popc_few_kernel<LS, RS>, dim3(blocks), dim3(PF_THREADS), smem, st, p.l_bvr, p.l_idx, p.l_idx_bytes,
+                                 p.l_cache, p.r_bvr, p.r_idx, p.r_idx_bytes, p.r_cache, p.bias, p.y, p.M, m0, p.N, p.K));
+    return SBVR_OK;
+}
+
+// Where popcounts are faster (four planes on the right, us, tensor cores in brackets): M = 1 with four planes on the left 8192 x 4096
+// 10.8 (11.1), 14336 x 4096 17.8 (21.3), 16384 x 8192 32 (42), with two 9.1 (11.2), 15 (21), 26 (43); M = 2 with two planes 14336 x 4096
+// 17.7 (21.4), 16384 x 8192 32 (43), but 8192 x 4096 12.6 (11.2), and with four 25 (21) at 14336 x 4096; up to 4096 rows
+// never: 8.3 (7.1) at 4096 x 4096.
+template <int LS, int RS>
+static bool popc_few_rows(const PmParams& p, int sm_count) {
+    constexpr int ROWS = 32 / ((RS == 3) ? 4 : RS);
+    const long long blocks = (p.N + PF_RB * ROWS - 1) / (PF_RB * ROWS);
+    if (popc_few_smem<LS, RS>(p.K) > 200 * 1024) return false;
+    return (p.M == 1 && blocks > 3LL * sm_count) || (p.M == 2 && LS == 2 && blocks > 5LL * sm_count);
+}
+
+template <int LS, int RS>
+static int popc_launch(const PmParams& p, cudaStream_t st) {
+    constexpr int CM = 8 / (LS == 3 ? 4 : LS);
     int dev = 0;
     SBVR_CUDA_TRY(cudaGetDevice(&dev));
     DeviceInfo di;
     const int rc = device_info(dev, &di);
     if (rc) return rc;
-    const long long gy = (p.M + MT - 1) / MT, whole = (p.N + PM_WARPS * WR - 1) / (PM_WARPS * WR);
-    p.ks = 1;
-    while (p.ks * 2 <= PM_WARPS && p.ks * 2 <= p.K / 256 && whole * gy * p.ks * 2 <= (NT <= 2 ? 4 : 2) * di.sm_count) p.ks *= 2;
-    const int rows = (PM_WARPS / p.ks) * WR;
-    const dim3 grid((p.N + rows - 1) / rows, (p.M + MT - 1) / MT);
-    if (grid.y > 65535) return SBVR_ERR_SHAPE;
-    SBVR_CUDA_TRY(launch_pdl(popc_mm_kernel<LS, RS, NT>, grid, dim3(PM_THREADS), 0, st, p));
-    return SBVR_OK;
-}
-template <int LS, int RS>
-static int popc_launch(const PmParams& p, cudaStream_t st) {
-    constexpr int CM = 8 / (LS == 3 ? 4 : LS);
+    // the tensor-core kernel addresses by 32-bit offsets and has its passes over M in grid.y
+    const bool fits = (long long)p.N * RS * 8 < (1LL << 31) && (long long)p.M * LS * 8 < (1LL << 31) &&
+                      (long long)(p.K / 256) * (p.N > p.M ? p.N : p.M) < (1LL << 32) && (p.M + 4 * CM - 1) / (4 * CM) <= 65535;
+    if (!fits || popc_few_rows<LS, RS>(p, di.sm_count)) return popc_launch_few<LS, RS>(p, st);
     const int tiles = (p.M + CM - 1) / CM;
-    return tiles <= 1 ? popc_launch_nt<LS, RS, 1>(p, st) : tiles <= 2 ? popc_launch_nt<LS, RS, 2>(p, st) : popc_launch_nt<LS, RS, 4>(p, st);
+    return tiles <= 1 ? popc_launch_nt<LS, RS, 1>(p, di.sm_count, st) : tiles <= 2 ? popc_launch_nt<LS, RS, 2>(p, di.sm_count, st) : popc_launch_nt<LS, RS, 4>(p, di.sm_count, st);
 }
 
 }  // namespace sbvr
@@ -290,8 +420,6 @@ extern "C" int sbvr_popc_mm_f16(const uint32_t* l_bvr, const void* l_idx, int l_
     if ((l_idx_bytes != 1 && l_idx_bytes != 2) || (r_idx_bytes != 1 && r_idx_bytes != 2)) return SBVR_ERR_BAD_ARG;
     if ((l_idx_bytes == 1 && Cl > 256) || (r_idx_bytes == 1 && Cr > 256) || Cl > 65536 || Cr > 65536) return SBVR_ERR_BAD_ARG;
     if (K % 256) return SBVR_ERR_SHAPE;
-    if ((long long)N * RS * 8 >= (1LL << 31) || (long long)M * LS * 8 >= (1LL << 31) || (long long)(K / 256) * (N > M ? N : M) >= (1LL << 32))
-        return SBVR_ERR_UNSUPPORTED;                // 32-bit offsets
     if ((reinterpret_cast<uintptr_t>(l_bvr) | reinterpret_cast<uintptr_t>(r_bvr)) & 3) return SBVR_ERR_ALIGN;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     PmParams p;

@@ -323,3 +323,13 @@ def test_transposed_layout_one_large_product_among_small_ones(N, K, G, S, M):
         inf = torch.isinf(want[1])
         assert inf.any() and torch.equal(z[1][inf], want[1][inf]) and torch.equal(z[0], y[0])
     check_status()
+
+
+@pytest.mark.parametrize("N", [7120, 14333])
+@pytest.mark.parametrize("K", [256, 1280])
+@pytest.mark.parametrize("LS,RS", [(2, 3), (3, 2), (4, 4), (2, 4)])
+@pytest.mark.parametrize("M", [1, 2, 3])
+def test_product_of_two_encodings_many_rows(N, K, LS, RS, M):
+    """One or two activation rows on many weight rows (popcount instructions) and their neighbours (tensor cores); exact counts and
+    fp32 sums, one fp16 rounding (2^-11)."""
+    test_product_of_two_encodings_edges(N, K, LS, RS, M)
