@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(AP_THREADS, 2)
                 uint32_t v;
                 if (even) v = *reinterpret_cast<const uint32_t*>(e);
                 else v = (uint32_t)__half_as_ushort(e[0]) | ((uint32_t)__half_as_ushort(e[1]) << 16);
-                qf[kk][h + 2 * c] = v;
+                qf[kk][h + 2 * c] = scale > 0.0f ? v : scale < 0.0f ? v ^ 0x80008000u : scale == 0.0f ? 0u : v;
             }
     }
     float o[16][4], mx[2] = {-INFINITY, -INFINITY}, sum[2] = {0.0f, 0.0f};
@@ -464,7 +464,9 @@ __global__ void __launch_bounds__(AP_THREADS, 2)
     for (int i = 0; i < 16; ++i)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[i][e] = 0.0f;
-    const float sl2 = scale * 1.4426950408889634f;             // exponentials to base 2
+    // Exponentials to base 2.  The running maximum and the mask are those of the unscaled scores, so the factor has to be positive:
+    // a negative scale turns the queries' signs, a scale of zero makes every score zero.
+    const float sl2 = (scale == 0.0f ? 1.0f : fabsf(scale)) * 1.4426950408889634f;
     const int lrow = lane & 7;
     const uint32_t k_row = (uint32_t)((lrow + ((lane >> 4) & 1) * 8) * 256);
     const uint32_t v_row = (uint32_t)((lrow + ((lane >> 3) & 1) * 8) * 256);

@@ -333,3 +333,24 @@ def test_product_of_two_encodings_many_rows(N, K, LS, RS, M):
     """One or two activation rows on many weight rows (popcount instructions) and their neighbours (tensor cores); exact counts and
     fp32 sums, one fp16 rounding (2^-11)."""
     test_product_of_two_encodings_edges(N, K, LS, RS, M)
+
+
+@pytest.mark.parametrize("scale", [-0.05, 0.0, 0.2])
+@pytest.mark.parametrize("tps", [31, 130])
+def test_prefill_attention_any_scale(scale, tps):
+    """A negative scale prefers the smallest products, a scale of zero averages; fp32 scores and weights, one fp16 rounding."""
+    from sbvr import _lib
+    nh, nkv, d, mc = 4, 2, 128, 150
+    g = torch.Generator(device="cuda").manual_seed(tps)
+    qkv = torch.randn((tps, (nh + 2 * nkv) * d), device="cuda", generator=g).half()
+    K = torch.randn((1, nkv, mc, d), device="cuda", generator=g).half()
+    V = torch.randn((1, nkv, mc, d), device="cuda", generator=g).half()
+    pos = torch.arange(tps, device="cuda", dtype=torch.int32)
+    out = torch.empty((tps, nh * d), dtype=torch.float16, device="cuda")
+    _lib.check(_lib.lib.sbvr_attention_f16(qkv.data_ptr(), K.data_ptr(), V.data_ptr(), pos.data_ptr(), out.data_ptr(), None, tps, tps,
+                                           nh, nkv, d, mc, scale, 1, torch.cuda.current_stream().cuda_stream))
+    q = qkv[:, :nh * d].view(tps, nh, d).transpose(0, 1).double()
+    s = q @ K[0].double().repeat_interleave(nh // nkv, 0).transpose(1, 2) * scale
+    s = s.masked_fill(torch.arange(mc, device="cuda") > pos[:, None], float("-inf"))
+    ref = (torch.softmax(s, -1) @ V[0].double().repeat_interleave(nh // nkv, 0)).transpose(0, 1).reshape(tps, nh * d)
+    assert ((out.double() - ref).abs().max() / ref.abs().max()).item() < 1e-3
