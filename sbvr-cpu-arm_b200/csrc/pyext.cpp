@@ -73,14 +73,32 @@ struct Weight {
     int64_t K;                                     // original inner length
 };
 
-PyObject* field(PyObject* d, PyObject* params, PyObject* name) {
+struct Ref {                                       // an owned reference (or none)
+    PyObject* o;
+    explicit Ref(PyObject* p) : o(p) {}
+    ~Ref() { Py_XDECREF(o); }
+    Ref(const Ref&) = delete;
+};
+// An attribute of the container: from the module's dictionaries, which costs little; what is not there (a buffer, a property, an
+// object that is no module) the way Python looks it up.
+PyObject* field(PyObject* w, PyObject* d, PyObject* params, PyObject* name) {
     PyObject* v = params ? PyDict_GetItemWithError(params, name) : nullptr;
-    if (!v) v = PyDict_GetItemWithError(d, name);
-    return v;                                      // borrowed
+    if (!v && d) v = PyDict_GetItemWithError(d, name);
+    if (v) {
+        Py_INCREF(v);
+        return v;
+    }
+    if (PyErr_Occurred()) throw Raised();
+    v = PyObject_GetAttr(w, name);
+    if (!v) {
+        if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw Raised();
+        PyErr_Clear();
+    }
+    return v;
 }
-at::Tensor tensor_field(PyObject* v, const char* name) {
-    if (!v || !THPVariable_Check(v)) fail(PyExc_ValueError, std::string("not an sbvr weight: ") + name + " is missing");
-    return THPVariable_Unpack(v);
+at::Tensor tensor_field(const Ref& r, const char* name) {
+    if (!r.o || !THPVariable_Check(r.o)) fail(PyExc_ValueError, std::string("not an sbvr weight: ") + name + " is missing");
+    return THPVariable_Unpack(r.o);
 }
 
 int cuda_index(const at::Device& d) {
@@ -90,17 +108,18 @@ int cuda_index(const at::Device& d) {
 }
 
 void read_weight(PyObject* w, Weight* o) {
-    PyObject* d = PyObject_GetAttr(w, s_dict);
-    if (!d) throw Raised();
-    Py_DECREF(d);                                  // the object keeps it alive
-    PyObject* params = PyDict_GetItemWithError(d, s_params);
-    o->bvr = tensor_field(field(d, params, s_bvr), "bvr");
-    o->coeff = tensor_field(field(d, params, s_cache), "coeff_cache");
-    PyObject* ix = field(d, params, s_idx);
+    Ref dict(PyObject_GetAttr(w, s_dict));
+    if (!dict.o) PyErr_Clear();
+    PyObject* d = dict.o && PyDict_Check(dict.o) ? dict.o : nullptr;
+    PyObject* params = d ? PyDict_GetItemWithError(d, s_params) : nullptr;
+    if (params && !PyDict_Check(params)) params = nullptr;
+    o->bvr = tensor_field(Ref(field(w, d, params, s_bvr)), "bvr");
+    o->coeff = tensor_field(Ref(field(w, d, params, s_cache)), "coeff_cache");
+    Ref ix(field(w, d, params, s_idx));
     if (o->bvr.dim() != 3) fail(PyExc_ValueError, "bvr must have three dimensions");
     o->KW = (int)o->bvr.size(0), o->N = (int)o->bvr.size(1), o->S = (int)o->bvr.size(2);
     o->dev = cuda_index(o->bvr.device());
-    if (ix && ix != Py_None) {
+    if (ix.o && ix.o != Py_None) {
         o->idx = tensor_field(ix, "coeff_idx");
         o->idx_bytes = (int)o->idx.element_size();
         o->C = (int)o->coeff.size(0);
@@ -109,15 +128,14 @@ void read_weight(PyObject* w, Weight* o) {
     } else {
         o->idx_bytes = 0, o->C = 0;
     }
-    PyObject* gl = PyDict_GetItemWithError(d, s_glen);
-    PyObject* sh = PyDict_GetItemWithError(d, s_shape);
-    if (!gl || !sh) fail(PyExc_ValueError, "not an sbvr weight");
-    o->G = (int)PyLong_AsLong(gl);
-    const Py_ssize_t nd = PySequence_Size(sh);
-    PyObject* last = nd > 0 ? PySequence_GetItem(sh, nd - 1) : nullptr;
-    if (!last) throw Raised();
-    o->K = PyLong_AsLongLong(last);
-    Py_DECREF(last);
+    Ref gl(field(w, d, nullptr, s_glen)), sh(field(w, d, nullptr, s_shape));
+    if (!gl.o || !sh.o) fail(PyExc_ValueError, "not an sbvr weight");
+    o->G = (int)PyLong_AsLong(gl.o);
+    const Py_ssize_t nd = PySequence_Size(sh.o);
+    if (nd == 0) fail(PyExc_ValueError, "not an sbvr weight");
+    Ref last(nd > 0 ? PySequence_GetItem(sh.o, nd - 1) : nullptr);
+    if (!last.o) throw Raised();
+    o->K = PyLong_AsLongLong(last.o);
     if (PyErr_Occurred()) throw Raised();
 }
 const uint32_t* bvr_ptr(const Weight& w) { return reinterpret_cast<const uint32_t*>(w.bvr.data_ptr()); }

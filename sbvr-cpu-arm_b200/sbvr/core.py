@@ -315,11 +315,17 @@ def row_deq_mm_T(x: torch.Tensor, w_t: sbvr, bias: Optional[torch.Tensor] = None
     """`x @ W.T + bias` for a weight encoded transposed (`sbvr(W, trans=True)` in the reference, sbvr/core.py:244-245:
     `w_t` holds W^T, so `w_t.decode()` is [K, N]).  What the reference's `_sbvr_row_deq_mm_T` call sites compute
     (test_sbvr.py:588-592); the result has the padded width `w_t.in_features_padded`, as there."""
-    p = w_t._parameters
-    idx = p.get("coeff_idx")
+    p = getattr(w_t, "__dict__", {}).get("_parameters") or {}             # the plain attribute look-up of a module costs more than this
+
+    def field(name):
+        v = p.get(name)
+        return getattr(w_t, name) if v is None and name not in p else v
+
+    idx = field("coeff_idx")
     if idx is None:
         raise ValueError(_r_str("the transposed layout needs codebook indices (the reference has no direct form)"))
-    return _lib.native.row_deq(x if x.dim() == 2 else x.reshape(-1, x.shape[-1]), p["bvr"], idx, p["coeff_cache"], bias)
+    return _lib.native.row_deq(x if x.dim() == 2 else x.reshape(-1, x.shape[-1]), field("bvr"), idx, field("coeff_cache"),
+                                bias)
 
 
 def load(filename, device=None, verbose_level=1, cpu_kernel=False, cpu_kernel_v2=False) -> sbvr:

@@ -193,6 +193,35 @@ def test_encoder_config_and_search_space_on_cpu():
         encoder.encode(d.view(1, -1), encoder.EncoderConfig(), device=torch.device("cpu"))
 
 
+def test_weight_fields_are_found_like_attributes():
+    """A weight that is no module with parameters (buffers, slots, properties): its fields are looked up as attributes, and the call
+    gets as far as the device check."""
+    import types
+    import sbvr
+    from sbvr import _lib
+    fields = dict(bvr=torch.zeros((8, 64, 2), dtype=torch.int32), coeff_idx=torch.zeros((1, 64), dtype=torch.uint8),
+                  coeff_cache=torch.zeros((4, 2), dtype=torch.float16), original_data_shape=torch.Size((64, 256)), bvr_len=256)
+
+    class Slots:
+        __slots__ = tuple(fields)
+
+    slots, buffers = Slots(), torch.nn.Module()
+    for k, v in fields.items():
+        setattr(slots, k, v)
+        if isinstance(v, torch.Tensor):
+            buffers.register_buffer(k, v)
+        else:
+            setattr(buffers, k, v)
+    for w in (types.SimpleNamespace(**fields), slots, buffers):
+        with pytest.raises(RuntimeError, match="CUDA"):
+            _lib.native.decode(w)
+        with pytest.raises(ValueError, match="CUDA"):
+            sbvr.row_deq_mm_T(torch.zeros((1, 64), dtype=torch.float16),
+                              types.SimpleNamespace(**dict(fields, bvr=torch.zeros((2, 64, 2), dtype=torch.int32))) if w is not slots else w)
+    with pytest.raises(ValueError, match="bvr is missing"):
+        _lib.native.decode(types.SimpleNamespace(bvr_len=256))
+
+
 def test_step_partition_of_the_streaming_kernels(tmp_path):
     """The split of (tile, k step) work over the CTAs that the decode GEMV and the small-batch kernel share (TsSegs in
     csrc/tc_stream.cuh) is compiled for the host and checked over a few thousand (tiles, steps, CTAs) combinations: every
