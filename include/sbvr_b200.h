@@ -74,6 +74,10 @@ SBVR_API int sbvr_query(int device, int* sm_count, int* smem_per_block_optin, in
  * `bytes` = 0 picks a default that covers every Llama-3 8B/70B layer shape up to 32 activation rows.
  * One workspace must not be used by two calls that can overlap on the GPU. */
 SBVR_API int sbvr_workspace_create(sbvr_workspace_t** ws, int device, size_t bytes);
+/* The same for one linear on these operands: 0 where the decode GEMV serves them (any workspace holds what it needs), else
+ * sbvr_workspace_bytes(device, M, N, K). */
+SBVR_API int sbvr_linear_workspace_bytes(int device, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff,
+                                         int C, int M, int N, int K, int S, int G, size_t* bytes);
 SBVR_API int sbvr_workspace_destroy(sbvr_workspace_t* ws);
 /* Bytes to ask sbvr_workspace_create for so that every kernel (and the host-pointer entry point) can serve
  * linears of up to M activation rows on an N x K weight: the batched kernel keeps a re-tiled copy of the

@@ -183,6 +183,16 @@ int sbvr_workspace_bytes(int device, int M, int N, int K, size_t* bytes) {
     return SBVR_OK;
 }
 
+int sbvr_linear_workspace_bytes(int device, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff, int C,
+                                int M, int N, int K, int S, int G, size_t* bytes) {
+    PackedW w;
+    const int rc = make_packed(&w, bvr, coeff_idx, idx_bytes, coeff, C, N, K, S, G);
+    if (rc) return rc;
+    if (!bytes || M < 1) return SBVR_ERR_BAD_ARG;
+    *bytes = 0;
+    return linear_tcs_supported(w, M) ? SBVR_OK : sbvr_workspace_bytes(device, M, N, K, bytes);
+}
+
 int sbvr_workspace_destroy(sbvr_workspace_t* ws) {
     if (!ws) return SBVR_OK;
     int prev = 0;

@@ -11,6 +11,7 @@
 
 #include <ATen/ATen.h>
 #include <c10/core/InferenceMode.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -48,13 +49,17 @@ std::mutex g_ws_mu;
 std::map<std::pair<int, uintptr_t>, Ws> g_ws;
 PyObject* g_ws_callback = nullptr;                 // _lib.workspace(device, stream, nbytes): creates or enlarges, then reports here
 
-sbvr_workspace_t* workspace(int dev, uintptr_t stream, size_t need) {
+// `few`: a call on few rows, which some kernel serves in any workspace: under capture it takes what is there, since an allocation
+// would end the capture.
+sbvr_workspace_t* workspace(int dev, uintptr_t stream, size_t need, bool few = false) {
     const auto key = std::make_pair(dev, stream);
     for (int attempt = 0; attempt < 2; ++attempt) {
         {
             std::lock_guard<std::mutex> lock(g_ws_mu);
             auto it = g_ws.find(key);
-            if (it != g_ws.end() && it->second.bytes >= need) return it->second.handle;
+            if (it != g_ws.end() &&
+                (it->second.bytes >= need || (few && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)))
+                return it->second.handle;
         }
         if (attempt) break;
         PyObject* r = PyObject_CallFunction(g_ws_callback, "iKK", dev, (unsigned long long)stream, (unsigned long long)need);
@@ -138,6 +143,7 @@ void read_weight(PyObject* w, Weight* o) {
     o->K = PyLong_AsLongLong(last.o);
     if (PyErr_Occurred()) throw Raised();
 }
+size_t workspace_need(const Weight& w, const void* x, int64_t M);
 const uint32_t* bvr_ptr(const Weight& w) { return reinterpret_cast<const uint32_t*>(w.bvr.data_ptr()); }
 const void* idx_ptr(const Weight& w) { return w.idx.defined() ? w.idx.data_ptr() : nullptr; }
 
@@ -154,6 +160,19 @@ at::Tensor bias_tensor(PyObject* o, int64_t N) {
     return b.contiguous();
 }
 void* ptr(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
+
+// Which kernel a call runs on must not depend on the calls before it: the workspace is asked to hold what the automatic choice
+// would use, for few rows as for many.  One row, and two to four on weights that the decode GEMV takes, fit any workspace.
+size_t workspace_need(const Weight& w, const void* x, int64_t M) {
+    const int Kp = w.KW * 32;
+    size_t need = 0;
+    if (M > 4 || w.K != Kp || (M > 1 && (reinterpret_cast<uintptr_t>(x) & 15)))
+        check(sbvr_workspace_bytes(w.dev, (int)M, w.N, Kp, &need), "sbvr_workspace_bytes");
+    else if (M > 1)
+        check(sbvr_linear_workspace_bytes(w.dev, bvr_ptr(w), idx_ptr(w), w.idx_bytes, w.coeff.data_ptr(), w.C, (int)M, w.N, Kp, w.S,
+                                          w.G, &need), "sbvr_linear_workspace_bytes");
+    return need;
+}
 
 struct ReleaseGil {
     PyThreadState* st;
@@ -207,9 +226,7 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (!given) y = empty_half(shape, x.device());
         if (M > 0) {
             const uintptr_t st = (uintptr_t)c10::cuda::getCurrentCUDAStream(w.dev).stream();
-            size_t need = 0;
-            if (M > 4 || w.K != Kp) check(sbvr_workspace_bytes(w.dev, (int)M, w.N, (int)Kp, &need), "sbvr_workspace_bytes");
-            sbvr_workspace_t* ws = workspace(w.dev, st, need);
+            sbvr_workspace_t* ws = workspace(w.dev, st, workspace_need(w, x2.data_ptr(), M), M <= 4 && w.K == Kp);
             int rc;
             {
                 ReleaseGil nogil;
@@ -241,9 +258,7 @@ PyObject* py_linear_fused(PyObject*, PyObject* const* a, Py_ssize_t n) {
         c10::cuda::OptionalCUDAGuard guard;
         if (c10::cuda::current_device() != w.dev) guard.set_index(w.dev);
         const uintptr_t st = (uintptr_t)c10::cuda::getCurrentCUDAStream(w.dev).stream();
-        size_t need = 0;
-        if (M > 1) check(sbvr_workspace_bytes(w.dev, (int)M, w.N, (int)Kp, &need), "sbvr_workspace_bytes");
-        sbvr_workspace_t* ws = workspace(w.dev, st, need);
+        sbvr_workspace_t* ws = workspace(w.dev, st, workspace_need(w, x.data_ptr(), M), M <= 4);
         int rc;
         {
             ReleaseGil nogil;

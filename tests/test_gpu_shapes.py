@@ -354,3 +354,22 @@ def test_prefill_attention_any_scale(scale, tps):
     s = s.masked_fill(torch.arange(mc, device="cuda") > pos[:, None], float("-inf"))
     ref = (torch.softmax(s, -1) @ V[0].double().repeat_interleave(nh // nkv, 0)).transpose(0, 1).reshape(tps, nh * d)
     assert ((out.double() - ref).abs().max() / ref.abs().max()).item() < 1e-3
+
+
+def test_kernel_choice_does_not_depend_on_earlier_calls():
+    """Three rows that the decode GEMV does not take (activations off a 16-byte boundary), on a weight whose partial sums exceed the
+    default workspace: the same bits on a fresh stream and after a larger batch has made the workspace grow."""
+    import sbvr
+    N, K = 262144, 4096
+    g = torch.Generator(device="cuda").manual_seed(1)
+    bvr = torch.randint(-2 ** 31, 2 ** 31 - 1, (K // 32, N, 2), dtype=torch.int32, device="cuda", generator=g)
+    idx = torch.randint(0, 256, (K // 256, N), device="cuda", generator=g).to(torch.uint8)
+    w = sbvr.sbvr.from_packed(bvr, idx, (torch.randn((256, 2), device="cuda", generator=g) * 0.01).half(), group_len=256)
+    x = torch.randn(3 * K + 2, device="cuda", generator=g).half()[2:].view(3, K)
+    big = torch.randn((64, K), device="cuda", generator=g).half()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        first = sbvr.linear(x, w)
+        sbvr.linear(big, w)
+        assert torch.equal(first, sbvr.linear(x, w))
+        torch.cuda.synchronize()
