@@ -228,6 +228,8 @@ class _Codebook:
             for i in np.nonzero(rough)[0]:
                 if mag(stored[i] - line) < near:
                     return int(i), False
+        if self.n >= len(self.lines):              # (a warm-up longer than the codebook)
+            raise IndexError(f"the codebook has {len(self.lines)} lines")
         if self.n == len(self.host):
             self.host = np.concatenate((self.host, np.zeros_like(self.host)))
         self.host[self.n] = line
@@ -258,6 +260,10 @@ class _SearchTables:
             self.unit.append((powers / (sums.max(dim=1)[0] - sums.min(dim=1)[0]).unsqueeze(1)).contiguous())
             self.bias.append(b_list)
             self.per_dim.append(_grid_intervals(conf, S, extended))
+        # what the kernel's candidate numbers (31 bits) and fp16 grid positions can count; the limits of sbvr_encode_advance
+        self.covered = conf.s_search_num >= 1 and conf.extend_ratio > 0 and all(
+            len(u) >= 1 and len(b) >= 1 and 1 <= d <= 2000 and len(u) * len(b) * 1024 + (d + 1) ** S < 2.0e9
+            for u, b, d in zip(self.unit, self.bias, self.per_dim))
 
 
 def _sorted_line(bits, S: int, device) -> np.ndarray:
@@ -302,9 +308,9 @@ def encode(data: torch.Tensor, conf: EncoderConfig, device: Optional[torch.devic
                                best_at=line_of.data_ptr(), scratch=scratch.data_ptr(), result=pinned.data_ptr(), S=S, groups=NG,
                                s_search_num=conf.s_search_num, extend_ratio=conf.extend_ratio, append_at=-1)
         # one coefficient has a grid axis of 10^5 points, beyond what fp16 steps can count: tensor operations
-        kernel_search = conf.space_device == "cuda" and S > 1
+        tables = _SearchTables(conf, dev) if conf.space_device == "cuda" and S > 1 else None
+        kernel_search = tables is not None and tables.covered
         if kernel_search:
-            tables = _SearchTables(conf, dev)
             group_stats = torch.empty((NG, 4), dtype=torch.float32, device=dev)
             _lib.check(_lib.lib.sbvr_encode_stats_f16(groups.data_ptr(), NG, group_stats.data_ptr(), st), "sbvr_encode_stats_f16")
             walk.stats = group_stats.data_ptr()
@@ -354,6 +360,8 @@ def encode(data: torch.Tensor, conf: EncoderConfig, device: Optional[torch.devic
             gi = g + 1
             if progress:
                 progress(gi, NG)
+        if progress and gi < NG:
+            progress(NG, NG)
         if walk.append_at >= 0:
             book.lines[walk.append_at] = torch.from_numpy(book.host[walk.append_at]).to(dev)
 

@@ -74,9 +74,83 @@ def test_encoder_with_gpu_generated_search_space_is_as_good(golden, name):
     assert tuple(w.decode().shape) == tuple(W.shape)
 
 
+def _walk(W, conf):
+    """The walk one group at a time by the tensor operations (sbvr/core.py:555-653): every stored line against the group, then the
+    group's own search space.  Returns what `encoder.encode` returns, without the statistics."""
+    from sbvr import encoder
+    S = conf.num_sums
+    data = W.cuda()
+    N, K = data.shape
+    Kp = -(-K // 256) * 256
+    groups = torch.nn.functional.pad(data, (0, Kp - K)).contiguous().view(-1, 256)
+    lines, history, hits, line_of, sel = [], list(conf.mse_history), 0, [], []
+    for g in range(len(groups)):
+        group = groups[g:g + 1]
+        warm = len(lines) < conf.cache_warmup_num
+        cached, at = float("inf"), 0
+        own = None
+        if not warm:
+            mse = encoder._mse(group, torch.stack(lines), S)[0]
+            at = int(torch.argmin(mse))
+            cached = float(mse[at])
+            window = history[-min(len(history), conf.mse_window_size):]
+            if cached < max(sum(window) / len(window) * 0.99, conf.acceptable_mse):
+                hits += 1
+                own = False
+            elif len(lines) >= conf.max_cache_lines:
+                own = False
+        if own is None:
+            space = encoder.group_search_space(group[0], conf, warm or hits / (g + 1) > 0.6)
+            mse = encoder._mse(group, space, S)[0]
+            best = int(torch.argmin(mse))
+            own = not float(mse[best]) >= cached
+            if own:
+                line = space[best]
+                history.append(float(mse[best]))
+                near = [i for i, l in enumerate(lines) if bool((l - line).abs().sum(-1) < line.abs().sum(-1) * 0.0001)]
+                at = near[0] if near else len(lines)
+                if not near:
+                    lines.append(line.clone())
+        line_of.append(at)
+        out = torch.empty((1, 256), dtype=torch.uint8, device="cuda")
+        encoder._select(group.contiguous(), (line if own else lines[at]).view(1, S).contiguous(), torch.zeros(1, dtype=torch.int32, device="cuda"), S, out)
+        sel.append(out)
+    idx = torch.tensor(line_of).view(N, Kp // 256).T.contiguous()
+    return encoder.pack_selectors(torch.cat(sel).view(N, Kp), S), idx, torch.stack(lines)
+
+
+@pytest.mark.parametrize("kind", ["spread", "full_codebook", "wide_search"])
+@pytest.mark.parametrize("S", [2, 3, 4])
+def test_the_walk_equals_one_group_at_a_time(S, kind):
+    """The device walk (best stored lines kept per group, search kernel, appended and reused lines, the cutoff, the extended switch)
+    against the walk by tensor operations, bit for bit; with a codebook that fills up, and search settings that the search
+    kernel does not cover."""
+    from sbvr import encoder
+    g = torch.Generator().manual_seed(S)
+    W = (torch.randn((24, 500), generator=g) * 0.02).half()
+    W[:, :256] *= torch.linspace(0.5, 3.0, 24).view(-1, 1).half()         # spread the statistics: more misses
+    W[20] = W[3]                                                            # groups that come again
+    settings = {"num_sums": S}
+    if kind == "full_codebook":
+        settings["max_cache_lines"] = 12
+    if kind == "wide_search":
+        if S != 2:
+            pytest.skip("more than 2000 grid intervals per axis need two planes")
+        settings.update(r_search_num=130, b_search_num=130, s_search_num=130)
+        W = W[:4]
+    conf = encoder.EncoderConfig(**settings)
+    calls = []
+    bvr, idx, cache, stats = encoder.encode(W, conf, progress=lambda done, of: calls.append((done, of)))
+    ref_bvr, ref_idx, ref_cache = _walk(W, conf)
+    assert torch.equal(cache.view(torch.int16), ref_cache.view(torch.int16))
+    assert torch.equal(idx.cpu().to(torch.int64), ref_idx)
+    assert torch.equal(bvr.view(torch.int32), ref_bvr.view(torch.int32))
+    assert stats["cache_lines"] == len(ref_cache) and calls[-1] == (stats["groups"], stats["groups"])
+    assert kind == "wide_search" or stats["cache_hits"] > 0
+
+
 def test_batched_lookup_equals_the_sequential_walk():
-    """The speculative batch (codebook look-up of many groups in one launch, one-line updates after each addition) must
-    decide exactly as a walk that looks up one group at a time; trans=True encodes the transpose."""
+    """`batch_groups` is accepted and changes nothing (the walk itself is compared above); trans=True encodes the transpose."""
     import sbvr
     g = torch.Generator().manual_seed(3)
     W = (torch.randn((48, 512), generator=g) * 0.02).half()

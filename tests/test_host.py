@@ -222,6 +222,25 @@ def test_weight_fields_are_found_like_attributes():
         _lib.native.decode(types.SimpleNamespace(bvr_len=256))
 
 
+def test_codebook_refuses_more_lines_than_it_holds():
+    """A warm-up longer than the codebook: the line is refused on the host, before a kernel would write it past the end."""
+    from sbvr import encoder
+    book = encoder._Codebook(encoder.EncoderConfig(num_sums=2, max_cache_lines=2), torch.device("cpu"))
+    for i in (1.0, 2.0):
+        assert book.find_or_add(np.array([i, 3 * i], dtype=np.float16)) == (int(i) - 1, True)
+    assert book.find_or_add(np.array([1.0, 3.0], dtype=np.float16)) == (0, False)
+    with pytest.raises(IndexError):
+        book.find_or_add(np.array([7.0, 9.0], dtype=np.float16))
+
+
+def test_search_settings_the_kernel_does_not_cover():
+    """Settings beyond the search kernel's limits go through the tensor operations instead of being refused."""
+    from sbvr import encoder
+    cpu = torch.device("cpu")
+    assert encoder._SearchTables(encoder.EncoderConfig(num_sums=4), cpu).covered
+    assert not encoder._SearchTables(encoder.EncoderConfig(num_sums=2, r_search_num=200, b_search_num=200, s_search_num=200), cpu).covered
+
+
 def test_step_partition_of_the_streaming_kernels(tmp_path):
     """The split of (tile, k step) work over the CTAs that the decode GEMV and the small-batch kernel share (TsSegs in
     csrc/tc_stream.cuh) is compiled for the host and checked over a few thousand (tiles, steps, CTAs) combinations: every
