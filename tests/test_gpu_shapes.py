@@ -373,3 +373,44 @@ def test_kernel_choice_does_not_depend_on_earlier_calls():
         sbvr.linear(big, w)
         assert torch.equal(first, sbvr.linear(x, w))
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("K", [2304, 4352, 14592])
+@pytest.mark.parametrize("M,G,mode", [(5, 256, "u16"), (16, 256, "direct"), (32, 256, "u16"), (5, 128, "u8"), (16, 128, "direct")])
+@pytest.mark.parametrize("S,N", [(2, 192), (3, 96), (4, 416)])
+def test_small_batch_kernel_unequal_chunks(K, M, G, mode, S, N):
+    """9, 17 and 57 blocks of 256 k: chunks of K that differ in length."""
+    import sbvr
+    p = O.make_packed(N, K, S, G=G, mode=mode, C=256 if mode == "u8" else 1000, seed=N + K)
+    rng = np.random.default_rng(M)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    ref = O.linear_c(x, p["bvr"], p.get("coeff_idx"), p["coeff"], G=G).astype(np.float64)
+    w = to_sbvr(p)
+    y = sbvr.linear(torch.from_numpy(x).cuda(), w, None, algo=4)
+    assert np.abs(h2n(y) - ref).max() / np.abs(ref).max() <= 2e-3
+    assert torch.equal(y, sbvr.linear(torch.from_numpy(x).cuda(), w, None, algo=4))
+    check_status()
+
+
+@pytest.mark.parametrize("nh,nkv", [(2, 2), (4, 2), (8, 2), (16, 2)])
+@pytest.mark.parametrize("ctx,nsplit", [(1, 16), (5, 16), (5, 2), (70, 8), (300, 2), (1300, 16), (1400, 16), (1301, 1)])
+def test_decode_attention_splits(nh, nkv, ctx, nsplit):
+    """One query token: every number of query heads per KV head, contexts shorter than the number of splits and beyond the cache
+    (all of it is attended to); fp32 scores and weights, one fp16 rounding (2^-11) of the result."""
+    from sbvr import _lib
+    d, B, mc = 128, 2, 1300
+    g = torch.Generator(device="cuda").manual_seed(ctx + nh)
+    qkv = torch.randn((B, (nh + 2 * nkv) * d), device="cuda", generator=g).half()
+    K = torch.randn((B, nkv, mc, d), device="cuda", generator=g).half()
+    V = torch.randn((B, nkv, mc, d), device="cuda", generator=g).half()
+    pos = torch.full((B,), ctx - 1, dtype=torch.int32, device="cuda")
+    out = torch.full((B, nh * d), float("nan"), dtype=torch.float16, device="cuda")
+    scratch = torch.empty(B * nh * nsplit * 130, dtype=torch.float32, device="cuda")
+    _lib.check(_lib.lib.sbvr_attention_f16(qkv.data_ptr(), K.data_ptr(), V.data_ptr(), pos.data_ptr(), out.data_ptr(),
+                                           scratch.data_ptr(), B, 1, nh, nkv, d, mc, d ** -0.5, nsplit,
+                                           torch.cuda.current_stream().cuda_stream))
+    n = min(ctx, mc)
+    q = qkv[:, :nh * d].view(B, nh, 1, d).double()
+    kk, vv = (t[:, :, :n].double().repeat_interleave(nh // nkv, 1) for t in (K, V))
+    ref = (torch.softmax(q @ kk.transpose(2, 3) * d ** -0.5, -1) @ vv).reshape(B, nh * d)
+    assert ((out.double() - ref).abs().max() / ref.abs().max()).item() < 1e-3
