@@ -185,10 +185,11 @@ __global__ void __launch_bounds__(256) gemm_retile_x_kernel(const __half* __rest
 // the GEMM
 // ---------------------------------------------------------------------------------------------
 // Split K: the sum of the KS parts of one output tile (rows activation rows x cols weight rows, row pitch N), in part order.
-// A thread takes four neighbouring weight rows of four activation rows, all of a part's loads in flight together: one element
-// and one part at a time was a chain of 64 x KS L2 round trips (71 -> 38 us at 512 x 4096 x 4096).
-static __device__ __forceinline__ void gm_add_parts(const float* part, size_t plane, int KS, int rows, int cols, int N,
-                                                 const __half* bias, __half* y, int tid) {
+// A thread takes four neighbouring weight rows of U activation rows and loads Q parts of them together: one element and one part at a
+// time was a chain of 64 x KS L2 round trips (71 -> 38 us at 512 x 4096 x 4096), one part at a time of few rows one of KS.
+template <int U, int Q>
+static __device__ __forceinline__ void gm_add_rows(const float* part, size_t plane, int KS, int rows, int cols, int N,
+                                                   const __half* bias, __half* y, int tid) {
     constexpr int W = GM_DTHREADS / 32;
     const int c = (tid & 31) * 4;
     if (c >= cols) return;
@@ -196,34 +197,38 @@ static __device__ __forceinline__ void gm_add_parts(const float* part, size_t pl
     float b[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) b[j] = (bias && c + j < cols) ? __half2float(bias[c + j]) : 0.0f;
-    for (int m = tid >> 5; m < rows; m += 4 * W) {
-        float v[4][4];
+    for (int m = tid >> 5; m < rows; m += U * W) {
+        float v[U][4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int j = 0; j < 4; ++j) v[u][j] = 0.0f;
-        for (int q = 0; q < KS; ++q) {
-            const float* src = part + (size_t)q * plane + c;
-            float t[4][4];
+        for (int q0 = 0; q0 < KS; q0 += Q) {
+            float t[Q][U][4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int mu = m + u * W;
-                const float* s = src + (size_t)mu * N;
-                if (mu < rows && quad) {
-                    const float4 f = __ldcg(reinterpret_cast<const float4*>(s));
-                    t[u][0] = f.x, t[u][1] = f.y, t[u][2] = f.z, t[u][3] = f.w;
-                } else {
+            for (int q = 0; q < Q; ++q)
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) t[u][j] = (mu < rows && c + j < cols) ? __ldcg(s + j) : 0.0f;
+                for (int u = 0; u < U; ++u) {
+                    const int mu = m + u * W;
+                    const bool on = mu < rows && q0 + q < KS;
+                    const float* s = part + (size_t)(q0 + q) * plane + c + (size_t)mu * N;
+                    if (on && quad) {
+                        const float4 f = __ldcg(reinterpret_cast<const float4*>(s));
+                        t[q][u][0] = f.x, t[q][u][1] = f.y, t[q][u][2] = f.z, t[q][u][3] = f.w;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) t[q][u][j] = (on && c + j < cols) ? __ldcg(s + j) : 0.0f;
+                    }
                 }
-            }
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
+            for (int q = 0; q < Q; ++q)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) v[u][j] += t[u][j];
+                for (int u = 0; u < U; ++u)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) v[u][j] += t[q][u][j];
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < U; ++u) {
             const int mu = m + u * W;
             if (mu >= rows) break;
             __half* dst = y + (size_t)mu * N + c;
@@ -232,6 +237,13 @@ static __device__ __forceinline__ void gm_add_parts(const float* part, size_t pl
                 if (c + j < cols) dst[j] = __float2half_rn(v[u][j] + b[j]);
         }
     }
+}
+static __device__ __forceinline__ void gm_add_parts(const float* part, size_t plane, int KS, int rows, int cols, int N,
+                                                 const __half* bias, __half* y, int tid) {
+    constexpr int W = GM_DTHREADS / 32;
+    if (rows <= W) gm_add_rows<1, 4>(part, plane, KS, rows, cols, N, bias, y, tid);
+    else if (rows <= 2 * W) gm_add_rows<2, 2>(part, plane, KS, rows, cols, N, bias, y, tid);
+    else gm_add_rows<4, 1>(part, plane, KS, rows, cols, N, bias, y, tid);
 }
 
 // SPLIT: K is split over several CTAs (p.KS > 1).  A kernel of its own: its CTAs have one work item each (gm_plan), so that the
