@@ -259,6 +259,7 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
         shrunk.dyn_bytes = (ws->dyn_bytes - padded) / 256 * 256;
         ws = &shrunk;
     }
+    const bool chosen = algo == 0;
     if (algo == 0) {
         DeviceInfo di;
         algo = 1;
@@ -296,7 +297,7 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
     if (algo == 4) {
         if (!ws) return SBVR_ERR_WORKSPACE;
         return launch_linear_sb(xh, w, bh, yh, M, ws->device, ws->status, reinterpret_cast<unsigned int*>(ws->xchg), ws->dyn,
-                                ws->dyn_bytes, st);
+                                ws->dyn_bytes, chosen, st);
     }
     return launch_linear_simt(xh, w, bh, yh, M, st);
 }
@@ -338,7 +339,7 @@ int sbvr_linear_fused_f16(int x_op, const void* x, const void* delta, const void
         if (linear_sb_workspace_bytes(w, di) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
         return launch_linear_sb(reinterpret_cast<const __half*>(x), w, reinterpret_cast<const __half*>(bias),
                                 reinterpret_cast<__half*>(y), M, ws->device, ws->status, reinterpret_cast<unsigned int*>(ws->xchg),
-                                ws->dyn, ws->dyn_bytes, reinterpret_cast<cudaStream_t>(stream), &xop);
+                                ws->dyn, ws->dyn_bytes, true, reinterpret_cast<cudaStream_t>(stream), &xop);
     }
     if (linear_tcs_workspace_bytes(w, M, di.sm_count) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
     return launch_linear_tcs(reinterpret_cast<const __half*>(x), w, reinterpret_cast<const __half*>(bias),

@@ -68,6 +68,8 @@ static_assert(SB_CHUNK * SB_SFCOLS <= 64 && SB_SFA_COL + 32 <= TS_TMEM_COLS, "te
 
 struct SbParams {
     const unsigned char* xb;      // [KB][SB_BLOB] written by sb_quant_kernel
+    const __half* x;              // what was quantised, [M][K]; NULL: a row with a non-finite value becomes NaN
+    const uint32_t* bvr;
     const void* idx;
     const __half* coeff;
     const __half* bias;
@@ -75,7 +77,7 @@ struct SbParams {
     unsigned int* status;
     unsigned int* counters;       // one per quarter of a tile's rows, zero between launches
     float* part;                  // [KC][NT][SB_MP][TN] sums of the chunks (KC > 1)
-    int M, N, K, KB, NT, C, KC, GN, cache_in_smem, stages;
+    int M, N, K, KB, NT, C, KC, GN, cache_in_smem, stages, idx_bytes;
     int off_cache, off_ring, off_res;
 };
 
@@ -88,6 +90,7 @@ struct SbQuant {
     const __half* norm_w;
     __half* h_out;
     float eps;
+    __half* x_out;            // the row as it is quantised, or NULL
 };
 
 // ---------------------------------------------------------------------------------------------
@@ -171,6 +174,7 @@ __global__ void __launch_bounds__(64, 32) sb_quant_kernel(const SbQuant p) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) e[i] = p.x[off + i];
         }
+        if (p.x_out) *reinterpret_cast<uint4*>(p.x_out + off) = o;
         reinterpret_cast<uint4*>(row[wl])[lane] = o;
         __syncwarp();
         const __half* xp = row[wl] + 32 * kw + j;
@@ -254,6 +258,21 @@ __device__ __forceinline__ unsigned int sb_arrive(unsigned int* counter, int lan
     return old;
 }
 
+// Sum over a chunk of an activation row that holds something non-finite there, as products give it: the digits cannot say it.
+template <int S>
+static __device__ __noinline__ float sb_multiply_out(const SbParams& p, int G, int m, int n, int kb0, int nkb) {
+    if (!p.x) return __int_as_float(0x7fc00000);
+    float acc = 0.0f;
+    for (int k = kb0 * 256; k < (kb0 + nkb) * 256; ++k) {
+        const __half* line = coeff_line(p.idx, p.idx_bytes, p.coeff, k / G, n, p.N, S);
+        float w = 0.0f;
+        for (int s = 0; s < S; ++s)
+            if ((p.bvr[((size_t)(k >> 5) * p.N + n) * S + s] >> (k & 31)) & 1u) w += __half2float(line[s]);
+        acc = fmaf(__half2float(__ldcg(p.x + (size_t)m * p.K + k)), w, acc);
+    }
+    return acc;
+}
+
 // The chunks' sums of a quarter of a tile's rows -> y, in chunk order; the counter goes back to zero.
 template <int TN>
 __device__ __forceinline__ void sb_add_chunks(const SbParams& p, int tile, int quarter, int lane) {
@@ -288,7 +307,7 @@ __device__ __forceinline__ void sb_add_chunks(const SbParams& p, int tile, int q
 }
 
 template <int S, int NSUB, int IDXB>
-__global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_constant__ CUtensorMap tmap, const SbParams p) {
+__global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ SbParams p) {
     pdl_launch_dependents();
     extern __shared__ __align__(1024) unsigned char smem[];
     constexpr int SP = ts_sp(S);
@@ -525,7 +544,7 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                 const unsigned int pm = *poison_s;
 #pragma unroll
                 for (int e = 0; e < NV; ++e)
-                    if ((pm >> (s * NV + e)) & 1u) v[e] = __int_as_float(0x7fc00000);
+                    if ((pm >> (s * NV + e)) & 1u) v[e] = sb_multiply_out<S>(p, 256 / NSUB, s * NV + e, tile * TN + nl, kb0, nkb);
                 if (KC > 1) {
                     while (pend) settle();         // (one k block per chunk: a tile every unit)
                     float* dst = p.part + ((size_t)chunk * p.NT + tile) * (MP * TN) + nl;
@@ -669,7 +688,7 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                     const int a = w * units / SB_NWG, b = (w + 1) * units / SB_NWG;
                     if (a < (tl + 1) * nkb && b > tl * nkb && a < b) v += res[(size_t)(w * 2 + (tl > a / nkb ? 1 : 0)) * (MP * TN) + m * TN + nl];
                 }
-                if ((pm >> m) & 1u) v = __int_as_float(0x7fc00000);
+                if ((pm >> m) & 1u) v = sb_multiply_out<S>(p, 256 / NSUB, m, n, kb0, nkb);
                 if (KC > 1) __stcg(p.part + ((size_t)chunk * p.NT + t0 + tl) * (MP * TN) + m * TN + nl, v);
                 else p.y[(size_t)m * N + n] = __float2half_rn(v + (p.bias ? __half2float(p.bias[n]) : 0.0f));
             }
@@ -759,7 +778,7 @@ bool linear_sb_preferred(const PackedW& w) { return w.K <= 4096 || w.N <= 1024 |
 size_t linear_sb_workspace_bytes(const PackedW& w, const DeviceInfo& di) {
     SbPlan pl;
     if (sb_plan(w, di, &pl) != SBVR_OK) return 0;
-    return pl.blob_bytes + pl.part_bytes;
+    return pl.blob_bytes + pl.part_bytes + (size_t)SB_MP * w.K * 2;
 }
 
 // The kernel asks for all of the SM's shared memory, once per device: a CTA whose size just filled a smaller carve-out (196 KB
@@ -800,9 +819,10 @@ static int sb_launch_g(const CUtensorMap& tm, const SbParams& p, int G, int idxb
 }
 
 // `counters` (SBVR_WS_XCHG_BYTES, zero between calls: the kernel leaves them zero) and `scratch` (256-byte aligned,
-// linear_sb_workspace_bytes long: digit blob and the chunks' sums) are the caller's.
+// linear_sb_workspace_bytes long: digit blob, the chunks' sums, rows an op has made) are the caller's.
 int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, int device, unsigned int* status,
-                     unsigned int* counters, char* scratch, size_t scratch_bytes, cudaStream_t st, const XOp* xop) {
+                     unsigned int* counters, char* scratch, size_t scratch_bytes, bool multiply_out, cudaStream_t st,
+                     const XOp* xop) {
     if (!linear_sb_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
     if (!status || !counters || !scratch) return SBVR_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(x) & 1) return SBVR_ERR_ALIGN;
@@ -814,7 +834,7 @@ int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __ha
     SbPlan pl;
     rc = sb_plan(w, di, &pl);
     if (rc) return rc;
-    if (pl.blob_bytes + pl.part_bytes > scratch_bytes) return SBVR_ERR_WORKSPACE;
+    if (linear_sb_workspace_bytes(w, di) > scratch_bytes) return SBVR_ERR_WORKSPACE;
     CUtensorMap tm;
     rc = ts_tensor_map(w, 1, &tm);
     if (rc) return rc;
@@ -822,11 +842,14 @@ int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __ha
     q.x = x, q.xb = reinterpret_cast<unsigned char*>(scratch), q.M = M, q.K = w.K;
     rc = xop_check(xop, x, M, w.K, &q.x_op, &q.delta, &q.norm_w, &q.h_out, &q.eps);
     if (rc) return rc;
+    // (an op in front: its result is kept for rows that have to be multiplied out)
+    q.x_out = q.x_op != SBVR_XOP_NONE && multiply_out ? reinterpret_cast<__half*>(scratch + pl.blob_bytes + pl.part_bytes) : nullptr;
     SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel, dim3(pl.KB, SB_MP / 2), dim3(64), 0, st, q));
     SbParams p;
     p.xb = q.xb;
     p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status, p.counters = counters;
     p.part = reinterpret_cast<float*>(scratch + pl.blob_bytes);
+    p.x = !multiply_out ? nullptr : q.x_out ? q.x_out : x, p.bvr = w.bvr, p.idx_bytes = w.idx_bytes;
     p.M = M, p.N = w.N, p.K = w.K, p.KB = pl.KB, p.NT = pl.NT, p.C = w.C, p.KC = pl.KC, p.GN = pl.GN;
     p.cache_in_smem = pl.cache_in_smem, p.stages = pl.stages;
     p.off_cache = pl.off_cache, p.off_ring = pl.off_ring, p.off_res = pl.off_res;

@@ -414,3 +414,37 @@ def test_decode_attention_splits(nh, nkv, ctx, nsplit):
     kk, vv = (t[:, :, :n].double().repeat_interleave(nh // nkv, 1) for t in (K, V))
     ref = (torch.softmax(q @ kk.transpose(2, 3) * d ** -0.5, -1) @ vv).reshape(B, nh * d)
     assert ((out.double() - ref).abs().max() / ref.abs().max()).item() < 1e-3
+
+
+@pytest.mark.parametrize("M", [5, 16])
+@pytest.mark.parametrize("N,K,G,S,mode", [(192, 4096, 256, 4, "u16"), (64, 512, 128, 3, "u8"), (256, 2304, 256, 2, "direct")])
+@pytest.mark.parametrize("op", ["none", "silu"])
+def test_non_finite_activations_of_small_batches(M, N, K, G, S, mode, op):
+    """The automatic choice multiplies rows with a non-finite activation out: what the CUDA-core kernel gives, infinities with their
+    signs; the other rows keep their bits."""
+    import sbvr
+    from sbvr import _lib
+    from sbvr.core import XOP_SILU_MUL, linear_fused
+    p = O.make_packed(N, K, S, G=G, mode=mode, C=256 if mode == "u8" else 1000, seed=N + K)
+    w = to_sbvr(p)
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn((M, 2 * K if op == "silu" else K), device="cuda", generator=g).half()
+
+    def call(x):
+        if op == "none":
+            return sbvr.linear(x, w), sbvr.linear(x, w, None, algo=1)
+        y, act = torch.empty((M, N), dtype=torch.float16, device="cuda"), torch.empty((M, K), dtype=torch.float16, device="cuda")
+        _lib.check(_lib.lib.sbvr_silu_mul_f16(x.data_ptr(), act.data_ptr(), M, K, torch.cuda.current_stream().cuda_stream))
+        assert linear_fused(XOP_SILU_MUL, x, w, y)
+        return y, sbvr.linear(act, w, None, algo=1)
+
+    clean = call(x)[0]
+    x[0, K // 2], x[1, 3], x[2, K - 1] = float("inf"), float("-inf"), float("nan")
+    x[3, 7], x[3, K - 9] = float("inf"), float("-inf")
+    y, z = call(x)
+    assert torch.equal(y[4:], clean[4:])
+    assert torch.equal(torch.isnan(y), torch.isnan(z)) and torch.equal(torch.isinf(y), torch.isinf(z))
+    assert torch.isinf(z).any() and torch.equal(y[torch.isinf(z)], z[torch.isinf(z)])
+    ok = torch.isfinite(z)
+    assert ((y[ok].float() - z[ok].float()).abs().max() / z[ok].float().abs().max()).item() < 1e-3
+    check_status()
