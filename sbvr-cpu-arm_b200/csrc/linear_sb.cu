@@ -258,29 +258,34 @@ __device__ __forceinline__ unsigned int sb_arrive(unsigned int* counter, int lan
     return old;
 }
 
-// Sum over a chunk of an activation row that holds something non-finite there, as products give it: the digits cannot say it.
+// y[m, n] of an activation row that holds something non-finite, as products give it: the digits cannot say it and have left a NaN.
+// Inlined where few values are live (88 registers, 80 without it): as a function that is called it took the kernel to 94, which leaves
+// no room beside a CTA for the blocks of the GEMM's re-tiling (seven linears of a layer, 16 rows: 154 against 146 us).
 template <int S>
-static __device__ __noinline__ float sb_multiply_out(const SbParams& p, int G, int m, int n, int kb0, int nkb) {
-    if (!p.x) return __int_as_float(0x7fc00000);
+__device__ __forceinline__ void sb_multiply_out(const SbParams& p, int G, int m, int n) {
     float acc = 0.0f;
-    for (int k = kb0 * 256; k < (kb0 + nkb) * 256; ++k) {
+#pragma unroll 1
+    for (int k = 0; k < p.K; ++k) {
         const __half* line = coeff_line(p.idx, p.idx_bytes, p.coeff, k / G, n, p.N, S);
+        const uint32_t* words = p.bvr + ((size_t)(k >> 5) * p.N + n) * S;
         float w = 0.0f;
+#pragma unroll 1
         for (int s = 0; s < S; ++s)
-            if ((p.bvr[((size_t)(k >> 5) * p.N + n) * S + s] >> (k & 31)) & 1u) w += __half2float(line[s]);
+            if ((words[s] >> (k & 31)) & 1u) w += __half2float(line[s]);
         acc = fmaf(__half2float(__ldcg(p.x + (size_t)m * p.K + k)), w, acc);
     }
-    return acc;
+    p.y[(size_t)m * p.N + n] = __float2half_rn(acc + (p.bias ? __half2float(p.bias[n]) : 0.0f));
 }
 
 // The chunks' sums of a quarter of a tile's rows -> y, in chunk order; the counter goes back to zero.
-template <int TN>
+template <int S, int NSUB>
 __device__ __forceinline__ void sb_add_chunks(const SbParams& p, int tile, int quarter, int lane) {
-    constexpr int MP = SB_MP, QR = TN / 4, PER = MP * QR / 32, H = 16 / PER;
+    constexpr int TN = ts_tn(S), MP = SB_MP, QR = TN / 4, PER = MP * QR / 32, H = 16 / PER;
     if (lane == 0) p.counters[tile * 4 + quarter] = 0u;
     __threadfence();
     const size_t plane = (size_t)p.NT * (MP * TN);
     const float* src = p.part + (size_t)tile * (MP * TN) + quarter * QR;
+    unsigned int nan = 0u;
     float v[PER];
 #pragma unroll
     for (int u = 0; u < PER; ++u) v[u] = 0.0f;
@@ -302,7 +307,17 @@ __device__ __forceinline__ void sb_add_chunks(const SbParams& p, int tile, int q
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
         const int q = lane + 32 * u, m = q / QR, n = tile * TN + quarter * QR + q % QR;
-        if (m < p.M) p.y[(size_t)m * p.N + n] = __float2half_rn(v[u] + (p.bias ? __half2float(p.bias[n]) : 0.0f));
+        if (m < p.M) {
+            p.y[(size_t)m * p.N + n] = __float2half_rn(v[u] + (p.bias ? __half2float(p.bias[n]) : 0.0f));
+            if (v[u] != v[u]) nan |= 1u << u;
+        }
+    }
+    if (p.x) {
+#pragma unroll 1
+        for (; nan; nan &= nan - 1) {
+            const int q = lane + 32 * (__ffs((int)nan) - 1);
+            sb_multiply_out<S>(p, 256 / NSUB, q / QR, tile * TN + quarter * QR + q % QR);
+        }
     }
 }
 
@@ -517,7 +532,7 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                 pend = 2;
             } else if (pend == 2) {
                 pend = 0;
-                if (__shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<TN>(p, ptile, wl, lane);
+                if (__shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<S, NSUB>(p, ptile, wl, lane);
             }
         };
         // Sums of one tile's units: planes added across their lanes, after which a lane has the activation rows
@@ -544,7 +559,7 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                 const unsigned int pm = *poison_s;
 #pragma unroll
                 for (int e = 0; e < NV; ++e)
-                    if ((pm >> (s * NV + e)) & 1u) v[e] = sb_multiply_out<S>(p, 256 / NSUB, s * NV + e, tile * TN + nl, kb0, nkb);
+                    if ((pm >> (s * NV + e)) & 1u) v[e] = __int_as_float(0x7fc00000);
                 if (KC > 1) {
                     while (pend) settle();         // (one k block per chunk: a tile every unit)
                     float* dst = p.part + ((size_t)chunk * p.NT + tile) * (MP * TN) + nl;
@@ -558,6 +573,11 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
 #pragma unroll
                     for (int e = 0; e < NV; ++e)
                         if (s * NV + e < M) p.y[(size_t)(s * NV + e) * N + n] = __float2half_rn(v[e] + bias);
+                    if (p.x && pm) {
+#pragma unroll 1
+                        for (int m = s * NV; m < s * NV + NV; ++m)
+                            if ((pm >> m) & 1u) sb_multiply_out<S>(p, 256 / NSUB, m, n);
+                    }
                 }
             }
             have = 0;
@@ -688,9 +708,10 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                     const int a = w * units / SB_NWG, b = (w + 1) * units / SB_NWG;
                     if (a < (tl + 1) * nkb && b > tl * nkb && a < b) v += res[(size_t)(w * 2 + (tl > a / nkb ? 1 : 0)) * (MP * TN) + m * TN + nl];
                 }
-                if ((pm >> m) & 1u) v = sb_multiply_out<S>(p, 256 / NSUB, m, n, kb0, nkb);
+                if ((pm >> m) & 1u) v = __int_as_float(0x7fc00000);
                 if (KC > 1) __stcg(p.part + ((size_t)chunk * p.NT + t0 + tl) * (MP * TN) + m * TN + nl, v);
                 else p.y[(size_t)m * N + n] = __float2half_rn(v + (p.bias ? __half2float(p.bias[n]) : 0.0f));
+                if (KC == 1 && p.x && ((pm >> m) & 1u)) sb_multiply_out<S>(p, 256 / NSUB, m, n);
             }
             if (KC > 1) {
                 shared_tile = t0 + tl;
@@ -698,9 +719,9 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
             }
         }
     }
-    if (pend == 2 && __shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<TN>(p, ptile, warp & 3, lane);
+    if (pend == 2 && __shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<S, NSUB>(p, ptile, warp & 3, lane);
     if (shared_tile >= 0 && __shfl_sync(0xffffffffu, shared_old, 0) == (unsigned int)(KC - 1))
-        sb_add_chunks<TN>(p, shared_tile, warp & 3, lane);
+        sb_add_chunks<S, NSUB>(p, shared_tile, warp & 3, lane);
     if (threadIdx.x == 0 && *abort_flag) {         // which problem gave up: N, and K / 256 | M | CTA (for the host's message)
         atomicExch(p.status + 2, (unsigned int)p.N);
         atomicExch(p.status + 3, ((unsigned int)p.KB << 16) | ((unsigned int)M << 8) | (blockIdx.x & 0xFFu));
