@@ -35,10 +35,11 @@
 // for another CTA, and all of it but the last tile's runs beside the other warpgroups' units).  A tile that several warpgroups
 // share is put together in shared memory at the end.  Every wait is bounded.
 //
-// What bounds it: the tensor pipe on large weights (a unit is 24 MMAs of about 33 cycles, 790 of the 1 030 cycles that a unit takes at
-// 28672 x 8192), on small ones the two launches and the merge of the chunks.  Per call with the quantiser, M = 16, S = 4, us (the
-// fp16 GEMM in brackets): 4096 x 4096 12.5 (15.4), 1024 x 4096 10.8 (13.2), 14336 x 4096 27.9 (32.5), 10240 x 8192 46 (58),
-// 28672 x 8192 107 (112); with six digits, whose error the GEMM does not have, they took 11.8, 9.0, 21.9 and 67.
+// What bounds it: no pipe is saturated (14336 x 4096: tensor pipe 49 % active, issue slots 46 %); a unit takes 1 030 cycles of its SM
+// at 28672 x 8192, 650 with half the MMAs, which follow one another on one accumulator; on small weights the two launches and the
+// merge of the chunks.  Per call with the quantiser, M = 16, S = 4, us (the fp16 GEMM in brackets): 1024 x 4096 10.9 (11.1),
+// 4096 x 4096 12.6 (14.8), 14336 x 4096 28.1 (32.3), 10240 x 8192 46 (58), 28672 x 8192 109 (113); six digits, whose error the GEMM
+// does not have, took 9.0, 11.6, 22.0 and, at 28672 x 8192, 67.
 //
 // Replaces the M > 1 use of `_sbvr_row_deq_mm_T` (reference sbvr/kernels/sbvr_kernel.cu:121-191) for 2 .. 16 rows.
 #include <cuda.h>
@@ -789,12 +790,12 @@ bool linear_sb_supported(const PackedW& w, int M) {
     return sb_plan(w, di, &pl) == SBVR_OK;
 }
 
-// Where it is faster than the GEMM.  Up to four chunks of K always (M = 16, us, the GEMM in brackets: 2048 x 2048 9.4 (10.8),
-// 4096 x 4096 12.5 (15.4), with three planes 12.4 (14.4), two 12.4 (13.1), groups of 128 13.7 (15.1)), and on weights of few rows, which
-// leave the GEMM few tiles (128 x 14336 11.2 (23.6), 512 x 14336 17.0 (19.7), 1024 x 11008 17.8 (25.7), 1024 x 14336 19.4 (18.3)); with
-// up to eight chunks on weights of many rows (10240 x 8192 46 (58), 28672 x 8192 107 (112), but 8192 x 8192 38 (36) and, with groups of
-// 128, 28672 x 8192 116 (110)); beyond, the chunks' merge costs more than is gained: 4096 x 11008 33 (27), 4096 x 14336 40 (32).
-bool linear_sb_preferred(const PackedW& w) { return w.K <= 4096 || w.N <= 1024 || (w.K <= 8192 && w.N > 8192 && w.G == 256); }
+// Where it is faster than the GEMM.  Up to four chunks of K (M = 16, us, the GEMM in brackets: 1024 x 4096 10.9 (11.1), 2048 x 2048
+// 9.5 (9.8), 4096 x 4096 12.6 (14.8), with two planes 12.5 (12.5), groups of 128 13.8 (14.7), 14336 x 4096 28.1 (32.3)), on weights of so
+// few rows that the GEMM has one or two tiles (128 x 14336 11.0 (14.8), but 512 x 14336 18.6 (14.7)) and, with up to eight chunks, on
+// weights of many rows (10240 x 8192 46 (58), 28672 x 8192 109 (113), but 4096 x 8192 25 (22), 8192 x 8192 39 (36) and, with groups of
+// 128, 28672 x 8192 114 (110)); beyond, the chunks' merge costs more than is gained: 4096 x 11008 33 (27), 4096 x 14336 42 (32).
+bool linear_sb_preferred(const PackedW& w) { return w.K <= 4096 || w.N <= 256 || (w.K <= 8192 && w.N > 8192 && w.G == 256); }
 
 size_t linear_sb_workspace_bytes(const PackedW& w, const DeviceInfo& di) {
     SbPlan pl;
