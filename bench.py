@@ -552,7 +552,7 @@ def small_m_and_prefill(torch, dev, stream):
         rs_ = [mk(N, K) for _ in range(ncopy)]
         a = mk(1, K)
         us = median_graph_time_us(torch, stream, [(lambda w=w: sbvr.mm_T(a, w)) for w in rs_])
-        others.append(dict(row(N, K, 1, S, G, us, IDXB), kernel="popcount product, both operands encoded (popc_mm_kernel)"))
+        others.append(dict(row(N, K, 1, S, G, us, IDXB), kernel="product of two encodings (csrc/popc_mm.cu)"))
         try:
             from oracle import ref_cuda
             if ref_cuda.lib() is not None:
