@@ -29,17 +29,17 @@
 // each on its own, with two A buffers and one D buffer: while the MMAs of unit i run, unit i + 1 is expanded into the other
 // A buffer and unit i + 2 read from shared memory; as soon as they are done the sums are read and the MMAs of unit i + 1
 // released, and the multiply-adds run beside those.  (Two groups per k block take two D buffers and leave room for one A.)  A
-// warp holds all sums of a quarter of a tile's rows.  The chunks' sums of a
-// quarter meet in scratch: every warp stores its own, counts its arrival a unit later (the stores have landed by then), looks
-// at the answer another unit later, and adds them in chunk order if it was the last (the same bits on every run; nobody waits
-// for another CTA, and all of it but the last tile's runs beside the other warpgroups' units).  A tile that several warpgroups
-// share is put together in shared memory at the end.  Every wait is bounded.
+// warp holds all sums of a quarter of a tile's rows.  A tile that several warpgroups share is put together in shared memory at the
+// end.  The chunks' sums meet in scratch when the CTAs of a group (the chunks of the same tiles) are through: each adds an equal
+// share of them in chunk order (the same bits on every run).  Added by whichever warp arrived last at a tile's counter, as
+// before, the slow CTAs of a group got nearly all of that work on top: at 28672 x 8192 they ended 27 us behind the mean of 70.
+// Every wait is bounded.
 //
-// What bounds it: no pipe is saturated (14336 x 4096: tensor pipe 49 % active, issue slots 46 %); a unit takes 1 030 cycles of its SM
-// at 28672 x 8192, 650 with half the MMAs, which follow one another on one accumulator; on small weights the two launches and the
-// merge of the chunks.  Per call with the quantiser, M = 16, S = 4, us (the fp16 GEMM in brackets): 1024 x 4096 10.9 (11.1),
-// 4096 x 4096 12.6 (14.8), 14336 x 4096 28.1 (32.3), 10240 x 8192 46 (58), 28672 x 8192 109 (113); six digits, whose error the GEMM
-// does not have, took 9.0, 11.6, 22.0 and, at 28672 x 8192, 67.
+// What bounds it: the tensor pipe in the loop (a unit takes 485 cycles of its SM at 14336 x 4096, its 24 MMAs 391 of a pipe that
+// does nothing else); around it, per launch, 4.7 us from the end of the kernel in front to the digits in shared memory (of it 1 to 1.7
+// in the quantiser) and 2 to 3 us for the merge.  Per call with the quantiser, M = 16, S = 4, us (before; the fp16 GEMM):
+// 1024 x 4096 9.4 (11.0; 10.4), 4096 x 4096 10.9 (12.7; 14.8), 14336 x 4096 21.7 (27.8; 32.1), 4096 x 14336 26.6 (39.7; 31.6),
+// 28672 x 8192 60 (104; 112); groups of 128, 14336 x 4096: 24.2 (30.0; 31.9).
 //
 // Replaces the M > 1 use of `_sbvr_row_deq_mm_T` (reference sbvr/kernels/sbvr_kernel.cu:121-191) for 2 .. 16 rows.
 #include <cuda.h>
@@ -76,9 +76,10 @@ struct SbParams {
     const __half* bias;
     __half* y;
     unsigned int* status;
-    unsigned int* counters;       // one per quarter of a tile's rows, zero between launches
+    unsigned int* counters;       // one per group of CTAs that work on the same tiles, zero between launches
     float* part;                  // [KC][NT][SB_MP][TN] sums of the chunks (KC > 1)
     int M, N, K, KB, NT, C, KC, GN, cache_in_smem, stages, idx_bytes;
+    int tagged;                   // `part` lies in the exchange region, all zero between launches, and a sum's arrival is its own mark
     int off_cache, off_ring, off_res;
 };
 
@@ -97,25 +98,28 @@ struct SbQuant {
 // ---------------------------------------------------------------------------------------------
 // activations (with the op in front of the linear) -> digit blob, once per call
 // ---------------------------------------------------------------------------------------------
-// One block per 256-k block and two (padded) activation rows, one warp per row: with 64 threads of at most 32
-// registers a block fits beside a resident CTA of the product, which leaves 1 024 registers in each quarter of the SM, and both wait
-// for their predecessors there (with 40 registers a call took 6 us more: the quantiser started when the product had ended).  Lane (kw, j) owns the eight elements
+// One block per 256-k block and (padded) activation row; its four warps take a level and three of its digits each, so that the chain
+// from the arrival of the row to the last digit is a quarter as long (the product waits for it).  With at most 32 registers a thread
+// the blocks fit beside a resident CTA of the product, and both wait for their predecessors there (with blocks that did not fit, a call
+// took 6 us more: the quantiser started when the product had ended).  Lane (kw, j) owns the eight elements
 // k = 32 kw + j + 4 e, which are one 32-bit word (nibble e) of every digit: the K order in which the weight expansion
 // leaves the plane bits.  Blob of a k block: [MMA j (SB_NJ)][row group (4)][kw (8)][row (8)][16 B], then 32 rows x 16 B:
 // words 0 .. 2 hold the scale bytes of MMA 2 i (bytes 0, 1) and 2 i + 1 (bytes 2, 3) for that B row, word 3 of row m whether
 // activation row m of this block holds a non-finite value.
-__global__ void __launch_bounds__(64, 32) sb_quant_kernel(const SbQuant p) {
-    __shared__ __align__(16) __half row[2][256];
+__global__ void __launch_bounds__(128, 16) sb_quant_kernel(const SbQuant p) {
+    __shared__ __align__(16) __half row[4][256];
+    __shared__ float ssum[4];
     pdl_launch_dependents();
     pdl_wait();                                    // the activations come from the previous kernel of the stream
     const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kb = blockIdx.x, K = p.K, M = p.M, m = blockIdx.y * 2 + wl;
+    const int kb = blockIdx.x, K = p.K, M = p.M, m = blockIdx.y;
     const int kw = lane >> 2, j = lane & 3;
+    const int level = wl >> 1, d0 = (wl & 1) * 3;
     int ex = 15;
     bool poison = false;
     float inv = 0.0f;
     if (m < M) {
-        // this warp's 256 activations: lane l brings elements 8 l .. 8 l + 7
+        // 256 activations: lane l of every warp brings elements 8 l .. 8 l + 7
         const size_t off = (size_t)m * K + (size_t)kb * 256 + lane * 8;
         uint4 o;
         __half2* oh = reinterpret_cast<__half2*>(&o);
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(64, 32) sb_quant_kernel(const SbQuant p) {
             // mean of (h + delta)^2 over the whole row, the sum formed in fp16 like the separate kernel does
             float sq = 0.0f;
 #pragma unroll 4
-            for (int c = lane; c < K / 8; c += 32) {
+            for (int c = threadIdx.x; c < K / 8; c += 128) {
                 uint4 a = __ldg(reinterpret_cast<const uint4*>(p.x + (size_t)m * K) + c);
                 __half2* ah = reinterpret_cast<__half2*>(&a);
                 if (p.delta) {
@@ -151,7 +155,9 @@ __global__ void __launch_bounds__(64, 32) sb_quant_kernel(const SbQuant p) {
             }
 #pragma unroll
             for (int s = 16; s; s >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, s);
-            const float rs = rsqrtf(sq / (float)K + p.eps);
+            if (lane == 0) ssum[wl] = sq;
+            __syncthreads();
+            const float rs = rsqrtf((ssum[0] + ssum[1] + ssum[2] + ssum[3]) / (float)K + p.eps);
             uint4 a = __ldg(reinterpret_cast<const uint4*>(p.x + off));
             __half2* ah = reinterpret_cast<__half2*>(&a);
             if (p.delta) {
@@ -160,7 +166,7 @@ __global__ void __launch_bounds__(64, 32) sb_quant_kernel(const SbQuant p) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) ah[e] = __hadd2(ah[e], bh[e]);
             }
-            if (p.h_out) *reinterpret_cast<uint4*>(p.h_out + off) = a;
+            if (p.h_out && wl == 0) *reinterpret_cast<uint4*>(p.h_out + off) = a;
             const uint4 wv = __ldg(reinterpret_cast<const uint4*>(p.norm_w + (size_t)kb * 256 + lane * 8));
             const __half2* wh = reinterpret_cast<const __half2*>(&wv);
 #pragma unroll
@@ -175,17 +181,16 @@ __global__ void __launch_bounds__(64, 32) sb_quant_kernel(const SbQuant p) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) e[i] = p.x[off + i];
         }
-        if (p.x_out) *reinterpret_cast<uint4*>(p.x_out + off) = o;
-        reinterpret_cast<uint4*>(row[wl])[lane] = o;
-        __syncwarp();
-        const __half* xp = row[wl] + 32 * kw + j;
+        if (p.x_out && wl == 0) *reinterpret_cast<uint4*>(p.x_out + off) = o;
         float a = 0.0f;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            float av = fabsf(__half2float(xp[4 * e]));
-            if (!(av == av)) av = __int_as_float(0x7f800000);     // NaN counts as infinity
+        for (int e = 0; e < 4; ++e) {
+            const float2 f = __half22float2(oh[e]);
+            float av = fmaxf(fabsf(f.x), fabsf(f.y));
+            if (f.x != f.x || f.y != f.y) av = __int_as_float(0x7f800000);     // NaN counts as infinity
             a = fmaxf(a, av);
         }
+        reinterpret_cast<uint4*>(row[wl])[lane] = o;
 #pragma unroll
         for (int s = 16; s; s >>= 1) a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, s));
         if (a >= __int_as_float(0x7f800000)) {
@@ -194,36 +199,33 @@ __global__ void __launch_bounds__(64, 32) sb_quant_kernel(const SbQuant p) {
             ex = (int)((__float_as_uint(a) >> 23) & 0xFF) - 127;              // a = 1.f * 2^ex, ex in [-24, 15]
             inv = __uint_as_float((uint32_t)(15 - ex + 127) << 23);
         }
+        __syncwarp();
     }
     unsigned char* blob = p.xb + (size_t)kb * SB_BLOB;
     // E2M1 codes of digit t - 4 (t = 0 .. 7), one nibble each: the value itself for j = 0, 1, half of it for j = 2, 3
     const uint32_t lut = (j < 2) ? 0x5420ACDEu : 0x32109ABCu;
-    // one level after the other: a thread must not need more than 32 registers (see above)
-#pragma unroll 1
-    for (int level = 0; level < 2; ++level) {
-        uint32_t words[6] = {0u, 0u, 0u, 0u, 0u, 0u};
-        if (m < M && !poison) {
+    uint32_t words[3] = {0u, 0u, 0u};
+    if (m < M && !poison) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const float f = __half2float(row[wl][32 * kw + j + 4 * e]) * inv;              // exact
-                int q = __float2int_rn(f);                                                     // |q| <= 2^16
-                if (level) q = __float2int_rn((f - (float)q) * 131072.0f);                     // the difference is exact; |q| <= 2^16
-                const uint32_t u = (uint32_t)(q + 0x24924);
+        for (int e = 0; e < 8; ++e) {
+            const float f = __half2float(row[wl][32 * kw + j + 4 * e]) * inv;                  // exact
+            int q = __float2int_rn(f);                                                         // |q| <= 2^16
+            if (level) q = __float2int_rn((f - (float)q) * 131072.0f);                         // the difference is exact; |q| <= 2^16
+            const uint32_t u = (uint32_t)(q + 0x24924) >> (3 * d0);
 #pragma unroll
-                for (int d = 0; d < 6; ++d) words[d] |= ((lut >> (4u * ((u >> (3 * d)) & 7u))) & 0xFu) << (4 * e);
-            }
+            for (int d = 0; d < 3; ++d) words[d] |= ((lut >> (4u * ((u >> (3 * d)) & 7u))) & 0xFu) << (4 * e);
         }
+    }
 #pragma unroll
-        for (int d = 0; d < 6; ++d) {
-            const int dd = level * 6 + d;
-            const int r = (dd & 1) * 16 + m;
-            *reinterpret_cast<uint32_t*>(blob + (dd >> 1) * 4096 + (r >> 3) * 1024 + kw * 128 + (r & 7) * 16 + j * 4) = words[d];
-        }
+    for (int d = 0; d < 3; ++d) {
+        const int dd = level * 6 + d0 + d;
+        const int r = (dd & 1) * 16 + m;
+        *reinterpret_cast<uint32_t*>(blob + (dd >> 1) * 4096 + (r >> 3) * 1024 + kw * 128 + (r & 7) * 16 + j * 4) = words[d];
     }
     // scale bytes 127 + exponent, each twice (two 32-element blocks per MMA); rows beyond M: 2^0 on zero digits
     auto two = [&](int d) -> uint32_t { return (m < M ? (uint32_t)(127 + 3 * (d % 6) + ex - (d < 6 ? 15 : 32)) : 127u) * 0x0101u; };
     uint4* sf = reinterpret_cast<uint4*>(blob + SB_NJ * 4096);
-    if (lane < 2)                                  // even digits in row m, odd ones in row 16 + m; MMA j has digits 2 j, 2 j + 1
+    if (wl == 0 && lane < 2)                       // even digits in row m, odd ones in row 16 + m; MMA j has digits 2 j, 2 j + 1
         sf[lane * 16 + m] = make_uint4(two(lane) | (two(2 + lane) << 16), two(4 + lane) | (two(6 + lane) << 16),
                                        two(8 + lane) | (two(10 + lane) << 16), poison ? 1u : 0u);
 }
@@ -250,15 +252,6 @@ struct SbPair {
     }
 };
 
-// A warp's stores so far become visible, then its arrival is counted; lane 0 gets the arrivals before it.
-__device__ __forceinline__ unsigned int sb_arrive(unsigned int* counter, int lane) {
-    unsigned int old = 0u;
-    __threadfence();
-    __syncwarp();
-    if (lane == 0) old = atomicAdd(counter, 1u);
-    return old;
-}
-
 // y[m, n] of an activation row that holds something non-finite, as products give it: the digits cannot say it and have left a NaN.
 // Inlined where few values are live (88 registers, 80 without it): as a function that is called it took the kernel to 94, which leaves
 // no room beside a CTA for the blocks of the GEMM's re-tiling (seven linears of a layer, 16 rows: 154 against 146 us).
@@ -278,52 +271,81 @@ __device__ __forceinline__ void sb_multiply_out(const SbParams& p, int G, int m,
     p.y[(size_t)m * p.N + n] = __float2half_rn(acc + (p.bias ? __half2float(p.bias[n]) : 0.0f));
 }
 
-// The chunks' sums of a quarter of a tile's rows -> y, in chunk order; the counter goes back to zero.
+// A chunk's sum on its way to the CTA that adds it: never the bit pattern zero, which stands for "not there yet" (p.tagged).
+__device__ __forceinline__ void sb_put(float* dst, float v) { __stcg(dst, v == 0.0f ? -0.0f : v); }
+
+// The chunks' sums of the group's tiles [t0, t0 + ntc) -> y, in chunk order.  The KC CTAs of the group take equal shares of the
+// (tile, activation row, four output rows) list, whoever of them was slow; four chunks' loads are in flight per thread.
 template <int S, int NSUB>
-__device__ __forceinline__ void sb_add_chunks(const SbParams& p, int tile, int quarter, int lane) {
-    constexpr int TN = ts_tn(S), MP = SB_MP, QR = TN / 4, PER = MP * QR / 32, H = 16 / PER;
-    if (lane == 0) p.counters[tile * 4 + quarter] = 0u;
-    __threadfence();
-    const size_t plane = (size_t)p.NT * (MP * TN);
-    const float* src = p.part + (size_t)tile * (MP * TN) + quarter * QR;
-    unsigned int nan = 0u;
-    float v[PER];
-#pragma unroll
-    for (int u = 0; u < PER; ++u) v[u] = 0.0f;
+__device__ __forceinline__ void sb_add_chunks(const SbParams& p, int t0, int ntc, int chunk, volatile int* abort_flag) {
+    constexpr int TN = ts_tn(S), Q = TN / 4;
+    const int total = ntc * p.M * Q;               // (below 2^31: the host bounds the tiles)
+    const int e1 = (int)((long long)total * (chunk + 1) / p.KC);
+    const size_t plane = (size_t)p.NT * (SB_MP * TN);
+    const bool wide = (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
 #pragma unroll 1
-    for (int c = 0; c < p.KC; c += H) {            // H chunks' loads in flight
-        float t[H][PER];
+    for (int e = (int)((long long)total * chunk / p.KC) + (int)threadIdx.x; e < e1; e += SB_THREADS) {
+        const int q = e % Q, m = e / Q % p.M, tile = t0 + e / (Q * p.M);
+        float* src = p.part + ((size_t)tile * SB_MP + m) * TN + q * 4;
+        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+        for (int c = 0; c < p.KC; c += 4) {
+            float4 t[4];
+            const long long c0 = clock64();
+            for (;;) {
+                bool all = true;
 #pragma unroll
-        for (int h = 0; h < H; ++h)
+                for (int h = 0; h < 4; ++h) {
+                    t[h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (c + h < p.KC)
+                        asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(t[h].x), "=f"(t[h].y), "=f"(t[h].z), "=f"(t[h].w)
+                                     : "l"(src + (size_t)(c + h) * plane)
+                                     : "memory");
+                }
+                if (!p.tagged) break;
 #pragma unroll
-            for (int u = 0; u < PER; ++u) {
-                const int q = lane + 32 * u, m = q / QR;
-                t[h][u] = (c + h < p.KC && m < p.M) ? __ldcg(src + (size_t)(c + h) * plane + m * TN + q % QR) : 0.0f;
+                for (int h = 0; h < 4; ++h)
+                    if (c + h < p.KC)
+                        all = all && __float_as_uint(t[h].x) && __float_as_uint(t[h].y) && __float_as_uint(t[h].z) && __float_as_uint(t[h].w);
+                if (all || *abort_flag) break;
+                if (clock64() - c0 > 2000000000LL) {                          // a chunk never came
+                    *abort_flag = 1;
+                    atomicExch(p.status, 1u);
+                    atomicExch(p.status + 1, 0x441u);
+                    break;
+                }
             }
 #pragma unroll
-        for (int h = 0; h < H; ++h)
-#pragma unroll
-            for (int u = 0; u < PER; ++u) v[u] += t[h][u];
-    }
-#pragma unroll
-    for (int u = 0; u < PER; ++u) {
-        const int q = lane + 32 * u, m = q / QR, n = tile * TN + quarter * QR + q % QR;
-        if (m < p.M) {
-            p.y[(size_t)m * p.N + n] = __float2half_rn(v[u] + (p.bias ? __half2float(p.bias[n]) : 0.0f));
-            if (v[u] != v[u]) nan |= 1u << u;
+            for (int h = 0; h < 4; ++h) {
+                v[0] += t[h].x, v[1] += t[h].y, v[2] += t[h].z, v[3] += t[h].w;
+                if (p.tagged && c + h < p.KC)
+                    __stcg(reinterpret_cast<float4*>(src + (size_t)(c + h) * plane), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+            }
         }
-    }
-    if (p.x) {
+        const int n = tile * TN + q * 4;
+        __half* dst = p.y + (size_t)m * p.N + n;
+        __align__(8) __half o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = __float2half_rn(v[i] + (p.bias ? __half2float(p.bias[n + i]) : 0.0f));
+        if (wide) {                                // (N is a multiple of TN)
+            *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dst[i] = o[i];
+        }
+        if (p.x) {
 #pragma unroll 1
-        for (; nan; nan &= nan - 1) {
-            const int q = lane + 32 * (__ffs((int)nan) - 1);
-            sb_multiply_out<S>(p, 256 / NSUB, q / QR, tile * TN + quarter * QR + q % QR);
+            for (int i = 0; i < 4; ++i)
+                if (v[i] != v[i]) sb_multiply_out<S>(p, 256 / NSUB, m, n + i);
         }
     }
 }
 
+// (88 registers: beside a CTA there is room for two blocks of the next call's quantiser, which 16 rows of 4096 need to be resident at
+// once; with 96, at 4096 x 4096 and groups of 128, a call took 16.5 us instead of 11.8.)
 template <int S, int NSUB, int IDXB>
-__global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ SbParams p) {
+__global__ void __maxnreg__(88) linear_sb_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ SbParams p) {
     pdl_launch_dependents();
     extern __shared__ __align__(1024) unsigned char smem[];
     constexpr int SP = ts_sp(S);
@@ -369,8 +391,6 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
     __syncthreads();
     const bool bulk_cache = p.cache_in_smem && ((p.C * S * 2) % 16 == 0);
 
-    int pend = 0, ptile = 0;                       // a tile of which the chunks' sums are being counted: 1 stored, 2 counted
-    unsigned int old = 0u;
     if (warp < SB_NWG) {
         // ------------------------------ issuer warps, one per warpgroup ------------------------------
         const int w = warp;
@@ -527,15 +547,6 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
         for (int m = 0; m < MP / 2; ++m) acc[m] = SbPair(0.0f, 0.0f);
         const int wpos = nl * S + s;
         int tile = t0 + u0 / nkb, have = 0;        // tile of the sums, units of it in them
-        auto settle = [&]() {                      // the next step of counting the pending tile
-            if (pend == 1) {
-                old = sb_arrive(p.counters + ptile * 4 + wl, lane);
-                pend = 2;
-            } else if (pend == 2) {
-                pend = 0;
-                if (__shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<S, NSUB>(p, ptile, wl, lane);
-            }
-        };
         // Sums of one tile's units: planes added across their lanes, after which a lane has the activation rows
         // m = s NV .. s NV + NV - 1 of its output row.  A tile that is all this warpgroup's goes out at once, one that it
         // shares with a neighbour (its first or its last) to shared memory.
@@ -562,12 +573,10 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                 for (int e = 0; e < NV; ++e)
                     if ((pm >> (s * NV + e)) & 1u) v[e] = __int_as_float(0x7fc00000);
                 if (KC > 1) {
-                    while (pend) settle();         // (one k block per chunk: a tile every unit)
                     float* dst = p.part + ((size_t)chunk * p.NT + tile) * (MP * TN) + nl;
 #pragma unroll
                     for (int e = 0; e < NV; ++e)
-                        if (s * NV + e < M) __stcg(dst + (s * NV + e) * TN, v[e]);
-                    pend = 1, ptile = tile;
+                        if (s * NV + e < M) sb_put(dst + (s * NV + e) * TN, v[e]);
                 } else {
                     const int n = tile * TN + nl;
                     const float bias = p.bias ? __half2float(p.bias[n]) : 0.0f;
@@ -648,7 +657,7 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
             ts_wait(mbar, (uint32_t)(i & 1), abort_flag, p.status, 0x434u);
             ts_fence_after();
             // the sums of one group: even and odd digits of every activation row
-            SbPair v[NSUB][MP / 2];
+            SbPair v[MP / 2];
             auto read = [&](int sub) {
                 uint32_t d[4][8];
                 ts_ld16_issue(d_addr + sub * 32, d[0], d[1]);
@@ -658,28 +667,30 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                 for (int g4 = 0; g4 < 4; ++g4) ts_wait_ld(d[g4]);
 #pragma unroll
                 for (int m = 0; m < MP; m += 2)
-                    v[sub][m / 2] = SbPair(d[m >> 3][m & 7], d[m >> 3][(m & 7) + 1]) + SbPair(d[2 + (m >> 3)][m & 7], d[2 + (m >> 3)][(m & 7) + 1]);
+                    v[m / 2] = SbPair(d[m >> 3][m & 7], d[m >> 3][(m & 7) + 1]) + SbPair(d[2 + (m >> 3)][m & 7], d[2 + (m >> 3)][(m & 7) + 1]);
+            };
+            auto fold = [&](int sub) {
+#pragma unroll
+                for (int m = 0; m < MP / 2; ++m) acc[m] = v[m].mul_add(SbPair(c0[sub], c0[sub]), acc[m]);
             };
 #pragma unroll
-            for (int sub = 0; sub < NSUB; ++sub) read(sub);      // (one after the other: both groups' columns at once spill)
+            for (int sub = 0; sub < NSUB; ++sub) { // (one after the other: both groups' sums at once need 96 registers)
+                read(sub);
+                if (sub + 1 < NSUB) fold(sub);
+            }
             if (more) {
                 ts_wait_st();
                 ts_fence_before();
                 ts_bar_arrive(1 + w, 160);         // releases the MMAs of unit i + 1; also: its stage has been read
             }
-#pragma unroll
-            for (int sub = 0; sub < NSUB; ++sub)
-#pragma unroll
-                for (int m = 0; m < MP / 2; ++m) acc[m] = v[sub][m].mul_add(SbPair(c0[sub], c0[sub]), acc[m]);
+            fold(NSUB - 1);
             ++have;
-            if (KC > 1 && pend) settle();
             if (++kl == nkb || !more) {
                 kl = 0;
                 // (a shared tile's sums: the last tile of the warpgroup's range unless the range lies inside one tile)
                 deposit(!more && tile > t0 + u0 / nkb);
             }
         }
-        if (KC > 1 && pend == 1) settle();         // counted; the answer is looked at below
     }
     ts_fence_before();
     __syncthreads();
@@ -691,8 +702,6 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
     // ------------------------------ tiles shared by warpgroups ------------------------------
     // Tile `tl` of the range has units [tl nkb, (tl + 1) nkb), warpgroup w the units [w U / 4, (w + 1) U / 4); where a boundary
     // lies inside a tile its warpgroups' sums are added here, in warpgroup order, by a warp per quarter of the tile.
-    unsigned int shared_old = 0u;
-    int shared_tile = -1;
     if (warp < 4 * (SB_NWG - 1)) {
         constexpr int QR = TN / 4;                 // rows of a quarter
         const int wb = (warp >> 2) + 1, qt = warp & 3;
@@ -710,19 +719,39 @@ __global__ void __launch_bounds__(SB_THREADS, 1) linear_sb_kernel(const __grid_c
                     if (a < (tl + 1) * nkb && b > tl * nkb && a < b) v += res[(size_t)(w * 2 + (tl > a / nkb ? 1 : 0)) * (MP * TN) + m * TN + nl];
                 }
                 if ((pm >> m) & 1u) v = __int_as_float(0x7fc00000);
-                if (KC > 1) __stcg(p.part + ((size_t)chunk * p.NT + t0 + tl) * (MP * TN) + m * TN + nl, v);
+                if (KC > 1) sb_put(p.part + ((size_t)chunk * p.NT + t0 + tl) * (MP * TN) + m * TN + nl, v);
                 else p.y[(size_t)m * N + n] = __float2half_rn(v + (p.bias ? __half2float(p.bias[n]) : 0.0f));
                 if (KC == 1 && p.x && ((pm >> m) & 1u)) sb_multiply_out<S>(p, 256 / NSUB, m, n);
             }
-            if (KC > 1) {
-                shared_tile = t0 + tl;
-                shared_old = sb_arrive(p.counters + shared_tile * 4 + qt, lane);
-            }
         }
     }
-    if (pend == 2 && __shfl_sync(0xffffffffu, old, 0) == (unsigned int)(KC - 1)) sb_add_chunks<S, NSUB>(p, ptile, warp & 3, lane);
-    if (shared_tile >= 0 && __shfl_sync(0xffffffffu, shared_old, 0) == (unsigned int)(KC - 1))
-        sb_add_chunks<S, NSUB>(p, shared_tile, warp & 3, lane);
+    // ------------------------------ the chunks of K meet ------------------------------
+    // (The group's CTAs are all resident: there are at most as many as SMs.)  Few sums: their slots are zero before the launch, whoever
+    // needs one waits until it is not, and clears it.  Many: the CTAs arrive at a counter that wraps to zero with the last of them,
+    // and wait for that zero, which the counter had before the first came; a fence, an atomic and a poll take 1.5 us longer.
+    if (KC > 1) {
+        if (!p.tagged) {
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                __threadfence();
+                unsigned int left = atomicInc(p.counters + grp, (unsigned int)(KC - 1)) + 1u;
+                if (left == (unsigned int)KC) left = 0u;
+                const long long c0 = clock64();
+                while (left) {
+                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(left) : "l"(p.counters + grp) : "memory");
+                    if (*abort_flag || clock64() - c0 > 2000000000LL) break;
+                }
+                if (left && !*abort_flag) {
+                    *abort_flag = 1;
+                    atomicExch(p.status, 1u);
+                    atomicExch(p.status + 1, 0x440u);
+                }
+                __threadfence();
+            }
+            __syncthreads();
+        }
+        sb_add_chunks<S, NSUB>(p, t0, ntc, chunk, abort_flag);
+    }
     if (threadIdx.x == 0 && *abort_flag) {         // which problem gave up: N, and K / 256 | M | CTA (for the host's message)
         atomicExch(p.status + 2, (unsigned int)p.N);
         atomicExch(p.status + 3, ((unsigned int)p.KB << 16) | ((unsigned int)M << 8) | (blockIdx.x & 0xFFu));
@@ -790,12 +819,12 @@ bool linear_sb_supported(const PackedW& w, int M) {
     return sb_plan(w, di, &pl) == SBVR_OK;
 }
 
-// Where it is faster than the GEMM.  Up to four chunks of K (M = 16, us, the GEMM in brackets: 1024 x 4096 10.9 (11.1), 2048 x 2048
-// 9.5 (9.8), 4096 x 4096 12.6 (14.8), with two planes 12.5 (12.5), groups of 128 13.8 (14.7), 14336 x 4096 28.1 (32.3)), on weights of so
-// few rows that the GEMM has one or two tiles (128 x 14336 11.0 (14.8), but 512 x 14336 18.6 (14.7)) and, with up to eight chunks, on
-// weights of many rows (10240 x 8192 46 (58), 28672 x 8192 109 (113), but 4096 x 8192 25 (22), 8192 x 8192 39 (36) and, with groups of
-// 128, 28672 x 8192 114 (110)); beyond, the chunks' merge costs more than is gained: 4096 x 11008 33 (27), 4096 x 14336 42 (32).
-bool linear_sb_preferred(const PackedW& w) { return w.K <= 4096 || w.N <= 256 || (w.K <= 8192 && w.N > 8192 && w.G == 256); }
+// Where it is faster than the GEMM (M = 16, us, the GEMM in brackets).  Up to four chunks of K: 1024 x 4096 9.4 (10.4), 4096 x 4096 10.9
+// (14.8), 14336 x 4096 21.7 (32.1), 32768 x 1024 13.7 (23.1).  More chunks, with weights of many rows: 2048 x 16384 20.5 (23.7), 4096 x 8192
+// 19.5 (21.8), 4096 x 14336 26.6 (31.6; with groups of 128 30.6 (31.0)), 8192 x 28672 61.6 (104), 28672 x 8192 60 (112).  In between
+// the chunks' merge costs what the product gains: 1024 x 14336 16.2 (16.1; two planes 15.4 (13.1)), 512 x 28672 18.3 (18.4; two planes
+// 16.9 (15.4)); weights of so few rows that the GEMM has one or two tiles: 128 x 14336 12.3 (14.9).
+bool linear_sb_preferred(const PackedW& w) { return w.K <= 4096 || w.N <= 256 || w.N >= 2048; }
 
 size_t linear_sb_workspace_bytes(const PackedW& w, const DeviceInfo& di) {
     SbPlan pl;
@@ -866,11 +895,12 @@ int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __ha
     if (rc) return rc;
     // (an op in front: its result is kept for rows that have to be multiplied out)
     q.x_out = q.x_op != SBVR_XOP_NONE && multiply_out ? reinterpret_cast<__half*>(scratch + pl.blob_bytes + pl.part_bytes) : nullptr;
-    SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel, dim3(pl.KB, SB_MP / 2), dim3(64), 0, st, q));
+    SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel, dim3(pl.KB, SB_MP), dim3(128), 0, st, q));
     SbParams p;
     p.xb = q.xb;
     p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status, p.counters = counters;
-    p.part = reinterpret_cast<float*>(scratch + pl.blob_bytes);
+    p.tagged = pl.KC > 1 && pl.part_bytes <= SBVR_WS_XCHG_BYTES;
+    p.part = p.tagged ? reinterpret_cast<float*>(counters) : reinterpret_cast<float*>(scratch + pl.blob_bytes);
     p.x = !multiply_out ? nullptr : q.x_out ? q.x_out : x, p.bvr = w.bvr, p.idx_bytes = w.idx_bytes;
     p.M = M, p.N = w.N, p.K = w.K, p.KB = pl.KB, p.NT = pl.NT, p.C = w.C, p.KC = pl.KC, p.GN = pl.GN;
     p.cache_in_smem = pl.cache_in_smem, p.stages = pl.stages;

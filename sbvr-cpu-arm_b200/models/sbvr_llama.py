@@ -347,7 +347,7 @@ class SBVRLlamaForCausalLM(torch.nn.Module):
             w = lin.weight
             K = w.in_features_padded
             N = w.out_features
-            return T <= 4 or K <= 4096 or N <= 256 or (K <= 8192 and N > 8192 and w.bvr_len == 256)
+            return T <= 4 or K <= 4096 or N <= 256 or N >= 2048
         hc, ho = b.h, b.h2                         # current residual, spare buffer
 
         def norm_linear(lin, delta, weight, out, keep_residual=True):

@@ -448,3 +448,31 @@ def test_non_finite_activations_of_small_batches(M, N, K, G, S, mode, op):
     ok = torch.isfinite(z)
     assert ((y[ok].float() - z[ok].float()).abs().max() / z[ok].float().abs().max()).item() < 1e-3
     check_status()
+
+
+@pytest.mark.parametrize("M", [5, 16])
+@pytest.mark.parametrize("S,G,N,K", [(4, 256, 4096, 4096), (4, 256, 4128, 4096), (2, 256, 64, 8192), (3, 128, 96, 1280), (4, 256, 2048, 4352)])
+@pytest.mark.parametrize("what", ["random", "zero weight", "zero rows", "odd y"])
+def test_small_batch_kernel_merges_its_chunks(M, S, G, N, K, what):
+    """Up to 1 MiB of partial sums (4096 x 4096 fills it exactly, 4128 rows are beyond) an arrived sum is told from an empty slot by its
+    bits: sums of zero must arrive too, and the slots must be empty again for the next call.  Tolerance: one rounding of the
+    result (2^-11) and fp32 sums."""
+    import sbvr
+    p = O.make_packed(N, K, S, G=G, mode="u16", C=1000, seed=N + K)
+    if what == "zero weight":
+        p["coeff"][:] = 0
+    rng = np.random.default_rng(M)
+    x = rng.standard_normal((M, K)).astype(np.float16)
+    if what == "zero rows":
+        x[1:] = 0
+    ref = O.linear_c(x, p["bvr"], p["coeff_idx"], p["coeff"], G=G).astype(np.float64)
+    w, xd = to_sbvr(p), torch.from_numpy(x).cuda()
+    buf = torch.full((M * N + 1,), float("nan"), dtype=torch.float16, device="cuda")
+    out = buf[1:].view(M, N) if what == "odd y" else buf[:-1].view(M, N)
+    sbvr.linear(xd, w, None, algo=4, out=out)
+    first = out.clone()
+    assert np.abs(h2n(first) - ref).max() <= 1e-3 * max(np.abs(ref).max(), 1e-30)
+    assert not torch.signbit(first[first == 0]).any() or what == "random"
+    for _ in range(3):
+        assert torch.equal(first, sbvr.linear(xd, w, None, algo=4))
+    check_status()

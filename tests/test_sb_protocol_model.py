@@ -3,8 +3,9 @@
 Inside a CTA a warpgroup works on its own: an issuer (ring of weight stages, MMAs and their commits) and four compute warps (words
 of unit i + 1 into tensor memory and of unit i + 2 out of shared memory beside the MMAs of unit i; its sums read before the
 MMAs of unit i + 1 are released through a named barrier).  mbarriers are waited on by PARITY, as on the device, so a waiter that
-fell two phases behind would be caught as aliasing.  Between CTAs the K chunks' sums of a quarter tile are stored, counted a unit
-later and looked at another unit later.  The tests check: no deadlock, no aliasing, no stage, operand or sum that is overwritten
+fell two phases behind would be caught as aliasing.  Between CTAs the K chunks' sums meet when a group's CTAs are through: at a counter
+that wraps to zero, or in slots whose value is its own mark (`group`; `chunks` is the protocol before that: stored, counted a
+unit later and looked at another unit later).  The tests check: no deadlock, no aliasing, no stage, operand or sum that is overwritten
 before all of its readers are done, exactly one warp that adds a quarter and all chunks' stores before it; and that the same
 checks do flag protocols with a step out of place.
 """
@@ -213,3 +214,64 @@ def test_chunks_are_added_once_and_after_all_stores():
 
 def test_model_flags_a_count_in_front_of_the_store():
     assert any(chunks(4, 3, trial, "count first") for trial in range(40))
+
+
+def group(KC, launches, tagged, seed, mistake=None):
+    """KC CTAs of a group, launch after launch: sums stored, then all of them waited for and each CTA's share read (and cleared)."""
+    rnd = random.Random(seed)
+    slots = [[None] * KC for _ in range(KC)]       # [share][chunk]: launch whose sum it holds, None: empty
+    counter, errors = 0, []
+
+    def cta(chunk, launch):
+        nonlocal counter
+        if mistake == "count first":
+            counter = (counter + 1) % KC
+        for share in rnd.sample(range(KC), KC):
+            yield
+            if tagged and slots[share][chunk] is not None:
+                errors.append("slot still full")
+            slots[share][chunk] = launch
+        if not tagged:
+            yield
+            if mistake != "count first":
+                counter = (counter + 1) % KC
+            while counter:
+                yield
+        else:
+            while mistake != "no wait" and None in slots[chunk]:
+                yield
+        if slots[chunk] != [launch] * KC:
+            errors.append("share read before all chunks are stored")
+        if tagged:
+            for c in range(KC):
+                yield
+                slots[chunk][c] = None
+        yield
+
+    for launch in range(launches):                 # (a launch begins when the one before has ended)
+        agents = [cta(c, launch) for c in range(KC)]
+        steps = 0
+        while agents and not errors:
+            steps += 1
+            if steps > 100000:
+                return errors + ["deadlock"]
+            a = rnd.choice(agents)
+            try:
+                next(a)
+            except StopIteration:
+                agents.remove(a)
+        if counter:
+            errors.append("counter is not zero after a launch")
+    return errors
+
+
+@pytest.mark.parametrize("tagged", [False, True])
+def test_chunks_of_a_group_meet(tagged):
+    for trial in range(200):
+        rnd = random.Random(trial)
+        assert group(rnd.randint(2, 8), rnd.randint(1, 3), tagged, trial) == []
+
+
+@pytest.mark.parametrize("tagged,mistake", [(False, "count first"), (True, "no wait")])
+def test_group_model_flags_a_step_out_of_place(tagged, mistake):
+    assert any(group(4, 2, tagged, trial, mistake) for trial in range(40))
