@@ -227,6 +227,28 @@ typedef struct sbvr_encode_walk {
  * searches its own candidates.  Synchronises `stream`; the answer is in *result. */
 SBVR_API int sbvr_encode_advance(const sbvr_encode_walk_t* walk, sbvr_stream_t stream);
 
+/* Many steps of the walk in one cooperative launch, decisions included (sbvr/core.py:555-577, :605-653): up to `limit` misses, until
+ * nothing is left, the codebook is full, or a group needs the caller (sbvr_encode_advance from `outcome` on).  `walk` as
+ * above with search = 1 and append_at = -1; line1 and cutoff are not looked at.  Synchronises `stream`. */
+#define SBVR_ENCODE_WINDOW 64
+enum { SBVR_ENCODE_DONE = 1, SBVR_ENCODE_LIMIT = 2, SBVR_ENCODE_FULL = 3, SBVR_ENCODE_CALLER = 4, SBVR_ENCODE_TIMEOUT = 5 };
+typedef struct sbvr_encode_record {
+    int group, at;                      /* a group that keeps its own candidate; the line it is filed under */
+    float mse;
+    unsigned short line[4];             /* the candidate, ascending magnitude; line `at` of the codebook if `at` was its length */
+} sbvr_encode_record_t;
+typedef struct sbvr_encode_run {
+    void* ctl;                          /* 64 bytes of device memory */
+    sbvr_encode_record_t* records;      /* `limit` of them, pinned host memory */
+    int* outcome;                       /* six, pinned host memory: why it stopped, from, lines, line0, misses, records */
+    int n, capacity;                    /* lines the codebook holds and can hold */
+    int warmup;                         /* fewer lines: every group is searched */
+    int window, hist_n, limit;          /* accepted errors the cut-off looks back on (<= SBVR_ENCODE_WINDOW), those in hist */
+    double acceptable;
+    double hist[SBVR_ENCODE_WINDOW];    /* the newest last */
+} sbvr_encode_run_t;
+SBVR_API int sbvr_encode_run(const sbvr_encode_walk_t* walk, const sbvr_encode_run_t* run, sbvr_stream_t stream);
+
 /* ---- the kernels between the linears of a Llama decoder layer ----------------------------------------------
  * Each replaces a chain of eager PyTorch ops of the reference model (models/sbvr_llama.py) by one launch.
  * All tensors fp16, contiguous, 16-byte aligned unless noted. */

@@ -105,7 +105,7 @@ lib.sbvr_ll_reduce_add_rmsnorm_digits_f16.restype = _i
 lib.sbvr_allreduce_add_rmsnorm_digits_f16.argtypes = [_vp, _vp, _vp, _i, _i, _i, _i, _sz, _vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp, _vp]
 lib.sbvr_allreduce_add_rmsnorm_digits_f16.restype = _i
 
-EXPORTS = ["sbvr_linear_workspace_bytes", "sbvr_linear_padded_f16", "sbvr_encode_stats_f16", "sbvr_encode_advance", "sbvr_popc_mm_f16", "sbvr_linear_t_f16", "sbvr_encode_mse_f16", "sbvr_encode_select_f16", "sbvr_encode_pack", "sbvr_rope_attention_f16", "sbvr_linear_fused_f16", "sbvr_allreduce_add_rmsnorm_f16", "sbvr_linear_push_f16", "sbvr_ll_reduce_add_rmsnorm_f16", "sbvr_ll_reduce_add_rmsnorm_digits_f16", "sbvr_allreduce_add_rmsnorm_digits_f16", "sbvr_add_rmsnorm_f16", "sbvr_rope_append_f16", "sbvr_attention_f16", "sbvr_silu_mul_f16",
+EXPORTS = ["sbvr_linear_workspace_bytes", "sbvr_linear_padded_f16", "sbvr_encode_stats_f16", "sbvr_encode_advance", "sbvr_encode_run", "sbvr_popc_mm_f16", "sbvr_linear_t_f16", "sbvr_encode_mse_f16", "sbvr_encode_select_f16", "sbvr_encode_pack", "sbvr_rope_attention_f16", "sbvr_linear_fused_f16", "sbvr_allreduce_add_rmsnorm_f16", "sbvr_linear_push_f16", "sbvr_ll_reduce_add_rmsnorm_f16", "sbvr_ll_reduce_add_rmsnorm_digits_f16", "sbvr_allreduce_add_rmsnorm_digits_f16", "sbvr_add_rmsnorm_f16", "sbvr_rope_append_f16", "sbvr_attention_f16", "sbvr_silu_mul_f16",
            "sbvr_embedding_f16", "sbvr_argmax_f16", "sbvr_linear_f16_noalloc", "sbvr_workspace_bytes", "sbvr_strerror", "sbvr_last_cuda_error", "sbvr_last_timeout_where", "sbvr_last_timeout_info", "sbvr_query", "sbvr_workspace_create",
            "sbvr_workspace_destroy", "sbvr_workspace_status", "sbvr_decode_f16", "sbvr_linear_f16",
            "sbvr_linear_f16_host"]
@@ -129,6 +129,22 @@ lib.sbvr_encode_stats_f16.argtypes = [_vp, _i, _vp, _vp]
 lib.sbvr_encode_stats_f16.restype = _i
 lib.sbvr_encode_advance.argtypes = [ctypes.POINTER(EncodeWalk), _vp]
 lib.sbvr_encode_advance.restype = _i
+
+
+class EncodeRecord(ctypes.Structure):
+    """sbvr_encode_record_t of include/sbvr_b200.h."""
+    _fields_ = [("group", _i), ("at", _i), ("mse", _f), ("line", ctypes.c_ushort * 4)]
+
+
+class EncodeRun(ctypes.Structure):
+    """sbvr_encode_run_t of include/sbvr_b200.h."""
+    _fields_ = [("ctl", _vp), ("records", _vp), ("outcome", _vp), ("n", _i), ("capacity", _i), ("warmup", _i), ("window", _i),
+                ("hist_n", _i), ("limit", _i), ("acceptable", ctypes.c_double), ("hist", ctypes.c_double * 64)]
+
+
+ENCODE_DONE, ENCODE_LIMIT, ENCODE_FULL, ENCODE_CALLER = 1, 2, 3, 4
+lib.sbvr_encode_run.argtypes = [ctypes.POINTER(EncodeWalk), ctypes.POINTER(EncodeRun), _vp]
+lib.sbvr_encode_run.restype = _i
 
 
 class PushDesc(ctypes.Structure):

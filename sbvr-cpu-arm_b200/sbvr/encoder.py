@@ -12,8 +12,9 @@ to every candidate coefficient line as tensors.  What it decides per group is ke
 
 How it is computed is different.  A step of the walk (`sbvr_encode_advance`) compares the line the last step added with
 every undecided group, finds the first group whose best stored line is not good enough, and generates and evaluates that
-group's own candidates in one kernel; the host decides from the winner alone.  Nothing of size candidates x 256 x 2^S is
-ever stored, and every group meets every line exactly once, so the result is that of the sequential walk.
+group's own candidates in one kernel; what becomes of the winner is decided from it alone, on the device for many steps in a row
+(`sbvr_encode_run`) and here for what that leaves over.  Nothing of size candidates x 256 x 2^S is ever stored, and every
+group meets every line exactly once, so the result is that of the sequential walk.
 
 The search space of a group is generated with the same tensor operations and the same fp16 roundings as the
 reference's; `space_device` says where: "cpu" runs the tensor operations on the CPU and reproduces a reference run there
@@ -230,11 +231,14 @@ class _Codebook:
                     return int(i), False
         if self.n >= len(self.lines):              # (a warm-up longer than the codebook)
             raise IndexError(f"the codebook has {len(self.lines)} lines")
+        self.mirror(line)
+        return self.n - 1, True
+
+    def mirror(self, line: np.ndarray) -> None:
         if self.n == len(self.host):
             self.host = np.concatenate((self.host, np.zeros_like(self.host)))
         self.host[self.n] = line
         self.n += 1
-        return self.n - 1, True
 
 
 def _full_search(group: torch.Tensor, conf: EncoderConfig, extended: bool) -> Tuple[float, np.ndarray]:
@@ -264,6 +268,46 @@ class _SearchTables:
         self.covered = conf.s_search_num >= 1 and conf.extend_ratio > 0 and all(
             len(u) >= 1 and len(b) >= 1 and 1 <= d <= 2000 and len(u) * len(b) * 1024 + (d + 1) ** S < 2.0e9
             for u, b, d in zip(self.unit, self.bias, self.per_dim))
+
+
+class _ManySteps:
+    """`sbvr_encode_run`: steps of the walk on the device until the host has to look at a group."""
+    LIMIT, WINDOW = 1024, 64
+
+    def __init__(self, conf: EncoderConfig, device):
+        self.conf = conf
+        self.ctl = torch.empty(8, dtype=torch.int64, device=device)
+        size = ctypes.sizeof(_lib.EncodeRecord)
+        self.pinned = torch.empty(32 + self.LIMIT * size, dtype=torch.uint8, pin_memory=True)
+        at = self.pinned.data_ptr()
+        self.outcome = (ctypes.c_int * 6).from_address(at)
+        self.records = np.frombuffer((ctypes.c_ubyte * (self.LIMIT * size)).from_address(at + 32), dtype=np.dtype(
+            {"names": ["group", "at", "mse", "line"], "formats": [np.int32, np.int32, np.float32, (np.uint16, 4)], "offsets": [0, 4, 8, 12],
+             "itemsize": size}))
+        self.args = _lib.EncodeRun(ctl=self.ctl.data_ptr(), records=at + 32, outcome=at, capacity=conf.max_cache_lines,
+                                   warmup=conf.cache_warmup_num, window=conf.mse_window_size, limit=self.LIMIT,
+                                   acceptable=conf.acceptable_mse)
+
+    def run(self, walk, book: "_Codebook", stream: int, own_groups: list, own_lines: list, own_index: list) -> int:
+        """Walks on from `walk.from_`; returns the first group that is not decided."""
+        a, S = self.args, self.conf.num_sums
+        tail = book.history[-self.conf.mse_window_size:]
+        a.n, a.hist_n = book.n, len(tail)
+        a.hist[:len(tail)] = tail
+        _lib.check(_lib.lib.sbvr_encode_run(ctypes.byref(walk), ctypes.byref(a), stream), "sbvr_encode_run")
+        why, gi, n, walk.line0, walk.misses, accepted = self.outcome
+        rec = self.records[:accepted].copy()
+        lines = rec["line"][:, :S].copy().view(np.float16)
+        own_groups += rec["group"].tolist()
+        own_lines += list(lines)
+        own_index += rec["at"].tolist()
+        for at, line in zip(rec["at"].tolist(), lines):
+            if at == book.n:
+                book.mirror(line)
+        assert book.n == n
+        for mse in rec["mse"].tolist():
+            book.accept(mse)
+        return walk.groups if why == _lib.ENCODE_DONE else gi
 
 
 def _sorted_line(bits, S: int, device) -> np.ndarray:
@@ -319,10 +363,21 @@ def encode(data: torch.Tensor, conf: EncoderConfig, device: Optional[torch.devic
                 walk.R[e], walk.B[e] = tables.unit[e].shape[0], tables.bias[e].shape[0]
                 walk.per_dim[e] = tables.per_dim[e]
         advance, walk_ref = _lib.lib.sbvr_encode_advance, ctypes.byref(walk)
+        # many steps per launch, unless the caller wants to hear of each; one step at a time for what that leaves to the host
+        many = _ManySteps(conf, dev) if kernel_search and progress is None and 1 <= conf.mse_window_size <= _ManySteps.WINDOW else None
         own_groups, own_lines, own_index = [], [], []      # groups that keep their own candidate, it, the line it is filed under
         gi = 0
         hits = None
         while gi < NG:
+            if many is not None and (book.n < conf.max_cache_lines or book.n < conf.cache_warmup_num):
+                if walk.append_at >= 0:
+                    book.lines[walk.append_at] = torch.from_numpy(book.host[walk.append_at]).to(dev)
+                    walk.append_at = -1
+                walk.from_, walk.search = gi, 1
+                gi = many.run(walk, book, st, own_groups, own_lines, own_index)
+                if gi >= NG:
+                    hits = NG - walk.misses
+                    break
             warm = book.n < conf.cache_warmup_num          # every group searches its own space
             full = book.n >= conf.max_cache_lines          # the best stored line has to do
             walk.from_, walk.line1, walk.warm = gi, book.n, int(warm)

@@ -182,3 +182,26 @@ def test_encode_then_linear_end_to_end():
         assert float((y - ref).abs().max() / ref.abs().max()) <= 1e-2
         dense = x.double() @ W.double().T
         assert float((y - dense).abs().max() / dense.abs().max()) < 0.2
+
+
+@pytest.mark.parametrize("S", [2, 3, 4])
+@pytest.mark.parametrize("settings", [{}, {"cache_warmup_num": 1}, {"cache_warmup_num": 40, "mse_window_size": 64}, {"mse_window_size": 1},
+                                      {"max_cache_lines": 23}, {"acceptable_mse": 1e-4}, {"mse_history": [1e-7, 3e-6], "cache_warmup_num": 0},
+                                      {"mse_window_size": 65}])
+def test_many_steps_in_one_launch_equal_one_at_a_time(S, settings):
+    """With a progress callback the walk takes one step per launch and decides on the host; without, on the device: codebook, indices,
+    bit-planes and counts are the same.  Among the groups: repeated ones (a winner that is stored already), zeros, a large mean
+    and too few distinct values (left to the host), more misses than one launch takes (1 024, S = 4)."""
+    from sbvr import encoder
+    g = torch.Generator(device="cuda").manual_seed(S)
+    rows = 300 if S == 4 and settings == {"mse_window_size": 1} else 24
+    W = torch.randn((rows, 1024), device="cuda", generator=g) * 0.02 * torch.exp(0.4 * torch.randn((rows, 1), device="cuda", generator=g))
+    W[5] = W[2]
+    W[7] = 0
+    W[9] += 0.5
+    W[11] = torch.sign(W[11]) * 0.01
+    W[13, :256] = W[13, 0]
+    one = encoder.encode(W.half(), encoder.EncoderConfig(num_sums=S, **settings), progress=lambda done, of: None)
+    many = encoder.encode(W.half(), encoder.EncoderConfig(num_sums=S, **settings))
+    assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(one[:3], many[:3]))
+    assert one[3] == many[3]
