@@ -44,8 +44,11 @@ __host__ __device__ constexpr int ts_mpad(int M) { return M <= 2 ? 2 : 4; }
 // possible for a single activation row and one group per block.
 __host__ __device__ constexpr int ts_dcols(int NSUB, int M, int KS) { return KS == 2 ? 16 : NSUB * 8 * ts_mpad(M); }
 __host__ __device__ constexpr int ts_wgcols(int NSUB, int M, int KS) { return 64 * KS + 2 * ts_dcols(NSUB, M, KS); }
+// Warpgroups of a CTA: what tensor memory holds, five at most; three for two activation rows, whose work does
+// not go well into the 64 registers that five leave a thread (us per call, M = 2, S = 4, five and three: 6144 x 4096 11.0 and 8.9, 14336 x 4096 15.8 and 12.9, 28672 x 4096 21.6 and
+// 19.9, 4096 x 4096 7.3 and 7.4).  One row in steps of one block wants all five: 8192 x 11008 15.5, with three 17.7.
 __host__ __device__ constexpr int ts_nwg(int NSUB, int M, int KS) {
-    return (TS_SF_COL / ts_wgcols(NSUB, M, KS)) > 5 ? 5 : (TS_SF_COL / ts_wgcols(NSUB, M, KS));
+    return M == 2 ? 3 : (TS_SF_COL / ts_wgcols(NSUB, M, KS)) > 5 ? 5 : (TS_SF_COL / ts_wgcols(NSUB, M, KS));
 }
 __host__ __device__ constexpr int ts_stage_bytes(int KS) { return KS * TS_STAGE_WORDS + 512; }   // + the step's coefficient data
 // Warp roles: warps 0 .. NWG-1 issue (MMAs and copies), warp NWG finishes, compute warps start at the next multiple of
