@@ -94,9 +94,11 @@ struct XqParams {
 // predecessor beside a resident CTA of the product (ts_plan leaves the room).  Blocks of sixteen warps found none and started when
 // a CTA of the kernel in front had ended; what stood behind them on that SM started later still, up to 6.7 us after
 // that kernel's end.  M = 4, us per call: 4096 x 4096 8.5 -> 8.1, 14336 x 4096 17.6 -> 14.7.
-constexpr int XQ_WARPS = 4;
-template <int NSUB>
-__global__ void __launch_bounds__(XQ_WARPS * 32, 16) xquant_kernel(const XqParams p) {
+// One row of more than 4096 keeps sixteen warps: its sum of squares takes the smaller blocks, each of which forms it, longer than the
+// room beside a CTA gains (70B preset, one sequence: 9.4 ms a step, 9.6 with four).
+__host__ __device__ constexpr int xq_warps(int M, int K) { return M == 1 && K > 4096 ? 16 : 4; }
+template <int NSUB, int XQ_WARPS>
+__global__ void __launch_bounds__(XQ_WARPS * 32, XQ_WARPS == 4 ? 16 : 1) xquant_kernel(const XqParams p) {
     __shared__ __align__(16) unsigned char area[XQ_WARPS][1024];
     __shared__ float ssum[XQ_WARPS];
     pdl_launch_dependents();
@@ -1010,9 +1012,10 @@ int launch_linear_tcs(const __half* x, const PackedW& w, const __half* bias, __h
     // SBVR_XOP_DIGITS: the digits are in the scratch already (written by the reduce kernel in front of this call)
     if (xp.x_op == SBVR_XOP_DIGITS && w.G != 256) return SBVR_ERR_UNSUPPORTED;
     if (!in_kernel && xp.x_op != SBVR_XOP_DIGITS) {
-        const dim3 qgrid((pl.KB + XQ_WARPS - 1) / XQ_WARPS, M);
-        if (w.G == 256) SBVR_CUDA_TRY(launch_pdl(xquant_kernel<1>, qgrid, dim3(XQ_WARPS * 32), 0, st, xp));
-        else SBVR_CUDA_TRY(launch_pdl(xquant_kernel<2>, qgrid, dim3(XQ_WARPS * 32), 0, st, xp));
+        const int qw = xq_warps(M, w.K);
+        const dim3 qgrid((pl.KB + qw - 1) / qw, M), qblock(qw * 32);
+        if (w.G == 256) SBVR_CUDA_TRY(qw == 4 ? launch_pdl(xquant_kernel<1, 4>, qgrid, qblock, 0, st, xp) : launch_pdl(xquant_kernel<1, 16>, qgrid, qblock, 0, st, xp));
+        else SBVR_CUDA_TRY(qw == 4 ? launch_pdl(xquant_kernel<2, 4>, qgrid, qblock, 0, st, xp) : launch_pdl(xquant_kernel<2, 16>, qgrid, qblock, 0, st, xp));
     }
     TsParams p;
     p.x = x, p.x_in_kernel = in_kernel ? 1 : 0;
