@@ -90,17 +90,19 @@ struct XqParams {
 // ---------------------------------------------------------------------------------------------
 // activations -> digits, once per call
 // ---------------------------------------------------------------------------------------------
-// Blocks of four warps, a 256-k block of one row each: small enough in registers and shared memory for two of them to wait for their
-// predecessor beside a resident CTA of the product (ts_plan leaves the room).  Blocks of sixteen warps found none and started when
+// Blocks of four warps, a 256-k block of one row each: small enough in registers and shared memory for one or two of them to wait for
+// their predecessor beside a resident CTA of the product (ts_plan leaves the room).  Blocks of sixteen warps found none and started when
 // a CTA of the kernel in front had ended; what stood behind them on that SM started later still, up to 6.7 us after
 // that kernel's end.  M = 4, us per call: 4096 x 4096 8.5 -> 8.1, 14336 x 4096 17.6 -> 14.7.
 // One row of more than 4096 keeps sixteen warps: its sum of squares takes the smaller blocks, each of which forms it, longer than the
 // room beside a CTA gains (70B preset, one sequence: 9.4 ms a step, 9.6 with four).
+// 48 registers: with 32 the loads of the sum of squares come one after the other (8B preset, 63 tokens of one user 123.6 against 120.8 ms).
 __host__ __device__ constexpr int xq_warps(int M, int K) { return M == 1 && K > 4096 ? 16 : 4; }
+constexpr int XQ_SUMS = 16;                       // partial sums of a row's squares, one per warp of the larger form
 template <int NSUB, int XQ_WARPS>
-__global__ void __launch_bounds__(XQ_WARPS * 32, XQ_WARPS == 4 ? 16 : 1) xquant_kernel(const XqParams p) {
+__global__ void __launch_bounds__(XQ_WARPS * 32, XQ_WARPS == 4 ? 10 : 1) xquant_kernel(const XqParams p) {
     __shared__ __align__(16) unsigned char area[XQ_WARPS][1024];
-    __shared__ float ssum[XQ_WARPS];
+    __shared__ float ssum[XQ_SUMS];
     pdl_launch_dependents();
     pdl_wait();                                    // the activations come from the previous kernel of the stream
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -109,31 +111,50 @@ __global__ void __launch_bounds__(XQ_WARPS * 32, XQ_WARPS == 4 ? 16 : 1) xquant_
     const int K = p.K;
     float rs = 0.0f;
     if (p.x_op == SBVR_XOP_ADD_RMSNORM) {
-        // mean of (h + delta)^2 over the whole row, the sum formed in fp16 like the separate kernel does
-        float sq = 0.0f;
-#pragma unroll 4
-        for (int c = threadIdx.x; c < K / 8; c += XQ_WARPS * 32) {
-            uint4 a = __ldg(reinterpret_cast<const uint4*>(p.x + (size_t)m * K) + c);
-            __half2* ah = reinterpret_cast<__half2*>(&a);
-            if (p.delta) {
-                const uint4 b = __ldg(reinterpret_cast<const uint4*>(p.delta + (size_t)m * K) + c);
-                const __half2* bh = reinterpret_cast<const __half2*>(&b);
+        // mean of (h + delta)^2 over the whole row, h + delta formed in fp16 like the separate kernel does.  The squares are added in one
+        // order whatever the block's size -- as 512 threads, a chunk of eight values each per round, and sixteen warps would --, so that
+        // a row's digits do not depend on which form makes them.
+        constexpr int V = XQ_SUMS / XQ_WARPS;      // of the sixteen warps' sums this warp makes
+        float sq[V];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) ah[e] = __hadd2(ah[e], bh[e]);
+        for (int v = 0; v < V; ++v) sq[v] = 0.0f;
+#pragma unroll 1
+        for (int c0 = threadIdx.x; c0 < K / 8; c0 += XQ_SUMS * 32) {
+            uint4 a[V], b[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const int c = c0 + v * (XQ_WARPS * 32);
+                const bool in = c < K / 8;         // (the same for a whole warp)
+                a[v] = in ? __ldg(reinterpret_cast<const uint4*>(p.x + (size_t)m * K) + c) : make_uint4(0u, 0u, 0u, 0u);
+                b[v] = in && p.delta ? __ldg(reinterpret_cast<const uint4*>(p.delta + (size_t)m * K) + c) : make_uint4(0u, 0u, 0u, 0u);
             }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float2 f = __half22float2(ah[e]);
-                sq += f.x * f.x + f.y * f.y;
+            for (int v = 0; v < V; ++v) {
+                __half2* ah = reinterpret_cast<__half2*>(&a[v]);
+                const __half2* bh = reinterpret_cast<const __half2*>(&b[v]);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float2 f = __half22float2(__hadd2(ah[e], bh[e]));
+                    sq[v] += f.x * f.x + f.y * f.y;
+                }
             }
         }
+        // lanes in halves: 16, 8, 4, 2, 1 apart; while a lane has several sums it keeps half of them and hands the other half over
+        if constexpr (V == 4) {
+            const bool hi = (lane & 16) != 0, odd = (lane & 8) != 0;
+            const float s0 = hi ? sq[0] : sq[2], s1 = hi ? sq[1] : sq[3];
+            sq[0] = (hi ? sq[2] : sq[0]) + __shfl_xor_sync(0xffffffffu, s0, 16);
+            sq[1] = (hi ? sq[3] : sq[1]) + __shfl_xor_sync(0xffffffffu, s1, 16);
+            const float s2 = odd ? sq[0] : sq[1];
+            sq[0] = (odd ? sq[1] : sq[0]) + __shfl_xor_sync(0xffffffffu, s2, 8);
+        }
 #pragma unroll
-        for (int o = 16; o; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (lane == 0) ssum[warp] = sq;
+        for (int o = V == 4 ? 4 : 16; o; o >>= 1) sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], o);
+        if ((lane & (V == 4 ? 7 : 31)) == 0) ssum[warp + (V == 4 ? (lane >> 4) * 2 + ((lane >> 3) & 1) : 0) * XQ_WARPS] = sq[0];
         __syncthreads();
         float tot = 0.0f;
 #pragma unroll
-        for (int w = 0; w < XQ_WARPS; ++w) tot += ssum[w];
+        for (int w = 0; w < XQ_SUMS; ++w) tot += ssum[w];
         rs = rsqrtf(tot / (float)K + p.eps);
     }
     if (kb >= p.KB) return;

@@ -476,3 +476,49 @@ def test_small_batch_kernel_merges_its_chunks(M, S, G, N, K, what):
     for _ in range(3):
         assert torch.equal(first, sbvr.linear(xd, w, None, algo=4))
     check_status()
+
+
+def _square_sums(h):
+    """Sum of squares of each fp16 row in the order of the decode quantiser: 512 threads take chunks of eight values in turn, two squares
+    per fp32 addition; then the lanes of a warp in halves, then sixteen warps one after the other."""
+    M, K = h.shape
+    d = h.double() ** 2
+    pairs = (d[:, 0::2] + d[:, 1::2]).float().view(M, K // 8, 4)           # (squares are exact in fp32: one rounding)
+    rounds = -(-K // 4096)
+    pairs = torch.nn.functional.pad(pairs, (0, 0, 0, rounds * 512 - K // 8)).view(M, rounds, 512, 4)
+    s = torch.zeros((M, 512), device=h.device)
+    for r in range(rounds):
+        for e in range(4):
+            s = s + pairs[:, r, :, e]
+    s = s.view(M, 16, 32)
+    for o in (16, 8, 4, 2, 1):
+        s = s + s[:, :, torch.arange(32, device=h.device) ^ o]
+    tot = torch.zeros(M, device=h.device)
+    for w in range(16):
+        tot = tot + s[:, w, 0]
+    return tot
+
+
+@pytest.mark.parametrize("M", [1, 2, 4])
+@pytest.mark.parametrize("K,G", [(256, 256), (2048, 128), (3840, 256), (4096, 256), (4352, 256), (8192, 256), (8192, 128), (10496, 256)])
+@pytest.mark.parametrize("with_delta", [False, True])
+def test_folded_norm_adds_squares_in_one_order(M, K, G, with_delta):
+    """The bits of a folded residual add + RMSNorm do not depend on the quantiser's form (rows, K): those of the norm computed apart,
+    squares in the stated order, in front of the plain linear."""
+    import sbvr
+    from sbvr.core import XOP_ADD_RMSNORM, linear_fused
+    N, eps = 256, 1e-5
+    w = to_sbvr(O.make_packed(N, K, 4, G=G, mode="u16", C=1000, seed=K + M))
+    for seed in range(4):
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        x = torch.randn((M, K), device="cuda", generator=g).half()
+        delta = torch.randn((M, K), device="cuda", generator=g).half() if with_delta else None
+        nw = (1 + 0.1 * torch.randn(K, device="cuda", generator=g)).half()
+        y, h_out = torch.empty((M, N), dtype=torch.float16, device="cuda"), torch.empty_like(x)
+        assert linear_fused(XOP_ADD_RMSNORM, x, w, y, delta=delta, norm_weight=nw, h_out=h_out, eps=eps)
+        h = x + delta if with_delta else x
+        assert torch.equal(h_out, h)
+        rs = torch.rsqrt(_square_sums(h) / torch.full((M,), float(K), device="cuda") + eps)      # (a division by a number would multiply by its inverse)
+        normed = (h.float() * rs[:, None]).half() * nw
+        assert torch.equal(y, sbvr.linear(normed, w, None, algo=2))
+    check_status()
