@@ -94,13 +94,17 @@ struct XqParams {
 // their predecessor beside a resident CTA of the product (ts_plan leaves the room).  Blocks of sixteen warps found none and started when
 // a CTA of the kernel in front had ended; what stood behind them on that SM started later still, up to 6.7 us after
 // that kernel's end.  M = 4, us per call: 4096 x 4096 8.5 -> 8.1, 14336 x 4096 17.6 -> 14.7.
-// One row of more than 4096 keeps sixteen warps: its sum of squares takes the smaller blocks, each of which forms it, longer than the
-// room beside a CTA gains (70B preset, one sequence: 9.4 ms a step, 9.6 with four).
 // 48 registers: with 32 the loads of the sum of squares come one after the other (8B preset, 63 tokens of one user 123.6 against 120.8 ms).
-__host__ __device__ constexpr int xq_warps(int M, int K) { return M == 1 && K > 4096 ? 16 : 4; }
+// A folded norm of one row of more than 4096 has sixteen warps: its sum of squares takes the smaller blocks, each of which forms it, longer
+// than an early start gains (70B preset, 16 layers, 63 tokens of one user 127.1 ms, 127.9 with four).  At 32 registers such a block fits
+// beside the product's 512 threads of 96.  Rows without a sum have no reason to wait: four warps (K = 14336 of the 8B layer,
+// one row: the layer's seven linears 57.7 -> 56.4 us; with the sum in four and the rest in sixteen the 63 tokens took 120.8 ms, now 115.0).
+__host__ __device__ constexpr int xq_warps(int x_op, int M, int K) {
+    return x_op == SBVR_XOP_ADD_RMSNORM && M == 1 && K > 4096 ? 16 : 4;
+}
 constexpr int XQ_SUMS = 16;                       // partial sums of a row's squares, one per warp of the larger form
 template <int NSUB, int XQ_WARPS>
-__global__ void __launch_bounds__(XQ_WARPS * 32, XQ_WARPS == 4 ? 10 : 1) xquant_kernel(const XqParams p) {
+__global__ void __launch_bounds__(XQ_WARPS * 32, XQ_WARPS == 4 ? 10 : 4) xquant_kernel(const XqParams p) {
     __shared__ __align__(16) unsigned char area[XQ_WARPS][1024];
     __shared__ float ssum[XQ_SUMS];
     pdl_launch_dependents();
@@ -1033,7 +1037,7 @@ int launch_linear_tcs(const __half* x, const PackedW& w, const __half* bias, __h
     // SBVR_XOP_DIGITS: the digits are in the scratch already (written by the reduce kernel in front of this call)
     if (xp.x_op == SBVR_XOP_DIGITS && w.G != 256) return SBVR_ERR_UNSUPPORTED;
     if (!in_kernel && xp.x_op != SBVR_XOP_DIGITS) {
-        const int qw = xq_warps(M, w.K);
+        const int qw = xq_warps(xp.x_op, M, w.K);
         const dim3 qgrid((pl.KB + qw - 1) / qw, M), qblock(qw * 32);
         if (w.G == 256) SBVR_CUDA_TRY(qw == 4 ? launch_pdl(xquant_kernel<1, 4>, qgrid, qblock, 0, st, xp) : launch_pdl(xquant_kernel<1, 16>, qgrid, qblock, 0, st, xp));
         else SBVR_CUDA_TRY(qw == 4 ? launch_pdl(xquant_kernel<2, 4>, qgrid, qblock, 0, st, xp) : launch_pdl(xquant_kernel<2, 16>, qgrid, qblock, 0, st, xp));
