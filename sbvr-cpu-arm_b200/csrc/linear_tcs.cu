@@ -899,7 +899,9 @@ bool linear_tcs_supported(const PackedW& w, int M) {
     if ((size_t)(w.N / ts_tn(w.S)) * (size_t)(w.K / 256) >= ((size_t)1 << 24)) return false;   // 32-bit step arithmetic (steps x CTAs)
     if ((size_t)w.N * w.S >= ((size_t)1 << 31)) return false;                    // 32-bit tensor coordinates
     // the activation digits of the whole K stay resident in shared memory: K/256 * M KB, beside two stages at least
-    const int NSUB = 256 / w.G, KB = w.K / 256, KS = ts_choose_ks(w, M), NWG = ts_nwg(NSUB, M, KS);
+    // (Two rows: as five warpgroups would need.  The room that three leave is not for longer rows: those go to kernels that hold activations
+    // to 2^-33 of a block's largest or as they are, where the digits here end at 2^-16.)
+    const int NSUB = 256 / w.G, KB = w.K / 256, KS = ts_choose_ks(w, M), NWG = M == 2 && NSUB == 1 ? 5 : ts_nwg(NSUB, M, KS);
     const int need = ts_round_up(ts_round_up(TS_HDR + 2 * NWG * M * 128 * 4, 128) + NWG * 2 * ts_stage_bytes(KS), 1024) + 2048 +
                      KB * M * 1024 + ts_round_up(M * KB * NSUB * 4, 16) + TS_BSLACK;
     return need <= 227 * 1024;

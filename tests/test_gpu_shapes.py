@@ -522,3 +522,40 @@ def test_folded_norm_adds_squares_in_one_order(M, K, G, with_delta):
         normed = (h.float() * rs[:, None]).half() * nw
         assert torch.equal(y, sbvr.linear(normed, w, None, algo=2))
     check_status()
+
+
+@pytest.mark.parametrize("K", [20736, 21248, 23808, 24064])
+@pytest.mark.parametrize("S,mode", [(2, "u8"), (4, "u16")])
+def test_two_long_rows_keep_their_precision(K, S, mode):
+    """From K = 21 248 on two rows are not the decode kernel's, whose digits end at 2^-16 of a block's largest value: outputs that do not
+    see one activation of 2^13 per block keep the precision of the rest (2^-11 of the result, and fp16 weights: 2e-3), a row with an
+    infinity has the infinities of a product, and the kernel asked for by name refuses.  Below, the decode kernel's own results."""
+    import sbvr
+    from sbvr import _lib
+    from sbvr.core import XOP_SILU_MUL, linear_fused
+    N = 64
+    p = O.make_packed(N, K, S, G=256, mode=mode, C=256 if mode == "u8" else 1000, seed=K + S)
+    k = np.arange(K // 256) * 256 + np.random.default_rng(K).integers(0, 256, K // 256)
+    p["bvr"][k // 32] &= ~(np.uint32(1) << (k % 32).astype(np.uint32))[:, None, None]
+    w = to_sbvr(p)
+    g = torch.Generator(device="cuda").manual_seed(S)
+    x = torch.randn((2, K), device="cuda", generator=g).half()
+    x[0, torch.from_numpy(k).cuda()] = 8192.0
+    x[1, K - 5] = float("inf")
+    gate = torch.full_like(x, 20.0)
+    act, y2 = torch.empty_like(x), torch.empty((2, N), dtype=torch.float16, device="cuda")
+    both = torch.cat([gate, (x / 20).half()], 1)
+    _lib.check(_lib.lib.sbvr_silu_mul_f16(both.data_ptr(), act.data_ptr(), 2, K, torch.cuda.current_stream().cuda_stream))
+    assert linear_fused(XOP_SILU_MUL, both, w, y2)
+    y = sbvr.linear(x, w)
+    if K == 20736:
+        assert torch.equal(y.view(torch.int16), sbvr.linear(x, w, None, algo=2).view(torch.int16))
+        return
+    for got, rows in ((y, x), (y2, act)):
+        ref = sbvr.linear(rows, w, None, algo=1)
+        assert ((got[0].float() - ref[0].float()).abs().max() / ref[0].float().abs().max()).item() < 2e-3
+        assert torch.equal(torch.isnan(got[1]), torch.isnan(ref[1])) and torch.isinf(ref[1]).any()
+        assert torch.equal(got[1][torch.isinf(ref[1])], ref[1][torch.isinf(ref[1])])
+    with pytest.raises(RuntimeError):
+        sbvr.linear(x, w, None, algo=2)
+    check_status()
