@@ -86,6 +86,11 @@ SBVR_API int sbvr_workspace_destroy(sbvr_workspace_t* ws);
 SBVR_API int sbvr_workspace_bytes(int device, int M, int N, int K, size_t* bytes);
 /* Synchronises `stream`, then reads the device status word: SBVR_OK or SBVR_ERR_TIMEOUT. Resets it. */
 SBVR_API int sbvr_workspace_status(sbvr_workspace_t* ws, sbvr_stream_t stream);
+/* How many SM cycles a CTA of the small-batch kernel waits for the others that hold parts of its sums before it leaves its share of the
+ * additions to the last of them (SBVR_PATIENCE_CYCLES, about 0.15 ms, in a new workspace: several times what they end apart on a GPU of
+ * their own; what they lose when another stream's kernel keeps one of them from starting).  Results do not depend on it. */
+#define SBVR_PATIENCE_CYCLES (1u << 18)
+SBVR_API int sbvr_workspace_patience(sbvr_workspace_t* ws, unsigned int cycles);
 
 /* Packed weight -> dense fp16 W[N rows, row pitch ldw elements]; columns 0 .. K_out-1 of every row are
  * written.  K is the padded length the packed tensors cover (multiple of G); K_out <= K is the original

@@ -206,6 +206,13 @@ int sbvr_workspace_destroy(sbvr_workspace_t* ws) {
     return SBVR_OK;
 }
 
+int sbvr_workspace_patience(sbvr_workspace_t* ws, unsigned int cycles) {
+    if (!ws) return SBVR_ERR_BAD_ARG;
+    WsLock lock(ws);
+    ws->patience = cycles;
+    return SBVR_OK;
+}
+
 int sbvr_workspace_status(sbvr_workspace_t* ws, sbvr_stream_t stream) {
     if (!ws) return SBVR_ERR_BAD_ARG;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -296,8 +303,8 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
     if (algo == 3) return launch_linear_gemm(xh, Kin, w, bh, yh, M, ws, st);
     if (algo == 4) {
         if (!ws) return SBVR_ERR_WORKSPACE;
-        return launch_linear_sb(xh, w, bh, yh, M, ws->device, ws->status, reinterpret_cast<unsigned int*>(ws->xchg), ws->dyn,
-                                ws->dyn_bytes, chosen, st);
+        return launch_linear_sb(xh, w, bh, yh, M, ws->device, ws->status, reinterpret_cast<float*>(ws->xchg),
+                                reinterpret_cast<unsigned long long*>(ws->counters), ws->patience, ws->dyn, ws->dyn_bytes, chosen, st);
     }
     return launch_linear_simt(xh, w, bh, yh, M, st);
 }
@@ -338,8 +345,8 @@ int sbvr_linear_fused_f16(int x_op, const void* x, const void* delta, const void
         if (x_op == SBVR_XOP_DIGITS || M > 16 || !linear_sb_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
         if (linear_sb_workspace_bytes(w, di) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
         return launch_linear_sb(reinterpret_cast<const __half*>(x), w, reinterpret_cast<const __half*>(bias),
-                                reinterpret_cast<__half*>(y), M, ws->device, ws->status, reinterpret_cast<unsigned int*>(ws->xchg),
-                                ws->dyn, ws->dyn_bytes, true, reinterpret_cast<cudaStream_t>(stream), &xop);
+                                reinterpret_cast<__half*>(y), M, ws->device, ws->status, reinterpret_cast<float*>(ws->xchg),
+                                reinterpret_cast<unsigned long long*>(ws->counters), ws->patience, ws->dyn, ws->dyn_bytes, true, reinterpret_cast<cudaStream_t>(stream), &xop);
     }
     if (linear_tcs_workspace_bytes(w, M, di.sm_count) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
     return launch_linear_tcs(reinterpret_cast<const __half*>(x), w, reinterpret_cast<const __half*>(bias),

@@ -63,6 +63,7 @@ struct sbvr_workspace {
     // Held by a call while it launches kernels that hand data to one another through the workspace: another thread's launches on
     // the same stream must not come between them.  NULL where the caller serialises (sbvr_linear_f16_noalloc).
     std::recursive_mutex* mu;
+    unsigned int patience = SBVR_PATIENCE_CYCLES;      // see sbvr_workspace_patience
 };
 #define SBVR_WS_COUNTERS 8192
 #define SBVR_WS_XCHG_BYTES (1u << 20)
@@ -154,14 +155,14 @@ int launch_linear_tcs(const __half* x, const PackedW& w, const __half* bias, __h
 // Validates an op in front of a linear and spreads it over the quantiser's parameters (api.cu).
 int xop_check(const XOp* xop, const __half* x, int M, int K, int* op, const __half** delta, const __half** norm_w, __half** h_out,
               float* eps);
-// The small-batch kernel (linear_sb.cu), 2 .. 16 activation rows: status words, the zeroed exchange region (arrival counters, left zero)
+// The small-batch kernel (linear_sb.cu), 2 .. 16 activation rows: status words, the zeroed exchange region and arrival words (left zero)
 // and 256-byte aligned scratch are the caller's.  A row with a non-finite activation is multiplied out or becomes NaN.
 bool linear_sb_supported(const PackedW& w, int M);
 bool linear_sb_preferred(const PackedW& w);      // ... to the GEMM, by speed
 size_t linear_sb_workspace_bytes(const PackedW& w, const DeviceInfo& di);
 int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, int device, unsigned int* status,
-                     unsigned int* counters, char* scratch, size_t scratch_bytes, bool multiply_out, cudaStream_t st,
-                     const XOp* xop = nullptr);
+                     float* xchg, unsigned long long* arrive, unsigned int patience, char* scratch, size_t scratch_bytes,
+                     bool multiply_out, cudaStream_t st, const XOp* xop = nullptr);
 bool linear_gemm_supported(const PackedW& w, int M);
 size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count);
 // x rows of Kin <= K elements (row pitch Kin), as if padded with zeros to K

@@ -31,15 +31,16 @@
 // released, and the multiply-adds run beside those.  (Two groups per k block take two D buffers and leave room for one A.)  A
 // warp holds all sums of a quarter of a tile's rows.  A tile that several warpgroups share is put together in shared memory at the
 // end.  The chunks' sums meet in scratch when the CTAs of a group (the chunks of the same tiles) are through: each adds an equal
-// share of them in chunk order (the same bits on every run).  Added by whichever warp arrived last at a tile's counter, as
+// share of them in chunk order (the same bits on every run), or leaves it to the last of them.  Added by whichever warp arrived last at a tile's counter, as
 // before, the slow CTAs of a group got nearly all of that work on top: at 28672 x 8192 they ended 27 us behind the mean of 70.
 // Every wait is bounded.
 //
 // What bounds it: the tensor pipe in the loop (a unit takes 485 cycles of its SM at 14336 x 4096, its 24 MMAs 391 of a pipe that
 // does nothing else); around it, per launch, 4.7 us from the end of the kernel in front to the digits in shared memory (of it 1 to 1.7
-// in the quantiser) and 2 to 3 us for the merge.  Per call with the quantiser, M = 16, S = 4, us (before; the fp16 GEMM):
-// 1024 x 4096 9.4 (11.0; 10.4), 4096 x 4096 10.9 (12.7; 14.8), 14336 x 4096 21.7 (27.8; 32.1), 4096 x 14336 26.6 (39.7; 31.6),
-// 28672 x 8192 60 (104; 112); groups of 128, 14336 x 4096: 24.2 (30.0; 31.9).
+// in the quantiser) and 2 to 3 us for the merge.  That the merge does not count on its CTAs running together costs 0.4 us where the sums
+// are few (a fence and an atomic beside the sums), nothing elsewhere.  Per call with the quantiser, M = 16, S = 4, us (with sums added by
+// the last warp to arrive; the fp16 GEMM): 1024 x 4096 9.8 (11.0; 10.4), 4096 x 4096 11.4 (12.7; 14.8), 14336 x 4096 22.3 (27.8; 32.1),
+// 4096 x 14336 26.9 (39.7; 31.6), 28672 x 8192 60 (104; 112); groups of 128, 14336 x 4096: 24.6 (30.0; 31.9).
 //
 // Replaces the M > 1 use of `_sbvr_row_deq_mm_T` (reference sbvr/kernels/sbvr_kernel.cu:121-191) for 2 .. 16 rows.
 #include <cuda.h>
@@ -76,7 +77,8 @@ struct SbParams {
     const __half* bias;
     __half* y;
     unsigned int* status;
-    unsigned int* counters;       // one per group of CTAs that work on the same tiles, zero between launches
+    unsigned long long* arrive;   // a word per group of CTAs that work on the same tiles, zero between launches (see "the chunks of K meet")
+    unsigned int patience;        // SM cycles a CTA waits for its siblings before it hands its share of the sums over
     float* part;                  // [KC][NT][SB_MP][TN] sums of the chunks (KC > 1)
     int M, N, K, KB, NT, C, KC, GN, cache_in_smem, stages, idx_bytes;
     int tagged;                   // `part` lies in the exchange region, all zero between launches, and a sum's arrival is its own mark
@@ -253,8 +255,9 @@ struct SbPair {
 };
 
 // y[m, n] of an activation row that holds something non-finite, as products give it: the digits cannot say it and have left a NaN.
-// Inlined where few values are live (88 registers, 80 without it): as a function that is called it took the kernel to 94, which leaves
-// no room beside a CTA for the blocks of the GEMM's re-tiling (seven linears of a layer, 16 rows: 154 against 146 us).
+// Inlined where few values are live (76 to 79 registers with groups of 256, the limit of 88 with groups of 128): as a function that is
+// called it took the kernel beyond 88, which leaves no room beside a CTA for the blocks of the next call (seven linears of a
+// layer, 16 rows, with the GEMM among them: 154 against 146 us).
 template <int S>
 __device__ __forceinline__ void sb_multiply_out(const SbParams& p, int G, int m, int n) {
     float acc = 0.0f;
@@ -274,26 +277,30 @@ __device__ __forceinline__ void sb_multiply_out(const SbParams& p, int G, int m,
 // A chunk's sum on its way to the CTA that adds it: never the bit pattern zero, which stands for "not there yet" (p.tagged).
 __device__ __forceinline__ void sb_put(float* dst, float v) { __stcg(dst, v == 0.0f ? -0.0f : v); }
 
-// The chunks' sums of the group's tiles [t0, t0 + ntc) -> y, in chunk order.  The KC CTAs of the group take equal shares of the
-// (tile, activation row, four output rows) list, whoever of them was slow; four chunks' loads are in flight per thread.
+// Share `share` of the chunks' sums of the group's tiles [t0, t0 + ntc) -> y, in chunk order.  The KC shares are equal parts of the (tile,
+// activation row, four output rows) list; four chunks' loads are in flight per thread.  Slots that mark themselves (p.tagged): a thread
+// waits for the sums it needs, p.patience cycles at most, and clears their slots once it has all of them; what does not come is
+// left as it is, and false returned.  `all_here`: every sum has been stored, so slots that are empty belong to what is done.
 template <int S, int NSUB>
-__device__ __forceinline__ void sb_add_chunks(const SbParams& p, int t0, int ntc, int chunk, volatile int* abort_flag) {
+__device__ __forceinline__ bool sb_add_share(const SbParams& p, int t0, int ntc, int share, bool all_here) {
     constexpr int TN = ts_tn(S), Q = TN / 4;
-    const int total = ntc * p.M * Q;               // (below 2^31: the host bounds the tiles)
-    const int e1 = (int)((long long)total * (chunk + 1) / p.KC);
+    const int total = ntc * p.M * Q;               // (at most 65 536 x 16 x 8: sb_plan)
+    const int e1 = (int)((long long)total * (share + 1) / p.KC);
     const size_t plane = (size_t)p.NT * (SB_MP * TN);
     const bool wide = (reinterpret_cast<uintptr_t>(p.y) & 7) == 0;
+    bool done = true;
 #pragma unroll 1
-    for (int e = (int)((long long)total * chunk / p.KC) + (int)threadIdx.x; e < e1; e += SB_THREADS) {
+    for (int e = (int)((long long)total * share / p.KC) + (int)threadIdx.x; e < e1; e += SB_THREADS) {
         const int q = e % Q, m = e / Q % p.M, tile = t0 + e / (Q * p.M);
         float* src = p.part + ((size_t)tile * SB_MP + m) * TN + q * 4;
         float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        bool here = true;
 #pragma unroll 1
         for (int c = 0; c < p.KC; c += 4) {
             float4 t[4];
             const long long c0 = clock64();
             for (;;) {
-                bool all = true;
+                here = true;
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
                     t[h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -307,21 +314,20 @@ __device__ __forceinline__ void sb_add_chunks(const SbParams& p, int t0, int ntc
 #pragma unroll
                 for (int h = 0; h < 4; ++h)
                     if (c + h < p.KC)
-                        all = all && __float_as_uint(t[h].x) && __float_as_uint(t[h].y) && __float_as_uint(t[h].z) && __float_as_uint(t[h].w);
-                if (all || *abort_flag) break;
-                if (clock64() - c0 > 2000000000LL) {                          // a chunk never came
-                    *abort_flag = 1;
-                    atomicExch(p.status, 1u);
-                    atomicExch(p.status + 1, 0x441u);
-                    break;
-                }
+                        here = here && __float_as_uint(t[h].x) && __float_as_uint(t[h].y) && __float_as_uint(t[h].z) && __float_as_uint(t[h].w);
+                if (here || all_here || !done || clock64() - c0 > (long long)p.patience) break;
             }
+            if (!here) break;
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                v[0] += t[h].x, v[1] += t[h].y, v[2] += t[h].z, v[3] += t[h].w;
-                if (p.tagged && c + h < p.KC)
-                    __stcg(reinterpret_cast<float4*>(src + (size_t)(c + h) * plane), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-            }
+            for (int h = 0; h < 4; ++h) v[0] += t[h].x, v[1] += t[h].y, v[2] += t[h].z, v[3] += t[h].w;
+        }
+        if (!here) {
+            done = false;
+            continue;
+        }
+        if (p.tagged) {
+#pragma unroll 1
+            for (int c = 0; c < p.KC; ++c) __stcg(reinterpret_cast<float4*>(src + (size_t)c * plane), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
         }
         const int n = tile * TN + q * 4;
         __half* dst = p.y + (size_t)m * p.N + n;
@@ -340,6 +346,30 @@ __device__ __forceinline__ void sb_add_chunks(const SbParams& p, int t0, int ntc
                 if (v[i] != v[i]) sb_multiply_out<S>(p, 256 / NSUB, m, n + i);
         }
     }
+    return done;
+}
+
+__device__ __forceinline__ unsigned long long sb_load_acquire(const unsigned long long* a) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(a) : "memory");
+    return v;
+}
+
+// The upper half of a group's word counts arrivals in parts of 2^32: with the last of them it is zero again.
+__device__ __forceinline__ unsigned int sb_part_of_group(int chunk, int KC) {
+    const unsigned int q = 0xffffffffu / (unsigned int)KC;
+    return chunk ? q : 0u - q * (unsigned int)(KC - 1);
+}
+
+// A CTA that has given up waiting: true if the others have all arrived in the meantime, else its share is the last one's.
+__device__ __forceinline__ bool sb_hand_over(unsigned long long* word, int chunk) {
+    unsigned long long v = sb_load_acquire(word);
+    while (v >> 32) {
+        const unsigned long long old = atomicCAS(word, v, v | (1ull << chunk));
+        if (old == v) return false;
+        v = old;
+    }
+    return true;
 }
 
 // (88 registers: beside a CTA there is room for two blocks of the next call's quantiser, which 16 rows of 4096 need to be resident at
@@ -726,31 +756,47 @@ __global__ void __maxnreg__(88) linear_sb_kernel(const __grid_constant__ CUtenso
         }
     }
     // ------------------------------ the chunks of K meet ------------------------------
-    // (The group's CTAs are all resident: there are at most as many as SMs.)  Few sums: their slots are zero before the launch, whoever
-    // needs one waits until it is not, and clears it.  Many: the CTAs arrive at a counter that wraps to zero with the last of them,
-    // and wait for that zero, which the counter had before the first came; a fence, an atomic and a poll take 1.5 us longer.
+    // The CTAs of a group add equal shares of its sums, but nothing depends on their running at the same time: other streams' kernels may
+    // hold the SMs that some of them need.  A CTA that is through counts itself in the upper half of the group's word, which is zero
+    // again when all have: every sum is there then.  One that has stopped waiting for that leaves its bit in the lower half, unless the upper
+    // half is zero by now, and ends; the last one finds the bits in the value that its count met, and takes those shares over.  Few
+    // sums: their slots are zero before the launch, whoever needs one takes it as soon as it is not, and clears it; the word then
+    // only says who is last (waiting for it before the sums are read takes 1.5 us longer).
     if (KC > 1) {
-        if (!p.tagged) {
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                __threadfence();
-                unsigned int left = atomicInc(p.counters + grp, (unsigned int)(KC - 1)) + 1u;
-                if (left == (unsigned int)KC) left = 0u;
-                const long long c0 = clock64();
-                while (left) {
-                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(left) : "l"(p.counters + grp) : "memory");
-                    if (*abort_flag || clock64() - c0 > 2000000000LL) break;
-                }
-                if (left && !*abort_flag) {
-                    *abort_flag = 1;
-                    atomicExch(p.status, 1u);
-                    atomicExch(p.status + 1, 0x440u);
-                }
-                __threadfence();
-            }
-            __syncthreads();
+        volatile unsigned int* share_s = reinterpret_cast<volatile unsigned int*>(smem + SB_HDR - 32);
+        unsigned long long* word = p.arrive + grp;
+        const bool speaker = threadIdx.x == SB_THREADS - 32;          // (of a warp that has few sums to add or none)
+        const unsigned int part = sb_part_of_group(chunk, KC);
+        unsigned long long before = 0ull;
+        if (warp == SB_THREADS / 32 - 1) named_bar_sync(14, SB_THREADS);        // every warp's sums are stored
+        else ts_bar_arrive(14, SB_THREADS);
+        if (speaker) {
+            __threadfence();
+            before = atomicAdd(word, (unsigned long long)part << 32);
         }
-        sb_add_chunks<S, NSUB>(p, t0, ntc, chunk, abort_flag);
+        bool done = false;
+        if (p.tagged) done = __syncthreads_and(sb_add_share<S, NSUB>(p, t0, ntc, chunk, false));
+        if (speaker) {
+            const unsigned int mine = done ? 0u : 1u << chunk;
+            unsigned int shares = 0u;
+            if ((unsigned int)(before >> 32) + part == 0u) {          // the last one; nobody sets a bit from here on
+                shares = (unsigned int)before | mine;
+                if ((unsigned int)before) atomicExch(word, 0ull);
+            } else if (!done) {
+                const long long c0 = clock64();
+                bool all = false;
+                while (!p.tagged && !(all = (sb_load_acquire(word) >> 32) == 0ull) && clock64() - c0 <= (long long)p.patience) {
+                }
+                if (!all) __threadfence();         // (slots cleared here come before the bit that leaves the rest to another)
+                if (all || sb_hand_over(word, chunk)) shares = mine;
+            }
+            if (shares) __threadfence();
+            *share_s = shares;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (unsigned int shares = *share_s; shares; shares &= shares - 1)
+            sb_add_share<S, NSUB>(p, t0, ntc, __ffs((int)shares) - 1, true);
     }
     if (threadIdx.x == 0 && *abort_flag) {         // which problem gave up: N, and K / 256 | M | CTA (for the host's message)
         atomicExch(p.status + 2, (unsigned int)p.N);
@@ -781,7 +827,8 @@ static int sb_plan(const PackedW& w, const DeviceInfo& di, SbPlan* pl) {
         pl->KC *= 2;
     pl->GN = groups(pl->KC);
     const int nkb = (pl->KB + pl->KC - 1) / pl->KC;
-    if (pl->KC > 1 && (size_t)pl->NT * 16 > SBVR_WS_XCHG_BYTES) return SBVR_ERR_UNSUPPORTED;     // arrival counters
+    if (pl->KC > 1 && pl->NT > 65536) return SBVR_ERR_UNSUPPORTED;       // (what has been covered: two million rows)
+    if (pl->KC > 32) return SBVR_ERR_UNSUPPORTED;                        // bits of a group's word
     pl->blob_bytes = ((size_t)pl->KB * SB_BLOB + 255) / 256 * 256;
     pl->part_bytes = pl->KC > 1 ? (size_t)pl->KC * pl->NT * MP * TN * 4 : 0;
     const int cache_bytes = w.idx_bytes ? ts_round_up(w.C * w.S * 2, 16) : 0;
@@ -869,13 +916,13 @@ static int sb_launch_g(const CUtensorMap& tm, const SbParams& p, int G, int idxb
     return G == 128 ? sb_launch_idx<S, 2>(tm, p, idxb, grid, smem, st) : sb_launch_idx<S, 1>(tm, p, idxb, grid, smem, st);
 }
 
-// `counters` (SBVR_WS_XCHG_BYTES, zero between calls: the kernel leaves them zero) and `scratch` (256-byte aligned,
-// linear_sb_workspace_bytes long: digit blob, the chunks' sums, rows an op has made) are the caller's.
+// `xchg` (SBVR_WS_XCHG_BYTES), `arrive` (8 bytes per SM) -- both zero between calls: the kernel leaves them zero -- and `scratch`
+// (256-byte aligned, linear_sb_workspace_bytes long: digit blob, the chunks' sums, rows an op has made) are the caller's.
 int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, int device, unsigned int* status,
-                     unsigned int* counters, char* scratch, size_t scratch_bytes, bool multiply_out, cudaStream_t st,
-                     const XOp* xop) {
+                     float* xchg, unsigned long long* arrive, unsigned int patience, char* scratch, size_t scratch_bytes,
+                     bool multiply_out, cudaStream_t st, const XOp* xop) {
     if (!linear_sb_supported(w, M)) return SBVR_ERR_UNSUPPORTED;
-    if (!status || !counters || !scratch) return SBVR_ERR_WORKSPACE;
+    if (!status || !xchg || !arrive || !scratch) return SBVR_ERR_WORKSPACE;
     if (reinterpret_cast<uintptr_t>(x) & 1) return SBVR_ERR_ALIGN;
     if (reinterpret_cast<uintptr_t>(scratch) & 255) return SBVR_ERR_ALIGN;
     DeviceInfo di;
@@ -898,9 +945,9 @@ int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __ha
     SBVR_CUDA_TRY(launch_pdl(sb_quant_kernel, dim3(pl.KB, SB_MP), dim3(128), 0, st, q));
     SbParams p;
     p.xb = q.xb;
-    p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status, p.counters = counters;
+    p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status, p.arrive = arrive, p.patience = patience;
     p.tagged = pl.KC > 1 && pl.part_bytes <= SBVR_WS_XCHG_BYTES;
-    p.part = p.tagged ? reinterpret_cast<float*>(counters) : reinterpret_cast<float*>(scratch + pl.blob_bytes);
+    p.part = p.tagged ? xchg : reinterpret_cast<float*>(scratch + pl.blob_bytes);
     p.x = !multiply_out ? nullptr : q.x_out ? q.x_out : x, p.bvr = w.bvr, p.idx_bytes = w.idx_bytes;
     p.M = M, p.N = w.N, p.K = w.K, p.KB = pl.KB, p.NT = pl.NT, p.C = w.C, p.KC = pl.KC, p.GN = pl.GN;
     p.cache_in_smem = pl.cache_in_smem, p.stages = pl.stages;

@@ -52,6 +52,8 @@ lib.sbvr_workspace_destroy.argtypes = [_vp]
 lib.sbvr_workspace_destroy.restype = _i
 lib.sbvr_workspace_status.argtypes = [_vp, _vp]
 lib.sbvr_workspace_status.restype = _i
+lib.sbvr_workspace_patience.argtypes = [_vp, ctypes.c_uint]
+lib.sbvr_workspace_patience.restype = _i
 lib.sbvr_decode_f16.argtypes = [_vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp]
 lib.sbvr_decode_f16.restype = _i
 lib.sbvr_linear_f16.argtypes = [_vp, _vp, _vp, _i, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _vp, _vp]
@@ -107,7 +109,7 @@ lib.sbvr_allreduce_add_rmsnorm_digits_f16.restype = _i
 
 EXPORTS = ["sbvr_linear_workspace_bytes", "sbvr_linear_padded_f16", "sbvr_encode_stats_f16", "sbvr_encode_advance", "sbvr_encode_run", "sbvr_popc_mm_f16", "sbvr_linear_t_f16", "sbvr_encode_mse_f16", "sbvr_encode_select_f16", "sbvr_encode_pack", "sbvr_rope_attention_f16", "sbvr_linear_fused_f16", "sbvr_allreduce_add_rmsnorm_f16", "sbvr_linear_push_f16", "sbvr_ll_reduce_add_rmsnorm_f16", "sbvr_ll_reduce_add_rmsnorm_digits_f16", "sbvr_allreduce_add_rmsnorm_digits_f16", "sbvr_add_rmsnorm_f16", "sbvr_rope_append_f16", "sbvr_attention_f16", "sbvr_silu_mul_f16",
            "sbvr_embedding_f16", "sbvr_argmax_f16", "sbvr_linear_f16_noalloc", "sbvr_workspace_bytes", "sbvr_strerror", "sbvr_last_cuda_error", "sbvr_last_timeout_where", "sbvr_last_timeout_info", "sbvr_query", "sbvr_workspace_create",
-           "sbvr_workspace_destroy", "sbvr_workspace_status", "sbvr_decode_f16", "sbvr_linear_f16",
+           "sbvr_workspace_destroy", "sbvr_workspace_status", "sbvr_workspace_patience", "sbvr_decode_f16", "sbvr_linear_f16",
            "sbvr_linear_f16_host"]
 
 

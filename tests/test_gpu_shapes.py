@@ -559,3 +559,47 @@ def test_two_long_rows_keep_their_precision(K, S, mode):
     with pytest.raises(RuntimeError):
         sbvr.linear(x, w, None, algo=2)
     check_status()
+
+
+@pytest.mark.parametrize("M", [5, 16])
+@pytest.mark.parametrize("S,G,N,K", [(4, 256, 4096, 4096), (4, 256, 4128, 4096), (2, 256, 64, 8192), (3, 128, 96, 1280), (4, 256, 64, 32768), (4, 256, 512, 14336)])
+@pytest.mark.parametrize("patience", [0, 2000])
+def test_small_batch_chunks_that_do_not_wait(M, S, G, N, K, patience):
+    """CTAs that give up at once, or soon, leave their share of the sums to the last of them: the same bits, slots and words empty again."""
+    import sbvr
+    from sbvr import _lib
+    w = to_sbvr(O.make_packed(N, K, S, G=G, mode="u16", C=1000, seed=N + K))
+    x = torch.from_numpy(np.random.default_rng(M).standard_normal((M, K)).astype(np.float16)).cuda()
+    x[M - 1, K // 3] = float("nan")
+    first = sbvr.linear(x, w, None, algo=4)
+    ws = _lib.workspace(torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream)
+    assert _lib.lib.sbvr_workspace_patience(ws.handle, patience) == 0
+    try:
+        for _ in range(20):
+            assert torch.equal(first[:-1], sbvr.linear(x, w, None, algo=4)[:-1])
+    finally:
+        _lib.lib.sbvr_workspace_patience(ws.handle, 1 << 18)
+    assert torch.isnan(first[-1]).all() and torch.equal(first[:-1], sbvr.linear(x, w, None, algo=4)[:-1])
+    check_status()
+
+
+def test_small_batch_kernel_on_two_streams_at_once():
+    """Two streams whose grids each want every SM: calls of both interleave freely, results are those of a call by itself."""
+    import sbvr
+    shapes = [(4096, 4096), (2048, 16384), (4128, 4096), (64, 32768)]
+    ws = [to_sbvr(O.make_packed(N, K, 4, G=256, mode="u16", C=1000, seed=N + K)) for N, K in shapes]
+    xs = [torch.from_numpy(np.random.default_rng(K).standard_normal((16, K)).astype(np.float16)).cuda() for _, K in shapes]
+    want = [sbvr.linear(x, w, None, algo=4) for x, w in zip(xs, ws)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1)]
+    got = []
+    for i in range(60):
+        for k, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                j = (i + k) % len(shapes)
+                got.append((j, sbvr.linear(xs[j], ws[j], None, algo=4)))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, want[j]) for j, y in got)
+    for s in streams:
+        with torch.cuda.stream(s):
+            check_status()

@@ -3,10 +3,11 @@
 Inside a CTA a warpgroup works on its own: an issuer (ring of weight stages, MMAs and their commits) and four compute warps (words
 of unit i + 1 into tensor memory and of unit i + 2 out of shared memory beside the MMAs of unit i; its sums read before the
 MMAs of unit i + 1 are released through a named barrier).  mbarriers are waited on by PARITY, as on the device, so a waiter that
-fell two phases behind would be caught as aliasing.  Between CTAs the K chunks' sums meet when a group's CTAs are through: at a counter
-that wraps to zero, or in slots whose value is its own mark (`group`; `chunks` is the protocol before that: stored, counted a
-unit later and looked at another unit later).  The tests check: no deadlock, no aliasing, no stage, operand or sum that is overwritten
-before all of its readers are done, exactly one warp that adds a quarter and all chunks' stores before it; and that the same
+fell two phases behind would be caught as aliasing.  Between CTAs (`group`) the K chunks' sums meet when a group's CTAs are through, by a
+word in which each counts itself and, where the sums are few, in slots whose value is its own mark; a CTA that runs out of patience
+leaves its share to the last one, so that none depends on another's running at the same time.  The tests check: no deadlock, no
+aliasing, no stage, operand or sum that is overwritten before all of its readers are done, every sum added exactly once and after all
+chunks' stores, slots and word empty after a launch, whatever the number of CTAs that run at a time; and that the same
 checks do flag protocols with a step out of place.
 """
 import random
@@ -139,60 +140,6 @@ def warpgroup(n, ST, abuf, seed, mistake=None):
     return errors
 
 
-def chunks(KC, tiles, seed, mistake=None):
-    """KC CTAs, a warp each, over `tiles` whole tiles of one quarter: stored, counted a step later, looked at another step later."""
-    rnd = random.Random(seed)
-    stored = [set() for _ in range(tiles)]
-    counter, added, errors = [0] * tiles, [0] * tiles, []
-
-    def warp(chunk):
-        pend, tile, old = 0, None, 0
-
-        def settle():
-            nonlocal pend, old
-            if pend == 1:
-                old = counter[tile]
-                counter[tile] += 1
-                pend = 2
-            elif pend == 2:
-                pend = 0
-                if old == KC - 1:
-                    if len(stored[tile]) < KC:
-                        errors.append(("added before all chunks are stored", tile))
-                    counter[tile] = 0
-                    added[tile] += 1
-        for t in range(tiles):
-            for _ in range(rnd.choice([1, 1, 2, 4])):              # units of the tile
-                yield
-                if pend:
-                    settle()
-            while pend:
-                settle()
-                yield
-            if mistake == "count first":
-                pend, tile = 1, t
-                settle()
-                yield
-                stored[t].add(chunk)
-            else:
-                stored[t].add(chunk)
-                pend, tile = 1, t
-        while pend:
-            yield
-            settle()
-
-    agents = [warp(c) for c in range(KC)]
-    while agents:
-        a = rnd.choice(agents)
-        try:
-            next(a)
-        except StopIteration:
-            agents.remove(a)
-    if not errors and (added != [1] * tiles or counter != [0] * tiles):
-        errors.append(("adders, counters", added, counter))
-    return errors
-
-
 @pytest.mark.parametrize("abuf", [1, 2])
 def test_warpgroup_has_no_deadlock_aliasing_or_early_reuse(abuf):
     for trial in range(150):
@@ -206,52 +153,82 @@ def test_model_flags_a_step_out_of_place(abuf, mistake):
     assert any(warpgroup(12, 2, abuf, trial, mistake) for trial in range(40))
 
 
-def test_chunks_are_added_once_and_after_all_stores():
-    for trial in range(300):
-        rnd = random.Random(trial)
-        assert chunks(rnd.randint(2, 16), rnd.randint(1, 6), trial) == []
-
-
-def test_model_flags_a_count_in_front_of_the_store():
-    assert any(chunks(4, 3, trial, "count first") for trial in range(40))
-
-
-def group(KC, launches, tagged, seed, mistake=None):
-    """KC CTAs of a group, launch after launch: sums stored, then all of them waited for and each CTA's share read (and cleared)."""
+def group(KC, launches, tagged, seed, resident=None, late=0.0, mistake=None):
+    """KC CTAs of a group, launch after launch: a CTA stores its sums, counts itself in the group's word, and adds its share of every chunk's
+    sums -- or, out of patience (with probability `late` per look), leaves what is not there yet to the last CTA.  At most `resident`
+    of them run at a time; the next one starts when one has ended."""
     rnd = random.Random(seed)
-    slots = [[None] * KC for _ in range(KC)]       # [share][chunk]: launch whose sum it holds, None: empty
-    counter, errors = 0, []
+    E = 2                                          # elements of a share
+    slots = [[[None] * KC for _ in range(E)] for _ in range(KC)]          # [share][element][chunk]: launch whose sum it holds
+    added = []                                     # (launch, share, element)
+    errors = []
+    word = {"count": 0, "mask": 0}
 
-    def cta(chunk, launch):
-        nonlocal counter
-        if mistake == "count first":
-            counter = (counter + 1) % KC
-        for share in rnd.sample(range(KC), KC):
-            yield
-            if tagged and slots[share][chunk] is not None:
-                errors.append("slot still full")
-            slots[share][chunk] = launch
-        if not tagged:
-            yield
-            if mistake != "count first":
-                counter = (counter + 1) % KC
-            while counter:
-                yield
-        else:
-            while mistake != "no wait" and None in slots[chunk]:
-                yield
-        if slots[chunk] != [launch] * KC:
-            errors.append("share read before all chunks are stored")
+    def element(share, e, launch):                 # all sums have been seen: cleared one after the other
+        if slots[share][e] != [launch] * KC:
+            errors.append(("added before all chunks are stored", share, e))
+        added.append((launch, share, e))
         if tagged:
             for c in range(KC):
+                slots[share][e][c] = None
                 yield
-                slots[chunk][c] = None
+
+    def share_of(share, launch, all_here):
+        done = True
+        for e in range(E):
+            while tagged and None in slots[share][e]:
+                if all_here or not done or rnd.random() < late:
+                    break
+                yield
+            if tagged and None in slots[share][e]:
+                done = False
+                if all_here and mistake == "adds again":
+                    added.append((launch, share, e))
+                continue
+            yield from element(share, e, launch)
+        return done
+
+    def cta(chunk, launch):
+        for share in rnd.sample(range(KC), KC):
+            for e in range(E):
+                yield
+                if tagged and slots[share][e][chunk] is not None:
+                    errors.append("slot still full")
+                if mistake != "count first":
+                    slots[share][e][chunk] = launch
+        before = dict(word)                        # (one atomic addition; the count is zero again with the last of them)
+        word["count"] = (word["count"] + 1) % KC
         yield
+        if mistake == "count first":
+            for share in range(KC):
+                for e in range(E):
+                    yield
+                    slots[share][e][chunk] = launch
+        done = False
+        if tagged:
+            done = yield from share_of(chunk, launch, False)
+        mine, shares = set() if done else {chunk}, set()
+        if before["count"] == KC - 1:
+            shares = mine | {c for c in range(KC) if before["mask"] >> c & 1}
+            if mistake != "no reset":
+                word["mask"] = 0
+        elif not done:
+            while not tagged and word["count"] and rnd.random() >= late:
+                yield
+            yield
+            if word["count"] == 0 and mistake != "always leaves":          # (a compare-and-swap that finds zero: all are there)
+                shares = mine
+            else:
+                word["mask"] |= 1 << chunk
+        for share in sorted(shares):
+            yield from share_of(share, launch, True)
 
     for launch in range(launches):                 # (a launch begins when the one before has ended)
-        agents = [cta(c, launch) for c in range(KC)]
-        steps = 0
-        while agents and not errors:
+        waiting = [cta(c, launch) for c in rnd.sample(range(KC), KC)]
+        agents, steps = [], 0
+        while (agents or waiting) and not errors:
+            while waiting and len(agents) < (resident or KC):
+                agents.append(waiting.pop())
             steps += 1
             if steps > 100000:
                 return errors + ["deadlock"]
@@ -260,18 +237,30 @@ def group(KC, launches, tagged, seed, mistake=None):
                 next(a)
             except StopIteration:
                 agents.remove(a)
-        if counter:
-            errors.append("counter is not zero after a launch")
+        if not errors and sorted(x[1:] for x in added if x[0] == launch) != [(s, e) for s in range(KC) for e in range(E)]:
+            errors.append("an element is not added exactly once")
+        if not errors and (word["count"] or word["mask"]):
+            errors.append("the word is not zero after a launch")
+        if not errors and tagged and any(v is not None for sh in slots for el in sh for v in el):
+            errors.append("a slot is full after a launch")
     return errors
 
 
 @pytest.mark.parametrize("tagged", [False, True])
-def test_chunks_of_a_group_meet(tagged):
-    for trial in range(200):
+@pytest.mark.parametrize("late", [0.0, 0.02, 0.3, 1.0])
+def test_chunks_of_a_group_meet(tagged, late):
+    for trial in range(150):
         rnd = random.Random(trial)
-        assert group(rnd.randint(2, 8), rnd.randint(1, 3), tagged, trial) == []
+        KC = rnd.randint(2, 8)
+        assert group(KC, rnd.randint(1, 3), tagged, trial, resident=rnd.randint(1, KC) if late else KC, late=late) == []
 
 
-@pytest.mark.parametrize("tagged,mistake", [(False, "count first"), (True, "no wait")])
+@pytest.mark.parametrize("tagged", [False, True])
+def test_without_patience_a_group_that_does_not_fit_hangs(tagged):
+    assert group(4, 1, tagged, 1, resident=3, late=0.0) == ["deadlock"]
+
+
+@pytest.mark.parametrize("tagged,mistake", [(False, "count first"), (True, "count first"), (True, "adds again"), (False, "no reset"), (True, "no reset"),
+                                            (False, "always leaves"), (True, "always leaves")])
 def test_group_model_flags_a_step_out_of_place(tagged, mistake):
-    assert any(group(4, 2, tagged, trial, mistake) for trial in range(40))
+    assert any(group(4, 2, tagged, trial, late=late, mistake=mistake) for trial in range(300) for late in (0.3, 1.0))
