@@ -115,8 +115,8 @@ SBVR_API int sbvr_decode_f16(const uint32_t* bvr, const void* coeff_idx, int idx
  *   4 = tcgen05 FP4 tensor-core kernel for small batches (2 <= M <= 32, at most 16 for G = 128; S, G, N and alignment as
  *       for algo 2, K a multiple of 256 and at most 32768; the activations are quantised by a small kernel in front, to 2^-33 of
  *       the largest of a row's 256-k block; needs a workspace of sbvr_workspace_bytes(...); more than 16 rows run on 3).
- * algo 0 takes 2 for M <= 4, 4 for M <= 16 (and for fewer rows where 2 does not apply) where K <= 4096 or N <= 256 or N >= 2048, 3
- * otherwise, and 1 for what none of them covers and for very small problems.  A row with a non-finite
+ * algo 0 takes 2 for M <= 4, 4 for M <= 16 (and for fewer rows where 2 does not apply) where K <= 4096 or N <= 256, or N >= 2048 and 4 is
+ * the faster by an estimate from sizes and encoding, 3 otherwise, and 1 for what none of them covers and for very small problems.  A row with a non-finite
  * activation becomes NaN on 2 and on 4 by request; 1, 3 and 4 where algo 0 picked it multiply it out. */
 SBVR_API int sbvr_linear_f16(const void* x, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff,
                     int C, const void* bias, void* y, int M, int N, int K, int S, int G, int algo,
@@ -302,6 +302,9 @@ SBVR_API int sbvr_embedding_f16(const int* ids, const void* table, void* out, in
  * `scratch` (128 floats + 128 ints, may be NULL) lets few rows of a large vocabulary be scanned by many SMs. */
 SBVR_API int sbvr_argmax_f16(const void* logits, int* out, float* scratch, int rows, int vocab, sbvr_stream_t stream);
 
+/* *folds = 1 where algo 0 would serve M rows by a kernel that takes an op in front (sbvr_linear_fused_f16 is then the faster form), 0 where
+ * the op's own launch and the GEMM are. */
+SBVR_API int sbvr_linear_folds(int device, int M, int N, int K, int S, int G, int idx_bytes, int* folds);
 /* ---- decode linears with the preceding element-wise op folded in ---------------------------------------------
  * The decode GEMV (algo 2 of sbvr_linear_f16: M <= 4, N % 32 == 0, K % 256 == 0) turns the activation row into
  * block-fixed-point digits in a small kernel of its own before the product; the op in front of the linear is applied

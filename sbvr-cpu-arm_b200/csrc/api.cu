@@ -183,6 +183,18 @@ int sbvr_workspace_bytes(int device, int M, int N, int K, size_t* bytes) {
     return SBVR_OK;
 }
 
+int sbvr_linear_folds(int device, int M, int N, int K, int S, int G, int idx_bytes, int* folds) {
+    if (!folds || M < 1 || N < 1 || K < 1) return SBVR_ERR_BAD_ARG;
+    DeviceInfo di;
+    const int rc = device_info(device, &di);
+    if (rc) return rc;
+    PackedW w;
+    w.bvr = nullptr, w.idx = nullptr, w.coeff = nullptr, w.idx_bytes = idx_bytes, w.C = 0;
+    w.N = N, w.K = K, w.S = S, w.G = G;
+    *folds = M <= 4 || (M <= 16 && S >= 2 && S <= 4 && (G == 128 || G == 256) && K % 256 == 0 && linear_sb_preferred(w, M, di));
+    return SBVR_OK;
+}
+
 int sbvr_linear_workspace_bytes(int device, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff, int C,
                                 int M, int N, int K, int S, int G, size_t* bytes) {
     PackedW w;
@@ -273,7 +285,7 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
         if (ws && device_info(ws->device, &di) == SBVR_OK && di.cc_major == 10) {
             if (linear_tcs_supported(w, M) && (Kin != K || !(reinterpret_cast<uintptr_t>(x) & 15)) &&
                 linear_tcs_workspace_bytes(w, M, di.sm_count) <= ws->dyn_bytes) algo = 2;
-            else if (M <= 16 && linear_sb_supported(w, M) && linear_sb_preferred(w) && linear_sb_workspace_bytes(w, di) <= ws->dyn_bytes)
+            else if (M <= 16 && linear_sb_supported(w, M) && linear_sb_preferred(w, M, di) && linear_sb_workspace_bytes(w, di) <= ws->dyn_bytes)
                 algo = 4;
             // A small problem is done by the SIMT kernel's one launch before the GEMM's second has started: measured 2.8 against
             // 5.7 us at 64 x 128 (M = 1), 5.2 against 9.8 at 300 x 512 (M = 8), 7.0 against 8.2 at 3000 x 1024 (M = 4), but 22

@@ -158,13 +158,14 @@ int xop_check(const XOp* xop, const __half* x, int M, int K, int* op, const __ha
 // The small-batch kernel (linear_sb.cu), 2 .. 16 activation rows: status words, the zeroed exchange region and arrival words (left zero)
 // and 256-byte aligned scratch are the caller's.  A row with a non-finite activation is multiplied out or becomes NaN.
 bool linear_sb_supported(const PackedW& w, int M);
-bool linear_sb_preferred(const PackedW& w);      // ... to the GEMM, by speed
+bool linear_sb_preferred(const PackedW& w, int M, const DeviceInfo& di);      // ... to the GEMM, by speed
 size_t linear_sb_workspace_bytes(const PackedW& w, const DeviceInfo& di);
 int launch_linear_sb(const __half* x, const PackedW& w, const __half* bias, __half* y, int M, int device, unsigned int* status,
                      float* xchg, unsigned long long* arrive, unsigned int patience, char* scratch, size_t scratch_bytes,
                      bool multiply_out, cudaStream_t st, const XOp* xop = nullptr);
 bool linear_gemm_supported(const PackedW& w, int M);
 size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count);
+void linear_gemm_split(const PackedW& w, int M, int sm_count, int* parts, int* stages);      // parts of K, 64-k stages of each
 // x rows of Kin <= K elements (row pitch Kin), as if padded with zeros to K
 int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half* bias, __half* y, int M,
                        const sbvr_workspace* ws, cudaStream_t st);

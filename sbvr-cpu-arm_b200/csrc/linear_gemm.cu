@@ -757,6 +757,12 @@ size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count) {
     return pl.xt_bytes + pl.part_bytes;
 }
 
+void linear_gemm_split(const PackedW& w, int M, int sm_count, int* parts, int* stages) {
+    GmPlan pl;
+    gm_plan(w, M, sm_count, &pl);
+    *parts = pl.KS, *stages = pl.SPP * ((pl.items + sm_count - 1) / sm_count);
+}
+
 template <int S, int NX, bool SPLIT, bool EXACT>
 static int gm_launch_split(const GmParams& p, int grid, int smem, cudaStream_t st) {
     static SmemOnce once;

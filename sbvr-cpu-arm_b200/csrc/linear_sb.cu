@@ -866,12 +866,27 @@ bool linear_sb_supported(const PackedW& w, int M) {
     return sb_plan(w, di, &pl) == SBVR_OK;
 }
 
-// Where it is faster than the GEMM (M = 16, us, the GEMM in brackets).  Up to four chunks of K: 1024 x 4096 9.4 (10.4), 4096 x 4096 10.9
-// (14.8), 14336 x 4096 21.7 (32.1), 32768 x 1024 13.7 (23.1).  More chunks, with weights of many rows: 2048 x 16384 20.5 (23.7), 4096 x 8192
-// 19.5 (21.8), 4096 x 14336 26.6 (31.6; with groups of 128 30.6 (31.0)), 8192 x 28672 61.6 (104), 28672 x 8192 60 (112).  In between
-// the chunks' merge costs what the product gains: 1024 x 14336 16.2 (16.1; two planes 15.4 (13.1)), 512 x 28672 18.3 (18.4; two planes
-// 16.9 (15.4)); weights of so few rows that the GEMM has one or two tiles: 128 x 14336 12.3 (14.9).
-bool linear_sb_preferred(const PackedW& w) { return w.K <= 4096 || w.N <= 256 || w.N >= 2048; }
+// Where it is faster than the GEMM.  Up to four chunks of K: 1024 x 4096 9.8 us (the GEMM 10.4; M = 16, S = 4), 4096 x 4096 11.4 (14.8), 14336 x
+// 4096 22.3 (32.1), 32768 x 1024 13.7 (23.1).  Weights of so few rows that the GEMM has one or two tiles: 128 x 14336 12.3 (14.9); up
+// to 2048 rows the chunks' merge costs what the product gains: 1024 x 14336 16.2 (16.1), 512 x 28672 18.3 (18.4).  More chunks and more rows:
+// both times are near linear in what the plans say, the GEMM's in the 64-k stages of a part (dearer with the planes, cheaper without a
+// codebook) and in its fp32 parts,
+// this kernel's in the units of a warpgroup (dearer with two groups a block), the chunks and their sums.  The factors were fitted to
+// minimise what a wrong choice costs over 310 measured calls (2048 .. 14336 rows, K 4352 .. 28672, 5 and 16 rows, S = 2 .. 4, both group
+// lengths): 10 % at most, 0.3 % on average, and 0.5 % over 130 others drawn from the same ranges; taking this kernel always cost up to 28 % (S = 2, 4096 x 4352, 16 rows: 15.0 against 11.7),
+// the GEMM always up to 69 % (S = 4, 14336 x 5120: 17 against 10 with five rows).
+bool linear_sb_preferred(const PackedW& w, int M, const DeviceInfo& di) {
+    if (w.K <= 4096 || w.N <= 256) return true;
+    if (w.N < 2048) return false;
+    SbPlan pl;
+    if (sb_plan(w, di, &pl) != SBVR_OK) return false;
+    const int tiles = (pl.NT + pl.GN - 1) / pl.GN, blocks = (pl.KB + pl.KC - 1) / pl.KC;
+    const float units = (float)((tiles * blocks + SB_NWG - 1) / SB_NWG);
+    const float here = 10.0f + (w.G == 128 ? 1.6f : 1.15f) * units + 0.15f * (float)pl.KC + 4.2e-6f * (float)pl.KC * (float)w.N * (float)M;
+    int parts, stages;
+    linear_gemm_split(w, M, di.sm_count, &parts, &stages);
+    return here < 4.5f + (0.1f + 0.12f * (float)w.S) * (w.idx_bytes ? 1.0f : 0.87f) * (float)stages + 1.8e-4f * (float)parts * (float)w.N;
+}
 
 size_t linear_sb_workspace_bytes(const PackedW& w, const DeviceInfo& di) {
     SbPlan pl;

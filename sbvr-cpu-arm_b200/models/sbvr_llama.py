@@ -340,14 +340,13 @@ class SBVRLlamaForCausalLM(torch.nn.Module):
         fuse = self.fuse_glue and T <= 16
 
         def folds(lin) -> bool:
-            """More than four rows: the small-batch kernel takes the op, so fold where `linear` would take that kernel too (the rule of
-            algo 0: linear_sb_preferred in csrc/linear_sb.cu); elsewhere the op's own launch and the GEMM are faster."""
+            """More than four rows: the small-batch kernel takes the op, so fold where `linear` would take that kernel too; elsewhere the
+            op's own launch and the GEMM are faster."""
             if not (fuse and isinstance(lin, SBVRLinear)):
                 return False
             w = lin.weight
-            K = w.in_features_padded
-            N = w.out_features
-            return T <= 4 or K <= 4096 or N <= 256 or N >= 2048
+            return T <= 4 or _lib.linear_folds(self.device.index or 0, T, w.out_features, w.in_features_padded, w.num_sums, w.bvr_len,
+                                               0 if w.coeff_idx is None else w.coeff_idx.element_size())
         hc, ho = b.h, b.h2                         # current residual, spare buffer
 
         def norm_linear(lin, delta, weight, out, keep_residual=True):

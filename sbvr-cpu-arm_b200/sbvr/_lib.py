@@ -7,6 +7,7 @@ binding raised RuntimeError from `std::runtime_error` (reference sbvr/kernels/sb
 from __future__ import annotations
 
 import ctypes
+import functools
 import importlib.util
 import os
 import threading
@@ -52,6 +53,8 @@ lib.sbvr_workspace_destroy.argtypes = [_vp]
 lib.sbvr_workspace_destroy.restype = _i
 lib.sbvr_workspace_status.argtypes = [_vp, _vp]
 lib.sbvr_workspace_status.restype = _i
+lib.sbvr_linear_folds.argtypes = [_i, _i, _i, _i, _i, _i, _i, ctypes.POINTER(_i)]
+lib.sbvr_linear_folds.restype = _i
 lib.sbvr_workspace_patience.argtypes = [_vp, ctypes.c_uint]
 lib.sbvr_workspace_patience.restype = _i
 lib.sbvr_decode_f16.argtypes = [_vp, _vp, _i, _vp, _i, _vp, _i, _i, _i, _i, _i, _i, _vp]
@@ -107,7 +110,7 @@ lib.sbvr_ll_reduce_add_rmsnorm_digits_f16.restype = _i
 lib.sbvr_allreduce_add_rmsnorm_digits_f16.argtypes = [_vp, _vp, _vp, _i, _i, _i, _i, _sz, _vp, _vp, _vp, _vp, _i, _i, _f, _i, _vp, _vp]
 lib.sbvr_allreduce_add_rmsnorm_digits_f16.restype = _i
 
-EXPORTS = ["sbvr_linear_workspace_bytes", "sbvr_linear_padded_f16", "sbvr_encode_stats_f16", "sbvr_encode_advance", "sbvr_encode_run", "sbvr_popc_mm_f16", "sbvr_linear_t_f16", "sbvr_encode_mse_f16", "sbvr_encode_select_f16", "sbvr_encode_pack", "sbvr_rope_attention_f16", "sbvr_linear_fused_f16", "sbvr_allreduce_add_rmsnorm_f16", "sbvr_linear_push_f16", "sbvr_ll_reduce_add_rmsnorm_f16", "sbvr_ll_reduce_add_rmsnorm_digits_f16", "sbvr_allreduce_add_rmsnorm_digits_f16", "sbvr_add_rmsnorm_f16", "sbvr_rope_append_f16", "sbvr_attention_f16", "sbvr_silu_mul_f16",
+EXPORTS = ["sbvr_linear_folds", "sbvr_linear_workspace_bytes", "sbvr_linear_padded_f16", "sbvr_encode_stats_f16", "sbvr_encode_advance", "sbvr_encode_run", "sbvr_popc_mm_f16", "sbvr_linear_t_f16", "sbvr_encode_mse_f16", "sbvr_encode_select_f16", "sbvr_encode_pack", "sbvr_rope_attention_f16", "sbvr_linear_fused_f16", "sbvr_allreduce_add_rmsnorm_f16", "sbvr_linear_push_f16", "sbvr_ll_reduce_add_rmsnorm_f16", "sbvr_ll_reduce_add_rmsnorm_digits_f16", "sbvr_allreduce_add_rmsnorm_digits_f16", "sbvr_add_rmsnorm_f16", "sbvr_rope_append_f16", "sbvr_attention_f16", "sbvr_silu_mul_f16",
            "sbvr_embedding_f16", "sbvr_argmax_f16", "sbvr_linear_f16_noalloc", "sbvr_workspace_bytes", "sbvr_strerror", "sbvr_last_cuda_error", "sbvr_last_timeout_where", "sbvr_last_timeout_info", "sbvr_query", "sbvr_workspace_create",
            "sbvr_workspace_destroy", "sbvr_workspace_status", "sbvr_workspace_patience", "sbvr_decode_f16", "sbvr_linear_f16",
            "sbvr_linear_f16_host"]
@@ -209,6 +212,13 @@ _workspaces: dict = {}
 _retired: list = []
 # Torch's threads share the default stream, and creating a workspace lets other threads run.
 _ws_lock = threading.Lock()
+
+
+@functools.lru_cache(maxsize=4096)
+def linear_folds(device: int, M: int, N: int, K: int, S: int, G: int, idx_bytes: int) -> bool:
+    out = _i(0)
+    check(lib.sbvr_linear_folds(device, M, N, K, S, G, idx_bytes, ctypes.byref(out)), "sbvr_linear_folds")
+    return bool(out.value)
 
 
 def workspace_bytes(device: int, M: int, N: int, K: int) -> int:

@@ -603,3 +603,18 @@ def test_small_batch_kernel_on_two_streams_at_once():
     for s in streams:
         with torch.cuda.stream(s):
             check_status()
+
+
+@pytest.mark.parametrize("S,G,N,K,M,algo", [(4, 256, 4096, 4096, 16, 4), (4, 256, 4096, 14336, 16, 4), (4, 256, 4096, 14336, 5, 4), (4, 128, 14336, 8192, 16, 4),
+                                            (2, 256, 8192, 8192, 16, 4), (3, 256, 2048, 11008, 16, 4), (2, 256, 128, 14336, 16, 4), (2, 256, 4096, 4352, 16, 3),
+                                            (2, 256, 2048, 6144, 16, 3), (3, 256, 4096, 5120, 16, 3), (4, 128, 4096, 6144, 16, 3), (4, 256, 1024, 14336, 16, 3)])
+def test_automatic_choice_of_a_few_rows(S, G, N, K, M, algo):
+    """Five to sixteen rows go to whichever of the small-batch kernel and the GEMM was measured to be the faster (by 5 to 40 % in these
+    calls), and an op is folded where it is the former."""
+    import sbvr
+    from sbvr import _lib
+    w = to_sbvr(O.make_packed(N, K, S, G=G, mode="u16", C=1000, seed=N + K))
+    x = torch.from_numpy(np.random.default_rng(M).standard_normal((M, K)).astype(np.float16)).cuda()
+    y, small, gemm = (sbvr.linear(x, w, None, algo=a) for a in (0, 4, 3))
+    assert torch.equal(y, small if algo == 4 else gemm) and not torch.equal(small, gemm)
+    assert _lib.linear_folds(torch.cuda.current_device(), M, N, K, S, G, 2) == (algo == 4)
