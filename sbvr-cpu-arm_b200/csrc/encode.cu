@@ -637,6 +637,7 @@ __global__ void __launch_bounds__(ENC_THREADS) encode_walk_kernel(const __grid_c
             else if (!covered) stop = SBVR_ENCODE_CALLER;
             else if (enc_decide<S>(p, q, p.q.space[ext ? 1 : 0], g, cached, n, accepted, hist, hist_n)) stop = SBVR_ENCODE_CALLER;
             else ++misses, ++steps, from = g + 1;
+            if (stop == SBVR_ENCODE_CALLER) from = g;          // (every group in front of it is served)
             if (threadIdx.x == 0) publish(stop);
         }
         met = enc_meet(c, round);

@@ -368,8 +368,9 @@ def encode(data: torch.Tensor, conf: EncoderConfig, device: Optional[torch.devic
         own_groups, own_lines, own_index = [], [], []      # groups that keep their own candidate, it, the line it is filed under
         gi = 0
         hits = None
+        host_search = False                                # the last step's group was left to the tensor operations; the next one may be too
         while gi < NG:
-            if many is not None and (book.n < conf.max_cache_lines or book.n < conf.cache_warmup_num):
+            if many is not None and not host_search and (book.n < conf.max_cache_lines or book.n < conf.cache_warmup_num):
                 if walk.append_at >= 0:
                     book.lines[walk.append_at] = torch.from_numpy(book.host[walk.append_at]).to(dev)
                     walk.append_at = -1
@@ -389,6 +390,7 @@ def encode(data: torch.Tensor, conf: EncoderConfig, device: Optional[torch.devic
             if not warm:
                 walk.line0 = walk.line1
             g = res.group
+            host_search = res.status == 2
             if full:
                 hits = gi - walk.misses + int((best_mse[gi:].double() < book.cutoff()).sum())
                 break

@@ -1,5 +1,7 @@
 """The GPU encoder (`sbvr.sbvr(data, encoder_config)`, sbvr/encoder.py + csrc/encode.cu) against the reference encoder's
 golden output and against the CPU restatement of its error function (oracle/encoder_ref.py)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -205,3 +207,37 @@ def test_many_steps_in_one_launch_equal_one_at_a_time(S, settings):
     many = encoder.encode(W.half(), encoder.EncoderConfig(num_sums=S, **settings))
     assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(one[:3], many[:3]))
     assert one[3] == many[3]
+
+
+def _watch_runs(monkeypatch, limit=None, outcome=None):
+    """Counts why the launches of many steps end; `limit`: steps of one launch; `outcome`: what each is made to report."""
+    from sbvr import _lib, encoder
+    why, real = [], _lib.lib.sbvr_encode_run
+    if limit:
+        monkeypatch.setattr(encoder._ManySteps, "LIMIT", limit)
+
+    def run(walk, args, stream):
+        rc = real(walk, args, stream)
+        out = ctypes.cast(args._obj.outcome, ctypes.POINTER(ctypes.c_int))
+        if outcome:
+            out[0] = outcome
+        why.append(out[0])
+        return rc
+    monkeypatch.setattr(_lib.lib, "sbvr_encode_run", run)
+    return why
+
+
+@pytest.mark.parametrize("mean", [0.5, 0.08])
+def test_groups_the_kernel_leaves_to_the_host_are_not_looked_for_twice(monkeypatch, mean):
+    """A large mean takes every group's search to the tensor operations: after the first the walk goes on in single steps, as with a
+    progress callback, and gives the same encoding."""
+    from sbvr import encoder
+    g = torch.Generator(device="cuda").manual_seed(1)
+    W = (torch.randn((16, 1024), device="cuda", generator=g) * 0.02 + mean).half()
+    W[3] = torch.randn(1024, device="cuda", generator=g) * 0.02       # (back to the device for a row)
+    conf = encoder.EncoderConfig(num_sums=3)
+    one = encoder.encode(W, conf, progress=lambda done, of: None)
+    why = _watch_runs(monkeypatch)
+    many = encoder.encode(W, conf)
+    assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(one[:3], many[:3])) and one[3] == many[3]
+    assert one[3]["groups"] - one[3]["cache_hits"] > 10 and 1 <= len(why) <= 6, (one[3], why)
