@@ -873,7 +873,7 @@ bool linear_sb_supported(const PackedW& w, int M) {
 // codebook) and in its fp32 parts,
 // this kernel's in the units of a warpgroup (dearer with two groups a block), the chunks and their sums.  The factors were fitted to
 // minimise what a wrong choice costs over 310 measured calls (2048 .. 14336 rows, K 4352 .. 28672, 5 and 16 rows, S = 2 .. 4, both group
-// lengths): 10 % at most, 0.3 % on average, and 0.5 % over 130 others drawn from the same ranges; taking this kernel always cost up to 28 % (S = 2, 4096 x 4352, 16 rows: 15.0 against 11.7),
+// lengths): 10 % at most, 0.3 % on average, and 0.1 % over 200 others drawn from the same ranges, with other row counts and encodings; taking this kernel always cost up to 28 % (S = 2, 4096 x 4352, 16 rows: 15.0 against 11.7),
 // the GEMM always up to 69 % (S = 4, 14336 x 5120: 17 against 10 with five rows).
 bool linear_sb_preferred(const PackedW& w, int M, const DeviceInfo& di) {
     if (w.K <= 4096 || w.N <= 256) return true;

@@ -26,6 +26,7 @@ from __future__ import annotations
 import ctypes
 import itertools
 import math
+import sys
 from dataclasses import dataclass, field
 from typing import List, Optional, Tuple
 
@@ -192,6 +193,20 @@ def pack_selectors(sel: torch.Tensor, S: int) -> torch.Tensor:
 # ---------------------------------------------------------------------------------------------------------------
 # the walk over the groups
 # ---------------------------------------------------------------------------------------------------------------
+def _compensated_sum(values) -> float:
+    """A sum of floats with Neumaier's compensation (Z. angew. Math. Mech. 54, 1974): what the walk kernel forms, and `sum` from Python
+    3.12 on."""
+    total = lost = 0.0
+    for x in values:
+        t = total + x
+        lost += (total - t) + x if abs(total) >= abs(x) else (x - t) + total
+        total = t
+    return total + lost if lost and math.isfinite(lost) else total
+
+
+_sum = sum if sys.version_info >= (3, 12) else _compensated_sum
+
+
 class _Codebook:
     """The growing coefficient cache and the running statistics that steer the search (the mutable part of the
     reference's `_sbvr_enc_conf`: coeff_cache, num_coeff_cache_lines, mse_history, cache_hits, group_idx).  The lines are
@@ -213,7 +228,7 @@ class _Codebook:
         """0.99 x the mean MSE of the most recent accepted searches, not below `acceptable_mse` (sbvr/core.py:563-568)."""
         if self._cutoff is None:
             window = self.history[-min(len(self.history), self.conf.mse_window_size):]
-            self._cutoff = max((sum(window) / len(window)) * 0.99, self.conf.acceptable_mse)
+            self._cutoff = max((_sum(window) / len(window)) * 0.99, self.conf.acceptable_mse)
         return self._cutoff
 
     def find_or_add(self, line: np.ndarray) -> Tuple[int, bool]:

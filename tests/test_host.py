@@ -258,3 +258,40 @@ def test_step_partition_of_the_streaming_kernels(tmp_path):
     out = subprocess.run([exe], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout[-2000:]
     assert "0 failures" in out.stdout
+
+
+def test_encoder_cutoff_is_the_same_sum_on_every_interpreter(monkeypatch):
+    """The walk kernel forms the mean of accepted errors with a compensated sum, which `sum` is from Python 3.12 on only: an older
+    interpreter must not get another codebook where the host decides."""
+    import builtins
+    import importlib.util
+    import math
+    import random
+    import sys
+    from sbvr import encoder
+
+    def plain(values):
+        total = 0.0
+        for v in values:
+            total = total + v
+        return total
+    rnd = random.Random(1)
+    windows = [[rnd.lognormvariate(-9, 3) for _ in range(rnd.randint(1, 64))] for _ in range(300)]
+    windows += [[1.0, 1e100, 1.0, -1e100], [math.inf, 1.0], [1e308, 1e308, -1e308]]
+    assert any(plain(w) != encoder._compensated_sum(w) for w in windows[:300])
+    if sys.version_info >= (3, 12):
+        same = lambda a, b: a == b or (a != a and b != b)
+        assert all(same(sum(w), encoder._compensated_sum(w)) for w in windows)
+    want = []
+    for w in windows[:300]:
+        book = encoder._Codebook(encoder.EncoderConfig(mse_window_size=64, acceptable_mse=0.0, mse_history=w), "cpu")
+        want.append(book.cutoff())
+    with monkeypatch.context() as m:
+        m.setattr(builtins, "sum", plain)
+        m.setattr(sys, "version_info", (3, 11, 0, "final", 0))
+        spec = importlib.util.spec_from_file_location("sbvr._encoder_older", encoder.__file__)
+        older = importlib.util.module_from_spec(spec)
+        m.setitem(sys.modules, spec.name, older)
+        spec.loader.exec_module(older)
+        got = [older._Codebook(older.EncoderConfig(mse_window_size=64, acceptable_mse=0.0, mse_history=w), "cpu").cutoff() for w in windows[:300]]
+    assert got == want
