@@ -234,7 +234,8 @@ SBVR_API int sbvr_encode_advance(const sbvr_encode_walk_t* walk, sbvr_stream_t s
 
 /* Many steps of the walk in one cooperative launch, decisions included (sbvr/core.py:555-577, :605-653): up to `limit` misses, until
  * nothing is left, the codebook is full, or a group needs the caller (sbvr_encode_advance from `outcome` on, which names the group).  `walk` as
- * above with search = 1 and append_at = -1; line1 and cutoff are not looked at.  Synchronises `stream`. */
+ * above with search = 1 and append_at = -1; line1 and cutoff are not looked at.  Synchronises `stream`.  SBVR_ENCODE_TIMEOUT: the blocks did
+ * not meet within about a second, something else holds SMs; the walk stands as `outcome` says, sbvr_encode_advance needs no meeting. */
 #define SBVR_ENCODE_WINDOW 64
 enum { SBVR_ENCODE_DONE = 1, SBVR_ENCODE_LIMIT = 2, SBVR_ENCODE_FULL = 3, SBVR_ENCODE_CALLER = 4, SBVR_ENCODE_TIMEOUT = 5 };
 typedef struct sbvr_encode_record {

@@ -610,11 +610,15 @@ __global__ void __launch_bounds__(ENC_THREADS) encode_walk_kernel(const __grid_c
         from = __ldcg(&c->from), n = __ldcg(&c->n), line0 = __ldcg(&c->line0), misses = __ldcg(&c->misses);
         const double cutoff = __ldcg(&c->cutoff);
         const bool warm = n < p.warmup;
+        const int met_from = line0;                // (should the blocks not meet: lines that not every group has met)
         if (!warm) {
             enc_update_all<S>(p, from, line0, n, cutoff);
             line0 = n;
         }
-        if (!(met = enc_meet(c, round))) break;
+        if (!(met = enc_meet(c, round))) {
+            line0 = met_from;
+            break;
+        }
         const int g = __ldcg(&c->miss);
         float cached = INFINITY;
         bool covered = true;
@@ -630,7 +634,10 @@ __global__ void __launch_bounds__(ENC_THREADS) encode_walk_kernel(const __grid_c
                 enc_search<S>(q, p.q.space[ext ? 1 : 0], ds, cached, &c->best);
             }
         }
-        if (!(met = enc_meet(c, round))) break;
+        if (!(met = enc_meet(c, round))) {
+            line0 = met_from;
+            break;
+        }
         if (blockIdx.x == 0) {
             int stop = 0;
             if (g >= p.q.NG) stop = SBVR_ENCODE_DONE;
@@ -642,6 +649,8 @@ __global__ void __launch_bounds__(ENC_THREADS) encode_walk_kernel(const __grid_c
         }
         met = enc_meet(c, round);
     }
+    // Blocks that have not met -- another stream's kernel keeps some from running -- leave the walk at the last decision: block 0 decides only
+    // when all have searched, and a line that a group meets a second time changes nothing.
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         p.outcome[0] = met ? __ldcg(&c->stop) : SBVR_ENCODE_TIMEOUT;
         p.outcome[1] = from, p.outcome[2] = n, p.outcome[3] = line0, p.outcome[4] = misses, p.outcome[5] = accepted;
@@ -660,7 +669,7 @@ static int encode_run(const EncRun& r, int sm_count, cudaStream_t st) {
     SBVR_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(encode_walk_kernel<S>), dim3(per_sm * sm_count), dim3(ENC_THREADS),
                                               args, 0, st));
     SBVR_CUDA_TRY(cudaStreamSynchronize(st));
-    return r.outcome[0] == SBVR_ENCODE_TIMEOUT ? SBVR_ERR_TIMEOUT : SBVR_OK;
+    return SBVR_OK;
 }
 
 // device scratch of a walk: [0] next miss, [1] finished blocks, [2..3] best key

@@ -147,7 +147,7 @@ class EncodeRun(ctypes.Structure):
                 ("hist_n", _i), ("limit", _i), ("acceptable", ctypes.c_double), ("hist", ctypes.c_double * 64)]
 
 
-ENCODE_DONE, ENCODE_LIMIT, ENCODE_FULL, ENCODE_CALLER = 1, 2, 3, 4
+ENCODE_DONE, ENCODE_LIMIT, ENCODE_FULL, ENCODE_CALLER, ENCODE_TIMEOUT = 1, 2, 3, 4, 5
 lib.sbvr_encode_run.argtypes = [ctypes.POINTER(EncodeWalk), ctypes.POINTER(EncodeRun), _vp]
 lib.sbvr_encode_run.restype = _i
 

@@ -303,8 +303,8 @@ class _ManySteps:
                                    warmup=conf.cache_warmup_num, window=conf.mse_window_size, limit=self.LIMIT,
                                    acceptable=conf.acceptable_mse)
 
-    def run(self, walk, book: "_Codebook", stream: int, own_groups: list, own_lines: list, own_index: list) -> int:
-        """Walks on from `walk.from_`; returns the first group that is not decided."""
+    def run(self, walk, book: "_Codebook", stream: int, own_groups: list, own_lines: list, own_index: list) -> Tuple[int, int]:
+        """Walks on from `walk.from_`; returns the first group that is not decided, and why it stopped."""
         a, S = self.args, self.conf.num_sums
         tail = book.history[-self.conf.mse_window_size:]
         a.n, a.hist_n = book.n, len(tail)
@@ -322,7 +322,7 @@ class _ManySteps:
         assert book.n == n
         for mse in rec["mse"].tolist():
             book.accept(mse)
-        return walk.groups if why == _lib.ENCODE_DONE else gi
+        return walk.groups if why == _lib.ENCODE_DONE else gi, why
 
 
 def _sorted_line(bits, S: int, device) -> np.ndarray:
@@ -390,7 +390,9 @@ def encode(data: torch.Tensor, conf: EncoderConfig, device: Optional[torch.devic
                     book.lines[walk.append_at] = torch.from_numpy(book.host[walk.append_at]).to(dev)
                     walk.append_at = -1
                 walk.from_, walk.search = gi, 1
-                gi = many.run(walk, book, st, own_groups, own_lines, own_index)
+                gi, why = many.run(walk, book, st, own_groups, own_lines, own_index)
+                if why == _lib.ENCODE_TIMEOUT:             # its blocks cannot all run at the moment: single steps to the end
+                    many = None
                 if gi >= NG:
                     hits = NG - walk.misses
                     break

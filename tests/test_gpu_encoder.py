@@ -190,10 +190,10 @@ def test_encode_then_linear_end_to_end():
 @pytest.mark.parametrize("settings", [{}, {"cache_warmup_num": 1}, {"cache_warmup_num": 40, "mse_window_size": 64}, {"mse_window_size": 1},
                                       {"max_cache_lines": 23}, {"acceptable_mse": 1e-4}, {"mse_history": [1e-7, 3e-6], "cache_warmup_num": 0},
                                       {"mse_window_size": 65}])
-def test_many_steps_in_one_launch_equal_one_at_a_time(S, settings):
+def test_many_steps_in_one_launch_equal_one_at_a_time(monkeypatch, S, settings):
     """With a progress callback the walk takes one step per launch and decides on the host; without, on the device: codebook, indices,
     bit-planes and counts are the same.  Among the groups: repeated ones (a winner that is stored already), zeros, a large mean
-    and too few distinct values (left to the host), more misses than one launch takes (1 024, S = 4)."""
+    and too few distinct values (left to the host); a launch takes seven misses, and once as many as it does."""
     from sbvr import encoder
     g = torch.Generator(device="cuda").manual_seed(S)
     rows = 300 if S == 4 and settings == {"mse_window_size": 1} else 24
@@ -204,9 +204,45 @@ def test_many_steps_in_one_launch_equal_one_at_a_time(S, settings):
     W[11] = torch.sign(W[11]) * 0.01
     W[13, :256] = W[13, 0]
     one = encoder.encode(W.half(), encoder.EncoderConfig(num_sums=S, **settings), progress=lambda done, of: None)
-    many = encoder.encode(W.half(), encoder.EncoderConfig(num_sums=S, **settings))
-    assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(one[:3], many[:3]))
-    assert one[3] == many[3]
+    for limit in (None, 7):
+        why = _watch_runs(monkeypatch, limit)
+        many = encoder.encode(W.half(), encoder.EncoderConfig(num_sums=S, **settings))
+        assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(one[:3], many[:3]))
+        assert one[3] == many[3]
+        assert bool(why) == (settings != {"mse_window_size": 65})          # (more errors to look back on than the kernel keeps)
+
+
+@pytest.mark.parametrize("S", [2, 4])
+@pytest.mark.parametrize("settings,mean,reasons", [({"cache_warmup_num": 40}, 0.0, ["LIMIT", "DONE"]), ({"cache_warmup_num": 40}, 0.5, ["LIMIT", "CALLER"]),
+                                                   ({"cache_warmup_num": 10, "max_cache_lines": 10}, 0.0, ["LIMIT", "FULL"])])
+def test_launches_end_for_every_reason(monkeypatch, S, settings, mean, reasons):
+    """A launch of seven steps at most ends because it has taken them, at a group of a large mean, when the codebook is full or at the
+    end, and the walk goes on from there as in single steps."""
+    from sbvr import _lib, encoder
+    g = torch.Generator(device="cuda").manual_seed(S)
+    W = torch.randn((24, 1024), device="cuda", generator=g) * 0.02 * torch.exp(0.4 * torch.randn((24, 1), device="cuda", generator=g))
+    W[5] += mean
+    conf = encoder.EncoderConfig(num_sums=S, **settings)
+    one = encoder.encode(W.half(), conf, progress=lambda done, of: None)
+    why = _watch_runs(monkeypatch, limit=7)
+    many = encoder.encode(W.half(), conf)
+    assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(one[:3], many[:3])) and one[3] == many[3]
+    assert {getattr(_lib, "ENCODE_" + r) for r in reasons} <= set(why), why
+
+
+@pytest.mark.parametrize("S", [2, 4])
+@pytest.mark.parametrize("settings", [{}, {"cache_warmup_num": 40}])
+def test_blocks_that_do_not_meet_leave_the_walk_to_single_steps(monkeypatch, S, settings):
+    """A launch of many steps whose blocks could not all run reports so, with the walk as it stands; the rest is walked step by step."""
+    from sbvr import _lib, encoder
+    g = torch.Generator(device="cuda").manual_seed(S)
+    W = (torch.randn((24, 1024), device="cuda", generator=g) * 0.02 * torch.exp(0.4 * torch.randn((24, 1), device="cuda", generator=g))).half()
+    conf = encoder.EncoderConfig(num_sums=S, **settings)
+    one = encoder.encode(W, conf, progress=lambda done, of: None)
+    why = _watch_runs(monkeypatch, limit=5, outcome=_lib.ENCODE_TIMEOUT)
+    many = encoder.encode(W, conf)
+    assert all(torch.equal(a.view(torch.uint8), b.view(torch.uint8)) for a, b in zip(one[:3], many[:3])) and one[3] == many[3]
+    assert why == [_lib.ENCODE_TIMEOUT]
 
 
 def _watch_runs(monkeypatch, limit=None, outcome=None):
