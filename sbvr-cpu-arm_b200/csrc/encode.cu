@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(ENC_THREADS) encode_search_kernel(const EncSea
 // of it or a new one, and moves the cut-off -- while the others wait; three meetings of the grid.  1024 x 4096, S = 4: a step takes 54 us, 36
 // of them the search (459 000 candidates, 16 half-rate differences and minima per pair of values, about half of them before the
 // warp's last candidate is out), 13 the update, 4 the decision; with three launches, a synchronisation and the decision in Python
-// per step it took 87.  Whole encoding: 13.4 -> 8.9 ms.
+// per step it took 87.  Whole encoding: 11.3 -> 8.5 ms.
 //
 // The arithmetic of the decisions is the host's: a line's magnitude is the fp32 sum of its |c| in order, rounded to fp16; a difference
 // of lines is rounded to fp32 and then to fp16; the mean of the accepted errors is a sum in double with Neumaier's

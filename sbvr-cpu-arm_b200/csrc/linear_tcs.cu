@@ -45,8 +45,10 @@ __host__ __device__ constexpr int ts_mpad(int M) { return M <= 2 ? 2 : 4; }
 __host__ __device__ constexpr int ts_dcols(int NSUB, int M, int KS) { return KS == 2 ? 16 : NSUB * 8 * ts_mpad(M); }
 __host__ __device__ constexpr int ts_wgcols(int NSUB, int M, int KS) { return 64 * KS + 2 * ts_dcols(NSUB, M, KS); }
 // Warpgroups of a CTA: what tensor memory holds, five at most; three for two activation rows, whose work does
-// not go well into the 64 registers that five leave a thread (us per call, M = 2, S = 4, five and three: 6144 x 4096 11.0 and 8.9, 14336 x 4096 15.8 and 12.9, 28672 x 4096 21.6 and
-// 19.9, 4096 x 4096 7.3 and 7.4).  One row in steps of one block wants all five: 8192 x 11008 15.5, with three 17.7.
+// not go well into the 64 registers that five leave a thread (us per call, M = 2, S = 4, five and three: 8192 x 8192 17.4 and 13.7, 14336 x
+// 4096 15.8 and 12.9, 28672 x 8192 36.1 and 32.8, 4096 x 4096 7.7 and 7.3).  With three planes or direct coefficients, up to one tile per SM,
+// long rows lose: S = 3, 4096 x 11008 11.6 and 12.4, 4096 x 20480 17.9 and 19.1.  One row in steps of one block wants all five: 8192 x
+// 11008 15.5, with three 17.7.
 __host__ __device__ constexpr int ts_nwg(int NSUB, int M, int KS) {
     return M == 2 ? 3 : (TS_SF_COL / ts_wgcols(NSUB, M, KS)) > 5 ? 5 : (TS_SF_COL / ts_wgcols(NSUB, M, KS));
 }
