@@ -768,6 +768,7 @@ __global__ void __maxnreg__(88) linear_sb_kernel(const __grid_constant__ CUtenso
         const bool speaker = threadIdx.x == SB_THREADS - 32;          // (of a warp that has few sums to add or none)
         const unsigned int part = sb_part_of_group(chunk, KC);
         unsigned long long before = 0ull;
+        __syncwarp();
         if (warp == SB_THREADS / 32 - 1) named_bar_sync(14, SB_THREADS);        // every warp's sums are stored
         else ts_bar_arrive(14, SB_THREADS);
         if (speaker) {
