@@ -170,6 +170,12 @@ void linear_gemm_split(const PackedW& w, int M, int sm_count, int* parts, int* s
 int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half* bias, __half* y, int M,
                        const sbvr_workspace* ws, cudaStream_t st);
 
+// The GEMM over CTA pairs (linear_pair.cu), more than 256 rows; `scratch` is for sums of items that several pairs share, none is needed.
+bool linear_pair_supported(const __half* x, int Kin, const PackedW& w, const __half* y, int M);
+long long linear_pair_ns(const PackedW& w, int M, int sm_count, int device, size_t scratch);      // estimate, to choose between the two GEMMs
+int launch_linear_pair(const __half* x, int Kin, const PackedW& w, const __half* bias, __half* y, int M, unsigned int* status,
+                       char* scratch, size_t scratch_bytes, int sm_count, int device, cudaStream_t st);
+
 // ---------------------------------------------------------------------------------------------
 // device side
 // ---------------------------------------------------------------------------------------------

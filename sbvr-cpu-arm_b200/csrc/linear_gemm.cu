@@ -751,6 +751,17 @@ static void gm_plan(const PackedW& w, int M, int sm_count, GmPlan* pl) {
     pl->part_bytes = ks > 1 ? (size_t)ks * pl->MT * pl->NX * w.N * 4 : 0;
 }
 
+// Estimate of a call's time in ns for more than 256 rows, to choose between this kernel and the one over CTA pairs: rounds of tiles at
+// the stage times of gm_nx and 9 000 cycles for a tile's end, at 1.9 GHz; re-tiling; the parts of a split K (16.8 MB of them took
+// about 10 us).  Measured and estimated, us: 2048 x 14336 x 4096 209, 209; 512 x 8192 x 8192 67, 67; 1024 x 4096 x 4096 38, 38; 300 x
+// 14336 x 4096 41.5, 41; 3000 x 4096 x 14336 303, 307; 2048 x 1024 x 4096 37, 36.
+static long long gm_ns(const PackedW& w, const GmPlan& pl, int sm_count) {
+    const long long rounds = (pl.items + sm_count - 1) / sm_count;
+    const long long cycles = rounds * ((long long)pl.SPP * (pl.NX == 256 ? 610 + 60 * w.S : 3 * pl.NX) + 9000) +
+                             (long long)(pl.xt_bytes / 2000) + (long long)(pl.part_bytes / 900) + 6000;
+    return cycles * 10 / 19;
+}
+
 size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count) {
     GmPlan pl;
     gm_plan(w, M, sm_count, &pl);
@@ -802,6 +813,9 @@ int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half*
     GmPlan pl;
     gm_plan(w, M, di.sm_count, &pl);
     if (pl.xt_bytes + pl.part_bytes > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
+    if (linear_pair_supported(x, Kin, w, y, M) &&
+        linear_pair_ns(w, M, di.sm_count, ws->device, ws->dyn_bytes) < gm_ns(w, pl, di.sm_count))
+        return launch_linear_pair(x, Kin, w, bias, y, M, ws->status, ws->dyn, ws->dyn_bytes, di.sm_count, ws->device, st);
     __half* xt = reinterpret_cast<__half*>(ws->dyn);
     {
         const size_t nblk = ((size_t)pl.MT * pl.NX / 8 * (w.K / 64) + 7) / 8;

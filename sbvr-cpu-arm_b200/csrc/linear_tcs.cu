@@ -917,19 +917,9 @@ size_t linear_tcs_workspace_bytes(const PackedW& w, int M, int sm_count) {
 }
 
 // ---- tensor maps of the packed words: uint32 [K/32 rows][N * S], box 8 KS rows x TN * S words
-typedef CUresult (*TsEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-int ts_tensor_map(const PackedW& w, int KS, CUtensorMap* out) {
+int ts_encoder(TsEncodeFn* out) {
     static std::mutex mu;
     static TsEncodeFn encode = nullptr;
-    struct Entry {
-        const void* bvr;
-        int N, K, S, KS, valid;
-        CUtensorMap map;
-    };
-    static Entry cache[64];
     std::lock_guard<std::mutex> lock(mu);
     if (!encode) {
         void* fn = nullptr;
@@ -938,6 +928,22 @@ int ts_tensor_map(const PackedW& w, int KS, CUtensorMap* out) {
         if (!fn || qres != cudaDriverEntryPointSuccess) return SBVR_ERR_UNSUPPORTED;
         encode = reinterpret_cast<TsEncodeFn>(fn);
     }
+    *out = encode;
+    return SBVR_OK;
+}
+
+int ts_tensor_map(const PackedW& w, int KS, CUtensorMap* out) {
+    static std::mutex mu;
+    TsEncodeFn encode;
+    const int rc = ts_encoder(&encode);
+    if (rc) return rc;
+    struct Entry {
+        const void* bvr;
+        int N, K, S, KS, valid;
+        CUtensorMap map;
+    };
+    static Entry cache[64];
+    std::lock_guard<std::mutex> lock(mu);
     const size_t h = (reinterpret_cast<uintptr_t>(w.bvr) >> 8) * 0x9E3779B97F4A7C15ull;
     Entry& e = cache[(h >> 40) & 63];
     if (!(e.valid && e.bvr == w.bvr && e.N == w.N && e.K == w.K && e.S == w.S && e.KS == KS)) {
