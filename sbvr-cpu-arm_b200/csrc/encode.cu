@@ -293,11 +293,11 @@ struct EncGroup {
 
 // This block's share of a group's candidates, the group's values in shared memory; the least key (mse bits << 32 | candidate) below
 // that of `cached` goes to *best.
-template <int S>
+template <int S, int THREADS>
 __device__ __forceinline__ void enc_search(const EncGroup<S>& q, const EncSpace& sp, const __half2* ds, float cached, unsigned long long* best) {
     const unsigned long long start_key = (unsigned long long)__float_as_uint(cached) << 32;
     float bound = cached;
-    for (int c = blockIdx.x * ENC_THREADS + threadIdx.x; c - (int)threadIdx.x < q.total; c += gridDim.x * ENC_THREADS) {
+    for (int c = blockIdx.x * THREADS + threadIdx.x; c - (int)threadIdx.x < q.total; c += gridDim.x * THREADS) {
         float line[S];
         enc_candidate<S>(sp, min(c, q.total - 1), q.ns, q.s_start, q.s_step, q.a0, q.a1, line);
         // sums are formed in the order of the sorted line
@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(ENC_THREADS) encode_search_kernel(const EncSea
     }
     for (int i = threadIdx.x; i < ENC_G / 2; i += ENC_THREADS) ds[i] = reinterpret_cast<const __half2*>(p.data + (size_t)g * ENC_G)[i];
     __syncthreads();
-    enc_search<S>(q, sp, ds, cached, p.best);
+    enc_search<S, ENC_THREADS>(q, sp, ds, cached, p.best);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) last_s = (atomicAdd(p.done, 1u) == gridDim.x - 1) ? 1u : 0u;
@@ -379,12 +379,11 @@ __global__ void __launch_bounds__(ENC_THREADS) encode_search_kernel(const EncSea
 }
 
 // ---------------------------------------------------------------------------------------------
-// Many steps of the walk in one launch.  All blocks are resident (a cooperative launch) and go through a step together: new lines against
-// the undecided groups, the first miss's candidates, and then block 0 alone decides -- it files the winner under a line within 0.01 %
-// of it or a new one, and moves the cut-off -- while the others wait; three meetings of the grid.  1024 x 4096, S = 4: a step takes 54 us, 36
-// of them the search (459 000 candidates, 16 half-rate differences and minima per pair of values, about half of them before the
-// warp's last candidate is out), 13 the update, 4 the decision; with three launches, a synchronisation and the decision in Python
-// per step it took 87.  Whole encoding: 11.3 -> 8.5 ms.
+// Many steps of the walk in one launch.  All blocks are resident (a cooperative launch) and go through a step together, two meetings of the
+// grid each: new lines against the undecided groups; the first miss's candidates.  What becomes of the winner -- it is filed under a line
+// within 0.01 % of it or a new one, and moves the cut-off -- every block decides for itself from the same words; block 0 alone writes it
+// down.  1024 x 4096, S = 4, 16 384 groups, 201 misses of 459 000 candidates each: 11.1 -> 6.2 ms, 50 -> 24 us a step, of them 10 the bounds
+// of the candidates, 5 the two meetings, 4 a group's tables, 2 the first look at it, 1.5 the decision, 1 the new line against the window.
 //
 // The arithmetic of the decisions is the host's: a line's magnitude is the fp32 sum of its |c| in order, rounded to fp16; a difference
 // of lines is rounded to fp32 and then to fp16; the mean of the accepted errors is a sum in double with Neumaier's
@@ -395,11 +394,12 @@ constexpr int ENC_WINDOW = SBVR_ENCODE_WINDOW;                     // accepted e
 
 struct EncCtl {                                    // device memory, all zero before the launch
     unsigned int arrived;
-    int miss, from, n, line0, misses, steps, accepted, stop;
-    int pad;
-    double cutoff;
-    unsigned long long best;
+    unsigned int go;                               // steps that block 0 has seen everyone search: their decisions may be acted on
+    int miss[3];                                   // of step t in slot t % 3: first group that misses
+    float ub[3];                                   // an upper bound of the best candidate's mse
+    unsigned long long best[3];                    // (mse bits << 32 | candidate)
 };
+static_assert(sizeof(EncCtl) <= 64, "sbvr_encode_run_t::ctl");
 struct EncRun {
     EncSearch q;                                   // data, stats, best_mse, best_at, space, NG (the rest is the kernel's own)
     float* best_mse;
@@ -413,111 +413,531 @@ struct EncRun {
     double hist[ENC_WINDOW];
 };
 
-// All blocks meet; false: they did not within about a second of SM clock.
+// Waits until *word, an always growing counter, has reached `want`; false: it has not within about a second of SM clock.
+__device__ __forceinline__ bool enc_reached(const unsigned int* word, unsigned int want) {
+    const long long t0 = clock64();
+    for (;;) {
+        unsigned int v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+        if ((int)(v - want) >= 0) return true;
+        if (clock64() - t0 > 2000000000LL) return false;
+    }
+}
+
+// All blocks meet; false: they did not.
 __device__ __forceinline__ bool enc_meet(EncCtl* c, unsigned int& round) {
     __shared__ int ok_s;
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(&c->arrived, 1u);
-        const unsigned int want = ++round * gridDim.x;
-        const long long t0 = clock64();
-        unsigned int v;
-        int ok = 1;
-        for (;;) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&c->arrived) : "memory");
-            if ((int)(v - want) >= 0) break;
-            if (clock64() - t0 > 2000000000LL) {
-                ok = 0;
-                break;
-            }
-        }
-        __threadfence();
-        ok_s = ok;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&c->arrived) : "memory");
+        ok_s = enc_reached(&c->arrived, ++round * gridDim.x) ? 1 : 0;
     }
     __syncthreads();
     return ok_s != 0;
 }
 
-// Block 0: what becomes of group g.  Returns why the walk stops here (0: it does not).
+// ---- the search of one group by all blocks -----------------------------------------------------------------------------
+// Evaluated value by value a candidate is 2^S fp16 differences and minima per pair of 256 values, and half of its values were
+// needed on average before it was out: 36 us of a step's 50 (459 000 candidates, S = 4; with bounds 10).  Its squared error is much cheaper
+// to BOUND.
+// With the candidate's sums sorted, q_0 <= .. <= q_J, every value v belongs to the sum on its side of the midpoints b_j, and
+//   sum (v - nearest)^2 = sum (v - q_J)^2 - 2 sum_j (q_j+1 - q_j) F(b_j),   F(b) = sum over v of max(b - v, 0),
+// since moving the values below b_j from q_j+1 to q_j gains (v - q_j+1)^2 - (v - q_j)^2 = 2 (q_j+1 - q_j) (b_j - v).  F is convex
+// and piecewise linear: chords over ENC_NB equal intervals lie above it, by count * width / 4 of an interval at most.  So a table of
+// chords gives a lower bound of the error in 2^S - 1 look-ups, and an upper bound with the largest gap of a chord: about 0.8 % below
+// and 6 % above on 256 normal values.  Candidates whose lower bound is above the least upper bound (of the whole grid, as far as known)
+// or above the group's best stored line cannot win; what is left, a handful per block, is evaluated as ever, a warp per candidate.
+//
+// The bounds hold for the evaluated error, not only for the real one.  An evaluated value is fp16(fp16(|v - q|)^2): off by three relative
+// roundings of 2^-11, or by 2^-25 where the square is subnormal; their fp32 sum by 128 roundings of 2^-24.  ENC_REL and ENC_ABS
+// cover them.  The bound's own arithmetic is fp32 on values centred in their range [-R, R], with Rq = max(R, |q|): F is off by at most
+// 4.5e-4 Rq (the prefix sums of 256 values, slope and offset of a chord, the interval's index by 6e-5 of a width), so that twice
+// the sum of gap * F is off by 1.8e-3 Rq^2, its additions by 1.8e-3, the sums in front of it by 6e-4: 4.2e-3 Rq^2 in all, below ENC_EPS.
+constexpr int ENC_WT = 640;                        // threads of the walk's blocks, one per SM (512 and 768: 7.6 ms where 640 take 7.1)
+constexpr int ENC_WARPS = ENC_WT / 32;
+constexpr int ENC_NB = 512;
+constexpr int ENC_SMALL = 64;
+constexpr int ENC_ROUNDS = 5;                      // candidates of a thread between two evaluations
+constexpr int ENC_LIST = ENC_ROUNDS * ENC_WT;
+constexpr int ENC_SCALES = 1024, ENC_AXIS = 2001, ENC_RATIOS = 256, ENC_BIASES = 256;      // most that the tables in shared memory hold
+constexpr float ENC_REL = 1.6e-3f, ENC_ABS = 256.0f / 33554432.0f, ENC_EPS = 1.0f / 128.0f;
+
 template <int S>
-__device__ __forceinline__ int enc_decide(const EncRun& p, const EncGroup<S>& q, const EncSpace& sp, int g, float cached, int& n, int& accepted,
-                                          double* hist, int& hist_n) {
-    __shared__ __half line_s[S];
-    __shared__ float near_s;
-    __shared__ int at_s, state_s;
-    __shared__ float mse_s;
-    if (threadIdx.x == 0) {
-        const unsigned long long key = __ldcg(&p.ctl->best), start_key = (unsigned long long)__float_as_uint(cached) << 32;
-        state_s = key < start_key ? 1 : 0;
-        at_s = 0x7fffffff;
-        if (state_s) {
-            mse_s = __uint_as_float((unsigned int)(key >> 32));
-            float line[S];
-            enc_candidate<S>(sp, (int)(key & 0xffffffffu), q.ns, q.s_start, q.s_step, q.a0, q.a1, line);
+struct EncFast {                                   // shared memory of a block
+    float2 chord[ENC_NB + 2];                      // half the slope, offset; [0] below the values, [ENC_NB + 1] above
+    union {
+        struct {
+            int count[ENC_NB];
+            float sum[ENC_NB];
+        } b;
+        float2 err[ENC_WARPS][ENC_G / 2];
+        float2 own[ENC_WARPS][ENC_G / 2];          // chords of a warp's own group: ENC_OWN + 2 of them
+    };
+    float red[ENC_WARPS][4];
+    float small[ENC_SMALL + 1];                    // sum of v^2 over the values below k / ENC_SMALL of the largest magnitude
+    uint2 list[ENC_LIST];                          // candidate, lower bound
+    int alive[ENC_LIST];
+    int n_list, n_alive;
+    float unit[2][ENC_RATIOS][S], bias[2][ENC_BIASES];         // plain and extended lists
+    float scale[ENC_SCALES], axis[S][ENC_AXIS];    // a group's scales and axes
+};
+
+// Sums of all subsets of line[0 .. S) (magnitudes ascending), ascending, as fp16 values centred at `mid`.  A list L of sums without
+// coefficient c becomes L + min(c, 0) followed by L + max(c, 0); as |c| is at least every magnitude before it, only the ends of the two
+// halves can overlap: one comparison at the third coefficient, a merge of four and four at the fourth.  (Sums are rounded: two that
+// are equal but for that may come out an fp16 step in the wrong order, which is far below what the bounds allow for.)
+__device__ __forceinline__ void enc_cmp(float& a, float& b) {
+    const float lo = fminf(a, b), hi = fmaxf(a, b);
+    a = lo, b = hi;
+}
+template <int S>
+__device__ __forceinline__ void enc_sorted_sums(const float (&line)[S], float mid, float (&v)[1 << S]) {
+    v[0] = 0.0f;
 #pragma unroll
-            for (int i = 0; i < S; ++i)
+    for (int s = 0; s < S; ++s) {
+        const float lo = fminf(line[s], 0.0f), hi = fmaxf(line[s], 0.0f);
 #pragma unroll
-                for (int j = 0; j + 1 < S - i; ++j)
-                    if (fabsf(line[j]) > fabsf(line[j + 1])) {
-                        const float t = line[j];
-                        line[j] = line[j + 1], line[j + 1] = t;
-                    }
-            float mag = 0.0f;
+        for (int j = (1 << s) - 1; j >= 0; --j) v[j + (1 << s)] = v[j] + hi, v[j] += lo;
+        if (s == 2) enc_cmp(v[3], v[4]);
+        if (s == 3) {                              // Batcher's merge of v[4 .. 7] and v[8 .. 11]
+            enc_cmp(v[4], v[8]), enc_cmp(v[5], v[9]), enc_cmp(v[6], v[10]), enc_cmp(v[7], v[11]);
+            enc_cmp(v[6], v[8]), enc_cmp(v[7], v[9]);
+            enc_cmp(v[5], v[6]), enc_cmp(v[7], v[8]), enc_cmp(v[9], v[10]);
+        }
+    }
 #pragma unroll
-            for (int s = 0; s < S; ++s) {
-                if (s && !(fabsf(line[s]) > fabsf(line[s - 1]))) state_s = 2;
-                line_s[s] = __float2half_rn(line[s]);          // (exact: candidates are fp16 values)
-                mag = __fadd_rn(mag, fabsf(line[s]));
+    for (int j = 0; j < (1 << S); j += 2) {
+        const float2 f = __half22float2(__floats2half2_rn(v[j], v[j + 1]));
+        v[j] = f.x - mid, v[j + 1] = f.y - mid;
+    }
+}
+template <int S>
+__device__ __forceinline__ void enc_sort_line(float (&line)[S]) {
+#pragma unroll
+    for (int i = 0; i < S; ++i)
+#pragma unroll
+        for (int j = 0; j + 1 < S - i; ++j)
+            if (fabsf(line[j]) > fabsf(line[j + 1])) {
+                const float t = line[j];
+                line[j] = line[j + 1], line[j + 1] = t;
             }
-            near_s = enc_h(__fmul_rn(enc_h(mag), 0.0001f));
-        }
-    }
-    __syncthreads();
-    const int state = state_s;
-    if (state != 1) return state ? 2 : 0;          // 0: the codebook already has something at least as good
-    for (int i = threadIdx.x; i < n; i += ENC_THREADS) {
-        float mag = 0.0f;
+}
+template <int S>
+__device__ __forceinline__ void enc_line_points(const float (&line)[S], __half2 (&pt)[1 << S]) {
+    __half h[S];
 #pragma unroll
-        for (int s = 0; s < S; ++s) {
-            const float a = __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(p.lines) + (size_t)i * S + s)));
-            mag = __fadd_rn(mag, fabsf(enc_h(__fsub_rn(a, __half2float(line_s[s])))));
+    for (int s = 0; s < S; ++s) h[s] = __float2half_rn(line[s]);       // (exact: candidates are fp16 values)
+    enc_points<S>(h, pt);
+}
+__device__ __forceinline__ float enc_warp_sum(float v) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// The errors of a warp's 256 values (pairs lane, lane + 32, ..), added in the order of an evaluation: even and odd values apart, first to last.
+__device__ __forceinline__ float enc_ordered_mse(const float2 (&f)[4], float2* err, int lane) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) err[lane + 32 * e] = f[e];
+    __syncwarp();
+    float s = 0.0f;
+    if (lane < 2) {
+        const float* x = reinterpret_cast<const float*>(err) + lane;
+#pragma unroll 16
+        for (int i = 0; i < ENC_G / 2; ++i) s += x[2 * i];
+    }
+    __syncwarp();
+    return (__shfl_sync(0xffffffffu, s, 0) + __shfl_sync(0xffffffffu, s, 1)) * (1.0f / ENC_G);
+}
+
+// What enc_candidate makes of a number, from tables in shared memory: scales, axes (a division and five roundings a value) and the lists
+// that all groups share.  Quotients by the lists' lengths are products with the rounded-up reciprocal, exact for numbers below
+// 2^32 / length.
+struct EncLines {
+    int nline, ns;
+    unsigned int by_r, by_ns, by_axis, R, axis;
+    const float *unit, *bias;
+};
+__device__ __forceinline__ unsigned int enc_reciprocal(int d) { return d == 1 ? 0u : 0xffffffffu / (unsigned int)d + 1u; }
+__device__ __forceinline__ unsigned int enc_quotient(unsigned int n, unsigned int reciprocal) { return reciprocal ? __umulhi(n, reciprocal) : n; }
+template <int S>
+__device__ __forceinline__ bool enc_lines_fit(const EncGroup<S>& q, const EncSpace& sp) {
+    return q.total <= (1 << 21) && q.ns <= ENC_SCALES && sp.R <= ENC_RATIOS && sp.B <= ENC_BIASES && sp.per_dim + 1 <= ENC_AXIS;
+}
+template <int S>
+__device__ __forceinline__ void enc_lists_init(EncFast<S>& sm, const EncSpace (&space)[2]) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        for (int i = threadIdx.x; i < min(space[e].R, ENC_RATIOS) * S; i += ENC_WT) sm.unit[e][i / S][i % S] = __half2float(space[e].unit[i]);
+        for (int i = threadIdx.x; i < min(space[e].B, ENC_BIASES); i += ENC_WT) sm.bias[e][i] = __half2float(space[e].bias[i]);
+    }
+}
+template <int S>
+__device__ __forceinline__ EncLines enc_lines_init(EncFast<S>& sm, const EncGroup<S>& q, const EncSpace& sp, bool ext) {
+    const int n = sp.per_dim + 1;
+    for (int i = ENC_WT - 1 - (int)threadIdx.x; i < n * S; i += ENC_WT) {      // (the last threads: the first have the chords to make)
+#pragma unroll
+        for (int s = 0; s < S; ++s)
+            if (i / n == s) sm.axis[s][i % n] = enc_linspace(q.a0[s], q.a1[s], n, i % n);
+    }
+    for (int i = (ENC_WT + ENC_G - 1 - (int)threadIdx.x) % ENC_WT; i < q.ns; i += ENC_WT) sm.scale[i] = enc_h(fmaf(q.s_step, (float)i, q.s_start));
+    EncLines l;
+    l.R = (unsigned int)sp.R, l.ns = q.ns, l.axis = (unsigned int)n, l.nline = sp.B * q.ns * sp.R;
+    l.by_r = enc_reciprocal(sp.R), l.by_ns = enc_reciprocal(q.ns), l.by_axis = enc_reciprocal(n);
+    l.unit = sm.unit[ext ? 1 : 0][0], l.bias = sm.bias[ext ? 1 : 0];
+    return l;
+}
+template <int S>
+__device__ __forceinline__ void enc_line(const EncFast<S>& sm, const EncLines& l, int c, float (&line)[S]) {
+    if (c < l.nline) {
+        const unsigned int bs = enc_quotient((unsigned int)c, l.by_r), r = (unsigned int)c - bs * l.R;
+        const unsigned int b = enc_quotient(bs, l.by_ns), si = bs - b * (unsigned int)l.ns;
+        const float sv = sm.scale[si], bv = l.bias[b];
+#pragma unroll
+        for (int s = 0; s < S; ++s) line[s] = enc_h(bv + enc_h(sv * l.unit[r * S + s]));
+    } else {
+        unsigned int n = (unsigned int)(c - l.nline);
+#pragma unroll
+        for (int s = S - 1; s >= 0; --s) {
+            const unsigned int m = enc_quotient(n, l.by_axis);
+            line[s] = sm.axis[s][n - m * l.axis];
+            n = m;
         }
-        if (enc_h(mag) < near_s) atomicMin(&at_s, i);
+    }
+}
+
+// Whether the bounds' roundings are as above: a range that is neither empty nor where fp16 squares overflow.
+__device__ __forceinline__ bool enc_boundable(const EncStats& st) {
+    return st.d_max - st.d_min > 1e-6f && fmaxf(fabsf(st.d_max), fabsf(st.d_min)) <= 16.0f;
+}
+
+// One lower and one upper bound of a line's squared error (sums over the 256 values, the evaluated ones) by a table of NB chords.
+struct EncTable {
+    float mid, R, inv, total, squares, gap;        // range, sums over the centred values, twice the largest gap between a chord and F
+};
+// Interval of b = b2 / 2: 1 + floor((b + R) / width), 0 below, NB + 1 above.  x is the place in [0, 1] of the table, by a multiply-add that
+// saturates; the nearest whole number to x (NB + 1) is in the lower bits of that plus 2^23.
+template <int NB>
+__device__ __forceinline__ int enc_interval(float b2, float inv) {
+    const float x = __saturatef(fmaf(b2, 0.5f / (NB + 1) * inv, 0.5f));        // (b + R) inv = b inv + NB / 2
+    return __float_as_int(fmaf(x, (float)(NB + 1), 8388608.0f)) - 0x4B000000;
+}
+template <int S, int NB>
+__device__ __forceinline__ float2 enc_bounds(const EncTable& t, const float2* chord, const float (&line)[S]) {
+    constexpr int J = (1 << S) - 1;
+    float v[1 << S];
+    enc_sorted_sums<S>(line, t.mid, v);
+    float acc = 0.0f;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+        const float b2 = v[j] + v[j + 1];
+        const float2 ch = chord[enc_interval<NB>(b2, t.inv)];
+        acc = fmaf(v[j + 1] - v[j], fmaf(ch.x, b2, ch.y), acc);
+    }
+    const float raw = fmaf(-2.0f, acc, fmaf(v[J], fmaf((float)ENC_G, v[J], -2.0f * t.total), t.squares));
+    const float rq = fmaxf(t.R, fmaxf(fabsf(v[0]), fabsf(v[J]))), eps = ENC_EPS * rq * rq;
+    const float high = fmaf(raw + eps + t.gap * (v[J] - v[0]), 1.0f + ENC_REL, ENC_ABS);
+    return make_float2(fmaf(raw, 1.0f - ENC_REL, -eps - ENC_ABS), high < INFINITY && rq < 64.0f ? high : INFINITY);
+}
+
+// This block's share of a group's candidates; `best` and `ub` are the grid's words.
+template <int S>
+__device__ __forceinline__ void enc_search_bounded(EncFast<S>& sm, const EncGroup<S>& q, const EncSpace& sp, const EncStats& st, const __half2* ds,
+                                                   float cached, bool ext, unsigned long long* best, float* ub, EncLines& lines) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    EncTable t;
+    t.mid = 0.5f * (st.d_max + st.d_min), t.R = 0.5f * (st.d_max - st.d_min);
+    const float width = 2.0f * t.R / ENC_NB;
+    t.inv = (float)ENC_NB / (2.0f * t.R);
+    // ---- the tables
+    for (int i = tid; i < ENC_NB; i += ENC_WT) sm.b.count[i] = 0, sm.b.sum[i] = 0.0f;
+    if (tid <= ENC_SMALL) sm.small[tid] = 0.0f;
+    if (tid == 0) sm.n_list = 0, sm.n_alive = 0;
+    const float vabs = fmaxf(fabsf(st.d_max), fabsf(st.d_min)), per_v = (float)ENC_SMALL / vabs;
+    lines = enc_lines_init<S>(sm, q, sp, ext);
+    __syncthreads();
+    float sq = 0.0f;
+    if (tid < ENC_G) {
+        const float d = __half2float(reinterpret_cast<const __half*>(ds)[tid]), v = d - t.mid;
+        atomicAdd(&sm.small[min((int)(fabsf(d) * per_v) + 1, ENC_SMALL)], d * d);
+        const int k = min(max(enc_interval<ENC_NB>(2.0f * v, t.inv) - 1, 0), ENC_NB - 1);
+        atomicAdd(&sm.b.count[k], 1);
+        atomicAdd(&sm.b.sum[k], v);
+        sq = v * v;
     }
     __syncthreads();
-    int at = at_s;
-    const bool append = at == 0x7fffffff;
-    if (append && n >= p.capacity) return 2;
-    if (append) at = n;
+    const bool on = tid < ENC_NB;
+    const float cn = on ? (float)sm.b.count[tid] : 0.0f, cs = on ? sm.b.sum[tid] : 0.0f;
+    float n_in = cn, s_in = cs, top = cn;          // inclusive over the warp's lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float a = __shfl_up_sync(0xffffffffu, n_in, o), b = __shfl_up_sync(0xffffffffu, s_in, o);
+        if (lane >= o) n_in += a, s_in += b;
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    }
+    sq = enc_warp_sum(sq);
+    if (warp == ENC_WARPS - 1) {                   // running sums of small[1 .. ENC_SMALL]
+        float a = sm.small[1 + 2 * lane], b = a + sm.small[2 + 2 * lane], in = b;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float f = __shfl_up_sync(0xffffffffu, in, o);
+            if (lane >= o) in += f;
+        }
+        sm.small[1 + 2 * lane] = in - b + a, sm.small[2 + 2 * lane] = in;
+    }
+    if (lane == 31) sm.red[warp][0] = n_in, sm.red[warp][1] = s_in, sm.red[warp][2] = top, sm.red[warp][3] = sq;
+    __syncthreads();
+    float rank = n_in - cn, below = s_in - cs, largest = 0.0f;
+    t.total = 0.0f, t.squares = 0.0f;
+#pragma unroll
+    for (int i = 0; i < ENC_NB / 32; ++i) {
+        if (i < warp) rank += sm.red[i][0], below += sm.red[i][1];
+        t.total += sm.red[i][1], largest = fmaxf(largest, sm.red[i][2]);
+        if (i < ENC_G / 32) t.squares += sm.red[i][3];
+    }
+    if (on) {
+        const float x0 = fmaf(width, (float)tid, -t.R), x1 = fmaf(width, (float)(tid + 1), -t.R);
+        const float f0 = fmaf(rank, x0, -below), f1 = fmaf(rank + cn, x1, -(below + cs)), slope = (f1 - f0) * t.inv;
+        sm.chord[1 + tid] = make_float2(0.5f * slope, fmaf(-slope, x0, f0));
+    }
+    if (tid == 0) sm.chord[0] = make_float2(0.0f, 0.0f), sm.chord[ENC_NB + 1] = make_float2(0.5f * ENC_G, -t.total);
+    __syncthreads();
+    t.gap = 0.51f * largest * width;               // (a little more than twice count * width / 4)
+
+    // ---- bounds of every candidate, survivors into the list; then the survivors
+    const unsigned long long start_key = (unsigned long long)__float_as_uint(cached) << 32;
+    float bound = cached;                          // mse that a candidate must not exceed
+    const int stride = gridDim.x * ENC_WT;
+    for (int base = (int)blockIdx.x * 32 + warp * 32 * (int)gridDim.x; __syncthreads_or(base < q.total); base += ENC_ROUNDS * stride) {
+        float told = __ldcg(ub);
+        bound = fminf(bound, told);
+#pragma unroll 1
+        for (int i = 0; i < ENC_ROUNDS; ++i) {
+            const int c = base + i * stride + lane;
+            if (c - lane >= q.total) break;
+            float line[S];
+            enc_line<S>(sm, lines, min(c, q.total - 1), line);
+            // Coefficients of one sign: no sum but 0 is nearer to 0 than the smallest, to which values of at most half of it stay.
+            {
+                float lo = fabsf(line[0]);
+                bool plus = true, minus = true;
+#pragma unroll
+                for (int s = 0; s < S; ++s) lo = fminf(lo, fabsf(line[s])), plus = plus && line[s] > 0.0f, minus = minus && line[s] < 0.0f;
+                const float stay = sm.small[(int)fminf(0.499f * lo * per_v, (float)ENC_SMALL)];
+                if (__all_sync(0xffffffffu, (plus || minus) && fmaf(stay, 1.0f - ENC_REL, -ENC_ABS) > bound * (float)ENC_G)) continue;
+            }
+            enc_sort_line<S>(line);
+            const float2 lh = enc_bounds<S, ENC_NB>(t, sm.chord, line);
+            float least = lh.y * (1.0f / ENC_G);
+#pragma unroll
+            for (int o = 16; o; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+            if (least < bound) bound = least;
+            if (lane == 0 && least < told) atomicMin(reinterpret_cast<int*>(ub), __float_as_int(least)), told = least;     // (not negative: ordered like ints)
+            // (a bound that is not a number leaves the candidate to its evaluation)
+            if (c < q.total && !(lh.x > bound * (float)ENC_G)) sm.list[atomicAdd(&sm.n_list, 1)] = make_uint2((unsigned int)c, __float_as_uint(lh.x));
+        }
+        const float told2 = __ldcg(ub);
+        const unsigned long long have = __ldcg(best);
+        __syncthreads();
+        bound = fminf(bound, fminf(told2, __uint_as_float((unsigned int)(have >> 32))));       // (no candidate yet: not a number, which fminf leaves out)
+        const int n_list = sm.n_list;
+        for (int e = tid; e < n_list; e += ENC_WT)
+            if (!(__uint_as_float(sm.list[e].y) > bound * (float)ENC_G)) sm.alive[atomicAdd(&sm.n_alive, 1)] = (int)sm.list[e].x;
+        __syncthreads();
+        const int n_alive = sm.n_alive;
+        if (n_alive <= 8 * ENC_WARPS) {
+            for (int e = warp; e < n_alive; e += ENC_WARPS) {
+                const int c = sm.alive[e];
+                float line[S];
+                __half2 pt[1 << S];
+                enc_line<S>(sm, lines, c, line);
+                enc_sort_line<S>(line);
+                enc_line_points<S>(line, pt);
+                float2 f[4];
+                float sum = 0.0f;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) f[k] = enc_err<S>(ds[lane + 32 * k], pt), sum += f[k].x + f[k].y;
+                sum = enc_warp_sum(sum) * (1.0f / ENC_G);
+                if (sum * (1.0f - 2e-5f) > bound) continue;    // (the sum in another order is off by some 2^-17 at most)
+                const float mse = enc_ordered_mse(f, sm.err[warp], lane);
+                bound = fminf(bound, mse);
+                const unsigned long long key = ((unsigned long long)__float_as_uint(mse) << 32) | (unsigned int)c;
+                if (lane == 0 && key < start_key && key < __ldcg(best)) atomicMin(best, key);
+            }
+        } else {                                   // values so small that the bounds say little: a thread per survivor
+            for (int e0 = warp * 32; e0 < n_alive; e0 += ENC_WT) {
+                const int c = sm.alive[min(e0 + lane, n_alive - 1)];
+                float line[S];
+                __half2 pt[1 << S];
+                enc_line<S>(sm, lines, c, line);
+                enc_sort_line<S>(line);
+                enc_line_points<S>(line, pt);
+                float s0 = 0.0f, s1 = 0.0f;
+                bool alive = e0 + lane < n_alive;
+                for (int i = 0; i < ENC_G / 2; i += 8) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const float2 f = enc_err<S>(ds[i + e], pt);
+                        s0 += f.x, s1 += f.y;
+                    }
+                    if ((s0 + s1) * (1.0f / ENC_G) > bound) alive = false;
+                    if (!__any_sync(0xffffffffu, alive)) break;
+                    if (i % 32 == 24) bound = fminf(bound, __uint_as_float((unsigned int)(__ldcg(best) >> 32)));
+                }
+                if (alive) {
+                    const float mse = (s0 + s1) * (1.0f / ENC_G);
+                    const unsigned long long key = ((unsigned long long)__float_as_uint(mse) << 32) | (unsigned int)c;
+                    if (key < start_key && key < __ldcg(best)) atomicMin(best, key);
+                    bound = fminf(bound, mse);
+                }
+            }
+        }
+        __syncthreads();
+        if (tid == 0) sm.n_list = 0, sm.n_alive = 0;
+    }
+}
+
+// ---- new lines against undecided groups ----------------------------------------------------------------------------------
+// The groups are met in windows of one group per warp (all but one of a block's), which keep their group's values and best line in
+// registers from step to step: only the first group that misses matters, so that the groups behind the window may wait for their
+// lines until the window gets there.  A step compares one line with some 2 800 groups in registers; with every undecided group it read
+// 16 384 rows and took 13 us.  The errors' sum in the order of an evaluation, two chains of 128 additions, is formed only where the
+// sum in another order says that the line may be better.  A new window meets all lines since the walk's start: a warp makes a table of
+// ENC_OWN chords of its group and bounds 32 lines at a time, a lane each (80 us a window of 2 800 groups and 150 lines; 125 one line after
+// the other).
+constexpr int ENC_UWARPS = ENC_WARPS - 1;
+constexpr int ENC_OWN = 126;
+constexpr int ENC_MANY = 8;                        // lines from which the table pays
+static_assert(ENC_OWN + 2 <= ENC_G / 2, "EncFast::own");
+
+// The chords of the group whose values a warp has in d[].
+template <int S>
+__device__ __forceinline__ EncTable enc_own_table(float2* chord, const EncStats& st, const __half2 (&d)[4], int lane) {
+    constexpr int NB = ENC_OWN, PER = (NB + 31) / 32;
+    EncTable t;
+    t.mid = 0.5f * (st.d_max + st.d_min), t.R = 0.5f * (st.d_max - st.d_min);
+    const float width = 2.0f * t.R / NB;
+    t.inv = (float)NB / (2.0f * t.R);
+    for (int i = lane; i < NB + 2; i += 32) chord[i] = make_float2(0.0f, 0.0f);
+    __syncwarp();
+    float sq = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 f = __half22float2(d[k]);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float v = (h ? f.y : f.x) - t.mid;
+            float2* b = chord + 1 + min(max(enc_interval<NB>(2.0f * v, t.inv) - 1, 0), NB - 1);
+            atomicAdd(&b->x, 1.0f);
+            atomicAdd(&b->y, v);
+            sq = fmaf(v, v, sq);
+        }
+    }
+    __syncwarp();
+    float2 mine[PER];
+    float n = 0.0f, sv = 0.0f, top = 0.0f;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        mine[i] = lane * PER + i < NB ? chord[1 + lane * PER + i] : make_float2(0.0f, 0.0f);
+        n += mine[i].x, sv += mine[i].y, top = fmaxf(top, mine[i].x);
+    }
+    float n_in = n, s_in = sv;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float a = __shfl_up_sync(0xffffffffu, n_in, o), b = __shfl_up_sync(0xffffffffu, s_in, o);
+        if (lane >= o) n_in += a, s_in += b;
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    }
+    t.total = __shfl_sync(0xffffffffu, s_in, 31), t.squares = enc_warp_sum(sq), t.gap = 0.51f * top * width;
+    float rank = n_in - n, below = s_in - sv;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int k = lane * PER + i;
+        const float x0 = fmaf(width, (float)k, -t.R), x1 = fmaf(width, (float)(k + 1), -t.R), f0 = fmaf(rank, x0, -below);
+        rank += mine[i].x, below += mine[i].y;
+        const float f1 = fmaf(rank, x1, -below), slope = (f1 - f0) * t.inv;
+        if (k < NB) chord[1 + k] = make_float2(0.5f * slope, fmaf(-slope, x0, f0));
+    }
+    if (lane == 0) chord[0] = make_float2(0.0f, 0.0f), chord[NB + 1] = make_float2(0.5f * ENC_G, -t.total);
+    __syncwarp();
+    return t;
+}
+
+// All blocks, the same decision: what becomes of group g, whose winner is `line` (ascending magnitudes, the same in every thread).
+// Returns why the walk stops here (0: it does not).  `line_s`: the new line, if one is appended; `stored`: line threadIdx.x of the codebook,
+// fetched before the winner was known.
+template <int S>
+__device__ __forceinline__ void enc_stored_line(const __half* lines, int i, unsigned short (&h)[S]) {
+#pragma unroll
+    for (int s = 0; s < S; ++s) h[s] = __ldcg(reinterpret_cast<const unsigned short*>(lines) + (size_t)i * S + s);
+}
+template <int S>
+__device__ __forceinline__ int enc_decide(const EncRun& p, const float (&line)[S], const unsigned short (&stored)[S], int g, unsigned long long key,
+                                          int& n, int& accepted, double* hist, int& hist_n, int& head, __half* line_s, bool& append) {
+    __shared__ int at_s;
+    float mag = 0.0f;
+    bool twice = false;                            // two coefficients of one magnitude
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        if (s) twice = twice || !(fabsf(line[s]) > fabsf(line[s ? s - 1 : 0]));
+        mag = __fadd_rn(mag, fabsf(line[s]));
+    }
+    append = false;
+    if (twice) return 2;
+    const float near = enc_h(__fmul_rn(enc_h(mag), 0.0001f));
+    auto close = [&](const unsigned short (&h)[S]) {
+        float m = 0.0f;
+#pragma unroll
+        for (int s = 0; s < S; ++s) m = __fadd_rn(m, fabsf(enc_h(__fsub_rn(__half2float(__ushort_as_half(h[s])), line[s]))));
+        return enc_h(m) < near;
+    };
+    int at = 0x7fffffff;
+    if ((int)threadIdx.x < n && close(stored)) at = threadIdx.x;
+    for (int i = threadIdx.x + ENC_WT; i < n && at == 0x7fffffff; i += ENC_WT) {
+        unsigned short h[S];
+        enc_stored_line<S>(p.lines, i, h);
+        if (close(h)) at = i;
+    }
+    if (threadIdx.x == 0) at_s = 0x7fffffff;
+    append = !__syncthreads_or(at != 0x7fffffff);
+    if (!append) {
+        if (at != 0x7fffffff) atomicMin(&at_s, at);
+        __syncthreads();
+        at = at_s;
+    } else {
+        if (n >= p.capacity) return 2;
+        at = n;
+    }
+    const float mse = __uint_as_float((unsigned int)(key >> 32));
     if (threadIdx.x == 0) {
-        sbvr_encode_record_t r;
-        r.group = g, r.at = at, r.mse = mse_s;
 #pragma unroll
-        for (int s = 0; s < 4; ++s) r.line[s] = s < S ? __half_as_ushort(line_s[s < S ? s : 0]) : (unsigned short)0;
-        p.records[accepted] = r;
-        if (append)
+        for (int s = 0; s < S; ++s) line_s[s] = __float2half_rn(line[s]);      // (exact: candidates are fp16 values)
+        if (blockIdx.x == 0) {
+            sbvr_encode_record_t r;
+            r.group = g, r.at = at, r.mse = mse;
 #pragma unroll
-            for (int s = 0; s < S; ++s) __stcg(reinterpret_cast<unsigned short*>(p.lines) + (size_t)n * S + s, __half_as_ushort(line_s[s]));
-        // the last `window` accepted errors, the newest behind
-        if (hist_n == p.window) {
-            for (int i = 1; i < hist_n; ++i) hist[i - 1] = hist[i];
-            hist[hist_n - 1] = (double)mse_s;
-        } else {
-            hist[hist_n] = (double)mse_s;
+            for (int s = 0; s < 4; ++s) r.line[s] = s < S ? __half_as_ushort(__float2half_rn(line[s < S ? s : 0])) : (unsigned short)0;
+            p.records[accepted] = r;
+            if (append)
+#pragma unroll
+                for (int s = 0; s < S; ++s) __stcg(reinterpret_cast<unsigned short*>(p.lines) + (size_t)n * S + s, __half_as_ushort(__float2half_rn(line[s])));
         }
     }
-    if (hist_n < p.window) ++hist_n;
+    // the last `window` accepted errors, a ring with the oldest at `head`
+    const int to = hist_n == p.window ? head : (head + hist_n) % p.window;
+    if (threadIdx.x == 0) hist[to] = (double)mse;
+    if (hist_n == p.window) head = (head + 1) % p.window;
+    else ++hist_n;
     if (append) ++n;
     ++accepted;
     __syncthreads();
     return 0;
 }
 
-__device__ __forceinline__ double enc_cutoff(const double* hist, int n, double acceptable) {
+__device__ __forceinline__ double enc_cutoff(const double* hist, int n, int head, int window, double acceptable) {
     double sum = 0.0, c = 0.0;
     for (int i = 0; i < n; ++i) {
-        const double x = hist[i], t = __dadd_rn(sum, x);
+        const double x = hist[head + i < window ? head + i : head + i - window], t = __dadd_rn(sum, x);
         if (fabs(sum) >= fabs(x)) c = __dadd_rn(c, __dadd_rn(__dadd_rn(sum, -t), x));
         else c = __dadd_rn(c, __dadd_rn(__dadd_rn(x, -t), sum));
         sum = t;
@@ -527,147 +947,199 @@ __device__ __forceinline__ double enc_cutoff(const double* hist, int n, double a
     return acceptable > m ? acceptable : m;        // Python's max(m, acceptable): the first unless the second is greater
 }
 
-// Lines [line0, line1) against the undecided groups from `from` on, sixteen groups of a block at a time: a warp makes a group's 256 errors
-// (one 512-byte row per load), then a thread per group adds them in the order of `enc_update`.  With a thread per group throughout
-// -- a row each, a round trip to L2 per sixteen values -- this took 28 us a step for 16 384 groups.
-constexpr int ENC_UG = 16;
 template <int S>
-__device__ __forceinline__ void enc_update_all(const EncRun& p, int from, int line0, int line1, double cutoff) {
-    __shared__ __align__(16) float2 err[ENC_UG][ENC_G / 2 + 1];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int g0 = from + blockIdx.x * ENC_UG; g0 < p.q.NG; g0 += gridDim.x * ENC_UG) {
-        const int g = g0 + (int)threadIdx.x;
-        const bool mine = threadIdx.x < ENC_UG && g < p.q.NG;
-        float best = mine ? __ldcg(p.best_mse + g) : 0.0f;
-        int at = -1;
-        for (int n = line0; n < line1; ++n) {
-            __half line[S];
-            __half2 pt[1 << S];
-#pragma unroll
-            for (int s = 0; s < S; ++s) line[s] = __ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(p.lines) + (size_t)n * S + s));
-            enc_points<S>(line, pt);
-#pragma unroll
-            for (int k = 0; k < ENC_UG / (ENC_THREADS / 32); ++k) {
-                const int j = warp * (ENC_UG / (ENC_THREADS / 32)) + k;
-                if (g0 + j < p.q.NG) {
-                    const uint4 v = __ldg(reinterpret_cast<const uint4*>(p.q.data + (size_t)(g0 + j) * ENC_G) + lane);
-                    const __half2* d = reinterpret_cast<const __half2*>(&v);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) err[j][lane * 4 + e] = enc_err<S>(d[e], pt);
-                }
-            }
-            __syncthreads();
-            if (mine) {
-                float s0 = 0.0f, s1 = 0.0f;
-#pragma unroll 16
-                for (int i = 0; i < ENC_G / 2; ++i) {
-                    const float2 f = err[threadIdx.x][i];
-                    s0 += f.x, s1 += f.y;
-                }
-                const float mse = (s0 + s1) * (1.0f / ENC_G);
-                if (mse < best) best = mse, at = n;
-            }
-            __syncthreads();
-        }
-        if (at >= 0) {
-            __stcg(p.best_mse + g, best);
-            __stcg(p.best_at + g, at);
-        }
-        if (warp == 0) {
-            const unsigned int m = __ballot_sync(0xffffffffu, mine && !((double)best < cutoff));
-            if (m && lane == 0) atomicMin(&p.ctl->miss, g0 + __ffs((int)m) - 1);
-        }
-    }
-}
-
-template <int S>
-__global__ void __launch_bounds__(ENC_THREADS) encode_walk_kernel(const __grid_constant__ EncRun p) {
+__global__ void __launch_bounds__(ENC_WT, 1) encode_walk_kernel(const __grid_constant__ EncRun p) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    EncFast<S>& sm = *reinterpret_cast<EncFast<S>*>(smem);
     __shared__ __align__(16) __half2 ds[ENC_G / 2];
-    __shared__ double hist[ENC_WINDOW];
+    __shared__ double hist[ENC_WINDOW], cutoff_s;
+    __shared__ __half line_s[S];
+    __shared__ int miss_s, go_s;
     EncCtl* c = p.ctl;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, NG = p.q.NG;
     unsigned int round = 0;
-    int n = p.n, misses = p.misses, accepted = 0, steps = 0, hist_n = p.hist_n, from = p.from, line0 = p.line0;      // block 0's are the truth
-    auto publish = [&](int stop) {                 // block 0, one thread
-        const bool warm = n < p.warmup;
-        if (!stop && from >= p.q.NG) stop = SBVR_ENCODE_DONE;
-        if (!stop && !warm && n >= p.capacity) stop = SBVR_ENCODE_FULL;
-        if (!stop && !warm && hist_n == 0) stop = SBVR_ENCODE_CALLER;
-        if (!stop && steps >= p.limit) stop = SBVR_ENCODE_LIMIT;
-        c->from = from, c->n = n, c->line0 = line0, c->misses = misses, c->accepted = accepted;
-        c->cutoff = warm ? 0.0 : (hist_n ? enc_cutoff(hist, hist_n, p.acceptable) : 0.0);
-        c->miss = warm ? from : p.q.NG;
-        c->best = ~0ull;
-        c->stop = stop;
-    };
-    if (blockIdx.x == 0) {
-        for (int i = threadIdx.x; i < hist_n; i += ENC_THREADS) hist[i] = p.hist[i];
-        __syncthreads();
-        if (threadIdx.x == 0) publish(0);
-    }
+    int n = p.n, misses = p.misses, accepted = 0, steps = 0, hist_n = p.hist_n, head = 0, from = p.from;
+    const int rest = p.line0;                      // lines that the groups behind the window have met
+    int base = from, end = from, met_lines = rest; // the window and the lines that its groups have met
+    int stop = 0;
+    unsigned int t = 0;                            // steps, of the slots in *c
+    bool appended = false;                         // the last line is in line_s (and may not be in memory yet for all to see)
+    float best = 0.0f;                             // this warp's group of the window: best mse, values
+    __half2 d[4] = {};
+    bool mine = false, loaded = false;
+
+    for (int i = threadIdx.x; i < hist_n; i += ENC_WT) hist[i] = p.hist[i];
+    enc_lists_init<S>(sm, p.q.space);
+    auto clear = [&](int slot) { c->miss[slot] = NG, c->ub[slot] = INFINITY, c->best[slot] = ~0ull; };
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        for (int i = 0; i < 3; ++i) clear(i);
     bool met = enc_meet(c, round);
     while (met) {
-        if (__ldcg(&c->stop)) break;
-        from = __ldcg(&c->from), n = __ldcg(&c->n), line0 = __ldcg(&c->line0), misses = __ldcg(&c->misses);
-        const double cutoff = __ldcg(&c->cutoff);
         const bool warm = n < p.warmup;
-        const int met_from = line0;                // (should the blocks not meet: lines that not every group has met)
+        if (from >= NG) stop = SBVR_ENCODE_DONE;
+        else if (!warm && n >= p.capacity) stop = SBVR_ENCODE_FULL;
+        else if (!warm && hist_n == 0) stop = SBVR_ENCODE_CALLER;
+        else if (steps >= p.limit) stop = SBVR_ENCODE_LIMIT;
+        if (stop) break;
+        const int slot = (int)(t % 3);
+        int g = from;
         if (!warm) {
-            enc_update_all<S>(p, from, line0, n, cutoff);
-            line0 = n;
-        }
-        if (!(met = enc_meet(c, round))) {
-            line0 = met_from;
-            break;
-        }
-        const int g = __ldcg(&c->miss);
-        float cached = INFINITY;
-        bool covered = true;
-        EncGroup<S> q;
-        bool ext = warm;
-        if (g < p.q.NG) {
-            if (!warm) cached = __ldcg(p.best_mse + g);
-            ext = warm || (double)(g - misses) / (double)(g + 1) > 0.6;
-            covered = q.init(p.q.stats[g], p.q.space[ext ? 1 : 0], ext);
-            if (covered) {
-                for (int i = threadIdx.x; i < ENC_G / 2; i += ENC_THREADS) ds[i] = reinterpret_cast<const __half2*>(p.q.data + (size_t)g * ENC_G)[i];
-                __syncthreads();
-                enc_search<S>(q, p.q.space[ext ? 1 : 0], ds, cached, &c->best);
+            if (from >= end) base = from, end = (int)min((long long)NG, (long long)from + (long long)gridDim.x * ENC_UWARPS), met_lines = rest, loaded = false;
+            const int mg = base + (int)blockIdx.x * ENC_UWARPS + warp;
+            if (!loaded) {
+                mine = warp < ENC_UWARPS && mg < end;
+                if (mine) {
+                    best = __ldcg(p.best_mse + mg);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) d[k] = reinterpret_cast<const __half2*>(p.q.data + (size_t)mg * ENC_G)[lane + 32 * k];
+                }
+                loaded = true;
+            }
+            if (threadIdx.x == 0) miss_s = NG;
+            if (warp == ENC_UWARPS && lane == 0) cutoff_s = enc_cutoff(hist, hist_n, head, p.window, p.acceptable);
+            if (mine && mg >= from) {
+                int at = -1;
+                auto line_of = [&](int l, __half (&line)[S]) {
+#pragma unroll
+                    for (int s = 0; s < S; ++s)
+                        line[s] = appended && l == n - 1 ? line_s[s]
+                                                         : __ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(p.lines) + (size_t)l * S + s));
+                };
+                auto meet_line = [&](int l) {
+                    __half line[S];
+                    __half2 pt[1 << S];
+                    line_of(l, line);
+                    enc_points<S>(line, pt);
+                    float2 f[4];
+                    float sum = 0.0f;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) f[k] = enc_err<S>(d[k], pt), sum += f[k].x + f[k].y;
+                    sum = enc_warp_sum(sum) * (1.0f / ENC_G);
+                    if (sum * (1.0f - 2e-5f) > best) return;
+                    const float mse = enc_ordered_mse(f, sm.err[warp], lane);
+                    if (mse < best) best = mse, at = l;
+                };
+                const EncStats own = n - met_lines >= ENC_MANY ? p.q.stats[mg] : EncStats{0.0f, 0.0f, 0.0f, 0.0f};
+                if (enc_boundable(own)) {
+                    // (the table lies where enc_ordered_mse puts its errors: the lines that may be better are noted first)
+                    for (int l0 = met_lines; l0 < n; l0 += 32 * 32) {
+                        const EncTable table = enc_own_table<S>(sm.own[warp], own, d, lane);
+                        unsigned int maybe = 0;        // lane k: of lines l0 + 32 k ..
+                        float bound = best;
+                        const int last = min(32, (n - l0 + 31) / 32);
+#pragma unroll 1
+                        for (int k = 0; k < last; ++k) {
+                            const int l = l0 + 32 * k + lane;
+                            __half line[S];
+                            float lf[S];
+                            line_of(min(l, n - 1), line);
+#pragma unroll
+                            for (int s = 0; s < S; ++s) lf[s] = __half2float(line[s]);
+                            const float2 lh = enc_bounds<S, ENC_OWN>(table, sm.own[warp], lf);
+                            float least = lh.y * (1.0f / ENC_G);
+#pragma unroll
+                            for (int o = 16; o; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+                            bound = fminf(bound, least);
+                            const unsigned int m = __ballot_sync(0xffffffffu, l < n && !(lh.x > bound * (float)ENC_G));
+                            if (lane == k) maybe = m;
+                        }
+                        __syncwarp();
+#pragma unroll 1
+                        for (int k = 0; k < last; ++k)
+#pragma unroll 1
+                            for (unsigned int m = __shfl_sync(0xffffffffu, maybe, k); m; m &= m - 1) meet_line(l0 + 32 * k + __ffs((int)m) - 1);
+                    }
+                } else {
+                    for (int l = met_lines; l < n; ++l) meet_line(l);
+                }
+                if (at >= 0 && lane == 0) {
+                    __stcg(p.best_mse + mg, best);
+                    __stcg(p.best_at + mg, at);
+                }
+            }
+            met_lines = n;
+            appended = false;
+            __syncthreads();
+            if (mine && mg >= from && lane == 0 && !((double)best < cutoff_s)) atomicMin(&miss_s, mg);
+            __syncthreads();
+            if (threadIdx.x == 0 && miss_s < NG) atomicMin(&c->miss[slot], miss_s);
+            if (!(met = enc_meet(c, round))) break;
+            g = __ldcg(&c->miss[slot]);
+            // everyone has read the words of the step before: its slot is that of the step after the next
+            if (blockIdx.x == 0 && threadIdx.x == 0) clear((int)((t + 2) % 3));
+            if (g >= NG) {                         // every group of the window is served
+                from = end;
+                ++t;
+                continue;
             }
         }
-        if (!(met = enc_meet(c, round))) {
-            line0 = met_from;
+        const float cached = warm ? INFINITY : __ldcg(p.best_mse + g);
+        // extended search while the codebook serves well: hits / seen > 0.6
+        const bool ext = warm || (double)(g - misses) / (double)(g + 1) > 0.6;
+        const EncSpace& sp = p.q.space[ext ? 1 : 0];
+        const EncStats st = p.q.stats[g];
+        EncGroup<S> q;
+        if (!q.init(st, sp, ext)) {
+            stop = SBVR_ENCODE_CALLER;
+            from = g;                              // (every group in front of it is served)
             break;
         }
-        if (blockIdx.x == 0) {
-            int stop = 0;
-            if (g >= p.q.NG) stop = SBVR_ENCODE_DONE;
-            else if (!covered) stop = SBVR_ENCODE_CALLER;
-            else if (enc_decide<S>(p, q, p.q.space[ext ? 1 : 0], g, cached, n, accepted, hist, hist_n)) stop = SBVR_ENCODE_CALLER;
-            else ++misses, ++steps, from = g + 1;
-            if (stop == SBVR_ENCODE_CALLER) from = g;          // (every group in front of it is served)
-            if (threadIdx.x == 0) publish(stop);
+        for (int i = threadIdx.x; i < ENC_G / 2; i += ENC_WT) ds[i] = reinterpret_cast<const __half2*>(p.q.data + (size_t)g * ENC_G)[i];
+        __syncthreads();
+        unsigned short stored[S] = {};
+        if ((int)threadIdx.x < n) enc_stored_line<S>(p.lines, threadIdx.x, stored);
+        if (appended && (int)threadIdx.x == n - 1)             // (of the decision before, with no meeting since: while warming up)
+#pragma unroll
+            for (int s = 0; s < S; ++s) stored[s] = __half_as_ushort(line_s[s]);
+        const bool bounded = enc_boundable(st) && enc_lines_fit<S>(q, sp);
+        EncLines lines;
+        if (bounded) enc_search_bounded<S>(sm, q, sp, st, ds, cached, ext, &c->best[slot], &c->ub[slot], lines);
+        else enc_search<S, ENC_WT>(q, sp, ds, cached, &c->best[slot]);
+        if (!(met = enc_meet(c, round))) break;
+        if (blockIdx.x == 0 && threadIdx.x == 32) {
+            if (warm) clear((int)((t + 2) % 3));
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&c->go), "r"(t + 1u) : "memory");
         }
-        met = enc_meet(c, round);
+        const unsigned long long key = __ldcg(&c->best[slot]);
+        appended = false;
+        if (key < ((unsigned long long)__float_as_uint(cached) << 32)) {       // (else the codebook already has something at least as good)
+            float line[S];
+            if (bounded) enc_line<S>(sm, lines, (int)(key & 0xffffffffu), line);
+            else enc_candidate<S>(sp, (int)(key & 0xffffffffu), q.ns, q.s_start, q.s_step, q.a0, q.a1, line);
+            enc_sort_line<S>(line);
+            if (enc_decide<S>(p, line, stored, g, key, n, accepted, hist, hist_n, head, line_s, appended)) {
+                stop = SBVR_ENCODE_CALLER;
+                from = g;
+                break;
+            }
+        }
+        ++misses, ++steps, ++t, from = g + 1;
+        // Nobody acts on a decision that block 0, for want of a meeting, has not taken.
+        if (threadIdx.x == 0) go_s = blockIdx.x == 0 || enc_reached(&c->go, t) ? 1 : 0;
+        __syncthreads();
+        met = go_s != 0;
     }
-    // Blocks that have not met -- another stream's kernel keeps some from running -- leave the walk at the last decision: block 0 decides only
-    // when all have searched, and a line that a group meets a second time changes nothing.
+    // Blocks that have not met -- another stream's kernel keeps some from running -- leave the walk at the last decision, with the lines that
+    // every group has met: a line that a group meets a second time changes nothing.
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        p.outcome[0] = met ? __ldcg(&c->stop) : SBVR_ENCODE_TIMEOUT;
-        p.outcome[1] = from, p.outcome[2] = n, p.outcome[3] = line0, p.outcome[4] = misses, p.outcome[5] = accepted;
+        p.outcome[0] = met ? stop : SBVR_ENCODE_TIMEOUT;
+        p.outcome[1] = from, p.outcome[2] = n, p.outcome[3] = met && end >= NG ? met_lines : rest, p.outcome[4] = misses, p.outcome[5] = accepted;
     }
 }
 
 template <int S>
 static int encode_run(const EncRun& r, int sm_count, cudaStream_t st) {
     int per_sm = 0;
-    SBVR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, encode_walk_kernel<S>, ENC_THREADS, 0));
+    static SmemOnce once;
+    const int smem = (int)sizeof(EncFast<S>), rc = set_max_smem_once(once, encode_walk_kernel<S>, smem);
+    if (rc) return rc;
+    SBVR_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, encode_walk_kernel<S>, ENC_WT, smem));
     if (per_sm < 1) return SBVR_ERR_UNSUPPORTED;
-    if (per_sm > 8) per_sm = 8;
     EncRun copy = r;
     void* args[] = {&copy};
     SBVR_CUDA_TRY(cudaMemsetAsync(r.ctl, 0, sizeof(EncCtl), st));
-    SBVR_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(encode_walk_kernel<S>), dim3(per_sm * sm_count), dim3(ENC_THREADS),
-                                              args, 0, st));
+    SBVR_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(encode_walk_kernel<S>), dim3(sm_count), dim3(ENC_WT),
+                                              args, (size_t)smem, st));
     SBVR_CUDA_TRY(cudaStreamSynchronize(st));
     return SBVR_OK;
 }
