@@ -111,23 +111,27 @@ inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
-// cudaFuncSetAttribute(MaxDynamicSharedMemorySize) once per device for one kernel instantiation: the caller keeps one
+// cudaFuncSetAttribute (MaxDynamicSharedMemorySize for the second) once per device for one kernel instantiation: the caller keeps one
 // static SmemOnce per instantiation.  Safe from several host threads and with several devices in turn.
 struct SmemOnce {
     std::mutex mu;
     bool done[64] = {false};
 };
 template <typename Kernel>
-inline int set_max_smem_once(SmemOnce& once, Kernel kernel, int bytes) {
+inline int set_attribute_once(SmemOnce& once, Kernel kernel, cudaFuncAttribute attribute, int value) {
     int dev = 0;
     SBVR_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) return SBVR_ERR_BAD_ARG;
     std::lock_guard<std::mutex> lock(once.mu);
     if (!once.done[dev]) {
-        SBVR_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        SBVR_CUDA_TRY(cudaFuncSetAttribute(kernel, attribute, value));
         once.done[dev] = true;
     }
     return SBVR_OK;
+}
+template <typename Kernel>
+inline int set_max_smem_once(SmemOnce& once, Kernel kernel, int bytes) {
+    return set_attribute_once(once, kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 int launch_decode(const PackedW& w, __half* W, int ldw, int Kout, cudaStream_t st);
