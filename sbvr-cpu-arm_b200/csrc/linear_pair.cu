@@ -704,19 +704,9 @@ static int gp_launch(const CUtensorMap& xmap, const GpParams& p, int pairs, cuda
 
 int launch_linear_pair(const __half* x, int Kin, const PackedW& w, const __half* bias, __half* y, int M, unsigned int* status,
                        char* scratch, size_t scratch_bytes, int sm_count, int device, cudaStream_t st) {
-    TsEncodeFn encode;
-    int rc = ts_encoder(&encode);
-    if (rc) return rc;
     CUtensorMap xmap;
-    const cuuint64_t dims[2] = {(cuuint64_t)Kin, (cuuint64_t)M}, strides[1] = {(cuuint64_t)Kin * 2};
-    const cuuint32_t box[2] = {64u, 128u}, estr[2] = {1u, 1u};
-    const CUresult r = encode(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(x), dims, strides, box, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        g_last_cuda_error = (int)r;
-        return SBVR_ERR_CUDA;
-    }
+    int rc = ts_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, CU_TENSOR_MAP_SWIZZLE_128B, x, (size_t)M, (size_t)Kin, (size_t)Kin * 2, 128, 64);
+    if (rc) return rc;
     const GpPlan pl = gp_plan(w, M, sm_count, device, scratch_bytes);
     GpParams p;
     p.bvr = w.bvr, p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status;

@@ -917,26 +917,47 @@ size_t linear_tcs_workspace_bytes(const PackedW& w, int M, int sm_count) {
 }
 
 // ---- tensor maps of the packed words: uint32 [K/32 rows][N * S], box 8 KS rows x TN * S words
-int ts_encoder(TsEncodeFn* out) {
+int ts_map_2d(CUtensorMap* out, CUtensorMapDataType type, CUtensorMapSwizzle swizzle, const void* base, size_t rows, size_t cols,
+              size_t pitch, int box_rows, int box_cols) {
+    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
     static std::mutex mu;
-    static TsEncodeFn encode = nullptr;
-    std::lock_guard<std::mutex> lock(mu);
-    if (!encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        SBVR_CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
-        if (!fn || qres != cudaDriverEntryPointSuccess) return SBVR_ERR_UNSUPPORTED;
-        encode = reinterpret_cast<TsEncodeFn>(fn);
+    static EncodeFn found = nullptr;
+    EncodeFn encode;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!found) {
+            void* fn = nullptr;
+            cudaDriverEntryPointQueryResult qres;
+            SBVR_CUDA_TRY(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
+            if (!fn || qres != cudaDriverEntryPointSuccess) return SBVR_ERR_UNSUPPORTED;
+            found = reinterpret_cast<EncodeFn>(fn);
+        }
+        encode = found;
     }
-    *out = encode;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, estr[2] = {1u, 1u};
+    auto call = [&]() {
+        return encode(out, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = call();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {         // a thread that has not used the runtime yet: a driver call finds no context there
+        int device;
+        SBVR_CUDA_TRY(cudaGetDevice(&device));
+        SBVR_CUDA_TRY(cudaSetDevice(device));
+        r = call();
+    }
+    if (r != CUDA_SUCCESS) {
+        g_last_cuda_error = (int)r;
+        return SBVR_ERR_CUDA;
+    }
     return SBVR_OK;
 }
 
 int ts_tensor_map(const PackedW& w, int KS, CUtensorMap* out) {
     static std::mutex mu;
-    TsEncodeFn encode;
-    const int rc = ts_encoder(&encode);
-    if (rc) return rc;
     struct Entry {
         const void* bvr;
         int N, K, S, KS, valid;
@@ -947,18 +968,10 @@ int ts_tensor_map(const PackedW& w, int KS, CUtensorMap* out) {
     const size_t h = (reinterpret_cast<uintptr_t>(w.bvr) >> 8) * 0x9E3779B97F4A7C15ull;
     Entry& e = cache[(h >> 40) & 63];
     if (!(e.valid && e.bvr == w.bvr && e.N == w.N && e.K == w.K && e.S == w.S && e.KS == KS)) {
-        const cuuint64_t dims[2] = {(cuuint64_t)w.N * w.S, (cuuint64_t)w.K / 32};
-        const cuuint64_t strides[1] = {(cuuint64_t)w.N * w.S * 4};
-        const cuuint32_t box[2] = {(cuuint32_t)(ts_tn(w.S) * w.S), (cuuint32_t)(8 * KS)};
-        const cuuint32_t estr[2] = {1u, 1u};
-        const CUresult r = encode(&e.map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<uint32_t*>(w.bvr), dims, strides, box,
-                                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) {
-            e.valid = 0;
-            g_last_cuda_error = (int)r;
-            return SBVR_ERR_CUDA;
-        }
+        e.valid = 0;
+        const int rc = ts_map_2d(&e.map, CU_TENSOR_MAP_DATA_TYPE_UINT32, CU_TENSOR_MAP_SWIZZLE_NONE, w.bvr, (size_t)w.K / 32, (size_t)w.N * w.S,
+                                 (size_t)w.N * w.S * 4, 8 * KS, ts_tn(w.S) * w.S);
+        if (rc) return rc;
         e.bvr = w.bvr, e.N = w.N, e.K = w.K, e.S = w.S, e.KS = KS, e.valid = 1;
     }
     *out = e.map;

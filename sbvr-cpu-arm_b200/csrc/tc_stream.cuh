@@ -18,11 +18,9 @@ __host__ __device__ constexpr int ts_sp(int S) { return S == 2 ? 2 : 4; }       
 __host__ __device__ constexpr int ts_tn(int S) { return 128 / ts_sp(S); }            // output rows per tile
 __host__ __device__ inline int ts_round_up(int v, int a) { return (v + a - 1) / a * a; }
 
-// The driver's cuTensorMapEncodeTiled
-typedef CUresult (*TsEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-int ts_encoder(TsEncodeFn* out);
+// Tensor map of a matrix of rows x cols elements, its rows `pitch` bytes apart; boxes of box_rows x box_cols, zeros past the end.
+int ts_map_2d(CUtensorMap* out, CUtensorMapDataType type, CUtensorMapSwizzle swizzle, const void* base, size_t rows, size_t cols,
+              size_t pitch, int box_rows, int box_cols);
 // Tensor map of the packed words, uint32 [K/32 rows][N * S], box 8 KS rows x TN * S words (cached per weight).
 int ts_tensor_map(const PackedW& w, int KS, CUtensorMap* out);
 

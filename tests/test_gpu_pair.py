@@ -87,3 +87,24 @@ def test_calls_that_the_copies_cannot_serve(case):
     y = sbvr.linear(x, w, None, out=out) if out is not None else sbvr.linear(x, w)
     rel, top = errors(y, x, w)
     assert rel <= 5e-4 and top <= 3e-3, (rel, top)
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 14336, 512), (40, 512, 2048)])
+def test_first_call_of_a_thread(M, N, K):
+    """The first thing that a thread does on the GPU: the tensor map of x is a driver call, which needs the thread's context."""
+    import threading
+    import sbvr
+    w, g = packed(N, K, 4, 256, "u16", 11)
+    x = torch.randn((M, K), device="cuda", generator=g).half()
+    want, out = sbvr.linear(x, w), torch.empty((M, N), dtype=torch.float16, device="cuda")
+    same = []
+
+    def work():
+        sbvr.linear(x, w, out=out)
+        same.append(torch.equal(out, want))
+
+    torch.cuda.synchronize()
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert same == [True]
