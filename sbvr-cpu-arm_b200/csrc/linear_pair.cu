@@ -41,13 +41,18 @@ constexpr int GP_PWARP = GP_XWARP + 1;             // fetches packed words and c
 constexpr int GP_THREADS = (GP_PWARP + 1) * 32;
 constexpr int GP_WSLOTS = 4;                       // decoded 128 x 64 weight tiles
 constexpr int GP_ASLOTS = 3;                       // activations of a stage: a box of 128 x 64 per block
-constexpr int GP_PSLOTS = 3;                       // packed words and coefficients of a group of 128 weight rows
+// Packed words and coefficients of a group of 128 weight rows: 8 x S words (G = 128: 4 x S) and four halves per row.  With G = 128 a
+// decoder warpgroup uses every second group: an even number of slots, so that it meets every phase of those that it waits on (the parity of a
+// phase tells it only from the next).
+constexpr int GP_PSLOTS = 4;                       // at most
+__host__ __device__ constexpr int gp_pslots(int spg) { return spg == 4 ? 3 : 4; }
+__host__ __device__ constexpr uint32_t gp_coef_at(int spg) { return 128 * 2 * spg * 16; }
+__host__ __device__ constexpr uint32_t gp_pbytes(int spg) { return gp_coef_at(spg) + 128 * 8; }
 constexpr uint32_t GP_SLOT = 128 * 64 * 2;         // bytes of a decoded tile, of an activation box
-constexpr uint32_t GP_PBYTES = 128 * 8 * 16 + 128 * 8;         // 8 x S words and four halves per row
 constexpr int GP_OUT_PITCH = 80;                   // bytes between staged rows of 32 results: 16-byte accesses without bank conflicts
 constexpr int GP_HDR = 1024;
-constexpr int GP_SMEM = GP_HDR + (GP_WSLOTS + 2 * GP_ASLOTS) * (int)GP_SLOT + GP_PSLOTS * (int)GP_PBYTES + 4 * 32 * GP_OUT_PITCH;
-static_assert(GP_SMEM <= 227 * 1024, "shared memory");
+constexpr int GP_SMEM = GP_HDR + (GP_WSLOTS + 2 * GP_ASLOTS) * (int)GP_SLOT + gp_pslots(4) * (int)gp_pbytes(4) + 4 * 32 * GP_OUT_PITCH;
+static_assert(GP_SMEM <= 227 * 1024 && gp_pslots(2) * gp_pbytes(2) <= gp_pslots(4) * gp_pbytes(4), "shared memory");
 constexpr int GP_TURN = 12;                        // stages after which both rings are at their start again, that of the activations in its first phase
 static_assert(GP_TURN % GP_WSLOTS == 0 && GP_TURN % (2 * GP_ASLOTS) == 0, "the issuer's unrolled stages");
 
@@ -221,7 +226,8 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
     volatile int* dead = reinterpret_cast<volatile int*>(smem + 512);
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(smem + 516);
     const uint32_t w_ring = sbase + GP_HDR, a_ring = w_ring + GP_WSLOTS * GP_SLOT, p_ring = a_ring + 2 * GP_ASLOTS * GP_SLOT,
-                   out_s = p_ring + GP_PSLOTS * GP_PBYTES;
+                   out_s = p_ring + gp_pslots(4) * gp_pbytes(4);
+    const uint32_t pslots = gp_pslots(p.spg), pbytes = gp_pbytes(p.spg), coef_at = gp_coef_at(p.spg);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = gp_cta_rank();
     const int pair = (int)blockIdx.x >> 1, pairs = (int)gridDim.x >> 1;
@@ -467,10 +473,10 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
                 if (!gp_wait(p_empty + 8 * slot, ph, dead)) ok = false;
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                const uint32_t dst = p_ring + slot * GP_PBYTES;
+                const uint32_t dst = p_ring + slot * pbytes;
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(dst + 128 * 8 * 16 + (lane + 32 * i) * 8), "r"(c0[i].x), "r"(c0[i].y) : "memory");
+                    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(dst + coef_at + (lane + 32 * i) * 8), "r"(c0[i].x), "r"(c0[i].y) : "memory");
                 __syncwarp();
                 if (lane == 0)
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(p_full + 8 * slot), "r"(2 * spg * bytes) : "memory");
@@ -480,7 +486,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
                                      dst + lane * (uint32_t)(half * S * 4)),
                                  "l"(src + (size_t)(2 * g * spg + lane) * N * S), "r"(bytes), "r"(p_full + 8 * slot)
                                  : "memory");
-                if (++slot == GP_PSLOTS) slot = 0, ph ^= 1u;
+                if (++slot == (int)pslots) slot = 0, ph ^= 1u;
             }
         }
         if (!ok && lane == 0) {                    // copies that were issued land before the pair leaves
@@ -498,16 +504,16 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
         const int spg_shift = p.spg == 4 ? 2 : 1;
         const bool row_on = r < half;              // (the others only arrive)
         for (int it = wg; it < stages; it += GP_DWGS) {
-            const int slot = it % GP_WSLOTS, group = it >> spg_shift, pslot = group % GP_PSLOTS, in = it & (p.spg - 1);
-            const uint32_t dst = w_ring + slot * GP_SLOT + r * 16, src = p_ring + pslot * GP_PBYTES;
-            if (ok && !gp_wait(p_full + 8 * pslot, (uint32_t)(group / GP_PSLOTS) & 1u, dead)) ok = false;
+            const int slot = it % GP_WSLOTS, group = it >> spg_shift, turn = p.spg == 4 ? group / 3 : group / 4, pslot = group - turn * (int)pslots, in = it & (p.spg - 1);
+            const uint32_t dst = w_ring + slot * GP_SLOT + r * 16, src = p_ring + pslot * pbytes;
+            if (ok && !gp_wait(p_full + 8 * pslot, (uint32_t)turn & 1u, dead)) ok = false;
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             uint32_t w[2][S];
             unsigned short c[4] = {};
             if (row_on) {
                 uint32_t cx, cy;
-                asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(cx), "=r"(cy) : "r"(src + 128 * 8 * 16 + r * 8) : "memory");
+                asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(cx), "=r"(cy) : "r"(src + coef_at + r * 8) : "memory");
                 c[0] = (unsigned short)cx, c[1] = (unsigned short)(cx >> 16), c[2] = (unsigned short)cy, c[3] = (unsigned short)(cy >> 16);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {

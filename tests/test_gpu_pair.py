@@ -37,6 +37,7 @@ def errors(y, x, w, b=None):
     (257, 28672, 256, 4, 256, "u16", False),       # one row in the second block; a single group
     (512, 28672, 256, 2, 256, "u8", True),         # both blocks full
     (513, 28672, 384, 3, 128, "direct", False),    # one row in the third block, an odd number of groups of 128
+    (600, 14336, 2176, 4, 128, "u16", True),       # 17 groups of 128: every slot of their ring several times
     (768, 14464, 512, 4, 256, "direct", True),     # items of one block; 113 tiles of 128 rows, a last item that is narrower
     (1000, 9600, 1536, 3, 256, "u16", True),
     (1030, 13440, 2048, 2, 128, "u8", False),
