@@ -67,6 +67,7 @@ struct GpParams {
     int vec;                     // lines of S = 4 (2) can be read as 8 (4) bytes
     int n;                       // weight rows of an item (multiple of 32)
     int MT, MB;                  // activation tiles of 512 rows, blocks of 256 rows
+    int MF, full;                // activation tiles that are dealt out together, and their items: see gp_m
     int NG, spg;                 // coefficient groups along K, 64-k stages of each
     int items, steps;            // work items; steps of an item in the split over the pairs: NG, or 1 where items stay whole
     float* part;                 // sums of items that several pairs work on: [pair + left-over item][512 x n], see gp_part
@@ -174,6 +175,11 @@ struct GpSegs {
     // number of the part that the pair's sums of segment q are (a left-over item that it does not do alone), or -1
     __device__ __forceinline__ int part(int q) const { return sg.shared(q) ? pair + sg.rt_first + q : -1; }
 };
+// Activation tile and first weight row of an item.  Where the last activation tile has one block, its items, which are half as long, come
+// after all others: next to the others of the same weight rows they fell to the same
+// pairs every time (1100 x 14336 x 4096: 134 us, now 115).
+__device__ __forceinline__ int gp_m(const GpParams& p, int item) { return item < p.full ? item % p.MF : p.MF; }
+__device__ __forceinline__ int gp_n0(const GpParams& p, int item) { return (item < p.full ? item / p.MF : item - p.full) * p.n; }
 // A part holds the sums of 32 activation rows x 32 weight rows one after the other, each as eight runs of one float4 per activation
 // row: float4 i of row r is columns 4 i .. 4 i + 3.  `unit`: (block, CTA of the pair, warp), `chunk`: columns 32 chunk ..
 __device__ __forceinline__ float4* gp_part(float* part, int n, int number, int unit, int chunk) {
@@ -271,7 +277,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
     bool ok = tbase == 0;                          // (an allocation of all columns can only start at column 0)
 
     // blocks of 256 activation rows of an item: the last tile may have one
-    auto blocks_of = [&](int item) { return min(2, p.MB - 2 * (item % p.MT)); };
+    auto blocks_of = [&](int item) { return min(2, p.MB - 2 * gp_m(p, item)); };
 
     if (warp == GP_XWARP) {
         // ------------------------------ activation producer ------------------------------
@@ -281,7 +287,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
             uint32_t ph = 1;
             const uint32_t bar0 = gp_mapa(a_full, 0);
             for (int q = 0; q < sg.count() && ok; ++q) {
-                const int item = sg.item(q), nb = blocks_of(item), m0 = (item % p.MT) * 512 + (int)rank * 128, s1 = sg.g1(q) * p.spg;
+                const int item = sg.item(q), nb = blocks_of(item), m0 = gp_m(p, item) * 512 + (int)rank * 128, s1 = sg.g1(q) * p.spg;
                 for (int ks = sg.g0(q) * p.spg; ks < s1; ++ks) {
                     if (!gp_wait(a_empty + 8 * slot, ph, dead)) {
                         ok = false;
@@ -370,14 +376,14 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
         const uint32_t free0 = gp_mapa(d_empty, 0);
         uint32_t ph[2] = {0, 0};
         for (int q = 0; q < sg.count(); ++q) {
-            const int item = sg.item(q), nb = blocks_of(item), n0 = (item / p.MT) * p.n, part = sg.part(q);
+            const int item = sg.item(q), nb = blocks_of(item), n0 = gp_n0(p, item), part = sg.part(q);
             for (int b = 0; b < nb; ++b) {
                 if (ok && !gp_wait(d_full + 8 * b, ph[b], dead)) ok = false;
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 ph[b] ^= 1u;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const int m0 = (item % p.MT) * 512 + b * 256 + (int)rank * 128 + wl * 32;
+                const int m0 = gp_m(p, item) * 512 + b * 256 + (int)rank * 128 + wl * 32;
                 for (int c = 0; c < p.n; c += 32) {            // (of a last chunk of 16 columns the rest is not stored)
                     uint32_t d[32];
                     gp_ld32(((uint32_t)(wl * 32) << 16) + b * 256 + c, d);
@@ -417,7 +423,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
         auto set_seg = [&](Pos& a) {
             if (a.q >= sg.count()) return;
             a.g = sg.g0(a.q), a.end = sg.g1(a.q);
-            a.n = (sg.item(a.q) / p.MT) * p.n + (int)rank * half + lane;
+            a.n = gp_n0(p, sg.item(a.q)) + (int)rank * half + lane;
         };
         auto next_group = [&](Pos& a) {
             if (++a.g >= a.end) {
@@ -461,7 +467,7 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
         int slot = 0;
         uint32_t ph = 1;
         for (int q = 0; q < sg.count() && ok; ++q) {
-            const int n0 = (sg.item(q) / p.MT) * p.n + (int)rank * half, rows = min(half, N - n0);
+            const int n0 = gp_n0(p, sg.item(q)) + (int)rank * half, rows = min(half, N - n0);
             const uint32_t bytes = rows > 0 ? (uint32_t)(rows * S * 4) : 0u;
             const uint32_t* src = p.bvr + (size_t)n0 * S;
             for (int g = sg.g0(q), g1 = sg.g1(q); g < g1; ++g) {
@@ -639,7 +645,7 @@ __global__ void __launch_bounds__(128) gp_add_kernel(const GpParams p, int pairs
     const int item = sg.rem_tile0 + rt;
     if (item >= p.items) return;
     const int c0 = sg.cta_of((unsigned int)(rt * sg.KBS)), c1 = sg.cta_of((unsigned int)(rt * sg.KBS + sg.KBS - 1));
-    const int m0 = (item % p.MT) * 512 + (unit >> 3) * 256 + (unit & 7) * 32;
+    const int m0 = gp_m(p, item) * 512 + (unit >> 3) * 256 + (unit & 7) * 32;
     if (c0 == c1 || m0 >= p.M) return;             // one pair has done the item alone; rows past the last
     float4 v[8] = {};
     for (int c = c0; c <= c1; ++c) {
@@ -654,7 +660,7 @@ __global__ void __launch_bounds__(128) gp_add_kernel(const GpParams p, int pairs
 #pragma unroll
     for (int i = 0; i < 8; ++i)
         d[4 * i] = __float_as_uint(v[i].x), d[4 * i + 1] = __float_as_uint(v[i].y), d[4 * i + 2] = __float_as_uint(v[i].z), d[4 * i + 3] = __float_as_uint(v[i].w);
-    gp_store(p, d, smem_u32(out[warp]), lane, m0, (item / p.MT) * p.n, chunk * 32);
+    gp_store(p, d, smem_u32(out[warp]), lane, m0, gp_n0(p, item), chunk * 32);
 }
 
 struct GpPlan {
@@ -673,17 +679,22 @@ static GpPlan gp_plan(const PackedW& w, int M, int sm_count, int device, size_t 
     if (sbvr_workspace_bytes(device, M, w.N, w.K, &promised) != SBVR_OK) promised = SBVR_WS_FIXED_BYTES;
     scratch = std::min(scratch, promised - SBVR_WS_FIXED_BYTES);
     const long long pairs = sm_count / 2, MT = (M + 511) / 512, NG = w.K / w.G, stages = w.K / 64;
+    const bool odd = M > 512 && (M - 1) / 256 % 2 == 0;        // the last activation tile has one block
     GpPlan best = {};
     for (int n = 256; n >= 64; n -= 16) {
-        const long long stage = std::max(560, 160 + 20 * w.S + 215 * n / 100);
-        const long long items = (w.N + n - 1) / n * MT, rounds = (items + pairs - 1) / pairs, left = items % pairs;
+        const long long stage = std::max(560, 160 + 20 * w.S + 215 * n / 100), half = std::max(stage * 6 / 10, 150LL + 50 * w.S);
+        const long long NT = (w.N + n - 1) / n, items = NT * MT, full = odd ? items - NT : items, rounds = (items + pairs - 1) / pairs, left = items % pairs;
         if (items > (1 << 20)) continue;
-        GpPlan pl = {n, (int)items, (int)std::min(items, pairs), 1, 0, rounds * (stages * stage + 1500) + 6500};
+        const long long long_ones = (full + pairs - 1) / pairs;                // rounds in which the first pair has an item of two blocks
+        GpPlan pl = {n, (int)items, (int)std::min(items, pairs), 1, 0, stages * (long_ones * stage + (rounds - long_ones) * half) + rounds * 1500 + 6500};
         if (!best.n || pl.ns < best.ns) best = pl;
         if (left * NG < pairs || left * NG * pairs >= (1LL << 32)) continue;
         pl.part_bytes = (size_t)(pairs + left) * 16 * ((n + 31) / 32) * 4096;
         pl.pairs = (int)pairs, pl.steps = (int)NG;
-        pl.ns = (items * stages + pairs - 1) / pairs * stage + (rounds + 1) * 1500 + 9500 + (long long)(pl.part_bytes / 5000);
+        const long long whole = items / pairs, whole_long = std::min(whole, long_ones);
+        pl.ns = stages * (whole_long * stage + (whole - whole_long) * half) +
+                (left * stages + pairs - 1) / pairs * (full > whole * pairs ? stage : half) +              // (cut by steps, long and short)
+                (rounds + 1) * 1500 + 9500 + (long long)(pl.part_bytes / 5000);
         if (pl.part_bytes <= scratch && pl.ns < best.ns) best = pl;
     }
     return best;
@@ -718,7 +729,7 @@ int launch_linear_pair(const __half* x, int Kin, const PackedW& w, const __half*
     p.bvr = w.bvr, p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status;
     p.M = M, p.N = w.N, p.idx_bytes = w.idx_bytes, p.n = pl.n;
     p.vec = !(reinterpret_cast<uintptr_t>(w.coeff) & (2 * w.S - 1));
-    p.MB = (M + 255) / 256, p.MT = (p.MB + 1) / 2, p.NG = w.K / w.G, p.spg = w.G / 64, p.items = pl.items, p.steps = pl.steps;
+    p.MB = (M + 255) / 256, p.MT = (p.MB + 1) / 2, p.MF = p.MB % 2 && p.MT > 1 ? p.MT - 1 : p.MT, p.full = pl.items / p.MT * p.MF, p.NG = w.K / w.G, p.spg = w.G / 64, p.items = pl.items, p.steps = pl.steps;
     p.part = reinterpret_cast<float*>(scratch);
     switch (w.S) {
         case 2: rc = gp_launch<2>(xmap, p, pl.pairs, st); break;
