@@ -67,7 +67,7 @@ SBVR_API unsigned int sbvr_last_timeout_info(int i);
 SBVR_API int sbvr_query(int device, int* sm_count, int* smem_per_block_optin, int* l2_bytes, int* cc_major, int* cc_minor);
 
 /* Scratch memory: the device status word of the bounded waits, the quantised activations and the partial sums of
- * row tiles shared by two CTAs (decode kernel), the re-tiled activations and split-K partial sums (batched kernel),
+ * row tiles shared by two CTAs (decode kernel), padded activations and partial sums of cut tiles (batched kernel),
  * staging buffers of the host-pointer entry point.
  * The reference allocates nothing comparable (its kernels keep everything in registers); it does allocate
  * the output inside the binding (sbvr/kernels/sbvr_ops.cpp:100-101), which here is the caller's job.
@@ -80,8 +80,8 @@ SBVR_API int sbvr_linear_workspace_bytes(int device, const uint32_t* bvr, const 
                                          int C, int M, int N, int K, int S, int G, size_t* bytes);
 SBVR_API int sbvr_workspace_destroy(sbvr_workspace_t* ws);
 /* Bytes to ask sbvr_workspace_create for so that every kernel (and the host-pointer entry point) can serve
- * linears of up to M activation rows on an N x K weight: the batched kernel keeps a re-tiled copy of the
- * activations (M x K fp16, M rounded up to its tile) and, when it splits K, fp32 partial sums.  No reference
+ * linears of up to M activation rows on an N x K weight: the batched kernel keeps a padded copy of
+ * activations whose rows do not start on 16 bytes (M x K fp16, M rounded up to its tile) and fp32 sums of tiles that it cuts.  No reference
  * counterpart (the reference has no scratch). */
 SBVR_API int sbvr_workspace_bytes(int device, int M, int N, int K, size_t* bytes);
 /* Synchronises `stream`, then reads the device status word: SBVR_OK or SBVR_ERR_TIMEOUT. Resets it. */
@@ -146,8 +146,8 @@ SBVR_API int sbvr_linear_f16_host(const void* x_host, const uint32_t* bvr, const
  *     kernel attributes and may encode a tensor map: make such first calls outside stream capture, with that device
  *     current.
  *   - M <= 4 runs on the decode kernel (about 4 K M bytes of activation digits + 150 KB of partial sums: always
- *     fits); larger M runs on the batched tensor-core kernel, whose re-tiled activations (about 2 M K bytes) and
- *     split-K partial sums must fit the array (about 2.9 MB of it): M = 16 at K = 4096 and M = 64 at K = 14336 fit,
+ *     fits); larger M runs on the batched tensor-core kernel, for which a copy of the activations (about 2 M K bytes) and
+ *     partial sums must fit the array (about 2.9 MB of it): M = 16 at K = 4096 and M = 64 at K = 14336 fit,
  *     M = 2048 does not.  A problem that does not
  *     fit returns SBVR_ERR_NOALLOC_LIMIT and launches nothing.  Shapes neither kernel covers run on the SIMT kernel,
  *     which needs no scratch.

@@ -302,7 +302,7 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
         if (M > 32 || w.G != 256 || !linear_sb_supported(w, 16)) return SBVR_ERR_UNSUPPORTED;
         algo = 3;
     }
-    if (Kin != K && algo != 3) {                   // the GEMM pads while it re-tiles
+    if (Kin != K && algo != 3) {                   // the GEMM pads where it has to
         __half* xd = reinterpret_cast<__half*>(ws->dyn + ws->dyn_bytes);
         rc = launch_pad_rows(xh, xd, M, Kin, K, st);
         if (rc) return rc;

@@ -1,85 +1,92 @@
-// SBVR linear for more than four activation rows (small batches and prefill): a tcgen05 fp16 GEMM whose
+// SBVR linear for more than a few activation rows (batches and prefill): a tcgen05 fp16 GEMM whose
 // weight operand is dequantised inside the kernel and never exists in memory.
 //
 //   y[m, n] = sum_k x[m, k] * W[n, k] (+ bias[n]),   W[n, k] = sum_s c[k/G, n, s] * bit_s[n, k]
 //
-// Operands of tcgen05.mma kind::f16 (fp32 accumulation in tensor memory), D[128 weight rows, NX activation rows]:
+// Operands of tcgen05.mma kind::f16 (fp32 accumulation in tensor memory), D[128 weight rows, 32 .. 384 activation rows]:
 //
 //  A (weights, from tensor memory)  Decoder thread r of a warpgroup owns weight row r of the tile.  Per 64 k it
-//      loads its 2 x S packed words, turns them into 64 fp16 values and stores them to its tensor-memory lane
+//      turns its 2 x S packed words into 64 fp16 values and stores them to its tensor-memory lane
 //      (tcgen05.st): decoded weights never touch shared or global memory.  The value of an element is the sum of
 //      the c_s whose plane bit is set, formed two elements at a time in half2: a lone bit at position 10 .. 14 of a
 //      half is a power of two, so `word & (0x04000400 << i)` is (2^e * bit_j, 2^e * bit_{j+16}) and one HFMA2 with
 //      c_s / 2^e adds c_s where the bits are set: a mask and an HFMA2 per plane per pair of elements, plus three
 //      shifted copies per word (rows with |c_s| >= 3.9 use sign flips around sum_s c_s / 2 instead: shift, LOP3,
-//      HADD2).  Elements j and j + 16 of a word share a 32-bit column, so the K order inside each 32-k word is
-//      permuted (position p <-> k = p/2 + 16 (p & 1)).
-//  B (activations, from shared memory)  x is first re-tiled by a small kernel into the blocked layout the MMA
-//      reads (8-row x 16-byte core matrices, K-major, no swizzle) with the same K permutation, one contiguous
-//      block per (NX rows, 64 k); the GEMM fetches a block with a single bulk asynchronous copy.
+//      HADD2).  One byte permute per pair brings the elements into their natural order.
+//  B (activations, from shared memory)  TMA boxes of those rows x 64 k straight from x (128-byte swizzle); rows and columns past the end
+//      are filled with zeros by the copy.  Rows that do not start on 16 bytes are copied into such first.
 //
 // Replaces `x @ decode().T` of the reference's Llama flow for prefill (reference sbvr_utils/utils_llama.py:147,
 // sbvr/core.py:926-949) and the M > 1 use of `_sbvr_row_deq_mm_T` (sbvr/kernels/sbvr_kernel.cu:121-191).
 // Accuracy: weights are formed in fp16 with one rounding per plane (not the single rounding of decode()), which
 // perturbs a weight by at most a few fp16 ulps of its partial sums; products accumulate in fp32.
 //
-// Structure: persistent CTAs of 18 warps.  Warps 0-15 are four decoder warpgroups that take the 64-k stages
-// round-robin and, once the MMAs of a work item have finished, read D from tensor memory, add the bias and
-// write fp16 (or fp32 partial sums when K is split over several CTAs: small activation batches on wide GPUs;
-// the last CTA to arrive adds the parts in a fixed order, so results do not depend on timing).  Warp 16 issues
-// the MMAs from one elected lane; warp 17 streams the activation blocks.
+// Structure: persistent CTAs of 20 warps.  Warps 0-15 are four decoder warpgroups, one for each 64-k stage of a window of 256 k; when
+// the MMAs of a tile (or of a CTA's part of one) have finished they read D from tensor memory, add the bias and write fp16, or fp32 sums
+// where several CTAs share the tile (a second, small kernel adds them in the order of K).  Warp 16 issues the MMAs from one elected lane,
+// warp 17 fetches activations, warps 18 and 19 packed words and coefficient lines, a window each in turn.  The work is split by windows
+// (TsSegs): whole tiles, and the tiles that are left over cut into equal runs of windows.  Every wait is bounded; on a time-out the kernel
+// records it in the status word, skips the remaining work without skipping a barrier, frees its tensor memory and returns.
 //
-// What bounds it (2048 x 14336 x 4096, S = 4, 256-row tiles, about 850 cycles per 64-k stage): the decoders, about 540 instructions
-// per scheduler and stage with half of the integer pipe busy; without their arithmetic a stage takes 640, with 512 of tensor time.
-// The issuing lane was as long before (a probe of two barriers for the next stages, elections and descriptor arithmetic on the path
-// between two stages: 740 cycles with everything in place); now one barrier stands for both operands, the next stage's is read
-// ahead, descriptors move by constants and the tensor-memory addresses are immediates.  Every wait is bounded; on a time-out
-// the kernel records it in the status word, skips the remaining work without skipping a barrier, frees its
-// tensor memory and returns.
-#include "common.cuh"
+// What bounds it: up to 128 rows the decoders' integer pipe, about 200 half-rate instructions per thread and stage, 480 cycles with four
+// warps per scheduler (850 when they loaded words and lines themselves, a stage ahead); with more rows the MMAs, 520 for 256.  Around that,
+// per call, 1.5 us until a CTA has set itself up, 2 until its first words and coefficients are there, 2 for the last tile; and 3 to 5
+// where sums of parts of K are added by the second launch.  S = 4, us (and when activations were re-tiled by a kernel in front, K was split
+// evenly and the last CTA added the parts): 64 x 14336 x 4096 27.0 (34.3), 64 x 4096 x 14336 28.6 (36.1), 64 x 4096 x 4096 16.7 (17.8),
+// 64 x 1024 x 4096 11.7 (17.8), 256 x 14336 x 4096 31.7 (40.3), 256 x 4096 x 4096 24.1 (32.3), 256 x 1024 x 4096 17.2 (48.5), 300 x 4096 x
+// 14336 40.3 (68.2), 1024 x 4096 x 4096 32.4 (37.9); two parts: 37 x 3000 x 3000, S = 3, 14.3 (17.7), 200 x 3001 x 4096 27.7 (44.7).
+#include <algorithm>
+
+#include "tc_stream.cuh"
 
 namespace sbvr {
 
 constexpr int GM_DWGS = 4;
-constexpr int GM_DTHREADS = GM_DWGS * 128;
-constexpr int GM_IWARP = GM_DWGS * 4;
-constexpr int GM_PWARP = GM_IWARP + 1;
-constexpr int GM_THREADS = (GM_PWARP + 1) * 32;
+constexpr int GM_IWARP = GM_DWGS * 4;              // MMA issuer
+constexpr int GM_XWARP = GM_IWARP + 1;             // fetches activations
+constexpr int GM_PWARP = GM_XWARP + 1;             // first of two that fetch packed words and coefficient lines
+constexpr int GM_THREADS = (GM_PWARP + 2) * 32;
 constexpr int GM_TMEM_COLS = 512;
-// NX activation rows per tile.  NX = GM_WIDE stands for any multiple of 32 in (256, 384] (GmParams::nx): every stage is then two
-// MMAs per 16 k, 256 columns and the rest, and a decoded weight tile serves up to 1.5 times as many activations.
-constexpr int GM_WIDE = 384;
-// Ring of 64-k stages: a decoded 128 x 64 weight tile in tensor memory and the activation block in shared memory.
-__host__ __device__ constexpr int gm_slots(int NX, bool EXACT) { return (NX == GM_WIDE || EXACT) ? 4 : 6; }
-__host__ __device__ constexpr int gm_a_col(int NX) { return NX == GM_WIDE ? 384 : 256; }   // D occupies columns [0, NX), the A ring is behind
-constexpr int GM_HDR = 1024;
+// Ring of 64-k stages: a decoded 128 x 64 weight tile in tensor memory and the activations in shared memory; ring of windows: packed words
+// of 128 rows x 256 k, and the coefficients (four halves) of a row for one or two groups.
+constexpr int GM_WIDE = 384;                       // variant for tiles of 288 .. 384 activation rows (GmParams::nx, multiples of 32)
+__host__ __device__ constexpr int gm_slots(int NX, bool EXACT) { return EXACT || NX == GM_WIDE ? 4 : NX == 256 ? 5 : 6; }
+__host__ __device__ constexpr int gm_windows(int NX, bool EXACT) { return NX >= 256 && !EXACT ? 2 : 4; }
+__host__ __device__ constexpr int gm_window_bytes(int S, int G) { return 8 * 128 * S * 4 + 256 / G * 128 * 8; }
+__host__ __device__ constexpr int gm_a_col(int NX) { return NX == GM_WIDE ? 384 : 256; }       // D occupies columns [0, nx), the A ring is behind
+constexpr int GM_HDR = 1024, GM_SMEM_MAX = 227 * 1024;
+__host__ __device__ constexpr int gm_smem(int NX, int nx, bool EXACT, int S, int G) {
+    return GM_HDR + gm_slots(NX, EXACT) * nx * 128 + gm_windows(NX, EXACT) * gm_window_bytes(S, G);
+}
+static_assert(gm_smem(256, 256, false, 4, 128) <= GM_SMEM_MAX && gm_smem(256, 256, true, 4, 128) <= GM_SMEM_MAX &&
+              gm_smem(GM_WIDE, 384, false, 4, 256) <= GM_SMEM_MAX && gm_smem(GM_WIDE, 352, false, 4, 128) <= GM_SMEM_MAX, "shared memory");
 
 struct GmParams {
-    const __half* xt;            // re-tiled activations [MT][K/64][NX*64]
     const uint32_t* bvr;
     const void* idx;
     const __half* coeff;
     const __half* bias;
     __half* y;
-    float* part;                 // [KS][MT*NX][N] fp32 partial sums (KS > 1)
-    unsigned int* counters;      // one per output tile, zero between launches
+    float* part;                 // [CTA + left-over tile][nx][128] fp32 sums of tiles that several CTAs share
     unsigned int* status;
-    int M, N, K, C, G, idx_bytes;
+    int M, N, K, G, idx_bytes;
+    int vec;                     // lines of S = 4 (2) can be read as 8 (4) bytes
     int nx;                      // activation rows of a tile
-    int NT, MT, KS, SPP, items;  // weight-row tiles, activation-row tiles, k parts, 64-k stages per part
+    int MT, tiles, KBS;          // activation-row tiles, tiles, windows of a tile
+    int whole;                   // tiles are not split
 };
 
 __device__ __forceinline__ void gm_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void gm_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// B descriptor: K-major, no swizzle, 128 B between core matrices along K, 1024 B between 8-row groups; version 1.  Its upper word is
-// a constant; the lower one moves by (bytes >> 4).
-__device__ __forceinline__ uint32_t gm_bdesc_lo(uint32_t saddr) { return (saddr >> 4) | ((128u >> 4) << 16); }
+// B descriptor: K-major, 128-byte swizzle, 1024 B between 8-row groups; version 1.  Its upper word is a constant; the lower one moves by
+// (bytes >> 4).
+__device__ __forceinline__ uint32_t gm_bdesc_lo(uint32_t saddr) { return (saddr >> 4) | (1u << 16); }
 __device__ __forceinline__ void gm_mma(uint32_t d_t, uint32_t a_t, uint32_t bdesc_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b64 d;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 d, {%2, %5};\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %3, p;\n\t}" ::"r"(d_t),
-        "r"(a_t), "r"(bdesc_lo), "r"(idesc), "r"(accumulate), "r"((1024u >> 4) | (1u << 14))
+        "r"(a_t), "r"(bdesc_lo), "r"(idesc), "r"(accumulate), "r"((1024u >> 4) | (1u << 14) | (2u << 29))
         : "memory");
 }
 __device__ __forceinline__ void gm_commit(uint64_t* bar) {
@@ -135,159 +142,154 @@ __device__ __forceinline__ void gm_ld32(uint32_t taddr, float (&d)[32]) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// activations -> blocked, K-permuted layout
-// ---------------------------------------------------------------------------------------------
-// Position p of a 64-k stage is k = 64 kst + 32 (p / 32) + (p % 32) / 2 + 16 (p & 1): eight elements and the eight sixteen
-// further on interleave into two 16-byte chunks.  One thread makes such a pair from two 16-byte loads; the 32 lanes of a
-// warp are 8 rows x the 4 pairs of a stage, so that a warp reads whole 128-byte row segments and writes one whole 1 KB
-// core-matrix block [kc (8)][row (8)][16 B].  (One chunk per thread, gathered with eight 2-byte loads, took 32 us at
-// 2048 x 4096.)  Rows of Kin <= K elements are padded with zeros; rows that cannot be read in 16-byte pieces element by element.
-__global__ void __launch_bounds__(256) gemm_retile_x_kernel(const __half* __restrict__ x, __half* __restrict__ xt, int M, int Kin,
-                                                            int K, int NX, int MT) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const int KST = K / 64, RG = NX / 8;
-    const int lane = threadIdx.x & 31, rr = lane & 7, pr = lane >> 3;     // row of the group; pair: k offset 32 (pr / 2) + 8 (pr % 2)
-    const size_t blocks = (size_t)MT * KST * RG;                          // 1 KB blocks, in the order they lie in xt
-    const bool vec = (Kin % 8 == 0) && ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
-    const int koff = 32 * (pr >> 1) + 8 * (pr & 1);
-    for (size_t b = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); b < blocks; b += (size_t)gridDim.x * 8) {
-        const int rg = (int)(b % RG);
-        const size_t rest = b / RG;
-        const int kst = (int)(rest % KST), mt = (int)(rest / KST);
-        const int m = mt * NX + rg * 8 + rr;
-        const int k = kst * 64 + koff;
-        uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
-        if (m < M) {
-            const __half* row = x + (size_t)m * Kin;
-            if (vec) {
-                if (k < Kin) lo = __ldg(reinterpret_cast<const uint4*>(row + k));
-                if (k + 16 < Kin) hi = __ldg(reinterpret_cast<const uint4*>(row + k + 16));
-            } else {
-                __align__(16) __half a[8], c[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    a[e] = (k + e < Kin) ? row[k + e] : __float2half(0.0f);
-                    c[e] = (k + 16 + e < Kin) ? row[k + 16 + e] : __float2half(0.0f);
-                }
-                lo = *reinterpret_cast<const uint4*>(a), hi = *reinterpret_cast<const uint4*>(c);
-            }
-        }
-        uint4* dst = reinterpret_cast<uint4*>(xt) + b * 64 + (size_t)(2 * pr) * 8 + rr;
-        dst[0] = make_uint4(__byte_perm(lo.x, hi.x, 0x5410), __byte_perm(lo.x, hi.x, 0x7632), __byte_perm(lo.y, hi.y, 0x5410),
-                            __byte_perm(lo.y, hi.y, 0x7632));
-        dst[8] = make_uint4(__byte_perm(lo.z, hi.z, 0x5410), __byte_perm(lo.z, hi.z, 0x7632), __byte_perm(lo.w, hi.w, 0x5410),
-                            __byte_perm(lo.w, hi.w, 0x7632));
-    }
-}
-
-// ---------------------------------------------------------------------------------------------
 // the GEMM
 // ---------------------------------------------------------------------------------------------
-// Split K: the sum of the KS parts of one output tile (rows activation rows x cols weight rows, row pitch N), in part order.
-// A thread takes four neighbouring weight rows of U activation rows and loads Q parts of them together: one element and one part at a
-// time was a chain of 64 x KS L2 round trips (71 -> 38 us at 512 x 4096 x 4096), one part at a time of few rows one of KS.
-template <int U, int Q>
-static __device__ __forceinline__ void gm_add_rows(const float* part, size_t plane, int KS, int rows, int cols, int N,
-                                                   const __half* bias, __half* y, int tid) {
-    constexpr int W = GM_DTHREADS / 32;
-    const int c = (tid & 31) * 4;
-    if (c >= cols) return;
-    const bool quad = (N % 4 == 0) && c + 4 <= cols;
-    float b[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = (bias && c + j < cols) ? __half2float(bias[c + j]) : 0.0f;
-    for (int m = tid >> 5; m < rows; m += U * W) {
-        float v[U][4];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[u][j] = 0.0f;
-        for (int q0 = 0; q0 < KS; q0 += Q) {
-            float t[Q][U][4];
-#pragma unroll
-            for (int q = 0; q < Q; ++q)
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int mu = m + u * W;
-                    const bool on = mu < rows && q0 + q < KS;
-                    const float* s = part + (size_t)(q0 + q) * plane + c + (size_t)mu * N;
-                    if (on && quad) {
-                        const float4 f = __ldcg(reinterpret_cast<const float4*>(s));
-                        t[q][u][0] = f.x, t[q][u][1] = f.y, t[q][u][2] = f.z, t[q][u][3] = f.w;
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) t[q][u][j] = (on && c + j < cols) ? __ldcg(s + j) : 0.0f;
-                    }
-                }
-#pragma unroll
-            for (int q = 0; q < Q; ++q)
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) v[u][j] += t[q][u][j];
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int mu = m + u * W;
-            if (mu >= rows) break;
-            __half* dst = y + (size_t)mu * N + c;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (c + j < cols) dst[j] = __float2half_rn(v[u][j] + b[j]);
-        }
+// A CTA's work: its runs of windows of the left-over tiles first, then its own tiles.
+struct GmSegs {
+    TsSegs sg;
+    int KBS, cta;
+    bool whole;
+    __device__ __forceinline__ GmSegs(const GmParams& p) : KBS(p.KBS), cta((int)blockIdx.x), whole(p.whole != 0) {
+        sg.init(p.tiles, whole ? 1 : KBS, gridDim.x, blockIdx.x);
     }
-}
-static __device__ __forceinline__ void gm_add_parts(const float* part, size_t plane, int KS, int rows, int cols, int N,
-                                                 const __half* bias, __half* y, int tid) {
-    constexpr int W = GM_DTHREADS / 32;
-    if (rows <= W) gm_add_rows<1, 4>(part, plane, KS, rows, cols, N, bias, y, tid);
-    else if (rows <= 2 * W) gm_add_rows<2, 2>(part, plane, KS, rows, cols, N, bias, y, tid);
-    else gm_add_rows<4, 1>(part, plane, KS, rows, cols, N, bias, y, tid);
-}
+    __device__ __forceinline__ int k0(int q) const { return whole ? 0 : sg.k0(q); }
+    __device__ __forceinline__ int k1(int q) const { return whole ? KBS : sg.k1(q); }
+};
 
-// SPLIT: K is split over several CTAs (p.KS > 1).  A kernel of its own: its CTAs have one work item each (gm_plan), so that the
-// epilogue, which needs the registers of the decoding loop, comes behind that loop and not inside it.
 // EXACT: weights are formed in fp32 and multiplied in two fp16 parts (gm_two_parts), two MMAs per 16 k on the same activations, for
 // the row counts that are no multiple of 128, which the CUDA-core kernel with its fp32 weights served before.  Formed in fp16 with
 // one rounding per plane the weights gave errors of 3.1e-4 of the result (2-norm) where that kernel has 2.1e-4, the rounding of
-// the result; so have two parts.  37 x 3000 x 3000, S = 3: 17 us (14 with fp16 weights, 70 on CUDA cores); 1000 x 3000 x 4096,
-// S = 4: 62 us (37, 2 190).
-template <int S, int NX, bool SPLIT, bool EXACT>
-__global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmParams p) {
+// the result; so have two parts.
+template <int S, int NX, bool EXACT>
+__global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const __grid_constant__ CUtensorMap xmap, const GmParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
-    constexpr int NX1 = NX == GM_WIDE ? 256 : NX;  // columns of the first MMA
-    constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NX1 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-    constexpr int GM_SLOTS = gm_slots(NX, EXACT), GM_A_COL = gm_a_col(NX);
+    constexpr int BOXES = NX == GM_WIDE ? 2 : 1;   // an MMA has at most 256 columns, a box 256 rows
+    const int nx = NX == GM_WIDE ? p.nx : NX, box = nx / BOXES;
+    const uint32_t idesc = (1u << 4) | ((uint32_t)(box >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    constexpr int SLOTS = gm_slots(NX, EXACT), WINDOWS = gm_windows(NX, EXACT);
     constexpr int ACOLS = EXACT ? 64 : 32;         // tensor-memory columns of a decoded tile
-    static_assert(GM_A_COL + GM_SLOTS * ACOLS <= GM_TMEM_COLS && NX <= GM_A_COL, "tensor memory");
-    const int nx = NX == GM_WIDE ? p.nx : NX;
-    const uint32_t STAGE_BYTES = (uint32_t)nx * 128u;
-    const uint32_t idesc2 = (1u << 4) | ((uint32_t)((nx - NX1) >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    constexpr int A_COL = gm_a_col(NX);
+    const uint32_t stage_bytes = (uint32_t)nx * 128, window_bytes = gm_window_bytes(S, p.G);
+    static_assert(A_COL + SLOTS * ACOLS <= GM_TMEM_COLS && NX <= A_COL, "tensor memory");
 
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem);          // [GM_SLOTS] activation block landed and weight tile stored
-    uint64_t* empty = full + GM_SLOTS;                           // [GM_SLOTS] both read by the stage's MMAs
-    uint64_t* d_full = empty + GM_SLOTS;                         // [1] all MMAs of a work item done
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem);          // [SLOTS] activations landed and weight tile stored
+    uint64_t* empty = full + SLOTS;                              // [SLOTS] both read by the stage's MMAs
+    uint64_t* d_full = empty + SLOTS;                            // [1] all MMAs of a segment done
     uint64_t* d_empty = d_full + 1;                              // [1] D read out
-    volatile int* flags = reinterpret_cast<volatile int*>(d_empty + 1);     // [0] abort, [1] "last part" flag
+    uint64_t* p_full = d_empty + 1;                              // [WINDOWS] packed words and coefficients landed
+    uint64_t* p_empty = p_full + WINDOWS;                        // [WINDOWS] read by the decoders
+    volatile int* flags = reinterpret_cast<volatile int*>(p_empty + WINDOWS);      // [0] abort
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(smem + GM_HDR - 16);
-    unsigned char* xs = smem + GM_HDR;                           // [GM_SLOTS][STAGE_BYTES]
+    unsigned char* xs = smem + GM_HDR;                           // [SLOTS][stage_bytes]
+    unsigned char* ps = xs + SLOTS * stage_bytes;                // [WINDOWS][window_bytes]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     pdl_launch_dependents();
-    pdl_wait();                                    // the re-tiled activations come from the previous kernel
+    const GmSegs segs(p);
+    const TsSegs& sg = segs.sg;
+    const int KBS = p.KBS, N = p.N;
+    const int tail = (p.K & 255) ? 2 : 4;          // stages of a tile's last window
+    auto stages_of = [&](int kb) { return kb == KBS - 1 ? tail : 4; };
+    auto seg_stages = [&](int q) { return (segs.k1(q) - segs.k0(q)) * 4 - (segs.k1(q) == KBS ? 4 - tail : 0); };
+
+    // What the two fetching warps work with; they ask for their first window before anything else.
+    const int sets = p.G == 128 ? 2 : 1, groups = p.K / p.G;
+    struct Pos {
+        int q, kb, k1, n;                          // segment, window, end of its windows, this lane's first row
+    };
+    auto set_seg = [&](Pos& a) {
+        if (a.q >= sg.nseg) return;
+        a.kb = segs.k0(a.q), a.k1 = segs.k1(a.q), a.n = sg.tile(a.q) / p.MT * 128 + lane;
+    };
+    auto next = [&](Pos& a) {
+        if (a.q < sg.nseg && ++a.kb >= a.k1) {
+            ++a.q;
+            set_seg(a);
+        }
+    };
+    auto row = [&](const Pos& a, int i) { return min(a.n + 32 * i, N - 1); };                  // rows past the last one repeat it and are dropped
+    auto lines_of = [&](const Pos& a, uint32_t (&l)[2][4]) {
+        if (a.q >= sg.nseg) return;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            if (t >= sets) break;
+            const size_t g = (size_t)min(a.kb * sets + t, groups - 1) * N;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const size_t e = g + row(a, i);
+                if (p.idx_bytes == 1) l[t][i] = __ldg(reinterpret_cast<const uint8_t*>(p.idx) + e);
+                else if (p.idx_bytes == 2) l[t][i] = __ldg(reinterpret_cast<const uint16_t*>(p.idx) + e);
+                else l[t][i] = (uint32_t)e;
+            }
+        }
+    };
+    auto load_coef = [&](const Pos& a, const uint32_t (&l)[2][4], uint2 (&c)[2][4]) {
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                c[t][i] = make_uint2(0u, 0u);
+                if (t >= sets || a.q >= sg.nseg) continue;
+                const unsigned short* src = reinterpret_cast<const unsigned short*>(p.coeff) + (size_t)l[t][i] * S;
+                if (S == 4 && p.vec) c[t][i] = __ldg(reinterpret_cast<const uint2*>(src));
+                else if (S == 2 && p.vec) c[t][i].x = __ldg(reinterpret_cast<const uint32_t*>(src));
+                else {
+                    c[t][i].x = __ldg(src) | ((uint32_t)__ldg(src + 1) << 16);
+                    if (S > 2) c[t][i].y = __ldg(src + 2);
+                    if (S > 3) c[t][i].y |= (uint32_t)__ldg(src + 3) << 16;
+                }
+            }
+    };
+    auto copy_words = [&](const Pos& a, int slot) {
+        const uint32_t dst = smem_u32(ps) + slot * window_bytes + (uint32_t)(lane * S * 4);
+        const int runs = 2 * stages_of(a.kb);
+        const uint32_t* src[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) src[i] = p.bvr + ((size_t)a.kb * 8 * N + row(a, i)) * S;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if (k >= runs) break;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t d = dst + (uint32_t)((k * 128 + 32 * i) * S * 4);
+                if constexpr (S == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src[i]) : "memory");
+                else if constexpr (S == 2) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src[i]) : "memory");
+                else
+#pragma unroll
+                    for (int s = 0; s < S; ++s) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * s), "l"(src[i] + s) : "memory");
+                src[i] += (size_t)N * S;
+            }
+        }
+    };
+    Pos win{0, 0, 0, 0};                           // the window at hand: its coefficients in coef, the line numbers of the one after in lines
+    uint2 coef[2][4];
+    uint32_t lines[2][4] = {};
+    bool first_words = true;
+    if (warp >= GM_PWARP) {
+        set_seg(win);
+        if (warp != GM_PWARP) next(win);
+        lines_of(win, lines);
+        if (win.q < sg.nseg) copy_words(win, warp - GM_PWARP);
+        load_coef(win, lines, coef);               // (the line numbers have come meanwhile)
+        Pos ahead = win;
+        next(ahead), next(ahead);
+        lines_of(ahead, lines);
+    }
     if (threadIdx.x == 0) {
-        for (int i = 0; i < GM_SLOTS; ++i) {
+        for (int i = 0; i < SLOTS; ++i) {
             mbar_init(&full[i], 5);                // the activation producer and four decoder warps
             mbar_init(&empty[i], 1);
         }
         mbar_init(d_full, 1);
         mbar_init(d_empty, GM_DWGS * 4);
+        for (int i = 0; i < WINDOWS; ++i) {
+            mbar_init(&p_full[i], 33);             // every lane's copies, and its coefficients
+            mbar_init(&p_empty[i], GM_DWGS * 4);
+        }
         flags[0] = 0;
-        flags[1] = 0;
         fence_mbar_init();
     }
-    if (warp == GM_PWARP) {
+    if (warp == GM_XWARP) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base_s)),
                      "r"((uint32_t)GM_TMEM_COLS)
                      : "memory");
@@ -297,52 +299,55 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
     __syncthreads();
     gm_fence_after();
     const uint32_t tbase = *tmem_base_s;
-    const int grid = (int)gridDim.x;
-    const int SPP = p.SPP;
 
-    if (warp == GM_PWARP) {
+    if (warp == GM_XWARP) {
         // ------------------------------ activation producer ------------------------------
         if (lane == 0) {
-            int it = 0;
+            pdl_wait();                            // x comes from the previous kernel
+            int slot = 0;
+            uint32_t ph = 1;
             bool ok = true;
-            for (int item = blockIdx.x; item < p.items && ok; item += grid) {
-                const int kp = item % p.KS, mt = (item / p.KS) % p.MT;
-                const unsigned char* src = reinterpret_cast<const unsigned char*>(p.xt) +
-                                           ((size_t)mt * (p.K / 64) + (size_t)kp * SPP) * STAGE_BYTES;
-                for (int ks = 0; ks < SPP; ++ks, ++it) {
-                    const int st = it % GM_SLOTS;
-                    const uint32_t ph = (uint32_t)(it / GM_SLOTS) & 1u;
-                    if (flags[0] || !mbar_wait_async(&empty[st], ph ^ 1u)) {
+            for (int q = 0; q < sg.nseg && ok; ++q) {
+                const int m = sg.tile(q) % p.MT * nx, s0 = segs.k0(q) * 4, s1 = s0 + seg_stages(q);
+                for (int s = s0; s < s1; ++s) {
+                    if (flags[0] || !mbar_wait_async(&empty[slot], ph)) {
                         ok = false;
                         break;
                     }
-                    mbar_arrive_expect_tx(&full[st], STAGE_BYTES);
-                    bulk_g2s(xs + (size_t)st * STAGE_BYTES, src + (size_t)ks * STAGE_BYTES, STAGE_BYTES, &full[st]);
+                    mbar_arrive_expect_tx(&full[slot], stage_bytes);
+#pragma unroll
+                    for (int b = 0; b < BOXES; ++b) ts_tma_2d(xs + (size_t)slot * stage_bytes + b * box * 128, &xmap, s * 64, m + b * box, &full[slot]);
+                    if (++slot == SLOTS) slot = 0, ph ^= 1u;
                 }
             }
             if (!ok) {
                 flags[0] = 1;
                 atomicExch(p.status, 1u);
                 atomicExch(p.status + 1, 0x500u + blockIdx.x);
+                const long long t0 = clock64();    // (the copies that were issued land before the CTA leaves)
+                while (clock64() - t0 < (1LL << 22)) {}
             }
         }
     } else if (warp == GM_IWARP) {
         // ------------------------------ MMA issuer ------------------------------
         // One barrier per stage says that both operands are in place, and the barrier of the next stage is read before
         // the MMAs of this one are issued, so that its latency runs beside them.
-        const int total = (int)blockIdx.x < p.items ? ((p.items - 1 - (int)blockIdx.x) / grid + 1) * SPP : 0;
+        int total = 0;
+        for (int q = 0; q < sg.nseg; ++q) total += seg_stages(q);
         bool ok = tbase == 0;                      // (an allocation of all columns can only start at column 0)
         if (elect_one()) {
-            const uint32_t d0 = gm_bdesc_lo(smem_u32(xs)), dstep = STAGE_BYTES >> 4;
-            int ks = 0;
-            uint32_t ph = 0, dph = 1;              // dph: parity of the read-out of the item before
+            const uint32_t d0 = gm_bdesc_lo(smem_u32(xs));
+            int q = 0, left = 0;
+            uint32_t first = 0, ph = 0, dph = 1;   // dph: parity of the read-out of the segment before
             bool rdy = mbar_test(&full[0], 0u);
-            for (int it = 0; it < total && ok; it += GM_SLOTS, ph ^= 1u) {
+            for (int it = 0; it < total && ok; it += SLOTS, ph ^= 1u) {
 #pragma unroll
-                for (int slot = 0; slot < GM_SLOTS; ++slot) {
+                for (int slot = 0; slot < SLOTS; ++slot) {
                     if (it + slot >= total) break;
-                    if (ks == 0) {
-                        if (it + slot > 0 && !mbar_wait_timed(d_empty, dph)) ok = false;       // D of the previous item must have been read out
+                    if (left == 0) {
+                        left = seg_stages(q++);
+                        first = 1;
+                        if (!mbar_wait_timed(d_empty, dph)) ok = false;        // D of the previous segment must have been read out
                         dph ^= 1u;
                     }
                     if (!rdy) {                    // (spins: a warp parked by try_wait comes back later than the phase)
@@ -355,20 +360,18 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                     }
                     if (!ok) break;
                     gm_fence_after();
-                    rdy = mbar_test(&full[(slot + 1) % GM_SLOTS], slot + 1 == GM_SLOTS ? ph ^ 1u : ph);
-                    const uint32_t d = d0 + (uint32_t)slot * dstep;
+                    rdy = mbar_test(&full[(slot + 1) % SLOTS], slot + 1 == SLOTS ? ph ^ 1u : ph);
+                    const uint32_t d = d0 + (uint32_t)slot * (stage_bytes >> 4);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const uint32_t acc = q ? 1u : (uint32_t)(ks != 0);
-                        gm_mma(0, GM_A_COL + slot * ACOLS + q * 8, d + q * 16, IDESC, acc);
-                        if (EXACT) gm_mma(0, GM_A_COL + slot * ACOLS + 32 + q * 8, d + q * 16, IDESC, 1u);
-                        if (NX == GM_WIDE) gm_mma(NX1, GM_A_COL + slot * ACOLS + q * 8, d + NX1 * 8 + q * 16, idesc2, acc);
-                    }
+                    for (int b = 0; b < BOXES; ++b)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            gm_mma(b * box, A_COL + slot * ACOLS + k * 8, d + b * box * 8 + k * 2, idesc, k ? 1u : first ^ 1u);
+                            if (EXACT) gm_mma(b * box, A_COL + slot * ACOLS + 32 + k * 8, d + b * box * 8 + k * 2, idesc, 1u);
+                        }
                     gm_commit(&empty[slot]);
-                    if (++ks == SPP) {
-                        gm_commit(d_full);
-                        ks = 0;
-                    }
+                    first = 0;
+                    if (--left == 0) gm_commit(d_full);
                 }
             }
         }
@@ -380,163 +383,114 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                 atomicExch(p.status + 1, 0x600u + blockIdx.x);
             }
         }
+    } else if (warp >= GM_PWARP) {
+        // ------------------------------ packed words and coefficients ------------------------------
+        // Every second window.  A lane copies the words of four rows, asynchronously, and gathers their coefficient lines: line numbers
+        // two of its windows ahead, lines one ahead.  (By the decoders, a stage ahead, the loads were what they waited for most.)
+        int slot = warp - GM_PWARP;
+        uint32_t ph = 1;
+        bool ok = true;
+        while (win.q < sg.nseg) {
+            if (!first_words) {                    // (of its first window before the barriers were set up)
+                if (flags[0] || !mbar_wait_timed(&p_empty[slot], ph)) ok = false;
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                copy_words(win, slot);
+            }
+            first_words = false;
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&p_full[slot])) : "memory");
+            Pos ahead = win;
+            next(ahead), next(ahead);
+            uint2 c1[2][4];
+            load_coef(ahead, lines, c1);           // (its line numbers came with the window before)
+            const uint32_t dst = smem_u32(ps) + slot * window_bytes + 8 * 128 * S * 4;
+#pragma unroll
+            for (int t = 0; t < 2; ++t) {
+                if (t >= sets) break;
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(dst + t * 1024 + (lane + 32 * i) * 8), "r"(coef[t][i].x), "r"(coef[t][i].y) : "memory");
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_full[slot]);
+            win = ahead;
+            next(ahead), next(ahead);
+            lines_of(ahead, lines);
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) coef[t][i] = c1[t][i];
+            slot += 2;
+            if (slot >= WINDOWS) slot -= WINDOWS, ph ^= 1u;
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        if (!ok) {
+            flags[0] = 1;
+            if (lane == 0) {
+                atomicExch(p.status, 1u);
+                atomicExch(p.status + 1, 0xE00u + blockIdx.x);
+            }
+        }
     } else {
         // ------------------------------ decoder warpgroups ------------------------------
         const int wg = warp >> 2, wl = warp & 3;
         const int r = wl * 32 + lane;
-        const int dtid = threadIdx.x;              // 0 .. 511
         const uint32_t lane_sel = (uint32_t)(wl * 32) << 16;
-        const int N = p.N;
         bool dead = false;
 
-        // The stages of all work items of this CTA form one sequence; this warpgroup takes every fourth one.
-        struct Pos {
-            int item, ks, it;
-            int kst0, n;                           // first 64-k stage of the item's k part; this thread's weight row
-        };
-        auto set_item = [&](Pos& q) {              // the divisions happen once per work item, not per stage
-            q.kst0 = (q.item % p.KS) * SPP;
-            q.n = min((q.item / (p.KS * p.MT)) * 128 + r, p.N - 1);      // rows past the last one repeat it and are dropped
-        };
-        auto advance = [&](Pos& q, int by) {
-            q.ks += by;
-            q.it += by;
-            if (q.ks >= SPP) {
-                do {
-                    q.ks -= SPP;
-                    q.item += grid;
-                } while (q.ks >= SPP);
-                set_item(q);
-            }
-        };
-        const int group_shift = (p.G == 256) ? 2 : 1;      // 64-k stages per coefficient group, as a shift
-        auto load_words = [&](const Pos& q, uint32_t (&w)[2][S]) {
-            if (q.item >= p.items) return;
-            const uint32_t* src = p.bvr + ((size_t)(2 * (q.kst0 + q.ks)) * N + q.n) * S;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t* g = src + (size_t)h * N * S;
-                if constexpr (S == 4) {
-                    const uint4 v = __ldg(reinterpret_cast<const uint4*>(g));
-                    w[h][0] = v.x, w[h][1] = v.y, w[h][2] = v.z, w[h][3] = v.w;
-                } else if constexpr (S == 2) {
-                    const uint2 v = __ldg(reinterpret_cast<const uint2*>(g));
-                    w[h][0] = v.x, w[h][1] = v.y;
-                } else {
-#pragma unroll
-                    for (int s = 0; s < S; ++s) w[h][s] = __ldg(g + s);
-                }
-            }
-        };
-        // D of one finished work item -> y (or fp32 parts); every decoder warp takes part, also when dead.
-        int ep_item = blockIdx.x, ep_seq = 0;
-        auto epilogue = [&]() {
-            const int item = ep_item;
-            const int kp = item % p.KS, mt = (item / p.KS) % p.MT, nt = item / (p.KS * p.MT);
-            const int n = nt * 128 + r;
-            if (!dead && !mbar_wait_async(d_full, (uint32_t)ep_seq & 1u)) {
+        // D of one finished segment -> y (or fp32 sums); every decoder warp takes part, also when dead.
+        auto epilogue = [&](int q, uint32_t seq) {
+            const int tile = sg.tile(q), mt = tile % p.MT, nt = tile / p.MT, n = nt * 128 + r;
+            if (!dead && !mbar_wait_async(d_full, seq & 1u)) {
                 dead = true;
                 flags[0] = 1;
             }
             dead = __any_sync(0xffffffffu, dead);
             const int m0 = mt * nx;
+            const bool shared = sg.shared(q);
+            const int rt = shared ? sg.rt_first + q : 0;
             if (!dead) {
                 gm_fence_after();
                 const bool on = n < N;
-                const float bias = (p.bias && !SPLIT && on) ? __half2float(p.bias[n]) : 0.0f;
+                const float bias = (p.bias && !shared && on) ? __half2float(p.bias[n]) : 0.0f;
                 for (int c = wg; c < nx / 32; c += GM_DWGS) {
                     float d[32];
                     gm_ld32(tbase + lane_sel + c * 32, d);
-                    if constexpr (!SPLIT) {
+                    if (!shared) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) {
                             const int m = m0 + c * 32 + i;
                             if (on && m < p.M) p.y[(size_t)m * N + n] = __float2half_rn(d[i] + bias);
                         }
                     } else {
-                        float* dst = p.part + ((size_t)kp * p.MT * NX + m0 + c * 32) * N + n;
+                        float* dst = p.part + ((size_t)(segs.cta + rt) * nx + c * 32) * 128 + r;
 #pragma unroll
                         for (int i = 0; i < 32; ++i)
-                            if (on) dst[(size_t)i * N] = d[i];
+                            if (m0 + c * 32 + i < p.M) __stcg(dst + i * 128, d[i]);
                     }
                 }
                 gm_fence_before();
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(d_empty);
-            if constexpr (SPLIT) {
-                // split K: the CTA that delivers the last part adds all parts in part order
-                __threadfence();
-                named_bar_sync(1, GM_DTHREADS);
-                if (dtid == 0) {
-                    const unsigned int tile = (unsigned int)(mt * p.NT + nt);
-                    const unsigned int old = dead ? 0u : atomicAdd(p.counters + tile, 1u);
-                    const int last = (!dead && old == (unsigned int)(p.KS - 1)) ? 1 : 0;
-                    if (last) p.counters[tile] = 0u;           // ready for the next launch
-                    flags[1] = last;
-                }
-                named_bar_sync(1, GM_DTHREADS);
-                const bool last = flags[1] != 0;
-                named_bar_sync(1, GM_DTHREADS);                // everyone has read the flag before it is rewritten
-                if (last) {
-                    __threadfence();
-                    gm_add_parts(p.part + (size_t)m0 * N + nt * 128, (size_t)p.MT * NX * N, p.KS, min(NX, p.M - m0), min(128, N - nt * 128),
-                                 N, p.bias ? p.bias + nt * 128 : nullptr, p.y + (size_t)m0 * N + nt * 128, dtid);
-                }
+        };
+
+        // The slot of stage `it` may be stored to; false: a wait ran out here or elsewhere.  A parity tells a phase only from the next, so
+        // it must be certain that the slot's stage before last, it - 2 SLOTS, has been read.  At its stage before, it - 4, this warpgroup
+        // waited for it - 4 - SLOTS, and MMAs run in order: four slots are enough.  (After a window of two stages, which two warpgroups sit
+        // out, all of them wait for the end of the tile.)
+        static_assert(SLOTS >= GM_DWGS, "phases of the ring");
+        auto slot_free = [&](int it) -> bool {
+            if (!dead && !mbar_wait_async(&empty[it % SLOTS], ((uint32_t)(it / SLOTS) & 1u) ^ 1u)) {
+                dead = true;
+                flags[0] = 1;
             }
-            ep_item += grid;
-            ++ep_seq;
+            dead = __any_sync(0xffffffffu, dead);
+            if (!dead) gm_fence_after();
+            return !dead;
         };
-
-        // Coefficients are fetched ahead as well: the line index of a stage two steps before its use, the
-        // coefficient line itself one step before (it needs the index), so neither latency is exposed.
-        auto line_of = [&](const Pos& q) -> uint32_t {
-            if (q.item >= p.items) return 0u;
-            const int g = (q.kst0 + q.ks) >> group_shift;
-            const size_t e = (size_t)g * N + q.n;
-            if (p.idx_bytes == 1) return __ldg(reinterpret_cast<const uint8_t*>(p.idx) + e);
-            if (p.idx_bytes == 2) return __ldg(reinterpret_cast<const uint16_t*>(p.idx) + e);
-            return (uint32_t)e;
-        };
-        auto load_coef = [&](const Pos& q, uint32_t line, unsigned short (&c)[S]) {
-            if (q.item >= p.items) return;
-            const unsigned short* src = reinterpret_cast<const unsigned short*>(p.coeff) + (size_t)line * S;
-#pragma unroll
-            for (int s = 0; s < S; ++s) c[s] = __ldg(src + s);
-        };
-
-        Pos cur{(int)blockIdx.x, 0, 0, 0, 0};
-        set_item(cur);
-        advance(cur, wg);
-        Pos nxt = cur;
-        advance(nxt, GM_DWGS);
-        Pos nn = nxt;
-        advance(nn, GM_DWGS);
-        uint32_t w0[2][S], w1[2][S];               // packed words of `cur` and `nxt`: loads run one stage ahead
-        unsigned short c0[S], c1[S];               // their coefficient lines (fp16 bits)
-        load_words(cur, w0);
-        load_words(nxt, w1);
-        {
-            const uint32_t lc = line_of(cur), ln = line_of(nxt);
-            load_coef(cur, lc, c0);
-            load_coef(nxt, ln, c1);
-        }
-        uint32_t l_nn = line_of(nn);
-
-        auto decode_stage = [&](const Pos& q, const uint32_t (&w)[2][S], const unsigned short (&c)[S]) {
-            if constexpr (!SPLIT)                  // (a CTA of a split problem has one item)
-                while (ep_item < q.item) epilogue();   // items whose stages have all been handed to the issuer
-            const int slot = q.it % GM_SLOTS;
-            // false: a wait ran out here or elsewhere
-            auto slot_free = [&]() -> bool {
-                if (!dead && !mbar_wait_async(&empty[slot], ((uint32_t)(q.it / GM_SLOTS) & 1u) ^ 1u)) {
-                    dead = true;
-                    flags[0] = 1;
-                }
-                dead = __any_sync(0xffffffffu, dead);
-                if (!dead) gm_fence_after();
-                return !dead;
-            };
+        auto decode_stage = [&](int it, const uint32_t (&w)[2][S], const unsigned short (&c)[4]) {
+            const int slot = it % SLOTS;
             auto hand_over = [&]() {
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 gm_fence_before();
@@ -560,14 +514,14 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                         float v0 = 0.0f, v1 = 0.0f;
 #pragma unroll
                         for (int s = 0; s < S; ++s) {
-                            if (w[h][s] & (1u << j)) v0 += cf[s];
-                            if (w[h][s] & (0x10000u << j)) v1 += cf[s];
+                            if (w[h][s] & (1u << (2 * j))) v0 += cf[s];
+                            if (w[h][s] & (2u << (2 * j))) v1 += cf[s];
                         }
                         gm_two_parts(v0, v1, odd, hi[j], lo[j]);
                     }
-                    if (h == 0 && !slot_free()) return;
-                    gm_st16(tbase + lane_sel + GM_A_COL + slot * ACOLS + h * 16, hi);
-                    gm_st16(tbase + lane_sel + GM_A_COL + slot * ACOLS + 32 + h * 16, lo);
+                    if (h == 0 && !slot_free(it)) return;
+                    gm_st16(tbase + lane_sel + A_COL + slot * ACOLS + h * 16, hi);
+                    gm_st16(tbase + lane_sel + A_COL + slot * ACOLS + 32 + h * 16, lo);
                 }
                 hand_over();
                 return;
@@ -592,6 +546,14 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                 mul[s][4] = __hmul2(c2, __float2half2_rn(0.5f));
             }
             uint32_t a[32];
+            auto natural = [&](int h, const __half2 (&acc)[16]) {              // pairs (j, j + 16) -> pairs (2 j, 2 j + 1)
+                const uint32_t* f = reinterpret_cast<const uint32_t*>(acc);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    a[16 * h + j] = __byte_perm(f[2 * j], f[2 * j + 1], 0x5410);
+                    a[16 * h + 8 + j] = __byte_perm(f[2 * j], f[2 * j + 1], 0x7632);
+                }
+            };
             if (!__any_sync(0xffffffffu, big)) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
@@ -610,8 +572,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                             acc[j] = __hfma2(*reinterpret_cast<const __half2*>(&t), mul[s][pos], acc[j]);
                         }
                     }
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) a[16 * h + j] = *reinterpret_cast<const uint32_t*>(&acc[j]);
+                    natural(h, acc);
                 }
             } else {
                 uint32_t hc[S];                    // (c_s / 2, c_s / 2)
@@ -627,53 +588,74 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
                 const uint32_t base2 = bb | (bb << 16);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
+                    __half2 acc[16];
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
-                        __half2 acc = *reinterpret_cast<const __half2*>(&base2);
+                        acc[j] = *reinterpret_cast<const __half2*>(&base2);
 #pragma unroll
                         for (int s = 0; s < S; ++s) {
                             const uint32_t v = w[h][s] << (15 - j);
                             const uint32_t t = (~v & 0x80008000u) ^ hc[s];
-                            acc = __hadd2(acc, *reinterpret_cast<const __half2*>(&t));
+                            acc[j] = __hadd2(acc[j], *reinterpret_cast<const __half2*>(&t));
                         }
-                        a[16 * h + j] = *reinterpret_cast<const uint32_t*>(&acc);
                     }
+                    natural(h, acc);
                 }
             }
             // the slot is waited for with the values in registers: the decode runs beside the MMAs that still read the slot
-            if (!slot_free()) return;
-            gm_st32(tbase + lane_sel + GM_A_COL + slot * ACOLS, a);
+            if (!slot_free(it)) return;
+            gm_st32(tbase + lane_sel + A_COL + slot * ACOLS, a);
             hand_over();
         };
 
-        while (cur.item < p.items) {
-            decode_stage(cur, w0, c0);
-            cur = nxt, nxt = nn;
-            advance(nn, GM_DWGS);
-            {
-                const uint32_t ln = l_nn;          // index of the new look-ahead stage, loaded a step ago
-                l_nn = line_of(nn);
-                load_words(nxt, w0);               // the set just used is free: it becomes the look-ahead set
-                load_coef(nxt, ln, c0);
+        int it0 = 0, wi = 0;                       // stages and windows before the current window
+        bool waited = false;
+        for (int q = 0; q < sg.nseg; ++q) {
+            const int k1 = segs.k1(q);
+            for (int kb = segs.k0(q); kb < k1; ++kb, ++wi) {
+                const int nst = stages_of(kb), slot = wi % WINDOWS;
+                const unsigned char* src = ps + slot * window_bytes;
+                if (!dead && !mbar_wait_timed(&p_full[slot], (uint32_t)(wi / WINDOWS) & 1u)) {
+                    dead = true;
+                    flags[0] = 1;
+                }
+                dead = __any_sync(0xffffffffu, dead);
+                uint32_t w[2][S];
+                unsigned short c[4];
+                if (wg < nst) {
+                    const uint2 cc = *reinterpret_cast<const uint2*>(src + 8 * 128 * S * 4 + (p.G == 128 ? (wg >> 1) * 1024 : 0) + r * 8);
+                    c[0] = (unsigned short)cc.x, c[1] = (unsigned short)(cc.x >> 16), c[2] = (unsigned short)cc.y, c[3] = (unsigned short)(cc.y >> 16);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t* g = reinterpret_cast<const uint32_t*>(src) + ((2 * wg + h) * 128 + r) * S;
+                        if constexpr (S == 4) {
+                            const uint4 v = *reinterpret_cast<const uint4*>(g);
+                            w[h][0] = v.x, w[h][1] = v.y, w[h][2] = v.z, w[h][3] = v.w;
+                        } else if constexpr (S == 2) {
+                            const uint2 v = *reinterpret_cast<const uint2*>(g);
+                            w[h][0] = v.x, w[h][1] = v.y;
+                        } else {
+#pragma unroll
+                            for (int s = 0; s < S; ++s) w[h][s] = g[s];
+                        }
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&p_empty[slot]);
+                if (wg < nst && !dead) decode_stage(it0 + wg, w, c);
+                it0 += nst;
             }
-            if (cur.item >= p.items) break;
-            decode_stage(cur, w1, c1);
-            cur = nxt, nxt = nn;
-            advance(nn, GM_DWGS);
-            {
-                const uint32_t ln = l_nn;
-                l_nn = line_of(nn);
-                load_words(nxt, w1);
-                load_coef(nxt, ln, c1);
+            if (!waited) {
+                pdl_wait();                        // y and the parts may still be in use by the previous kernels
+                waited = true;
             }
+            epilogue(q, (uint32_t)q);
         }
-        while (ep_item < p.items) epilogue();
-
         if (dead) {
             flags[0] = 1;
             if (lane == 0) {
                 atomicExch(p.status, 1u);
-                atomicExch(p.status + 1, 0x400u + blockIdx.x);
+                atomicExch(p.status + 1, 0x800u + blockIdx.x);
             }
         }
     }
@@ -681,39 +663,103 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const GmPara
     gm_fence_before();
     __syncthreads();
     gm_fence_after();
-    if (warp == GM_PWARP)
+    if (warp == GM_XWARP)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"((uint32_t)GM_TMEM_COLS)
                      : "memory");
+}
+
+// The sums of the shared tiles, added in the order of K: a thread four weight rows of an activation row.  A launch of its own, over the
+// whole GPU: the last CTA to arrive at a tile had up to eighteen sums of 128 KB to add (256 x 1024 x 4096: 39 us, now 15).  Blocks of 128
+// threads with 32 registers fit beside a CTA of the product.  Where little is to be added one per SM does it, and is there when the
+// product ends, so that the next call's product may start (37 x 3000 x 3000: 16.1 -> 14.3 us); else a warp has one row, in as many
+// blocks as that takes (128 x 14336 x 4096: 33 us, 47 by a block per SM).
+constexpr int GM_ADD_WARPS = 4;
+__global__ void __launch_bounds__(GM_ADD_WARPS * 32, 16) gm_add_kernel(const float* __restrict__ part, const __half* __restrict__ bias,
+                                                                                  __half* __restrict__ y, int M, int N, int MT, int nx, int tiles, int KBS,
+                                                                                  int ctas) {
+    pdl_launch_dependents();
+    TsSegs sg;
+    sg.init(tiles, KBS, (unsigned int)ctas, 0u);
+    const int rows = min(nx, M), left = tiles - sg.rem_tile0, c = (threadIdx.x & 31) * 4;      // (rows past the last of a last tile are skipped)
+    const bool wide = N % 4 == 0 && !(reinterpret_cast<uintptr_t>(y) & 7);
+    const long long jobs = (long long)left * rows;
+    pdl_wait();
+    int rt0 = -1, c0 = 0, parts = 0, m0 = 0, n = 0;
+    for (long long job = (long long)blockIdx.x * GM_ADD_WARPS + (threadIdx.x >> 5); job < jobs; job += (long long)gridDim.x * GM_ADD_WARPS) {
+        const int rt = (int)(job / rows), i = (int)(job - (long long)rt * rows);
+        if (rt != rt0) {
+            rt0 = rt;
+            c0 = sg.cta_of((unsigned int)(rt * sg.KBS)), parts = sg.cta_of((unsigned int)(rt * sg.KBS + sg.KBS - 1)) - c0 + 1;
+            const int tile = sg.rem_tile0 + rt;
+            m0 = tile % MT * nx, n = tile / MT * 128 + c;
+        }
+        if (parts == 1 || m0 + i >= M || n >= N) continue;     // (one CTA has done the tile alone)
+        const float* src = part + ((size_t)(c0 + rt) * nx + i) * 128 + c;
+        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int q = 0; q < parts; q += 3) {
+            float4 t[3];
+#pragma unroll
+            for (int h = 0; h < 3; ++h) {
+                t[h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (q + h < parts) t[h] = __ldcg(reinterpret_cast<const float4*>(src));
+                src += (size_t)nx * 128;
+            }
+#pragma unroll
+            for (int h = 0; h < 3; ++h) v.x += t[h].x, v.y += t[h].y, v.z += t[h].z, v.w += t[h].w;
+        }
+        const float o[4] = {v.x, v.y, v.z, v.w};
+        __half* dst = y + (size_t)(m0 + i) * N + n;
+        __align__(8) __half h[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) h[k] = __float2half_rn(o[k] + (bias && n + k < N ? __half2float(bias[n + k]) : 0.0f));
+        if (wide) {
+            *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(h);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (n + k < N) dst[k] = h[k];
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
 // host
 // ---------------------------------------------------------------------------------------------
-struct GmPlan {
-    int NX, MT, NT, KS, SPP, items, grid, smem;
-    bool exact;
-    size_t xt_bytes, part_bytes;
+// The scratch that a call is accepted by, and the shares of K that the choice between this kernel and the small-batch kernel counts
+// with: both as they were when activations were re-tiled into blocks of NX rows (up to 384 where that saved rounds of tiles) and K
+// was split evenly, so that workspaces, the fixed array of the no-allocation entry and the precision of few rows stay what they were.
+struct GmScratch {
+    int KS, SPP, items;
+    size_t bytes;
 };
-
-// Activation rows of a tile.  More than 256 rows: the width with the least work on the busiest SM, whole rounds of tiles times the
-// time of a 64-k stage.  A stage of a 256-row tile waits for the decoders (the more planes the longer), one of a wider tile for
-// its MMAs; measured per stage at 2048 x 14336 x 4096, in cycles: 850 (S = 4), about 730 (S = 2) at 256 rows, 3 per row for wider
-// tiles (a second, small MMA costs more than its share of the columns).  Wide tiles win where they save rounds: 232 -> 210 us at
-// 2048 x 14336 x 4096 (7 rounds -> 5 of 352 rows), 350 -> 302 us at 3000 x 4096 x 14336 (3 -> 2), 78 -> 59 us at 1500 x 4096 x
-// 4096 (2 -> 1 of 384 rows); 2048 x 4096 stays at 256 rows (2 rounds either way).  Problems that do not fill the GPU at 256 rows
-// split K instead.
-// Two-part weights fill the tensor memory of wide tiles: 256 rows at most, 64 at least (one instantiation less).
-static int gm_nx(int M, int NT, int S, int sm_count, bool exact) {
+static int gm_scratch_rows(int M, int NT, int S, int sm_count, bool exact) {
     if (M <= 256 || exact) return (M <= 32 && !exact) ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256;
     int best = 256;
     long long cost = 0;
-    for (int nx = 256; nx <= GM_WIDE; nx += 32) {
+    for (int nx = 256; nx <= 384; nx += 32) {
         const long long items = (long long)NT * ((M + nx - 1) / nx);
         if (nx == 256 && items < sm_count) break;
         const long long c = (items + sm_count - 1) / sm_count * (nx == 256 ? 610 + 60 * S : 3 * nx);
         if (nx == 256 || c < cost) best = nx, cost = c;
     }
     return best;
+}
+static GmScratch gm_scratch(const PackedW& w, int M, int sm_count) {
+    const int NT = (w.N + 127) / 128, NX = gm_scratch_rows(M, NT, w.S, sm_count, w.N % 128 != 0), MT = (M + NX - 1) / NX, KST = w.K / 64;
+    const int tiles = NT * MT;
+    GmScratch s;
+    s.KS = 1;
+    if (NX <= 256 && tiles < sm_count && tiles <= SBVR_WS_COUNTERS)
+        for (int cand = 2; cand <= KST / 4 && tiles * cand <= sm_count; ++cand)
+            if (KST % cand == 0) s.KS = cand;
+    s.SPP = KST / s.KS, s.items = tiles * s.KS;
+    s.bytes = ((size_t)MT * NX * w.K * 2 + 255) / 256 * 256 + (s.KS > 1 ? (size_t)s.KS * MT * NX * w.N * 4 : 0);
+    return s;
+}
+size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count) { return gm_scratch(w, M, sm_count).bytes; }
+void linear_gemm_split(const PackedW& w, int M, int sm_count, int* parts, int* stages) {
+    const GmScratch s = gm_scratch(w, M, sm_count);
+    *parts = s.KS, *stages = s.SPP * ((s.items + sm_count - 1) / sm_count);
 }
 
 bool linear_gemm_supported(const PackedW& w, int M) {
@@ -726,79 +772,73 @@ bool linear_gemm_supported(const PackedW& w, int M) {
     return true;
 }
 
-static void gm_plan(const PackedW& w, int M, int sm_count, GmPlan* pl) {
-    pl->NT = (w.N + 127) / 128;
-    pl->exact = w.N % 128 != 0;
-    pl->NX = gm_nx(M, pl->NT, w.S, sm_count, pl->exact);
-    pl->MT = (M + pl->NX - 1) / pl->NX;
-    const int KST = w.K / 64;
-    int ks = 1;
-    const int tiles = pl->NT * pl->MT;
-    if (pl->NX <= 256 && tiles < sm_count && tiles <= SBVR_WS_COUNTERS) {
-        // split K so that more SMs work, keeping at least 4 stages per part
-        for (int cand = 2; cand <= KST / 4; ++cand) {
-            if (KST % cand) continue;
-            if (tiles * cand > sm_count) break;
-            ks = cand;
-        }
+struct GmPlan {
+    int nx, MT, tiles, KBS, grid;
+    bool exact, whole;
+    size_t part_bytes;
+    long long ns;
+};
+
+// Activation rows of a tile, and whether the tiles that are left over after whole rounds are cut: the least time in ns by these figures
+// (17 .. 384 rows, 1024 .. 28672 x 2048 .. 14336, S = 2 .. 4).  A 64-k stage takes its decoding, 150 + 50 S (in two parts 200 + 120 S), or
+// for many rows 1.05 a row + 40 S (2.1 a row + 120; beyond two rounds, with the clock at the
+// power limit, 1.15 a row and 1.2 in tiles of 256); a call 3 000 + 8 a row, another round's ends 1 500.  Cutting adds a launch, 5 000, and
+// 0.36 per KB of sums out and back.  Measured whole and cut, us, S = 4: 64 x 14336 x 4096 (112 tiles) 27.6, 30.8; 64 x 4096 x 14336 76.7, 29.1;
+// 64 x 4096 x 4096 23.6, 16.9; 64 x 28672 x 8192 95, 80.  More than 256 rows in two tiles and in one: 270 x 28672 x 8192 212, 119; 384 x 14336 x
+// 4096 62, 40; 384 x 4096 x 4096 28, 36.
+static GmPlan gm_plan_nx(const PackedW& w, int M, int nx, int sm_count, size_t scratch) {
+    GmPlan pl;
+    pl.exact = w.N % 128 != 0;
+    pl.nx = nx;
+    pl.MT = (M + nx - 1) / nx;
+    pl.tiles = (w.N + 127) / 128 * pl.MT;
+    pl.KBS = (w.K + 255) / 256;
+    const long long call = 3000 + 8 * std::min(nx, 256), rounds = (pl.tiles + sm_count - 1) / sm_count;
+    const int row = rounds <= 2 ? 105 : nx > 256 ? 115 : 120;
+    const long long stage = pl.exact ? std::max(200 + 120 * w.S, 21 * nx / 10 + 120) : std::max(150 + 50 * w.S, row * nx / 100 + 40 * w.S);
+    pl.whole = true, pl.part_bytes = 0;
+    pl.grid = std::min(pl.tiles, sm_count);
+    pl.ns = call + rounds * (w.K / 64 * stage + 1500) - 1500;
+    const long long windows = (long long)pl.tiles * pl.KBS, ctas = std::min<long long>(windows, sm_count), left = pl.tiles % ctas;
+    if (left && left * pl.KBS >= ctas && left * pl.KBS * ctas < (1LL << 32)) {             // (every CTA has a window of them at least)
+        const size_t bytes = (size_t)(ctas + left) * nx * 512;
+        const long long ns = call + 5000 + (windows + ctas - 1) / ctas * 4 * stage + (rounds - 1) * 1500 + (long long)(bytes * 9 / 25000);
+        if (ns < pl.ns && bytes <= scratch) pl.whole = false, pl.part_bytes = bytes, pl.grid = (int)ctas, pl.ns = ns;
     }
-    pl->KS = ks;
-    pl->SPP = KST / ks;
-    pl->items = tiles * ks;
-    pl->grid = pl->items < sm_count ? pl->items : sm_count;
-    pl->smem = GM_HDR + gm_slots(pl->NX > 256 ? GM_WIDE : pl->NX, pl->exact) * pl->NX * 128;
-    pl->xt_bytes = ((size_t)pl->MT * pl->NX * w.K * 2 + 255) / 256 * 256;
-    pl->part_bytes = ks > 1 ? (size_t)ks * pl->MT * pl->NX * w.N * 4 : 0;
+    return pl;
+}
+static GmPlan gm_plan(const PackedW& w, int M, int sm_count, size_t scratch) {
+    const bool exact = w.N % 128 != 0;
+    GmPlan best = gm_plan_nx(w, M, (M <= 32 && !exact) ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256, sm_count, scratch);
+    if (M <= 256 || exact) return best;
+    for (int nx = 288; nx <= GM_WIDE && gm_smem(GM_WIDE, nx, false, w.S, w.G) <= GM_SMEM_MAX; nx += 32) {
+        const GmPlan pl = gm_plan_nx(w, M, nx, sm_count, scratch);
+        if (pl.ns < best.ns) best = pl;
+    }
+    return best;
 }
 
-// Estimate of a call's time in ns for more than 256 rows, to choose between this kernel and the one over CTA pairs: rounds of tiles at
-// the stage times of gm_nx and 9 000 cycles for a tile's end, at 1.9 GHz; re-tiling; the parts of a split K (16.8 MB of them took
-// about 10 us).  Measured and estimated, us: 2048 x 14336 x 4096 209, 209; 512 x 8192 x 8192 67, 67; 1024 x 4096 x 4096 38, 38; 300 x
-// 14336 x 4096 41.5, 41; 3000 x 4096 x 14336 303, 307; 2048 x 1024 x 4096 37, 36.
-static long long gm_ns(const PackedW& w, const GmPlan& pl, int sm_count) {
-    const long long rounds = (pl.items + sm_count - 1) / sm_count;
-    const long long cycles = rounds * ((long long)pl.SPP * (pl.NX == 256 ? 610 + 60 * w.S : 3 * pl.NX) + 9000) +
-                             (long long)(pl.xt_bytes / 2000) + (long long)(pl.part_bytes / 900) + 6000;
-    return cycles * 10 / 19;
-}
-
-size_t linear_gemm_workspace_bytes(const PackedW& w, int M, int sm_count) {
-    GmPlan pl;
-    gm_plan(w, M, sm_count, &pl);
-    return pl.xt_bytes + pl.part_bytes;
-}
-
-void linear_gemm_split(const PackedW& w, int M, int sm_count, int* parts, int* stages) {
-    GmPlan pl;
-    gm_plan(w, M, sm_count, &pl);
-    *parts = pl.KS, *stages = pl.SPP * ((pl.items + sm_count - 1) / sm_count);
-}
-
-template <int S, int NX, bool SPLIT, bool EXACT>
-static int gm_launch_split(const GmParams& p, int grid, int smem, cudaStream_t st) {
+template <int S, int NX, bool EXACT = false>
+static int gm_launch(const CUtensorMap& xmap, const GmParams& p, int grid, cudaStream_t st) {
     static SmemOnce once;
-    const int rc = set_max_smem_once(once, linear_gemm_kernel<S, NX, SPLIT, EXACT>, 227 * 1024);
+    const int rc = set_max_smem_once(once, linear_gemm_kernel<S, NX, EXACT>, GM_SMEM_MAX);
     if (rc) return rc;
-    SBVR_CUDA_TRY(launch_pdl(linear_gemm_kernel<S, NX, SPLIT, EXACT>, dim3(grid), dim3(GM_THREADS), (size_t)smem, st, p));
+    SBVR_CUDA_TRY(launch_pdl(linear_gemm_kernel<S, NX, EXACT>, dim3(grid), dim3(GM_THREADS), (size_t)gm_smem(NX, p.nx, EXACT, S, p.G), st, xmap, p));
     return SBVR_OK;
 }
-template <int S, int NX, bool EXACT = false>
-static int gm_launch_inst(const GmParams& p, int grid, int smem, cudaStream_t st) {
-    return p.KS > 1 ? gm_launch_split<S, NX, true, EXACT>(p, grid, smem, st) : gm_launch_split<S, NX, false, EXACT>(p, grid, smem, st);
-}
 template <int S>
-static int gm_launch_nx(const GmParams& p, const GmPlan& pl, cudaStream_t st) {
-    if (pl.exact) switch (pl.NX) {
-        case 64: return gm_launch_inst<S, 64, true>(p, pl.grid, pl.smem, st);
-        case 128: return gm_launch_inst<S, 128, true>(p, pl.grid, pl.smem, st);
-        default: return gm_launch_inst<S, 256, true>(p, pl.grid, pl.smem, st);
+static int gm_launch_nx(const CUtensorMap& xmap, const GmParams& p, const GmPlan& pl, cudaStream_t st) {
+    if (pl.exact) switch (pl.nx) {
+        case 64: return gm_launch<S, 64, true>(xmap, p, pl.grid, st);
+        case 128: return gm_launch<S, 128, true>(xmap, p, pl.grid, st);
+        default: return gm_launch<S, 256, true>(xmap, p, pl.grid, st);
     }
-    switch (pl.NX) {
-        case 32: return gm_launch_inst<S, 32>(p, pl.grid, pl.smem, st);
-        case 64: return gm_launch_inst<S, 64>(p, pl.grid, pl.smem, st);
-        case 128: return gm_launch_inst<S, 128>(p, pl.grid, pl.smem, st);
-        case 256: return gm_launch_inst<S, 256>(p, pl.grid, pl.smem, st);
-        default: return gm_launch_split<S, GM_WIDE, false, false>(p, pl.grid, pl.smem, st);
+    switch (pl.nx) {
+        case 32: return gm_launch<S, 32>(xmap, p, pl.grid, st);
+        case 64: return gm_launch<S, 64>(xmap, p, pl.grid, st);
+        case 128: return gm_launch<S, 128>(xmap, p, pl.grid, st);
+        case 256: return gm_launch<S, 256>(xmap, p, pl.grid, st);
+        default: return gm_launch<S, GM_WIDE>(xmap, p, pl.grid, st);
     }
 }
 
@@ -810,29 +850,44 @@ int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half*
     int rc = device_info(ws->device, &di);
     if (rc) return rc;
     if (di.cc_major != 10) return SBVR_ERR_UNSUPPORTED;
-    GmPlan pl;
-    gm_plan(w, M, di.sm_count, &pl);
-    if (pl.xt_bytes + pl.part_bytes > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
-    if (linear_pair_supported(x, Kin, w, y, M) &&
-        linear_pair_ns(w, M, di.sm_count, ws->device, ws->dyn_bytes) < gm_ns(w, pl, di.sm_count))
+    if (linear_gemm_workspace_bytes(w, M, di.sm_count) > ws->dyn_bytes) return SBVR_ERR_WORKSPACE;
+    // What a plan may count on beside the padded rows: what sbvr_workspace_bytes promises, whatever the workspace has grown to for other calls.
+    size_t promised = 0;
+    if (sbvr_workspace_bytes(ws->device, M, w.N, w.K, &promised) != SBVR_OK) promised = SBVR_WS_FIXED_BYTES;
+    const size_t rows = ((size_t)M * w.K * 2 + 255) / 256 * 256, scratch = std::min(ws->dyn_bytes, promised - SBVR_WS_FIXED_BYTES);
+    const GmPlan pl = gm_plan(w, M, di.sm_count, scratch > rows ? scratch - rows : 0);
+    if (linear_pair_supported(x, Kin, w, y, M) && linear_pair_ns(w, M, di.sm_count, ws->device, ws->dyn_bytes) < pl.ns)
         return launch_linear_pair(x, Kin, w, bias, y, M, ws->status, ws->dyn, ws->dyn_bytes, di.sm_count, ws->device, st);
-    __half* xt = reinterpret_cast<__half*>(ws->dyn);
-    {
-        const size_t nblk = ((size_t)pl.MT * pl.NX / 8 * (w.K / 64) + 7) / 8;
-        const int blocks = (int)(nblk < (size_t)di.sm_count * 16 ? nblk : (size_t)di.sm_count * 16);
-        SBVR_CUDA_TRY(launch_pdl(gemm_retile_x_kernel, dim3(blocks), dim3(256), 0, st, x, xt, M, Kin, w.K, pl.NX, pl.MT));
+    if (Kin % 8 || (reinterpret_cast<uintptr_t>(x) & 15)) {        // rows that TMA cannot read
+        __half* xp = reinterpret_cast<__half*>(ws->dyn);
+        rc = launch_pad_rows(x, xp, M, Kin, w.K, st);
+        if (rc) return rc;
+        x = xp, Kin = w.K;
     }
+    CUtensorMap xmap;
+    rc = ts_map_2d(&xmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, CU_TENSOR_MAP_SWIZZLE_128B, x, (size_t)M, (size_t)Kin, (size_t)Kin * 2,
+                   pl.nx > 256 ? pl.nx / 2 : pl.nx, 64);
+    if (rc) return rc;
     GmParams p;
-    p.xt = xt, p.bvr = w.bvr, p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y;
-    p.part = reinterpret_cast<float*>(ws->dyn + pl.xt_bytes);
-    p.counters = ws->counters, p.status = ws->status;
-    p.M = M, p.N = w.N, p.K = w.K, p.C = w.C, p.G = w.G, p.idx_bytes = w.idx_bytes, p.nx = pl.NX;
-    p.NT = pl.NT, p.MT = pl.MT, p.KS = pl.KS, p.SPP = pl.SPP, p.items = pl.items;
+    p.bvr = w.bvr, p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y;
+    p.part = reinterpret_cast<float*>(ws->dyn + rows);
+    p.status = ws->status;
+    p.M = M, p.N = w.N, p.K = w.K, p.G = w.G, p.idx_bytes = w.idx_bytes;
+    p.vec = !(reinterpret_cast<uintptr_t>(w.coeff) & (2 * w.S - 1));
+    p.nx = pl.nx, p.MT = pl.MT, p.tiles = pl.tiles, p.KBS = pl.KBS, p.whole = pl.whole;
     switch (w.S) {
-        case 2: return gm_launch_nx<2>(p, pl, st);
-        case 3: return gm_launch_nx<3>(p, pl, st);
-        default: return gm_launch_nx<4>(p, pl, st);
+        case 2: rc = gm_launch_nx<2>(xmap, p, pl, st); break;
+        case 3: rc = gm_launch_nx<3>(xmap, p, pl, st); break;
+        default: rc = gm_launch_nx<4>(xmap, p, pl, st);
     }
+    if (rc || pl.whole) return rc;
+    const long long left = pl.tiles % pl.grid, jobs = left * std::min(pl.nx, M);
+    if (jobs) {
+        const bool few = jobs <= 2LL * GM_ADD_WARPS * di.sm_count && pl.grid <= 8 * left;
+        SBVR_CUDA_TRY(launch_pdl(gm_add_kernel, dim3(few ? (unsigned)di.sm_count : (unsigned)((jobs + GM_ADD_WARPS - 1) / GM_ADD_WARPS)),
+                                 dim3(GM_ADD_WARPS * 32), 0, st, p.part, bias, y, M, w.N, pl.MT, pl.nx, pl.tiles, pl.KBS, pl.grid));
+    }
+    return SBVR_OK;
 }
 
 }  // namespace sbvr

@@ -9,8 +9,8 @@
 // the `sbvr_workspace_t` the regular entry point wants, because creating it is a cudaMalloc.
 //
 // What it does instead.  The scratch the kernels need (the time-out status word, the arrival counters,
-// the quantised activations and partial sums of the decode kernel, the re-tiled activations and the
-// split-K partial sums of the batched kernel) lives in ONE
+// the quantised activations and partial sums of the decode kernel, the padded activations and the
+// partial sums of the batched kernel) lives in ONE
 // fixed array that is part of this library's device image, `g_noalloc_scratch` below: SBVR_NOALLOC_BYTES = 4 MiB per
 // GPU that loads the library, held until the process exits.  Nothing is allocated or freed here,
 // by this file or by anything it calls.
@@ -26,8 +26,8 @@
 //     any stream capture, with the device current; later calls only enqueue work.
 //   * A problem whose scratch does not fit is refused with SBVR_ERR_NOALLOC_LIMIT before anything is
 //     launched.  The decode kernel (M <= 4) needs about 4 K M bytes for the activation digits plus 150 KB of
-//     partial sums: every shape it serves fits.  Batches (M > 4) run on the tensor-core GEMM, whose re-tiled
-//     activations take M K 2 bytes (M rounded up to its tile): M = 128 at K = 14336 fits, M = 2048 does not
+//     partial sums: every shape it serves fits.  Batches (M > 4) run on the tensor-core GEMM, which is
+//     taken where M K 2 bytes fit (M rounded up to its tile, room for a padded copy of the activations): M = 128 at K = 14336 fits, M = 2048 does not
 //     and is refused.  Shapes neither kernel serves run on the SIMT kernel, which needs no scratch.
 //   * A time-out of a bounded device wait is recorded in the array but this entry point has no
 //     synchronising call to report it; use the workspace form if you need that.
@@ -117,7 +117,7 @@ extern "C" int sbvr_linear_f16_noalloc(const void* x, const uint32_t* bvr, const
         kind = 1;
         need = linear_tcs_workspace_bytes(w, M, di.sm_count);       // activation digits + partial sums of shared row tiles
     } else if (di.cc_major == 10 && linear_gemm_supported(w, M)) {
-        need = linear_gemm_workspace_bytes(w, M, di.sm_count);      // re-tiled activations + fp32 parts of a split K
+        need = linear_gemm_workspace_bytes(w, M, di.sm_count);      // padded activations + fp32 sums of cut tiles
         if (need <= ws.dyn_bytes || N % 128 == 0) kind = 2;         // ragged rows that do not fit: the SIMT kernel
     }
     if (kind == 0) return launch_linear_simt(xh, w, bh, yh, M, st);

@@ -179,8 +179,8 @@ def query(device: int = 0) -> dict:
 
 
 class Workspace:
-    """Owns one `sbvr_workspace_t`: the device status word of the kernels' bounded waits, the re-tiled
-    activations and split-K partial sums of the batched kernel, staging buffers of the host-pointer call."""
+    """Owns one `sbvr_workspace_t`: the device status word of the kernels' bounded waits, padded
+    activations and partial sums of the batched kernel, staging buffers of the host-pointer call."""
 
     DEFAULT_BYTES = 32 << 20
 
