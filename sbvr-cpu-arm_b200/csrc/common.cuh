@@ -174,6 +174,11 @@ void linear_gemm_split(const PackedW& w, int M, int sm_count, int* parts, int* s
 int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half* bias, __half* y, int M,
                        const sbvr_workspace* ws, cudaStream_t st);
 
+// Prefill attention on the tensor cores (attention_prefill.cu); R: query heads of a KV head, a power of two
+bool attention_tc_supported(const void* qkv, const void* out, int tokens, int tokens_per_seq, int n_kv, int R);
+int launch_attention_tc(const __half* qkv, const __half* kcache, const __half* vcache, const int* positions, __half* out, int tokens,
+                        int tokens_per_seq, int n_heads, int n_kv, int max_ctx, float scale, cudaStream_t st);
+
 // The GEMM over CTA pairs (linear_pair.cu), more than 256 rows; `scratch` is for sums of items that several pairs share, none is needed.
 bool linear_pair_supported(const __half* x, int Kin, const PackedW& w, const __half* y, int M);
 long long linear_pair_ns(const PackedW& w, int M, int sm_count, int device, size_t scratch);      // estimate, to choose between the two GEMMs

@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(128) attention_kernel(const __half* __restrict
 }
 
 // ---------------------------------------------------------------------------------------------
-// Causal prefill on the tensor cores: a CTA takes 64 (query token, query head) pairs that share one KV head (64 / R
+// Causal prefill of short prompts (attention_prefill.cu has the others) on the tensor cores: a CTA takes 64 (query token, query head) pairs that share one KV head (64 / R
 // consecutive tokens of a sequence x its R query heads), each of its four warps 16 of them, and walks the keys 64 at a time
 // with a running maximum and sum per pair.  grid sequences * n_kv * ceil(tokens / (64 / R)), longest contexts first.
 //
@@ -759,6 +759,8 @@ static int attention_launch(const void* qkv, void* kcache, void* vcache, const i
     __half* o = reinterpret_cast<__half*>(out);
     if (!inv_freq && nsplit == 1 && tokens_per_seq >= 8) {      // prefill: tokens of a sequence share K / V fetches
         if (R != 1 && R != 2 && R != 4 && R != 8) return SBVR_ERR_UNSUPPORTED;
+        if (attention_tc_supported(qkv, out, tokens, tokens_per_seq, n_kv, R))
+            return launch_attention_tc(q, kc, vc, positions, o, tokens, tokens_per_seq, n_heads, n_kv, max_ctx, scale, st);
         const int QT = AP_ROWS / R, nblk = (tokens_per_seq + QT - 1) / QT;
         const dim3 bgrid((unsigned)((tokens / tokens_per_seq) * n_kv * nblk));
 #define SBVR_ATTP(RR)                                                                                                       \
