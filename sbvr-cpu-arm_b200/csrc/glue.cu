@@ -124,6 +124,65 @@ __global__ void __launch_bounds__(256) rope_append_kernel(__half* __restrict__ q
     }
 }
 
+// The same, eight elements at a time (16 bytes of either half of a head), for heads of a multiple of 16 in rows and caches on 16 bytes: the
+// first two items of a thread are on their way while the angles are made.  An element at a time a call took 22.2 us at 3000 tokens of 32 + 8 heads of 128 (now 10.9; its
+// bytes 9), 5.7 at 16 (now 2.3).
+__global__ void __launch_bounds__(256) rope_append_vec_kernel(__half* __restrict__ qkv, const int* __restrict__ positions,
+                                                              const float* __restrict__ inv_freq, float attn_scaling,
+                                                              __half* __restrict__ kcache, __half* __restrict__ vcache,
+                                                              int tokens_per_seq, int n_heads, int n_kv, int d, int max_ctx) {
+    __shared__ __align__(16) __half cs_s[2][256];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int t = blockIdx.x, half_d = d / 2, ch = half_d / 8;
+    const int rot = (n_heads + n_kv) * ch, all = rot + n_kv * ch;  // a head's turn, or 16 values of v, per item
+    __half* row = qkv + (size_t)t * (n_heads + 2 * n_kv) * d;
+    auto load = [&](int it, uint4 (&x)[2]) {
+        if (it >= all) return;
+        const int head = it / ch;
+        const __half* p = row + (size_t)head * d + (it - head * ch) * 8;
+        x[0] = *reinterpret_cast<const uint4*>(p), x[1] = *reinterpret_cast<const uint4*>(p + half_d);
+    };
+    uint4 x[2][2];
+    load(threadIdx.x, x[0]);
+    load(threadIdx.x + 256, x[1]);
+    const int pos = positions[t], seq = t / tokens_per_seq;
+    for (int i = threadIdx.x; i < half_d; i += blockDim.x) {
+        const float ang = (float)pos * inv_freq[i];
+        cs_s[0][i] = __float2half_rn(cosf(ang) * attn_scaling);
+        cs_s[1][i] = __float2half_rn(sinf(ang) * attn_scaling);
+    }
+    __syncthreads();
+    auto finish = [&](int it, uint4 (&v)[2]) {
+        if (it >= all) return;
+        const int head = it / ch, i = (it - head * ch) * 8;
+        if (it < rot) {
+            const uint4 c = *reinterpret_cast<const uint4*>(&cs_s[0][i]), s = *reinterpret_cast<const uint4*>(&cs_s[1][i]);
+            const __half2 *c2 = reinterpret_cast<const __half2*>(&c), *s2 = reinterpret_cast<const __half2*>(&s);
+            __half2 *a = reinterpret_cast<__half2*>(&v[0]), *b = reinterpret_cast<__half2*>(&v[1]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const __half2 x1 = a[e], x2 = b[e];
+                a[e] = __hadd2(__hmul2(x1, c2[e]), __hmul2(__hneg2(x2), s2[e]));
+                b[e] = __hadd2(__hmul2(x2, c2[e]), __hmul2(x1, s2[e]));
+            }
+            __half* p = row + (size_t)head * d + i;
+            *reinterpret_cast<uint4*>(p) = v[0], *reinterpret_cast<uint4*>(p + half_d) = v[1];
+        }
+        if (head >= n_heads && pos < max_ctx) {
+            const int kv = it < rot ? head - n_heads : head - n_heads - n_kv;
+            __half* p = (it < rot ? kcache : vcache) + (((size_t)seq * n_kv + kv) * max_ctx + pos) * d + i;
+            *reinterpret_cast<uint4*>(p) = v[0], *reinterpret_cast<uint4*>(p + half_d) = v[1];
+        }
+    };
+    finish(threadIdx.x, x[0]);
+    finish(threadIdx.x + 256, x[1]);
+    for (int it = threadIdx.x + 512; it < all; it += 256) {
+        load(it, x[0]);
+        finish(it, x[0]);
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
 // attention of one query token over cache positions [0, pos]; head_dim 128; grouped-query: the R = n_heads / n_kv
 // query heads of a KV head are served together.  grid tokens * n_kv * nsplit, 128 threads; the nsplit CTAs of a (token, KV
@@ -734,7 +793,9 @@ int sbvr_rope_append_f16(void* qkv, const int* positions, const float* inv_freq,
     if (tokens < 1 || tokens_per_seq < 1 || tokens % tokens_per_seq || n_heads < 1 || n_kv < 1 || head_dim < 2 ||
         head_dim % 2 || max_ctx < 1)
         return SBVR_ERR_BAD_ARG;
-    SBVR_CUDA_TRY(launch_pdl(rope_append_kernel, dim3(tokens), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
+    const bool vec = head_dim % 16 == 0 && !((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kcache) |
+                                              reinterpret_cast<uintptr_t>(vcache)) & 15);
+    SBVR_CUDA_TRY(launch_pdl(vec ? rope_append_vec_kernel : rope_append_kernel, dim3(tokens), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),
                              reinterpret_cast<__half*>(qkv), positions, inv_freq, attn_scaling,
                              reinterpret_cast<__half*>(kcache), reinterpret_cast<__half*>(vcache), tokens_per_seq, n_heads,
                              n_kv, head_dim, max_ctx));
