@@ -13,7 +13,8 @@
 // tensor memory, and the sum of its weights) are scaled.  Weights are at most 2^8 instead of 1, which fp16's exponent holds; every other
 // time the output is not touched by the threads.
 //
-// Seven warps: 0-3 weights, 4 issues the MMAs (one lane), 5 and 6 bring K and V (cp.async, zeros past the last key).  S and the weights of two
+// Seven warps: 0-3 weights, 4 issues the MMAs (one lane), 5 and 6 bring K and V (whole tiles by TMA, the last one by cp.async with zeros past
+// the last key).  S and the weights of two
 // tiles (64 columns each) and O take 256 columns of tensor memory, 97 KB of shared memory: two CTAs per SM, so that one computes weights while
 // the other has the tensor pipe.  Tensor memory is only asked for when the kernel in front has ended, and the kernel behind may start only
 // when this one has it: neither can wait for columns that the other holds while the other waits for it to end.  Every wait is bounded; after
@@ -21,8 +22,10 @@
 //
 // What bounds it: the weights, about 600 instructions and 64 exponentials per thread and tile, on two warps per scheduler; the tensor pipe
 // would take 768 cycles a tile, 26 us at 2 x 1500 tokens.  Per layer, 32 query heads, 8 KV heads, us (mma.sync on blocks of 64, in
-// brackets): 2 x 1500 tokens 64 (157), 1 x 4000 171 (505), 8 x 256 22 (35), 1 x 512 14 (23).
+// brackets): 2 x 1500 tokens 59 (157), 1 x 4000 162 (505), 8 x 256 22 (35), 1 x 512 14 (23).  (With whole tiles by cp.async, too, 63 and 173; with
+// K and V on their way before the queries are staged 60 and 164.)
 #include "common.cuh"
+#include "tc_stream.cuh"
 
 namespace sbvr {
 
@@ -145,7 +148,8 @@ __device__ __noinline__ void aq_multiply_out(const AqParams& p, uint32_t q_s, co
     }
 }
 
-__global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const AqParams p) {
+__global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const __grid_constant__ CUtensorMap kmap,
+                                                                         const __grid_constant__ CUtensorMap vmap, const AqParams p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     uint64_t* k_full = reinterpret_cast<uint64_t*>(smem);        // [2] a tile of K is in shared memory
     uint64_t* v_full = k_full + 2;                               // [2] of V
@@ -219,19 +223,32 @@ __global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const AqPar
             if (t >= 2 && (*dead_s || !mbar_wait_timed(empty + b, (uint32_t)((t - 2) >> 1) & 1u))) ok = false;
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
-#pragma unroll
-            for (int i = 0; i < AQ_KEYS / 2; ++i) {              // two rows at a time, a 16-byte chunk per lane
-                const int row = 2 * i + (lane >> 4), key = t * AQ_KEYS + row;
-                const bool on = key < P;
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + b * AQ_TILE + row * 128 + (((lane & 7) ^ (row & 7)) << 4)),
-                             "l"(base + (size_t)(on ? key : 0) * AQ_D), "r"(on ? 16u : 0u)
-                             : "memory");
+            if ((t + 1) * AQ_KEYS <= P) {                        // a whole tile
+                if (lane == 0) {
+                    mbar_arrive_expect_tx(full + b, AQ_TILE);
+                    unsigned char* dst = smem + AQ_HDR + 2 * AQ_QBOX + ((is_k ? 0 : 2) + b) * AQ_TILE;
+                    const int y = (seq * p.n_kv + kvh) * p.max_ctx + t * AQ_KEYS;
+                    ts_tma_2d(dst, is_k ? &kmap : &vmap, 0, y, full + b);
+                    ts_tma_2d(dst + AQ_KBOX, is_k ? &kmap : &vmap, 64, y, full + b);
+                } else {
+                    mbar_arrive(full + b);
+                }
+            } else {
+#pragma unroll 4
+                for (int i = 0; i < AQ_KEYS / 2; ++i) {              // two rows at a time, a 16-byte chunk per lane
+                    const int row = 2 * i + (lane >> 4), key = t * AQ_KEYS + row;
+                    const bool on = key < P;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + b * AQ_TILE + row * 128 + (((lane & 7) ^ (row & 7)) << 4)),
+                                 "l"(base + (size_t)(on ? key : 0) * AQ_D), "r"(on ? 16u : 0u)
+                                 : "memory");
+                }
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                fence_proxy_async();
+                mbar_arrive(full + b);
             }
-            asm volatile("cp.async.wait_all;" ::: "memory");
-            fence_proxy_async();
-            mbar_arrive(full + b);
             if (!is_k && (t + 1) * AQ_KEYS > pmin) {             // keys that not every token attends to: a weight of zero hides finite values only
                 uint32_t any = 0;
+                if (!mbar_wait_timed(full + b, (uint32_t)(t >> 1) & 1u)) ok = false;
 #pragma unroll 4
                 for (int i = 0; i < AQ_KEYS / 2; ++i) {
                     const int row = 2 * i + (lane >> 4);
@@ -243,9 +260,15 @@ __global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const AqPar
                     for (int e = 0; e < 4; ++e) any |= (v[e] & 0x7c007c00u) + 0x04000400u;     // (an exponent of all ones: bit 15)
                 }
                 if (any & 0x80008000u) *odd_s = 1;
+                fence_proxy_async();                             // read before the next copy writes there
+                __syncwarp();
             }
         }
-        if (!ok) *dead_s = 1;
+        if (!ok) {                                               // copies that were issued land before the CTA leaves
+            *dead_s = 1;
+            const long long c0 = clock64();
+            while (clock64() - c0 < (1LL << 22)) {}
+        }
     } else if (warp == AQ_IWARP) {
         // ------------------------------ MMA issuer ------------------------------
         if (elect_one()) {
@@ -394,8 +417,8 @@ __global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const AqPar
 }
 
 // Setting up costs 3 us more than in attention_prefill_kernel, a tile of keys 1 us less, and that kernel has two blocks of 64 pairs on an SM.
-// us, here and there, 32 query heads, 8 KV heads: 1 x 64 tokens 7.4, 4.5; 1 x 128 8.2, 7.2; 1 x 160 9.0, 8.7; 1 x 192 9.0, 10.2; 1 x 256 9.9, 12.6; 2 x 128
-// 8.2, 8.6; 8 x 64 7.7, 6.8; 12 x 64 9.3, 10.1; 4 heads, 4 KV heads: 1 x 200 8.8, 7.6.
+// us, here and there, 32 query heads, 8 KV heads: 1 x 64 tokens 7.4, 4.5; 1 x 128 8.2, 7.2; 1 x 160 9.0, 8.7; 1 x 192 8.9, 10.2; 1 x 256 9.7, 12.6; 2 x 128
+// 8.2, 8.6; 8 x 64 7.7, 6.8; 12 x 64 9.5, 10.1; 4 heads, 4 KV heads: 1 x 200 8.8, 7.6.
 bool attention_tc_supported(const void* qkv, const void* out, int tokens, int tokens_per_seq, int n_kv, int R) {
     if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) return false;
     const long long blocks = (long long)(tokens / tokens_per_seq) * n_kv * (((long long)tokens_per_seq * R + 63) / 64);
@@ -409,8 +432,13 @@ int launch_attention_tc(const __half* qkv, const __half* kcache, const __half* v
     if (rc) return rc;
     AqParams p{qkv, kcache, vcache, positions, out, tokens_per_seq, n_heads, n_kv, max_ctx, 0, scale};
     while (n_kv << (p.r_shift + 1) <= n_heads) ++p.r_shift;
+    CUtensorMap kmap, vmap;
+    const size_t rows = (size_t)(tokens / tokens_per_seq) * n_kv * max_ctx;
+    int err = ts_map_2d(&kmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, CU_TENSOR_MAP_SWIZZLE_128B, kcache, rows, AQ_D, AQ_D * 2, AQ_KEYS, 64);
+    if (!err) err = ts_map_2d(&vmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, CU_TENSOR_MAP_SWIZZLE_128B, vcache, rows, AQ_D, AQ_D * 2, AQ_KEYS, 64);
+    if (err) return err;
     const int QT = AQ_ROWS >> p.r_shift, nblk = (tokens_per_seq + QT - 1) / QT;
-    SBVR_CUDA_TRY(launch_pdl(attention_tc_kernel, dim3((unsigned)((tokens / tokens_per_seq) * n_kv * nblk)), dim3(AQ_THREADS), (size_t)AQ_SMEM, st, p));
+    SBVR_CUDA_TRY(launch_pdl(attention_tc_kernel, dim3((unsigned)((tokens / tokens_per_seq) * n_kv * nblk)), dim3(AQ_THREADS), (size_t)AQ_SMEM, st, kmap, vmap, p));
     return SBVR_OK;
 }
 
