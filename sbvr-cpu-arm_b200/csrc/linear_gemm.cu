@@ -52,14 +52,23 @@ constexpr int GM_TMEM_COLS = 512;
 constexpr int GM_WIDE = 384;                       // variant for tiles of 288 .. 384 activation rows (GmParams::nx, multiples of 32)
 __host__ __device__ constexpr int gm_slots(int NX, bool EXACT) { return EXACT || NX == GM_WIDE ? 4 : NX == 256 ? 5 : 6; }
 __host__ __device__ constexpr int gm_windows(int NX, bool EXACT) { return NX >= 256 && !EXACT ? 2 : 4; }
-__host__ __device__ constexpr int gm_window_bytes(int S, int G) { return 8 * 128 * S * 4 + 256 / G * 128 * 8; }
+__host__ __device__ constexpr int gm_word_bytes(int S) { return 8 * 128 * S * 4; }
+__host__ __device__ constexpr int gm_coef_bytes(int G) { return 256 / G * 128 * 8; }
 __host__ __device__ constexpr int gm_a_col(int NX) { return NX == GM_WIDE ? 384 : 256; }       // D occupies columns [0, nx), the A ring is behind
 constexpr int GM_HDR = 1024, GM_SMEM_MAX = 227 * 1024;
+__host__ __device__ constexpr int gm_smem_with(int NX, int nx, bool EXACT, int S, int G, int coefs) {
+    return GM_HDR + gm_slots(NX, EXACT) * nx * 128 + gm_windows(NX, EXACT) * gm_word_bytes(S) + coefs * gm_coef_bytes(G);
+}
+// Windows whose coefficients have a place: all of the ring, or where those do not fit (384 rows, four planes, groups of 128: 2 KB over) one,
+// filled when the decoders have taken the window before (384 x 28672 x 8192: 166 us in tiles that leave room for two, 151 so).
+__host__ __device__ constexpr int gm_coef_windows(int NX, int nx, bool EXACT, int S, int G) {
+    return NX == GM_WIDE && gm_smem_with(NX, nx, EXACT, S, G, gm_windows(NX, EXACT)) > GM_SMEM_MAX ? 1 : gm_windows(NX, EXACT);
+}
 __host__ __device__ constexpr int gm_smem(int NX, int nx, bool EXACT, int S, int G) {
-    return GM_HDR + gm_slots(NX, EXACT) * nx * 128 + gm_windows(NX, EXACT) * gm_window_bytes(S, G);
+    return gm_smem_with(NX, nx, EXACT, S, G, gm_coef_windows(NX, nx, EXACT, S, G));
 }
 static_assert(gm_smem(256, 256, false, 4, 128) <= GM_SMEM_MAX && gm_smem(256, 256, true, 4, 128) <= GM_SMEM_MAX &&
-              gm_smem(GM_WIDE, 384, false, 4, 256) <= GM_SMEM_MAX && gm_smem(GM_WIDE, 352, false, 4, 128) <= GM_SMEM_MAX, "shared memory");
+              gm_smem(GM_WIDE, 384, false, 4, 256) <= GM_SMEM_MAX && gm_smem(GM_WIDE, 384, false, 4, 128) <= GM_SMEM_MAX, "shared memory");
 
 struct GmParams {
     const uint32_t* bvr;
@@ -169,7 +178,9 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const __grid
     constexpr int SLOTS = gm_slots(NX, EXACT), WINDOWS = gm_windows(NX, EXACT);
     constexpr int ACOLS = EXACT ? 64 : 32;         // tensor-memory columns of a decoded tile
     constexpr int A_COL = gm_a_col(NX);
-    const uint32_t stage_bytes = (uint32_t)nx * 128, window_bytes = gm_window_bytes(S, p.G);
+    constexpr uint32_t word_bytes = gm_word_bytes(S);
+    const uint32_t stage_bytes = (uint32_t)nx * 128, coef_bytes = gm_coef_bytes(p.G);
+    const bool one_coef = NX == GM_WIDE && gm_coef_windows(NX, nx, EXACT, S, p.G) == 1;
     static_assert(A_COL + SLOTS * ACOLS <= GM_TMEM_COLS && NX <= A_COL, "tensor memory");
 
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);          // [SLOTS] activations landed and weight tile stored
@@ -181,7 +192,8 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const __grid
     volatile int* flags = reinterpret_cast<volatile int*>(p_empty + WINDOWS);      // [0] abort
     uint32_t* tmem_base_s = reinterpret_cast<uint32_t*>(smem + GM_HDR - 16);
     unsigned char* xs = smem + GM_HDR;                           // [SLOTS][stage_bytes]
-    unsigned char* ps = xs + SLOTS * stage_bytes;                // [WINDOWS][window_bytes]
+    unsigned char* ps = xs + SLOTS * stage_bytes;                // [WINDOWS][word_bytes]
+    unsigned char* cs = ps + WINDOWS * word_bytes;               // [WINDOWS, or one][coef_bytes]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     pdl_launch_dependents();
@@ -241,7 +253,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const __grid
             }
     };
     auto copy_words = [&](const Pos& a, int slot) {
-        const uint32_t dst = smem_u32(ps) + slot * window_bytes + (uint32_t)(lane * S * 4);
+        const uint32_t dst = smem_u32(ps) + slot * word_bytes + (uint32_t)(lane * S * 4);
         const int runs = 2 * stages_of(a.kb);
         const uint32_t* src[4];
 #pragma unroll
@@ -403,7 +415,14 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const __grid
             next(ahead), next(ahead);
             uint2 c1[2][4];
             load_coef(ahead, lines, c1);           // (its line numbers came with the window before)
-            const uint32_t dst = smem_u32(ps) + slot * window_bytes + 8 * 128 * S * 4;
+            if (one_coef) {                        // (the window before is in the other of two slots; the parity of its phase, which its warp has met)
+                static_assert(NX != GM_WIDE || WINDOWS == 2, "a window before in the other slot");
+                const int mine = warp - GM_PWARP;
+                if (flags[0] || !mbar_wait_timed(&p_empty[slot ^ 1], ph ^ (uint32_t)mine)) ok = false;
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+            }
+            const uint32_t dst = smem_u32(cs) + (one_coef ? 0 : slot * coef_bytes);
 #pragma unroll
             for (int t = 0; t < 2; ++t) {
                 if (t >= sets) break;
@@ -614,7 +633,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const __grid
             const int k1 = segs.k1(q);
             for (int kb = segs.k0(q); kb < k1; ++kb, ++wi) {
                 const int nst = stages_of(kb), slot = wi % WINDOWS;
-                const unsigned char* src = ps + slot * window_bytes;
+                const unsigned char *src = ps + slot * word_bytes, *csrc = cs + (one_coef ? 0 : slot * coef_bytes);
                 if (!dead && !mbar_wait_timed(&p_full[slot], (uint32_t)(wi / WINDOWS) & 1u)) {
                     dead = true;
                     flags[0] = 1;
@@ -623,7 +642,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) linear_gemm_kernel(const __grid
                 uint32_t w[2][S];
                 unsigned short c[4];
                 if (wg < nst) {
-                    const uint2 cc = *reinterpret_cast<const uint2*>(src + 8 * 128 * S * 4 + (p.G == 128 ? (wg >> 1) * 1024 : 0) + r * 8);
+                    const uint2 cc = *reinterpret_cast<const uint2*>(csrc + (p.G == 128 ? (wg >> 1) * 1024 : 0) + r * 8);
                     c[0] = (unsigned short)cc.x, c[1] = (unsigned short)(cc.x >> 16), c[2] = (unsigned short)cc.y, c[3] = (unsigned short)(cc.y >> 16);
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
@@ -811,7 +830,7 @@ static GmPlan gm_plan(const PackedW& w, int M, int sm_count, size_t scratch) {
     const bool exact = w.N % 128 != 0;
     GmPlan best = gm_plan_nx(w, M, (M <= 32 && !exact) ? 32 : M <= 64 ? 64 : M <= 128 ? 128 : 256, sm_count, scratch);
     if (M <= 256 || exact) return best;
-    for (int nx = 288; nx <= GM_WIDE && gm_smem(GM_WIDE, nx, false, w.S, w.G) <= GM_SMEM_MAX; nx += 32) {
+    for (int nx = 288; nx <= GM_WIDE; nx += 32) {
         const GmPlan pl = gm_plan_nx(w, M, nx, sm_count, scratch);
         if (pl.ns < best.ns) best = pl;
     }

@@ -9,6 +9,7 @@ two parts, off by 2^-21: the rounding of the result, 2.1e-4 in 2-norm, beside th
 import pytest
 import torch
 
+from launched import kernels
 from test_gpu_pair import errors, packed
 
 pytestmark = pytest.mark.gpu
@@ -43,6 +44,20 @@ def test_gemm(M, N, K, S, G, mode, bias):
     rel, top = errors(y, x, w, b)
     assert rel <= (5e-4 if N % 128 == 0 else 4e-4) and top <= 3e-3, (rel, top)
     assert torch.equal(y, sbvr.linear(x, w, b))    # sums in a fixed order
+
+
+@pytest.mark.parametrize("M,N,K", [(384, 14336, 768), (353, 13440, 1408), (384, 28672, 640), (380, 14336, 128)])
+def test_widest_tile_with_groups_of_128(M, N, K):
+    """Four planes, groups of 128: the coefficients of one window at a time beside a tile of 384 rows; windows of two stages, two tiles per CTA,
+    a single window."""
+    import sbvr
+    w, g = packed(N, K, 4, 128, "u16", M + K)
+    x = torch.randn((M, K), device="cuda", generator=g).half()
+    assert any("linear_gemm_kernelILi4ELi384E" in k for k in kernels(lambda: sbvr.linear(x, w)))
+    y = sbvr.linear(x, w)
+    rel, top = errors(y, x, w)
+    assert rel <= 5e-4 and top <= 3e-3, (rel, top)
+    assert torch.equal(y, sbvr.linear(x, w))
 
 
 @pytest.mark.parametrize("M,N,kin,offset", [(48, 2048, 1024, 2), (48, 2048, 1003, 0), (300, 14336, 509, 2), (100, 1000, 700, 2)])
