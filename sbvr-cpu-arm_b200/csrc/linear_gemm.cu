@@ -798,13 +798,21 @@ struct GmPlan {
     long long ns;
 };
 
-// Activation rows of a tile, and whether the tiles that are left over after whole rounds are cut: the least time in ns by these figures
-// (17 .. 384 rows, 1024 .. 28672 x 2048 .. 14336, S = 2 .. 4).  A 64-k stage takes its decoding, 150 + 50 S (in two parts 200 + 120 S), or
-// for many rows 1.05 a row + 40 S (2.1 a row + 120; beyond two rounds, with the clock at the
-// power limit, 1.15 a row and 1.2 in tiles of 256); a call 3 000 + 8 a row, another round's ends 1 500.  Cutting adds a launch, 5 000, and
-// 0.36 per KB of sums out and back.  Measured whole and cut, us, S = 4: 64 x 14336 x 4096 (112 tiles) 27.6, 30.8; 64 x 4096 x 14336 76.7, 29.1;
-// 64 x 4096 x 4096 23.6, 16.9; 64 x 28672 x 8192 95, 80.  More than 256 rows in two tiles and in one: 270 x 28672 x 8192 212, 119; 384 x 14336 x
-// 4096 62, 40; 384 x 4096 x 4096 28, 36.
+// Activation rows of a tile, and whether the tiles that are left over after whole rounds are cut: the least time in ns by these figures.
+// Up to 256 rows, and in two parts (17 .. 256 rows, 1024 .. 28672 x 2048 .. 14336, S = 2 .. 4): a 64-k stage takes its decoding, 150 + 50 S (in two
+// parts 200 + 120 S), or 1.05 a row + 40 S (2.1 a row + 120); a call 3 000 + 8 a row, another round's ends 1 500; cutting adds a launch, 5 000,
+// and 0.36 per KB of sums out and back.  Measured whole and cut, us, S = 4: 64 x 14336 x 4096 (112 tiles) 27.6, 30.8; 64 x 4096 x 14336 76.7, 29.1; 64 x
+// 4096 x 4096 23.6, 16.9; 64 x 28672 x 8192 95, 80.
+// More rows: see gm_many_ns.  270 x 28672 x 8192 in two tiles and in one 212, 119; 384 x 14336 x 4096 62, 40; 384 x 4096 x 4096 28, 36.
+//
+// gm_many_ns and the figures of gp_plan (linear_pair.cu), which decide between the kernels, were fitted to both kernels' times, this one's in tiles
+// of 256 .. 384 rows, at 499 sizes (257 .. 4096 rows, 1024 .. 28672 x 256 .. 14336, S = 2 .. 4, both group lengths): a choice by them costs 0.8 % on average
+// against the fastest of the six, 5 % and more at 25 sizes, 19 % at most.  (By figures that took 1 500 for the ends of every round it was 5.1 %, 129 sizes
+// and 51 %: a tile's results take 2 to 8 us out of D, in which this kernel's MMAs rest.)
+static long long gm_many_ns(int S, int nx, long long rounds, long long last, long long stages, int sm_count) {
+    const long long stage = (stages <= 200 ? 106 : 121) * nx / 100 + 26 * S;               // (longer runs meet the power limit)
+    return 6500 + stages * stage + (rounds - 1) * (2000 + 164 * nx / 10) + 147 * nx / 10 * last / sm_count;
+}
 static GmPlan gm_plan_nx(const PackedW& w, int M, int nx, int sm_count, size_t scratch) {
     GmPlan pl;
     pl.exact = w.N % 128 != 0;
@@ -812,16 +820,20 @@ static GmPlan gm_plan_nx(const PackedW& w, int M, int nx, int sm_count, size_t s
     pl.MT = (M + nx - 1) / nx;
     pl.tiles = (w.N + 127) / 128 * pl.MT;
     pl.KBS = (w.K + 255) / 256;
+    const bool many = M > 256 && !pl.exact;
     const long long call = 3000 + 8 * std::min(nx, 256), rounds = (pl.tiles + sm_count - 1) / sm_count;
-    const int row = rounds <= 2 ? 105 : nx > 256 ? 115 : 120;
+    const int row = rounds <= 2 ? 105 : 120;
     const long long stage = pl.exact ? std::max(200 + 120 * w.S, 21 * nx / 10 + 120) : std::max(150 + 50 * w.S, row * nx / 100 + 40 * w.S);
     pl.whole = true, pl.part_bytes = 0;
     pl.grid = std::min(pl.tiles, sm_count);
-    pl.ns = call + rounds * (w.K / 64 * stage + 1500) - 1500;
+    pl.ns = many ? gm_many_ns(w.S, nx, rounds, pl.tiles - (rounds - 1) * sm_count, rounds * (w.K / 64), sm_count)
+                 : call + rounds * (w.K / 64 * stage + 1500) - 1500;
     const long long windows = (long long)pl.tiles * pl.KBS, ctas = std::min<long long>(windows, sm_count), left = pl.tiles % ctas;
     if (left && left * pl.KBS >= ctas && left * pl.KBS * ctas < (1LL << 32)) {             // (every CTA has a window of them at least)
         const size_t bytes = (size_t)(ctas + left) * nx * 512;
-        const long long ns = call + 5000 + (windows + ctas - 1) / ctas * 4 * stage + (rounds - 1) * 1500 + (long long)(bytes * 9 / 25000);
+        const long long run = (windows + ctas - 1) / ctas * 4;
+        const long long ns = many ? gm_many_ns(w.S, nx, rounds, 0, run, sm_count) + (long long)(bytes / 2000)
+                                  : call + 5000 + run * stage + (rounds - 1) * 1500 + (long long)(bytes * 9 / 25000);
         if (ns < pl.ns && bytes <= scratch) pl.whole = false, pl.part_bytes = bytes, pl.grid = (int)ctas, pl.ns = ns;
     }
     return pl;

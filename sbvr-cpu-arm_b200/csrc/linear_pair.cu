@@ -684,9 +684,9 @@ struct GpPlan {
 };
 
 // Weight rows of an item, and whether the items that are left over after whole rounds are split over K: the least time in ns, by these
-// figures (bursts of calls, S = 2 and 4, n = 64 .. 256).  A 64-k stage of two blocks takes 160 + 20 S + 2.15 n (790 at n = 256, S = 4), at
-// least 560: the way of three stages of activations through L2 and back.  A launch and its ends take 8 000, another round's ends 1 500.
-// A split adds a launch, and 0.2 per KB of parts out and back (62 us against 79 at 512 x 8192 x 8192, n = 224: 37 items on 74 pairs).
+// figures (see also gm_many_ns, linear_gemm.cu).  A 64-k stage of two blocks takes 160 + 20 S + 2.15 n (790 at n = 256, S = 4), at least 560: the way of
+// three stages of activations through L2 and back.  A launch and its ends take 7 000, another round's ends 1 500 + 9 n, the last one's 6.5 n where
+// all pairs have an item.  A split adds a launch, 5 000, and 0.2 per KB of parts out and back.
 // The scratch it may count on is what sbvr_workspace_bytes promises, whatever the workspace has grown to for other calls.
 static GpPlan gp_plan(const PackedW& w, int M, int sm_count, int device, size_t scratch) {
     size_t promised = 0;
@@ -700,7 +700,9 @@ static GpPlan gp_plan(const PackedW& w, int M, int sm_count, int device, size_t 
         const long long NT = (w.N + n - 1) / n, items = NT * MT, full = odd ? items - NT : items, rounds = (items + pairs - 1) / pairs, left = items % pairs;
         if (items > (1 << 20)) continue;
         const long long long_ones = (full + pairs - 1) / pairs;                // rounds in which the first pair has an item of two blocks
-        GpPlan pl = {n, (int)items, (int)std::min(items, pairs), 1, 0, stages * (long_ones * stage + (rounds - long_ones) * half) + rounds * 1500 + 6500};
+        const long long end = 1500 + 9 * n;
+        GpPlan pl = {n, (int)items, (int)std::min(items, pairs), 1, 0, 0};
+        pl.ns = stages * (long_ones * stage + (rounds - long_ones) * half) + (rounds - 1) * end + 13 * n / 2 * (items - (rounds - 1) * pairs) / pairs + 7000;
         if (!best.n || pl.ns < best.ns) best = pl;
         if (left * NG < pairs || left * NG * pairs >= (1LL << 32)) continue;
         pl.part_bytes = (size_t)(pairs + left) * 16 * ((n + 31) / 32) * 4096;
@@ -708,7 +710,7 @@ static GpPlan gp_plan(const PackedW& w, int M, int sm_count, int device, size_t 
         const long long whole = items / pairs, whole_long = std::min(whole, long_ones);
         pl.ns = stages * (whole_long * stage + (whole - whole_long) * half) +
                 (left * stages + pairs - 1) / pairs * (full > whole * pairs ? stage : half) +              // (cut by steps, long and short)
-                (rounds + 1) * 1500 + 9500 + (long long)(pl.part_bytes / 5000);
+                whole * end + 12000 + (long long)(pl.part_bytes / 5000);
         if (pl.part_bytes <= scratch && pl.ns < best.ns) best = pl;
     }
     return best;

@@ -46,10 +46,10 @@ def test_gemm(M, N, K, S, G, mode, bias):
     assert torch.equal(y, sbvr.linear(x, w, b))    # sums in a fixed order
 
 
-@pytest.mark.parametrize("M,N,K", [(384, 14336, 768), (353, 13440, 1408), (384, 28672, 640), (380, 14336, 128)])
+@pytest.mark.parametrize("M,N,K", [(384, 14336, 2176), (353, 13440, 1408), (384, 28672, 2176), (384, 1024, 2176)])
 def test_widest_tile_with_groups_of_128(M, N, K):
     """Four planes, groups of 128: the coefficients of one window at a time beside a tile of 384 rows; windows of two stages, two tiles per CTA,
-    a single window."""
+    tiles that are cut."""
     import sbvr
     w, g = packed(N, K, 4, 128, "u16", M + K)
     x = torch.randn((M, K), device="cuda", generator=g).half()

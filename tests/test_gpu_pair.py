@@ -8,6 +8,8 @@ one-CTA kernel, 6e-4 of the largest; asserted 5e-4 and 3e-3.
 import pytest
 import torch
 
+from launched import kernels
+
 pytestmark = pytest.mark.gpu
 
 
@@ -31,6 +33,24 @@ def errors(y, x, w, b=None):
         ref += b.double()
     d = y.double() - ref
     return (d.norm() / ref.norm()).item(), (d.abs().max() / ref.abs().max()).item()
+
+
+@pytest.mark.parametrize("M,N,K,S,G,which", [      # us by the GEMM over CTA pairs and by the one-CTA GEMM
+    (1100, 14336, 2048, 4, 256, "pair"),           # 64, 71
+    (1100, 28672, 512, 4, 128, "pair"),            # 50, 61 in tiles of 384, 73 of 288
+    (768, 28672, 512, 3, 256, "pair"),             # 36, 47
+    (384, 1024, 4096, 3, 256, "gemm"),             # 22.8, 19.2
+    (600, 14336, 2176, 4, 128, "gemm"),            # 46.2, 46.2
+    (2048, 4096, 14336, 4, 256, "pair"),           # 171, 198
+    (300, 4096, 14336, 4, 256, "gemm"),            # 57, 41
+])
+def test_the_faster_kernel_is_chosen(M, N, K, S, G, which):
+    import sbvr
+    w, g = packed(N, K, S, G, "u16", 1)
+    x = torch.randn((M, K), device="cuda", generator=g).half()
+    want = {"pair": f"linear_pair_kernelILi{S}E", "gemm": f"linear_gemm_kernelILi{S}E"}[which]
+    names = kernels(lambda: sbvr.linear(x, w))
+    assert any(want in k for k in names), names
 
 
 @pytest.mark.parametrize("M,N,K,S,G,mode,bias", [
