@@ -31,8 +31,8 @@ pytestmark = pytest.mark.gpu
     (257, 1001, 4096, 4, 128, "u16", True),        # two tiles of 256, the second with one row
     (257, 14336, 512, 4, 256, "u16", True),        # more than 256 rows in one tile
     (300, 4096, 8192, 3, 128, "u8", False),
-    (352, 28672, 640, 4, 128, "u16", True),
-    (384, 14336, 768, 2, 256, "direct", False),
+    (352, 28672, 2176, 4, 128, "u16", True),
+    (384, 14336, 1536, 2, 256, "direct", False),
     (700, 8192, 1280, 4, 256, "u8", True),
 ])
 def test_gemm(M, N, K, S, G, mode, bias):
@@ -40,6 +40,7 @@ def test_gemm(M, N, K, S, G, mode, bias):
     w, g = packed(N, K, S, G, mode, M + N + K)
     x = torch.randn((M, K), device="cuda", generator=g).half()
     b = torch.randn(N, device="cuda", generator=g).half() if bias else None
+    assert any(f"linear_gemm_kernelILi{S}E" in k for k in kernels(lambda: sbvr.linear(x, w, b)))
     y = sbvr.linear(x, w, b)
     rel, top = errors(y, x, w, b)
     assert rel <= (5e-4 if N % 128 == 0 else 4e-4) and top <= 3e-3, (rel, top)

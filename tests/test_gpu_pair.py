@@ -1,9 +1,9 @@
 """The GEMM over CTA pairs (csrc/linear_pair.cu), which the automatic choice takes for many activation rows: edges of its blocks of 256
 activation rows, item widths that do not divide N, items split over K, every encoding, and the calls that stay with the one-CTA kernel.
 
-Sizes are such that the estimate picks it.  Bound: weights are formed in fp16 with one rounding per plane (a weight is off by at most S fp16
-roundings of a partial sum, 2^-11 each), sums are fp32, the result is rounded to fp16: 3.4e-4 of the result in 2-norm at S = 4 as for the
-one-CTA kernel, 6e-4 of the largest; asserted 5e-4 and 3e-3.
+Every case asserts which kernel it runs, so that a rule that moves does not leave this file empty.  Bound: weights are formed in fp16 with one
+rounding per plane (a weight is off by at most S fp16 roundings of a partial sum, 2^-11 each), sums are fp32, the result is rounded to fp16:
+3.4e-4 of the result in 2-norm at S = 4 as for the one-CTA kernel, 6e-4 of the largest; asserted 5e-4 and 3e-3.
 """
 import pytest
 import torch
@@ -48,34 +48,62 @@ def test_the_faster_kernel_is_chosen(M, N, K, S, G, which):
     import sbvr
     w, g = packed(N, K, S, G, "u16", 1)
     x = torch.randn((M, K), device="cuda", generator=g).half()
-    want = {"pair": f"linear_pair_kernelILi{S}E", "gemm": f"linear_gemm_kernelILi{S}E"}[which]
-    names = kernels(lambda: sbvr.linear(x, w))
-    assert any(want in k for k in names), names
+    runs(lambda: sbvr.linear(x, w), which == "pair", S)
 
 
-@pytest.mark.parametrize("M,N,K,S,G,mode,bias", [
-    (257, 28672, 256, 4, 256, "u16", False),       # one row in the second block; a single group
-    (512, 28672, 256, 2, 256, "u8", True),         # both blocks full
-    (513, 28672, 384, 3, 128, "direct", False),    # one row in the third block, an odd number of groups of 128
-    (600, 14336, 2176, 4, 128, "u16", True),       # 17 groups of 128: every slot of their ring several times
-    (768, 14464, 512, 4, 256, "direct", True),     # items of one block; 113 tiles of 128 rows, a last item that is narrower
-    (1000, 9600, 1536, 3, 256, "u16", True),
-    (1030, 13440, 2048, 2, 128, "u8", False),
-    (2048, 1024, 4096, 4, 256, "u16", True),       # fewer items than pairs: all split over K
-    (300, 4096, 14336, 4, 256, "u8", False),
-    (700, 1152, 14336, 3, 128, "u16", True),
-    (3000, 4096, 3072, 2, 256, "u16", False),      # whole rounds and split items
-    (2048, 4096, 4000, 4, 256, "u16", False),      # K padded to the group: x ends before the weight
-])
-def test_pair_gemm(M, N, K, S, G, mode, bias):
+def runs(call, pair, S, cut=None):
+    """Asserts which GEMM `call` runs, and whether (`cut`) sums of items that several pairs share are added."""
+    names = kernels(call)
+    assert any(f"linear_pair_kernelILi{S}E" in k for k in names) == pair and any("linear_gemm_kernel" in k for k in names) != pair, names
+    assert cut is None or any("gp_add_kernel" in k for k in names) == cut, names
+
+
+def product(M, N, K, S, G, mode, bias, pair, cut=None):
     import sbvr
     w, g = packed(N, K, S, G, mode, M + N + K)
     x = torch.randn((M, K), device="cuda", generator=g).half()
     b = torch.randn(N, device="cuda", generator=g).half() if bias else None
+    runs(lambda: sbvr.linear(x, w, b), pair, S, cut)
     y = sbvr.linear(x, w, b)
     rel, top = errors(y, x, w, b)
     assert rel <= 5e-4 and top <= 3e-3, (rel, top)
     assert torch.equal(y, sbvr.linear(x, w, b))    # sums in a fixed order
+
+
+@pytest.mark.parametrize("M,N,K,S,G,mode,bias,cut", [
+    (257, 28672, 256, 4, 256, "u16", False, False),            # one row in the second block; a single group
+    (512, 28672, 256, 2, 256, "u8", True, False),              # both blocks full
+    (513, 28672, 384, 3, 128, "direct", False, False),         # one row in the third block, an odd number of groups of 128
+    (768, 14464, 512, 4, 256, "direct", True, False),          # items of one block; 113 tiles of 128 rows, a last item that is narrower
+    (768, 7168, 768, 4, 128, "u8", False, False),
+    (448, 14336, 768, 4, 256, "u16", True, False),             # a last block that is not full
+    (1000, 9600, 1536, 3, 256, "u16", True, False),
+    (1280, 6016, 1408, 4, 128, "u16", True, False),            # 11 groups of 128: every slot of their ring several times; items of one block last
+    (1280, 5760, 1408, 2, 128, "direct", False, False),
+    (1800, 4224, 2432, 4, 128, "direct", True, False),         # 19 groups
+    (1280, 28672, 512, 3, 256, "u8", True, False),             # five rounds of items
+    (2048, 4096, 4000, 4, 256, "u16", False, False),           # K padded to the group: x ends before the weight
+    (511, 1024, 2432, 4, 128, "u16", True, True),              # fewer items than pairs: all split over K
+    (512, 640, 3968, 3, 128, "direct", False, True),           # 31 groups
+    (511, 1152, 2304, 3, 256, "u8", True, True),
+    (512, 896, 2816, 2, 256, "u16", False, True),              # a last item that is narrower
+    (768, 768, 2304, 4, 256, "direct", True, True),            # items of one block, split
+    (1000, 9600, 4352, 4, 256, "u16", True, True),             # whole rounds and split items
+])
+def test_pair_gemm(M, N, K, S, G, mode, bias, cut):
+    product(M, N, K, S, G, mode, bias, True, cut)
+
+
+@pytest.mark.parametrize("M,N,K,S,G,mode,bias", [
+    (600, 14336, 2176, 4, 128, "u16", True),
+    (1030, 13440, 2048, 2, 128, "u8", False),
+    (2048, 1024, 4096, 4, 256, "u16", True),
+    (300, 4096, 14336, 4, 256, "u8", False),
+    (700, 1152, 14336, 3, 128, "u16", True),
+    (3000, 4096, 3072, 2, 256, "u16", False),
+])
+def test_sizes_that_the_one_cta_kernel_serves(M, N, K, S, G, mode, bias):
+    product(M, N, K, S, G, mode, bias, False)
 
 
 def test_pair_gemm_large_coefficients_and_special_rows():
@@ -83,6 +111,7 @@ def test_pair_gemm_large_coefficients_and_special_rows():
     import sbvr
     w, g = packed(28672, 512, 4, 256, "u16", 5, scale=4.0)
     x = torch.randn((600, 512), device="cuda", generator=g).half() * 0.01
+    runs(lambda: sbvr.linear(x, w), True, 4)
     clean = sbvr.linear(x, w)
     rel, top = errors(clean, x, w)
     assert rel <= 6e-4 and top <= 3e-3, (rel, top)          # (sums of coefficients of either sign: partial sums are larger than weights)
@@ -105,12 +134,13 @@ def test_calls_that_the_copies_cannot_serve(case):
     out = None
     if case == "y off by 2 bytes":
         out = torch.empty(512 * 28672 + 1, dtype=torch.float16, device="cuda")[1:].view(512, 28672)
+    runs(lambda: sbvr.linear(x, w, None, out=out), False, 4)
     y = sbvr.linear(x, w, None, out=out) if out is not None else sbvr.linear(x, w)
     rel, top = errors(y, x, w)
     assert rel <= 5e-4 and top <= 3e-3, (rel, top)
 
 
-@pytest.mark.parametrize("M,N,K", [(300, 14336, 512), (40, 512, 2048)])
+@pytest.mark.parametrize("M,N,K", [(300, 14336, 512), (448, 14336, 512), (40, 512, 2048)])
 def test_first_call_of_a_thread(M, N, K):
     """The first thing that a thread does on the GPU: the tensor map of x is a driver call, which needs the thread's context."""
     import threading
