@@ -269,7 +269,8 @@ SBVR_API int sbvr_add_rmsnorm_f16(const void* h_in, const void* delta, const voi
  * append of the rotated k and of v to the caches [seqs][n_kv][max_ctx][head_dim] at positions[token]
  * (int32; sequence = token / tokens_per_seq).  cos/sin = fp16(cos|sin(pos * inv_freq[i]) * attn_scaling),
  * products and sum in fp16: LlamaRotaryEmbedding.forward, rotate_half, apply_rotary_pos_emb
- * (models/sbvr_llama.py:169-224) and the cache update of LlamaAttention.forward (:330-336). */
+ * (models/sbvr_llama.py:169-224) and the cache update of LlamaAttention.forward (:330-336).
+ * head_dim even, at most 512 (SBVR_ERR_UNSUPPORTED above). */
 SBVR_API int sbvr_rope_append_f16(void* qkv, const int* positions, const float* inv_freq, float attn_scaling,
                                   void* kcache, void* vcache, int tokens, int tokens_per_seq, int n_heads, int n_kv,
                                   int head_dim, int max_ctx, sbvr_stream_t stream);

@@ -83,11 +83,13 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(const __half* h_in, co
 // rotary embedding of q and k in place + append of k, v to the cache            one CTA per token
 //   qkv row: [n_heads * d | n_kv * d | n_kv * d];  cache [seq, n_kv, max_ctx, d]
 // ---------------------------------------------------------------------------------------------
+constexpr int ROPE_HALF = 256;                     // head_dim / 2 at most
+
 __global__ void __launch_bounds__(256) rope_append_kernel(__half* __restrict__ qkv, const int* __restrict__ positions,
                                                           const float* __restrict__ inv_freq, float attn_scaling,
                                                           __half* __restrict__ kcache, __half* __restrict__ vcache,
                                                           int tokens_per_seq, int n_heads, int n_kv, int d, int max_ctx) {
-    __shared__ __half cs_s[2][256];                // cos, sin of this token's position for i < head_dim / 2 <= 256
+    __shared__ __half cs_s[2][ROPE_HALF];          // cos, sin of this token's position for i < head_dim / 2
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x;
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(256) rope_append_vec_kernel(__half* __restrict
                                                               const float* __restrict__ inv_freq, float attn_scaling,
                                                               __half* __restrict__ kcache, __half* __restrict__ vcache,
                                                               int tokens_per_seq, int n_heads, int n_kv, int d, int max_ctx) {
-    __shared__ __align__(16) __half cs_s[2][256];
+    __shared__ __align__(16) __half cs_s[2][ROPE_HALF];
     pdl_launch_dependents();
     pdl_wait();
     const int t = blockIdx.x, half_d = d / 2, ch = half_d / 8;
@@ -793,6 +795,7 @@ int sbvr_rope_append_f16(void* qkv, const int* positions, const float* inv_freq,
     if (tokens < 1 || tokens_per_seq < 1 || tokens % tokens_per_seq || n_heads < 1 || n_kv < 1 || head_dim < 2 ||
         head_dim % 2 || max_ctx < 1)
         return SBVR_ERR_BAD_ARG;
+    if (head_dim > 2 * ROPE_HALF) return SBVR_ERR_UNSUPPORTED;
     const bool vec = head_dim % 16 == 0 && !((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kcache) |
                                               reinterpret_cast<uintptr_t>(vcache)) & 15);
     SBVR_CUDA_TRY(launch_pdl(vec ? rope_append_vec_kernel : rope_append_kernel, dim3(tokens), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream),

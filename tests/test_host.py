@@ -170,6 +170,14 @@ def test_glue_and_fused_entry_points_validate_before_any_cuda_call():
     assert L.sbvr_workspace_bytes(0, 0, 64, 256, ctypes.byref(out)) == -1
 
 
+@pytest.mark.parametrize("head_dim", [514, 528, 1024, 4096])
+def test_rope_refuses_heads_longer_than_its_table(head_dim):
+    """The kernels hold the cosines and sines of 256 angles: a longer head is refused by the host, before anything is launched."""
+    from sbvr import _lib
+    p = ctypes.addressof((ctypes.c_uint32 * 64)())
+    assert _lib.lib.sbvr_rope_append_f16(p, p, p, 1.0, p, p, 1, 1, 1, 1, head_dim, 64, None) == -7
+
+
 def test_encoder_config_and_search_space_on_cpu():
     """Host side of the encoder: unknown keys are ignored, unsupported settings are refused, and the candidate lines of a
     group have the reference's counts (r x b x s lists plus the plain grid; sbvr/core.py:400-483) and are sorted by
