@@ -416,13 +416,9 @@ __global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const __gri
     if (warp == AQ_IWARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(AQ_COLS) : "memory");
 }
 
-// Setting up costs 3 us more than in attention_prefill_kernel, a tile of keys 1 us less, and that kernel has two blocks of 64 pairs on an SM.
-// us, here and there, 32 query heads, 8 KV heads: 1 x 64 tokens 7.4, 4.5; 1 x 128 8.2, 7.2; 1 x 160 9.0, 8.7; 1 x 192 8.9, 10.2; 1 x 256 9.7, 12.6; 2 x 128
-// 8.2, 8.6; 8 x 64 7.7, 6.8; 12 x 64 9.5, 10.1; 4 heads, 4 KV heads: 1 x 200 8.8, 7.6.
-bool attention_tc_supported(const void* qkv, const void* out, int tokens, int tokens_per_seq, int n_kv, int R) {
+bool attention_tc_supported(const void* qkv, const void* out, int tokens, int tokens_per_seq, int n_kv, int R, int sm_count) {
     if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(out)) & 15) return false;
-    const long long blocks = (long long)(tokens / tokens_per_seq) * n_kv * (((long long)tokens_per_seq * R + 63) / 64);
-    return tokens_per_seq >= 256 || blocks > 2 * 148 || (tokens_per_seq >= 128 && blocks >= 96);
+    return attention_tc_faster((long long)(tokens / tokens_per_seq) * n_kv * (((long long)tokens_per_seq * R + 63) / 64), tokens_per_seq, sm_count);
 }
 
 int launch_attention_tc(const __half* qkv, const __half* kcache, const __half* vcache, const int* positions, __half* out, int tokens,

@@ -175,7 +175,13 @@ int launch_linear_gemm(const __half* x, int Kin, const PackedW& w, const __half*
                        const sbvr_workspace* ws, cudaStream_t st);
 
 // Prefill attention on the tensor cores (attention_prefill.cu); R: query heads of a KV head, a power of two
-bool attention_tc_supported(const void* qkv, const void* out, int tokens, int tokens_per_seq, int n_kv, int R);
+bool attention_tc_supported(const void* qkv, const void* out, int tokens, int tokens_per_seq, int n_kv, int R, int sm_count);
+// Whether it is faster than attention_prefill_kernel (glue.cu), which has `blocks` blocks of 64 (token, query head) pairs, two on an SM.  Setting up
+// costs 3 us more there, a tile of keys 1 us less.  us, there and here, 148 SMs, 32 query heads, 8 KV heads: 1 x 64 tokens 7.4, 4.5; 1 x 128 8.2, 7.2;
+// 1 x 160 9.0, 8.7; 1 x 192 8.9, 10.2; 1 x 256 9.7, 12.6; 2 x 128 8.2, 8.6; 8 x 64 7.7, 6.8; 12 x 64 9.5, 10.1; 4 heads, 4 KV heads: 1 x 200 8.8, 7.6.
+inline bool attention_tc_faster(long long blocks, int tokens_per_seq, int sm_count) {
+    return tokens_per_seq >= 256 || blocks > 2LL * sm_count || (tokens_per_seq >= 128 && 37 * blocks >= 24LL * sm_count);      // (96 blocks on 148)
+}
 int launch_attention_tc(const __half* qkv, const __half* kcache, const __half* vcache, const int* positions, __half* out, int tokens,
                         int tokens_per_seq, int n_heads, int n_kv, int max_ctx, float scale, cudaStream_t st);
 

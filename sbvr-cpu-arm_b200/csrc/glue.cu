@@ -823,7 +823,12 @@ static int attention_launch(const void* qkv, void* kcache, void* vcache, const i
     __half* o = reinterpret_cast<__half*>(out);
     if (!inv_freq && nsplit == 1 && tokens_per_seq >= 8) {      // prefill: tokens of a sequence share K / V fetches
         if (R != 1 && R != 2 && R != 4 && R != 8) return SBVR_ERR_UNSUPPORTED;
-        if (attention_tc_supported(qkv, out, tokens, tokens_per_seq, n_kv, R))
+        DeviceInfo di;
+        int dev = 0;
+        SBVR_CUDA_TRY(cudaGetDevice(&dev));
+        const int rc = device_info(dev, &di);
+        if (rc) return rc;
+        if (attention_tc_supported(qkv, out, tokens, tokens_per_seq, n_kv, R, di.sm_count))
             return launch_attention_tc(q, kc, vc, positions, o, tokens, tokens_per_seq, n_heads, n_kv, max_ctx, scale, st);
         const int QT = AP_ROWS / R, nblk = (tokens_per_seq + QT - 1) / QT;
         const dim3 bgrid((unsigned)((tokens / tokens_per_seq) * n_kv * nblk));

@@ -249,23 +249,33 @@ def test_search_settings_the_kernel_does_not_cover():
     assert not encoder._SearchTables(encoder.EncoderConfig(num_sums=2, r_search_num=200, b_search_num=200, s_search_num=200), cpu).covered
 
 
-def test_step_partition_of_the_streaming_kernels(tmp_path):
-    """The split of (tile, k step) work over the CTAs that the decode GEMV and the small-batch kernel share (TsSegs in
-    csrc/tc_stream.cuh) is compiled for the host and checked over a few thousand (tiles, steps, CTAs) combinations: every
-    step owned once, shared segments first and at most two per CTA, owners of the left-over steps as cta_of() says."""
+def native_check(tmp_path, name):
+    """Compiles tests/native/<name>.cu for the host and runs it."""
     import shutil
     import subprocess
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     if not os.path.exists(nvcc):
         pytest.skip("nvcc not available")
-    exe = str(tmp_path / "partition_check")
-    src = os.path.join(ROOT, "tests", "native", "partition_check.cu")
+    exe = str(tmp_path / name)
+    src = os.path.join(ROOT, "tests", "native", name + ".cu")
     subprocess.check_call([nvcc, "-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=sm_100a",
                            "-I", os.path.join(ROOT, "include"), "-I", os.path.join(ROOT, "sbvr-cpu-arm_b200", "csrc"),
                            "-o", exe, src])
     out = subprocess.run([exe], capture_output=True, text=True)
     assert out.returncode == 0, out.stdout[-2000:]
     assert "0 failures" in out.stdout
+
+
+def test_step_partition_of_the_streaming_kernels(tmp_path):
+    """The split of (tile, k step) work over the CTAs that the decode GEMV and the small-batch kernel share (TsSegs in
+    csrc/tc_stream.cuh) is compiled for the host and checked over a few thousand (tiles, steps, CTAs) combinations: every
+    step owned once, shared segments first and at most two per CTA, owners of the left-over steps as cta_of() says."""
+    native_check(tmp_path, "partition_check")
+
+
+def test_rule_between_the_prefill_attention_kernels(tmp_path):
+    """Its lines follow the number of SMs of the device."""
+    native_check(tmp_path, "attention_rule_check")
 
 
 def test_encoder_cutoff_is_the_same_sum_on_every_interpreter(monkeypatch):
