@@ -17,8 +17,8 @@
 // the last key).  S and the weights of two
 // tiles (64 columns each) and O take 256 columns of tensor memory, 97 KB of shared memory: two CTAs per SM, so that one computes weights while
 // the other has the tensor pipe.  Tensor memory is only asked for when the kernel in front has ended, and the kernel behind may start only
-// when this one has it: neither can wait for columns that the other holds while the other waits for it to end.  Every wait is bounded; after
-// a time-out the CTA's results are NaN.
+// when this one has it: neither can wait for columns that the other holds while the other waits for it to end.  Every wait is bounded; a CTA in
+// which one runs out multiplies its pairs out without the tensor cores.
 //
 // What bounds it: the weights, about 600 instructions and 64 exponentials per thread and tile, on two warps per scheduler; the tensor pipe
 // would take 768 cycles a tile, 26 us at 2 x 1500 tokens.  Per layer, 32 query heads, 8 KV heads, us (mma.sync on blocks of 64, in
@@ -109,8 +109,8 @@ __device__ __forceinline__ float aq_exp2(float x) {
     return y;
 }
 
-// A CTA among whose keys values are not finite that only some of its tokens attend to: all of its pairs once more, a warp each, four dims a
-// lane, key by key as far as the token goes.
+// A CTA in which a wait has run out, or among whose keys values are not finite that only some of its tokens attend to: all of its pairs (once
+// more), a warp each, four dims a lane, key by key as far as the token goes.
 __device__ __noinline__ void aq_multiply_out(const AqParams& p, uint32_t q_s, const int* ctx_s, int t0, int nq, int seq, int kvh) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, R = 1 << p.r_shift;
     const float sl2 = (p.scale == 0.0f ? 1.0f : fabsf(p.scale)) * 1.4426950408889634f;
@@ -264,11 +264,7 @@ __global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const __gri
                 __syncwarp();
             }
         }
-        if (!ok) {                                               // copies that were issued land before the CTA leaves
-            *dead_s = 1;
-            const long long c0 = clock64();
-            while (clock64() - c0 < (1LL << 22)) {}
-        }
+        if (!ok) *dead_s = 1;
     } else if (warp == AQ_IWARP) {
         // ------------------------------ MMA issuer ------------------------------
         if (elect_one()) {
@@ -384,10 +380,10 @@ __global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const __gri
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) *dead_s = 1;
         aq_fence_after();
-        const float inv = !ok ? NAN : sum > 0.0f ? 1.0f / sum : 0.0f;
+        const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
         __half* dst = p.out + ((size_t)(t0 + min(j, nq - 1)) * p.n_heads + kvh * R + (row & (R - 1))) * AQ_D;
 #pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
+        for (int c = 0; c < 4 && ok; ++c) {
             uint32_t o[32];
             aq_ld32(mine + AQ_O_COL + c * 32, o);
             aq_ld_wait(o);
@@ -412,7 +408,11 @@ __global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const __gri
     // ------------------------------ teardown ------------------------------
     __syncthreads();
     aq_fence_after();
-    if (*odd_s && !*dead_s) aq_multiply_out(p, q_s, ctx_s, t0, nq, seq, kvh);
+    if (*dead_s) {                                               // copies that were issued land before the CTA leaves
+        const long long c0 = clock64();
+        while (clock64() - c0 < (1LL << 22)) {}
+    }
+    if (*odd_s || *dead_s) aq_multiply_out(p, q_s, ctx_s, t0, nq, seq, kvh);
     if (warp == AQ_IWARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(AQ_COLS) : "memory");
 }
 

@@ -98,3 +98,38 @@ def test_values_that_are_not_finite_stay_with_the_tokens_that_see_them():
     assert not seen[20:, :, 3].any() and seen[:20].all() and seen[:, :, :3].all() and seen[:, :, 4:].all()
     e = torch.where(seen, a.double() - b.double(), torch.zeros_like(b.double()))
     assert e.abs().max() / b.abs().max() < 1e-3    # (one fp16 rounding each)
+
+
+@pytest.fixture(scope="module")
+def impatient(tmp_path_factory):
+    """The kernel with a wait that runs out (tests/native/attention_timeout.cu)."""
+    import ctypes
+    import os
+    import shutil
+    import subprocess
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    so = str(tmp_path_factory.mktemp("native") / "attention_timeout.so")
+    subprocess.check_call([nvcc, "-std=c++17", "-O3", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-Xcompiler", "-fPIC",
+                           "-I", os.path.join(root, "include"), "-I", os.path.join(root, "sbvr-cpu-arm_b200", "csrc"),
+                           "-o", so, os.path.join(root, "tests", "native", "attention_timeout.cu")])
+    f = ctypes.CDLL(so).attention_with_a_wait_that_runs_out
+    f.argtypes = [ctypes.c_void_p] * 5 + [ctypes.c_int] * 5 + [ctypes.c_float] + [ctypes.c_int] * 3 + [ctypes.c_void_p]
+    return f
+
+
+@pytest.mark.parametrize("warp,bar,parity", [
+    (4, 0, 0), (4, 1, 1), (4, 2, 1), (4, 8, 0),    # the issuer's wait for the first and the fourth tile of K, the third of V, the first weights
+    (5, 4, 0), (6, 7, 0),                          # the warps that bring K and V, for a place
+    (2, 5, 1), (0, 4, 0), (3, 6, 0),               # warps that form weights: for scores, for the output
+])
+def test_a_wait_that_runs_out_costs_time_and_no_result(impatient, warp, bar, parity):
+    qkv, K, V, _ = inputs(2, 300, 8, 2, 310, 7)
+    pos = (torch.arange(300, device="cuda", dtype=torch.int32) + 8).repeat(2)
+    out = torch.full((600, 8 * D), float("nan"), dtype=torch.float16, device="cuda")
+    rc = impatient(qkv.data_ptr(), K.data_ptr(), V.data_ptr(), pos.data_ptr(), out.data_ptr(), 600, 300, 8, 2, 310, D ** -0.5, warp, bar, parity,
+                   torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    close(out, oracle(qkv, K, V, pos, 300, 8, 2))
