@@ -17,6 +17,12 @@
  *   W[n][k] = fp16_rn( sum_s float(line(k/G, n)[s]) * bit_s[n][k] )        (plane order, fp32)
  *
  * G (group length along K) is 256 in the reference (sbvr/core.py:222); 128 is also accepted.
+ *
+ * Kernels are launched with programmatic stream serialization and read packed weights (bvr, coeff_idx, coeff) ahead of their wait for the work
+ * in front of them on the stream; everything else (activations, residuals, scratch, results) behind it.  A weight may be rewritten on the
+ * stream right before a call by anything that lets its successor start only at its end: copies, ordinary kernels, and all that this library
+ * does.  A kernel that executes griddepcontrol.launch_dependents (cudaTriggerProgrammaticLaunchCompletion) before its last write to a weight
+ * must be followed by an event or another stream-ordered operation without that attribute.
  * fp16 values are passed as `const void*` / `void*` pointing at IEEE binary16 data.
  */
 #ifndef SBVR_B200_H
