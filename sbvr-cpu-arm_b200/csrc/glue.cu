@@ -8,6 +8,8 @@
 // probabilities to fp16), which is inside the 1e-2 tolerance of the layer outputs.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace sbvr {
@@ -662,13 +664,13 @@ __global__ void embedding_kernel(const int* __restrict__ ids, const __half* __re
 }
 
 // rows of Kin halves -> rows of K (K % 8 == 0), zeros behind; one thread per 8 output elements, any Kin
-__global__ void __launch_bounds__(256) pad_rows_kernel(const __half* __restrict__ in, __half* __restrict__ out, int M, int Kin,
-                                                       int K) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS, 2048 / THREADS) pad_rows_kernel(const __half* __restrict__ in, __half* __restrict__ out, int M, int Kin, int K) {
     pdl_launch_dependents();
     pdl_wait();
     const int kv = K / 8;
     const size_t nvec = (size_t)M * kv;
-    for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += (size_t)gridDim.x * blockDim.x) {
+    for (size_t v = (size_t)blockIdx.x * THREADS + threadIdx.x; v < nvec; v += (size_t)gridDim.x * THREADS) {
         const size_t m = v / kv;
         const int k0 = (int)(v - m * kv) * 8;
         __align__(16) __half o[8];
@@ -678,10 +680,17 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(const __half* __restrict_
     }
 }
 
+// Few rows: blocks of 128 threads with 32 registers, which find room beside a CTA of the GEMM in front and leave room for one of the GEMM behind
+// (70 x 18945 x 415, S = 3, 25.4 us with blocks of 256, 23.8 so; 300 x 16146 x 415 31.5, 29.7; 64 x 4096 x 4095 20.5, 20.3).  More: blocks of 256, which
+// copy faster (2048 x 4096 x 4095 71.1 us, 73.4 with blocks of 128).
+constexpr size_t PAD_FEW = 76 * 1024;              // pieces of 16 bytes: four blocks of 128 per SM
 int launch_pad_rows(const __half* in, __half* out, int M, int Kin, int K, cudaStream_t st) {
     if (K % 8) return SBVR_ERR_SHAPE;
-    const size_t blocks = ((size_t)M * (K / 8) + 255) / 256;
-    SBVR_CUDA_TRY(launch_pdl(pad_rows_kernel, dim3((unsigned)(blocks < 2368 ? blocks : 2368)), dim3(256), 0, st, in, out, M, Kin, K));
+    const size_t nvec = (size_t)M * (K / 8);
+    if (nvec <= PAD_FEW)
+        SBVR_CUDA_TRY(launch_pdl(pad_rows_kernel<128>, dim3((unsigned)((nvec + 127) / 128)), dim3(128), 0, st, in, out, M, Kin, K));
+    else
+        SBVR_CUDA_TRY(launch_pdl(pad_rows_kernel<256>, dim3((unsigned)std::min<size_t>((nvec + 255) / 256, 2368)), dim3(256), 0, st, in, out, M, Kin, K));
     return SBVR_OK;
 }
 

@@ -61,7 +61,8 @@ def test_widest_tile_with_groups_of_128(M, N, K):
     assert torch.equal(y, sbvr.linear(x, w))
 
 
-@pytest.mark.parametrize("M,N,kin,offset", [(48, 2048, 1024, 2), (48, 2048, 1003, 0), (300, 14336, 509, 2), (100, 1000, 700, 2)])
+@pytest.mark.parametrize("M,N,kin,offset", [(48, 2048, 1024, 2), (48, 2048, 1003, 0), (300, 14336, 509, 2), (100, 1000, 700, 2),
+                                             (19, 500, 255, 0), (152, 256, 4095, 0), (153, 256, 4089, 2)])
 def test_activations_that_tma_cannot_read(M, N, kin, offset):
     """x off by 4 bytes, rows of a length that is no multiple of 16 bytes: a copy is read instead, the same values."""
     import sbvr
