@@ -296,8 +296,8 @@ static int linear_any(const void* x, int Kin, const uint32_t* bvr, const void* c
         }
     }
     // Algo 4 takes up to 32 rows (16 with groups of 128); beyond sixteen the GEMM does the work, on the weights the kernel takes.  The
-    // kernel's form for them (six digits) took 37 us at 14336 x 4096, M = 32, S = 4, 51 at 4096 x 14336 and 17.4 at 4096 x 4096,
-    // against the GEMM's 33, 34 and 16.
+    // form that the kernel once had for them (six digits) took 37 us at 14336 x 4096, M = 32, S = 4, 51 at 4096 x 14336 and 17.4 at 4096 x
+    // 4096; the GEMM takes 28, 27 and 15.
     if (algo == 4 && M > 16) {
         if (M > 32 || w.G != 256 || !linear_sb_supported(w, 16)) return SBVR_ERR_UNSUPPORTED;
         algo = 3;

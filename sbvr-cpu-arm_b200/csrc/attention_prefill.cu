@@ -277,7 +277,8 @@ __global__ void __launch_bounds__(AQ_THREADS, 2) attention_tc_kernel(const __gri
                 aq_fence_after();
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    aq_mma_ss(tbase + b * 64, qd + (k >> 2) * (AQ_QBOX >> 4) + (k & 3) * 2, kd + b * (AQ_TILE >> 4) + (k >> 2) * (AQ_KBOX >> 4) + (k & 3) * 2, QK, k ? 1u : 0u);
+                    aq_mma_ss(tbase + b * 64, qd + (k >> 2) * (AQ_QBOX >> 4) + (k & 3) * 2,
+                              kd + b * (AQ_TILE >> 4) + (k >> 2) * (AQ_KBOX >> 4) + (k & 3) * 2, QK, k ? 1u : 0u);
                 aq_commit(s_full + b);
                 return true;
             };
@@ -434,7 +435,8 @@ int launch_attention_tc(const __half* qkv, const __half* kcache, const __half* v
     if (!err) err = ts_map_2d(&vmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, CU_TENSOR_MAP_SWIZZLE_128B, vcache, rows, AQ_D, AQ_D * 2, AQ_KEYS, 64);
     if (err) return err;
     const int QT = AQ_ROWS >> p.r_shift, nblk = (tokens_per_seq + QT - 1) / QT;
-    SBVR_CUDA_TRY(launch_pdl(attention_tc_kernel, dim3((unsigned)((tokens / tokens_per_seq) * n_kv * nblk)), dim3(AQ_THREADS), (size_t)AQ_SMEM, st, kmap, vmap, p));
+    const unsigned blocks = (unsigned)((tokens / tokens_per_seq) * n_kv * nblk);
+    SBVR_CUDA_TRY(launch_pdl(attention_tc_kernel, dim3(blocks), dim3(AQ_THREADS), (size_t)AQ_SMEM, st, kmap, vmap, p));
     return SBVR_OK;
 }
 

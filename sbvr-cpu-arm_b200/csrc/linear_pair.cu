@@ -7,9 +7,10 @@
 // 256 to 384 activation rows (512 to 768 cycles of tensor time).  Here two SMs share one MMA (`cta_group::2`): each decodes HALF of the
 // tile's weight rows into its own shared memory, where the MMAs of both read them, and a decoded row serves 2 x 256 activation rows, so
 // that a stage is up to 1024 cycles of tensor time for the same decoding.  What bounds this kernel is the power limit (the clock falls to
-// 1.35 .. 1.5 GHz with the tensor pipe 85 % busy).  S = 4, us in bursts of eight calls, with the one-CTA kernel's time and that of a dense
-// fp16 product of the same shape by cuBLAS: 2048 x 14336 x 4096 184 (209, 185), 2048 x 4096 x 14336 166 (234, 165), 2048 x 4096 x 4096
-// 52 (70, 47), 3000 x 28672 x 4096 507 (628, 488), 3000 x 4096 x 14336 259 (304), 512 x 28672 x 8192 170 (245, 186).
+// 1.35 .. 1.5 GHz with the tensor pipe 85 % busy).  S = 4, us in bursts of eight calls one after the other on one GPU, with the one-CTA kernel's time
+// (its best tile) and that of a dense fp16 product of the same shape by cuBLAS: 2048 x 14336 x 4096 195 (207, 185), 2048 x 4096 x 14336 187 (204, 161),
+// 2048 x 4096 x 4096 55 (69, 64), 3000 x 28672 x 4096 579 (632, 505), 512 x 28672 x 8192 181 (258, 234), 512 x 28672 x 4096 92 (130, 114); about
+// equal 3000 x 4096 x 4096 83 (82, 95) and 1100 x 14336 x 4096 116 (119), slower 300 x 4096 x 14336 57 (41).
 //
 // Operands of tcgen05.mma kind::f16, D[256 activation rows, n weight rows] (128 rows of D in each SM's tensor memory), n <= 256:
 //  A (activations, shared memory)  TMA boxes of 128 rows x 64 k straight from x (128-byte swizzle): no re-tiled copy of x exists.
@@ -65,7 +66,7 @@ struct GpParams {
     unsigned int* status;
     int M, N, idx_bytes;
     int vec;                     // lines of S = 4 (2) can be read as 8 (4) bytes
-    int n;                       // weight rows of an item (multiple of 32)
+    int n;                       // weight rows of an item (multiple of 16)
     int MT, MB;                  // activation tiles of 512 rows, blocks of 256 rows
     int MF, full;                // activation tiles that are dealt out together, and their items: see gp_m
     int NG, spg;                 // coefficient groups along K, 64-k stages of each
@@ -177,7 +178,7 @@ struct GpSegs {
 };
 // Activation tile and first weight row of an item.  Where the last activation tile has one block, its items, which are half as long, come
 // after all others: next to the others of the same weight rows they fell to the same
-// pairs every time (1100 x 14336 x 4096: 134 us, now 115).
+// pairs every time (1100 x 14336 x 4096, where this kernel did it: 134 us, so 115).
 __device__ __forceinline__ int gp_m(const GpParams& p, int item) { return item < p.full ? item % p.MF : p.MF; }
 __device__ __forceinline__ int gp_n0(const GpParams& p, int item) { return (item < p.full ? item / p.MF : item - p.full) * p.n; }
 // A part holds the sums of 32 activation rows x 32 weight rows one after the other, each as eight runs of one float4 per activation
@@ -510,7 +511,8 @@ __global__ void __launch_bounds__(GP_THREADS, 1) linear_pair_kernel(const __grid
         const int spg_shift = p.spg == 4 ? 2 : 1;
         const bool row_on = r < half;              // (the others only arrive)
         for (int it = wg; it < stages; it += GP_DWGS) {
-            const int slot = it % GP_WSLOTS, group = it >> spg_shift, turn = p.spg == 4 ? group / 3 : group / 4, pslot = group - turn * (int)pslots, in = it & (p.spg - 1);
+            const int slot = it % GP_WSLOTS, group = it >> spg_shift, in = it & (p.spg - 1);
+            const int turn = p.spg == 4 ? group / 3 : group / 4, pslot = group - turn * (int)pslots;
             const uint32_t dst = w_ring + slot * GP_SLOT + r * 16, src = p_ring + pslot * pbytes;
             if (ok && !gp_wait(p_full + 8 * pslot, (uint32_t)turn & 1u, dead)) ok = false;
             ok = __all_sync(0xffffffffu, ok);
@@ -745,7 +747,10 @@ int launch_linear_pair(const __half* x, int Kin, const PackedW& w, const __half*
     p.bvr = w.bvr, p.idx = w.idx, p.coeff = w.coeff, p.bias = bias, p.y = y, p.status = status;
     p.M = M, p.N = w.N, p.idx_bytes = w.idx_bytes, p.n = pl.n;
     p.vec = !(reinterpret_cast<uintptr_t>(w.coeff) & (2 * w.S - 1));
-    p.MB = (M + 255) / 256, p.MT = (p.MB + 1) / 2, p.MF = p.MB % 2 && p.MT > 1 ? p.MT - 1 : p.MT, p.full = pl.items / p.MT * p.MF, p.NG = w.K / w.G, p.spg = w.G / 64, p.items = pl.items, p.steps = pl.steps;
+    p.MB = (M + 255) / 256, p.MT = (p.MB + 1) / 2;
+    p.MF = p.MB % 2 && p.MT > 1 ? p.MT - 1 : p.MT;
+    p.items = pl.items, p.full = pl.items / p.MT * p.MF;
+    p.NG = w.K / w.G, p.spg = w.G / 64, p.steps = pl.steps;
     p.part = reinterpret_cast<float*>(scratch);
     switch (w.S) {
         case 2: rc = gp_launch<2>(xmap, p, pl.pairs, st); break;

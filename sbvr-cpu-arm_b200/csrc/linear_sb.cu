@@ -867,15 +867,14 @@ bool linear_sb_supported(const PackedW& w, int M) {
     return sb_plan(w, di, &pl) == SBVR_OK;
 }
 
-// Where it is faster than the GEMM.  Up to four chunks of K: 1024 x 4096 9.8 us (the GEMM 10.4; M = 16, S = 4), 4096 x 4096 11.4 (14.8), 14336 x
-// 4096 22.3 (32.1), 32768 x 1024 13.7 (23.1).  Weights of so few rows that the GEMM has one or two tiles: 128 x 14336 12.3 (14.9); up
-// to 2048 rows the chunks' merge costs what the product gains: 1024 x 14336 16.2 (16.1), 512 x 28672 18.3 (18.4).  More chunks and more rows:
-// both times are near linear in what the plans say, the GEMM's in the 64-k stages of a part (dearer with the planes, cheaper without a
-// codebook) and in its fp32 parts,
-// this kernel's in the units of a warpgroup (dearer with two groups a block), the chunks and their sums.  The factors were fitted to
-// minimise what a wrong choice costs over 310 measured calls (2048 .. 14336 rows, K 4352 .. 28672, 5 and 16 rows, S = 2 .. 4, both group
-// lengths): 10 % at most, 0.3 % on average, and 0.1 % over 200 others drawn from the same ranges, with other row counts and encodings; taking this kernel always cost up to 28 % (S = 2, 4096 x 4352, 16 rows: 15.0 against 11.7),
-// the GEMM always up to 69 % (S = 4, 14336 x 5120: 17 against 10 with five rows).
+// Where the automatic choice takes it.  Up to four chunks of K, and few rows of a long K, it is the faster one: M = 16, S = 4, us, here and the GEMM:
+// 1024 x 4096 11.2, 11.1; 4096 x 4096 12.5, 13.8; 14336 x 4096 23.8, 27.9; 32768 x 1024 15.4, 20.9; 128 x 14336 12.8, 20.2.  Up to 2048 rows the
+// chunks' merge costs what the product gains: 1024 x 14336 17.5, 15.0; 512 x 28672 19.7, 22.0.
+// More chunks and more rows: the line lies where it was drawn against an earlier GEMM, which split K evenly (linear_gemm_split still says how), by
+// estimates of both kernels' times.  It stays there for the sake of the results: this kernel's are off by 2.1e-4 (2-norm;
+// the rounding to fp16), the GEMM's by 3.1e-4 to 3.6e-4 with its weights formed in fp16, and a call that had the former keeps it.  What that costs
+// now, over 140 calls drawn from 2048 .. 14336 rows, K 4352 .. 28672, 5 .. 16 rows of x: 10 % on average, nothing at half of them, at most 73 % (2176 x
+// 26368, S = 3, groups of 128, M = 16: 41.9 us, 24.3).
 bool linear_sb_preferred(const PackedW& w, int M, const DeviceInfo& di) {
     if (w.K <= 4096 || w.N <= 256) return true;
     if (w.N < 2048) return false;

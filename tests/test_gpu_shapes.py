@@ -262,8 +262,8 @@ def test_odd_row_counts_keep_fp32_weights(M, N, K, S, mode):
 
 
 def test_threads_on_one_stream():
-    """Calls of several threads on the stream they share: a quantiser and the product that reads its digits, a re-tiling and its
-    GEMM, stay together."""
+    """Calls of several threads on the stream they share: a quantiser and the product that reads its digits, a GEMM and the
+    launch that adds its sums, stay together."""
     import threading
     import sbvr
     N, K = 512, 2048

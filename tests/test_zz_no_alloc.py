@@ -109,7 +109,7 @@ def test_noalloc_matches_regular_entry_point_twice(M):
 
 
 def test_noalloc_batch_that_fits_runs_on_the_batched_kernel():
-    """M = 16 at 1024 x 4096: the batched kernel's re-tiled activations and partial sums fit the 4 MiB array."""
+    """M = 16 at 1024 x 4096: room for a copy of the batched kernel's activations and its partial sums fit the 4 MiB array."""
     import sbvr  # noqa: F401
     from sbvr import _lib
     L = _lib.lib
@@ -129,7 +129,7 @@ def test_noalloc_batch_that_fits_runs_on_the_batched_kernel():
 
 
 def test_noalloc_refuses_what_cannot_fit():
-    """M = 2048 at 4096 x 14336 needs 56 MiB of re-tiled activations: refused with SBVR_ERR_NOALLOC_LIMIT, nothing launched."""
+    """M = 2048 at 4096 x 14336 needs 56 MiB for a copy of the activations: refused with SBVR_ERR_NOALLOC_LIMIT, nothing launched."""
     import sbvr  # noqa: F401
     from sbvr import _lib
     L = _lib.lib
