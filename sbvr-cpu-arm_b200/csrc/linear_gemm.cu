@@ -806,12 +806,14 @@ struct GmPlan {
 // More rows: see gm_many_ns.  270 x 28672 x 8192 in two tiles and in one 212, 119; 384 x 14336 x 4096 62, 40; 384 x 4096 x 4096 28, 36.
 //
 // gm_many_ns and the figures of gp_plan (linear_pair.cu), which decide between the kernels, were fitted to both kernels' times, this one's in tiles
-// of 256 .. 384 rows, at 499 sizes (257 .. 4096 rows, 1024 .. 28672 x 256 .. 14336, S = 2 .. 4, both group lengths): a choice by them costs 0.8 % on average
-// against the fastest of the six, 5 % and more at 25 sizes, 19 % at most.  (By figures that took 1 500 for the ends of every round it was 5.1 %, 129 sizes
-// and 51 %: a tile's results take 2 to 8 us out of D, in which this kernel's MMAs rest.)
+// of 256 .. 384 rows, at 278 sizes (257 .. 4096 rows, 1024 .. 28672 x 256 .. 14336, S = 2 .. 4, both group lengths) in loops of 25 to 60 ms: long runs meet
+// the power limit, as in a model's prefill, and this kernel, which decodes a weight twice as often, more than the other (1024 x 4096 x 14336 101 us, the
+// other 100, in bursts; 124, 111 in loops).  A choice by them costs 0.8 % on average against the fastest of the six, 0.9 % at 220 other sizes, 22 % at most.
+// (By figures that took 1 500 for the ends of every round it was 3.6 and 7 % in bursts, 51 % at most: a tile's results take 4 to 8 us out of D,
+// in which this kernel's MMAs rest.)
 static long long gm_many_ns(int S, int nx, long long rounds, long long last, long long stages, int sm_count) {
-    const long long stage = (stages <= 200 ? 106 : 121) * nx / 100 + 26 * S;               // (longer runs meet the power limit)
-    return 6500 + stages * stage + (rounds - 1) * (2000 + 164 * nx / 10) + 147 * nx / 10 * last / sm_count;
+    const long long t = stages * (115 * nx / 100 + 29 * S), run = t + t * 26 / 100 * std::min(std::max(t - 40000, 0LL), 110000LL) / 110000;
+    return 4100 + run + (rounds - 1) * (4000 + 10 * nx) + 33 * nx / 2 * last / sm_count;
 }
 static GmPlan gm_plan_nx(const PackedW& w, int M, int nx, int sm_count, size_t scratch) {
     GmPlan pl;
@@ -832,7 +834,7 @@ static GmPlan gm_plan_nx(const PackedW& w, int M, int nx, int sm_count, size_t s
     if (left && left * pl.KBS >= ctas && left * pl.KBS * ctas < (1LL << 32)) {             // (every CTA has a window of them at least)
         const size_t bytes = (size_t)(ctas + left) * nx * 512;
         const long long run = (windows + ctas - 1) / ctas * 4;
-        const long long ns = many ? gm_many_ns(w.S, nx, rounds, 0, run, sm_count) + (long long)(bytes / 2000)
+        const long long ns = many ? gm_many_ns(w.S, nx, rounds, 0, run, sm_count) - 600 + (long long)(bytes * 13 / 25000)
                                   : call + 5000 + run * stage + (rounds - 1) * 1500 + (long long)(bytes * 9 / 25000);
         if (ns < pl.ns && bytes <= scratch) pl.whole = false, pl.part_bytes = bytes, pl.grid = (int)ctas, pl.ns = ns;
     }

@@ -687,9 +687,10 @@ struct GpPlan {
 
 // Weight rows of an item, and whether the items that are left over after whole rounds are split over K: the least time in ns, by these
 // figures (see also gm_many_ns, linear_gemm.cu).  A 64-k stage of two blocks takes 160 + 20 S + 2.15 n (790 at n = 256, S = 4), at least 560: the way of
-// three stages of activations through L2 and back.  A launch and its ends take 7 000, another round's ends 1 500 + 9 n, the last one's 6.5 n where
-// all pairs have an item.  A split adds a launch, 5 000, and 0.2 per KB of parts out and back.
+// three stages of activations through L2 and back; runs of 50 to 300 us up to an eighth more (the power limit).  A launch takes 3 100, a round's ends
+// 2 000 + 7 n, the last one's 21 n where all pairs have an item.  A split adds a launch, 6 300, and 0.25 per KB of parts out and back.
 // The scratch it may count on is what sbvr_workspace_bytes promises, whatever the workspace has grown to for other calls.
+static long long gp_run_ns(long long t) { return t + t / 8 * std::min(std::max(t - 50000, 0LL), 250000LL) / 250000; }
 static GpPlan gp_plan(const PackedW& w, int M, int sm_count, int device, size_t scratch) {
     size_t promised = 0;
     if (sbvr_workspace_bytes(device, M, w.N, w.K, &promised) != SBVR_OK) promised = SBVR_WS_FIXED_BYTES;
@@ -702,17 +703,18 @@ static GpPlan gp_plan(const PackedW& w, int M, int sm_count, int device, size_t 
         const long long NT = (w.N + n - 1) / n, items = NT * MT, full = odd ? items - NT : items, rounds = (items + pairs - 1) / pairs, left = items % pairs;
         if (items > (1 << 20)) continue;
         const long long long_ones = (full + pairs - 1) / pairs;                // rounds in which the first pair has an item of two blocks
-        const long long end = 1500 + 9 * n;
+        const long long end = 2000 + 7 * n;
         GpPlan pl = {n, (int)items, (int)std::min(items, pairs), 1, 0, 0};
-        pl.ns = stages * (long_ones * stage + (rounds - long_ones) * half) + (rounds - 1) * end + 13 * n / 2 * (items - (rounds - 1) * pairs) / pairs + 7000;
+        pl.ns = gp_run_ns(stages * (long_ones * stage + (rounds - long_ones) * half)) + (rounds - 1) * end +
+                21 * n * (items - (rounds - 1) * pairs) / pairs + 3100;
         if (!best.n || pl.ns < best.ns) best = pl;
         if (left * NG < pairs || left * NG * pairs >= (1LL << 32)) continue;
         pl.part_bytes = (size_t)(pairs + left) * 16 * ((n + 31) / 32) * 4096;
         pl.pairs = (int)pairs, pl.steps = (int)NG;
         const long long whole = items / pairs, whole_long = std::min(whole, long_ones);
-        pl.ns = stages * (whole_long * stage + (whole - whole_long) * half) +
-                (left * stages + pairs - 1) / pairs * (full > whole * pairs ? stage : half) +              // (cut by steps, long and short)
-                whole * end + 12000 + (long long)(pl.part_bytes / 5000);
+        pl.ns = gp_run_ns(stages * (whole_long * stage + (whole - whole_long) * half) +
+                          (left * stages + pairs - 1) / pairs * (full > whole * pairs ? stage : half)) +  // (cut by steps, long and short)
+                whole * end + 9400 + (long long)(pl.part_bytes / 4000);
         if (pl.part_bytes <= scratch && pl.ns < best.ns) best = pl;
     }
     return best;

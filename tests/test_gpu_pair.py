@@ -35,13 +35,15 @@ def errors(y, x, w, b=None):
     return (d.norm() / ref.norm()).item(), (d.abs().max() / ref.abs().max()).item()
 
 
-@pytest.mark.parametrize("M,N,K,S,G,which", [      # us by the GEMM over CTA pairs and by the one-CTA GEMM
-    (1100, 14336, 2048, 4, 256, "pair"),           # 64, 71
-    (1100, 28672, 512, 4, 128, "pair"),            # 50, 61 in tiles of 384, 73 of 288
+@pytest.mark.parametrize("M,N,K,S,G,which", [      # us by the GEMM over CTA pairs and by the one-CTA GEMM in loops of calls
+    (1100, 14336, 2048, 4, 256, "pair"),           # 71, 78
+    (1100, 28672, 512, 4, 128, "pair"),            # 50, 61 in tiles of 384 rows, 73 of 288
     (768, 28672, 512, 3, 256, "pair"),             # 36, 47
+    (1024, 4096, 14336, 4, 256, "pair"),           # 111, 124
+    (2048, 4096, 14336, 4, 256, "pair"),           # 194, 236
     (384, 1024, 4096, 3, 256, "gemm"),             # 22.8, 19.2
     (600, 14336, 2176, 4, 128, "gemm"),            # 46.2, 46.2
-    (2048, 4096, 14336, 4, 256, "pair"),           # 171, 198
+    (384, 28672, 8192, 4, 128, "gemm"),            # 193, 177
     (300, 4096, 14336, 4, 256, "gemm"),            # 57, 41
 ])
 def test_the_faster_kernel_is_chosen(M, N, K, S, G, which):
@@ -87,7 +89,8 @@ def product(M, N, K, S, G, mode, bias, pair, cut=None):
     (512, 640, 3968, 3, 128, "direct", False, True),           # 31 groups
     (511, 1152, 2304, 3, 256, "u8", True, True),
     (512, 896, 2816, 2, 256, "u16", False, True),              # a last item that is narrower
-    (768, 768, 2304, 4, 256, "direct", True, True),            # items of one block, split
+    (1100, 1920, 6400, 4, 256, "direct", True, True),          # items of one block, split
+    (1750, 5632, 5248, 4, 128, "u16", False, True),            # whole rounds, items of two blocks and of one split
     (1000, 9600, 4352, 4, 256, "u16", True, True),             # whole rounds and split items
 ])
 def test_pair_gemm(M, N, K, S, G, mode, bias, cut):
