@@ -121,8 +121,8 @@ SBVR_API int sbvr_decode_f16(const uint32_t* bvr, const void* coeff_idx, int idx
  *   4 = tcgen05 FP4 tensor-core kernel for small batches (2 <= M <= 32, at most 16 for G = 128; S, G, N and alignment as
  *       for algo 2, K a multiple of 256 and at most 32768; the activations are quantised by a small kernel in front, to 2^-33 of
  *       the largest of a row's 256-k block; needs a workspace of sbvr_workspace_bytes(...); more than 16 rows run on 3).
- * algo 0 takes 2 for M <= 4, 4 for M <= 16 (and for fewer rows where 2 does not apply) where K <= 4096 or N <= 256, or N >= 2048 and 4 is
- * the faster by an estimate from sizes and encoding, 3 otherwise, and 1 for what none of them covers and for very small problems.  A row with a non-finite
+ * algo 0 takes 2 for M <= 4, 4 for M <= 16 (and for fewer rows where 2 does not apply) where K <= 4096 or N <= 256, or N >= 2048 and an
+ * estimate from sizes and encoding takes it, 3 otherwise, and 1 for what none of them covers and for very small problems.  A row with a non-finite
  * activation becomes NaN on 2 and on 4 by request; 1, 3 and 4 where algo 0 picked it multiply it out. */
 SBVR_API int sbvr_linear_f16(const void* x, const uint32_t* bvr, const void* coeff_idx, int idx_bytes, const void* coeff,
                     int C, const void* bias, void* y, int M, int N, int K, int S, int G, int algo,
